@@ -13,6 +13,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace {
 
@@ -32,6 +33,7 @@ struct Context {
     float *rope_cos = nullptr, *rope_sin = nullptr;
     int rope_n_ctx = 0, rope_n_dims = 0;
     float rope_base = 0.f;
+    int *wait_error = nullptr; // host-mapped: a kernel's bounded wait ran out
     int64_t launches = 0;
     bool capturing = false;
     int64_t capture_launches = 0;
@@ -65,6 +67,7 @@ void ggb_count_launch(int n) {
 }
 const uint16_t *ggb_exp_table_dev() { return g_ctx.exp_table; }
 const uint16_t *ggb_gelu_table_dev() { return g_ctx.gelu_table; }
+int *ggb_wait_error_flag() { return g_ctx.wait_error; }
 size_t ggb_tables_bytes() { return 2 * 65536 * 2; } // exp then gelu, contiguous from ggb_exp_table_dev()
 const float *ggb_rope_cos_dev() { return g_ctx.rope_cos; }
 const float *ggb_rope_sin_dev() { return g_ctx.rope_sin; }
@@ -126,6 +129,8 @@ int ggb_init(int device) {
     g_ctx.device = device;
     int rc = build_tables();
     if (rc) return rc;
+    GGB_CUDA(cudaHostAlloc(&g_ctx.wait_error, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    *g_ctx.wait_error = 0;
     g_ctx.init = true;
     return GGB_OK;
 }
@@ -137,6 +142,7 @@ int ggb_shutdown(void) {
     cudaFree(g_ctx.exp_table);
     cudaFree(g_ctx.rope_cos);
     cudaFree(g_ctx.rope_sin);
+    cudaFreeHost(g_ctx.wait_error);
     for (auto &kv : g_ctx.prof) {
         for (auto &p : kv.second.pending) {
             cudaEventDestroy(p.first);
@@ -167,10 +173,19 @@ int ggb_device_info(char *buf, size_t buflen) {
 
 int ggb_sm_count(void) { return g_ctx.init ? g_ctx.prop.multiProcessorCount : 0; }
 
+// after a synchronisation: a kernel whose bounded wait ran out has said so
+static int wait_error_status() {
+    volatile int *e = g_ctx.wait_error;
+    if (!*e) return GGB_OK;
+    *e = 0;
+    ggb_set_error("a kernel's wait ran out: its results are not valid");
+    return GGB_ERR_CUDA;
+}
+
 int ggb_sync(void) {
     GGB_REQUIRE_INIT();
     GGB_CUDA(cudaStreamSynchronize(g_ctx.stream));
-    return GGB_OK;
+    return wait_error_status();
 }
 
 void *ggb_stream(void) { return (void *)g_ctx.stream; }
@@ -202,7 +217,7 @@ int ggb_download(void *dst_host, const void *src_dev, size_t bytes) {
     GGB_REQUIRE_INIT();
     GGB_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDeviceToHost, g_ctx.stream));
     GGB_CUDA(cudaStreamSynchronize(g_ctx.stream));
-    return GGB_OK;
+    return wait_error_status();
 }
 int ggb_host_alloc(size_t bytes, void **hptr) {
     GGB_REQUIRE_INIT();

@@ -10,7 +10,7 @@
 //
 // qkv_store: one CTA per token.  The query is multiplied by its temperature 1 + coef ln(floor((p + 1) / every) + 1) and
 // by the score scale; each value head is divided by its root mean square before it is cached.
-// sigmoid_attn, portions (sigmoid_attn_tile_kernel): a CTA owns 32 consecutive tokens of one head, 4 per warp; tiles of
+// sigmoid_attn, portions: bf16 caches of whole 16-wide heads on the tensor cores (tile_attention.cuh); else sigmoid_attn_tile_kernel: a CTA owns 32 consecutive tokens of one head, 4 per warp; tiles of
 // 32 cache rows are staged once in shared memory as fp32 and serve all 32 queries.  The penalty depends on i - j only:
 // the 63 distances a tile can meet are computed once per tile (63 logarithms instead of 1024).
 // sigmoid_attn, steps of few tokens (sigmoid_attn_step_kernel): 8 warps x up to 16 CTAs split one (token, head)'s keys a
@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "tile_attention.cuh"
 
 namespace {
 
@@ -295,6 +296,17 @@ __global__ void __launch_bounds__(32 * kWarps) sigmoid_attn_tile_kernel(const fl
     }
 }
 
+// what the tensor-core form does with a row of sums (a warp a row)
+struct tile_store {
+    __nv_bfloat16 *out;
+    int H, Dv;
+    struct reads {};
+    __device__ __forceinline__ void load(reads &, int64_t, int64_t, int, int) const {}
+    __device__ __forceinline__ void row(const reads &, const float *o, const float *, float, float, float, int64_t t, int h, int lane) const {
+        for (int c = lane; c < Dv; c += 32) out[(t * H + h) * Dv + c] = __float2bfloat16_rn(o[c]);
+    }
+};
+
 } // namespace
 
 extern "C" {
@@ -334,6 +346,10 @@ int ggb_op_sigmoid_attn(int dt, const float *q, const void *cache, const int32_t
     // 16-byte pieces: rows start 8 numbers apart at least; a head's keys and values must start on such a piece too
     const int vec = D % vn == 0 && ((int64_t)G * D) % vn == 0 && ((uintptr_t)cache % 16 == 0);
     cudaStream_t st = ggb_cuda_stream();
+    if (dt == GGB_TYPE_BF16 && tile_attn::fits(tile_attn::SIGMOID, 1, D, Dv, H, G, q, cache, T)) {
+        const tile_attn::shape sh{q, (const __nv_bfloat16 *)cache, cld, block_table, block_size, pos0, T, H, G, D, Dv, window, 0, 0, 0.f, r1, r2, pb, ggb_wait_error_flag()};
+        return tile_attn::launch<tile_attn::SIGMOID, 1>(sh, tile_store{(__nv_bfloat16 *)out, H, Dv}, st);
+    }
     if (T >= kQT) {
         const bool tv = vec && Dv % vn == 0;
         int kp = D | 1, vp = Dv;

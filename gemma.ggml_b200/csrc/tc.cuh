@@ -1,0 +1,118 @@
+// tc.cuh — tensor-core plumbing of the sm_100a kernels: mbarriers with bounded waits, shared-memory matrix descriptors, tcgen05
+// instructions and tensor-memory loads and stores.
+#pragma once
+
+#include <cuda_bf16.h>
+#include <stdint.h>
+
+// set by a kernel whose wait ran out (host-mapped, checked by ggb_sync): a wait that ends so is an error in the program, never a
+// matter of timing
+int *ggb_wait_error_flag();
+
+#ifdef __CUDACC__
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits for a phase.  Every wait ends: after kWaitTries tries (seconds) the CTA's `dead` word is set, which ends all of its other
+// waits at once; the kernel then runs through with whatever is in its buffers, gives its tensor memory back and reports the failure.
+constexpr int kWaitTries = 1 << 21;
+__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int *dead) {
+    if (mbar_try(bar, parity)) return;
+    for (int i = 0; i < kWaitTries; i++) {
+        if (mbar_try(bar, parity)) return;
+        if (*dead) return;
+    }
+    *dead = 1;
+}
+
+// Shared-memory matrix operands, 128-byte swizzle: rows of 128 bytes, 16-byte piece c of row r at place c ^ (r & 7), 1024-byte atoms
+// of 8 rows that follow one another.  K-major: rows are M / N.  MN-major: rows are K, a row holds 64 numbers of M / N, and lbo is the
+// distance between blocks of 64 numbers of M / N.  A descriptor's upper half (distance of the atoms, version, swizzle) is the same for
+// all of them; the lower one holds the address and lbo.
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr, uint32_t lbo) { return ((saddr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16); }
+constexpr uint32_t kUmmaDescHi = (1024u >> 4) | (1u << 14) | (2u << 29); // 1024 bytes between atoms, sm_100, 128-byte swizzle
+// instruction descriptor, kind::f16: fp32 accumulators, A and B bf16, A K-major, B K-major or (b_mn) MN-major
+__device__ __forceinline__ constexpr uint32_t umma_idesc(int M, int N, bool b_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// MMAs are issued by a whole converged warp, of which the elected lane acts: descriptors and addresses then stay in uniform registers
+// (an `if (lane == 0)` around the loop costs a move per operand and MMA, more than a small MMA takes)
+#define GGB_ELECT "elect.sync _|e, 0xffffffff;\n"
+__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p, e;\n.reg .b64 a, b;\n" GGB_ELECT "setp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+                 "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi)
+                 : "memory");
+}
+// A from tensor memory: row = lane, a 32-bit column holds two neighbours of K
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p, e;\n.reg .b64 b;\n" GGB_ELECT "setp.ne.b32 p, %4, 0;\nmov.b64 b, {%2, %5};\n"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n" ::"r"(tmem_d),
+                 "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi)
+                 : "memory");
+}
+__device__ __forceinline__ void umma_arrive(uint32_t bar) { // arrives when all MMAs issued so far are done
+    asm volatile("{\n.reg .pred e;\n" GGB_ELECT "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar) : "memory");
+}
+#undef GGB_ELECT
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+#define GGB_R8(v, o) "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]), "=r"(v[o + 4]), "=r"(v[o + 5]), "=r"(v[o + 6]), "=r"(v[o + 7])
+#define GGB_S8(v, o) "r"(v[o]), "r"(v[o + 1]), "r"(v[o + 2]), "r"(v[o + 3]), "r"(v[o + 4]), "r"(v[o + 5]), "r"(v[o + 6]), "r"(v[o + 7])
+// 32 lanes x 16 (8) columns.  A load and the wait for it are one statement: no use of a register can move in front of it
+__device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : GGB_R8(v, 0), GGB_R8(v, 8)
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t *v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), GGB_S8(v, 0),
+                 GGB_S8(v, 8)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_store8(uint32_t taddr, const uint32_t *v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), GGB_S8(v, 0) : "memory");
+}
+#undef GGB_R8
+#undef GGB_S8
+// all 512 columns (one CTA a SM), by one warp
+__device__ __forceinline__ void tmem_alloc512(uint32_t slot) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free512(uint32_t base) { asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory"); }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Two fp32 numbers as three pairs of bf16 numbers whose sums they are: 3 x 8 significant bits hold the 24 of an fp32 number, each
+// remainder is exact.  An fp32 x bf16 product is then three bf16 x bf16 products of the tensor cores, each exact before it is added.
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&p);
+}
+__device__ __forceinline__ void split3(float a, float b, uint32_t &h, uint32_t &m, uint32_t &l) {
+    h = pack_bf16x2(a, b);
+    a -= __uint_as_float(h << 16);
+    b -= __uint_as_float(h & 0xffff0000u);
+    m = pack_bf16x2(a, b);
+    a -= __uint_as_float(m << 16);
+    b -= __uint_as_float(m & 0xffff0000u);
+    l = pack_bf16x2(a, b);
+}
+#endif

@@ -8,7 +8,7 @@
 // qkv_store: one CTA per token: root mean square over the whole q and the whole k projection, weights, rotation, store.
 // window_attn, both forms: lane = key for the scores, lane = pair of value coordinates for the weighted sum, running
 // maximum and sum in registers.
-//   portions (window_attn_tile_kernel): a CTA owns 32 consecutive tokens of one head, 4 per warp.  Their windows
+//   portions: bf16 caches of whole 16-wide heads on the tensor cores (tile_attention.cuh); else window_attn_tile_kernel: a CTA owns 32 consecutive tokens of one head, 4 per warp.  Their windows
 //   overlap almost wholly, so every tile of 32 cache rows is staged once in shared memory as fp32 (row pitch odd in words:
 //   lane = row reads are conflict-free) and serves all 32 queries; a K word read feeds 4 multiply-adds.
 //   steps of few tokens (window_attn_kernel): 8 warps split one (token, head)'s keys, rows straight from the cache
@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "tile_attention.cuh"
 
 namespace {
 
@@ -631,6 +632,67 @@ __global__ void __launch_bounds__(32 * kWarps) window_attn_tile_kernel(const flo
     }
 }
 
+// what the tensor-core form does with a row of sums (a warp a row): as window_finish and diff_finish
+template <int MAPS> struct tile_finish {
+    finish_args fa;
+    const float *cs_v;
+    __nv_bfloat16 *out;
+    int H, Dv;
+    struct reads {
+        float gate[4], cs[4], sink;
+    };
+    __device__ __forceinline__ static int coord(int lane, int r) { return 2 * lane + 64 * (r >> 1) + (r & 1); }
+    __device__ __forceinline__ void load(reads &rd, int64_t i, int64_t t, int h, int lane) const {
+        rd.sink = fa.sink ? __ldg(fa.sink + h) : 0.f;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int c = coord(lane, r);
+            rd.gate[r] = fa.gate && c < Dv ? __ldg(fa.gate + t * fa.ldg + (int64_t)h * Dv + c) : 0.f;
+            rd.cs[r] = cs_v && c < Dv ? __ldg(cs_v + i * Dv + c) : 0.f; // pair c / 2: [cos, sin]
+        }
+    }
+    __device__ __forceinline__ void row(const reads &rd, const float *o1, const float *o2, float m, float l, float l2, int64_t t, int h, int lane) const {
+        float o[4];
+        if (MAPS == 1) {
+            float inv = 1.0f / l;
+            if (fa.sink) {
+                const float M = fmaxf(m, rd.sink), f = expf(m - M);
+                inv = f / (l * f + expf(rd.sink - M));
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++) o[r] = coord(lane, r) < Dv ? o1[coord(lane, r)] * inv : 0.f;
+            if (cs_v) {
+#pragma unroll
+                for (int r = 0; r < 4; r += 2) { // turned back: by -i
+                    const float u = o[r] * rd.cs[r] + o[r + 1] * rd.cs[r + 1], w = o[r + 1] * rd.cs[r] - o[r] * rd.cs[r + 1];
+                    o[r] = u, o[r + 1] = w;
+                }
+            }
+        } else {
+            const float i1 = 1.0f / l, i2 = fa.lambda / l2;
+            float ss = 0.f;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                o[r] = coord(lane, r) < Dv ? o1[coord(lane, r)] * i1 - o2[coord(lane, r)] * i2 : 0.f;
+                ss = fmaf(o[r], o[r], ss);
+            }
+            const float f = fa.scale / sqrtf(warp_sum_f32(ss) / (float)Dv + fa.eps);
+#pragma unroll
+            for (int r = 0; r < 4; r++) o[r] *= f;
+        }
+        if (fa.gate) {
+#pragma unroll
+            for (int r = 0; r < 4; r++) o[r] *= tile_attn::sigmoid_fast(rd.gate[r]);
+        }
+        __nv_bfloat16 *orow = out + (t * H + h) * Dv;
+#pragma unroll
+        for (int r = 0; r < 4; r += 2) {
+            const int c = coord(lane, r);
+            if (c < Dv) *reinterpret_cast<uint32_t *>(orow + c) = pack_bf16x2(o[r], o[r + 1]);
+        }
+    }
+};
+
 } // namespace
 
 extern "C" {
@@ -726,6 +788,11 @@ static int masked_attn_launch(int dt, const float *q, const void *cache, const i
     const int es = dt == GGB_TYPE_BF16 ? 2 : 4, vn = 16 / es;
     const int vec = D % vn == 0 && ((uintptr_t)cache % 16 == 0); // rows are 8 numbers apart at least: 16-byte aligned in both types
     cudaStream_t st = ggb_cuda_stream();
+    if (dt == GGB_TYPE_BF16 && (uintptr_t)out % 4 == 0 && tile_attn::fits(tile_attn::SOFTMAX, MAPS, D, Dv, H, G, q, cache, T)) {
+        const tile_attn::shape sh{q, (const __nv_bfloat16 *)cache, cld, block_table, block_size, pos0, T, H, G, D, Dv, window, chunked, keep, softcap,
+                                  nullptr, nullptr, nullptr, ggb_wait_error_flag()};
+        return tile_attn::launch<tile_attn::SOFTMAX, MAPS>(sh, tile_finish<MAPS>{da, cos_sin_v, (__nv_bfloat16 *)out, H, Dv}, st);
+    }
     if (T >= kQT) { // a portion: tiles of cache rows staged once for 32 queries
         // 16-byte pieces need every head's keys and values to start on one: D, Dv and G * D whole pieces
         const bool tv = vec && Dv % vn == 0 && ((int64_t)G * D) % vn == 0;

@@ -1,0 +1,108 @@
+"""The tensor-core form of attention over portions (csrc/tile_attention.cuh) against float64, at the edges of its tiles: 128 query rows
+(tokens x heads of a key head, or half as many with two maps) and 64 keys.  Both sides see the same bf16 cache and fp32 queries; the
+result differs by its rounding to bf16, at most 2^-9 of a value, plus fp32 sums (1e-6): a relative error (2-norm) of 2.5e-3 at most."""
+import numpy as np
+import pytest
+
+from device_util import BF16, F32, as_dt, dev, f32, from_dt, i32, ptr, release, zeros
+
+pytestmark = pytest.mark.gpu
+LIMIT = 2.5e-3
+
+
+@pytest.fixture(autouse=True)
+def _release_buffers():
+    yield
+    release()
+
+
+def inputs(gpu, dt, H, G, D, Dv, maps, pos, T, page, seed, scale):
+    r = np.random.default_rng(seed)
+    n, ld = pos + T, int(gpu.cuda_lib().ggb_window_cache_ld(G, D * maps, Dv))
+    pages = (n + page - 1) // page
+    table = r.permutation(pages + 2)[:pages].astype(np.int32)
+    cache, raw = as_dt(BF16, r.standard_normal(((pages + 2) * page, ld)))
+    rows = cache[table[np.arange(n) // page].astype(np.int64) * page + np.arange(n) % page]
+    q = f32(r.standard_normal((T, H, maps, D)) * scale)
+    if dt == F32:
+        raw = f32(cache)
+    K = rows[:, :G * maps * D].reshape(n, G, maps, D)
+    V = rows[:, G * maps * D:G * (maps * D + Dv)].reshape(n, G, Dv)
+    return r, q, K, V, dev(gpu, raw), dev(gpu, table), dev(gpu, i32([pos]))
+
+
+def seen(pos, T, window, keep, chunked):
+    i, j = np.arange(pos, pos + T)[:, None], np.arange(pos + T)[None]
+    if window <= 0:
+        return j <= i
+    lo = i - i % window if chunked else i - window + 1
+    return (j <= i) & ((j >= lo) | (j < keep))
+
+
+def soft(q, K, V, vis, cap, sink):
+    s = q @ K.T
+    s = np.where(vis, cap * np.tanh(s / cap) if cap else s, -np.inf)
+    m = np.maximum(s.max(1), sink if sink is not None else -np.inf)
+    e = np.exp(s - m[:, None])
+    return (e @ V) / (e.sum(1) + (np.exp(sink - m) if sink is not None else 0.0))[:, None]
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+# H, Gk, D, Dv, T, pos, page, window, keep, chunked, cap, scale, sink, gate
+SOFT = [(1, 1, 16, 16, 32, 0, 64, 0, 0, 0, 0.0, 0.3, 1, 0), (4, 1, 64, 64, 33, 31, 64, 0, 0, 0, 0.0, 0.1, 0, 1), (3, 1, 80, 112, 129, 64, 7, 65, 1, 0, 30.0, 0.2, 1, 1),
+        (2, 2, 128, 128, 128, 0, 64, 64, 0, 0, 30.0, 1.0, 0, 0), (16, 1, 128, 128, 40, 500, 64, 300, 70, 0, 2.0, 0.5, 0, 1), (6, 2, 192, 128, 127, 129, 16, 100, 0, 1, 0.0, 0.1, 0, 0),
+        (5, 5, 48, 96, 200, 3, 64, 1, 130, 0, 0.0, 0.3, 1, 0), (8, 8, 96, 80, 300, 700, 64, 128, 64, 0, 0.0, 2.0, 0, 1), (128, 1, 32, 32, 35, 66, 64, 0, 0, 0, 5.0, 0.4, 0, 0)]
+
+
+@pytest.mark.parametrize("dt", [BF16, F32])
+@pytest.mark.parametrize("H,Gk,D,Dv,T,pos,page,window,keep,chunked,cap,scale,sink,gate", SOFT)
+def test_soft_max_heads(gpu, dt, H, Gk, D, Dv, T, pos, page, window, keep, chunked, cap, scale, sink, gate):
+    G = Gk
+    r, q, K, V, cache, table, pos0 = inputs(gpu, dt, H, G, D, Dv, 1, pos, T, page, D + T, scale)
+    s, g = r.standard_normal(H), r.standard_normal((T, H * Dv))
+    out = zeros(gpu, T * H * Dv * (2 if dt == BF16 else 4))
+    lib = gpu.cuda_lib()
+    if chunked:
+        gpu.check(lib.ggb_op_masked_attn(dt, dev(gpu, q).ptr, cache.ptr, table.ptr, page, pos0.ptr, T, H, G, D, Dv, window, 1, cap, None, out.ptr, None), "attn")
+    else:
+        gpu.check(lib.ggb_op_masked_attn_gated(dt, dev(gpu, q).ptr, cache.ptr, table.ptr, page, pos0.ptr, T, H, G, D, Dv, window, keep, cap, ptr(dev(gpu, f32(s)) if sink else None),
+                                               ptr(dev(gpu, f32(g)) if gate else None), H * Dv, out.ptr, None), "attn")
+    vis = seen(pos, T, window, keep, chunked)
+    want = np.stack([soft(q[:, h, 0].astype(np.float64), K[:, h // (H // G), 0], V[:, h // (H // G)], vis, cap, f32(s)[h].astype(np.float64) if sink else None) for h in range(H)], 1)
+    want = want.reshape(T, H * Dv) / (1.0 + np.exp(-f32(g).astype(np.float64)) if gate else 1.0)
+    assert rel(from_dt(dt, out, (T, H * Dv)), want) < (LIMIT if dt == BF16 else 1e-5)
+
+
+@pytest.mark.parametrize("H,Gk,D,Dv,T,pos,window,keep,cap", [(2, 1, 16, 16, 32, 0, 0, 0, 0.0), (4, 2, 64, 128, 65, 63, 64, 3, 30.0), (3, 3, 128, 128, 64, 200, 0, 0, 2.0), (64, 1, 32, 48, 33, 90, 70, 65, 0.0)])
+def test_differential_heads(gpu, H, Gk, D, Dv, T, pos, window, keep, cap):
+    G = Gk
+    r, q, K, V, cache, table, pos0 = inputs(gpu, BF16, H, G, D, Dv, 2, pos, T, 64, D + T, 0.3)
+    out, lam, eps = zeros(gpu, T * H * Dv * 2), 0.4, 1e-5
+    gpu.check(gpu.cuda_lib().ggb_op_diff_attn(BF16, dev(gpu, q).ptr, cache.ptr, table.ptr, 64, pos0.ptr, T, H, G, D, Dv, window, keep, cap, lam, 0.7, eps, None, 0, out.ptr, None), "attn")
+    vis, q = seen(pos, T, window, keep, 0), q.astype(np.float64)
+    o = np.stack([soft(q[:, h, 0], K[:, h // (H // G), 0], V[:, h // (H // G)], vis, cap, None) - np.float32(lam) * soft(q[:, h, 1], K[:, h // (H // G), 1], V[:, h // (H // G)], vis, cap, None)
+                  for h in range(H)], 1)
+    o = o / np.sqrt((o ** 2).mean(-1, keepdims=True) + eps) * 0.7
+    assert rel(from_dt(BF16, out, (T, H, Dv)), o) < LIMIT
+
+
+@pytest.mark.parametrize("H,Gk,D,Dv,T,pos,window,page,bare", [(1, 1, 16, 16, 32, 0, 0, 64, 0), (4, 1, 64, 64, 33, 31, 0, 5, 0), (16, 1, 128, 128, 129, 64, 65, 64, 0), (6, 2, 80, 96, 200, 700, 128, 64, 0),
+                                                            (64, 1, 48, 32, 40, 100, 0, 64, 0), (3, 3, 128, 128, 128, 0, 1, 64, 1)])
+def test_sigmoid_heads(gpu, H, Gk, D, Dv, T, pos, window, page, bare):
+    G = Gk
+    r, q, K, V, cache, table, pos0 = inputs(gpu, BF16, H, G, D, Dv, 1, pos, T, page, D + T, 1.5)
+    r1, r2, pb = f32(r.uniform(0.2, 1.0, H)), f32(r.uniform(0.1, 1.5, H)), f32(r.uniform(-2.5, 0.0, H))
+    d = [None if bare else dev(gpu, a) for a in (r1, r2, pb)]
+    out = zeros(gpu, T * H * Dv * 2)
+    gpu.check(gpu.cuda_lib().ggb_op_sigmoid_attn(BF16, dev(gpu, q).ptr, cache.ptr, table.ptr, page, pos0.ptr, T, H, G, D, Dv, window, *(ptr(x) for x in d), out.ptr, None), "attn")
+    vis, dist = seen(pos, T, window, 0, 0), np.maximum(np.arange(pos, pos + T)[:, None] - np.arange(pos + T)[None], 0)
+    want = []
+    for h in range(H):
+        z = q[:, h, 0].astype(np.float64) @ K[:, h // (H // G), 0].T
+        if not bare:
+            z = z - np.float64(r1[h]) * np.log1p(np.float64(r2[h]) * dist) + np.float64(pb[h])
+        want.append((vis / (1.0 + np.exp(-z))) @ V[:, h // (H // G)])
+    assert rel(from_dt(BF16, out, (T, H, Dv)), np.stack(want, 1)) < LIMIT
