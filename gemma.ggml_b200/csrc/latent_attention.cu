@@ -8,6 +8,8 @@
 // that borrows another layer's cache only brings its own W_uk / W_uv.  The soft-max carries a per-head sink: one more
 // term exp(sink_h) in the denominator that has no key and no value.
 //
+// Portions over a bf16 cache run on the tensor cores (latent_tile.cuh).
+//
 // Scores, soft-max and the weighted sums are fp32 whatever the storage type of the cache; -fmad=false: fmaf() spelled.
 // The cache is paged: position j lives in row table[j / B] * B + j % B.  Positions of a step's tokens are
 // *pos0 + t with *pos0 read on the device, so a captured step can be replayed at another position.
@@ -16,6 +18,7 @@
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "latent_tile.cuh"
 
 namespace {
 
@@ -688,6 +691,15 @@ int ggb_op_latent_attn_window(int dt, const float *qa, const void *cache, const 
                       n_split <= 65535 && block_size > 0,
                   "latent_attn: bad arguments (latent size up to 1024)");
     const int64_t ldk = ggb_latent_cache_ld(R, Dr);
+    if (dt == GGB_TYPE_BF16 && latent_tile::fits(R, Dr, H, T, qa, cache)) {
+        const int vp = R <= 256 ? R : R / 2, tq = latent_tile::kRows / H;
+        const latent_tile::args a{qa, (const __nv_bfloat16 *)cache, ldk, block_table, block_size, pos0, (int)T, H, R, R + Dr, vp, window, part, ggb_wait_error_flag()};
+        GGB_CUDA(cudaFuncSetAttribute(latent_tile::latent_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)latent_tile::kSmem));
+        latent_tile::latent_tile_kernel<<<dim3((unsigned)((T + tq - 1) / tq), (unsigned)n_split, (unsigned)(R / vp)), latent_tile::kThreads, latent_tile::kSmem,
+                                          ggb_cuda_stream()>>>(a);
+        GGB_LAUNCH_CHECK();
+        return GGB_OK;
+    }
     if (dt == GGB_TYPE_BF16)
         return attn_partial_launch<__nv_bfloat16>(qa, cache, ldk, block_table, block_size, pos0, T, H, R, Dr, n_split, window, part);
     return attn_partial_launch<float>(qa, cache, ldk, block_table, block_size, pos0, T, H, R, Dr, n_split, window, part);
@@ -704,6 +716,14 @@ int ggb_op_latent_attn_out_gated(int dt, const float *part, int n_split, const f
     GGB_REQUIRE_INIT();
     GGB_CHECK_DT(dt);
     GGB_CHECK_ARG((!gate || ldg >= H) && part && w_uv && out && T > 0 && H > 0 && R > 0 && Dv > 0 && n_split > 0, "latent_attn_out: bad arguments");
+    if (dt == GGB_TYPE_BF16 && latent_tile::out_fits(R, Dv, T, n_split, w_uv, out)) {
+        const latent_tile::out_args a{part, n_split, sink, (const __nv_bfloat16 *)w_uv, (int)T, H, R, Dv, gate, ldg, (__nv_bfloat16 *)out, ggb_wait_error_flag()};
+        GGB_CUDA(cudaFuncSetAttribute(latent_tile::latent_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)latent_tile::kOutSmem));
+        latent_tile::latent_out_kernel<<<dim3((unsigned)((T + latent_tile::kRows - 1) / latent_tile::kRows), (unsigned)H), latent_tile::kThreads, latent_tile::kOutSmem,
+                                         ggb_cuda_stream()>>>(a);
+        GGB_LAUNCH_CHECK();
+        return GGB_OK;
+    }
     // few tokens: spread a head's outputs over several CTAs; many tokens: the grid is large already, merge once per head
     const int v_chunk = T * H >= 1024 ? Dv : 16;
     const dim3 grid((unsigned)((T + kOutT - 1) / kOutT), (unsigned)H, (unsigned)((Dv + v_chunk - 1) / v_chunk));
