@@ -21,12 +21,12 @@ struct ggb_moe_groups {
 int ggb_linear_grouped_launch(int dt, const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int max_tiles, float *c,
                               void *c_act, int64_t ldc, int act, const ggb_moe_groups &grp);
 
-// the tcgen05 GEMM of prefill.cu on plain bf16 matrices: C[T][N] (fp32) = A[T][K] W[N][K]^T; with c_act it leaves as bf16 act(C)
+// the tcgen05 GEMM on plain bf16 matrices (gemm.cu): C[T][N] (fp32) = A[T][K] W[N][K]^T; with c_act it leaves as bf16 act(C)
 // instead (GGB_ACT_*, ldc %% 8 == 0)
 bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc);
 int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t T, float *c, int64_t ldc, void *c_act = nullptr, int act = 0);
 
-// the grouped tcgen05 form: w [n_exp][N][K] bf16, a rows in sorted-slot order, offsets [n_exp + 1] on the device;
+// the grouped tcgen05 form: w [n_exp][N][K] bf16, a: n_rows rows in all, in sorted-slot order, offsets [n_exp + 1] on the device;
 // c fp32 or (c_act) bf16 act(c)
 bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc);
 int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, float *c,

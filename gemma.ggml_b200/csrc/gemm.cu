@@ -1,0 +1,389 @@
+// gemm.cu — products of plain bf16 matrices on the tensor cores: C[T][N] = A[T][K] W[N][K]^T, and the grouped form for a mixture of experts.
+//
+// A tile of C is 256 x 256 or 128 x (256, 128, 64).  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
+// in a ring that takes all of shared memory but the epilogue's corner; one warp issues the MMAs, eight drain tensor memory.  CTAs are
+// persistent: where a tile needs half of tensor memory, the next one's products run while the last one's are stored.  The epilogue
+// turns 32 x 32 pieces in shared memory, so that a store instruction writes whole 128-byte lines.
+//
+// A product along a long K is summed in `chunks` pieces of K, each with an accumulator of its own in tensor memory, added up in order by
+// the epilogue (the tensor cores truncate a running sum at every step: shorter sums are more exact), and, where that still leaves SMs
+// without work, over several CTAs that meet in a workspace.  The number of pieces is what a split over the SMs in 256 x 256 tiles needs;
+// the tile is then the one with the least estimated time.
+//
+// What bounds it: 1024 x 8192 x 2048 runs in one round of 128 tiles, 32 stages of 1024 cycles of the tensor cores each (61 % of the kernel's
+// cycles); the stores behind the last stage, which nothing hides in a single round, take 6 us.  38.8 us, 885 TFLOP/s (47.6 us with both
+// operands copied by cp.async and rows stored by their own lanes; 40.9 us in 128 x 256 tiles).  32 experts x 128 rows, 1408 x 2048: 47 us a
+// product, 4.2 TB/s of matrices (256-row tiles, half of them empty: 68 us).
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "dense.cuh"
+#include "tc.cuh"
+
+namespace {
+
+constexpr int BK = 64;
+constexpr int kThreads = 384; // warp 0: TMA, 1: MMA, 2: tensor memory, 4..11: epilogue
+constexpr uint32_t kRing = 192 * 1024, kTurn = 8 * 4096;
+constexpr int kMaxStages = 8, kMaxGroups = 256; // groups whose first tiles are kept in shared memory
+constexpr size_t kSmem = 1024 + kRing + kTurn + 256;
+enum { FULL = 0, EMPTY = 64, ACC_FULL = 128, ACC_FREE = 144, SLOT = 160, DEAD = 168 };
+
+struct gemm_args {
+    int T, N, kblocks;
+    int BN, n_tiles, m_tiles;
+    int chunks, chunk_kb, splits; // K pieces a CTA sums, their blocks of 64, CTAs along K
+    int stages;
+    const int32_t *m_ranges; // grouped: group g has the rows [m_ranges[g], m_ranges[g + 1]) of A and C and the rows g * N .. of W
+    int n_groups;
+    float *c;
+    __nv_bfloat16 *act_out; // when set: bf16 act(c) instead of c
+    int act;
+    int64_t ldc;
+    int vec; // rows of C start on 16 bytes
+    float *ws; // [splits][T][N] or null
+    int *wait_error;
+};
+
+struct tile_at {
+    int m0, m_end, n0, split, group;
+};
+
+template <int BM>
+__global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
+    extern __shared__ uint8_t gm_raw[];
+    __shared__ int first_tile[kMaxGroups + 1]; // grouped: the first row tile of a group
+    const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, turn = base + kRing, bars = turn + kTurn;
+    uint8_t *ctl = gm_raw + (bars - raw0);
+    volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t a_bytes = BM * 128, stage_bytes = a_bytes + (uint32_t)a.BN * 128;
+    const uint32_t acc_cols = (uint32_t)(BM / 128 * a.chunks * a.BN);
+    const int n_acc = acc_cols <= 256 ? 2 : 1;
+    if (tid == 0) {
+        for (int s = 0; s < a.stages; s++) {
+            mbar_init(bars + FULL + 8 * s, 1);
+            mbar_init(bars + EMPTY + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(bars + ACC_FULL + 8 * s, 1);
+            mbar_init(bars + ACC_FREE + 8 * s, 8);
+        }
+        *dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) tmem_alloc512(bars + SLOT);
+    const bool listed = a.m_ranges && a.n_groups <= kMaxGroups;
+    if (listed && warp == 3) { // prefix sums of the groups' row tiles
+        int sum = 0;
+        for (int g0 = 0; g0 < a.n_groups; g0 += 32) {
+            const int g = g0 + lane;
+            int v = g < a.n_groups ? (a.m_ranges[g + 1] - a.m_ranges[g] + BM - 1) / BM : 0;
+            for (int off = 1; off < 32; off *= 2) {
+                const int o = __shfl_up_sync(0xffffffffu, v, off);
+                if (lane >= off) v += o;
+            }
+            if (g < a.n_groups) first_tile[g + 1] = sum + v;
+            sum += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) first_tile[0] = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
+    int row_tiles = a.m_tiles;
+    if (listed) row_tiles = first_tile[a.n_groups];
+    else if (a.m_ranges) {
+        row_tiles = 0;
+        for (int g = 0; g < a.n_groups; g++) row_tiles += (a.m_ranges[g + 1] - a.m_ranges[g] + BM - 1) / BM;
+    }
+    const int total = row_tiles * a.n_tiles * a.splits;
+    auto locate = [&](int t) {
+        tile_at r;
+        r.group = 0;
+        if (!a.m_ranges) { // row tiles first: those that share a piece of W run together
+            r.m0 = t % a.m_tiles * BM;
+            r.m_end = a.T;
+            t /= a.m_tiles;
+            r.n0 = t % a.n_tiles * a.BN;
+            r.split = t / a.n_tiles;
+            return r;
+        }
+        const int rt = t / a.n_tiles;
+        r.n0 = (t - rt * a.n_tiles) * a.BN;
+        r.split = 0;
+        int f;
+        if (listed) {
+            int lo = 0, hi = a.n_groups - 1; // the last group whose first tile is not behind rt
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (first_tile[mid] <= rt) lo = mid;
+                else hi = mid - 1;
+            }
+            r.group = lo;
+            f = first_tile[lo];
+        } else {
+            f = 0;
+            for (;; r.group++) {
+                const int n = (a.m_ranges[r.group + 1] - a.m_ranges[r.group] + BM - 1) / BM;
+                if (f + n > rt) break;
+                f += n;
+            }
+        }
+        r.m0 = a.m_ranges[r.group] + (rt - f) * BM;
+        r.m_end = a.m_ranges[r.group + 1];
+        return r;
+    };
+    auto k_range = [&](int split, int &kb0, int &kb1) {
+        kb0 = split * a.chunks * a.chunk_kb;
+        kb1 = min(kb0 + a.chunks * a.chunk_kb, a.kblocks);
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 0;
+            for (int t = blockIdx.x; t < total; t += gridDim.x) {
+                const tile_at at = locate(t);
+                int kb0, kb1;
+                k_range(at.split, kb0, kb1);
+                for (int kb = kb0; kb < kb1; kb++) {
+                    mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead);
+                    const uint32_t sa = base + s * stage_bytes, bar = bars + FULL + 8 * s;
+                    mbar_expect_tx(bar, stage_bytes);
+                    tma_load_2d(sa, &map_a, kb * BK, at.m0, bar);
+                    tma_load_2d(sa + a_bytes, &map_w, kb * BK, at.group * a.N + at.n0, bar);
+                    if (++s == a.stages) s = 0, ph ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        const uint32_t idesc = umma_idesc(128, a.BN);
+        int s = 0, it = 0;
+        uint32_t ph = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
+            int kb0, kb1, chunk = 0, left = a.chunk_kb;
+            k_range(locate(t).split, kb0, kb1);
+            const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
+            mbar_wait_bounded(bars + ACC_FREE + 8 * buf, (use & 1) ^ 1, dead);
+            tc_fence_after();
+            for (int kb = kb0; kb < kb1; kb++) {
+                mbar_wait_bounded(bars + FULL + 8 * s, ph, dead);
+                tc_fence_after();
+                const uint32_t a_lo = umma_desc_lo(base + s * stage_bytes, 16), w_lo = umma_desc_lo(base + s * stage_bytes + a_bytes, 16);
+                const uint32_t first = left == a.chunk_kb ? 0u : 1u;
+#pragma unroll
+                for (int mt = 0; mt < BM / 128; mt++) {
+                    const uint32_t d = tmem + buf * 256 + (mt * a.chunks + chunk) * a.BN;
+#pragma unroll
+                    for (int k = 0; k < BK / 16; k++) umma_ss(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, w_lo + 2 * k, idesc, k > 0 ? 1u : first);
+                }
+                umma_arrive(bars + EMPTY + 8 * s);
+                if (++s == a.stages) s = 0, ph ^= 1u;
+                if (--left == 0) chunk++, left = a.chunk_kb;
+            }
+            umma_arrive(bars + ACC_FULL + 8 * buf);
+        }
+    } else if (warp >= 4) {
+        const int w8 = warp - 4, lq = warp & 3, half = w8 >> 2;
+        const uint32_t my = turn + w8 * 4096;
+        int it = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
+            const tile_at at = locate(t);
+            int kb0, kb1;
+            k_range(at.split, kb0, kb1);
+            const int chunks = (kb1 - kb0 + a.chunk_kb - 1) / a.chunk_kb; // the last CTA along K may have fewer
+            const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
+            mbar_wait_bounded(bars + ACC_FULL + 8 * buf, use & 1, dead);
+            tc_fence_after();
+            // a warp's 32 rows, every other 32 columns (the two warps of a quarter share them)
+            for (int mt = 0; mt < BM / 128; mt++) {
+                const int row0 = at.m0 + mt * 128 + lq * 32;
+                if (row0 >= at.m_end) break;
+                for (int c0 = 32 * half; c0 < a.BN; c0 += 64) {
+                    if (at.n0 + c0 >= a.N) break;
+                    uint32_t v[32];
+                    const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + mt * a.chunks * a.BN + c0;
+                    if (chunks > 0) tmem_load32(col, v);
+                    else // no block of K is left for this CTA
+                        for (int q = 0; q < 32; q++) v[q] = 0;
+                    for (int ch = 1; ch < chunks; ch++) {
+                        uint32_t u[32];
+                        tmem_load32(col + ch * a.BN, u);
+#pragma unroll
+                        for (int q = 0; q < 32; q++) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(u[q]));
+                    }
+                    // row = lane -> eight lanes a row: 16-byte piece p of row r at place p ^ (r & 7)
+                    __syncwarp();
+#pragma unroll
+                    for (int p = 0; p < 8; p++)
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(my + lane * 128 + ((p ^ (lane & 7)) << 4)), "r"(v[4 * p]), "r"(v[4 * p + 1]), "r"(v[4 * p + 2]),
+                                     "r"(v[4 * p + 3])
+                                     : "memory");
+                    __syncwarp();
+                    const int p = lane & 7, n = at.n0 + c0 + 4 * p;
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const int r = 4 * q + (lane >> 3), row = row0 + r;
+                        float4 o;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(my + r * 128 + ((p ^ (r & 7)) << 4)) : "memory");
+                        if (row >= at.m_end || n >= a.N) continue;
+                        if (a.act_out && !a.ws) { // the next product's operand; N and ldc are multiples of 8
+                            uint2 y;
+                            y.x = pack_bf16x2(act_f32(o.x, a.act), act_f32(o.y, a.act));
+                            y.y = pack_bf16x2(act_f32(o.z, a.act), act_f32(o.w, a.act));
+                            *reinterpret_cast<uint2 *>(a.act_out + row * a.ldc + n) = y;
+                        } else { // N is a multiple of 4
+                            float *dst = a.ws ? a.ws + ((int64_t)at.split * a.T + row) * a.N + n : a.c + row * a.ldc + n;
+                            if (a.vec) *reinterpret_cast<float4 *>(dst) = o;
+                            else dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + ACC_FREE + 8 * buf);
+        }
+    }
+    __syncthreads();
+    if (warp == 2) {
+        tc_fence_after();
+        tmem_free512(tmem);
+        if (lane == 0 && *dead) *a.wait_error = 1;
+    }
+}
+
+// the CTAs' sums along K in order
+__global__ void splits_add_kernel(const float *__restrict__ ws, int splits, int64_t T, int64_t N, float *__restrict__ c, __nv_bfloat16 *__restrict__ act_out, int act,
+                                  int64_t ldc) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; // N is a multiple of 4
+    if (i >= T * N) return;
+    const int64_t t = i / N, n = i - t * N;
+    float4 s = *reinterpret_cast<const float4 *>(ws + i);
+    for (int k = 1; k < splits; k++) {
+        const float4 v = *reinterpret_cast<const float4 *>(ws + (int64_t)k * T * N + i);
+        s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+    }
+    const float o[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        if (act_out) act_out[t * ldc + n + u] = __float2bfloat16_rn(act_f32(o[u], act));
+        else c[t * ldc + n + u] = o[u];
+    }
+}
+
+int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int BM, const gemm_args &g, int ctas) {
+    CUtensorMap ma, mw;
+    int rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
+    if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
+    if (rc) return rc;
+    auto kfn = BM == 256 ? gemm_tma_kernel<256> : gemm_tma_kernel<128>;
+    GGB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    kfn<<<std::min(ctas, ggb_sm_count()), kThreads, kSmem, ggb_cuda_stream()>>>(ma, mw, g);
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
+}
+
+int stages_of(int BM, int BN) { return std::min<int>(kMaxStages, (int)(kRing / (uint32_t)((BM + BN) * 128))); }
+
+} // namespace
+
+int ggb_tensor_map_bf16(CUtensorMap_st *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+    typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static encode_fn encode = nullptr;
+    if (!encode) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        GGB_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr));
+        GGB_CHECK_ARG(fn && qr == cudaDriverEntryPointSuccess, "cuTensorMapEncodeTiled is not in the driver");
+        encode = (encode_fn)fn;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, pitch[1] = {(cuuint64_t)ld * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, step[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, pitch, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    GGB_CHECK_ARG(r == CUDA_SUCCESS, "tensor map of %lld x %lld numbers, pitch %lld: error %d", (long long)rows, (long long)cols, (long long)ld, (int)r);
+    return GGB_OK;
+}
+
+bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc) {
+    return T >= 64 && K % 64 == 0 && N % 32 == 0 && ldc % 4 == 0 && N < (1ll << 31) && K < (1ll << 31) && T < (1ll << 31);
+}
+
+// The K-split workspace belongs to the library and only grows (one stream, no capture: products of 64 rows and more).
+int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
+    GGB_REQUIRE_INIT();
+    GGB_CHECK_ARG(w && a && (c || c_act) && ((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
+    GGB_CHECK_ARG(!c_act || ldc % 8 == 0, "gemm: an activation takes rows of whole 16-byte pieces");
+    const int sms = ggb_sm_count(), kblocks = (int)(K / BK);
+    int pieces = 1; // along K, until every SM has a piece of a 256 x 256 tile
+    const int64_t big = (N + 255) / 256 * ((T + 255) / 256);
+    while (pieces < 8 && big * pieces * 2 <= sms && kblocks / (pieces * 2) >= 4) pieces *= 2;
+    gemm_args g{};
+    double best = 0.0;
+    int BM = 0;
+    static const int shapes[4][2] = {{256, 256}, {128, 256}, {128, 128}, {128, 64}};
+    for (const auto &sh : shapes)
+        for (int splits = 1; splits <= pieces; splits *= 2) {
+            const int chunks = pieces / splits, bm = sh[0], bn = sh[1];
+            if (bm / 128 * chunks * bn > 512) continue;
+            const int chunk_kb = (kblocks + pieces - 1) / pieces;
+            const int64_t mt = (T + bm - 1) / bm, nt = (N + bn - 1) / bn, tiles = mt * nt * splits;
+            // cycles: a stage takes what its MMAs or its bytes (64 a cycle and SM) take, a round of tiles its first stage and its stores
+            const double stage = std::max(bm / 128 * std::max(bn, 96) * 2.0, (bm + bn) * 2.0), store = bm * bn / 32.0;
+            const double rounds = (double)((tiles + sms - 1) / sms);
+            double cost = rounds * (chunks * chunk_kb * stage + (bm / 128 * chunks * bn > 256 ? store : 0.0)) + store + 1500.0;
+            if (splits > 1) cost += 4000.0 + (double)splits * T * N * 8.0 / (32.0 * sms);
+            if (!BM || cost < best) {
+                best = cost;
+                BM = bm;
+                g.BN = bn, g.n_tiles = (int)nt, g.m_tiles = (int)mt, g.chunks = chunks, g.chunk_kb = chunk_kb, g.splits = splits;
+            }
+        }
+    static void *ws = nullptr;
+    static size_t ws_bytes = 0;
+    if (g.splits > 1) {
+        const size_t need = (size_t)g.splits * (size_t)T * (size_t)N * 4;
+        if (need > ws_bytes) {
+            if (ws) cudaFree(ws);
+            ws = nullptr, ws_bytes = 0;
+            GGB_CUDA(cudaMalloc(&ws, need));
+            ws_bytes = need;
+        }
+        g.ws = (float *)ws;
+    }
+    g.T = (int)T, g.N = (int)N, g.kblocks = kblocks, g.stages = stages_of(BM, g.BN);
+    g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc;
+    g.vec = g.ws || ((uintptr_t)c % 16 == 0 && ldc % 4 == 0);
+    g.wait_error = ggb_wait_error_flag();
+    const int rc = launch(w, N, K, a, T, BM, g, g.m_tiles * g.n_tiles * g.splits);
+    if (rc || g.splits == 1) return rc;
+    splits_add_kernel<<<(unsigned)((T * N / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(g.ws, g.splits, T, N, c, g.act_out, act, ldc);
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
+}
+
+// The grouped form: w = [n_exp][N][K], a / c rows in sorted-slot order, offsets[e] .. offsets[e + 1] the rows of expert e (device).  Row
+// tiles of 128: an expert of a portion has about that many rows (256 would be computed for nothing to a half).
+bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc) { return K % 64 == 0 && N % 32 == 0 && ldc % 8 == 0; }
+int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, float *c, void *c_act, int act, int64_t ldc) {
+    GGB_REQUIRE_INIT();
+    GGB_CHECK_ARG(((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
+    gemm_args g{};
+    const int BM = 128;
+    g.BN = N <= 64 ? 64 : N <= 128 ? 128 : 256;
+    g.T = (int)n_rows, g.N = (int)N, g.kblocks = (int)(K / BK), g.n_tiles = (int)((N + g.BN - 1) / g.BN);
+    g.chunks = 1, g.chunk_kb = g.kblocks, g.splits = 1, g.stages = stages_of(BM, g.BN);
+    g.m_ranges = offsets, g.n_groups = n_exp;
+    g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc, g.vec = (uintptr_t)c % 16 == 0;
+    g.wait_error = ggb_wait_error_flag();
+    const int64_t most = ((n_rows + BM - 1) / BM + n_exp) * g.n_tiles;
+    return launch(w, (int64_t)n_exp * N, K, a, n_rows, BM, g, (int)std::min<int64_t>(most, 1 << 20));
+}

@@ -108,11 +108,6 @@ struct GemmArgs {
     float *ws;         // K-split workspace [ksplit][T][N] or null (ksplit == 1: tiles go straight to seg.c)
     const float *resid; // [T][seg[0].ldc] or null (single segment, ksplit == 1)
     int kblocks_per_split; // 64-wide K blocks per split
-    // grouped form (mixture of experts, plain bf16 matrices): blockIdx.z = expert e, whose matrix is seg[0].qs + e * rows * K
-    // and whose rows of A / C are [m_ranges[e], m_ranges[e + 1]) (device int32); tiles past the range leave at once
-    const int32_t *m_ranges;
-    __nv_bfloat16 *act_out; // when set: C is stored as bf16 act(c) (GGB_ACT_*) with row pitch seg[0].ldc instead of fp32
-    int act;
 };
 
 // int8 / int4 code -> fp32 without the conversion pipe: the (biased) code is dropped into the mantissa of
@@ -165,16 +160,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16w_kernel(const GemmA
     const uint32_t bars = smem0 + kStages * kStageBytes;                // full[kStages], empty[kStages], tmem_full
     const uint32_t tmem_slot = bars + 8 * (2 * kStages + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int m_begin = 0, m_end = A.T, split = blockIdx.z;
-    size_t w_off = 0; // bytes from the segment's matrix to this CTA's matrix (grouped form)
-    if (A.m_ranges) {
-        m_begin = A.m_ranges[blockIdx.z];
-        m_end = A.m_ranges[blockIdx.z + 1];
-        split = 0;
-        w_off = (size_t)blockIdx.z * (size_t)A.seg[0].rows * (size_t)A.K * 2;
-    }
-    const int n0 = blockIdx.x * BN, m0 = m_begin + blockIdx.y * BM;
-    if (m0 >= m_end) return; // the whole CTA, before any barrier or tensor memory exists
+    const int m_end = A.T, split = blockIdx.z, n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
     int si = 0;
     if (A.n_seg > 1 && n0 >= A.seg[1].n_begin) si = (A.n_seg > 2 && n0 >= A.seg[2].n_begin) ? 2 : 1;
     const GemmSeg &sg = A.seg[si];
@@ -215,7 +201,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16w_kernel(const GemmA
         uint4 raw[kStages][PBW];
         __half dd[kStages];
         auto fetch = [&](int kb, uint4 (&r)[PBW], __half &d1) {
-            if (TYPE == GGB_TYPE_BF16 || !wlive || kb >= kb1) return;
+            if (!wlive || kb >= kb1) return;
             const size_t blk = (size_t)wrow * A.nb + (size_t)kb * 2 + whalf;
             d1 = sg.d[blk];
             const uint4 *src = reinterpret_cast<const uint4 *>(sg.qs + blk * (TYPE == GGB_TYPE_Q8_0 ? 32 : 16));
@@ -253,22 +239,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16w_kernel(const GemmA
                         }
                     }
                 }
-                // W tile.  Plain bf16 matrix: the same copy as the A tile (rows of the matrix are K-major already)
-                if (TYPE == GGB_TYPE_BF16) {
-                    const int ch = tid & 7;
-                    const __nv_bfloat16 *wm = reinterpret_cast<const __nv_bfloat16 *>(sg.qs + w_off);
-#pragma unroll
-                    for (int r = tid >> 3; r < BN; r += kProducerThreads / 8) {
-                        const int row = sn0 + r;
-                        const uint32_t dst = sb + r * 128 + ((ch ^ (r & 7)) << 4);
-                        if (row < sg.rows) {
-                            const void *src = reinterpret_cast<const uint4 *>(wm + (size_t)row * A.K + (size_t)kb * BK) + ch;
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-                        } else {
-                            sts_u4(dst, make_uint4(0, 0, 0, 0));
-                        }
-                    }
-                } else
                 // quantised matrix: convert the block requested kStages K blocks ago, then request block kb + kStages
                 {
                     uint4 cur[PBW];
@@ -324,18 +294,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16w_kernel(const GemmA
             for (int c0 = chalf * (BN / 4); c0 < (chalf + 1) * (BN / 4); c0 += 32) {
                 uint32_t v[32];
                 tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(mt * BN + c0), v);
-                if (row < m_end && sn0 + c0 < sg.rows && A.act_out && !A.ws) { // the next product's operand
-                    __nv_bfloat16 *dst = A.act_out + (size_t)row * sg.ldc + sn0 + c0;
-#pragma unroll
-                    for (int u = 0; u < 32; u += 8) {
-                        __align__(16) __nv_bfloat16 o[8];
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            o[q] = __float2bfloat16_rn(act_f32(__uint_as_float(v[u + q]), A.act));
-                        }
-                        *reinterpret_cast<uint4 *>(dst + u) = *reinterpret_cast<const uint4 *>(o);
-                    }
-                } else
                 if (row < m_end && sn0 + c0 < sg.rows) { // rows % 32 == 0
                     float *dst = cbase + (size_t)row * cld + c0;
                     const float *rs = A.resid ? A.resid + (size_t)row * sg.ldc + sn0 + c0 : nullptr;
@@ -404,8 +362,7 @@ __global__ void splitk_reduce_kernel(const GemmArgs A, int splits) {
     float acc = A.ws[i];
     for (int s = 1; s < splits; s++) acc += A.ws[(int64_t)s * T * N + i];
     if (A.resid) acc += A.resid[t * sg.ldc + col];
-    if (A.act_out) A.act_out[t * sg.ldc + col] = __float2bfloat16_rn(act_f32(acc, A.act));
-    else sg.c[t * sg.ldc + col] = acc;
+    sg.c[t * sg.ldc + col] = acc;
 }
 
 // rms_norm * w -> bf16 (the A operand of the next GEMM): same double-sum order as rms_norm_kernel (elementwise.cu)
@@ -767,18 +724,17 @@ int ggb_op_geglu_bf16(const float *gate, const float *up, int64_t n, void *y_bf1
 }
 
 static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, const int64_t *ldc,
-                       const float *resid, void *workspace, size_t workspace_bytes, void *act_out = nullptr, int act = 0) {
+                       const float *resid, void *workspace, size_t workspace_bytes) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(n >= 1 && n <= kMaxSegs && w && a_bf16 && c && ldc && T > 0, "bad gemm args");
-    GGB_CHECK_ARG(n == 1 || (!resid && !act_out), "gemm: a residual or an activation needs a single matrix");
-    GGB_CHECK_ARG(!act_out || (!resid && ldc[0] % 8 == 0), "gemm: an activation takes no residual and rows of whole 16-byte pieces");
+    GGB_CHECK_ARG(n == 1 || !resid, "gemm: a residual needs a single matrix");
     const int64_t K = w[0]->cols;
     const int type = w[0]->type;
-    GGB_CHECK_ARG(type == GGB_TYPE_Q4_0 || type == GGB_TYPE_Q8_0 || type == GGB_TYPE_BF16, "gemm: weight type %d", type);
+    GGB_CHECK_ARG(type == GGB_TYPE_Q4_0 || type == GGB_TYPE_Q8_0, "gemm: weight type %d", type);
     GemmArgs A{};
     int64_t N = 0;
     for (int i = 0; i < n; i++) {
-        GGB_CHECK_ARG(w[i] && (c[i] || act_out) && w[i]->cols == K && w[i]->type == type, "gemm: matrices of one launch share K and the type");
+        GGB_CHECK_ARG(w[i] && c[i] && w[i]->cols == K && w[i]->type == type, "gemm: matrices of one launch share K and the type");
         const int64_t rows = w[i]->rows;
         GGB_CHECK_ARG(K % 64 == 0 && rows % 32 == 0 && ldc[i] >= rows && ldc[i] % 4 == 0,
                       "gemm needs K %% 64 == 0, N %% 32 == 0 (N=%lld K=%lld)", (long long)rows, (long long)K);
@@ -790,7 +746,6 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     if (!attr_done) {
         GGB_CUDA(cudaFuncSetAttribute(gemm_bf16w_kernel<GGB_TYPE_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
         GGB_CUDA(cudaFuncSetAttribute(gemm_bf16w_kernel<GGB_TYPE_Q8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-        GGB_CUDA(cudaFuncSetAttribute(gemm_bf16w_kernel<GGB_TYPE_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
         attr_done = true;
     }
     const int n_tiles = (int)((N + BN - 1) / BN), m_tiles = (int)((T + BM - 1) / BM), kblocks = (int)(K / BK);
@@ -804,12 +759,9 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     A.kblocks_per_split = (kblocks + splits - 1) / splits;
     A.ws = splits > 1 ? (float *)workspace : nullptr;
     A.resid = resid;
-    A.act_out = (__nv_bfloat16 *)act_out;
-    A.act = act;
     const dim3 grid((unsigned)n_tiles, (unsigned)m_tiles, (unsigned)splits);
     if (splits > 1) A.resid = nullptr; // added by the reducer
     if (type == GGB_TYPE_Q4_0) gemm_bf16w_kernel<GGB_TYPE_Q4_0><<<grid, kGemmThreads, kGemmSmem, ggb_cuda_stream()>>>(A);
-    else if (type == GGB_TYPE_BF16) gemm_bf16w_kernel<GGB_TYPE_BF16><<<grid, kGemmThreads, kGemmSmem, ggb_cuda_stream()>>>(A);
     else gemm_bf16w_kernel<GGB_TYPE_Q8_0><<<grid, kGemmThreads, kGemmSmem, ggb_cuda_stream()>>>(A);
     GGB_LAUNCH_CHECK();
     if (splits > 1) {
@@ -870,59 +822,3 @@ int ggb_op_attn_prefill(const float *q, const void *kcache, const void *vcache, 
 }
 
 } // extern "C"
-
-// The grouped form for a mixture of experts: w = [n_exp][N][K] bf16, a / c rows in sorted-slot order, offsets[e] .. offsets[e+1]
-// the rows of expert e (device).  One launch: grid (N tiles, row tiles of the longest possible group, experts).
-bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc) { return K % 64 == 0 && N % 32 == 0 && ldc % 8 == 0; }
-int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, float *c,
-                          void *c_act, int act, int64_t ldc) {
-    GGB_REQUIRE_INIT();
-    static bool attr_done = false;
-    if (!attr_done) {
-        GGB_CUDA(cudaFuncSetAttribute(gemm_bf16w_kernel<GGB_TYPE_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-        attr_done = true;
-    }
-    GemmArgs A{};
-    A.seg[0] = GemmSeg{reinterpret_cast<const uint8_t *>(w), nullptr, c, (int)ldc, 0, (int)N};
-    A.n_seg = 1;
-    A.N = (int)N; A.K = (int)K; A.nb = (int)(K / 32);
-    A.a = (const __nv_bfloat16 *)a; A.T = (int)n_rows;
-    A.kblocks_per_split = (int)(K / BK);
-    A.m_ranges = offsets;
-    A.act_out = (__nv_bfloat16 *)c_act;
-    A.act = act;
-    const dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((n_rows + BM - 1) / BM), (unsigned)n_exp);
-    gemm_bf16w_kernel<GGB_TYPE_BF16><<<grid, kGemmThreads, kGemmSmem, ggb_cuda_stream()>>>(A);
-    GGB_LAUNCH_CHECK();
-    return GGB_OK;
-}
-
-// the GEMM on plain bf16 matrices (both operands copied by cp.async, nothing to dequantise): the matrix is described
-// as a ggb_weight of type BF16 whose payload plane is the matrix itself.  The K-split workspace belongs to the library
-// and only grows.
-bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc) {
-    return T >= 64 && K % 64 == 0 && N % 32 == 0 && ldc % 4 == 0 && N < (1ll << 31) && K < (1ll << 31) && T < (1ll << 31);
-}
-int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
-    GGB_REQUIRE_INIT();
-    static void *ws = nullptr;
-    static size_t ws_bytes = 0;
-    const int n_tiles = (int)((N + BN - 1) / BN), m_tiles = (int)((T + BM - 1) / BM);
-    if (n_tiles * m_tiles * 2 <= ggb_sm_count()) { // small enough to be split along K
-        const size_t need = ggb_gemm_workspace_bytes(T, N, K);
-        if (need > ws_bytes) {
-            if (ws) cudaFree(ws);
-            ws = nullptr, ws_bytes = 0;
-            GGB_CUDA(cudaMalloc(&ws, need));
-            ws_bytes = need;
-        }
-    }
-    ggb_weight wd{};
-    wd.type = GGB_TYPE_BF16;
-    wd.rows = N, wd.cols = K, wd.nb = K / 32;
-    wd.qs = reinterpret_cast<uint8_t *>(const_cast<void *>(w));
-    const ggb_weight *wp[1] = {&wd};
-    float *cs[1] = {c};
-    const int64_t ls[1] = {ldc};
-    return gemm_launch(1, wp, a, T, cs, ls, nullptr, ws, ws_bytes, c_act, act);
-}

@@ -9,6 +9,10 @@
 // matter of timing
 int *ggb_wait_error_flag();
 
+// a tensor map over a row-major bf16 matrix [rows][cols] with row pitch ld (numbers): boxes of 64 columns x box_rows, 128-byte swizzle
+struct CUtensorMap_st;
+int ggb_tensor_map_bf16(CUtensorMap_st *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows);
+
 #ifdef __CUDACC__
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -70,11 +74,19 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 
 #define GGB_R8(v, o) "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]), "=r"(v[o + 4]), "=r"(v[o + 5]), "=r"(v[o + 6]), "=r"(v[o + 7])
 #define GGB_S8(v, o) "r"(v[o]), "r"(v[o + 1]), "r"(v[o + 2]), "r"(v[o + 3]), "r"(v[o + 4]), "r"(v[o + 5]), "r"(v[o + 6]), "r"(v[o + 7])
-// 32 lanes x 16 (8) columns.  A load and the wait for it are one statement: no use of a register can move in front of it
+// 32 lanes x 16 (32, 8) columns.  A load and the wait for it are one statement: no use of a register can move in front of it
 __device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t *v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
                  "tcgen05.wait::ld.sync.aligned;"
                  : GGB_R8(v, 0), GGB_R8(v, 8)
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, "
+                 "%24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : GGB_R8(v, 0), GGB_R8(v, 8), GGB_R8(v, 16), GGB_R8(v, 24)
                  : "r"(taddr)
                  : "memory");
 }
@@ -94,6 +106,16 @@ __device__ __forceinline__ void tmem_alloc512(uint32_t slot) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_free512(uint32_t base) { asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory"); }
+
+// TMA: a box of a 2-dimensional tensor map, x (a multiple of 16 bytes) and y of its first element, to shared memory; out-of-range elements
+// arrive as zeros.  One thread.
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
