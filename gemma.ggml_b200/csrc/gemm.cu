@@ -52,6 +52,46 @@ struct tile_at {
     int m0, m_end, n0, split, group;
 };
 
+// a warp's 32 rows x 32 columns of accumulators, K pieces added in order, stored as whole lines
+__device__ __forceinline__ void store_piece(const gemm_args &a, uint32_t col, int chunks, uint32_t my, int lane, int row0, int m_end, int n0, int split) {
+    uint32_t v[32];
+    if (chunks > 0) tmem_load32(col, v);
+    else // no block of K is left for this CTA
+        for (int q = 0; q < 32; q++) v[q] = 0;
+    for (int ch = 1; ch < chunks; ch++) {
+        uint32_t u[32];
+        tmem_load32(col + ch * a.BN, u);
+#pragma unroll
+        for (int q = 0; q < 32; q++) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(u[q]));
+    }
+    // row = lane -> eight lanes a row: 16-byte piece p of row r at place p ^ (r & 7)
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 8; p++)
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(my + lane * 128 + ((p ^ (lane & 7)) << 4)), "r"(v[4 * p]), "r"(v[4 * p + 1]), "r"(v[4 * p + 2]),
+                     "r"(v[4 * p + 3])
+                     : "memory");
+    __syncwarp();
+    const int p = lane & 7, n = n0 + 4 * p;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int r = 4 * q + (lane >> 3), row = row0 + r;
+        float4 o;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(my + r * 128 + ((p ^ (r & 7)) << 4)) : "memory");
+        if (row >= m_end || n >= a.N) continue;
+        if (a.act_out && !a.ws) { // the next product's operand; N and ldc are multiples of 8
+            uint2 y;
+            y.x = pack_bf16x2(act_f32(o.x, a.act), act_f32(o.y, a.act));
+            y.y = pack_bf16x2(act_f32(o.z, a.act), act_f32(o.w, a.act));
+            *reinterpret_cast<uint2 *>(a.act_out + row * a.ldc + n) = y;
+        } else { // N is a multiple of 4
+            float *dst = a.ws ? a.ws + ((int64_t)split * a.T + row) * a.N + n : a.c + row * a.ldc + n;
+            if (a.vec) *reinterpret_cast<float4 *>(dst) = o;
+            else dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;
+        }
+    }
+}
+
 template <int BM>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
     extern __shared__ uint8_t gm_raw[];
@@ -207,43 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
                 if (row0 >= at.m_end) break;
                 for (int c0 = 32 * half; c0 < a.BN; c0 += 64) {
                     if (at.n0 + c0 >= a.N) break;
-                    uint32_t v[32];
-                    const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + mt * a.chunks * a.BN + c0;
-                    if (chunks > 0) tmem_load32(col, v);
-                    else // no block of K is left for this CTA
-                        for (int q = 0; q < 32; q++) v[q] = 0;
-                    for (int ch = 1; ch < chunks; ch++) {
-                        uint32_t u[32];
-                        tmem_load32(col + ch * a.BN, u);
-#pragma unroll
-                        for (int q = 0; q < 32; q++) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(u[q]));
-                    }
-                    // row = lane -> eight lanes a row: 16-byte piece p of row r at place p ^ (r & 7)
-                    __syncwarp();
-#pragma unroll
-                    for (int p = 0; p < 8; p++)
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(my + lane * 128 + ((p ^ (lane & 7)) << 4)), "r"(v[4 * p]), "r"(v[4 * p + 1]), "r"(v[4 * p + 2]),
-                                     "r"(v[4 * p + 3])
-                                     : "memory");
-                    __syncwarp();
-                    const int p = lane & 7, n = at.n0 + c0 + 4 * p;
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const int r = 4 * q + (lane >> 3), row = row0 + r;
-                        float4 o;
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(my + r * 128 + ((p ^ (r & 7)) << 4)) : "memory");
-                        if (row >= at.m_end || n >= a.N) continue;
-                        if (a.act_out && !a.ws) { // the next product's operand; N and ldc are multiples of 8
-                            uint2 y;
-                            y.x = pack_bf16x2(act_f32(o.x, a.act), act_f32(o.y, a.act));
-                            y.y = pack_bf16x2(act_f32(o.z, a.act), act_f32(o.w, a.act));
-                            *reinterpret_cast<uint2 *>(a.act_out + row * a.ldc + n) = y;
-                        } else { // N is a multiple of 4
-                            float *dst = a.ws ? a.ws + ((int64_t)at.split * a.T + row) * a.N + n : a.c + row * a.ldc + n;
-                            if (a.vec) *reinterpret_cast<float4 *>(dst) = o;
-                            else dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;
-                        }
-                    }
+                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + mt * a.chunks * a.BN + c0, chunks, my, lane, row0, at.m_end, at.n0 + c0, at.split);
                 }
             }
             tc_fence_before();
@@ -255,6 +259,129 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
     if (warp == 2) {
         tc_fence_after();
         tmem_free512(tmem);
+        if (lane == 0 && *dead) *a.wait_error = 1;
+    }
+}
+
+// Two CTAs a tile of MT x 256 rows and 256 columns: each holds MT x 128 rows of A and of the accumulators and half of W's rows.  A single CTA
+// reads A and W tiles of 12 KB from shared memory for an MMA of 128 cycles while TMA writes 64 bytes a cycle: 160 of the 128 bytes a cycle that
+// shared memory has; a pair needs 112.  2048 x 8192 x 4096: 104 us, 1320 TFLOP/s (107 us single, 131 us before either); 1024 x 32000 x 2048: 109 us
+// (125, 190 us).
+template <int MT>
+__global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
+    extern __shared__ uint8_t gm_raw[];
+    const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, turn = base + kRing, bars = turn + kTurn;
+    uint8_t *ctl = gm_raw + (bars - raw0);
+    volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t rank = cluster_rank(), bars0 = cluster_addr(bars, 0);
+    constexpr uint32_t a_bytes = MT * 16384, stage_bytes = a_bytes + 16384;
+    constexpr int kStages = (int)(kRing / stage_bytes);
+    const int n_acc = MT * a.chunks * 256 <= 256 ? 2 : 1;
+    if (tid == 0) {
+        for (int s = 0; s < kStages; s++) {
+            mbar_init(bars + FULL + 8 * s, 1);
+            mbar_init(bars + EMPTY + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(bars + ACC_FULL + 8 * s, 1);
+            mbar_init(bars + ACC_FREE + 8 * s, 16); // eight warps of each CTA
+        }
+        *dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) tmem_alloc512_pair(bars + SLOT);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
+    const int total = a.m_tiles * a.n_tiles * a.splits, pairs = gridDim.x / 2, me = blockIdx.x / 2;
+    // row tiles first: those that share a piece of W run together
+    auto locate = [&](int t, int &m0, int &n0, int &split) {
+        m0 = t % a.m_tiles * (MT * 256);
+        t /= a.m_tiles;
+        n0 = t % a.n_tiles * 256;
+        split = t / a.n_tiles;
+    };
+    auto k_range = [&](int split, int &kb0, int &kb1) {
+        kb0 = split * a.chunks * a.chunk_kb;
+        kb1 = min(kb0 + a.chunks * a.chunk_kb, a.kblocks);
+    };
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 0;
+            for (int t = me; t < total; t += pairs) {
+                int m0, n0, split, kb0, kb1;
+                locate(t, m0, n0, split);
+                k_range(split, kb0, kb1);
+                for (int kb = kb0; kb < kb1; kb++) {
+                    mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead);
+                    const uint32_t sa = base + s * stage_bytes;
+                    if (rank == 0) mbar_expect_tx(bars + FULL + 8 * s, 2 * stage_bytes);
+                    tma_load_2d_pair(sa, &map_a, kb * BK, m0 + (int)rank * MT * 128, bars0 + FULL + 8 * s);
+                    tma_load_2d_pair(sa + a_bytes, &map_w, kb * BK, n0 + (int)rank * 128, bars0 + FULL + 8 * s);
+                    if (++s == kStages) s = 0, ph ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1 && rank == 0) {
+        const uint32_t idesc = umma_idesc(256, 256);
+        int s = 0, it = 0;
+        uint32_t ph = 0;
+        for (int t = me; t < total; t += pairs, it++) {
+            int m0, n0, split, kb0, kb1, chunk = 0, left = a.chunk_kb;
+            locate(t, m0, n0, split);
+            k_range(split, kb0, kb1);
+            const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
+            mbar_wait_bounded(bars + ACC_FREE + 8 * buf, (use & 1) ^ 1, dead);
+            tc_fence_after();
+            for (int kb = kb0; kb < kb1; kb++) {
+                mbar_wait_bounded(bars + FULL + 8 * s, ph, dead);
+                tc_fence_after();
+                const uint32_t a_lo = umma_desc_lo(base + s * stage_bytes, 16), w_lo = umma_desc_lo(base + s * stage_bytes + a_bytes, 16);
+                const uint32_t first = left == a.chunk_kb ? 0u : 1u;
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    const uint32_t d = tmem + buf * 256 + (mt * a.chunks + chunk) * 256;
+#pragma unroll
+                    for (int k = 0; k < BK / 16; k++) umma_ss_pair(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, w_lo + 2 * k, idesc, k > 0 ? 1u : first);
+                }
+                umma_arrive_pair(bars + EMPTY + 8 * s);
+                if (++s == kStages) s = 0, ph ^= 1u;
+                if (--left == 0) chunk++, left = a.chunk_kb;
+            }
+            umma_arrive_pair(bars + ACC_FULL + 8 * buf);
+        }
+    } else if (warp >= 4) {
+        const int w8 = warp - 4, lq = warp & 3, half = w8 >> 2;
+        int it = 0;
+        for (int t = me; t < total; t += pairs, it++) {
+            int m0, n0, split, kb0, kb1;
+            locate(t, m0, n0, split);
+            k_range(split, kb0, kb1);
+            const int chunks = kb1 > kb0 ? (kb1 - kb0 + a.chunk_kb - 1) / a.chunk_kb : 0;
+            const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
+            mbar_wait_bounded(bars + ACC_FULL + 8 * buf, use & 1, dead);
+            tc_fence_after();
+            for (int mt = 0; mt < MT; mt++) {
+                const int row0 = m0 + ((int)rank * MT + mt) * 128 + lq * 32;
+                if (row0 >= a.T) break;
+                for (int c0 = 32 * half; c0 < 256 && n0 + c0 < a.N; c0 += 64)
+                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + mt * a.chunks * 256 + c0, chunks, turn + w8 * 4096, lane, row0, a.T, n0 + c0, split);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(bars0 + ACC_FREE + 8 * buf);
+        }
+    }
+    __syncthreads();
+    cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
+    if (warp == 2) {
+        tc_fence_after();
+        tmem_free512_pair(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;
     }
 }
@@ -278,13 +405,47 @@ __global__ void splits_add_kernel(const float *__restrict__ ws, int splits, int6
     }
 }
 
+int allow_smem() { // once a process: a call's host time is launch and tensor maps
+    static const cudaError_t e = [] {
+        cudaError_t r = cudaSuccess;
+        for (auto k : {gemm_tma_kernel<256>, gemm_tma_kernel<128>, gemm_pair_kernel<2>, gemm_pair_kernel<1>}) {
+            const cudaError_t x = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+            if (x != cudaSuccess) r = x;
+        }
+        return r;
+    }();
+    GGB_CUDA(e);
+    return GGB_OK;
+}
+
+int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int MT, const gemm_args &g, int pairs) {
+    CUtensorMap ma, mw;
+    int rc = allow_smem();
+    if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, MT * 128);
+    if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, 128);
+    if (rc) return rc;
+    auto kfn = MT == 2 ? gemm_pair_kernel<2> : gemm_pair_kernel<1>;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(2 * std::min(pairs, ggb_sm_count() / 2)));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = ggb_cuda_stream();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+    cfg.attrs = at, cfg.numAttrs = 1;
+    GGB_CUDA(cudaLaunchKernelEx(&cfg, kfn, ma, mw, g));
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
+}
+
 int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int BM, const gemm_args &g, int ctas) {
     CUtensorMap ma, mw;
-    int rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
+    int rc = allow_smem();
+    if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
     auto kfn = BM == 256 ? gemm_tma_kernel<256> : gemm_tma_kernel<128>;
-    GGB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
     kfn<<<std::min(ctas, ggb_sm_count()), kThreads, kSmem, ggb_cuda_stream()>>>(ma, mw, g);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -294,7 +455,8 @@ int stages_of(int BM, int BN) { return std::min<int>(kMaxStages, (int)(kRing / (
 
 } // namespace
 
-int ggb_tensor_map_bf16(CUtensorMap_st *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+static int tensor_map_2d(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void *base, int64_t rows, int64_t cols, int64_t pitch_bytes, int box_cols,
+                         int box_rows) {
     typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static encode_fn encode = nullptr;
@@ -305,12 +467,18 @@ int ggb_tensor_map_bf16(CUtensorMap_st *map, const void *base, int64_t rows, int
         GGB_CHECK_ARG(fn && qr == cudaDriverEntryPointSuccess, "cuTensorMapEncodeTiled is not in the driver");
         encode = (encode_fn)fn;
     }
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, pitch[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, step[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, pitch, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    GGB_CHECK_ARG(r == CUDA_SUCCESS, "tensor map of %lld x %lld numbers, pitch %lld: error %d", (long long)rows, (long long)cols, (long long)ld, (int)r);
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, pitch[1] = {(cuuint64_t)pitch_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, step[2] = {1, 1};
+    const CUresult r = encode(map, type, 2, const_cast<void *>(base), dims, pitch, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    GGB_CHECK_ARG(r == CUDA_SUCCESS, "tensor map of %lld x %lld numbers, pitch %lld bytes: error %d", (long long)rows, (long long)cols, (long long)pitch_bytes, (int)r);
     return GGB_OK;
+}
+int ggb_tensor_map_bf16(CUtensorMap_st *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+    return tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, base, rows, cols, ld * 2, 64, box_rows);
+}
+int ggb_tensor_map_bytes(CUtensorMap_st *map, const void *base, int64_t rows, int64_t row_bytes, int box_bytes, int box_rows) {
+    return tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_NONE, base, rows, row_bytes, row_bytes, box_bytes, box_rows);
 }
 
 bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc) {
@@ -328,23 +496,28 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
     while (pieces < 8 && big * pieces * 2 <= sms && kblocks / (pieces * 2) >= 4) pieces *= 2;
     gemm_args g{};
     double best = 0.0;
-    int BM = 0;
-    static const int shapes[4][2] = {{256, 256}, {128, 256}, {128, 128}, {128, 64}};
+    int BM = 0, pair = 0; // rows of a CTA; two CTAs a tile
+    static const struct {
+        int bm, bn, pair;
+    } shapes[] = {{256, 256, 1}, {128, 256, 1}, {256, 256, 0}, {128, 256, 0}, {128, 128, 0}, {128, 64, 0}};
     for (const auto &sh : shapes)
         for (int splits = 1; splits <= pieces; splits *= 2) {
-            const int chunks = pieces / splits, bm = sh[0], bn = sh[1];
-            if (bm / 128 * chunks * bn > 512) continue;
-            const int chunk_kb = (kblocks + pieces - 1) / pieces;
-            const int64_t mt = (T + bm - 1) / bm, nt = (N + bn - 1) / bn, tiles = mt * nt * splits;
-            // cycles: a stage takes what its MMAs or its bytes (64 a cycle and SM) take, a round of tiles its first stage and its stores
-            const double stage = std::max(bm / 128 * std::max(bn, 96) * 2.0, (bm + bn) * 2.0), store = bm * bn / 32.0;
-            const double rounds = (double)((tiles + sms - 1) / sms);
-            double cost = rounds * (chunks * chunk_kb * stage + (bm / 128 * chunks * bn > 256 ? store : 0.0)) + store + 1500.0;
-            if (splits > 1) cost += 4000.0 + (double)splits * T * N * 8.0 / (32.0 * sms);
+            const int chunks = pieces / splits, mt = sh.bm / 128;
+            if (mt * chunks * sh.bn > 512) continue;
+            const int chunk_kb = (kblocks + pieces - 1) / pieces, rows = sh.bm * (1 + sh.pair), cs = 1 + sh.pair;
+            const int64_t m_tiles = (T + rows - 1) / rows, n_tiles = (N + sh.bn - 1) / sh.bn, tiles = m_tiles * n_tiles * splits;
+            // cycles of a stage: its MMAs, or the bytes that pass through shared memory at 128 a cycle (written by TMA, read for the MMAs); a round of
+            // tiles: its stages and, unless the next tile runs meanwhile, its stores
+            const double mma = mt * std::max(sh.bn, 96) * 2.0, smem = ((sh.bm + sh.bn / cs) * 128.0 + mt * 4 * (4096.0 + sh.bn * 32.0 / cs)) / 128.0;
+            const double stage = std::max(mma, smem), store = sh.bm * sh.bn / 12.0;
+            const double rounds = (double)((tiles + sms / cs - 1) / (sms / cs));
+            double cost = rounds * (chunks * chunk_kb * stage + (mt * chunks * sh.bn > 256 ? store : 0.0)) + store + 2000.0;
+            if (splits > 1) cost += 12000.0 + (double)splits * T * N * 8.0 / (32.0 * sms); // another launch, the sums' way through memory
+            cost += sh.pair ? 4000.0 : 0.0;                                               // a cluster's launch
             if (!BM || cost < best) {
                 best = cost;
-                BM = bm;
-                g.BN = bn, g.n_tiles = (int)nt, g.m_tiles = (int)mt, g.chunks = chunks, g.chunk_kb = chunk_kb, g.splits = splits;
+                BM = sh.bm, pair = sh.pair;
+                g.BN = sh.bn, g.n_tiles = (int)n_tiles, g.m_tiles = (int)m_tiles, g.chunks = chunks, g.chunk_kb = chunk_kb, g.splits = splits;
             }
         }
     static void *ws = nullptr;
@@ -363,7 +536,7 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
     g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc;
     g.vec = g.ws || ((uintptr_t)c % 16 == 0 && ldc % 4 == 0);
     g.wait_error = ggb_wait_error_flag();
-    const int rc = launch(w, N, K, a, T, BM, g, g.m_tiles * g.n_tiles * g.splits);
+    const int tiles = g.m_tiles * g.n_tiles * g.splits, rc = pair ? launch_pair(w, N, K, a, T, BM / 128, g, tiles) : launch(w, N, K, a, T, BM, g, tiles);
     if (rc || g.splits == 1) return rc;
     splits_add_kernel<<<(unsigned)((T * N / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(g.ws, g.splits, T, N, c, g.act_out, act, ldc);
     GGB_LAUNCH_CHECK();

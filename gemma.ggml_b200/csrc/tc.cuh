@@ -12,6 +12,8 @@ int *ggb_wait_error_flag();
 // a tensor map over a row-major bf16 matrix [rows][cols] with row pitch ld (numbers): boxes of 64 columns x box_rows, 128-byte swizzle
 struct CUtensorMap_st;
 int ggb_tensor_map_bf16(CUtensorMap_st *map, const void *base, int64_t rows, int64_t cols, int64_t ld, int box_rows);
+// over rows of bytes: boxes of box_bytes x box_rows, as they lie
+int ggb_tensor_map_bytes(CUtensorMap_st *map, const void *base, int64_t rows, int64_t row_bytes, int box_bytes, int box_rows);
 
 #ifdef __CUDACC__
 
@@ -20,9 +22,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) { // (cluster scope: the arrivals may come from another CTA)
     uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
 // Waits for a phase.  Every wait ends: after kWaitTries tries (seconds) the CTA's `dead` word is set, which ends all of its other
@@ -66,7 +68,42 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32
 __device__ __forceinline__ void umma_arrive(uint32_t bar) { // arrives when all MMAs issued so far are done
     asm volatile("{\n.reg .pred e;\n" GGB_ELECT "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar) : "memory");
 }
+
+// Two CTAs of a cluster on one tile (cta_group::2): M = 256, the rows of A and of the accumulators half in each CTA, the rows of B (columns of
+// the tile) half in each CTA's shared memory at the same offsets.  The CTA of rank 0 issues; a commit arrives on both CTAs' barriers.
+__device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p, e;\n.reg .b64 a, b;\n" GGB_ELECT "setp.ne.b32 p, %4, 0;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n"
+                 "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+                 "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi)
+                 : "memory");
+}
+__device__ __forceinline__ void umma_arrive_pair(uint32_t bar) {
+    asm volatile("{\n.reg .pred e;\n" GGB_ELECT "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n" ::"r"(bar),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
 #undef GGB_ELECT
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t smem, uint32_t rank) { // the same offset in another CTA's shared memory
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc512_pair(uint32_t slot) { // one warp of each CTA
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free512_pair(uint32_t base) { asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -114,6 +151,13 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+
+// the same from a CTA of a pair, whose bytes count on the barrier of the CTA of rank 0 (a cluster address)
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void *map, int x, int y, uint32_t cluster_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y),
+                 "r"(cluster_bar)
                  : "memory");
 }
 
