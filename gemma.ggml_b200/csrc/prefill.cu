@@ -5,109 +5,71 @@
 //
 //   C[T][N] (fp32) = A[T][K] (bf16 activations) x dequant(W[N][K] Q4_0 | Q8_0)^T       (+ residual)
 //
-// One CTA computes a 256 x 256 tile of C.  Per 64-wide K block
-//   * warps 0-15 (PRODUCERS) copy the A tile (bf16, L2) and DEQUANTISE the W tile (int8/int4 codes x fp16 block
-//     scale -> bf16, exact product rounded once) into shared memory in the canonical K-major 128-byte-swizzled
-//     UMMA layout, fence the async proxy and arrive on the stage's mbarrier;
-//   * one lane of warp 16 (MMA ISSUER) waits for the stage and issues 2 x 4 tcgen05.mma (M = 128, N = 256,
-//     K = 16, kind::f16, bf16 x bf16 -> fp32) whose accumulators live in TENSOR MEMORY (2 x 256 columns =
-//     all 512), then tcgen05.commit releases the stage;
-//   * after the last K block the producer warps become the EPILOGUE: tcgen05.ld 32 lanes x 32 columns at a
-//     time, add the residual, store fp32.
-// Small-N matrices (o-proj, down-proj: 16 tiles) are split along K so that every SM has a tile; the partial
-// tiles go to a workspace and are reduced in split order by a second kernel (deterministic).
+// More than 128 rows: two CTAs of a cluster compute a tile (cta_group::2) of 512 or 256 rows x up to 256 columns; each holds half of the
+// rows of A and dequantises half of the tile's weight rows, so a prompt of 512 tokens dequantises every weight once.  Fewer rows: one
+// CTA, 128 rows x up to 128 columns.  Per 64-wide K block
+//   * one thread requests the CTA's A rows by TMA, another one the raw codes (a ring of their own: they are needed a dequantisation earlier);
+//   * two groups of eight warps take the K blocks alternately and DEQUANTISE the W rows (int8 / int4 codes x fp16 block scale -> bf16, exact
+//     product rounded once) from shared memory into shared memory, canonical K-major 128-byte-swizzled UMMA layout;
+//   * one warp (of the pair's first CTA) issues the tcgen05.mma (K = 16, kind::f16, bf16 x bf16 -> fp32) whose accumulators live in TENSOR
+//     MEMORY, up to all 512 columns; tcgen05.commit releases the buffers of both CTAs;
+//   * after the last K block the sixteen warps become the EPILOGUE: 32 x 32 pieces turned in shared memory, residual added, whole lines stored.
+//     gate | up of a feed-forward: each CTA dequantises rows of one of the two matrices, so both products of an output stand in the same row
+//     of tensor memory and leave as gelu(gate) * up in bf16.
+// A product along a long K is summed in pieces of K (as many as a split over the SMs in 256 x 256 tiles needs): several accumulators a
+// CTA in tensor memory, added in order by the epilogue, and, where SMs are left, several CTAs whose sums meet in a workspace and are
+// added in order by a second kernel (deterministic).
+//
+// What bounds it: shared memory (128 bytes a cycle).  A K block of a pair's CTA (256 rows, 128 weight rows) moves 40 KB in by TMA, 8 KB of codes
+// out, 16 KB of weights in and 64 to 96 KB out for the MMAs: 1550 cycles where the MMAs alone take 1024; the weights of a block stand half a
+// block before its MMAs.  512 tokens, Q8_0: gate | up with gelu 81 us, 848 TFLOP/s (115 us in two launches before), 2048 x 16384 60 us (85 us
+// with its reduction), 2048 x 2048 27 us.
 //
 // Numerics: weights q*d are exact in fp32 (8 x 11 bits) and rounded once to bf16; activations are rounded
 // to bf16 instead of being re-quantised to Q8_0 per 32 (the reference's INIT stage), so prefill agrees with
 // the reference within a tolerance (tests/test_prefill_gpu.py), not bit for bit — the decode path is the
 // bit-exact one.
+#include <cuda.h>
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "tc.cuh"
 
 namespace {
 
-constexpr int BM = 256, BN = 256, BK = 64;
-constexpr int kStages = 3;
-constexpr int kAStage = BM * BK * 2, kBStage = BN * BK * 2; // 32 KB each
-constexpr int kStageBytes = kAStage + kBStage;
-constexpr int kProducerWarps = 16, kProducerThreads = 512;
-constexpr int kGemmThreads = kProducerThreads + 32;
-constexpr int kTmemCols = 512;
-constexpr size_t kGemmSmem = (size_t)kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int BK = 64;
+constexpr int kWorkWarps = 16, kGroupWarps = 8, kTmaWarp = 16, kMmaWarp = 17, kCodesWarp = 18, kGemmThreads = 32 * 19;
+constexpr uint32_t kRing = 224 * 1024;
+constexpr int kMaxStages = 6;
+constexpr size_t kGemmSmem = 1024 + kRing + 384;
+constexpr int kTiles = 2, kCodeStages = 4; // buffers of dequantised weights, of codes
+enum { A_FULL = 0, A_FREE = 48, B_FULL = 96, B_FREE = 128, PEER_FULL = 160, C_FULL = 192, C_FREE = 240, DONE = 288, SLOT = 296, DEAD = 304 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
-    asm volatile(
-        "{\n.reg .pred p;\nWAIT_LOOP:\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n"
-        "@p bra WAIT_DONE;\nbra WAIT_LOOP;\nWAIT_DONE:\n}\n" ::"r"(bar), "r"(parity) : "memory");
-}
-
-// UMMA shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows of 64 bf16 (128 B), 8-row
-// atoms of 1024 B (stride-dimension byte offset), descriptor version 1 (sm_100), layout type 2.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);       // start address, 16-byte units
-    d |= (uint64_t)1 << 16;                          // leading-dimension byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024u >> 4) << 32;               // stride-dimension byte offset: 8 rows x 128 B
-    d |= (uint64_t)1 << 46;                          // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                          // SWIZZLE_128B
-    return d;
-}
-// instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major, M = 128, N = 256
-__device__ __forceinline__ uint32_t umma_idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc),
-        "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) { // arrives on the mbarrier when all prior MMAs are done
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// up to 3 weight matrices that share the A operand run as ONE launch (Q | K | V, gate | up): a segment = one matrix,
-// its first row is a multiple of the tile height, so a tile belongs to exactly one segment
+// up to 3 weight matrices that share the A operand run as ONE launch (Q | K | V, gate | up): a segment = one matrix, its first row is a
+// multiple of 256, so a tile belongs to exactly one segment
 constexpr int kMaxSegs = 3;
 struct GemmSeg {
-    const uint8_t *qs; // weight payload plane [rows][nb][16|32]
-    const __half *d;   // weight scale plane [rows][nb]
-    float *c;          // [T][ldc] output of this matrix
+    const __half *d;     // weight scale plane [rows][nb]
+    float *c;            // [T][ldc] output of this matrix
     int ldc;
-    int n_begin, rows; // first row of the segment in the concatenated N, its row count
+    int n_begin, rows;   // first row of the segment in the concatenated N, its row count
 };
 struct GemmArgs {
     GemmSeg seg[kMaxSegs];
     int n_seg;
-    int N, K, nb;      // N = concatenated rows (tile-padded between segments), nb = K / 32
-    const __nv_bfloat16 *a; // [T][K]
-    int T;
-    float *ws;         // K-split workspace [ksplit][T][N] or null (ksplit == 1: tiles go straight to seg.c)
-    const float *resid; // [T][seg[0].ldc] or null (single segment, ksplit == 1)
-    int kblocks_per_split; // 64-wide K blocks per split
+    int N, nb, kblocks;  // N = concatenated rows (padded between segments), nb = K / 32, kblocks = K / 64
+    int T, MT, BN;       // a CTA's rows: MT x 128; a tile's columns
+    int chunks, chunk_kb, stages; // stages of A rows
+    float *ws;           // workspace [splits][T][N] or null (one CTA along K: tiles go straight to seg.c)
+    const float *resid;  // [T][seg[0].ldc] or null (single segment, no workspace)
+    __nv_bfloat16 *geglu; // two segments, gate and up, of which every tile takes BN / 2 rows each: [T][rows] gelu(gate) * up
+    int *wait_error;
+};
+struct GemmMaps {
+    CUtensorMap a, w[kMaxSegs];
 };
 
 // int8 / int4 code -> fp32 without the conversion pipe: the (biased) code is dropped into the mantissa of
@@ -152,217 +114,264 @@ __device__ __forceinline__ void dequant32_q4(const uint4 w, float d, uint4 (&o)[
 __device__ __forceinline__ void sts_u4(uint32_t addr, const uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+__device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
 
-template <int TYPE>
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16w_kernel(const GemmArgs A) {
+// gelu of an fp16 number, rounded to fp16, as the reference's table has it
+__device__ __forceinline__ float gelu_f16(float g) {
+    const float x = __half2float(__float2half_rn(g));
+    return __half2float(__float2half_rn(0.5f * x * (1.0f + tanhf(0.79788456080286535587989211986876f * x * (1.0f + 0.044715f * x * x)))));
+}
+
+template <int TYPE, bool PAIR>
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs A) {
     extern __shared__ uint8_t gemm_smem_raw[];
-    const uint32_t smem0 = (smem_u32(gemm_smem_raw) + 1023u) & ~1023u; // SWIZZLE_128B atoms need 1024-byte alignment
-    const uint32_t bars = smem0 + kStages * kStageBytes;                // full[kStages], empty[kStages], tmem_full
-    const uint32_t tmem_slot = bars + 8 * (2 * kStages + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m_end = A.T, split = blockIdx.z, n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
+    constexpr int PB = TYPE == GGB_TYPE_Q8_0 ? 32 : 16; // payload bytes of a block of 32 weights
+    const uint32_t raw0 = smem_u32(gemm_smem_raw), smem0 = (raw0 + 1023u) & ~1023u, bars = smem0 + kRing;
+    uint8_t *gbase = gemm_smem_raw + (smem0 - raw0);
+    volatile int *dead = reinterpret_cast<volatile int *>(gbase + kRing + DEAD);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int rank = PAIR ? (int)cluster_rank() : 0, CTAS = PAIR ? 2 : 1;
+    const int n0 = blockIdx.y * A.BN, m0 = (PAIR ? blockIdx.x / 2 * 2 + rank : blockIdx.x) * A.MT * 128, split = blockIdx.z, BR = A.BN / CTAS;
     int si = 0;
-    if (A.n_seg > 1 && n0 >= A.seg[1].n_begin) si = (A.n_seg > 2 && n0 >= A.seg[2].n_begin) ? 2 : 1;
+    if (A.geglu) si = rank;
+    else if (A.n_seg > 1 && n0 >= A.seg[1].n_begin) si = (A.n_seg > 2 && n0 >= A.seg[2].n_begin) ? 2 : 1;
     const GemmSeg &sg = A.seg[si];
-    const int sn0 = n0 - sg.n_begin; // first row of this tile inside its matrix
-    const int kb0 = split * A.kblocks_per_split;
-    const int kb1 = min(kb0 + A.kblocks_per_split, (A.K + BK - 1) / BK);
+    const int sn0 = A.geglu ? n0 / 2 : n0 - sg.n_begin; // first row of this tile inside its matrix
+    const int w_row0 = A.geglu ? sn0 : sn0 + rank * BR; // first weight row of this CTA
+    const int kb0 = split * A.chunks * A.chunk_kb, kb1 = min(kb0 + A.chunks * A.chunk_kb, A.kblocks);
+    if (sn0 >= sg.rows) return; // padding between matrices: all CTAs of the tile, before any barrier or tensor memory exists
+    const uint32_t b_bytes = (uint32_t)BR * 128, a_bytes = (uint32_t)A.MT * 16384, c_bytes = (uint32_t)BR * 2 * PB;
+    const uint32_t codes = smem0 + kTiles * b_bytes, ring = codes + kCodeStages * c_bytes; // dequantised tiles | codes | A rows
 
     if (tid == 0) {
-        for (int s = 0; s < kStages; s++) {
-            mbar_init(bars + 8 * s, kProducerWarps);        // full: one arrive per producer warp
-            mbar_init(bars + 8 * (kStages + s), 1);          // empty: tcgen05.commit
+        for (int s = 0; s < A.stages; s++) {
+            mbar_init(bars + A_FULL + 8 * s, 1);
+            mbar_init(bars + A_FREE + 8 * s, 1);
         }
-        mbar_init(bars + 8 * 2 * kStages, 1);                // accumulators complete
+        for (int s = 0; s < kCodeStages; s++) {
+            mbar_init(bars + C_FULL + 8 * s, 1);
+            mbar_init(bars + C_FREE + 8 * s, kGroupWarps);
+        }
+        for (int s = 0; s < kTiles; s++) {
+            mbar_init(bars + B_FULL + 8 * s, kGroupWarps);
+            mbar_init(bars + B_FREE + 8 * s, 1);
+            mbar_init(bars + PEER_FULL + 8 * s, 1);
+        }
+        mbar_init(bars + DONE, 1);
+        *dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kProducerWarps) { // the MMA warp owns tensor memory
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "n"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (warp == kMmaWarp) {
+        if (PAIR) tmem_alloc512_pair(bars + SLOT);
+        else tmem_alloc512(bars + SLOT);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    tc_fence_before();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t tmem_base;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+    if (PAIR) cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(gbase + kRing + SLOT), 0);
 
-    if (warp < kProducerWarps) {
-        // ================= producers: thread t owns weight row n0 + t of the tile (64 weights per K block) and
-        // 8 of the 2048 16-byte chunks of the A tile.  The raw codes of the NEXT K block are requested before the
-        // current one is converted (register double buffer), and the A tile travels with cp.async, so the
-        // memory latency of both operands overlaps the dequantisation arithmetic.
-        // thread t owns ONE quant block (32 weights) per K block: row n0 + (t >> 1), block 2 kb + (t & 1)
-        const int wr = tid >> 1, whalf = tid & 1;
-        const int wrow = sn0 + wr;
-        const bool wlive = wrow < sg.rows;
-        constexpr int PBW = TYPE == GGB_TYPE_Q8_0 ? 2 : 1; // 16-byte payload words per quant block
-        // register ring of raw codes, kStages K blocks deep: HBM latency under load (~2000 cycles) is longer
-        // than one K block of MMA time, so the codes are requested kStages blocks before they are converted
-        uint4 raw[kStages][PBW];
-        __half dd[kStages];
-        auto fetch = [&](int kb, uint4 (&r)[PBW], __half &d1) {
-            if (!wlive || kb >= kb1) return;
-            const size_t blk = (size_t)wrow * A.nb + (size_t)kb * 2 + whalf;
-            d1 = sg.d[blk];
-            const uint4 *src = reinterpret_cast<const uint4 *>(sg.qs + blk * (TYPE == GGB_TYPE_Q8_0 ? 32 : 16));
+    if (warp < kWorkWarps) {
+        // ================= a group takes every other K block; thread t of it owns ONE quant block (32 weights): row w_row0 + (t >> 1), block 2 kb + (t & 1)
+        const int grp = warp / kGroupWarps, gt = tid & (32 * kGroupWarps - 1), wr = gt >> 1, whalf = gt & 1, wrow = w_row0 + wr;
+        const bool mine = wr < BR, live = mine && wrow < sg.rows;
+        const __half *dp = sg.d + (size_t)wrow * A.nb + whalf;
+        __half cur[4], nxt[4]; // scales of the group's next four K blocks, requested while the four before are used
+        auto scales = [&](int kb, __half (&d)[4]) {
 #pragma unroll
-            for (int j = 0; j < PBW; j++) r[j] = __ldg(src + j);
+            for (int u = 0; u < 4; u++) d[u] = live && kb + 2 * u < kb1 ? __ldg(dp + 2 * (kb + 2 * u)) : __float2half(0.f);
         };
+        scales(kb0 + grp, nxt);
+        uint32_t use = 0; // the group's K blocks so far
+        int s = grp;
+        uint32_t ph = 0;
+        for (int kbase = kb0 + grp; kbase < kb1; kbase += 8) {
 #pragma unroll
-        for (int u = 0; u < kStages; u++) {
-            dd[u] = __float2half(0.f);
+            for (int u = 0; u < 4; u++) cur[u] = nxt[u];
+            scales(kbase + 8, nxt);
 #pragma unroll
-            for (int j = 0; j < PBW; j++) raw[u][j] = make_uint4(0, 0, 0, 0);
-            fetch(kb0 + u, raw[u], dd[u]);
-        }
-        uint32_t parity = 0;
-        for (int kbase = kb0; kbase < kb1; kbase += kStages, parity ^= 1u) {
-#pragma unroll
-            for (int u = 0; u < kStages; u++) { // stage == u: the K loop is unrolled by the ring depth
-                const int kb = kbase + u;
-                if (kb >= kb1) break;
-                const int stage = u;
-                mbar_wait(bars + 8 * (kStages + stage), parity ^ 1u);
-                const uint32_t sa = smem0 + stage * kStageBytes, sb = sa + kAStage;
-                // A tile: 256 rows x 128 B; 8 threads per row (16-byte chunks), 64 rows per sweep
-                {
-                    const int ch = tid & 7;
-#pragma unroll
-                    for (int r = tid >> 3; r < BM; r += kProducerThreads / 8) {
-                        const int row = m0 + r;
-                        const uint32_t dst = sa + r * 128 + ((ch ^ (r & 7)) << 4);
-                        if (row < m_end) {
-                            const void *src = reinterpret_cast<const uint4 *>(A.a + (size_t)row * A.K + (size_t)kb * BK) + ch;
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-                        } else {
-                            sts_u4(dst, make_uint4(0, 0, 0, 0));
-                        }
-                    }
-                }
-                // quantised matrix: convert the block requested kStages K blocks ago, then request block kb + kStages
-                {
-                    uint4 cur[PBW];
-#pragma unroll
-                    for (int j = 0; j < PBW; j++) cur[j] = raw[u][j];
-                    const float d0 = __half2float(dd[u]);
-                    fetch(kb + kStages, raw[u], dd[u]);
-                    const uint32_t dst = sb + wr * 128;
-                    const int sw = wr & 7, c0 = 4 * whalf; // this block's four 16-byte chunks of the 128-byte row
-                    uint4 o[4];
-                    if (wlive) {
-                        if (TYPE == GGB_TYPE_Q8_0) {
-                            dequant16_q8(cur[0], d0, o[0], o[1]);
-                            dequant16_q8(cur[PBW - 1], d0, o[2], o[3]);
-                        } else {
-                            dequant32_q4(cur[0], d0, o);
-                        }
+            for (int u = 0; u < 4; u++) {
+                if (kbase + 2 * u >= kb1) break;
+                mbar_wait_bounded(bars + C_FULL + 8 * s, ph, dead);
+                uint4 o[4];
+                if (mine) { // rows past the matrix: zero codes (TMA) and zero scales
+                    const float d0 = __half2float(cur[u]);
+                    const uint32_t src = codes + s * c_bytes + gt * PB;
+                    if (TYPE == GGB_TYPE_Q8_0) {
+                        // the two 16-byte pieces in an order in which eight lanes meet eight groups of banks
+                        const uint32_t first = (lane >> 2) & 1;
+                        const uint4 x = lds_u4(src + 16 * first), y = lds_u4(src + 16 * (first ^ 1));
+                        dequant16_q8(first ? y : x, d0, o[0], o[1]);
+                        dequant16_q8(first ? x : y, d0, o[2], o[3]);
                     } else {
-#pragma unroll
-                        for (int q = 0; q < 4; q++) o[q] = make_uint4(0, 0, 0, 0);
+                        dequant32_q4(lds_u4(src), d0, o);
                     }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bars + C_FREE + 8 * s); // the codes are in registers
+                constexpr uint32_t kOwn = kTiles / 2;
+                const uint32_t b = grp + 2 * (use % kOwn);
+                if (use >= kOwn) mbar_wait_bounded(bars + B_FREE + 8 * b, (use / kOwn - 1) & 1, dead);
+                if (mine) {
+                    const uint32_t dst = smem0 + b * b_bytes + wr * 128;
 #pragma unroll
-                    for (int q = 0; q < 4; q++) sts_u4(dst + (((c0 + q) ^ sw) << 4), o[q]);
+                    for (int q = 0; q < 4; q++) sts_u4(dst + (((4 * whalf + q) ^ (wr & 7)) << 4), o[q]);
                 }
-                // The A copies of THIS block stay in flight (one L2 round trip) while the next block is converted:
-                // wait only for the previous block's group, then hand the PREVIOUS stage over.  generic-proxy /
-                // cp.async writes -> visible to the tensor core (async proxy) -> arrive.
-                asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
-                if (kb > kb0) {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bars + 8 * (stage == 0 ? kStages - 1 : stage - 1));
-                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bars + B_FULL + 8 * b);
+                use++;
+                s += 2;
+                if (s >= kCodeStages) s -= kCodeStages, ph ^= 1u;
             }
         }
-        if (kb0 < kb1) { // last stage
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bars + 8 * ((kb1 - kb0 - 1) % kStages));
-        }
-        // ================= epilogue: warp w reads TMEM lanes 32w .. 32w+31 (accumulator rows)
-        mbar_wait(bars + 8 * 2 * kStages, 0);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // straight to the matrix's output, or (K-split) into this split's [T][N] plane of the workspace
+        // ================= epilogue: pieces of 32 rows x 32 columns, dealt to the four warps of a lane quarter
+        mbar_wait_bounded(bars + DONE, 0, dead);
+        tc_fence_after();
+        const int chunks = kb1 > kb0 ? (kb1 - kb0 + A.chunk_kb - 1) / A.chunk_kb : 0, lq = warp & 3, cols = (A.geglu ? A.BN / 2 : A.BN) / 32;
         float *cbase = A.ws ? A.ws + (size_t)split * A.T * A.N + n0 : sg.c + sn0;
         const int cld = A.ws ? A.N : sg.ldc;
-#pragma unroll 1
-        for (int mt = 0; mt < BM / 128; mt++) {
-            const int lq = warp & 3, chalf = warp >> 2; // TMEM lane quarter of this warp, column quarter it drains
-            const int row = m0 + mt * 128 + lq * 32 + lane;
-#pragma unroll 1
-            for (int c0 = chalf * (BN / 4); c0 < (chalf + 1) * (BN / 4); c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(mt * BN + c0), v);
-                if (row < m_end && sn0 + c0 < sg.rows) { // rows % 32 == 0
-                    float *dst = cbase + (size_t)row * cld + c0;
-                    const float *rs = A.resid ? A.resid + (size_t)row * sg.ldc + sn0 + c0 : nullptr;
+        const uint32_t my = smem0 + warp * 4096; // the ring is no longer used
+        for (int piece = warp >> 2; piece < A.MT * cols; piece += kWorkWarps / 4) {
+            const int mt = piece / cols, c0 = (piece - mt * cols) * 32, row0 = m0 + mt * 128 + lq * 32;
+            if (row0 >= A.T || sn0 + c0 >= sg.rows) continue;
+            uint32_t v[32];
+            const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(mt * A.chunks * A.BN + c0);
+            auto add_columns = [&](uint32_t at) {
 #pragma unroll
-                    for (int u = 0; u < 32; u += 4) {
-                        float4 o = make_float4(__uint_as_float(v[u]), __uint_as_float(v[u + 1]), __uint_as_float(v[u + 2]),
-                                               __uint_as_float(v[u + 3]));
-                        if (rs) {
-                            const float4 r4 = *reinterpret_cast<const float4 *>(rs + u);
-                            o.x += r4.x; o.y += r4.y; o.z += r4.z; o.w += r4.w;
-                        }
-                        *reinterpret_cast<float4 *>(dst + u) = o;
-                    }
+                for (int hf = 0; hf < 2; hf++) {
+                    uint32_t u[16];
+                    tmem_load16(at + 16 * hf, u);
+#pragma unroll
+                    for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__uint_as_float(v[16 * hf + q]) + __uint_as_float(u[q]));
                 }
+            };
+            if (chunks > 0) tmem_load32(col, v);
+            else // no K block is left for this CTA
+                for (int q = 0; q < 32; q++) v[q] = 0;
+            for (int ch = 1; ch < chunks; ch++) add_columns(col + ch * A.BN);
+            if (A.geglu) { // the other half of the tile's columns is up (one K piece)
+#pragma unroll
+                for (int hf = 0; hf < 2; hf++) {
+                    uint32_t u[16];
+                    tmem_load16(col + A.BN / 2 + 16 * hf, u);
+#pragma unroll
+                    for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__fmul_rn(gelu_f16(__uint_as_float(v[16 * hf + q])), __uint_as_float(u[q])));
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < 8; p++) sts_u4(my + lane * 128 + ((p ^ (lane & 7)) << 4), make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]));
+            __syncwarp();
+            const int p = lane & 7;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int r = 4 * q + (lane >> 3), row = row0 + r;
+                const uint4 w = lds_u4(my + r * 128 + ((p ^ (r & 7)) << 4));
+                if (row >= A.T) continue; // rows of a matrix are a multiple of 32
+                float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+                if (A.geglu) {
+                    *reinterpret_cast<uint2 *>(A.geglu + (size_t)row * sg.rows + sn0 + c0 + 4 * p) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+                    continue;
+                }
+                if (A.resid) {
+                    const float4 r4 = *reinterpret_cast<const float4 *>(A.resid + (size_t)row * sg.ldc + sn0 + c0 + 4 * p);
+                    o.x += r4.x, o.y += r4.y, o.z += r4.z, o.w += r4.w;
+                }
+                *reinterpret_cast<float4 *>(cbase + (size_t)row * cld + c0 + 4 * p) = o;
             }
         }
-    } else {
-        // ================= MMA issuer (one lane)
+        tc_fence_before();
+    } else if (warp == kTmaWarp || warp == kCodesWarp) {
+        // ================= A rows wait for the MMAs of their stage, codes, requested further ahead, for the warps that read them
         if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16(128, BN);
-            int stage = 0;
-            uint32_t parity = 0;
+            const bool is_a = warp == kTmaWarp;
+            const int n = is_a ? A.stages : kCodeStages, full = is_a ? A_FULL : C_FULL, fre = is_a ? A_FREE : C_FREE;
+            int s = 0;
+            uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
-                mbar_wait(bars + 8 * stage, parity);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t sa = smem0 + stage * kStageBytes, sb = sa + kAStage;
-                const uint64_t bdesc = umma_desc_sw128(sb);
+                mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead);
+                const uint32_t bar = bars + full + 8 * s;
+                mbar_expect_tx(bar, is_a ? a_bytes : c_bytes);
+                if (is_a) tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, bar);
+                else tma_load_2d(codes + s * c_bytes, &maps.w[si], kb * 2 * PB, w_row0, bar);
+                if (++s == n) s = 0, ph ^= 1u;
+            }
+        }
+        __syncwarp();
+    } else if (rank == 0) {
+        // ================= MMA issuer
+        const uint32_t idesc = umma_idesc(128 * CTAS, A.BN);
+        int s = 0, chunk = 0, left = A.chunk_kb;
+        uint32_t ph = 0, it = 0;
+        for (int kb = kb0; kb < kb1; kb++, it++) {
+            const uint32_t b = it & (kTiles - 1), first = left == A.chunk_kb ? 0u : 1u;
+            mbar_wait_bounded(bars + A_FULL + 8 * s, ph, dead);
+            mbar_wait_bounded(bars + B_FULL + 8 * b, (it / kTiles) & 1, dead);
+            if (PAIR) mbar_wait_bounded(bars + PEER_FULL + 8 * b, (it / kTiles) & 1, dead);
+            tc_fence_after();
+            const uint32_t a_lo = umma_desc_lo(ring + s * a_bytes, 16), b_lo = umma_desc_lo(smem0 + b * b_bytes, 16);
+            for (int mt = 0; mt < A.MT; mt++) {
+                const uint32_t d = tmem + (mt * A.chunks + chunk) * A.BN;
 #pragma unroll
-                for (int mt = 0; mt < BM / 128; mt++) {
-                    const uint64_t adesc = umma_desc_sw128(sa + mt * 128 * 128);
-#pragma unroll
-                    for (int k = 0; k < BK / 16; k++) // 16 bf16 = 32 B = 2 descriptor units along K
-                        umma_bf16(tmem_base + (uint32_t)(mt * BN), adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc,
-                                  (kb > kb0 || k > 0) ? 1u : 0u);
-                }
-                umma_commit(bars + 8 * (kStages + stage)); // frees the stage when these MMAs have read it
-                if (++stage == kStages) {
-                    stage = 0;
-                    parity ^= 1u;
+                for (int k = 0; k < BK / 16; k++) {
+                    if (PAIR) umma_ss_pair(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, b_lo + 2 * k, idesc, k > 0 ? 1u : first);
+                    else umma_ss(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, b_lo + 2 * k, idesc, k > 0 ? 1u : first);
                 }
             }
-            umma_commit(bars + 8 * 2 * kStages); // accumulators final
+            if (PAIR) umma_arrive_pair(bars + A_FREE + 8 * s), umma_arrive_pair(bars + B_FREE + 8 * b);
+            else umma_arrive(bars + A_FREE + 8 * s), umma_arrive(bars + B_FREE + 8 * b);
+            if (--left == 0) chunk++, left = A.chunk_kb;
+            if (++s == A.stages) s = 0, ph ^= 1u;
+        }
+        if (PAIR) umma_arrive_pair(bars + DONE);
+        else umma_arrive(bars + DONE);
+    } else {
+        // ================= the second CTA's word that its A rows and weights of a K block stand
+        const uint32_t peer = cluster_addr(bars + PEER_FULL, 0);
+        int s = 0;
+        uint32_t ph = 0, it = 0;
+        for (int kb = kb0; kb < kb1; kb++, it++) {
+            mbar_wait_bounded(bars + A_FULL + 8 * s, ph, dead);
+            mbar_wait_bounded(bars + B_FULL + 8 * (it & (kTiles - 1)), (it / kTiles) & 1, dead);
+            if (lane == 0) mbar_arrive_cluster(peer + 8 * (it & (kTiles - 1)));
+            if (++s == A.stages) s = 0, ph ^= 1u;
         }
         __syncwarp();
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == kProducerWarps) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(kTmemCols) : "memory");
+    if (PAIR) cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
+    if (warp == kMmaWarp) {
+        tc_fence_after();
+        if (PAIR) tmem_free512_pair(tmem);
+        else tmem_free512(tmem);
+        if (lane == 0 && *dead) *A.wait_error = 1;
     }
 }
 
 // partial tiles of a K-split GEMM summed in split order (+ residual)
 __global__ void splitk_reduce_kernel(const GemmArgs A, int splits) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t T = A.T, N = A.N;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4, T = A.T, N = A.N; // N and the segments: multiples of 32
     if (i >= T * N) return;
     const int64_t t = i / N;
-    const int n = (int)(i % N);
+    const int n = (int)(i - t * N);
     int si = 0;
     if (A.n_seg > 1 && n >= A.seg[1].n_begin) si = (A.n_seg > 2 && n >= A.seg[2].n_begin) ? 2 : 1;
     const GemmSeg &sg = A.seg[si];
     const int col = n - sg.n_begin;
     if (col >= sg.rows) return; // tile padding between segments
-    float acc = A.ws[i];
-    for (int s = 1; s < splits; s++) acc += A.ws[(int64_t)s * T * N + i];
-    if (A.resid) acc += A.resid[t * sg.ldc + col];
-    sg.c[t * sg.ldc + col] = acc;
+    float4 acc = *reinterpret_cast<const float4 *>(A.ws + i);
+    auto add = [&](const float *p) {
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
+    };
+    for (int s = 1; s < splits; s++) add(A.ws + (int64_t)s * T * N + i);
+    if (A.resid) add(A.resid + t * sg.ldc + col);
+    *reinterpret_cast<float4 *>(sg.c + t * sg.ldc + col) = acc;
 }
 
 // rms_norm * w -> bf16 (the A operand of the next GEMM): same double-sum order as rms_norm_kernel (elementwise.cu)
@@ -724,7 +733,7 @@ int ggb_op_geglu_bf16(const float *gate, const float *up, int64_t n, void *y_bf1
 }
 
 static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, const int64_t *ldc,
-                       const float *resid, void *workspace, size_t workspace_bytes) {
+                       const float *resid, void *workspace, size_t workspace_bytes, void *geglu = nullptr) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(n >= 1 && n <= kMaxSegs && w && a_bf16 && c && ldc && T > 0, "bad gemm args");
     GGB_CHECK_ARG(n == 1 || !resid, "gemm: a residual needs a single matrix");
@@ -732,42 +741,86 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     const int type = w[0]->type;
     GGB_CHECK_ARG(type == GGB_TYPE_Q4_0 || type == GGB_TYPE_Q8_0, "gemm: weight type %d", type);
     GemmArgs A{};
+    GemmMaps maps{};
     int64_t N = 0;
     for (int i = 0; i < n; i++) {
-        GGB_CHECK_ARG(w[i] && c[i] && w[i]->cols == K && w[i]->type == type, "gemm: matrices of one launch share K and the type");
+        GGB_CHECK_ARG(w[i] && (c[i] || geglu) && w[i]->cols == K && w[i]->type == type, "gemm: matrices of one launch share K and the type");
         const int64_t rows = w[i]->rows;
         GGB_CHECK_ARG(K % 64 == 0 && rows % 32 == 0 && ldc[i] >= rows && ldc[i] % 4 == 0,
                       "gemm needs K %% 64 == 0, N %% 32 == 0 (N=%lld K=%lld)", (long long)rows, (long long)K);
-        A.seg[i] = GemmSeg{w[i]->qs, w[i]->d, c[i], (int)ldc[i], (int)N, (int)rows};
-        N += i + 1 < n ? (rows + BN - 1) / BN * BN : rows; // the next matrix starts on a tile boundary
+        A.seg[i] = GemmSeg{w[i]->d, c[i], (int)ldc[i], (int)N, (int)rows};
+        N += i + 1 < n ? (rows + 255) / 256 * 256 : rows;
     }
     A.n_seg = n;
-    static bool attr_done = false;
-    if (!attr_done) {
-        GGB_CUDA(cudaFuncSetAttribute(gemm_bf16w_kernel<GGB_TYPE_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-        GGB_CUDA(cudaFuncSetAttribute(gemm_bf16w_kernel<GGB_TYPE_Q8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-        attr_done = true;
-    }
-    const int n_tiles = (int)((N + BN - 1) / BN), m_tiles = (int)((T + BM - 1) / BM), kblocks = (int)(K / BK);
-    // split K until every SM has a tile (partials are reduced in split order: deterministic)
+    const int kblocks = (int)(K / BK), sms = ggb_sm_count(), pb = ggb_payload_bytes(type);
+    // pieces along K: until every SM has a piece of a 256 x 256 tile
+    int pieces = 1;
+    const int64_t big = (N + 255) / 256 * ((T + 255) / 256);
+    while (pieces < 8 && big * pieces * 2 <= sms && kblocks / (pieces * 2) >= 4) pieces *= 2;
+    if (pieces > 1 && (!workspace || workspace_bytes < (size_t)pieces * T * N * 4)) pieces = 1;
+    const bool pair = T > 128;
+    GGB_CHECK_ARG(!geglu || (pair && n == 2 && w[0]->rows == w[1]->rows && w[0]->rows % 256 == 0), "gemm_geglu: two matrices of as many rows and more than 128 tokens");
+    if (geglu) pieces = 1, N = 2 * w[0]->rows;
+    // the tile and the CTAs along K with the least estimated time (cycles): a stage takes what its MMAs, the bytes through shared memory (128 a
+    // cycle: written by TMA, read and written by the dequantisation, read for the MMAs) or the dequantisation take (2.7 a row: 32 weights are
+    // 170 instructions of one lane)
+    double best = -1.0;
     int splits = 1;
-    const int sms = ggb_sm_count();
-    while (splits < 8 && n_tiles * m_tiles * splits * 2 <= sms && kblocks / (splits * 2) >= 4) splits *= 2;
-    if (splits > 1 && (!workspace || workspace_bytes < (size_t)splits * T * N * 4)) splits = 1;
-    A.N = (int)N; A.K = (int)K; A.nb = (int)w[0]->nb;
-    A.a = (const __nv_bfloat16 *)a_bf16; A.T = (int)T;
-    A.kblocks_per_split = (kblocks + splits - 1) / splits;
+    for (int MT = T > 256 ? 2 : 1; MT >= 1; MT--)
+        for (int bn = pair ? 256 : 128; bn >= (geglu ? 256 : 64); bn /= 2)
+            for (int sp = 1; sp <= pieces; sp *= 2) {
+                const int chunks = pieces / sp, chunk_kb = (kblocks + pieces - 1) / pieces, br = pair ? bn / 2 : bn, rows = MT * (pair ? 256 : 128);
+                if (MT * chunks * bn > 512) continue;
+                const int64_t tiles = (N + bn - 1) / bn * ((T + rows - 1) / rows) * sp, slots = pair ? sms / 2 : sms;
+                const double mma = MT * std::max(bn, 96) * 2.0, smem = (MT * 16384.0 + br * (4.0 * pb + 128.0) + MT * 4 * (4096.0 + br * 32.0)) / 128.0;
+                const double stage = std::max(std::max(mma, smem), std::max(br * 2.7, 350.0));
+                double cost = (double)((tiles + slots - 1) / slots) * (chunks * chunk_kb * stage + MT * 128.0 * bn / (geglu ? 24.0 : 12.0) + 3000.0);
+                if (sp > 1) cost += 6000.0 + (double)sp * T * N * 8.0 / (32.0 * sms);
+                if (best < 0.0 || cost < best) {
+                    best = cost;
+                    splits = sp;
+                    A.MT = MT, A.BN = bn, A.chunks = chunks, A.chunk_kb = chunk_kb;
+                }
+            }
+    const int br = pair ? A.BN / 2 : A.BN;
+    A.N = (int)N, A.nb = (int)w[0]->nb, A.kblocks = kblocks, A.T = (int)T;
+    A.stages = std::min<int>(kMaxStages, (int)((kRing - kTiles * br * 128 - kCodeStages * br * 2 * pb) / (A.MT * 16384)));
     A.ws = splits > 1 ? (float *)workspace : nullptr;
-    A.resid = resid;
-    const dim3 grid((unsigned)n_tiles, (unsigned)m_tiles, (unsigned)splits);
-    if (splits > 1) A.resid = nullptr; // added by the reducer
-    if (type == GGB_TYPE_Q4_0) gemm_bf16w_kernel<GGB_TYPE_Q4_0><<<grid, kGemmThreads, kGemmSmem, ggb_cuda_stream()>>>(A);
-    else gemm_bf16w_kernel<GGB_TYPE_Q8_0><<<grid, kGemmThreads, kGemmSmem, ggb_cuda_stream()>>>(A);
+    A.resid = splits > 1 ? nullptr : resid; // added by the reducer
+    A.geglu = (__nv_bfloat16 *)geglu;
+    A.wait_error = ggb_wait_error_flag();
+    int rc = ggb_tensor_map_bf16(&maps.a, a_bf16, T, K, K, A.MT * 128);
+    for (int i = 0; i < n && !rc; i++) rc = ggb_tensor_map_bytes(&maps.w[i], w[i]->qs, w[i]->rows, K / 32 * pb, 2 * pb, br);
+    if (rc) return rc;
+    static const cudaError_t allowed = [] {
+        cudaError_t r = cudaSuccess;
+        for (auto k : {gemm_quant_kernel<GGB_TYPE_Q4_0, true>, gemm_quant_kernel<GGB_TYPE_Q8_0, true>, gemm_quant_kernel<GGB_TYPE_Q4_0, false>, gemm_quant_kernel<GGB_TYPE_Q8_0, false>}) {
+            const cudaError_t x = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+            if (x != cudaSuccess) r = x;
+        }
+        return r;
+    }();
+    GGB_CUDA(allowed);
+    const bool q4 = type == GGB_TYPE_Q4_0;
+    auto kfn = pair ? (q4 ? gemm_quant_kernel<GGB_TYPE_Q4_0, true> : gemm_quant_kernel<GGB_TYPE_Q8_0, true>)
+                    : (q4 ? gemm_quant_kernel<GGB_TYPE_Q4_0, false> : gemm_quant_kernel<GGB_TYPE_Q8_0, false>);
+    // row tiles first: those that share a piece of W run together
+    const int rows = A.MT * (pair ? 256 : 128);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((T + rows - 1) / rows * (pair ? 2 : 1)), (unsigned)((N + A.BN - 1) / A.BN), (unsigned)splits);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = kGemmSmem;
+    cfg.stream = ggb_cuda_stream();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+    cfg.attrs = at, cfg.numAttrs = pair ? 1 : 0;
+    GGB_CUDA(cudaLaunchKernelEx(&cfg, kfn, maps, A));
     GGB_LAUNCH_CHECK();
     if (splits > 1) {
         A.resid = resid;
         const int64_t cnt = T * N;
-        splitk_reduce_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, splits);
+        splitk_reduce_kernel<<<(unsigned)((cnt / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, splits);
         GGB_LAUNCH_CHECK();
     }
     return GGB_OK;
@@ -785,6 +838,14 @@ int ggb_op_gemm_bf16(const ggb_weight *w, const void *a_bf16, int64_t T, float *
 int ggb_op_gemm_bf16_multi(int n, const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, const int64_t *ldc,
                            void *workspace, size_t workspace_bytes) {
     return gemm_launch(n, w, a_bf16, T, c, ldc, nullptr, workspace, workspace_bytes);
+}
+
+int ggb_op_gemm_geglu_bf16(const ggb_weight *gate, const ggb_weight *up, const void *a_bf16, int64_t T, void *y_bf16) {
+    GGB_CHECK_ARG(gate && up && y_bf16, "bad gemm_geglu args");
+    const ggb_weight *ws[2] = {gate, up};
+    float *cs[2] = {nullptr, nullptr};
+    const int64_t ls[2] = {gate->rows, up->rows};
+    return gemm_launch(2, ws, a_bf16, T, cs, ls, nullptr, nullptr, 0, y_bf16);
 }
 
 int ggb_op_attn_prefill(const float *q, const void *kcache, const void *vcache, int64_t T, int pos0, int H, int Hkv, int d,

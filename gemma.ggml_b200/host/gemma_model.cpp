@@ -714,12 +714,12 @@ int gemma_model::generate(const std::vector<token_id> &prompt, int n_decode, std
 
 // ---------------------------------------------------------------- batched prefill (tcgen05 GEMMs)
 void gemma_model::free_prefill() {
-    void *bufs[] = {pf_ids_, pf_pos_, pf_x_, pf_xn_, pf_q_, pf_k_, pf_v_, pf_attn_, pf_sa_, pf_g_, pf_u_, pf_logits_, pf_a_, pf_ws_};
+    void *bufs[] = {pf_ids_, pf_pos_, pf_x_, pf_xn_, pf_q_, pf_k_, pf_v_, pf_attn_, pf_sa_, pf_g_, pf_u_, pf_logits_, pf_a_, pf_act_, pf_ws_};
     for (void *b : bufs)
         if (b) ggb_buffer_free(b);
     pf_ids_ = pf_pos_ = nullptr;
     pf_x_ = pf_xn_ = pf_q_ = pf_k_ = pf_v_ = pf_attn_ = pf_sa_ = pf_g_ = pf_u_ = pf_logits_ = nullptr;
-    pf_a_ = pf_ws_ = nullptr;
+    pf_a_ = pf_act_ = pf_ws_ = nullptr;
     pf_T_ = 0;
 }
 
@@ -740,10 +740,12 @@ int gemma_model::alloc_prefill(int T) {
     GM_TRY(ggb_buffer_alloc(t * KD * 4, (void **)&pf_v_));
     GM_TRY(ggb_buffer_alloc(t * QD * 4, (void **)&pf_attn_));
     GM_TRY(ggb_buffer_alloc(t * E * 4, (void **)&pf_sa_));
-    GM_TRY(ggb_buffer_alloc(t * F * 4, (void **)&pf_g_));
-    GM_TRY(ggb_buffer_alloc(t * F * 4, (void **)&pf_u_));
+    const size_t t_gu = F % 256 == 0 && t > 128 ? 128 : t; // longer prompts: gate and up never stand in memory
+    GM_TRY(ggb_buffer_alloc(t_gu * F * 4, (void **)&pf_g_));
+    GM_TRY(ggb_buffer_alloc(t_gu * F * 4, (void **)&pf_u_));
     GM_TRY(ggb_buffer_alloc(t * V * 4, (void **)&pf_logits_));
     GM_TRY(ggb_buffer_alloc(t * widest * 2, &pf_a_));
+    GM_TRY(ggb_buffer_alloc(t * F * 2, &pf_act_));
     // the K-split is only taken for small N (o-proj, down-proj, the fused q | k | v launch)
     const size_t KDp = (size_t)cfg_.n_head_kv * cfg_.head_dim;
     const size_t qkv_n = (QD + 255) / 256 * 256 + (KDp + 255) / 256 * 256 + KDp;
@@ -766,12 +768,13 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
     for (int i = 0; i < T; i++) pos[(size_t)i] = pos0 + i;
     GM_TRY(ggb_upload(pf_ids_, tokens, (size_t)T * 4));
     GM_TRY(ggb_upload(pf_pos_, pos.data(), (size_t)T * 4));
-    auto gemm = [&](const ggb_weight *w, int64_t K, float *out, const float *resid) -> int {
+    auto gemm_of = [&](const ggb_weight *w, int64_t K, const void *a, float *out, const float *resid) -> int {
         pf_flops_ += 2.0 * (double)t * (double)K * (double)ggb_weight_rows(w);
         const int64_t N = ggb_weight_rows(w);
         const bool small = N <= pf_ws_n_;
-        return ggb_op_gemm_bf16(w, pf_a_, t, out, N, resid, small ? pf_ws_ : nullptr, small ? pf_ws_bytes_ : 0);
+        return ggb_op_gemm_bf16(w, a, t, out, N, resid, small ? pf_ws_ : nullptr, small ? pf_ws_bytes_ : 0);
     };
+    auto gemm = [&](const ggb_weight *w, int64_t K, float *out, const float *resid) -> int { return gemm_of(w, K, pf_a_, out, resid); };
     // matrices that share the A operand go out as ONE launch (more tiles per launch, one pass over A)
     auto gemm_multi = [&](int n, const ggb_weight *const *w, int64_t K, float *const *outs) -> int {
         int64_t ld[3], total = 0;
@@ -803,13 +806,16 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
                                                capture_acts_ ? pf_attn_ : nullptr, pf_a_)); // :454-489
         PROFILE("op_mul_mat", gemm(l.attn_output, QD, pf_sa_, pf_x_));                                   // :493 + :723
         PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_sa_, l.ffn_norm, c.eps, E, t, pf_a_));            // :727
-        {
+        if (t > 128 && F % 256 == 0) { // both products and gelu(gate) * up in one launch                      // :446-449
+            pf_flops_ += 4.0 * (double)t * (double)E * (double)F;
+            PROFILE("op_mul_mat", ggb_op_gemm_geglu_bf16(l.ffn_gate, l.ffn_up, pf_a_, t, pf_act_));
+        } else {
             const ggb_weight *w2[2] = {l.ffn_gate, l.ffn_up};
             float *o2[2] = {pf_g_, pf_u_};
             PROFILE("op_mul_mat", gemm_multi(2, w2, E, o2));                                             // :446-447
+            PROFILE("op_gelu", ggb_op_geglu_bf16(pf_g_, pf_u_, t * F, pf_act_));                         // :448-449
         }
-        PROFILE("op_gelu", ggb_op_geglu_bf16(pf_g_, pf_u_, t * F, pf_a_));                               // :448-449
-        PROFILE("op_mul_mat", gemm(l.ffn_down, F, pf_x_, pf_sa_));                                       // :450 + :731
+        PROFILE("op_mul_mat", gemm_of(l.ffn_down, F, pf_act_, pf_x_, pf_sa_));                           // :450 + :731
     }
     PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_x_, output_norm_, c.eps, E, t, pf_a_));               // :735
     PROFILE("op_mul_mat", gemm(token_embd_, E, pf_logits_, nullptr));                                    // :740 (all T rows)

@@ -190,7 +190,7 @@ class gemma_model {
     int32_t *pf_ids_ = nullptr, *pf_pos_ = nullptr;
     float *pf_x_ = nullptr, *pf_xn_ = nullptr, *pf_q_ = nullptr, *pf_k_ = nullptr, *pf_v_ = nullptr, *pf_attn_ = nullptr;
     float *pf_sa_ = nullptr, *pf_g_ = nullptr, *pf_u_ = nullptr, *pf_logits_ = nullptr;
-    void *pf_a_ = nullptr, *pf_ws_ = nullptr; // bf16 A operand, K-split workspace
+    void *pf_a_ = nullptr, *pf_act_ = nullptr, *pf_ws_ = nullptr; // bf16 A operands (norms and attention, feed-forward), K-split workspace
     size_t pf_ws_bytes_ = 0;
     int64_t pf_ws_n_ = 0; // widest N the K-split workspace covers
 };
