@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(256) linear_vec_kernel(const E *__restrict__ w
     constexpr int VE = 16 / (int)sizeof(E);
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    step_wait();
     if (n >= N) return;
     float acc[TT];
     const bool vec = (K % VE == 0) && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(a)) % 16 == 0) &&
@@ -329,7 +330,7 @@ int linear_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, int
     if (T <= kVecT) {
         const dim3 grid((unsigned)((N + 7) / 8));
         switch ((int)T) {
-#define VEC_CASE(TT) case TT: linear_vec_kernel<E, TT><<<grid, 256, 0, st>>>(w, N, K, a, lda, c, ldc); break;
+#define VEC_CASE(TT) case TT: ggb_launch_step(linear_vec_kernel<E, TT>, grid, dim3(256), 0, w, N, K, a, lda, c, ldc, nullptr); break;
             VEC_CASE(1) VEC_CASE(2) VEC_CASE(3) VEC_CASE(4) VEC_CASE(5) VEC_CASE(6) VEC_CASE(7) VEC_CASE(8)
 #undef VEC_CASE
         }
@@ -348,7 +349,7 @@ int linear_act_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda,
     if (T <= kVecT) {
         const dim3 grid((unsigned)((N + 7) / 8));
         switch ((int)T) {
-#define VEC_CASE(TT) case TT: linear_vec_kernel<E, TT, ACT><<<grid, 256, 0, st>>>(w, N, K, a, lda, nullptr, N, y); break;
+#define VEC_CASE(TT) case TT: ggb_launch_step(linear_vec_kernel<E, TT, ACT>, grid, dim3(256), 0, w, N, K, a, lda, nullptr, N, y); break;
             VEC_CASE(1) VEC_CASE(2) VEC_CASE(3) VEC_CASE(4) VEC_CASE(5) VEC_CASE(6) VEC_CASE(7) VEC_CASE(8)
 #undef VEC_CASE
         }

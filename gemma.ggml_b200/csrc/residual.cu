@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(TB) residual_layer_norm_kernel(residual_args<E
     extern __shared__ __align__(16) float rl_row[]; // [W]
     __shared__ float red[32], s_wt[kMaxSlots];
     __shared__ int64_t s_off[kMaxSlots];
+    step_wait();
     const int64_t b = blockIdx.x, t = p.rows ? p.rows[b] : b, W = p.W;
     if (p.y2) { // the token's slots, looked up once: the loads below then depend on nothing
         if ((int)threadIdx.x < p.top) {
@@ -125,7 +126,7 @@ template <typename E> int residual_launch(const residual_args<E> &p, int64_t T) 
     {                                                                                                                           \
         auto k = residual_layer_norm_kernel<E, V, TB>;                                                                          \
         if (smem > 48 * 1024) GGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));         \
-        k<<<(unsigned)T, TB, smem, ggb_cuda_stream()>>>(p);                                                                     \
+        GGB_CUDA(ggb_launch_step(k, dim3((unsigned)T), dim3(TB), smem, p));                                                     \
     }
 #define RL_TB(V)                                                                                                                \
     {                                                                                                                           \

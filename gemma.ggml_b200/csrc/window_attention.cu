@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(256) window_qkv_store_kernel(const float *__re
                                                                const int32_t *__restrict__ pos0, const int32_t *__restrict__ table, int B,
                                                                E *__restrict__ cache, int64_t cache_ld, float *__restrict__ q_out) {
     __shared__ float red[2][8];
+    step_wait();
     const int64_t t = blockIdx.x;
     const int64_t pos = (int64_t)*pos0 + t;
     const float *qr = q + t * ld, *kr = k + t * ld, *vr = v + t * ld;
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(256) head_qkv_store_kernel(const float *__rest
                                                              const int32_t *__restrict__ pos0, const int32_t *__restrict__ table, int B,
                                                              E *__restrict__ cache, int64_t cache_ld, float *__restrict__ q_out) {
     const int lane = threadIdx.x & 31, item = (int)blockIdx.y * 8 + (int)(threadIdx.x >> 5);
+    step_wait();
     if (item >= H + 2 * G) return;
     const int64_t t = blockIdx.x, pos = (int64_t)*pos0 + t;
     E *row = cache + ((int64_t)table[pos / B] * B + pos % B) * cache_ld;
@@ -275,6 +277,7 @@ __global__ void __launch_bounds__(32 * kWarps) window_attn_kernel(const float *_
                                                                   float cap, const float *__restrict__ cs_v, finish_args da, E *__restrict__ out,
                                                                   int vec, float *__restrict__ part_out) {
     extern __shared__ __align__(16) float wa_smem[]; // q: [kWarps][MAPS][Dp]; merge: [kWarps][MAPS][kPartW]
+    step_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int h = blockIdx.y, g = h / (H / G);
     const int Dp = (D + 3) & ~3;
@@ -443,6 +446,7 @@ __global__ void __launch_bounds__(32) window_merge_kernel(const float *__restric
     const int64_t t = blockIdx.x;
     const int h = blockIdx.y, lane = threadIdx.x;
     constexpr int pw = MAPS * kPartW;
+    step_wait();
     float m[MAPS], l[MAPS], acc[MAPS][kMaxDvRegs];
 #pragma unroll
     for (int a = 0; a < MAPS; a++) {
@@ -717,14 +721,11 @@ static int qkv_store_launch(int dt, const float *q, const float *k, const float 
                   "window_qkv_store: bad arguments");
     GGB_CHECK_ARG(D > 0 && D % 2 == 0 && Dv > 0 && Dv % 2 == 0 && rot_dims >= 0 && rot_dims <= D && rot_dims % 2 == 0 && (!rot_dims || cos_sin_k),
                   "window_qkv_store: head sizes %d / %d and %d rotated dimensions must be even", D, Dv, rot_dims);
-    if (dt == GGB_TYPE_BF16)
-        window_qkv_store_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(q, k, v, ld, H, Gk, D, Gv, Dv, qn_w, kn_w, eps, rot_dims, rot_halves,
-                                                                            rot_dims ? cos_sin_k : nullptr, cos_sin_v, scale, pos0, block_table,
-                                                                            block_size, (__nv_bfloat16 *)cache, cld, q_out);
-    else
-        window_qkv_store_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(q, k, v, ld, H, Gk, D, Gv, Dv, qn_w, kn_w, eps, rot_dims, rot_halves,
-                                                                            rot_dims ? cos_sin_k : nullptr, cos_sin_v, scale, pos0, block_table,
-                                                                            block_size, (float *)cache, cld, q_out);
+#define QS_LAUNCH(ET)                                                                                                                                \
+    GGB_CUDA(ggb_launch_step(window_qkv_store_kernel<ET>, dim3((unsigned)T), dim3(256), 0, q, k, v, ld, H, Gk, D, Gv, Dv, qn_w, kn_w, eps, rot_dims, \
+                             rot_halves, rot_dims ? cos_sin_k : nullptr, cos_sin_v, scale, pos0, block_table, block_size, (ET *)cache, cld, q_out));
+    if (dt == GGB_TYPE_BF16) { QS_LAUNCH(__nv_bfloat16) } else { QS_LAUNCH(float) }
+#undef QS_LAUNCH
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -747,12 +748,11 @@ int ggb_op_head_qkv_store(int dt, const float *q, const float *k, const float *v
     GGB_CHECK_ARG(rot_dims >= 0 && rot_dims <= D && rot_dims % 2 == 0 && (!rot_dims || cos_sin), "head_qkv_store: %d of %d dimensions cannot turn", rot_dims, D);
     const int64_t cld = ggb_window_cache_ld(G, D, Dv);
     const dim3 grid((unsigned)T, (unsigned)((H + 2 * G + 7) / 8));
-    if (dt == GGB_TYPE_BF16)
-        head_qkv_store_kernel<<<grid, 256, 0, ggb_cuda_stream()>>>(q, k, v, ld, H, G, D, Dv, qn_w, kn_w, eps, rot_dims, rot_halves, cos_sin, scale, pos0,
-                                                                   block_table, block_size, (__nv_bfloat16 *)cache, cld, q_out);
-    else
-        head_qkv_store_kernel<<<grid, 256, 0, ggb_cuda_stream()>>>(q, k, v, ld, H, G, D, Dv, qn_w, kn_w, eps, rot_dims, rot_halves, cos_sin, scale, pos0,
-                                                                   block_table, block_size, (float *)cache, cld, q_out);
+#define HS_LAUNCH(ET)                                                                                                                              \
+    GGB_CUDA(ggb_launch_step(head_qkv_store_kernel<ET>, grid, dim3(256), 0, q, k, v, ld, H, G, D, Dv, qn_w, kn_w, eps, rot_dims, rot_halves, cos_sin, \
+                             scale, pos0, block_table, block_size, (ET *)cache, cld, q_out));
+    if (dt == GGB_TYPE_BF16) { HS_LAUNCH(__nv_bfloat16) } else { HS_LAUNCH(float) }
+#undef HS_LAUNCH
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -834,12 +834,13 @@ static int masked_attn_launch(int dt, const float *q, const void *cache, const i
         if (scratch && window > 0) n_split = (int)std::min<int64_t>(kMaxSplit, ((window + 62) / 32 + (keep + 31) / 32 + kWarps - 1) / kWarps);
         else if (scratch) n_split = kMaxSplit / 2;
         const dim3 grid((unsigned)T, (unsigned)H, (unsigned)n_split);
-#define WS_LAUNCH(ET)                                                                                                                        \
-    window_attn_kernel<ET, MAPS><<<grid, 32 * kWarps, smem, st>>>(q, (const ET *)cache, cld, block_table, block_size, pos0, T, H, G, D, Dv, window,  \
-                                                                  chunked, keep, softcap, cos_sin_v, da, (ET *)out, vec, scratch);            \
-    if (n_split > 1) {                                                                                                                       \
-        GGB_LAUNCH_CHECK();                                                                                                                  \
-        window_merge_kernel<ET, MAPS><<<dim3((unsigned)T, (unsigned)H), 32, 0, st>>>(scratch, n_split, pos0, H, Dv, cos_sin_v, da, (ET *)out); \
+#define WS_LAUNCH(ET)                                                                                                                                \
+    GGB_CUDA(ggb_launch_step(window_attn_kernel<ET, MAPS>, grid, dim3(32 * kWarps), smem, q, (const ET *)cache, cld, block_table, block_size, pos0, T, \
+                             H, G, D, Dv, window, chunked, keep, softcap, cos_sin_v, da, (ET *)out, vec, scratch));                                  \
+    if (n_split > 1) {                                                                                                                               \
+        GGB_LAUNCH_CHECK();                                                                                                                          \
+        GGB_CUDA(ggb_launch_step(window_merge_kernel<ET, MAPS>, dim3((unsigned)T, (unsigned)H), dim3(32), 0, scratch, n_split, pos0, H, Dv, cos_sin_v, \
+                                 da, (ET *)out));                                                                                                    \
     }
         if (dt == GGB_TYPE_BF16) { WS_LAUNCH(__nv_bfloat16) } else { WS_LAUNCH(float) }
 #undef WS_LAUNCH
