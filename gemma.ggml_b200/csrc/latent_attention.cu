@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(128) latent_kv_store_kernel(const float *__res
                                                               const int32_t *__restrict__ pos0, const int32_t *__restrict__ table,
                                                               int B, E *__restrict__ cache, int64_t ldk, int halves,
                                                               const float *__restrict__ dq, int Rq, const float *__restrict__ qnw, E *__restrict__ cq) {
+    step_wait();
     __shared__ float red[4];
     const int t = blockIdx.x, tid = threadIdx.x;
     if (blockIdx.y == 1) {
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(256) latent_q_absorb_kernel(const float *__res
                                                               int dims, const float *__restrict__ cs, const int32_t *__restrict__ pos0,
                                                               const E *__restrict__ w_uk, int R, float scale, float *__restrict__ qa,
                                                               int halves) {
+    step_wait();
     extern __shared__ float qs[]; // [kAbsT][D], then [4][kAbsT][64] partial sums
     float *ps = qs + kAbsT * D;
     const int h = blockIdx.y, tid = threadIdx.x, rl = tid & 63, dg = tid >> 6;
@@ -217,6 +219,7 @@ __global__ void __launch_bounds__(512) latent_attn_partial_kernel(const float *_
                                                                   const int32_t *__restrict__ table, int B, const int32_t *__restrict__ pos0,
                                                                   int T, int H, int R, int Dr, int n_split, int SW, int hpc,
                                                                   int64_t window, float *__restrict__ part) {
+    step_wait();
     // TQ consecutive tokens per CTA (portions): a warp scores and accumulates its head for all of them from ONE read of
     // every tile word; the later token's extra position is masked for the earlier one.
     extern __shared__ __align__(16) uint32_t la_smem[];
@@ -354,6 +357,7 @@ template <typename E>
 __global__ void __launch_bounds__(256) latent_attn_out_kernel(const float *__restrict__ part, int n_split, const float *__restrict__ sink,
                                                               const E *__restrict__ w_uv, int64_t T, int H, int R, int Dv,
                                                               int v_chunk, const float *__restrict__ gate, int64_t ldg, E *__restrict__ out) {
+    step_wait();
     extern __shared__ __align__(16) float ol[]; // [kOutT][R]
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t t0 = (int64_t)blockIdx.x * kOutT;
@@ -523,7 +527,7 @@ int attn_partial_launch(const float *qa, const void *cache, int64_t ldk, const i
     {                                                                                                                        \
         auto k = latent_attn_partial_kernel<E, RC, TQ>;                                                                      \
         if (smem > 48 * 1024) GGB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
-        k<<<grid, NW * 32, smem, ggb_cuda_stream()>>>(qa, (const E *)cache, ldk, table, B, pos0, (int)T, H, R, Dr, n_split, SW, hpc, window, part); \
+        ggb_launch_step(k, grid, dim3(NW * 32), smem, qa, (const E *)cache, ldk, table, B, pos0, (int)T, H, R, Dr, n_split, SW, hpc, window, part);     \
     }
 #define LA_CASE(RC)                       \
     {                                     \
@@ -560,10 +564,10 @@ static int latent_kv_store_launch(int dt, const float *d, int64_t ldd, int64_t T
     const int64_t ldk = ggb_latent_cache_ld(R, Dr);
     const dim3 grid((unsigned)T, dq ? 2 : 1);
     if (dt == GGB_TYPE_BF16)
-        latent_kv_store_kernel<<<grid, 128, 0, ggb_cuda_stream()>>>(d, ldd, R, Dr, rot_dims, norm_w, eps, cos_sin, pos0, block_table, block_size,
+        ggb_launch_step(latent_kv_store_kernel<__nv_bfloat16>, grid, dim3(128), 0, d, ldd, R, Dr, rot_dims, norm_w, eps, cos_sin, pos0, block_table, block_size,
                                                                     (__nv_bfloat16 *)cache, ldk, halves, dq, Rq, q_norm_w, (__nv_bfloat16 *)cq);
     else
-        latent_kv_store_kernel<<<grid, 128, 0, ggb_cuda_stream()>>>(d, ldd, R, Dr, rot_dims, norm_w, eps, cos_sin, pos0, block_table, block_size,
+        ggb_launch_step(latent_kv_store_kernel<float>, grid, dim3(128), 0, d, ldd, R, Dr, rot_dims, norm_w, eps, cos_sin, pos0, block_table, block_size,
                                                                     (float *)cache, ldk, halves, dq, Rq, q_norm_w, (float *)cq);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -591,10 +595,10 @@ static int latent_q_absorb_launch(int dt, const float *q, int64_t ldq, int64_t T
     const size_t smem = (size_t)kAbsT * D * 4 + (size_t)4 * kAbsT * 64 * 4;
     GGB_CHECK_ARG(smem <= 48 * 1024, "latent_q_absorb: head dimension %d too large", D);
     if (dt == GGB_TYPE_BF16)
-        latent_q_absorb_kernel<<<grid, 256, smem, ggb_cuda_stream()>>>(q, ldq, T, H, D, Dr, rot_dims, cos_sin, pos0,
+        ggb_launch_step(latent_q_absorb_kernel<__nv_bfloat16>, grid, dim3(256), smem, q, ldq, T, H, D, Dr, rot_dims, cos_sin, pos0,
                                                                        (const __nv_bfloat16 *)w_uk, R, scale, qa, halves);
     else
-        latent_q_absorb_kernel<<<grid, 256, smem, ggb_cuda_stream()>>>(q, ldq, T, H, D, Dr, rot_dims, cos_sin, pos0, (const float *)w_uk, R,
+        ggb_launch_step(latent_q_absorb_kernel<float>, grid, dim3(256), smem, q, ldq, T, H, D, Dr, rot_dims, cos_sin, pos0, (const float *)w_uk, R,
                                                                        scale, qa, halves);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -730,10 +734,10 @@ int ggb_op_latent_attn_out_gated(int dt, const float *part, int n_split, const f
     const size_t smem = (size_t)kOutT * (R + n_split) * 4;
     GGB_CHECK_ARG(smem <= 48 * 1024, "latent_attn_out: latent size %d with %d splits too large", R, n_split);
     if (dt == GGB_TYPE_BF16)
-        latent_attn_out_kernel<<<grid, 256, smem, ggb_cuda_stream()>>>(part, n_split, sink, (const __nv_bfloat16 *)w_uv, T, H, R, Dv,
+        ggb_launch_step(latent_attn_out_kernel<__nv_bfloat16>, grid, dim3(256), smem, part, n_split, sink, (const __nv_bfloat16 *)w_uv, T, H, R, Dv,
                                                                        v_chunk, gate, ldg, (__nv_bfloat16 *)out);
     else
-        latent_attn_out_kernel<<<grid, 256, smem, ggb_cuda_stream()>>>(part, n_split, sink, (const float *)w_uv, T, H, R, Dv, v_chunk, gate, ldg, (float *)out);
+        ggb_launch_step(latent_attn_out_kernel<float>, grid, dim3(256), smem, part, n_split, sink, (const float *)w_uv, T, H, R, Dv, v_chunk, gate, ldg, (float *)out);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

@@ -39,6 +39,7 @@ __device__ __forceinline__ float router_dot(const E *__restrict__ hr, const floa
 template <typename E>
 __global__ void __launch_bounds__(256) moe_logits_kernel(const E *__restrict__ h, int64_t W, int64_t T, const float *__restrict__ w,
                                                          const float *__restrict__ b, int n_exp, float *__restrict__ z) {
+    step_wait();
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (i >= T * n_exp) return;
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(256) moe_logits_kernel(const E *__restrict__ h
 // one warp per token: `top` rounds of arg-max over its logits (ties: the lower index), soft-max over the chosen
 __global__ void __launch_bounds__(32) moe_select_kernel(const float *__restrict__ zg, int n_exp, int top, int32_t *__restrict__ idx,
                                                         float *__restrict__ wt) {
+    step_wait();
     extern __shared__ float z[]; // [n_exp] logits, then [top] chosen values
     float *sel = z + n_exp;
     const int64_t t = blockIdx.x;
@@ -212,6 +214,7 @@ __device__ __forceinline__ void select_softmax_warp(float *sc, float *ch, float 
 
 __global__ void __launch_bounds__(32) moe_select_softmax_kernel(const float *__restrict__ zg, int64_t ldz, const float *__restrict__ corr, int n_exp, int top,
                                                                 int n_groups, int keep, float scale, int32_t *__restrict__ idx, float *__restrict__ wt) {
+    step_wait();
     extern __shared__ float sm[]; // [n_exp] scores, [n_exp] choice scores, [n_groups] group scores
     for (int e = threadIdx.x; e < n_exp; e += 32) sm[e] = zg[(int64_t)blockIdx.x * ldz + e];
     __syncwarp();
@@ -220,6 +223,7 @@ __global__ void __launch_bounds__(32) moe_select_softmax_kernel(const float *__r
 
 __global__ void __launch_bounds__(32) moe_select_sigmoid_kernel(const float *__restrict__ zg, const float *__restrict__ corr, int n_exp, int top,
                                                                 int n_groups, int keep, int32_t *__restrict__ idx, float *__restrict__ wt) {
+    step_wait();
     extern __shared__ float sm[]; // [n_exp] scores, [n_exp] choice scores, [n_groups] group scores
     for (int e = threadIdx.x; e < n_exp; e += 32) sm[e] = zg[(int64_t)blockIdx.x * n_exp + e];
     __syncwarp();
@@ -241,6 +245,7 @@ __global__ void __launch_bounds__(32 * kRouteStepWarps) moe_route_sigmoid_step_k
                                                                      float scale, float *zg, int32_t *__restrict__ idx, float *__restrict__ wt,
                                                                      int32_t *__restrict__ row_src, int32_t *__restrict__ inv,
                                                                      int32_t *__restrict__ row_expert) {
+    step_wait();
     extern __shared__ float sm[];
     __shared__ bool last;
     const int64_t t = blockIdx.x;
@@ -280,6 +285,7 @@ __global__ void __launch_bounds__(32 * kRouteStepWarps) moe_route_sigmoid_step_k
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t *__restrict__ idx, int n, int top, int n_exp, int n_real, int32_t *offsets,
                                                          int32_t *row_src, int32_t *inv, int32_t *tile_expert, int32_t *tile_row0,
                                                          int32_t *n_tiles, int32_t *row_expert) {
+    step_wait();
     extern __shared__ int32_t cnt[]; // [n_exp] counts, then cursors
     for (int e = threadIdx.x; e < n_exp; e += blockDim.x) cnt[e] = 0;
     __syncthreads();
@@ -316,6 +322,7 @@ __global__ void __launch_bounds__(256) moe_vec_kernel(const E *__restrict__ w, i
                                                       const int32_t *__restrict__ row_src, const int32_t *__restrict__ row_expert,
                                                       float *__restrict__ c, E *__restrict__ c_act, int64_t ldc, int vec, int n_real, float limit,
                                                       float alpha) {
+    step_wait();
     constexpr int VE = 16 / (int)sizeof(E);
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -376,6 +383,7 @@ __global__ void __launch_bounds__(256) moe_vec_shared_kernel(const E *__restrict
                                                              const int32_t *__restrict__ row_src, const int32_t *__restrict__ row_expert,
                                                              float *__restrict__ c, E *__restrict__ c_act, int64_t ldc, int vec, int n_slots,
                                                              shared_product<E> sh) {
+    step_wait();
     constexpr int VE = 16 / (int)sizeof(E);
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -412,12 +420,14 @@ __global__ void __launch_bounds__(256) moe_vec_shared_kernel(const E *__restrict
 
 // rows of A in sorted-slot order (the tensor-core product reads its operand contiguously): y[i] = a[row_src[i]], 16 bytes a thread
 __global__ void moe_gather_kernel(const uint4 *__restrict__ a, int64_t row_u4, const int32_t *__restrict__ row_src, uint4 *__restrict__ y) {
+    step_wait();
     const uint4 *src = a + (int64_t)row_src[blockIdx.x] * row_u4;
     for (int64_t i = threadIdx.x; i < row_u4; i += blockDim.x) y[(int64_t)blockIdx.x * row_u4 + i] = src[i];
 }
 
 __global__ void moe_combine_kernel(const float *__restrict__ y, const int32_t *__restrict__ inv, const float *__restrict__ wt, int top,
                                    int64_t W, float *__restrict__ out) {
+    step_wait();
     const int64_t t = blockIdx.x;
     for (int64_t i = threadIdx.x; i < W; i += blockDim.x) {
         float s = 0.f;
@@ -431,6 +441,7 @@ template <typename E>
 __global__ void moe_combine_identity_kernel(const float *__restrict__ y, const int32_t *__restrict__ inv, const float *__restrict__ wt,
                                             const int32_t *__restrict__ idx, int top, int n_real, int64_t W, const E *__restrict__ h,
                                             float *__restrict__ out) {
+    step_wait();
     const int64_t t = blockIdx.x;
     for (int64_t i = threadIdx.x; i < W; i += blockDim.x) {
         float s = 0.f;
@@ -458,11 +469,11 @@ int ggb_op_moe_route(int dt, const void *h, int64_t W, int64_t T, const float *w
     const size_t smem = (size_t)(n_exp + top) * 4;
     const unsigned blocks = (unsigned)((T * n_exp + 7) / 8);
     if (dt == GGB_TYPE_BF16)
-        moe_logits_kernel<<<blocks, 256, 0, ggb_cuda_stream()>>>((const __nv_bfloat16 *)h, W, T, w_router, bias, n_exp, logits);
+        ggb_launch_step(moe_logits_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, (const __nv_bfloat16 *)h, W, T, w_router, bias, n_exp, logits);
     else
-        moe_logits_kernel<<<blocks, 256, 0, ggb_cuda_stream()>>>((const float *)h, W, T, w_router, bias, n_exp, logits);
+        ggb_launch_step(moe_logits_kernel<float>, dim3(blocks), dim3(256), 0, (const float *)h, W, T, w_router, bias, n_exp, logits);
     GGB_LAUNCH_CHECK();
-    moe_select_kernel<<<(unsigned)T, 32, smem, ggb_cuda_stream()>>>(logits, n_exp, top, idx, wt);
+    ggb_launch_step(moe_select_kernel, dim3((unsigned)T), dim3(32), smem, logits, n_exp, top, idx, wt);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -483,21 +494,21 @@ int ggb_op_moe_route_sigmoid(int dt, const void *h, int64_t W, int64_t T, const 
         const bool lists = ws && ggb_moe_step_form(n);
         int32_t *row_src = lists ? ws + n_exp + 1 : nullptr, *inv = lists ? row_src + n : nullptr, *row_expert = lists ? inv + n + 2 * mt + 1 : nullptr;
         if (dt == GGB_TYPE_BF16)
-            moe_route_sigmoid_step_kernel<__nv_bfloat16, false><<<dim3((unsigned)T, (unsigned)((n_exp + kRouteStepWarps - 1) / kRouteStepWarps)), 32 * kRouteStepWarps, smem, ggb_cuda_stream()>>>((const __nv_bfloat16 *)h, W, w_router, correction, n_exp, 0, top, n_groups,
+            ggb_launch_step(moe_route_sigmoid_step_kernel<__nv_bfloat16, false>, dim3((unsigned)T, (unsigned)((n_exp + kRouteStepWarps - 1) / kRouteStepWarps)), dim3(32 * kRouteStepWarps), smem, (const __nv_bfloat16 *)h, W, w_router, correction, n_exp, 0, top, n_groups,
                                                                                          keep, 1.f, logits, idx, wt, row_src, inv, row_expert);
         else
-            moe_route_sigmoid_step_kernel<float, false><<<dim3((unsigned)T, (unsigned)((n_exp + kRouteStepWarps - 1) / kRouteStepWarps)), 32 * kRouteStepWarps, smem, ggb_cuda_stream()>>>((const float *)h, W, w_router, correction, n_exp, 0, top, n_groups, keep, 1.f,
+            ggb_launch_step(moe_route_sigmoid_step_kernel<float, false>, dim3((unsigned)T, (unsigned)((n_exp + kRouteStepWarps - 1) / kRouteStepWarps)), dim3(32 * kRouteStepWarps), smem, (const float *)h, W, w_router, correction, n_exp, 0, top, n_groups, keep, 1.f,
                                                                                          logits, idx, wt, row_src, inv, row_expert);
         GGB_LAUNCH_CHECK();
         return GGB_OK;
     }
     const unsigned blocks = (unsigned)((T * n_exp + 7) / 8);
     if (dt == GGB_TYPE_BF16)
-        moe_logits_kernel<<<blocks, 256, 0, ggb_cuda_stream()>>>((const __nv_bfloat16 *)h, W, T, w_router, nullptr, n_exp, logits);
+        ggb_launch_step(moe_logits_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, (const __nv_bfloat16 *)h, W, T, w_router, nullptr, n_exp, logits);
     else
-        moe_logits_kernel<<<blocks, 256, 0, ggb_cuda_stream()>>>((const float *)h, W, T, w_router, nullptr, n_exp, logits);
+        ggb_launch_step(moe_logits_kernel<float>, dim3(blocks), dim3(256), 0, (const float *)h, W, T, w_router, nullptr, n_exp, logits);
     GGB_LAUNCH_CHECK();
-    moe_select_sigmoid_kernel<<<(unsigned)T, 32, smem, ggb_cuda_stream()>>>(logits, correction, n_exp, top, n_groups,
+    ggb_launch_step(moe_select_sigmoid_kernel, dim3((unsigned)T), dim3(32), smem, logits, correction, n_exp, top, n_groups,
                                                                                                          keep, idx, wt);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -525,21 +536,21 @@ int ggb_op_moe_route_softmax_groups(int dt, const void *h, int64_t W, int64_t T,
         int32_t *row_src = lists ? ws + n_exp + 1 : nullptr, *inv = lists ? row_src + n : nullptr, *row_expert = lists ? inv + n + 2 * mt + 1 : nullptr;
         const dim3 grid((unsigned)T, (unsigned)((ldz + kRouteStepWarps - 1) / kRouteStepWarps));
         if (dt == GGB_TYPE_BF16)
-            moe_route_sigmoid_step_kernel<__nv_bfloat16, true><<<grid, 32 * kRouteStepWarps, smem, ggb_cuda_stream()>>>(
+            ggb_launch_step(moe_route_sigmoid_step_kernel<__nv_bfloat16, true>, grid, dim3(32 * kRouteStepWarps), smem,
                 (const __nv_bfloat16 *)h, W, w_router, correction, n_exp, n_extra, top, n_groups, keep, scale, logits, idx, wt, row_src, inv, row_expert);
         else
-            moe_route_sigmoid_step_kernel<float, true><<<grid, 32 * kRouteStepWarps, smem, ggb_cuda_stream()>>>(
+            ggb_launch_step(moe_route_sigmoid_step_kernel<float, true>, grid, dim3(32 * kRouteStepWarps), smem,
                 (const float *)h, W, w_router, correction, n_exp, n_extra, top, n_groups, keep, scale, logits, idx, wt, row_src, inv, row_expert);
         GGB_LAUNCH_CHECK();
         return GGB_OK;
     }
     const unsigned blocks = (unsigned)((T * ldz + 7) / 8);
     if (dt == GGB_TYPE_BF16)
-        moe_logits_kernel<<<blocks, 256, 0, ggb_cuda_stream()>>>((const __nv_bfloat16 *)h, W, T, w_router, nullptr, ldz, logits);
+        ggb_launch_step(moe_logits_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, (const __nv_bfloat16 *)h, W, T, w_router, nullptr, ldz, logits);
     else
-        moe_logits_kernel<<<blocks, 256, 0, ggb_cuda_stream()>>>((const float *)h, W, T, w_router, nullptr, ldz, logits);
+        ggb_launch_step(moe_logits_kernel<float>, dim3(blocks), dim3(256), 0, (const float *)h, W, T, w_router, nullptr, ldz, logits);
     GGB_LAUNCH_CHECK();
-    moe_select_softmax_kernel<<<(unsigned)T, 32, smem, ggb_cuda_stream()>>>(logits, ldz, correction, n_exp, top, n_groups, keep, scale, idx, wt);
+    ggb_launch_step(moe_select_softmax_kernel, dim3((unsigned)T), dim3(32), smem, logits, ldz, correction, n_exp, top, n_groups, keep, scale, idx, wt);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -569,7 +580,7 @@ int ggb_op_moe_group_identity(const int32_t *idx, int64_t T, int top, int n_exp,
                   "moe_group: bad arguments");
     const int mt = ggb_moe_max_tiles(n, n_exp);
     int32_t *offsets = ws, *row_src = ws + n_exp + 1, *inv = row_src + n, *te = inv + n, *tr = te + mt, *nt = tr + mt, *re = nt + 1;
-    moe_group_kernel<<<1, 1024, (size_t)n_exp * 4, ggb_cuda_stream()>>>(idx, (int)n, top, n_exp, n_exp - n_identity, offsets, row_src, inv, te, tr, nt, re);
+    ggb_launch_step(moe_group_kernel, dim3(1), dim3(1024), (size_t)n_exp * 4, idx, (int)n, top, n_exp, n_exp - n_identity, offsets, row_src, inv, te, tr, nt, re);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -595,11 +606,11 @@ int ggb_op_moe_linear_identity(int dt, const void *w, int64_t N, int64_t K, cons
         const int32_t *row_expert = g.n_tiles + 1;
         const dim3 grid((unsigned)((N + 7) / 8), (unsigned)(T * top));
 #define MV(E)                                                                                                                         \
-    if (act == GGB_ACT_GELU_ERF) moe_vec_kernel<E, GGB_ACT_GELU_ERF><<<grid, 256, 0, ggb_cuda_stream()>>>((const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, 0.f, 0.f); \
-    else if (act == 3) moe_vec_kernel<E, 3><<<grid, 256, 0, ggb_cuda_stream()>>>((const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, limit, alpha); \
-    else if (act == 2) moe_vec_kernel<E, 2><<<grid, 256, 0, ggb_cuda_stream()>>>((const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, 0.f, 0.f); \
-    else if (act) moe_vec_kernel<E, 1><<<grid, 256, 0, ggb_cuda_stream()>>>((const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, 0.f, 0.f); \
-    else moe_vec_kernel<E, 0><<<grid, 256, 0, ggb_cuda_stream()>>>((const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, (float *)c, nullptr, ldc, vec, n_real, 0.f, 0.f);
+    if (act == GGB_ACT_GELU_ERF) ggb_launch_step(moe_vec_kernel<E, GGB_ACT_GELU_ERF>, grid, dim3(256), 0, (const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, 0.f, 0.f); \
+    else if (act == 3) ggb_launch_step(moe_vec_kernel<E, 3>, grid, dim3(256), 0, (const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, limit, alpha); \
+    else if (act == 2) ggb_launch_step(moe_vec_kernel<E, 2>, grid, dim3(256), 0, (const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, 0.f, 0.f); \
+    else if (act) ggb_launch_step(moe_vec_kernel<E, 1>, grid, dim3(256), 0, (const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, nullptr, (E *)c, ldc, vec, n_real, 0.f, 0.f); \
+    else ggb_launch_step(moe_vec_kernel<E, 0>, grid, dim3(256), 0, (const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert, (float *)c, nullptr, ldc, vec, n_real, 0.f, 0.f);
         if (dt == GGB_TYPE_BF16) { MV(__nv_bfloat16) } else { MV(float) }
 #undef MV
         GGB_LAUNCH_CHECK();
@@ -619,7 +630,7 @@ int ggb_op_moe_linear_identity(int dt, const void *w, int64_t N, int64_t K, cons
                 GGB_CUDA(cudaMalloc(&gbuf, need));
                 gbytes = need;
             }
-            moe_gather_kernel<<<(unsigned)n, 128, 0, ggb_cuda_stream()>>>((const uint4 *)a, K / 8, g.row_src, (uint4 *)gbuf);
+            ggb_launch_step(moe_gather_kernel, dim3((unsigned)n), dim3(128), 0, (const uint4 *)a, K / 8, g.row_src, (uint4 *)gbuf);
             GGB_LAUNCH_CHECK();
             a_sorted = gbuf;
         }
@@ -649,7 +660,7 @@ int ggb_op_moe_linear_shared(int dt, const void *w, int64_t N, int64_t K, const 
     const int vec_s = K_s % ve == 0 && lda_s % ve == 0 && ((uintptr_t)w_s | (uintptr_t)a_s) % 16 == 0;
     const dim3 grid((unsigned)((std::max(N, N_s) + 7) / 8), (unsigned)(T * top + T));
 #define MVS(E, ACT)                                                                                                                             \
-    moe_vec_shared_kernel<E, ACT><<<grid, 256, 0, ggb_cuda_stream()>>>((const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert,               \
+    ggb_launch_step(moe_vec_shared_kernel<E, ACT>, grid, dim3(256), 0, (const E *)w, N, K, (const E *)a, lda, g.row_src, row_expert,               \
                                                                        ACT ? nullptr : (float *)c, ACT ? (E *)c : nullptr, ldc, vec, (int)(T * top), \
                                                                        shared_product<E>{(const E *)w_s, (const E *)a_s, N_s, K_s, lda_s, N_s,      \
                                                                                          ACT ? nullptr : (float *)c_s, ACT ? (E *)c_s : nullptr, vec_s});
@@ -677,9 +688,9 @@ int ggb_op_moe_combine_identity(int dt, const float *y, const int32_t *ws, const
                   "moe_combine_identity: bad arguments");
     const int32_t *inv = ws + n_exp + 1 + T * top;
     if (dt == GGB_TYPE_BF16)
-        moe_combine_identity_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(y, inv, wt, idx, top, n_exp - n_identity, W, (const __nv_bfloat16 *)h, out);
+        ggb_launch_step(moe_combine_identity_kernel<__nv_bfloat16>, dim3((unsigned)T), dim3(256), 0, y, inv, wt, idx, top, n_exp - n_identity, W, (const __nv_bfloat16 *)h, out);
     else
-        moe_combine_identity_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(y, inv, wt, idx, top, n_exp - n_identity, W, (const float *)h, out);
+        ggb_launch_step(moe_combine_identity_kernel<float>, dim3((unsigned)T), dim3(256), 0, y, inv, wt, idx, top, n_exp - n_identity, W, (const float *)h, out);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -688,7 +699,7 @@ int ggb_op_moe_combine(const float *y, const int32_t *ws, const float *wt, int64
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(y && ws && wt && out && T > 0 && top > 0 && W > 0, "moe_combine: bad arguments");
     const int32_t *inv = ws + n_exp + 1 + T * top;
-    moe_combine_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(y, inv, wt, top, W, out);
+    ggb_launch_step(moe_combine_kernel, dim3((unsigned)T), dim3(256), 0, y, inv, wt, top, W, out);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

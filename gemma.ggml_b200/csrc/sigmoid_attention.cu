@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(256) sigmoid_qkv_store_kernel(const float *__r
                                                                 float vnorm_eps, float scale, const int32_t *__restrict__ pos0,
                                                                 const int32_t *__restrict__ table, int B, E *__restrict__ cache, int64_t cache_ld,
                                                                 float *__restrict__ q_out) {
+    step_wait();
     const int64_t t = blockIdx.x;
     const int64_t pos = (int64_t)*pos0 + t;
     const float *qr = q + t * ld, *kr = k + t * ld, *vr = v + t * ld;
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(32 * kWarps) sigmoid_attn_step_kernel(const fl
                                                                         int H, int G, int D, int Dv, int64_t window, const float *__restrict__ r1,
                                                                         const float *__restrict__ r2, const float *__restrict__ pb,
                                                                         E *__restrict__ out, int vec, float *__restrict__ part_out) {
+    step_wait();
     extern __shared__ __align__(16) float sa_smem[]; // q: [kWarps][Dp]; sums: [kWarps][32 * kMaxDvRegs]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int h = blockIdx.y, g = h / (H / G);
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(32 * kWarps) sigmoid_attn_step_kernel(const fl
 // one warp per (token, head): the splits' sums in split order
 template <typename E>
 __global__ void __launch_bounds__(32) sigmoid_merge_kernel(const float *__restrict__ part, int n_split, int H, int Dv, E *__restrict__ out) {
+    step_wait();
     const int64_t t = blockIdx.x;
     const int h = blockIdx.y, lane = threadIdx.x;
     const float *pp = part + ((t * H + h) * n_split) * (kMaxDvRegs * 32);
@@ -321,10 +324,10 @@ int ggb_op_sigmoid_qkv_store(int dt, const float *q, const float *k, const float
                   "sigmoid_qkv_store: bad arguments");
     const int64_t cld = ggb_window_cache_ld(G, D, Dv);
     if (dt == GGB_TYPE_BF16)
-        sigmoid_qkv_store_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(q, k, v, ld, H, G, D, Dv, temp_coef, temp_every, vnorm_eps, scale, pos0,
+        ggb_launch_step(sigmoid_qkv_store_kernel<__nv_bfloat16>, dim3((unsigned)T), dim3(256), 0, q, k, v, ld, H, G, D, Dv, temp_coef, temp_every, vnorm_eps, scale, pos0,
                                                                              block_table, block_size, (__nv_bfloat16 *)cache, cld, q_out);
     else
-        sigmoid_qkv_store_kernel<<<(unsigned)T, 256, 0, ggb_cuda_stream()>>>(q, k, v, ld, H, G, D, Dv, temp_coef, temp_every, vnorm_eps, scale, pos0,
+        ggb_launch_step(sigmoid_qkv_store_kernel<float>, dim3((unsigned)T), dim3(256), 0, q, k, v, ld, H, G, D, Dv, temp_coef, temp_every, vnorm_eps, scale, pos0,
                                                                              block_table, block_size, (float *)cache, cld, q_out);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -391,11 +394,11 @@ int ggb_op_sigmoid_attn(int dt, const float *q, const void *cache, const int32_t
         else if (scratch) n_split = kMaxSplit / 2;
         const dim3 grid((unsigned)T, (unsigned)H, (unsigned)n_split);
 #define SS_LAUNCH(ET)                                                                                                                       \
-    sigmoid_attn_step_kernel<ET><<<grid, 32 * kWarps, smem, st>>>(q, (const ET *)cache, cld, block_table, block_size, pos0, H, G, D, Dv, window, \
+    ggb_launch_step(sigmoid_attn_step_kernel<ET>, grid, dim3(32 * kWarps), smem, q, (const ET *)cache, cld, block_table, block_size, pos0, H, G, D, Dv, window, \
                                                                   r1, r2, pb, (ET *)out, vec, scratch);                                     \
     if (n_split > 1) {                                                                                                                      \
         GGB_LAUNCH_CHECK();                                                                                                                 \
-        sigmoid_merge_kernel<ET><<<dim3((unsigned)T, (unsigned)H), 32, 0, st>>>(scratch, n_split, H, Dv, (ET *)out);                         \
+        ggb_launch_step(sigmoid_merge_kernel<ET>, dim3((unsigned)T, (unsigned)H), dim3(32), 0, scratch, n_split, H, Dv, (ET *)out);                         \
     }
         if (dt == GGB_TYPE_BF16) { SS_LAUNCH(__nv_bfloat16) } else { SS_LAUNCH(float) }
 #undef SS_LAUNCH
