@@ -250,7 +250,7 @@ def sub_record_prefill(G, L, args):
     rec = {"workload": "gemma-2b q8_0 prefill of 512 tokens (host call: H2D ids, per-op launches, D2H token)",
            "value": T * steps / wall, "unit": "tokens/s", "ms_per_step": 1000.0 * wall / steps,
            "gemm_tflops": ach, "gemm_frac_of_tensor_peak": ach / peak_tf, "gemm_ms_per_step": gemm_ms / steps,
-           "tensor_peak_tflops": peak_tf, "kernel": "gemm_bf16w_kernel (tcgen05.mma kind::f16, TMEM accumulators)"}
+           "tensor_peak_tflops": peak_tf, "kernel": "gemm_quant_kernel (tcgen05.mma kind::f16, cta_group::2, TMEM accumulators)"}
     m.close()
     return rec
 
@@ -561,7 +561,7 @@ def run_prefill(args):
                    "timing": "value / ms_per_step: eager per-op launches, no probes; roofline and op_classes: a second pass of the same steps with cudaEvent probes per operator (the probes add ~1 ms of launch gaps per step)"},
         "clocks": clocks.summary(),
         "roofline": {"bound": "tensor", "achieved": ach, "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf,
-                     "traffic": None, "kernel": "gemm_bf16w_kernel (tcgen05.mma kind::f16, TMEM accumulators)",
+                     "traffic": None, "kernel": "gemm_quant_kernel (tcgen05.mma kind::f16, cta_group::2, TMEM accumulators)",
                      "algorithmic_flops_per_step": flops, "gemm_ms_per_step": gemm_ms / steps,
                      "launches_per_step": gemm_calls / steps, "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained"},
         "op_classes": classes,
