@@ -15,7 +15,7 @@
 //     MEMORY, up to all 512 columns; tcgen05.commit releases the buffers of both CTAs;
 //   * after the last K block the sixteen warps become the EPILOGUE: 32 x 32 pieces turned in shared memory, residual added, whole lines stored.
 //     gate | up of a feed-forward: each CTA dequantises rows of one of the two matrices, so both products of an output stand in the same row
-//     of tensor memory and leave as gelu(gate) * up in bf16.
+//     of tensor memory and leave as gelu(gate) * up in bf16; the 128 KB gelu table is brought into the ring behind the last MMA.
 // A product along a long K is summed in pieces of K (as many as a split over the SMs in 256 x 256 tiles needs): several accumulators a
 // CTA in tensor memory, added in order by the epilogue, and, where SMs are left, several CTAs whose sums meet in a workspace and are
 // added in order by a second kernel (deterministic).
@@ -46,7 +46,8 @@ constexpr uint32_t kRing = 224 * 1024;
 constexpr int kMaxStages = 6;
 constexpr size_t kGemmSmem = 1024 + kRing + 384;
 constexpr int kTiles = 2, kCodeStages = 4; // buffers of dequantised weights, of codes
-enum { A_FULL = 0, A_FREE = 48, B_FULL = 96, B_FREE = 128, PEER_FULL = 160, C_FULL = 192, C_FREE = 240, DONE = 288, SLOT = 296, DEAD = 304 };
+enum { A_FULL = 0, A_FREE = 48, B_FULL = 96, B_FREE = 128, PEER_FULL = 160, C_FULL = 192, C_FREE = 240, DONE = 288, SLOT = 296, DEAD = 304, TABLE_FULL = 312 };
+constexpr uint32_t kGeluBytes = 65536 * 2, kGeluAt = 64 * 1024; // the gelu table, behind the epilogue's 16 x 4 KB: where only TMA wrote and MMAs read
 
 // up to 3 weight matrices that share the A operand run as ONE launch (Q | K | V, gate | up): a segment = one matrix, its first row is a
 // multiple of 256, so a tile belongs to exactly one segment
@@ -66,6 +67,7 @@ struct GemmArgs {
     float *ws;           // workspace [splits][T][N] or null (one CTA along K: tiles go straight to seg.c)
     const float *resid;  // [T][seg[0].ldc] or null (single segment, no workspace)
     __nv_bfloat16 *geglu; // two segments, gate and up, of which every tile takes BN / 2 rows each: [T][rows] gelu(gate) * up
+    const uint16_t *gelu; // the fp16 table of gelu
     int *wait_error;
 };
 struct GemmMaps {
@@ -120,12 +122,6 @@ __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
     return v;
 }
 
-// gelu of an fp16 number, rounded to fp16, as the reference's table has it
-__device__ __forceinline__ float gelu_f16(float g) {
-    const float x = __half2float(__float2half_rn(g));
-    return __half2float(__float2half_rn(0.5f * x * (1.0f + tanhf(0.79788456080286535587989211986876f * x * (1.0f + 0.044715f * x * x)))));
-}
-
 template <int TYPE, bool PAIR>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs A) {
     extern __shared__ uint8_t gemm_smem_raw[];
@@ -162,6 +158,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
             mbar_init(bars + PEER_FULL + 8 * s, 1);
         }
         mbar_init(bars + DONE, 1);
+        mbar_init(bars + TABLE_FULL, 1);
         *dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -236,6 +233,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         float *cbase = A.ws ? A.ws + (size_t)split * A.T * A.N + n0 : sg.c + sn0;
         const int cld = A.ws ? A.N : sg.ldc;
         const uint32_t my = smem0 + warp * 4096; // the ring is no longer used
+        if (A.geglu) mbar_wait_bounded(bars + TABLE_FULL, 0, dead);
+        auto gelu = [&](uint32_t g) { // of an fp16 number, rounded to fp16: the table, as ggb_op_geglu_bf16 reads it
+            uint16_t h;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(smem0 + kGeluAt + 2u * float_to_half_bits(__uint_as_float(g))) : "memory");
+            return half_bits_to_float(h);
+        };
         for (int piece = warp >> 2; piece < A.MT * cols; piece += kWorkWarps / 4) {
             const int mt = piece / cols, c0 = (piece - mt * cols) * 32, row0 = m0 + mt * 128 + lq * 32;
             if (row0 >= A.T || sn0 + c0 >= sg.rows) continue;
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                     uint32_t u[16];
                     tmem_load16(col + A.BN / 2 + 16 * hf, u);
 #pragma unroll
-                    for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__fmul_rn(gelu_f16(__uint_as_float(v[16 * hf + q])), __uint_as_float(u[q])));
+                    for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__fmul_rn(gelu(v[16 * hf + q]), __uint_as_float(u[q])));
                 }
             }
             __syncwarp();
@@ -300,6 +303,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                 if (is_a) tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, bar);
                 else tma_load_2d(codes + s * c_bytes, &maps.w[si], kb * 2 * PB, w_row0, bar);
                 if (++s == n) s = 0, ph ^= 1u;
+            }
+            if (A.geglu && is_a) { // the MMAs have read the ring: the gelu table takes its place
+                mbar_wait_bounded(bars + DONE, 0, dead);
+                if (!*dead) {
+                    mbar_expect_tx(bars + TABLE_FULL, kGeluBytes);
+                    for (uint32_t o = 0; o < kGeluBytes; o += 32768)
+                        bulk_load(smem0 + kGeluAt + o, reinterpret_cast<const uint8_t *>(A.gelu) + o, 32768, bars + TABLE_FULL);
+                }
             }
         }
         __syncwarp();
@@ -708,6 +719,14 @@ size_t ggb_gemm_workspace_bytes(int64_t T, int64_t N, int64_t K) {
     return (size_t)8 * (size_t)T * (size_t)N * 4; // up to 8 K-splits
 }
 
+// until every SM has a piece of a 256 x 256 tile
+int ggb_gemm_pieces(int64_t T, int64_t N, int64_t K) {
+    const int64_t big = (N + 255) / 256 * ((T + 255) / 256), sms = ggb_sm_count(), kblocks = K / BK;
+    int pieces = 1;
+    while (pieces < 8 && big * pieces * 2 <= sms && kblocks / (pieces * 2) >= 4) pieces *= 2;
+    return pieces;
+}
+
 int ggb_op_cvt_f32_bf16(const float *x, int64_t n, void *y_bf16) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(x && y_bf16 && n > 0, "bad cvt args");
@@ -753,14 +772,12 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     }
     A.n_seg = n;
     const int kblocks = (int)(K / BK), sms = ggb_sm_count(), pb = ggb_payload_bytes(type);
-    // pieces along K: until every SM has a piece of a 256 x 256 tile
-    int pieces = 1;
-    const int64_t big = (N + 255) / 256 * ((T + 255) / 256);
-    while (pieces < 8 && big * pieces * 2 <= sms && kblocks / (pieces * 2) >= 4) pieces *= 2;
+    int pieces = ggb_gemm_pieces(T, N, K);
     if (pieces > 1 && (!workspace || workspace_bytes < (size_t)pieces * T * N * 4)) pieces = 1;
     const bool pair = T > 128;
     GGB_CHECK_ARG(!geglu || (pair && n == 2 && w[0]->rows == w[1]->rows && w[0]->rows % 256 == 0), "gemm_geglu: two matrices of as many rows and more than 128 tokens");
     if (geglu) pieces = 1, N = 2 * w[0]->rows;
+    A.gelu = ggb_gelu_table_dev();
     // the tile and the CTAs along K with the least estimated time (cycles): a stage takes what its MMAs, the bytes through shared memory (128 a
     // cycle: written by TMA, read and written by the dequantisation, read for the MMAs) or the dequantisation take (2.7 a row: 32 weights are
     // 170 instructions of one lane)

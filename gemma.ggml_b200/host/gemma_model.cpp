@@ -729,8 +729,10 @@ int gemma_model::alloc_prefill(int T) {
     const gemma_config &c = cfg_;
     const size_t E = (size_t)c.n_embd, F = (size_t)c.n_ff, V = (size_t)c.n_vocab, t = (size_t)T;
     const size_t QD = (size_t)c.n_head * c.head_dim, KD = (size_t)c.n_head_kv * c.head_dim;
-    size_t widest = E > QD ? E : QD;
-    if (F > widest) widest = F;
+    const size_t widest = E > QD ? E : QD;
+    // the K-split is only taken for small N (o-proj, down-proj, the fused q | k | v launch, a narrow gate | up)
+    const size_t qkv_n = (QD + 255) / 256 * 256 + (KD + 255) / 256 * 256 + KD;
+    pf_ws_n_ = (int64_t)std::max(std::max(E, QD), qkv_n);
     GM_TRY(ggb_buffer_alloc(t * 4, (void **)&pf_ids_));
     GM_TRY(ggb_buffer_alloc(t * 4, (void **)&pf_pos_));
     GM_TRY(ggb_buffer_alloc(t * E * 4, (void **)&pf_x_));
@@ -740,16 +742,13 @@ int gemma_model::alloc_prefill(int T) {
     GM_TRY(ggb_buffer_alloc(t * KD * 4, (void **)&pf_v_));
     GM_TRY(ggb_buffer_alloc(t * QD * 4, (void **)&pf_attn_));
     GM_TRY(ggb_buffer_alloc(t * E * 4, (void **)&pf_sa_));
-    const size_t t_gu = F % 256 == 0 && t > 128 ? 128 : t; // longer prompts: gate and up never stand in memory
+    // wide feed-forwards of longer prompts: gate and up never stand in memory
+    const size_t t_gu = F % 256 == 0 && t > 128 && 2 * (int64_t)F > pf_ws_n_ ? 128 : t;
     GM_TRY(ggb_buffer_alloc(t_gu * F * 4, (void **)&pf_g_));
     GM_TRY(ggb_buffer_alloc(t_gu * F * 4, (void **)&pf_u_));
     GM_TRY(ggb_buffer_alloc(t * V * 4, (void **)&pf_logits_));
     GM_TRY(ggb_buffer_alloc(t * widest * 2, &pf_a_));
     GM_TRY(ggb_buffer_alloc(t * F * 2, &pf_act_));
-    // the K-split is only taken for small N (o-proj, down-proj, the fused q | k | v launch)
-    const size_t KDp = (size_t)cfg_.n_head_kv * cfg_.head_dim;
-    const size_t qkv_n = (QD + 255) / 256 * 256 + (KDp + 255) / 256 * 256 + KDp;
-    pf_ws_n_ = (int64_t)std::max(std::max(E, QD), qkv_n);
     pf_ws_bytes_ = ggb_gemm_workspace_bytes((int64_t)t, pf_ws_n_, 0);
     GM_TRY(ggb_buffer_alloc(pf_ws_bytes_, &pf_ws_));
     pf_T_ = T;
@@ -786,6 +785,9 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
         const bool small = total <= pf_ws_n_;
         return ggb_op_gemm_bf16_multi(n, w, pf_a_, t, outs, ld, small ? pf_ws_ : nullptr, small ? pf_ws_bytes_ : 0);
     };
+    // gate | up and gelu in one launch sums along K in one piece: where the two launches would take more (their workspace covers both
+    // matrices and they leave SMs without work), those run
+    const bool fuse_gate_up = t > 128 && F % 256 == 0 && (2 * F > pf_ws_n_ || ggb_gemm_pieces(t, 2 * F, E) == 1);
     pf_flops_ = 0.0;
     PROFILE("op_get_rows", ggb_op_get_rows(token_embd_, pf_ids_, t, sqrtf((float)c.n_embd), pf_x_));   // :675-679
     for (int il = 0; il < c.n_layer; il++) {
@@ -806,7 +808,7 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
                                                capture_acts_ ? pf_attn_ : nullptr, pf_a_)); // :454-489
         PROFILE("op_mul_mat", gemm(l.attn_output, QD, pf_sa_, pf_x_));                                   // :493 + :723
         PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_sa_, l.ffn_norm, c.eps, E, t, pf_a_));            // :727
-        if (t > 128 && F % 256 == 0) { // both products and gelu(gate) * up in one launch                      // :446-449
+        if (fuse_gate_up) { // both products and gelu(gate) * up in one launch                                // :446-449
             pf_flops_ += 4.0 * (double)t * (double)E * (double)F;
             PROFILE("op_mul_mat", ggb_op_gemm_geglu_bf16(l.ffn_gate, l.ffn_up, pf_a_, t, pf_act_));
         } else {

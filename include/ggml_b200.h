@@ -238,8 +238,10 @@ int ggb_op_gemm_bf16(const ggb_weight *w, const void *a_bf16, int64_t T, float *
  * row counts rounded up to 256 each, K). */
 int ggb_op_gemm_bf16_multi(int n, const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c,
                            const int64_t *ldc, void *workspace, size_t workspace_bytes);
-/* gate and up of a feed-forward and gelu(gate x) * (up x) in one launch: y (bf16, [T][rows]), what ggb_op_gemm_bf16_multi and
- * ggb_op_geglu_bf16 make together; T > 128, rows %% 256 == 0 */
+/* the pieces along K in which such a product is summed where its workspace is given (one where it is not) */
+int ggb_gemm_pieces(int64_t T, int64_t N, int64_t K);
+/* gate and up of a feed-forward and gelu(gate x) * (up x) in one launch: y (bf16, [T][rows]), the same bits as ggb_op_gemm_bf16_multi
+ * without a workspace and ggb_op_geglu_bf16; T > 128, rows %% 256 == 0 */
 int ggb_op_gemm_geglu_bf16(const ggb_weight *gate, const ggb_weight *up, const void *a_bf16, int64_t T, void *y_bf16);
 int ggb_op_cvt_f32_bf16(const float *x, int64_t n, void *y_bf16);
 /* fused producers of the GEMM's bf16 A operand: rms_norm(x) * w, and gelu(gate) * up (graph_build_norm /

@@ -62,5 +62,50 @@ def test_gate_up_gelu(gpu, wtype, T, F, K):
     cg, cu = zeros(gpu, T * F * 4), zeros(gpu, T * F * 4)
     gpu.check(lib.ggb_op_gemm_bf16_multi(2, (C.c_void_p * 2)(g.h, u.h), a.ptr, T, (C.c_void_p * 2)(cg.ptr, cu.ptr), (C.c_int64 * 2)(F, F), None, 0))
     gpu.check(lib.ggb_op_geglu_bf16(cg.ptr, cu.ptr, T * F, y2.ptr))
-    assert np.mean(y.download(np.uint16) != y2.download(np.uint16)) < 1e-3  # the same sums; the table's gelu may round an fp16 number the other way
+    assert (y.download(np.uint16) == y2.download(np.uint16)).all()  # the same sums, the same table
     assert lib.ggb_op_gemm_geglu_bf16(g.h, u.h, a.ptr, 128, y.ptr) != 0
+
+
+def test_gelu_of_every_fp16_number(gpu):
+    """One number of K: gate = code * d * a exactly, its fp16 number spread over all signs and exponents."""
+    lib, T, F, K = gpu.cuda_lib(), 1024, 512, 64
+    r = np.random.default_rng(5)
+    w = f32(np.zeros((F, K)))
+    w[:, 0] = r.integers(-127, 128, F)
+    w[:, 1] = 127.0  # the block's scale is 1
+    q = O.quantize(O.TYPE_Q8_0, w)
+    g = gpu.Weight.upload(O.TYPE_Q8_0, q, K)
+    u = gpu.Weight.upload(O.TYPE_Q8_0, O.quantize(O.TYPE_Q8_0, f32(np.ones((F, K)))), K)
+    av = np.zeros((T, K))
+    av[:, 0] = np.exp2(r.uniform(-24.0, 10.0, T)) * r.choice([-1.0, 1.0], T)
+    av[:4, 0] = [0.0, np.inf, -np.inf, np.nan]
+    a = dev(gpu, bf16_round(av)[1])
+    y, y2, cg, cu = zeros(gpu, T * F * 2), zeros(gpu, T * F * 2), zeros(gpu, T * F * 4), zeros(gpu, T * F * 4)
+    gpu.check(lib.ggb_op_gemm_geglu_bf16(g.h, u.h, a.ptr, T, y.ptr))
+    gpu.check(lib.ggb_op_gemm_bf16_multi(2, (C.c_void_p * 2)(g.h, u.h), a.ptr, T, (C.c_void_p * 2)(cg.ptr, cu.ptr), (C.c_int64 * 2)(F, F), None, 0))
+    gpu.check(lib.ggb_op_geglu_bf16(cg.ptr, cu.ptr, T * F, y2.ptr))
+    assert len(np.unique(cg.download(np.float32).astype(np.float16).view(np.uint16))) > 20000
+    assert (y.download(np.uint16) == y2.download(np.uint16)).all()
+
+
+@pytest.mark.parametrize("heads,kv,ff,fused", [(8, 8, 1024, False), (2, 1, 1024, True)])
+def test_narrow_gate_up_is_summed_in_pieces(gpu, heads, kv, ff, fused):
+    """A gate | up no wider than the workspace of the other products is summed along K in as many pieces as they are: two launches."""
+    m = gpu.GemmaModel(gpu.make_config(1024, 2, heads, kv, 256, ff, 2048, 256, wtype=gpu.TYPE_Q8_0))
+    m.init_synthetic_weights()
+    m.init_kv_cache()
+    m.build_compute_graph()
+    lib, T = gpu.cuda_lib(), 200
+    assert lib.ggb_gemm_pieces(T, 2 * ff, 1024) > 1
+    gpu.check(lib.ggb_prof_reset())
+    gpu.check(lib.ggb_prof_enable(1))
+    try:
+        m.prefill(np.arange(T, dtype=np.int32))
+    finally:
+        gpu.check(lib.ggb_prof_enable(0))
+    assert (gpu.prof_get("op_gelu")[1] == 0) == fused
+    first = m.prefill_logits(T - 1).copy()
+    m.prefill(np.arange(128, dtype=np.int32))  # buffers sized for the longer prompt
+    m.prefill(np.arange(T, dtype=np.int32))
+    assert (m.prefill_logits(T - 1) == first).all()
+    m.close()
