@@ -102,10 +102,12 @@ __device__ __forceinline__ void soft_cap16(float *z, float cap, float inv_cap) {
 #pragma unroll
     for (int c = 0; c < 16; c++) z[c] = cap * t[c];
 }
-// 1 / (1 + exp(-z)): the reciprocal by one Newton step from the approximate one (no division's slow path); exp(-z) stays finite
+// 1 / (1 + exp(-z)): the reciprocal by one Newton step from the approximate one (no division's slow path); exp(-z) stays finite, a NaN
+// stays one
 __device__ __forceinline__ float sigmoid_fast(float z) {
-    const float d = 1.0f + expf(fminf(-z, 88.0f));
-    float r;
+    float e, r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(e) : "f"(-z), "f"(88.0f));
+    const float d = 1.0f + expf(e);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }

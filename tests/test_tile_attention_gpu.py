@@ -106,3 +106,46 @@ def test_sigmoid_heads(gpu, H, Gk, D, Dv, T, pos, window, page, bare):
             z = z - np.float64(r1[h]) * np.log1p(np.float64(r2[h]) * dist) + np.float64(pb[h])
         want.append((vis / (1.0 + np.exp(-z))) @ V[:, h // (H // G)])
     assert rel(from_dt(BF16, out, (T, H, Dv)), np.stack(want, 1)) < LIMIT
+
+
+def attend(gpu, kind, q, cache, table, pos0, T, pos, H, G, D, Dv, cap=0.0, window=0, keep=0, sink=None, gate=None, offsets=None):
+    """one call of soft-max, differential or sigmoid heads over a bf16 cache: [T][H][Dv]"""
+    lib, out = gpu.cuda_lib(), zeros(gpu, T * H * Dv * 2)
+    head = (BF16, dev(gpu, q).ptr, cache.ptr, table.ptr, 64, pos0.ptr, T, H, G, D, Dv, window)
+    g, s = ptr(dev(gpu, f32(gate)) if gate is not None else None), ptr(dev(gpu, f32(sink)) if sink is not None else None)
+    if kind == "soft":
+        gpu.check(lib.ggb_op_masked_attn_gated(*head, keep, cap, s, g, H * Dv, out.ptr, None), "attn")
+    elif kind == "diff":
+        gpu.check(lib.ggb_op_diff_attn(*head, keep, cap, 0.4, 0.7, 1e-5, g, H * Dv, out.ptr, None), "attn")
+    else:
+        gpu.check(lib.ggb_op_sigmoid_attn(*head, *(ptr(dev(gpu, f32(o))) for o in (offsets or np.zeros((3, H)))), out.ptr, None), "attn")
+    return from_dt(BF16, out, (T, H, Dv))
+
+
+@pytest.mark.parametrize("kind,cap", [("soft", 0.0), ("soft", 30.0), ("diff", 0.0), ("sigmoid", 0.0)])
+@pytest.mark.parametrize("where", ["query", "key", "gate"])
+def test_nan_stays_nan_and_where_it_is(gpu, kind, cap, where):
+    if kind == "sigmoid" and where == "gate":
+        pytest.skip("these heads have no gate")
+    H, G, D, Dv, T, pos, maps = 4, 2, 64, 64, 70, 90, 2 if kind == "diff" else 1
+    r, q, K, V, cache, table, pos0 = inputs(gpu, BF16, H, G, D, Dv, maps, pos, T, 64, 3, 0.3)
+    gate = r.standard_normal((T, H * Dv)) if kind != "sigmoid" else None
+    call = lambda: attend(gpu, kind, q, cache, table, pos0, T, pos, H, G, D, Dv, cap, gate=gate)  # noqa: E731
+    want = call()
+    assert np.isfinite(want).all()
+    bad = np.zeros((T, H, Dv), bool)
+    t0, g, c = 33, 1, 5  # a token, a key head, a coordinate
+    if where == "query":
+        q[t0, 2, maps - 1, c] = np.nan
+        bad[t0, 2] = True
+    elif where == "gate":
+        gate[t0, 2 * Dv + c] = np.nan
+        bad[t0, 2, c] = True
+    else:
+        raw, tab = cache.download(np.uint16).reshape(-1, int(gpu.cuda_lib().ggb_window_cache_ld(G, D * maps, Dv))), table.download(np.int32)
+        raw[tab[(pos + t0) // 64] * 64 + (pos + t0) % 64, g * maps * D + c] = 0x7fc0
+        cache.upload(raw)
+        bad[t0:, 2 * g:2 * g + 2] = True
+    got = call()
+    assert np.isnan(got[bad]).all()
+    assert (got[~bad] == want[~bad]).all()
