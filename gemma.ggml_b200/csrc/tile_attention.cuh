@@ -15,6 +15,11 @@
 // (cp.async, page table per row), one warp issues every MMA.  A maximum is kept until a score exceeds it by 8 (the weights then reach
 // e^8, and sum and output are relative to the kept one all the same), so the output is hardly ever rescaled.
 //
+// An infinite number is not the sum of its three parts (inf, NaN, NaN), and a part of a finite query or weight that is zero makes NaN of an
+// infinite key or value; so does a weight of zero of a value that the row does not see.  A row whose sums are not all finite is therefore
+// computed once more over its visible keys by fp32 multiply-adds (plain_row): an infinite key, value or query gives what the plain
+// arithmetic gives for it.
+//
 // What bounds it: the instructions around the weights, about 40 a number with a soft cap (2.2 us a tile on the 128 rows of an SM, of which
 // 1.0 us would be the MMAs alone).  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft
 // cap, gate: 55 us, 156 TFLOP/s of the products asked for (785 us by the fp32 CUDA cores, tiles of 32 queries x 32 keys); 777 tokens
@@ -182,6 +187,50 @@ template <int MAPS, int KS> __device__ __forceinline__ void mma_role(const mma_a
         if (n + 2 < m.NT) scores(n + 2); // behind this tile's weights: the MMAs of a thread run in order
     }
     umma_arrive(m.bars + DONE);
+}
+
+struct row_job {
+    const float *q;
+    const __nv_bfloat16 *k, *v; // a head's keys (of the map) and values in cache row 0
+    int64_t ld;
+    const int32_t *table;
+    int B;
+    int64_t lo, keep, i; // positions [0, min(keep, lo)) and [lo, i]
+    int D, Dv;
+    float cap, r1, r2, pb;
+};
+// one row by one warp, a key a lane: weighted sums to out[Dv], maximum and denominator to *m_out and *l_out
+template <int MODE> __device__ __noinline__ void plain_row(const row_job &j, float *out, float *m_out, float *l_out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t n_keep = MODE == SOFTMAX ? min(j.keep, j.lo) : 0, total = n_keep + (j.i - j.lo + 1);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f}, m = -INFINITY, l = 0.f; // Dv <= 128
+    for (int64_t n0 = 0; n0 < total; n0 += 32) {
+        const int keys = (int)min((int64_t)32, total - n0);
+        const int64_t n = n0 + min(lane, keys - 1), at = n < n_keep ? n : j.lo + (n - n_keep);
+        const int64_t row = ((int64_t)j.table[at / j.B] * j.B + at % j.B) * j.ld;
+        float s = 0.f, p = 0.f;
+        for (int d = 0; d < j.D; d++) s = fmaf(to_f32(j.k[row + d]), j.q[d], s);
+        if (MODE == SOFTMAX) {
+            if (j.cap > 0.f) s = j.cap * tanhf(s / j.cap);
+            const float mx = fmaxf(m, warp_max_f32(lane < keys ? s : -INFINITY)), corr = mx == -INFINITY ? 1.f : expf(m - mx);
+            if (lane < keys && s != -INFINITY) p = expf(s - mx);
+            l = fmaf(l, corr, warp_sum_f32(p));
+            for (int r = 0; r < 4; r++) acc[r] *= corr;
+            m = mx;
+        } else if (lane < keys) {
+            p = sigmoid_fast(s - penalty(j.r1, j.r2, j.i - at) + j.pb);
+        }
+        for (int u = 0; u < keys; u++) {
+            const float pu = __shfl_sync(0xffffffffu, p, u);
+            const __nv_bfloat16 *v = j.v + __shfl_sync(0xffffffffu, row, u);
+            for (int r = 0; r < 4; r++)
+                if (lane + 32 * r < j.Dv) acc[r] = fmaf(pu, to_f32(v[lane + 32 * r]), acc[r]);
+        }
+    }
+    for (int r = 0; r < 4; r++)
+        if (lane + 32 * r < j.Dv) out[lane + 32 * r] = acc[r];
+    if (lane == 0) *m_out = m, *l_out = l;
+    __syncwarp();
 }
 
 // FIN: what becomes of a row, a warp's work when the sums stand in shared memory: load() requests what a row needs from memory, row()
@@ -443,6 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const 
         }
         float *of = reinterpret_cast<float *>(gbase);
         const int op = a.Dv + 1, n16 = a.Dv / 16;
+        float odd = MODE == SOFTMAX ? 0.f * L : 0.f; // 0, or NaN when a sum of the row is not finite
         for (int cb = grp; cb < n16; cb += 2) {
             uint32_t o0[16], o1[16];
             tmem_load16(tmem + lanes + o_col + 16 * cb, o0);
@@ -452,9 +502,26 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const 
                 float v = __uint_as_float(o0[u]) * f0;
                 if (NT > 1) v = fmaf(__uint_as_float(o1[u]), f1, v);
                 of[r * op + 16 * cb + u] = v;
+                odd = fmaf(0.f, v, odd);
             }
         }
+        st[(2 + grp) * kRows + r] = odd;
         bar_sync(3, 256);
+        // a warp's 16 rows: warp, warp + 8, ...; those whose sums are not finite once more, without the split
+        {
+            const int er = warp + 8 * (lane & 15);
+            uint32_t again = __ballot_sync(0xffffffffu, st[2 * kRows + er] + st[3 * kRows + er] != 0.f) & 0xffffu;
+            while (again) {
+                const int rr = warp + 8 * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
+                again &= again - 1;
+                if (rp >= n_pairs) continue;
+                row_job j{a.q + (((t0 + rq) * a.H + h) * MAPS + rm) * a.D, a.cache + ((int64_t)g * MAPS + rm) * a.D, a.cache + (int64_t)a.G * MAPS * a.D + (int64_t)g * a.Dv,
+                          a.cache_ld, a.table, a.B, first_visible(i0 + rq, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i0 + rq, a.D, a.Dv, a.cap, 0.f, 0.f, 0.f};
+                if (MODE == SIGMOID && a.r1) j.r1 = a.r1[h], j.r2 = a.r2[h];
+                if (MODE == SIGMOID && a.pb) j.pb = a.pb[h];
+                plain_row<MODE>(j, of + rr * op, st + rr, st + kRows + rr);
+            }
+        }
         // a warp a row, four rows' reads from memory in flight
         for (int p0 = warp; p0 < n_pairs; p0 += 32) {
             typename FIN::reads rd[4];

@@ -123,7 +123,7 @@ def attend(gpu, kind, q, cache, table, pos0, T, pos, H, G, D, Dv, cap=0.0, windo
 
 
 @pytest.mark.parametrize("kind,cap", [("soft", 0.0), ("soft", 30.0), ("diff", 0.0), ("sigmoid", 0.0)])
-@pytest.mark.parametrize("where", ["query", "key", "gate"])
+@pytest.mark.parametrize("where", ["query", "key", "value", "gate"])
 def test_nan_stays_nan_and_where_it_is(gpu, kind, cap, where):
     if kind == "sigmoid" and where == "gate":
         pytest.skip("these heads have no gate")
@@ -143,9 +143,69 @@ def test_nan_stays_nan_and_where_it_is(gpu, kind, cap, where):
         bad[t0, 2, c] = True
     else:
         raw, tab = cache.download(np.uint16).reshape(-1, int(gpu.cuda_lib().ggb_window_cache_ld(G, D * maps, Dv))), table.download(np.int32)
-        raw[tab[(pos + t0) // 64] * 64 + (pos + t0) % 64, g * maps * D + c] = 0x7fc0
+        raw[tab[(pos + t0) // 64] * 64 + (pos + t0) % 64, (g * maps * D if where == "key" else G * maps * D + g * Dv) + c] = 0x7fc0
         cache.upload(raw)
         bad[t0:, 2 * g:2 * g + 2] = True
+        if where == "value" and kind != "diff":  # one coordinate; the norm of a differential head reaches all of them
+            bad[:, :, np.arange(Dv) != c] = False
     got = call()
     assert np.isnan(got[bad]).all()
-    assert (got[~bad] == want[~bad]).all()
+    if where == "value":  # tokens that do not see it, and the other coordinates: finite numbers by another order of sums
+        assert rel(got[~bad], want[~bad]) < LIMIT
+    else:
+        assert (got[~bad] == want[~bad]).all()
+
+
+def plain_heads(kind, q, K, V, vis, cap, offsets, dist):
+    """soft-max, differential or sigmoid heads in float64, only visible keys taking part (0 times an invisible infinity is nothing)"""
+    T, H, maps, _ = q.shape
+    out = np.empty((T, H, V.shape[2]))
+    for t in range(T):
+        j = vis[t]
+        for h in range(H):
+            g, o = h // (H // K.shape[1]), []
+            for mp in range(maps):
+                s = K[j, g, mp].astype(np.float64) @ q[t, h, mp].astype(np.float64)
+                if kind == "sigmoid":
+                    p = 1.0 / (1.0 + np.exp(-(s - offsets[0][h] * np.log1p(offsets[1][h] * dist[t, j]) + offsets[2][h])))
+                else:
+                    s = cap * np.tanh(s / cap) if cap else s
+                    p = np.exp(s - s.max())
+                    p = p / p.sum()
+                o.append(p @ V[j, g])
+            if maps == 2:
+                o = [o[0] - np.float32(0.4) * o[1]]
+                o[0] = o[0] / np.sqrt((o[0] ** 2).mean() + 1e-5) * 0.7
+            out[t, h] = o[0]
+    return out
+
+
+@pytest.mark.parametrize("kind,cap,window,keep", [("soft", 0.0, 0, 0), ("soft", 30.0, 50, 3), ("diff", 0.0, 0, 0), ("diff", 30.0, 0, 0), ("sigmoid", 0.0, 0, 0), ("sigmoid", 0.0, 40, 0)])
+@pytest.mark.parametrize("where", ["query", "key", "value"])
+def test_infinities_as_plain_arithmetic_has_them(gpu, kind, cap, window, keep, where):
+    H, G, D, Dv, T, pos, maps = 6, 2, 48, 80, 45, 30, 2 if kind == "diff" else 1
+    r, q, K, V, cache, table, pos0 = inputs(gpu, BF16, H, G, D, Dv, maps, pos, T, 64, 7, 0.3)
+    K, V = K.copy(), V.copy()
+    offsets = np.float32([r.uniform(0.2, 1.0, H), r.uniform(0.1, 1.5, H), r.uniform(-2.5, 0.0, H)])
+    ld = int(gpu.cuda_lib().ggb_window_cache_ld(G, D * maps, Dv))
+    raw, tab = cache.download(np.uint16).reshape(-1, ld), table.download(np.int32)
+    q[5, 1, 0, 3] = np.float32(1.5)  # a query number whose second and third parts are zero
+    for at, c, v in [(1, 3, np.inf), (pos + 7, 9, -np.inf), (pos + 33, 3, np.inf)]:  # first page, inside the portion
+        slot = tab[at // 64] * 64 + at % 64
+        if where == "key":
+            K[at, 1, 0, c] = v
+            raw[slot, maps * D + c] = 0x7f80 if v > 0 else 0xff80
+        elif where == "value":
+            V[at, 0, c] = v
+            raw[slot, G * maps * D + c] = 0x7f80 if v > 0 else 0xff80
+        elif at >= pos:
+            q[at - pos, 4, 0, c] = v
+    cache.upload(raw)
+    vis = seen(pos, T, window, keep, 0)
+    dist = np.maximum(np.arange(pos, pos + T)[:, None] - np.arange(pos + T)[None], 0)
+    got = attend(gpu, kind, q, cache, table, pos0, T, pos, H, G, D, Dv, cap, window, keep, offsets=offsets)
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = plain_heads(kind, q, K, V, vis, cap, offsets.astype(np.float64), dist)
+    assert np.isfinite(want).any() and (np.isnan(got) == np.isnan(want)).all() and (got[np.isinf(want)] == want[np.isinf(want)]).all()
+    ok = np.isfinite(want)
+    assert np.isfinite(got[ok]).all() and rel(got[ok], want[ok]) < LIMIT
