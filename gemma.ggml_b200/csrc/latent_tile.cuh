@@ -15,6 +15,9 @@
 // of a tile wait for its last scores.  1024 tokens x 16 heads at position 1024, R = 512, Dr = 64: 245 us, 228 TFLOP/s of the products asked
 // for (3420 us on the fp32 CUDA cores, two tokens a CTA); from 9 tokens on: fewer are steps, which spread their positions over warps.
 //
+// Infinite numbers are not the sums of their parts: a row (of a CTA) or an output whose sums are not finite is computed once more by fp32
+// multiply-adds over what it sees (plain_part, plain_out), as tile_attention.cuh does.
+//
 // latent_out_kernel.  out = W_uv (sum of the parts): 128 tokens of one head, the merged fp32 rows converted in blocks of 64 (244 -> 28 us
 // for the 1024 tokens above, bound by reading the parts).
 #pragma once
@@ -29,7 +32,7 @@ constexpr int kWarps = 8, kThreads = 32 * (kWarps + 1);
 constexpr uint32_t kPart = kRows * 128;         // one bf16 part of a left operand: 128 rows of 64 numbers
 constexpr uint32_t kLeft = 3 * kPart, kRight = kKeys * 128;
 constexpr uint32_t kTiles = 2 * kLeft + 4 * kRight;
-constexpr size_t kSmem = 1024 + kTiles + 256 + 2 * kRows * 4;
+constexpr size_t kSmem = 1024 + kTiles + 256 + 3 * kRows * 4;
 enum { FULL = 0, FREE = 16, S_FULL = 32, SLOT = 64, DEAD = 72 };
 
 struct args {
@@ -74,6 +77,48 @@ __device__ __forceinline__ void mma_block(uint32_t d, uint32_t a_lo, uint32_t b_
                 umma_ss(d, a_lo + part * (kPart >> 4) + 2 * k, b_lo + k * b_step, idesc, acc);
                 acc = 1;
             }
+}
+
+struct row_job {
+    const float *q;
+    const __nv_bfloat16 *cache;
+    int64_t ld;
+    const int32_t *table;
+    int B;
+    int64_t lo, i, jlo; // the row sees [lo, i]; tiles count from jlo
+    int split, n_split, QK, v0, Vp;
+};
+// one row's part by one warp, a position a lane: weighted sums to out[Vp], maximum and denominator to m and l
+__device__ __noinline__ void plain_part(const row_job &j, float *out, float &m, float &l) {
+    const int lane = threadIdx.x & 31;
+    float acc[8]; // Vp <= 256
+    for (int r = 0; r < 8; r++) acc[r] = 0.f;
+    m = -INFINITY, l = 0.f;
+    for (int64_t j0 = j.jlo + (int64_t)kKeys * j.split; j0 <= j.i; j0 += (int64_t)kKeys * j.n_split)
+        for (int n0 = 0; n0 < kKeys; n0 += 32) {
+            const int64_t at = min(max(j0 + n0 + lane, j.lo), j.i);
+            const bool vis = at == j0 + n0 + lane;
+            const uint32_t seen = __ballot_sync(0xffffffffu, vis);
+            if (!seen) continue;
+            const int64_t row = ((int64_t)j.table[at / j.B] * j.B + at % j.B) * j.ld;
+            float s = 0.f, p = 0.f;
+            for (int d = 0; d < j.QK; d++) s = fmaf(to_f32(j.cache[row + d]), j.q[d], s);
+            const float mx = fmaxf(m, warp_max_f32(vis ? s : -INFINITY)), corr = mx == -INFINITY ? 1.f : expf(m - mx);
+            if (vis && s != -INFINITY) p = expf(s - mx);
+            l = fmaf(l, corr, warp_sum_f32(p));
+            for (int r = 0; r < 8; r++) acc[r] *= corr;
+            m = mx;
+            for (int u = 0; u < 32; u++) {
+                if (!(seen >> u & 1)) continue;
+                const float pu = __shfl_sync(0xffffffffu, p, u);
+                const __nv_bfloat16 *v = j.cache + __shfl_sync(0xffffffffu, row, u) + j.v0;
+                for (int r = 0; r < 8; r++)
+                    if (lane + 32 * r < j.Vp) acc[r] = fmaf(pu, to_f32(v[lane + 32 * r]), acc[r]);
+            }
+        }
+    for (int r = 0; r < 8; r++)
+        if (lane + 32 * r < j.Vp) out[lane + 32 * r] = acc[r];
+    __syncwarp();
 }
 
 __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) {
@@ -304,21 +349,52 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
         }
         mxs[grp * kRows + r] = l;
         bar_sync(1, 32 * kWarps);
-        const float f = m == -INFINITY ? 0.f : expf(m - m_true);
+        const float f = m == -INFINITY ? 0.f : expf(m - m_true), l_row = (mxs[r] + mxs[kRows + r]) * f;
+        float odd = 0.f * l_row; // 0, or NaN when a sum of the row is not finite
+        if (grp == 0) mxs[2 * kRows + r] = l_row - l_row == 0.f ? m_true : NAN; // what this row's sums are relative to, where that is known
+        bar_sync(1, 32 * kWarps);
         float *of = reinterpret_cast<float *>(gbase);
         const int op = a.Vp + 1;
         for (int c = 16 * grp; c < a.Vp; c += 32) {
             uint32_t o[16];
             if (n_mine > 0) tmem_load16(t_o + lanes + c, o);
 #pragma unroll
-            for (int u = 0; u < 16; u++) of[r * op + c + u] = f > 0.f ? __uint_as_float(o[u]) * f : 0.f;
+            for (int u = 0; u < 16; u++) {
+                const float v = f == 0.f ? 0.f : __uint_as_float(o[u]) * f;
+                of[r * op + c + u] = v;
+                odd = fmaf(0.f, v, odd);
+            }
         }
+        mxs[grp * kRows + r] = odd;
         if (grp == 0 && live && blockIdx.z == 0) {
             float *o = a.part + (((int64_t)(t0 + r / a.H) * n_split + split) * a.H + r % a.H) * (a.R + 2);
             o[0] = m_true;
-            o[1] = (mxs[r] + mxs[kRows + r]) * f;
+            o[1] = l_row;
         }
         bar_sync(1, 32 * kWarps);
+        { // a warp's 16 rows: warp, warp + 8, ...; those whose sums are not finite once more, without the split
+            const int er = warp + kWarps * (lane & 15);
+            uint32_t again = __ballot_sync(0xffffffffu, mxs[er] + mxs[kRows + er] != 0.f) & 0xffffu;
+            while (again) {
+                const int p = warp + kWarps * (__ffs((int)again) - 1);
+                again &= again - 1;
+                if (p >= rows) continue;
+                const int64_t pi = i0 + p / a.H;
+                const row_job j{q0 + (int64_t)p * a.QK, a.cache, a.ldk, a.table, a.B, a.window > 0 ? max((int64_t)0, pi - a.window + 1) : 0, pi, jlo, split, n_split, a.QK, v0, a.Vp};
+                float pm, pl;
+                plain_part(j, of + p * op, pm, pl);
+                const float known = mxs[2 * kRows + p];
+                if (known == known) { // the other half of the latent stays relative to this maximum: so does this one
+                    const float g = pm == -INFINITY ? 1.f : expf(pm - known);
+                    for (int c = lane; c < a.Vp; c += 32) of[p * op + c] *= g;
+                } else if (lane == 0 && blockIdx.z == 0) {
+                    float *o = a.part + (((int64_t)(t0 + p / a.H) * n_split + split) * a.H + p % a.H) * (a.R + 2);
+                    o[0] = pm;
+                    o[1] = pl;
+                }
+                __syncwarp();
+            }
+        }
         for (int p = warp; p < rows; p += kWarps) {
             float *o = a.part + (((int64_t)(t0 + p / a.H) * n_split + split) * a.H + p % a.H) * (a.R + 2) + 2 + v0;
             for (int c = lane; c < a.Vp; c += 32) o[c] = of[p * op + c];
@@ -350,6 +426,17 @@ constexpr int kOutSplits = 16;        // parts a row's weights are kept for
 constexpr size_t kOutSmem = 1024 + 2 * (kLeft + kOutW) + 256 + (size_t)kRows * kOutSplits * 4;
 inline bool out_fits(int R, int Dv, int64_t T, int n_split, const void *w_uv, const void *out) {
     return T >= 32 && T < (1 << 24) && R % 16 == 0 && Dv % 16 == 0 && Dv <= 256 && n_split <= kOutSplits && (uintptr_t)w_uv % 16 == 0 && (uintptr_t)out % 4 == 0;
+}
+
+// one output by one thread: w_uv's row against the merged parts (p0, weights wsm, ps numbers from one part to the next)
+__device__ __noinline__ float plain_out(const float *p0, const float *wsm, int ns, int64_t ps, const __nv_bfloat16 *w, int R) {
+    float y = 0.f;
+    for (int d = 0; d < R; d++) {
+        float x = 0.f;
+        for (int s = 0; s < ns; s++) x = fmaf(p0[s * ps + 2 + d], wsm[s], x);
+        y = fmaf(to_f32(w[d]), x, y);
+    }
+    return y;
 }
 
 __global__ void __launch_bounds__(kThreads, 1) latent_out_kernel(const out_args a) {
@@ -435,6 +522,10 @@ __global__ void __launch_bounds__(kThreads, 1) latent_out_kernel(const out_args 
             uint32_t o[16];
             tmem_load16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + c, o);
             if (r < nq) {
+#pragma unroll
+                for (int u = 0; u < 16; u++)
+                    if (!(fabsf(__uint_as_float(o[u])) < INFINITY))
+                        o[u] = __float_as_uint(plain_out(p0 + (int64_t)r * ns * ps, wsm + r * ns, ns, ps, a.w_uv + ((int64_t)h * a.Dv + c + u) * a.R, a.R));
                 uint32_t *dst = reinterpret_cast<uint32_t *>(a.out + ((int64_t)t * a.H + h) * a.Dv + c);
 #pragma unroll
                 for (int u = 0; u < 8; u++) {

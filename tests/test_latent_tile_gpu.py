@@ -54,3 +54,38 @@ def test_parts_and_output(gpu, H, R, Dr, Dv, T, pos, window, ns, page, gate, sca
     o = acc / (e.sum(2, keepdims=True) + np.exp(sink.astype(np.float64)[None, :, None] - m))
     want = np.einsum("thr,hvr->thv", o, w) * (1.0 / (1.0 + np.exp(-g.astype(np.float64)))[..., None] if gate else 1.0)
     assert rel(from_dt(BF16, out, (T, H, Dv)), want) < 2.5e-3
+
+
+@pytest.mark.parametrize("where", ["rotated", "latent", "w_uv", "query", "nan"])
+@pytest.mark.parametrize("H,R,Dr,Dv,T,pos,window,ns", [(5, 320, 48, 32, 40, 20, 0, 2), (4, 128, 16, 48, 33, 500, 300, 1)])
+def test_infinities_as_plain_arithmetic_has_them(gpu, where, H, R, Dr, Dv, T, pos, window, ns):
+    r = np.random.default_rng(R)
+    lib, QK, n, page = gpu.cuda_lib(), R + Dr, pos + T, 64
+    ld, pages = int(lib.ggb_latent_cache_ld(R, Dr)), (n + page - 1) // page
+    table = r.permutation(pages).astype(np.int32)
+    cache, raw = as_dt(BF16, r.standard_normal((pages * page, ld)))
+    at = table[np.arange(n) // page].astype(np.int64) * page + np.arange(n) % page
+    qa, (w, wraw) = f32(r.standard_normal((T, H, QK)) * QK ** -0.5), as_dt(BF16, r.standard_normal((H, Dv, R)) * R ** -0.5)
+    bits = {np.inf: 0x7f80, -np.inf: 0xff80, np.nan: 0x7fc0}
+    for j, c, v in [(pos - 1, R + 3, np.inf), (pos + 30, R + 3, -np.inf)] if where == "rotated" else [(pos + 30, 7, -np.inf)] if where == "latent" else [(pos + 20, 5, np.nan)] if where == "nan" else []:
+        cache[at[j], c], raw[at[j], c] = v, bits[v]
+    if where == "w_uv":
+        w[1, 2, 9], wraw[1, 2, 9] = -np.inf, 0xff80
+    if where == "query":
+        qa[3, 2, R + 1] = np.inf
+    part, out = zeros(gpu, lib.ggb_latent_attn_scratch_bytes(T, H, R, ns)), zeros(gpu, T * H * Dv * 2)
+    gpu.check(lib.ggb_op_latent_attn_window(BF16, dev(gpu, qa).ptr, dev(gpu, raw).ptr, dev(gpu, table).ptr, page, dev(gpu, i32([pos])).ptr, T, H, R, Dr, window, ns, part.ptr), "attn")
+    gpu.check(lib.ggb_op_latent_attn_out_gated(BF16, part.ptr, ns, None, dev(gpu, wraw).ptr, T, H, R, Dv, None, H, out.ptr), "out")
+    want = np.empty((T, H, Dv))
+    with np.errstate(invalid="ignore"):
+        for t in range(T):
+            rows = cache[at[max(0, pos + t - window + 1) if window else 0:pos + t + 1], :QK]
+            for h in range(H):
+                s = rows @ qa[t, h].astype(np.float64)
+                p = np.exp(s - s.max())
+                want[t, h] = w[h] @ ((p / p.sum()) @ rows[:, :R])
+    got = from_dt(BF16, out, (T, H, Dv))
+    assert np.isfinite(want).any() and not np.isfinite(want).all()
+    assert (np.isnan(got) == np.isnan(want)).all() and (got[np.isinf(want)] == want[np.isinf(want)]).all()
+    ok = np.isfinite(want)
+    assert rel(got[ok], want[ok]) < 2.5e-3
