@@ -96,8 +96,10 @@ __device__ __forceinline__ uint4 ldg_stream_u4(const void *p) {
     return r;
 }
 
-// Holds until the kernels before this one are done and their writes are seen: the first statement of a kernel that ggb_launch_step launches,
-// run by every thread.
+// Holds until the kernels before this one are done and their writes are seen: ahead of every access to memory in a kernel that
+// ggb_launch_step launches, run by every thread.  No pointer parameter of such a kernel is __restrict__: what that promises (a const one is
+// not written while the kernel runs, none is reached by another way) does not hold until here, and a compiler that believes it may read
+// through the read-only cache or ahead of this statement.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ float half_bits_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }

@@ -52,8 +52,8 @@ __device__ __forceinline__ void vec_row_dot(const E *__restrict__ wr, const E *_
 
 // ACT: the output is act(.) in the matrices' type (c_act) instead of fp32 (c)
 template <typename E, int TT, int ACT = 0>
-__global__ void __launch_bounds__(256) linear_vec_kernel(const E *__restrict__ w, int64_t N, int64_t K, const E *__restrict__ a,
-                                                         int64_t lda, float *__restrict__ c, int64_t ldc, E *__restrict__ c_act = nullptr) {
+__global__ void __launch_bounds__(256) linear_vec_kernel(const E *w, int64_t N, int64_t K, const E *a,
+                                                         int64_t lda, float *c, int64_t ldc, E *c_act = nullptr) {
     constexpr int VE = 16 / (int)sizeof(E);
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -36,11 +36,11 @@ __device__ __forceinline__ void rot_pair(int m, int dims, int halves, int *i0, i
 // cs: [n_pos][dims / 2][2] (cos, sin) with the rotation's magnitude factor already applied.  blockIdx.y 1: the query latent
 // of the same token instead, cq = rms(dq) * qnw.
 template <typename E>
-__global__ void __launch_bounds__(128) latent_kv_store_kernel(const float *__restrict__ d, int64_t ldd, int R, int Dr, int dims,
-                                                              const float *__restrict__ nw, float eps, const float *__restrict__ cs,
-                                                              const int32_t *__restrict__ pos0, const int32_t *__restrict__ table,
-                                                              int B, E *__restrict__ cache, int64_t ldk, int halves,
-                                                              const float *__restrict__ dq, int Rq, const float *__restrict__ qnw, E *__restrict__ cq) {
+__global__ void __launch_bounds__(128) latent_kv_store_kernel(const float *d, int64_t ldd, int R, int Dr, int dims,
+                                                              const float *nw, float eps, const float *cs,
+                                                              const int32_t *pos0, const int32_t *table,
+                                                              int B, E *cache, int64_t ldk, int halves,
+                                                              const float *dq, int Rq, const float *qnw, E *cq) {
     step_wait();
     __shared__ float red[4];
     const int t = blockIdx.x, tid = threadIdx.x;
@@ -85,9 +85,9 @@ __global__ void __launch_bounds__(128) latent_kv_store_kernel(const float *__res
 // D terms (loads of a group are independent and in flight together) and the quarters are added in a fixed order.
 constexpr int kAbsT = 8;
 template <typename E>
-__global__ void __launch_bounds__(256) latent_q_absorb_kernel(const float *__restrict__ q, int64_t ldq, int64_t T, int H, int D, int Dr,
-                                                              int dims, const float *__restrict__ cs, const int32_t *__restrict__ pos0,
-                                                              const E *__restrict__ w_uk, int R, float scale, float *__restrict__ qa,
+__global__ void __launch_bounds__(256) latent_q_absorb_kernel(const float *q, int64_t ldq, int64_t T, int H, int D, int Dr,
+                                                              int dims, const float *cs, const int32_t *pos0,
+                                                              const E *w_uk, int R, float scale, float *qa,
                                                               int halves) {
     step_wait();
     extern __shared__ float qs[]; // [kAbsT][D], then [4][kAbsT][64] partial sums
@@ -215,10 +215,10 @@ template <> struct TileWord<__nv_bfloat16> {
 };
 
 template <typename E, int RC, int TQ>
-__global__ void __launch_bounds__(512) latent_attn_partial_kernel(const float *__restrict__ qa, const E *__restrict__ cache, int64_t ldk,
-                                                                  const int32_t *__restrict__ table, int B, const int32_t *__restrict__ pos0,
+__global__ void __launch_bounds__(512) latent_attn_partial_kernel(const float *qa, const E *cache, int64_t ldk,
+                                                                  const int32_t *table, int B, const int32_t *pos0,
                                                                   int T, int H, int R, int Dr, int n_split, int SW, int hpc,
-                                                                  int64_t window, float *__restrict__ part) {
+                                                                  int64_t window, float *part) {
     step_wait();
     // TQ consecutive tokens per CTA (portions): a warp scores and accumulates its head for all of them from ONE read of
     // every tile word; the later token's extra position is masked for the earlier one.
@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(512) latent_attn_partial_kernel(const float *_
 // ---- merge the splits with the sink, then out[t][h] = W_uv_h (sum_j p_j c_j).  kOutT tokens of one head per CTA.
 constexpr int kOutT = 8; // tokens of one head per CTA; v_chunk outputs per CTA (every CTA of a head repeats the merge)
 template <typename E>
-__global__ void __launch_bounds__(256) latent_attn_out_kernel(const float *__restrict__ part, int n_split, const float *__restrict__ sink,
-                                                              const E *__restrict__ w_uv, int64_t T, int H, int R, int Dv,
-                                                              int v_chunk, const float *__restrict__ gate, int64_t ldg, E *__restrict__ out) {
+__global__ void __launch_bounds__(256) latent_attn_out_kernel(const float *part, int n_split, const float *sink,
+                                                              const E *w_uv, int64_t T, int H, int R, int Dv,
+                                                              int v_chunk, const float *gate, int64_t ldg, E *out) {
     step_wait();
     extern __shared__ __align__(16) float ol[]; // [kOutT][R]
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

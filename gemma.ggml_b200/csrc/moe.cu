@@ -37,8 +37,8 @@ __device__ __forceinline__ float router_dot(const E *__restrict__ hr, const floa
 
 // router logits: a warp per (token, expert), z[t][e] = w[e] . h[t] + b[e] in fp32
 template <typename E>
-__global__ void __launch_bounds__(256) moe_logits_kernel(const E *__restrict__ h, int64_t W, int64_t T, const float *__restrict__ w,
-                                                         const float *__restrict__ b, int n_exp, float *__restrict__ z) {
+__global__ void __launch_bounds__(256) moe_logits_kernel(const E *h, int64_t W, int64_t T, const float *w,
+                                                         const float *b, int n_exp, float *z) {
     step_wait();
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(256) moe_logits_kernel(const E *__restrict__ h
 }
 
 // one warp per token: `top` rounds of arg-max over its logits (ties: the lower index), soft-max over the chosen
-__global__ void __launch_bounds__(32) moe_select_kernel(const float *__restrict__ zg, int n_exp, int top, int32_t *__restrict__ idx,
-                                                        float *__restrict__ wt) {
+__global__ void __launch_bounds__(32) moe_select_kernel(const float *zg, int n_exp, int top, int32_t *idx,
+                                                        float *wt) {
     step_wait();
     extern __shared__ float z[]; // [n_exp] logits, then [top] chosen values
     float *sel = z + n_exp;
@@ -212,8 +212,8 @@ __device__ __forceinline__ void select_softmax_warp(float *sc, float *ch, float 
     }
 }
 
-__global__ void __launch_bounds__(32) moe_select_softmax_kernel(const float *__restrict__ zg, int64_t ldz, const float *__restrict__ corr, int n_exp, int top,
-                                                                int n_groups, int keep, float scale, int32_t *__restrict__ idx, float *__restrict__ wt) {
+__global__ void __launch_bounds__(32) moe_select_softmax_kernel(const float *zg, int64_t ldz, const float *corr, int n_exp, int top,
+                                                                int n_groups, int keep, float scale, int32_t *idx, float *wt) {
     step_wait();
     extern __shared__ float sm[]; // [n_exp] scores, [n_exp] choice scores, [n_groups] group scores
     for (int e = threadIdx.x; e < n_exp; e += 32) sm[e] = zg[(int64_t)blockIdx.x * ldz + e];
@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(32) moe_select_softmax_kernel(const float *__r
     select_softmax_warp(sm, sm + n_exp, sm + 2 * n_exp, corr, n_exp, top, n_groups, keep, scale, blockIdx.x, threadIdx.x, idx, wt);
 }
 
-__global__ void __launch_bounds__(32) moe_select_sigmoid_kernel(const float *__restrict__ zg, const float *__restrict__ corr, int n_exp, int top,
-                                                                int n_groups, int keep, int32_t *__restrict__ idx, float *__restrict__ wt) {
+__global__ void __launch_bounds__(32) moe_select_sigmoid_kernel(const float *zg, const float *corr, int n_exp, int top,
+                                                                int n_groups, int keep, int32_t *idx, float *wt) {
     step_wait();
     extern __shared__ float sm[]; // [n_exp] scores, [n_exp] choice scores, [n_groups] group scores
     for (int e = threadIdx.x; e < n_exp; e += 32) sm[e] = zg[(int64_t)blockIdx.x * n_exp + e];
@@ -240,11 +240,11 @@ constexpr int kRouteStepTokens = 32, kRouteStepWarps = 8;
 __device__ unsigned int g_route_done[kRouteStepTokens];
 
 template <typename E, bool SOFTMAX>
-__global__ void __launch_bounds__(32 * kRouteStepWarps) moe_route_sigmoid_step_kernel(const E *__restrict__ h, int64_t W, const float *__restrict__ w,
-                                                                     const float *__restrict__ corr, int n_exp, int n_extra, int top, int n_groups, int keep,
-                                                                     float scale, float *zg, int32_t *__restrict__ idx, float *__restrict__ wt,
-                                                                     int32_t *__restrict__ row_src, int32_t *__restrict__ inv,
-                                                                     int32_t *__restrict__ row_expert) {
+__global__ void __launch_bounds__(32 * kRouteStepWarps) moe_route_sigmoid_step_kernel(const E *h, int64_t W, const float *w,
+                                                                     const float *corr, int n_exp, int n_extra, int top, int n_groups, int keep,
+                                                                     float scale, float *zg, int32_t *idx, float *wt,
+                                                                     int32_t *row_src, int32_t *inv,
+                                                                     int32_t *row_expert) {
     step_wait();
     extern __shared__ float sm[];
     __shared__ bool last;
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(32 * kRouteStepWarps) moe_route_sigmoid_step_k
 
 // one CTA: counts per expert, offsets, the list of 64-row tiles, and the sorted order of the n = T * top slots
 // experts n_real .. n_exp - 1 have no matrices (identity experts): their slots are sorted like the others but get no tile
-__global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t *__restrict__ idx, int n, int top, int n_exp, int n_real, int32_t *offsets,
+__global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t *idx, int n, int top, int n_exp, int n_real, int32_t *offsets,
                                                          int32_t *row_src, int32_t *inv, int32_t *tile_expert, int32_t *tile_row0,
                                                          int32_t *n_tiles, int32_t *row_expert) {
     step_wait();
@@ -318,9 +318,9 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t *__restri
 
 // few slots (decode): a warp per (sorted row, output) streams the expert's weight row with 16-byte loads
 template <typename E, int ACT>
-__global__ void __launch_bounds__(256) moe_vec_kernel(const E *__restrict__ w, int64_t N, int64_t K, const E *__restrict__ a, int64_t lda,
-                                                      const int32_t *__restrict__ row_src, const int32_t *__restrict__ row_expert,
-                                                      float *__restrict__ c, E *__restrict__ c_act, int64_t ldc, int vec, int n_real, float limit,
+__global__ void __launch_bounds__(256) moe_vec_kernel(const E *w, int64_t N, int64_t K, const E *a, int64_t lda,
+                                                      const int32_t *row_src, const int32_t *row_expert,
+                                                      float *c, E *c_act, int64_t ldc, int vec, int n_real, float limit,
                                                       float alpha) {
     step_wait();
     constexpr int VE = 16 / (int)sizeof(E);
@@ -379,9 +379,9 @@ template <typename E> struct shared_product {
     int vec;
 };
 template <typename E, int ACT>
-__global__ void __launch_bounds__(256) moe_vec_shared_kernel(const E *__restrict__ w, int64_t N, int64_t K, const E *__restrict__ a, int64_t lda,
-                                                             const int32_t *__restrict__ row_src, const int32_t *__restrict__ row_expert,
-                                                             float *__restrict__ c, E *__restrict__ c_act, int64_t ldc, int vec, int n_slots,
+__global__ void __launch_bounds__(256) moe_vec_shared_kernel(const E *w, int64_t N, int64_t K, const E *a, int64_t lda,
+                                                             const int32_t *row_src, const int32_t *row_expert,
+                                                             float *c, E *c_act, int64_t ldc, int vec, int n_slots,
                                                              shared_product<E> sh) {
     step_wait();
     constexpr int VE = 16 / (int)sizeof(E);
@@ -419,14 +419,14 @@ __global__ void __launch_bounds__(256) moe_vec_shared_kernel(const E *__restrict
 }
 
 // rows of A in sorted-slot order (the tensor-core product reads its operand contiguously): y[i] = a[row_src[i]], 16 bytes a thread
-__global__ void moe_gather_kernel(const uint4 *__restrict__ a, int64_t row_u4, const int32_t *__restrict__ row_src, uint4 *__restrict__ y) {
+__global__ void moe_gather_kernel(const uint4 *a, int64_t row_u4, const int32_t *row_src, uint4 *y) {
     step_wait();
     const uint4 *src = a + (int64_t)row_src[blockIdx.x] * row_u4;
     for (int64_t i = threadIdx.x; i < row_u4; i += blockDim.x) y[(int64_t)blockIdx.x * row_u4 + i] = src[i];
 }
 
-__global__ void moe_combine_kernel(const float *__restrict__ y, const int32_t *__restrict__ inv, const float *__restrict__ wt, int top,
-                                   int64_t W, float *__restrict__ out) {
+__global__ void moe_combine_kernel(const float *y, const int32_t *inv, const float *wt, int top,
+                                   int64_t W, float *out) {
     step_wait();
     const int64_t t = blockIdx.x;
     for (int64_t i = threadIdx.x; i < W; i += blockDim.x) {
@@ -438,9 +438,9 @@ __global__ void moe_combine_kernel(const float *__restrict__ y, const int32_t *_
 
 // the same with experts that hand their input through: a slot whose expert is n_real or later adds wt * h[t]
 template <typename E>
-__global__ void moe_combine_identity_kernel(const float *__restrict__ y, const int32_t *__restrict__ inv, const float *__restrict__ wt,
-                                            const int32_t *__restrict__ idx, int top, int n_real, int64_t W, const E *__restrict__ h,
-                                            float *__restrict__ out) {
+__global__ void moe_combine_identity_kernel(const float *y, const int32_t *inv, const float *wt,
+                                            const int32_t *idx, int top, int n_real, int64_t W, const E *h,
+                                            float *out) {
     step_wait();
     const int64_t t = blockIdx.x;
     for (int64_t i = threadIdx.x; i < W; i += blockDim.x) {

@@ -40,11 +40,11 @@ template <typename E> struct RowVec { // 16 bytes of a cache row
 };
 
 template <typename E>
-__global__ void __launch_bounds__(256) sigmoid_qkv_store_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
+__global__ void __launch_bounds__(256) sigmoid_qkv_store_kernel(const float *q, const float *k, const float *v,
                                                                 int64_t ld, int H, int G, int D, int Dv, float temp_coef, int temp_every,
-                                                                float vnorm_eps, float scale, const int32_t *__restrict__ pos0,
-                                                                const int32_t *__restrict__ table, int B, E *__restrict__ cache, int64_t cache_ld,
-                                                                float *__restrict__ q_out) {
+                                                                float vnorm_eps, float scale, const int32_t *pos0,
+                                                                const int32_t *table, int B, E *cache, int64_t cache_ld,
+                                                                float *q_out) {
     step_wait();
     const int64_t t = blockIdx.x;
     const int64_t pos = (int64_t)*pos0 + t;
@@ -69,11 +69,11 @@ __global__ void __launch_bounds__(256) sigmoid_qkv_store_kernel(const float *__r
 
 // ---- steps of few tokens: CTA (token, head, split); its warps take the key tiles split * 8 + warp modulo 8 * splits
 template <typename E>
-__global__ void __launch_bounds__(32 * kWarps) sigmoid_attn_step_kernel(const float *__restrict__ q, const E *__restrict__ cache, int64_t cache_ld,
-                                                                        const int32_t *__restrict__ table, int B, const int32_t *__restrict__ pos0,
-                                                                        int H, int G, int D, int Dv, int64_t window, const float *__restrict__ r1,
-                                                                        const float *__restrict__ r2, const float *__restrict__ pb,
-                                                                        E *__restrict__ out, int vec, float *__restrict__ part_out) {
+__global__ void __launch_bounds__(32 * kWarps) sigmoid_attn_step_kernel(const float *q, const E *cache, int64_t cache_ld,
+                                                                        const int32_t *table, int B, const int32_t *pos0,
+                                                                        int H, int G, int D, int Dv, int64_t window, const float *r1,
+                                                                        const float *r2, const float *pb,
+                                                                        E *out, int vec, float *part_out) {
     step_wait();
     extern __shared__ __align__(16) float sa_smem[]; // q: [kWarps][Dp]; sums: [kWarps][32 * kMaxDvRegs]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(32 * kWarps) sigmoid_attn_step_kernel(const fl
 
 // one warp per (token, head): the splits' sums in split order
 template <typename E>
-__global__ void __launch_bounds__(32) sigmoid_merge_kernel(const float *__restrict__ part, int n_split, int H, int Dv, E *__restrict__ out) {
+__global__ void __launch_bounds__(32) sigmoid_merge_kernel(const float *part, int n_split, int H, int Dv, E *out) {
     step_wait();
     const int64_t t = blockIdx.x;
     const int h = blockIdx.y, lane = threadIdx.x;

@@ -58,12 +58,12 @@ __device__ __forceinline__ int64_t first_visible(int64_t i, int64_t size, int ch
 __device__ __forceinline__ float soft_cap(float s, float cap) { return cap > 0.f ? cap * tanhf(s / cap) : s; }
 
 template <typename E>
-__global__ void __launch_bounds__(256) window_qkv_store_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
-                                                               int64_t ld, int H, int G, int D, int Gv, int Dv, const float *__restrict__ qn_w,
-                                                               const float *__restrict__ kn_w, float eps, int rot_dims, int rot_halves,
-                                                               const float *__restrict__ cs_k, const float *__restrict__ cs_v, float scale,
-                                                               const int32_t *__restrict__ pos0, const int32_t *__restrict__ table, int B,
-                                                               E *__restrict__ cache, int64_t cache_ld, float *__restrict__ q_out) {
+__global__ void __launch_bounds__(256) window_qkv_store_kernel(const float *q, const float *k, const float *v,
+                                                               int64_t ld, int H, int G, int D, int Gv, int Dv, const float *qn_w,
+                                                               const float *kn_w, float eps, int rot_dims, int rot_halves,
+                                                               const float *cs_k, const float *cs_v, float scale,
+                                                               const int32_t *pos0, const int32_t *table, int B,
+                                                               E *cache, int64_t cache_ld, float *q_out) {
     __shared__ float red[2][8];
     step_wait();
     const int64_t t = blockIdx.x;
@@ -145,11 +145,11 @@ __global__ void __launch_bounds__(256) window_qkv_store_kernel(const float *__re
 // the same with a norm per head: a warp takes one head of q, k or v of one token (rows y * 8 + warp of H + 2 G).  q and k are divided
 // by the root mean square over the head's D numbers, times a weight of D numbers that all heads share (null: none), before the rotation.
 template <typename E>
-__global__ void __launch_bounds__(256) head_qkv_store_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v, int64_t ld,
-                                                             int H, int G, int D, int Dv, const float *__restrict__ qn_w, const float *__restrict__ kn_w,
-                                                             float eps, int rot_dims, int rot_halves, const float *__restrict__ cs, float scale,
-                                                             const int32_t *__restrict__ pos0, const int32_t *__restrict__ table, int B,
-                                                             E *__restrict__ cache, int64_t cache_ld, float *__restrict__ q_out) {
+__global__ void __launch_bounds__(256) head_qkv_store_kernel(const float *q, const float *k, const float *v, int64_t ld,
+                                                             int H, int G, int D, int Dv, const float *qn_w, const float *kn_w,
+                                                             float eps, int rot_dims, int rot_halves, const float *cs, float scale,
+                                                             const int32_t *pos0, const int32_t *table, int B,
+                                                             E *cache, int64_t cache_ld, float *q_out) {
     const int lane = threadIdx.x & 31, item = (int)blockIdx.y * 8 + (int)(threadIdx.x >> 5);
     step_wait();
     if (item >= H + 2 * G) return;
@@ -271,11 +271,11 @@ struct key_tiles {
 // split * 8 + warp modulo 8 * splits, one warp a tile.  One split: the result goes to `out`; several: the CTA's merged
 // part goes to `part` and window_merge_kernel finishes.
 template <typename E, int MAPS>
-__global__ void __launch_bounds__(32 * kWarps) window_attn_kernel(const float *__restrict__ q, const E *__restrict__ cache, int64_t cache_ld,
-                                                                  const int32_t *__restrict__ table, int B, const int32_t *__restrict__ pos0,
+__global__ void __launch_bounds__(32 * kWarps) window_attn_kernel(const float *q, const E *cache, int64_t cache_ld,
+                                                                  const int32_t *table, int B, const int32_t *pos0,
                                                                   int64_t T, int H, int G, int D, int Dv, int64_t window, int chunked, int64_t keep,
-                                                                  float cap, const float *__restrict__ cs_v, finish_args da, E *__restrict__ out,
-                                                                  int vec, float *__restrict__ part_out) {
+                                                                  float cap, const float *cs_v, finish_args da, E *out,
+                                                                  int vec, float *part_out) {
     extern __shared__ __align__(16) float wa_smem[]; // q: [kWarps][MAPS][Dp]; merge: [kWarps][MAPS][kPartW]
     step_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -441,8 +441,8 @@ __global__ void __launch_bounds__(32 * kWarps) window_attn_kernel(const float *_
 
 // one warp per (token, head): the splits' parts merged, then as above
 template <typename E, int MAPS>
-__global__ void __launch_bounds__(32) window_merge_kernel(const float *__restrict__ part, int n_split, const int32_t *__restrict__ pos0, int H, int Dv,
-                                                         const float *__restrict__ cs_v, finish_args da, E *__restrict__ out) {
+__global__ void __launch_bounds__(32) window_merge_kernel(const float *part, int n_split, const int32_t *pos0, int H, int Dv,
+                                                         const float *cs_v, finish_args da, E *out) {
     const int64_t t = blockIdx.x;
     const int h = blockIdx.y, lane = threadIdx.x;
     constexpr int pw = MAPS * kPartW;

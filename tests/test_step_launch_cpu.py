@@ -1,0 +1,54 @@
+"""Kernels that are launched before the one ahead of them has ended: every one of them waits (step_wait) before it touches memory, and no
+pointer parameter promises the compiler that its memory is not written meanwhile (__restrict__), which would let it read early."""
+import glob
+import os
+import re
+
+import gemma_ggml_b200 as G
+
+CSRC = os.path.join(os.path.dirname(G.CUDA_LIB), "csrc")
+
+
+def kernels():
+    """(file, name) -> (parameter list, body) of every __global__ function"""
+    out = {}
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        s = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", s):
+            i = s.index("{", m.start())
+            depth, k = 0, i
+            while True:
+                depth += {"{": 1, "}": -1}.get(s[k], 0)
+                if depth == 0:
+                    break
+                k += 1
+            sig = re.sub(r"__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)", "", s[m.start():i])
+            name = re.search(r"(\w+)\s*\(", sig).group(1)
+            out[path, name] = (sig, s[i + 1:k])
+    return out
+
+
+def launched():
+    names = set()
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):
+        s = open(path).read()
+        for m in re.finditer(r"ggb_launch_step\(\s*(\w+)", s):
+            name = m.group(1)
+            if name == "k":  # a variable
+                name = re.findall(r"auto k = (\w+)", s[:m.start()])[-1]
+            names.add((path, name))
+    return names
+
+
+def test_every_early_launched_kernel_waits_before_it_touches_memory():
+    ks, names = kernels(), launched()
+    waiting = {n for n, (_, body) in ks.items() if "step_wait()" in body}
+    assert len(names) > 15 and names == waiting
+    for n in names:
+        ahead = re.sub(r"(extern )?__shared__[^;]*;", "", ks[n][1].split("step_wait()")[0])
+        assert not re.search(r"\[|->|[=(,]\s*\*\s*\w|\b(if|return|for|while)\b", ahead), (n, ahead)
+
+
+def test_no_pointer_of_theirs_is_restrict():
+    ks = kernels()
+    assert not [n for n in launched() if "__restrict__" in ks[n][0]]
