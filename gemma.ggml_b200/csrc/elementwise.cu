@@ -514,8 +514,10 @@ int ggb_op_sample_from_candidates(const void *cands, int n_cands, int32_t *state
 int ggb_op_argmax(const float *x, int64_t n, int32_t *out) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(x && out && n > 0, "bad argmax args");
-    static Cand *scratch = nullptr; // small, lives for the process
-    if (!scratch) GGB_CUDA(cudaMalloc(&scratch, sizeof(Cand) * kArgmaxParts));
+    void *ws;
+    const int rc = ggb_workspace(GGB_WS_ARGMAX, sizeof(Cand) * kArgmaxParts, &ws);
+    if (rc) return rc;
+    Cand *scratch = (Cand *)ws;
     argmax_stage1<<<kArgmaxParts, 256, 0, ggb_cuda_stream()>>>(x, n, scratch);
     GGB_LAUNCH_CHECK();
     argmax_stage2<<<1, 256, 0, ggb_cuda_stream()>>>(scratch, kArgmaxParts, out, nullptr, nullptr);

@@ -405,26 +405,13 @@ __global__ void splits_add_kernel(const float *__restrict__ ws, int splits, int6
     }
 }
 
-int allow_smem() { // once a process: a call's host time is launch and tensor maps
-    static const cudaError_t e = [] {
-        cudaError_t r = cudaSuccess;
-        for (auto k : {gemm_tma_kernel<256>, gemm_tma_kernel<128>, gemm_pair_kernel<2>, gemm_pair_kernel<1>}) {
-            const cudaError_t x = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
-            if (x != cudaSuccess) r = x;
-        }
-        return r;
-    }();
-    GGB_CUDA(e);
-    return GGB_OK;
-}
-
 int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int MT, const gemm_args &g, int pairs) {
     CUtensorMap ma, mw;
-    int rc = allow_smem();
+    auto kfn = MT == 2 ? gemm_pair_kernel<2> : gemm_pair_kernel<1>;
+    int rc = ggb_allow_smem(kfn, kSmem);
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, MT * 128);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, 128);
     if (rc) return rc;
-    auto kfn = MT == 2 ? gemm_pair_kernel<2> : gemm_pair_kernel<1>;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(2 * std::min(pairs, ggb_sm_count() / 2)));
     cfg.blockDim = dim3(kThreads);
@@ -441,11 +428,11 @@ int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t
 
 int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int BM, const gemm_args &g, int ctas) {
     CUtensorMap ma, mw;
-    int rc = allow_smem();
+    auto kfn = BM == 256 ? gemm_tma_kernel<256> : gemm_tma_kernel<128>;
+    int rc = ggb_allow_smem(kfn, kSmem);
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
-    auto kfn = BM == 256 ? gemm_tma_kernel<256> : gemm_tma_kernel<128>;
     kfn<<<std::min(ctas, ggb_sm_count()), kThreads, kSmem, ggb_cuda_stream()>>>(ma, mw, g);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -485,7 +472,7 @@ bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc) {
     return T >= 64 && K % 64 == 0 && N % 32 == 0 && ldc % 4 == 0 && N < (1ll << 31) && K < (1ll << 31) && T < (1ll << 31);
 }
 
-// The K-split workspace belongs to the library and only grows (one stream, no capture: products of 64 rows and more).
+// The K-split workspace only grows (one stream, no capture: products of 64 rows and more).
 int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(w && a && (c || c_act) && ((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
@@ -520,16 +507,10 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
                 g.BN = sh.bn, g.n_tiles = (int)n_tiles, g.m_tiles = (int)m_tiles, g.chunks = chunks, g.chunk_kb = chunk_kb, g.splits = splits;
             }
         }
-    static void *ws = nullptr;
-    static size_t ws_bytes = 0;
     if (g.splits > 1) {
-        const size_t need = (size_t)g.splits * (size_t)T * (size_t)N * 4;
-        if (need > ws_bytes) {
-            if (ws) cudaFree(ws);
-            ws = nullptr, ws_bytes = 0;
-            GGB_CUDA(cudaMalloc(&ws, need));
-            ws_bytes = need;
-        }
+        void *ws;
+        const int e = ggb_workspace(GGB_WS_GEMM_SPLITS, (size_t)g.splits * (size_t)T * (size_t)N * 4, &ws);
+        if (e) return e;
         g.ws = (float *)ws;
     }
     g.T = (int)T, g.N = (int)N, g.kblocks = kblocks, g.stages = stages_of(BM, g.BN);

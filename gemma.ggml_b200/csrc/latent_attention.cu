@@ -698,7 +698,8 @@ int ggb_op_latent_attn_window(int dt, const float *qa, const void *cache, const 
     if (dt == GGB_TYPE_BF16 && latent_tile::fits(R, Dr, H, T, qa, cache)) {
         const int vp = R <= 256 ? R : R / 2, tq = latent_tile::kRows / H;
         const latent_tile::args a{qa, (const __nv_bfloat16 *)cache, ldk, block_table, block_size, pos0, (int)T, H, R, R + Dr, vp, window, part, ggb_wait_error_flag()};
-        GGB_CUDA(cudaFuncSetAttribute(latent_tile::latent_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)latent_tile::kSmem));
+        const int rc = ggb_allow_smem(latent_tile::latent_tile_kernel, latent_tile::kSmem);
+        if (rc) return rc;
         latent_tile::latent_tile_kernel<<<dim3((unsigned)((T + tq - 1) / tq), (unsigned)n_split, (unsigned)(R / vp)), latent_tile::kThreads, latent_tile::kSmem,
                                           ggb_cuda_stream()>>>(a);
         GGB_LAUNCH_CHECK();
@@ -722,7 +723,8 @@ int ggb_op_latent_attn_out_gated(int dt, const float *part, int n_split, const f
     GGB_CHECK_ARG((!gate || ldg >= H) && part && w_uv && out && T > 0 && H > 0 && R > 0 && Dv > 0 && n_split > 0, "latent_attn_out: bad arguments");
     if (dt == GGB_TYPE_BF16 && latent_tile::out_fits(R, Dv, T, n_split, w_uv, out)) {
         const latent_tile::out_args a{part, n_split, sink, (const __nv_bfloat16 *)w_uv, (int)T, H, R, Dv, gate, ldg, (__nv_bfloat16 *)out, ggb_wait_error_flag()};
-        GGB_CUDA(cudaFuncSetAttribute(latent_tile::latent_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)latent_tile::kOutSmem));
+        const int rc = ggb_allow_smem(latent_tile::latent_out_kernel, latent_tile::kOutSmem);
+        if (rc) return rc;
         latent_tile::latent_out_kernel<<<dim3((unsigned)((T + latent_tile::kRows - 1) / latent_tile::kRows), (unsigned)H), latent_tile::kThreads, latent_tile::kOutSmem,
                                          ggb_cuda_stream()>>>(a);
         GGB_LAUNCH_CHECK();

@@ -621,15 +621,9 @@ int ggb_op_moe_linear_identity(int dt, const void *w, int64_t N, int64_t K, cons
         const int64_t n = T * top;
         const void *a_sorted = a;
         if (gather) {
-            static void *gbuf = nullptr;
-            static size_t gbytes = 0;
-            const size_t need = (size_t)n * (size_t)K * 2;
-            if (need > gbytes) {
-                if (gbuf) cudaFree(gbuf);
-                gbuf = nullptr, gbytes = 0;
-                GGB_CUDA(cudaMalloc(&gbuf, need));
-                gbytes = need;
-            }
+            void *gbuf;
+            const int rc = ggb_workspace(GGB_WS_MOE_GATHER, (size_t)n * (size_t)K * 2, &gbuf);
+            if (rc) return rc;
             ggb_launch_step(moe_gather_kernel, dim3((unsigned)n), dim3(128), 0, (const uint4 *)a, K / 8, g.row_src, (uint4 *)gbuf);
             GGB_LAUNCH_CHECK();
             a_sorted = gbuf;

@@ -809,18 +809,10 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     int rc = ggb_tensor_map_bf16(&maps.a, a_bf16, T, K, K, A.MT * 128);
     for (int i = 0; i < n && !rc; i++) rc = ggb_tensor_map_bytes(&maps.w[i], w[i]->qs, w[i]->rows, K / 32 * pb, 2 * pb, br);
     if (rc) return rc;
-    static const cudaError_t allowed = [] {
-        cudaError_t r = cudaSuccess;
-        for (auto k : {gemm_quant_kernel<GGB_TYPE_Q4_0, true>, gemm_quant_kernel<GGB_TYPE_Q8_0, true>, gemm_quant_kernel<GGB_TYPE_Q4_0, false>, gemm_quant_kernel<GGB_TYPE_Q8_0, false>}) {
-            const cudaError_t x = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
-            if (x != cudaSuccess) r = x;
-        }
-        return r;
-    }();
-    GGB_CUDA(allowed);
     const bool q4 = type == GGB_TYPE_Q4_0;
     auto kfn = pair ? (q4 ? gemm_quant_kernel<GGB_TYPE_Q4_0, true> : gemm_quant_kernel<GGB_TYPE_Q8_0, true>)
                     : (q4 ? gemm_quant_kernel<GGB_TYPE_Q4_0, false> : gemm_quant_kernel<GGB_TYPE_Q8_0, false>);
+    if ((rc = ggb_allow_smem(kfn, kGemmSmem))) return rc;
     // row tiles first: those that share a piece of W run together
     const int rows = A.MT * (pair ? 256 : 128);
     cudaLaunchConfig_t cfg{};

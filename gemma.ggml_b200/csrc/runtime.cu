@@ -39,6 +39,9 @@ struct Context {
     int64_t capture_launches = 0;
     bool prof_on = false;
     std::map<std::string, ProfEntry> prof;
+    void *ws[GGB_WS_COUNT] = {};
+    size_t ws_bytes[GGB_WS_COUNT] = {};
+    std::map<const void *, size_t> smem_allowed;
 };
 
 Context g_ctx;
@@ -68,6 +71,28 @@ void ggb_count_launch(int n) {
 const uint16_t *ggb_exp_table_dev() { return g_ctx.exp_table; }
 const uint16_t *ggb_gelu_table_dev() { return g_ctx.gelu_table; }
 int *ggb_wait_error_flag() { return g_ctx.wait_error; }
+int ggb_workspace(ggb_workspace_id id, size_t bytes, void **p) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    if (bytes > g_ctx.ws_bytes[id]) {
+        cudaFree(g_ctx.ws[id]);
+        g_ctx.ws[id] = nullptr, g_ctx.ws_bytes[id] = 0;
+        GGB_CUDA(cudaMalloc(&g_ctx.ws[id], bytes));
+        g_ctx.ws_bytes[id] = bytes;
+    }
+    *p = g_ctx.ws[id];
+    return GGB_OK;
+}
+int ggb_allow_smem_of(const void *kernel, size_t bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    size_t &allowed = g_ctx.smem_allowed[kernel];
+    if (bytes > allowed) {
+        GGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        allowed = bytes;
+    }
+    return GGB_OK;
+}
 size_t ggb_tables_bytes() { return 2 * 65536 * 2; } // exp then gelu, contiguous from ggb_exp_table_dev()
 const float *ggb_rope_cos_dev() { return g_ctx.rope_cos; }
 const float *ggb_rope_sin_dev() { return g_ctx.rope_sin; }
@@ -143,6 +168,7 @@ int ggb_shutdown(void) {
     cudaFree(g_ctx.rope_cos);
     cudaFree(g_ctx.rope_sin);
     cudaFreeHost(g_ctx.wait_error);
+    for (void *w : g_ctx.ws) cudaFree(w);
     for (auto &kv : g_ctx.prof) {
         for (auto &p : kv.second.pending) {
             cudaEventDestroy(p.first);

@@ -550,7 +550,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const 
 template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin, cudaStream_t st) {
     const size_t smem = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G);
     auto kfn = attn_kernel<MODE, MAPS, FIN>;
-    GGB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rc = ggb_allow_smem(kfn, smem);
+    if (rc) return rc;
     const int TQ = kRows / MAPS / (a.H / a.G);
     kfn<<<dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), kThreads, smem, st>>>(a, fin);
     GGB_LAUNCH_CHECK();
