@@ -507,12 +507,13 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
                 g.BN = sh.bn, g.n_tiles = (int)n_tiles, g.m_tiles = (int)m_tiles, g.chunks = chunks, g.chunk_kb = chunk_kb, g.splits = splits;
             }
         }
-    if (g.splits > 1) {
-        void *ws;
-        const int e = ggb_workspace(GGB_WS_GEMM_SPLITS, (size_t)g.splits * (size_t)T * (size_t)N * 4, &ws);
+    // sized by T and N alone, for every product that some K would cut: where one of them has run, a captured one allocates nothing
+    void *ws = nullptr;
+    if (big * 2 <= sms) {
+        const int e = ggb_workspace(GGB_WS_GEMM_SPLITS, ggb_gemm_workspace_bytes(T, N, K), &ws);
         if (e) return e;
-        g.ws = (float *)ws;
     }
+    if (g.splits > 1) g.ws = (float *)ws;
     g.T = (int)T, g.N = (int)N, g.kblocks = kblocks, g.stages = stages_of(BM, g.BN);
     g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc;
     g.vec = g.ws || ((uintptr_t)c % 16 == 0 && ldc % 4 == 0);

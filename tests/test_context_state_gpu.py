@@ -1,5 +1,5 @@
 """What the library keeps between calls belongs to its context: ggb_shutdown gives the memory back, and after another ggb_init every form of the
-products runs as before."""
+products runs as before.  A captured product finds the workspace of an earlier one of its T and N.  Each in a process of its own."""
 import os
 import subprocess
 import sys
@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-PROGRAM = """
+SHUTDOWN = """
 import sys
 sys.path[:0] = sys.argv[1:3]
 import numpy as np, torch
@@ -40,7 +40,36 @@ print("ok")
 """
 
 
-def test_shutdown_gives_the_workspaces_back():
+CAPTURE = """
+import sys
+sys.path[:0] = sys.argv[1:3]
+import ctypes as C
+import numpy as np
+import gemma_ggml_b200 as G
+from device_util import BF16, as_dt, dev, zeros
+
+G.init(0)
+lib, T, N, K = G.cuda_lib(), 192, 2048, 8192
+r = np.random.default_rng(1)
+(w, wr), (a, ar) = as_dt(BF16, r.standard_normal((N, K))), as_dt(BF16, r.standard_normal((T, K)))
+dw, da, c, c2 = dev(G, wr), dev(G, ar), zeros(G, T * N * 4), zeros(G, T * N * 4)
+G.check(lib.ggb_op_linear(BF16, dw.ptr, N, 128, da.ptr, 128, T, c.ptr, N), "linear")  # too short to be cut along K
+G.sync()
+G.check(lib.ggb_capture_begin())
+rc = lib.ggb_op_linear(BF16, dw.ptr, N, K, da.ptr, K, T, c.ptr, N)
+g = C.c_void_p()
+G.check(lib.ggb_capture_end(C.byref(g)))
+G.check(rc, "captured linear")
+G.check(lib.ggb_graph_launch(g))
+G.check(lib.ggb_op_linear(BF16, dw.ptr, N, K, da.ptr, K, T, c2.ptr, N), "linear")
+got, again, want = c.download(np.float32).reshape(T, N), c2.download(np.float32).reshape(T, N), a @ w.T
+assert (got == again).all() and np.linalg.norm(got - want) < 1e-4 * np.linalg.norm(want)
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("program", [SHUTDOWN, CAPTURE], ids=["shutdown", "capture"])
+def test_in_a_process_of_its_own(program):
     tests = os.path.dirname(os.path.abspath(__file__))
-    r = subprocess.run([sys.executable, "-c", PROGRAM, os.path.dirname(tests), tests], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", program, os.path.dirname(tests), tests], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
