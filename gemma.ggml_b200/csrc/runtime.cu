@@ -131,6 +131,15 @@ static int build_tables() {
     return GGB_OK;
 }
 
+// after a synchronisation: a kernel whose bounded wait ran out has said so
+static int wait_error_status() {
+    volatile int *e = g_ctx.wait_error;
+    if (!*e) return GGB_OK;
+    *e = 0;
+    ggb_set_error("a kernel's wait ran out: results computed since the last ggb_sync or ggb_download are not valid");
+    return GGB_ERR_CUDA;
+}
+
 extern "C" {
 
 int ggb_init(int device) {
@@ -163,6 +172,7 @@ int ggb_init(int device) {
 int ggb_shutdown(void) {
     if (!g_ctx.init) return GGB_OK;
     cudaStreamSynchronize(g_ctx.stream);
+    const int status = wait_error_status();
     ggb_comm_destroy();
     cudaFree(g_ctx.exp_table);
     cudaFree(g_ctx.rope_cos);
@@ -178,7 +188,7 @@ int ggb_shutdown(void) {
     g_ctx.prof.clear();
     cudaStreamDestroy(g_ctx.stream);
     g_ctx = Context();
-    return GGB_OK;
+    return status;
 }
 
 const char *ggb_last_error(void) {
@@ -198,15 +208,6 @@ int ggb_device_info(char *buf, size_t buflen) {
 }
 
 int ggb_sm_count(void) { return g_ctx.init ? g_ctx.prop.multiProcessorCount : 0; }
-
-// after a synchronisation: a kernel whose bounded wait ran out has said so
-static int wait_error_status() {
-    volatile int *e = g_ctx.wait_error;
-    if (!*e) return GGB_OK;
-    *e = 0;
-    ggb_set_error("a kernel's wait ran out: its results are not valid");
-    return GGB_ERR_CUDA;
-}
 
 int ggb_sync(void) {
     GGB_REQUIRE_INIT();

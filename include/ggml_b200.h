@@ -53,6 +53,9 @@ int ggb_shutdown(void);
 const char *ggb_last_error(void);
 int ggb_device_info(char *buf, size_t buflen); /* name, SMs, memory, compute capability */
 int ggb_sm_count(void);
+/* A kernel that waits for its own parts gives up after seconds instead of hanging the GPU; ggb_sync, ggb_download and ggb_shutdown then
+ * return an error, once, whichever call launched it.  A program that waits on ggb_stream() by other means asks ggb_sync before it trusts
+ * what was computed. */
 int ggb_sync(void);
 void *ggb_stream(void); /* the cudaStream_t all ops are enqueued on */
 int64_t ggb_launch_count(void); /* kernels launched (or replayed via graphs) since init */

@@ -1,5 +1,7 @@
 """What the library keeps between calls belongs to its context: ggb_shutdown gives the memory back, and after another ggb_init every form of the
-products runs as before.  A captured product finds the workspace of an earlier one of its T and N.  Each in a process of its own."""
+products runs as before.  A captured product finds the workspace of an earlier one of its T and N.  Each in a process of its own.  And a wait
+that ran out in a kernel is reported once, by the call that next waits for the GPU."""
+import ctypes as C
 import os
 import subprocess
 import sys
@@ -8,9 +10,13 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+# the host-mapped word a kernel sets
+FLAG = "_Z19ggb_wait_error_flagv"
+
 SHUTDOWN = """
 import sys
 sys.path[:0] = sys.argv[1:3]
+import ctypes as C
 import numpy as np, torch
 import gemma_ggml_b200 as G
 from device_util import BF16, as_dt, dev, release, zeros
@@ -36,6 +42,9 @@ assert freed >= 1 << 24, freed  # the sums of a product cut along K: 2 x 1024 x 
 G.check(G.cuda_lib().ggb_init(0))
 for x, y in zip(first, products()):
     assert (x == y).all()
+G.cuda_lib()._Z19ggb_wait_error_flagv.restype = C.POINTER(C.c_int)
+G.cuda_lib()._Z19ggb_wait_error_flagv()[0] = 1
+assert G.cuda_lib().ggb_shutdown() != 0
 print("ok")
 """
 
@@ -73,3 +82,15 @@ def test_in_a_process_of_its_own(program):
     tests = os.path.dirname(os.path.abspath(__file__))
     r = subprocess.run([sys.executable, "-c", program, os.path.dirname(tests), tests], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+def test_a_wait_that_ran_out_is_an_error_once(gpu):
+    lib, flag = gpu.cuda_lib(), getattr(gpu.cuda_lib(), FLAG)
+    flag.restype = C.POINTER(C.c_int)
+    word, host = flag(), (C.c_char * 16)()
+    buf = gpu.DeviceBuffer(16)
+    for call in (lambda: lib.ggb_sync(), lambda: lib.ggb_download(host, buf.ptr, 16)):
+        assert call() == 0
+        word[0] = 1
+        assert call() != 0 and b"wait ran out" in lib.ggb_last_error()
+        assert call() == 0 and word[0] == 0
