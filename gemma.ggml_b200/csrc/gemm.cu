@@ -1,6 +1,6 @@
 // gemm.cu — products of plain bf16 matrices on the tensor cores: C[T][N] = A[T][K] W[N][K]^T, and the grouped form for a mixture of experts.
 //
-// A tile of C is 256 x 256 or 128 x (256, 128, 64).  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
+// A tile of C is 256 x 256, by two CTAs of a cluster, or 128 x (256, 128, 64), by one.  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
 // in a ring that takes all of shared memory but the epilogue's corner; one warp issues the MMAs, eight drain tensor memory.  CTAs are
 // persistent: where a tile needs half of tensor memory, the next one's products run while the last one's are stored.  The epilogue
 // turns 32 x 32 pieces in shared memory, so that a store instruction writes whole 128-byte lines.
@@ -25,7 +25,7 @@
 
 namespace {
 
-constexpr int BK = 64;
+constexpr int BK = 64, BM = 128; // a stage of K, the rows of a CTA
 constexpr int kThreads = 384; // warp 0: TMA, 1: MMA, 2: tensor memory, 4..11: epilogue
 constexpr uint32_t kRing = 192 * 1024, kTurn = 8 * 4096;
 constexpr int kMaxStages = 8, kMaxGroups = 256; // groups whose first tiles are kept in shared memory
@@ -92,7 +92,6 @@ __device__ __forceinline__ void store_piece(const gemm_args &a, uint32_t col, in
     }
 }
 
-template <int BM>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
     extern __shared__ uint8_t gm_raw[];
     __shared__ int first_tile[kMaxGroups + 1]; // grouped: the first row tile of a group
@@ -101,8 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
     volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t a_bytes = BM * 128, stage_bytes = a_bytes + (uint32_t)a.BN * 128;
-    const uint32_t acc_cols = (uint32_t)(BM / 128 * a.chunks * a.BN);
-    const int n_acc = acc_cols <= 256 ? 2 : 1;
+    const int n_acc = a.chunks * a.BN <= 256 ? 2 : 1;
     if (tid == 0) {
         for (int s = 0; s < a.stages; s++) {
             mbar_init(bars + FULL + 8 * s, 1);
@@ -217,12 +215,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
                 tc_fence_after();
                 const uint32_t a_lo = umma_desc_lo(base + s * stage_bytes, 16), w_lo = umma_desc_lo(base + s * stage_bytes + a_bytes, 16);
                 const uint32_t first = left == a.chunk_kb ? 0u : 1u;
+                const uint32_t d = tmem + buf * 256 + chunk * a.BN;
 #pragma unroll
-                for (int mt = 0; mt < BM / 128; mt++) {
-                    const uint32_t d = tmem + buf * 256 + (mt * a.chunks + chunk) * a.BN;
-#pragma unroll
-                    for (int k = 0; k < BK / 16; k++) umma_ss(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, w_lo + 2 * k, idesc, k > 0 ? 1u : first);
-                }
+                for (int k = 0; k < BK / 16; k++) umma_ss(d, a_lo + 2 * k, w_lo + 2 * k, idesc, k > 0 ? 1u : first);
                 umma_arrive(bars + EMPTY + 8 * s);
                 if (++s == a.stages) s = 0, ph ^= 1u;
                 if (--left == 0) chunk++, left = a.chunk_kb;
@@ -242,14 +237,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
             mbar_wait_bounded(bars + ACC_FULL + 8 * buf, use & 1, dead);
             tc_fence_after();
             // a warp's 32 rows, every other 32 columns (the two warps of a quarter share them)
-            for (int mt = 0; mt < BM / 128; mt++) {
-                const int row0 = at.m0 + mt * 128 + lq * 32;
-                if (row0 >= at.m_end) break;
-                for (int c0 = 32 * half; c0 < a.BN; c0 += 64) {
-                    if (at.n0 + c0 >= a.N) break;
-                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + mt * a.chunks * a.BN + c0, chunks, my, lane, row0, at.m_end, at.n0 + c0, at.split);
-                }
-            }
+            const int row0 = at.m0 + lq * 32;
+            if (row0 < at.m_end)
+                for (int c0 = 32 * half; c0 < a.BN && at.n0 + c0 < a.N; c0 += 64)
+                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, chunks, my, lane, row0, at.m_end, at.n0 + c0, at.split);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + ACC_FREE + 8 * buf);
@@ -263,11 +254,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
     }
 }
 
-// Two CTAs a tile of MT x 256 rows and 256 columns: each holds MT x 128 rows of A and of the accumulators and half of W's rows.  A single CTA
+// Two CTAs a tile of 256 rows and 256 columns: each holds 128 rows of A and of the accumulators and half of W's rows.  A single CTA
 // reads A and W tiles of 12 KB from shared memory for an MMA of 128 cycles while TMA writes 64 bytes a cycle: 160 of the 128 bytes a cycle that
 // shared memory has; a pair needs 112.  2048 x 8192 x 4096: 104 us, 1320 TFLOP/s (107 us single, 131 us before either); 1024 x 32000 x 2048: 109 us
 // (125, 190 us).
-template <int MT>
 __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
     extern __shared__ uint8_t gm_raw[];
     const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, turn = base + kRing, bars = turn + kTurn;
@@ -275,9 +265,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
     volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t rank = cluster_rank(), bars0 = cluster_addr(bars, 0);
-    constexpr uint32_t a_bytes = MT * 16384, stage_bytes = a_bytes + 16384;
+    constexpr uint32_t a_bytes = BM * 128, stage_bytes = a_bytes + 16384;
     constexpr int kStages = (int)(kRing / stage_bytes);
-    const int n_acc = MT * a.chunks * 256 <= 256 ? 2 : 1;
+    const int n_acc = a.chunks == 1 ? 2 : 1;
     if (tid == 0) {
         for (int s = 0; s < kStages; s++) {
             mbar_init(bars + FULL + 8 * s, 1);
@@ -299,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
     const int total = a.m_tiles * a.n_tiles * a.splits, pairs = gridDim.x / 2, me = blockIdx.x / 2;
     // row tiles first: those that share a piece of W run together
     auto locate = [&](int t, int &m0, int &n0, int &split) {
-        m0 = t % a.m_tiles * (MT * 256);
+        m0 = t % a.m_tiles * (2 * BM);
         t /= a.m_tiles;
         n0 = t % a.n_tiles * 256;
         split = t / a.n_tiles;
@@ -320,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
                     mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead);
                     const uint32_t sa = base + s * stage_bytes;
                     if (rank == 0) mbar_expect_tx(bars + FULL + 8 * s, 2 * stage_bytes);
-                    tma_load_2d_pair(sa, &map_a, kb * BK, m0 + (int)rank * MT * 128, bars0 + FULL + 8 * s);
+                    tma_load_2d_pair(sa, &map_a, kb * BK, m0 + (int)rank * BM, bars0 + FULL + 8 * s);
                     tma_load_2d_pair(sa + a_bytes, &map_w, kb * BK, n0 + (int)rank * 128, bars0 + FULL + 8 * s);
                     if (++s == kStages) s = 0, ph ^= 1u;
                 }
@@ -343,12 +333,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
                 tc_fence_after();
                 const uint32_t a_lo = umma_desc_lo(base + s * stage_bytes, 16), w_lo = umma_desc_lo(base + s * stage_bytes + a_bytes, 16);
                 const uint32_t first = left == a.chunk_kb ? 0u : 1u;
+                const uint32_t d = tmem + buf * 256 + chunk * 256;
 #pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    const uint32_t d = tmem + buf * 256 + (mt * a.chunks + chunk) * 256;
-#pragma unroll
-                    for (int k = 0; k < BK / 16; k++) umma_ss_pair(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, w_lo + 2 * k, idesc, k > 0 ? 1u : first);
-                }
+                for (int k = 0; k < BK / 16; k++) umma_ss_pair(d, a_lo + 2 * k, w_lo + 2 * k, idesc, k > 0 ? 1u : first);
                 umma_arrive_pair(bars + EMPTY + 8 * s);
                 if (++s == kStages) s = 0, ph ^= 1u;
                 if (--left == 0) chunk++, left = a.chunk_kb;
@@ -366,12 +353,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
             const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
             mbar_wait_bounded(bars + ACC_FULL + 8 * buf, use & 1, dead);
             tc_fence_after();
-            for (int mt = 0; mt < MT; mt++) {
-                const int row0 = m0 + ((int)rank * MT + mt) * 128 + lq * 32;
-                if (row0 >= a.T) break;
+            const int row0 = m0 + (int)rank * BM + lq * 32;
+            if (row0 < a.T)
                 for (int c0 = 32 * half; c0 < 256 && n0 + c0 < a.N; c0 += 64)
-                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + mt * a.chunks * 256 + c0, chunks, turn + w8 * 4096, lane, row0, a.T, n0 + c0, split);
-            }
+                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, chunks, turn + w8 * 4096, lane, row0, a.T, n0 + c0, split);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(bars0 + ACC_FREE + 8 * buf);
@@ -405,11 +390,10 @@ __global__ void splits_add_kernel(const float *__restrict__ ws, int splits, int6
     }
 }
 
-int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int MT, const gemm_args &g, int pairs) {
+int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, const gemm_args &g, int pairs) {
     CUtensorMap ma, mw;
-    auto kfn = MT == 2 ? gemm_pair_kernel<2> : gemm_pair_kernel<1>;
-    int rc = ggb_allow_smem(kfn, kSmem);
-    if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, MT * 128);
+    int rc = ggb_allow_smem(gemm_pair_kernel, kSmem);
+    if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, 128);
     if (rc) return rc;
     cudaLaunchConfig_t cfg{};
@@ -421,24 +405,23 @@ int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
     cfg.attrs = at, cfg.numAttrs = 1;
-    GGB_CUDA(cudaLaunchKernelEx(&cfg, kfn, ma, mw, g));
+    GGB_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
 
-int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, int BM, const gemm_args &g, int ctas) {
+int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, const gemm_args &g, int ctas) {
     CUtensorMap ma, mw;
-    auto kfn = BM == 256 ? gemm_tma_kernel<256> : gemm_tma_kernel<128>;
-    int rc = ggb_allow_smem(kfn, kSmem);
+    int rc = ggb_allow_smem(gemm_tma_kernel, kSmem);
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
-    kfn<<<std::min(ctas, ggb_sm_count()), kThreads, kSmem, ggb_cuda_stream()>>>(ma, mw, g);
+    gemm_tma_kernel<<<std::min(ctas, ggb_sm_count()), kThreads, kSmem, ggb_cuda_stream()>>>(ma, mw, g);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
 
-int stages_of(int BM, int BN) { return std::min<int>(kMaxStages, (int)(kRing / (uint32_t)((BM + BN) * 128))); }
+int stages_of(int BN) { return std::min<int>(kMaxStages, (int)(kRing / (uint32_t)((BM + BN) * 128))); }
 
 } // namespace
 
@@ -477,48 +460,46 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(w && a && (c || c_act) && ((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
     GGB_CHECK_ARG(!c_act || ldc % 8 == 0, "gemm: an activation takes rows of whole 16-byte pieces");
-    const int sms = ggb_sm_count(), kblocks = (int)(K / BK);
-    int pieces = 1; // along K, until every SM has a piece of a 256 x 256 tile
-    const int64_t big = (N + 255) / 256 * ((T + 255) / 256);
-    while (pieces < 8 && big * pieces * 2 <= sms && kblocks / (pieces * 2) >= 4) pieces *= 2;
+    const int sms = ggb_sm_count(), kblocks = (int)(K / BK), pieces = ggb_gemm_pieces(T, N, K);
     gemm_args g{};
     double best = 0.0;
-    int BM = 0, pair = 0; // rows of a CTA; two CTAs a tile
+    int pair = -1; // two CTAs a tile
+    // (256 rows a CTA never have the least estimate: half as many tiles, whose stages take twice as long and more)
     static const struct {
-        int bm, bn, pair;
-    } shapes[] = {{256, 256, 1}, {128, 256, 1}, {256, 256, 0}, {128, 256, 0}, {128, 128, 0}, {128, 64, 0}};
+        int bn, pair;
+    } shapes[] = {{256, 1}, {256, 0}, {128, 0}, {64, 0}};
     for (const auto &sh : shapes)
         for (int splits = 1; splits <= pieces; splits *= 2) {
-            const int chunks = pieces / splits, mt = sh.bm / 128;
-            if (mt * chunks * sh.bn > 512) continue;
-            const int chunk_kb = (kblocks + pieces - 1) / pieces, rows = sh.bm * (1 + sh.pair), cs = 1 + sh.pair;
+            const int chunks = pieces / splits;
+            if (chunks * sh.bn > 512) continue;
+            const int chunk_kb = (kblocks + pieces - 1) / pieces, cs = 1 + sh.pair, rows = BM * cs;
             const int64_t m_tiles = (T + rows - 1) / rows, n_tiles = (N + sh.bn - 1) / sh.bn, tiles = m_tiles * n_tiles * splits;
             // cycles of a stage: its MMAs, or the bytes that pass through shared memory at 128 a cycle (written by TMA, read for the MMAs); a round of
             // tiles: its stages and, unless the next tile runs meanwhile, its stores
-            const double mma = mt * std::max(sh.bn, 96) * 2.0, smem = ((sh.bm + sh.bn / cs) * 128.0 + mt * 4 * (4096.0 + sh.bn * 32.0 / cs)) / 128.0;
-            const double stage = std::max(mma, smem), store = sh.bm * sh.bn / 12.0;
+            const double mma = std::max(sh.bn, 96) * 2.0, smem = ((BM + sh.bn / cs) * 128.0 + 4 * (4096.0 + sh.bn * 32.0 / cs)) / 128.0;
+            const double stage = std::max(mma, smem), store = BM * sh.bn / 12.0;
             const double rounds = (double)((tiles + sms / cs - 1) / (sms / cs));
-            double cost = rounds * (chunks * chunk_kb * stage + (mt * chunks * sh.bn > 256 ? store : 0.0)) + store + 2000.0;
+            double cost = rounds * (chunks * chunk_kb * stage + (chunks * sh.bn > 256 ? store : 0.0)) + store + 2000.0;
             if (splits > 1) cost += 12000.0 + (double)splits * T * N * 8.0 / (32.0 * sms); // another launch, the sums' way through memory
             cost += sh.pair ? 4000.0 : 0.0;                                               // a cluster's launch
-            if (!BM || cost < best) {
+            if (pair < 0 || cost < best) {
                 best = cost;
-                BM = sh.bm, pair = sh.pair;
+                pair = sh.pair;
                 g.BN = sh.bn, g.n_tiles = (int)n_tiles, g.m_tiles = (int)m_tiles, g.chunks = chunks, g.chunk_kb = chunk_kb, g.splits = splits;
             }
         }
     // sized by T and N alone, for every product that some K would cut: where one of them has run, a captured one allocates nothing
     void *ws = nullptr;
-    if (big * 2 <= sms) {
+    if ((N + 255) / 256 * ((T + 255) / 256) * 2 <= sms) {
         const int e = ggb_workspace(GGB_WS_GEMM_SPLITS, ggb_gemm_workspace_bytes(T, N, K), &ws);
         if (e) return e;
     }
     if (g.splits > 1) g.ws = (float *)ws;
-    g.T = (int)T, g.N = (int)N, g.kblocks = kblocks, g.stages = stages_of(BM, g.BN);
+    g.T = (int)T, g.N = (int)N, g.kblocks = kblocks, g.stages = stages_of(g.BN);
     g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc;
     g.vec = g.ws || ((uintptr_t)c % 16 == 0 && ldc % 4 == 0);
     g.wait_error = ggb_wait_error_flag();
-    const int tiles = g.m_tiles * g.n_tiles * g.splits, rc = pair ? launch_pair(w, N, K, a, T, BM / 128, g, tiles) : launch(w, N, K, a, T, BM, g, tiles);
+    const int tiles = g.m_tiles * g.n_tiles * g.splits, rc = pair ? launch_pair(w, N, K, a, T, g, tiles) : launch(w, N, K, a, T, g, tiles);
     if (rc || g.splits == 1) return rc;
     splits_add_kernel<<<(unsigned)((T * N / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(g.ws, g.splits, T, N, c, g.act_out, act, ldc);
     GGB_LAUNCH_CHECK();
@@ -532,13 +513,12 @@ int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, in
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
     gemm_args g{};
-    const int BM = 128;
     g.BN = N <= 64 ? 64 : N <= 128 ? 128 : 256;
     g.T = (int)n_rows, g.N = (int)N, g.kblocks = (int)(K / BK), g.n_tiles = (int)((N + g.BN - 1) / g.BN);
-    g.chunks = 1, g.chunk_kb = g.kblocks, g.splits = 1, g.stages = stages_of(BM, g.BN);
+    g.chunks = 1, g.chunk_kb = g.kblocks, g.splits = 1, g.stages = stages_of(g.BN);
     g.m_ranges = offsets, g.n_groups = n_exp;
     g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc, g.vec = (uintptr_t)c % 16 == 0;
     g.wait_error = ggb_wait_error_flag();
     const int64_t most = ((n_rows + BM - 1) / BM + n_exp) * g.n_tiles;
-    return launch(w, (int64_t)n_exp * N, K, a, n_rows, BM, g, (int)std::min<int64_t>(most, 1 << 20));
+    return launch(w, (int64_t)n_exp * N, K, a, n_rows, g, (int)std::min<int64_t>(most, 1 << 20));
 }

@@ -23,8 +23,15 @@ def rel(a, b):
     return np.linalg.norm(a - b) / np.linalg.norm(b)
 
 
-@pytest.mark.parametrize("T,N,K,pad", [(64, 32, 64, 0), (65, 96, 128, 4), (127, 256, 576, 0), (128, 288, 2112, 0), (129, 64, 4096, 0), (255, 2048, 2048, 8), (256, 2080, 192, 0), (257, 544, 1024, 0),
-                                       (300, 4096, 64, 0), (1000, 1056, 1408, 0), (1024, 8192, 256, 0), (64, 160, 8192, 0), (2048, 32, 320, 0), (700, 8224, 448, 0)])
+# what the rule of csrc/gemm.cu takes for them on 148 SMs: tiles of 128 rows
+SINGLE = [(64, 32, 64, 0), (65, 96, 128, 4), (127, 256, 576, 0), (128, 288, 2112, 0), (129, 64, 4096, 0), (255, 2048, 2048, 8), (256, 2080, 192, 0), (257, 544, 1024, 0),
+          (300, 4096, 64, 0), (1000, 1056, 1408, 0), (1024, 8192, 256, 0), (64, 160, 8192, 0), (2048, 32, 320, 0), (700, 8224, 448, 0),
+          (528, 3744, 512, 0), (142, 5184, 1024, 0), (155, 9760, 512, 4), (650, 9600, 192, 0), (67, 2432, 4928, 0)]
+# two CTAs a tile of 256 x 256: accumulators a CTA x CTAs along K 2 x 1, 1 x 8 (two rounds of tiles), 2 x 2, 2 x 4, and 1 x 1 in several rounds
+PAIRS = [(131, 10368, 960, 0), (141, 2528, 5184, 8), (154, 5280, 5184, 0), (260, 1568, 5824, 0), (385, 9952, 704, 0), (1024, 8192, 2048, 0)]
+
+
+@pytest.mark.parametrize("T,N,K,pad", SINGLE + PAIRS)
 def test_dense(gpu, T, N, K, pad):
     r = np.random.default_rng(T + N)
     (w, wr), (a, ar) = as_dt(BF16, r.standard_normal((N, K))), as_dt(BF16, r.standard_normal((T, K)))
