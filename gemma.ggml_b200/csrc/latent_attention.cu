@@ -721,7 +721,9 @@ int ggb_op_latent_attn_out_gated(int dt, const float *part, int n_split, const f
     GGB_REQUIRE_INIT();
     GGB_CHECK_DT(dt);
     GGB_CHECK_ARG((!gate || ldg >= H) && part && w_uv && out && T > 0 && H > 0 && R > 0 && Dv > 0 && n_split > 0, "latent_attn_out: bad arguments");
-    if (dt == GGB_TYPE_BF16 && latent_tile::out_fits(R, Dv, T, n_split, w_uv, out)) {
+    const size_t smem = (size_t)kOutT * (R + n_split) * 4;
+    GGB_CHECK_ARG(smem <= 48 * 1024, "latent_attn_out: latent size %d with %d splits too large", R, n_split);
+    if (dt == GGB_TYPE_BF16 && latent_tile::out_fits(R, Dv, T, n_split, part, w_uv, out)) {
         const latent_tile::out_args a{part, n_split, sink, (const __nv_bfloat16 *)w_uv, (int)T, H, R, Dv, gate, ldg, (__nv_bfloat16 *)out, ggb_wait_error_flag()};
         const int rc = ggb_allow_smem(latent_tile::latent_out_kernel, latent_tile::kOutSmem);
         if (rc) return rc;
@@ -733,8 +735,6 @@ int ggb_op_latent_attn_out_gated(int dt, const float *part, int n_split, const f
     // few tokens: spread a head's outputs over several CTAs; many tokens: the grid is large already, merge once per head
     const int v_chunk = T * H >= 1024 ? Dv : 16;
     const dim3 grid((unsigned)((T + kOutT - 1) / kOutT), (unsigned)H, (unsigned)((Dv + v_chunk - 1) / v_chunk));
-    const size_t smem = (size_t)kOutT * (R + n_split) * 4;
-    GGB_CHECK_ARG(smem <= 48 * 1024, "latent_attn_out: latent size %d with %d splits too large", R, n_split);
     if (dt == GGB_TYPE_BF16)
         ggb_launch_step(latent_attn_out_kernel<__nv_bfloat16>, grid, dim3(256), smem, part, n_split, sink, (const __nv_bfloat16 *)w_uv, T, H, R, Dv,
                                                                        v_chunk, gate, ldg, (__nv_bfloat16 *)out);

@@ -424,8 +424,9 @@ struct out_args {
 constexpr uint32_t kOutW = 256 * 128; // a block of W_uv: up to 256 rows of 64 numbers
 constexpr int kOutSplits = 16;        // parts a row's weights are kept for
 constexpr size_t kOutSmem = 1024 + 2 * (kLeft + kOutW) + 256 + (size_t)kRows * kOutSplits * 4;
-inline bool out_fits(int R, int Dv, int64_t T, int n_split, const void *w_uv, const void *out) {
-    return T >= 32 && T < (1 << 24) && R % 16 == 0 && Dv % 16 == 0 && Dv <= 256 && n_split <= kOutSplits && (uintptr_t)w_uv % 16 == 0 && (uintptr_t)out % 4 == 0;
+inline bool out_fits(int R, int Dv, int64_t T, int n_split, const void *part, const void *w_uv, const void *out) {
+    return T >= 32 && T < (1 << 24) && R % 16 == 0 && Dv % 16 == 0 && Dv <= 256 && n_split <= kOutSplits && (uintptr_t)part % 8 == 0 && (uintptr_t)w_uv % 16 == 0 &&
+           (uintptr_t)out % 4 == 0;
 }
 
 // one output by one thread: w_uv's row against the merged parts (p0, weights wsm, ps numbers from one part to the next)

@@ -89,3 +89,25 @@ def test_infinities_as_plain_arithmetic_has_them(gpu, where, H, R, Dr, Dv, T, po
     assert (np.isnan(got) == np.isnan(want)).all() and (got[np.isinf(want)] == want[np.isinf(want)]).all()
     ok = np.isfinite(want)
     assert rel(got[ok], want[ok]) < 2.5e-3
+
+
+def test_parts_on_any_4_byte_boundary(gpu):
+    lib, T, H, R, Dr, Dv, pos, page = gpu.cuda_lib(), 40, 4, 64, 16, 32, 10, 64
+    r = np.random.default_rng(2)
+    ld = int(lib.ggb_latent_cache_ld(R, Dr))
+    cache, table, p0 = dev(gpu, as_dt(BF16, r.standard_normal((page, ld)))[1]), dev(gpu, i32([0])), dev(gpu, i32([pos]))
+    qa, w = dev(gpu, f32(r.standard_normal((T, H, R + Dr)) * 0.1)), dev(gpu, as_dt(BF16, r.standard_normal((H, Dv, R)) * R ** -0.5)[1])
+    n, got = int(lib.ggb_latent_attn_scratch_bytes(T, H, R, 1)), []
+    for skip in (0, 1):
+        part, out = zeros(gpu, n + 16), zeros(gpu, T * H * Dv * 2)
+        gpu.check(lib.ggb_op_latent_attn(BF16, qa.ptr, cache.ptr, table.ptr, page, p0.ptr, T, H, R, Dr, 1, part.ptr.value + 4 * skip), "attn")
+        gpu.check(lib.ggb_op_latent_attn_out_gated(BF16, part.ptr.value + 4 * skip, 1, None, w.ptr, T, H, R, Dv, None, H, out.ptr), "out")
+        got.append(from_dt(BF16, out, (T, H, Dv)))
+    assert np.abs(got[0]).max() > 0.1 and rel(got[1], got[0]) < 3e-3  # two forms of the output product: a rounding to bf16
+
+
+@pytest.mark.parametrize("T", [8, 64])
+def test_latents_too_wide_for_the_output_product_are_refused_for_every_portion(gpu, T):
+    lib, H, R, Dv = gpu.cuda_lib(), 2, 2048, 16
+    part, w, out = zeros(gpu, T * H * (R + 2) * 4), zeros(gpu, H * Dv * R * 2), zeros(gpu, T * H * Dv * 2)
+    assert lib.ggb_op_latent_attn_out_gated(BF16, part.ptr, 1, None, w.ptr, T, H, R, Dv, None, H, out.ptr) != 0
