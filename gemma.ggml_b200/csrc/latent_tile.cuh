@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
         }
         tc_fence_before();
     }
+    settle(dead);
     __syncthreads();
     if (warp == kWarps) {
         tc_fence_after();
@@ -538,6 +539,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_out_kernel(const out_args 
         }
         tc_fence_before();
     }
+    settle(dead);
     __syncthreads();
     if (warp == kWarps) {
         tc_fence_after();

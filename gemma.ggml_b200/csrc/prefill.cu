@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
                 mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead);
+                if (*dead) break;
                 const uint32_t bar = bars + full + 8 * s;
                 mbar_expect_tx(bar, is_a ? a_bytes : c_bytes);
                 if (is_a) tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, bar);
@@ -354,6 +355,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         }
         __syncwarp();
     }
+    settle(dead);
     __syncthreads();
     if (PAIR) cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
     if (warp == kMmaWarp) {

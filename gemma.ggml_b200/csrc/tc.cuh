@@ -28,7 +28,8 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Waits for a phase.  Every wait ends: after kWaitTries tries (seconds) the CTA's `dead` word is set, which ends all of its other
-// waits at once; the kernel then runs through with whatever is in its buffers, gives its tensor memory back and reports the failure.
+// waits at once; the kernel then requests no more copies, runs through with whatever is in its buffers, gives what it has requested time to
+// arrive (settle), gives its tensor memory back and reports the failure.
 constexpr int kWaitTries = 1 << 21;
 __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int *dead) {
     if (mbar_try(bar, parity)) return;
@@ -37,6 +38,11 @@ __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity,
         if (*dead) return;
     }
     *dead = 1;
+}
+// behind a wait that ran out: copies and MMAs may still be under way, and what they write stays this CTA's for another half second
+__device__ __forceinline__ void settle(volatile int *dead) {
+    if (*dead)
+        for (int i = 0; i < 500; i++) __nanosleep(1000000);
 }
 
 // Shared-memory matrix operands, 128-byte swizzle: rows of 128 bytes, 16-byte piece c of row r at place c ^ (r & 7), 1024-byte atoms

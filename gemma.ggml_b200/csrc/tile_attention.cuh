@@ -539,6 +539,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const 
         }
         tc_fence_before();
     }
+    settle(dead);
     __syncthreads();
     if (warp == kMmaWarp) {
         tc_fence_after();

@@ -52,3 +52,16 @@ def test_every_early_launched_kernel_waits_before_it_touches_memory():
 def test_no_pointer_of_theirs_is_restrict():
     ks = kernels()
     assert not [n for n in launched() if "__restrict__" in ks[n][0]]
+
+
+def test_a_kernel_whose_wait_ran_out_lets_its_copies_arrive():
+    """Behind a wait that gave up, copies that were requested are still under way: no more are requested, and the CTA outlives them."""
+    waiting = {n: body for n, (_, body) in kernels().items() if "mbar_wait_bounded(" in body}
+    assert len(waiting) >= 5
+    for n, body in waiting.items():
+        end = body[body.rindex("settle(dead);"):]
+        assert "__syncthreads()" in end and "tmem_free512" in end, n
+        for m in re.finditer(r"mbar_expect_tx\(", body):
+            ahead = body[:m.start()]
+            since = ahead[ahead.rindex("mbar_wait_bounded("):]
+            assert "if (*dead) break;" in since or "if (!*dead)" in since, n
