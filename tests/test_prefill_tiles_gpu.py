@@ -30,7 +30,11 @@ def rel(a, b):
 
 @pytest.mark.parametrize("wtype", [O.TYPE_Q4_0, O.TYPE_Q8_0])
 @pytest.mark.parametrize("T,N,K,resid", [(1, 32, 64, 0), (128, 96, 576, 1), (129, 32, 64, 0), (200, 288, 128, 1), (256, 2080, 192, 0), (257, 64, 1024, 1), (512, 256, 2048, 1), (513, 544, 320, 0),
-                                         (130, 4096, 64, 0), (300, 2048, 4096, 1), (70, 1056, 2112, 1)])
+                                         (130, 4096, 64, 0), (300, 2048, 4096, 1), (70, 1056, 2112, 1),
+                                         # pairs of 512 rows x 64, 64 (two accumulators), 128 and 256 columns
+                                         (898, 2368, 64, 1), (795, 2368, 640, 0), (826, 4736, 64, 0), (277, 9536, 64, 1),
+                                         # pairs of 256 rows: 64 x 8 accumulators, 128 x 4, 256 x 2, 256 x 2 x 4 CTAs along K, 128 x 8 CTAs
+                                         (270, 800, 2048, 0), (297, 2464, 1024, 1), (130, 10176, 512, 0), (276, 1184, 3200, 1), (282, 288, 2240, 0)])
 def test_products(gpu, wtype, T, N, K, resid):
     r = np.random.default_rng(T + N + K)
     w, wv = matrix(gpu, r, wtype, N, K)
@@ -46,7 +50,7 @@ def test_products(gpu, wtype, T, N, K, resid):
 
 
 @pytest.mark.parametrize("wtype", [O.TYPE_Q4_0, O.TYPE_Q8_0])
-@pytest.mark.parametrize("T,F,K", [(129, 256, 64), (300, 512, 320), (512, 1024, 256), (700, 256, 1024)])
+@pytest.mark.parametrize("T,F,K", [(129, 256, 64), (300, 512, 320), (512, 1024, 256), (700, 256, 1024), (270, 5120, 64), (600, 5120, 192)])  # the last two: pairs of 512 rows
 def test_gate_up_gelu(gpu, wtype, T, F, K):
     r = np.random.default_rng(T + F)
     (g, gv), (u, uv) = matrix(gpu, r, wtype, F, K), matrix(gpu, r, wtype, F, K)

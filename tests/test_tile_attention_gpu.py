@@ -54,7 +54,9 @@ def rel(a, b):
 # H, Gk, D, Dv, T, pos, page, window, keep, chunked, cap, scale, sink, gate
 SOFT = [(1, 1, 16, 16, 32, 0, 64, 0, 0, 0, 0.0, 0.3, 1, 0), (4, 1, 64, 64, 33, 31, 64, 0, 0, 0, 0.0, 0.1, 0, 1), (3, 1, 80, 112, 129, 64, 7, 65, 1, 0, 30.0, 0.2, 1, 1),
         (2, 2, 128, 128, 128, 0, 64, 64, 0, 0, 30.0, 1.0, 0, 0), (16, 1, 128, 128, 40, 500, 64, 300, 70, 0, 2.0, 0.5, 0, 1), (6, 2, 192, 128, 127, 129, 16, 100, 0, 1, 0.0, 0.1, 0, 0),
-        (5, 5, 48, 96, 200, 3, 64, 1, 130, 0, 0.0, 0.3, 1, 0), (8, 8, 96, 80, 300, 700, 64, 128, 64, 0, 0.0, 2.0, 0, 1), (128, 1, 32, 32, 35, 66, 64, 0, 0, 0, 5.0, 0.4, 0, 0)]
+        (5, 5, 48, 96, 200, 3, 64, 1, 130, 0, 0.0, 0.3, 1, 0), (8, 8, 96, 80, 300, 700, 64, 128, 64, 0, 0.0, 2.0, 0, 1), (128, 1, 32, 32, 35, 66, 64, 0, 0, 0, 5.0, 0.4, 0, 0),
+        # keys of three blocks of 64 with values of one, the most that shared memory holds (192 with 128 above runs on the CUDA cores)
+        (6, 2, 192, 64, 127, 129, 16, 100, 0, 1, 0.0, 0.1, 0, 0), (4, 1, 176, 48, 70, 30, 64, 0, 0, 0, 30.0, 0.5, 1, 1)]
 
 
 @pytest.mark.parametrize("dt", [BF16, F32])
