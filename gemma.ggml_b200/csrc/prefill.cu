@@ -64,6 +64,7 @@ struct GemmArgs {
     int N, nb, kblocks;  // N = concatenated rows (padded between segments), nb = K / 32, kblocks = K / 64
     int T, MT, BN;       // a CTA's rows: MT x 128; a tile's columns
     int chunks, chunk_kb, stages; // stages of A rows
+    int vec;             // rows of every C and of resid start on 16 bytes
     float *ws;           // workspace [splits][T][N] or null (one CTA along K: tiles go straight to seg.c)
     const float *resid;  // [T][seg[0].ldc] or null (single segment, no workspace)
     __nv_bfloat16 *geglu; // two segments, gate and up, of which every tile takes BN / 2 rows each: [T][rows] gelu(gate) * up
@@ -120,6 +121,12 @@ __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
+}
+
+__device__ __forceinline__ float4 load4(const float *p, int vec) { return vec ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]); }
+__device__ __forceinline__ void store4(float *p, const float4 v, int vec) {
+    if (vec) *reinterpret_cast<float4 *>(p) = v;
+    else p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
 }
 
 template <int TYPE, bool PAIR>
@@ -282,10 +289,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                     continue;
                 }
                 if (A.resid) {
-                    const float4 r4 = *reinterpret_cast<const float4 *>(A.resid + (size_t)row * sg.ldc + sn0 + c0 + 4 * p);
+                    const float4 r4 = load4(A.resid + (size_t)row * sg.ldc + sn0 + c0 + 4 * p, A.vec);
                     o.x += r4.x, o.y += r4.y, o.z += r4.z, o.w += r4.w;
                 }
-                *reinterpret_cast<float4 *>(cbase + (size_t)row * cld + c0 + 4 * p) = o;
+                store4(cbase + (size_t)row * cld + c0 + 4 * p, o, A.ws || A.vec);
             }
         }
         tc_fence_before();
@@ -378,13 +385,13 @@ __global__ void splitk_reduce_kernel(const GemmArgs A, int splits) {
     const int col = n - sg.n_begin;
     if (col >= sg.rows) return; // tile padding between segments
     float4 acc = *reinterpret_cast<const float4 *>(A.ws + i);
-    auto add = [&](const float *p) {
-        const float4 v = *reinterpret_cast<const float4 *>(p);
+    auto add = [&](const float *p, int vec) {
+        const float4 v = load4(p, vec);
         acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
     };
-    for (int s = 1; s < splits; s++) add(A.ws + (int64_t)s * T * N + i);
-    if (A.resid) add(A.resid + t * sg.ldc + col);
-    *reinterpret_cast<float4 *>(sg.c + t * sg.ldc + col) = acc;
+    for (int s = 1; s < splits; s++) add(A.ws + (int64_t)s * T * N + i, 1);
+    if (A.resid) add(A.resid + t * sg.ldc + col, A.vec);
+    store4(sg.c + t * sg.ldc + col, acc, A.vec);
 }
 
 // rms_norm * w -> bf16 (the A operand of the next GEMM): same double-sum order as rms_norm_kernel (elementwise.cu)
@@ -764,7 +771,9 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     GemmArgs A{};
     GemmMaps maps{};
     int64_t N = 0;
+    uintptr_t at16 = (uintptr_t)resid;
     for (int i = 0; i < n; i++) {
+        at16 |= (uintptr_t)c[i];
         GGB_CHECK_ARG(w[i] && (c[i] || geglu) && w[i]->cols == K && w[i]->type == type, "gemm: matrices of one launch share K and the type");
         const int64_t rows = w[i]->rows;
         GGB_CHECK_ARG(K % 64 == 0 && rows % 32 == 0 && ldc[i] >= rows && ldc[i] % 4 == 0,
@@ -773,6 +782,8 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
         N += i + 1 < n ? (rows + 255) / 256 * 256 : rows;
     }
     A.n_seg = n;
+    A.vec = at16 % 16 == 0; // row pitches are whole 16-byte pieces
+    GGB_CHECK_ARG((uintptr_t)geglu % 8 == 0, "gemm_geglu: y starts on 8 bytes");
     const int kblocks = (int)(K / BK), sms = ggb_sm_count(), pb = ggb_payload_bytes(type);
     int pieces = ggb_gemm_pieces(T, N, K);
     if (pieces > 1 && (!workspace || workspace_bytes < (size_t)pieces * T * N * 4)) pieces = 1;

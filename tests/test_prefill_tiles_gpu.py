@@ -49,6 +49,25 @@ def test_products(gpu, wtype, T, N, K, resid):
         assert rel(c.download(np.float32).reshape(T, N), want) < (K / 16 + 8) * 2.0 ** -23 + 1e-7
 
 
+@pytest.mark.parametrize("T,N,K", [(128, 96, 576), (300, 2048, 4096), (257, 64, 1024), (512, 256, 2048), (129, 32, 64)])
+def test_outputs_that_start_anywhere(gpu, T, N, K):
+    """Results and residuals on any 4-byte boundary, whether the product is cut along K in tensor memory, over CTAs or not at all."""
+    r = np.random.default_rng(T)
+    w, _ = matrix(gpu, r, O.TYPE_Q8_0, N, K)
+    lib, a, x = gpu.cuda_lib(), dev(gpu, bf16_round(r.standard_normal((T, K)))[1]), f32(r.standard_normal((T, N)))
+    n_ws = lib.ggb_gemm_workspace_bytes(T, N, K)
+    ws, got = zeros(gpu, n_ws), []
+    for skip in (0, 1, 2, 3):
+        c, dx = zeros(gpu, (T * N + 8) * 4), dev(gpu, np.concatenate([np.zeros(skip, np.float32), x.reshape(-1)]))
+        for with_ws in (True, False):
+            gpu.check(lib.ggb_op_gemm_bf16(w.h, a.ptr, T, c.ptr.value + 4 * skip, N, dx.ptr.value + 4 * skip, ws.ptr if with_ws else None, n_ws if with_ws else 0))
+            y = c.download(np.float32)
+            assert not y[:skip].any() and not y[skip + T * N:].any()
+            got.append(y[skip:skip + T * N])
+    for i in range(2, 8):
+        assert (got[i] == got[i % 2]).all()
+
+
 @pytest.mark.parametrize("wtype", [O.TYPE_Q4_0, O.TYPE_Q8_0])
 @pytest.mark.parametrize("T,F,K", [(129, 256, 64), (300, 512, 320), (512, 1024, 256), (700, 256, 1024), (270, 5120, 64), (600, 5120, 192)])  # the last two: pairs of 512 rows
 def test_gate_up_gelu(gpu, wtype, T, F, K):
