@@ -120,7 +120,7 @@ def attend(gpu, kind, q, cache, table, pos0, T, pos, H, G, D, Dv, cap=0.0, windo
     elif kind == "diff":
         gpu.check(lib.ggb_op_diff_attn(*head, keep, cap, 0.4, 0.7, 1e-5, g, H * Dv, out.ptr, None), "attn")
     else:
-        gpu.check(lib.ggb_op_sigmoid_attn(*head, *(ptr(dev(gpu, f32(o))) for o in (offsets or np.zeros((3, H)))), out.ptr, None), "attn")
+        gpu.check(lib.ggb_op_sigmoid_attn(*head, *(ptr(dev(gpu, f32(o))) for o in (np.zeros((3, H)) if offsets is None else offsets)), out.ptr, None), "attn")
     return from_dt(BF16, out, (T, H, Dv))
 
 
