@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
                 int kb0, kb1;
                 k_range(at.split, kb0, kb1);
                 for (int kb = kb0; kb < kb1; kb++) {
-                    mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead);
-                    if (*dead) break;
+                    if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead)) break;
                     const uint32_t sa = base + s * stage_bytes, bar = bars + FULL + 8 * s;
                     mbar_expect_tx(bar, stage_bytes);
                     tma_load_2d(sa, &map_a, kb * BK, at.m0, bar);
@@ -247,9 +246,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
             if (lane == 0) mbar_arrive(bars + ACC_FREE + 8 * buf);
         }
     }
-    settle(dead);
     __syncthreads();
     if (warp == 2) {
+        settle(dead);
         tc_fence_after();
         tmem_free512(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;
@@ -309,8 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
                 locate(t, m0, n0, split);
                 k_range(split, kb0, kb1);
                 for (int kb = kb0; kb < kb1; kb++) {
-                    mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead);
-                    if (*dead) break;
+                    if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead)) break;
                     const uint32_t sa = base + s * stage_bytes;
                     if (rank == 0) mbar_expect_tx(bars + FULL + 8 * s, 2 * stage_bytes);
                     tma_load_2d_pair(sa, &map_a, kb * BK, m0 + (int)rank * BM, bars0 + FULL + 8 * s);
@@ -365,8 +363,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
             if (lane == 0) mbar_arrive_cluster(bars0 + ACC_FREE + 8 * buf);
         }
     }
-    settle(dead);
     __syncthreads();
+    if (warp == 2) settle(dead);
     cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
     if (warp == 2) {
         tc_fence_after();

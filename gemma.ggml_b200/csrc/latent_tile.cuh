@@ -401,9 +401,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
         }
         tc_fence_before();
     }
-    settle(dead);
     __syncthreads();
     if (warp == kWarps) {
+        settle(dead);
         tc_fence_after();
         tmem_free512(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;
@@ -539,9 +539,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_out_kernel(const out_args 
         }
         tc_fence_before();
     }
-    settle(dead);
     __syncthreads();
     if (warp == kWarps) {
+        settle(dead);
         tc_fence_after();
         tmem_free512(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;

@@ -304,8 +304,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
             int s = 0;
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
-                mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead);
-                if (*dead) break;
+                if (!mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead)) break;
                 const uint32_t bar = bars + full + 8 * s;
                 mbar_expect_tx(bar, is_a ? a_bytes : c_bytes);
                 if (is_a) tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, bar);
@@ -313,8 +312,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                 if (++s == n) s = 0, ph ^= 1u;
             }
             if (A.geglu && is_a) { // the MMAs have read the ring: the gelu table takes its place
-                mbar_wait_bounded(bars + DONE, 0, dead);
-                if (!*dead) {
+                if (mbar_wait_bounded(bars + DONE, 0, dead)) {
                     mbar_expect_tx(bars + TABLE_FULL, kGeluBytes);
                     for (uint32_t o = 0; o < kGeluBytes; o += 32768)
                         bulk_load(smem0 + kGeluAt + o, reinterpret_cast<const uint8_t *>(A.gelu) + o, 32768, bars + TABLE_FULL);
@@ -362,8 +360,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         }
         __syncwarp();
     }
-    settle(dead);
     __syncthreads();
+    if (warp == kMmaWarp) settle(dead);
     if (PAIR) cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
     if (warp == kMmaWarp) {
         tc_fence_after();

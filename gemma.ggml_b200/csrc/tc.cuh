@@ -31,15 +31,17 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // waits at once; the kernel then requests no more copies, runs through with whatever is in its buffers, gives what it has requested time to
 // arrive (settle), gives its tensor memory back and reports the failure.
 constexpr int kWaitTries = 1 << 21;
-__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int *dead) {
-    if (mbar_try(bar, parity)) return;
+__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int *dead) { // false: given up
+    if (mbar_try(bar, parity)) return true;
     for (int i = 0; i < kWaitTries; i++) {
-        if (mbar_try(bar, parity)) return;
-        if (*dead) return;
+        if (mbar_try(bar, parity)) return true;
+        if (*dead) return false;
     }
     *dead = 1;
+    return false;
 }
-// behind a wait that ran out: copies and MMAs may still be under way, and what they write stays this CTA's for another half second
+// Behind a wait that ran out: copies and MMAs may still be under way, and what they write stays this CTA's for another half second.  By one
+// warp, when all of them are done.
 __device__ __forceinline__ void settle(volatile int *dead) {
     if (*dead)
         for (int i = 0; i < 500; i++) __nanosleep(1000000);

@@ -539,9 +539,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const 
         }
         tc_fence_before();
     }
-    settle(dead);
     __syncthreads();
     if (warp == kMmaWarp) {
+        settle(dead);
         tc_fence_after();
         tmem_free512(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;
