@@ -5,9 +5,9 @@
 //
 //   C[T][N] (fp32) = A[T][K] (bf16 activations) x dequant(W[N][K] Q4_0 | Q8_0)^T       (+ residual)
 //
-// More than 128 rows: two CTAs of a cluster compute a tile (cta_group::2) of 512 or 256 rows x up to 256 columns; each holds half of the
+// More than 256 rows: two CTAs of a cluster compute a tile (cta_group::2) of 512 or 256 rows x up to 256 columns; each holds half of the
 // rows of A and dequantises half of the tile's weight rows, so a prompt of 512 tokens dequantises every weight once.  Fewer rows: one
-// CTA, 128 rows x up to 128 columns.  Per 64-wide K block
+// CTA, 256 or 128 rows x up to 128 columns.  Per 64-wide K block
 //   * one thread requests the CTA's A rows by TMA, another one the raw codes (a ring of their own: they are needed a dequantisation earlier);
 //   * two groups of eight warps take the K blocks alternately and DEQUANTISE the W rows (int8 / int4 codes x fp16 block scale -> bf16, exact
 //     product rounded once) from shared memory into shared memory, canonical K-major 128-byte-swizzled UMMA layout;
@@ -44,10 +44,10 @@ constexpr int BK = 64;
 constexpr int kWorkWarps = 16, kGroupWarps = 8, kTmaWarp = 16, kMmaWarp = 17, kCodesWarp = 18, kGemmThreads = 32 * 19;
 constexpr uint32_t kRing = 224 * 1024;
 constexpr int kMaxStages = 6;
-constexpr size_t kGemmSmem = 1024 + kRing + 384;
-constexpr int kTiles = 2, kCodeStages = 4; // buffers of dequantised weights, of codes
-enum { A_FULL = 0, A_FREE = 48, B_FULL = 96, B_FREE = 128, PEER_FULL = 160, C_FULL = 192, C_FREE = 240, DONE = 288, SLOT = 296, DEAD = 304, TABLE_FULL = 312 };
-constexpr uint32_t kGeluBytes = 65536 * 2, kGeluAt = 64 * 1024; // the gelu table, behind the epilogue's 16 x 4 KB: where only TMA wrote and MMAs read
+constexpr size_t kGemmSmem = 1024 + kRing + 512;
+constexpr int kTiles = 2, kMaxCodeStages = 12; // buffers of dequantised weights, of codes
+enum { A_FULL = 0, A_FREE = 48, B_FULL = 96, B_FREE = 128, PEER_FULL = 160, C_FULL = 192, C_FREE = 288, DONE = 384, SLOT = 392, DEAD = 400, TABLE_FULL = 408 };
+constexpr uint32_t kGeluBytes = 65536 * 2, kGeluAt = 64 * 1024; // the gelu table, behind the epilogue's 16 x 4 KB, in the ring, which the last MMA has left
 
 // up to 3 weight matrices that share the A operand run as ONE launch (Q | K | V, gate | up): a segment = one matrix, its first row is a
 // multiple of 256, so a tile belongs to exactly one segment
@@ -63,7 +63,8 @@ struct GemmArgs {
     int n_seg;
     int N, nb, kblocks;  // N = concatenated rows (padded between segments), nb = K / 32, kblocks = K / 64
     int T, MT, BN;       // a CTA's rows: MT x 128; a tile's columns
-    int chunks, chunk_kb, stages; // stages of A rows
+    int chunks, chunk_kb, stages, code_stages; // stages of A rows, of codes (an even number: two groups take them in turn)
+    uint32_t a_tx;       // bytes of a stage of A that are loaded: a single row tile leaves out what lies 8 rows and more past the last
     int vec;             // rows of every C and of resid start on 16 bytes
     float *ws;           // workspace [splits][T][N] or null (one CTA along K: tiles go straight to seg.c)
     const float *resid;  // [T][seg[0].ldc] or null (single segment, no workspace)
@@ -148,14 +149,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
     const int kb0 = split * A.chunks * A.chunk_kb, kb1 = min(kb0 + A.chunks * A.chunk_kb, A.kblocks);
     if (sn0 >= sg.rows) return; // padding between matrices: all CTAs of the tile, before any barrier or tensor memory exists
     const uint32_t b_bytes = (uint32_t)BR * 128, a_bytes = (uint32_t)A.MT * 16384, c_bytes = (uint32_t)BR * 2 * PB;
-    const uint32_t codes = smem0 + kTiles * b_bytes, ring = codes + kCodeStages * c_bytes; // dequantised tiles | codes | A rows
+    const uint32_t codes = smem0 + kTiles * b_bytes, ring = codes + A.code_stages * c_bytes; // dequantised tiles | codes | A rows
 
     if (tid == 0) {
         for (int s = 0; s < A.stages; s++) {
             mbar_init(bars + A_FULL + 8 * s, 1);
             mbar_init(bars + A_FREE + 8 * s, 1);
         }
-        for (int s = 0; s < kCodeStages; s++) {
+        for (int s = 0; s < A.code_stages; s++) {
             mbar_init(bars + C_FULL + 8 * s, 1);
             mbar_init(bars + C_FREE + 8 * s, kGroupWarps);
         }
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                 if (lane == 0) mbar_arrive(bars + B_FULL + 8 * b);
                 use++;
                 s += 2;
-                if (s >= kCodeStages) s -= kCodeStages, ph ^= 1u;
+                if (s >= A.code_stages) s -= A.code_stages, ph ^= 1u;
             }
         }
         // ================= epilogue: pieces of 32 rows x 32 columns, dealt to the four warps of a lane quarter
@@ -300,13 +301,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         // ================= A rows wait for the MMAs of their stage, codes, requested further ahead, for the warps that read them
         if (lane == 0) {
             const bool is_a = warp == kTmaWarp;
-            const int n = is_a ? A.stages : kCodeStages, full = is_a ? A_FULL : C_FULL, fre = is_a ? A_FREE : C_FREE;
+            const int n = is_a ? A.stages : A.code_stages, full = is_a ? A_FULL : C_FULL, fre = is_a ? A_FREE : C_FREE;
             int s = 0;
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
                 if (!mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead)) break;
                 const uint32_t bar = bars + full + 8 * s;
-                mbar_expect_tx(bar, is_a ? a_bytes : c_bytes);
+                mbar_expect_tx(bar, is_a ? A.a_tx : c_bytes);
                 if (is_a) tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, bar);
                 else tma_load_2d(codes + s * c_bytes, &maps.w[si], kb * 2 * PB, w_row0, bar);
                 if (++s == n) s = 0, ph ^= 1u;
@@ -785,23 +786,24 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     const int kblocks = (int)(K / BK), sms = ggb_sm_count(), pb = ggb_payload_bytes(type);
     int pieces = ggb_gemm_pieces(T, N, K);
     if (pieces > 1 && (!workspace || workspace_bytes < (size_t)pieces * T * N * 4)) pieces = 1;
-    const bool pair = T > 128;
-    GGB_CHECK_ARG(!geglu || (pair && n == 2 && w[0]->rows == w[1]->rows && w[0]->rows % 256 == 0), "gemm_geglu: two matrices of as many rows and more than 128 tokens");
+    // a prompt of up to 256 rows fits one CTA's tile: 256000 x 2048, Q4_0, 129 rows: @S129@ us (pairs of CTAs: 408)
+    const bool pair = geglu || T > 256;
+    GGB_CHECK_ARG(!geglu || (T > 128 && n == 2 && w[0]->rows == w[1]->rows && w[0]->rows % 256 == 0), "gemm_geglu: two matrices of as many rows and more than 128 tokens");
     if (geglu) pieces = 1, N = 2 * w[0]->rows;
     A.gelu = ggb_gelu_table_dev();
     // the tile and the CTAs along K with the least estimated time (cycles): a stage takes what its MMAs, the bytes through shared memory (128 a
     // cycle: written by TMA, read and written by the dequantisation, read for the MMAs) or the dequantisation take (2.7 a row: 32 weights are
-    // 170 instructions of one lane)
+    // 170 instructions of one lane), and no less than 1000, the way of a K block through its hands, however narrow the tile
     double best = -1.0;
     int splits = 1;
-    for (int MT = T > 256 ? 2 : 1; MT >= 1; MT--)
+    for (int MT = T > (pair ? 256 : 128) ? 2 : 1; MT >= 1; MT--)
         for (int bn = pair ? 256 : 128; bn >= (geglu ? 256 : 64); bn /= 2)
             for (int sp = 1; sp <= pieces; sp *= 2) {
                 const int chunks = pieces / sp, chunk_kb = (kblocks + pieces - 1) / pieces, br = pair ? bn / 2 : bn, rows = MT * (pair ? 256 : 128);
                 if (MT * chunks * bn > 512) continue;
                 const int64_t tiles = (N + bn - 1) / bn * ((T + rows - 1) / rows) * sp, slots = pair ? sms / 2 : sms;
                 const double mma = MT * std::max(bn, 96) * 2.0, smem = (MT * 16384.0 + br * (4.0 * pb + 128.0) + MT * 4 * (4096.0 + br * 32.0)) / 128.0;
-                const double stage = std::max(std::max(mma, smem), std::max(br * 2.7, 350.0));
+                const double stage = std::max(std::max(mma, smem), std::max(br * 2.7, 1000.0));
                 double cost = (double)((tiles + slots - 1) / slots) * (chunks * chunk_kb * stage + MT * 128.0 * bn / (geglu ? 24.0 : 12.0) + 3000.0);
                 if (sp > 1) cost += 6000.0 + (double)sp * T * N * 8.0 / (32.0 * sms);
                 if (best < 0.0 || cost < best) {
@@ -812,12 +814,17 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
             }
     const int br = pair ? A.BN / 2 : A.BN;
     A.N = (int)N, A.nb = (int)w[0]->nb, A.kblocks = kblocks, A.T = (int)T;
-    A.stages = std::min<int>(kMaxStages, (int)((kRing - kTiles * br * 128 - kCodeStages * br * 2 * pb) / (A.MT * 16384)));
+    // Codes come from memory, A rows from L2: what is in flight of the codes bounds a product of few rows (256000 x 2048, Q4_0, 33 to 128 rows:
+    // 4 stages 276 to 289 us, 12 stages 263 to 275), the MMAs and shared memory one of 512 rows a tile.
+    A.code_stages = A.MT == 1 ? kMaxCodeStages : pair ? 4 : 8;
+    A.stages = std::min<int>(kMaxStages, (int)((kRing - kTiles * br * 128 - A.code_stages * br * 2 * pb) / (A.MT * 16384)));
+    const int a_rows = !pair && T <= A.MT * 128 ? (int)(T + 7) / 8 * 8 : A.MT * 128;
+    A.a_tx = (uint32_t)a_rows * 128;
     A.ws = splits > 1 ? (float *)workspace : nullptr;
     A.resid = splits > 1 ? nullptr : resid; // added by the reducer
     A.geglu = (__nv_bfloat16 *)geglu;
     A.wait_error = ggb_wait_error_flag();
-    int rc = ggb_tensor_map_bf16(&maps.a, a_bf16, T, K, K, A.MT * 128);
+    int rc = ggb_tensor_map_bf16(&maps.a, a_bf16, T, K, K, a_rows);
     for (int i = 0; i < n && !rc; i++) rc = ggb_tensor_map_bytes(&maps.w[i], w[i]->qs, w[i]->rows, K / 32 * pb, 2 * pb, br);
     if (rc) return rc;
     const bool q4 = type == GGB_TYPE_Q4_0;
