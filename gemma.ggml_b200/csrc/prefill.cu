@@ -17,8 +17,8 @@
 //     gate | up of a feed-forward: each CTA dequantises rows of one of the two matrices, so both products of an output stand in the same row
 //     of tensor memory and leave as gelu(gate) * up in bf16; the 128 KB gelu table is brought into the ring behind the last MMA.
 // A product along a long K is summed in pieces of K (as many as a split over the SMs in 256 x 256 tiles needs): several accumulators a
-// CTA in tensor memory, added in order by the epilogue, and, where SMs are left, several CTAs whose sums meet in a workspace and are
-// added in order by a second kernel (deterministic).
+// CTA in tensor memory, added in order by the epilogue, and, where SMs are left, several CTAs, whose pieces all meet in a workspace and are
+// added in order by a second kernel: the same bits whichever tile is chosen.
 //
 // What bounds it: shared memory (128 bytes a cycle).  A K block of a pair's CTA (256 rows, 128 weight rows) moves 40 KB in by TMA, 8 KB of codes
 // out, 16 KB of weights in and 64 to 96 KB out for the MMAs: 1550 cycles where the MMAs alone take 1024; the weights of a block stand half a
@@ -66,7 +66,7 @@ struct GemmArgs {
     int chunks, chunk_kb, stages, code_stages; // stages of A rows, of codes (an even number: two groups take them in turn)
     uint32_t a_tx;       // bytes of a stage of A that are loaded: a single row tile leaves out what lies 8 rows and more past the last
     int vec;             // rows of every C and of resid start on 16 bytes
-    float *ws;           // workspace [splits][T][N] or null (one CTA along K: tiles go straight to seg.c)
+    float *ws;           // workspace [pieces of K][T][N] or null (one CTA along K: tiles go straight to seg.c)
     const float *resid;  // [T][seg[0].ldc] or null (single segment, no workspace)
     __nv_bfloat16 *geglu; // two segments, gate and up, of which every tile takes BN / 2 rows each: [T][rows] gelu(gate) * up
     const uint16_t *gelu; // the fp16 table of gelu
@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         mbar_wait_bounded(bars + DONE, 0, dead);
         tc_fence_after();
         const int chunks = kb1 > kb0 ? (kb1 - kb0 + A.chunk_kb - 1) / A.chunk_kb : 0, lq = warp & 3, cols = (A.geglu ? A.BN / 2 : A.BN) / 32;
-        float *cbase = A.ws ? A.ws + (size_t)split * A.T * A.N + n0 : sg.c + sn0;
+        const int planes = A.ws ? chunks : 1; // in a workspace every piece along K stands alone: they are added in order, whichever CTA summed them
+        float *cbase = A.ws ? A.ws + (size_t)split * A.chunks * A.T * A.N + n0 : sg.c + sn0;
         const int cld = A.ws ? A.N : sg.ldc;
         const uint32_t my = smem0 + warp * 4096; // the ring is no longer used
         if (A.geglu) mbar_wait_bounded(bars + TABLE_FULL, 0, dead);
@@ -261,39 +262,40 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                     for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__uint_as_float(v[16 * hf + q]) + __uint_as_float(u[q]));
                 }
             };
-            if (chunks > 0) tmem_load32(col, v);
-            else // no K block is left for this CTA
-                for (int q = 0; q < 32; q++) v[q] = 0;
-            for (int ch = 1; ch < chunks; ch++) add_columns(col + ch * A.BN);
-            if (A.geglu) { // the other half of the tile's columns is up (one K piece)
+            for (int plane = 0; plane < planes; plane++) {
+                tmem_load32(col + plane * A.BN, v);
+                if (!A.ws)
+                    for (int ch = 1; ch < chunks; ch++) add_columns(col + ch * A.BN);
+                if (A.geglu) { // the other half of the tile's columns is up (one K piece)
 #pragma unroll
-                for (int hf = 0; hf < 2; hf++) {
-                    uint32_t u[16];
-                    tmem_load16(col + A.BN / 2 + 16 * hf, u);
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t u[16];
+                        tmem_load16(col + A.BN / 2 + 16 * hf, u);
 #pragma unroll
-                    for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__fmul_rn(gelu(v[16 * hf + q]), __uint_as_float(u[q])));
+                        for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__fmul_rn(gelu(v[16 * hf + q]), __uint_as_float(u[q])));
+                    }
                 }
-            }
-            __syncwarp();
+                __syncwarp();
 #pragma unroll
-            for (int p = 0; p < 8; p++) sts_u4(my + lane * 128 + ((p ^ (lane & 7)) << 4), make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]));
-            __syncwarp();
-            const int p = lane & 7;
+                for (int p = 0; p < 8; p++) sts_u4(my + lane * 128 + ((p ^ (lane & 7)) << 4), make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]));
+                __syncwarp();
+                const int p = lane & 7;
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const int r = 4 * q + (lane >> 3), row = row0 + r;
-                const uint4 w = lds_u4(my + r * 128 + ((p ^ (r & 7)) << 4));
-                if (row >= A.T) continue; // rows of a matrix are a multiple of 32
-                float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
-                if (A.geglu) {
-                    *reinterpret_cast<uint2 *>(A.geglu + (size_t)row * sg.rows + sn0 + c0 + 4 * p) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
-                    continue;
+                for (int q = 0; q < 8; q++) {
+                    const int r = 4 * q + (lane >> 3), row = row0 + r;
+                    const uint4 w = lds_u4(my + r * 128 + ((p ^ (r & 7)) << 4));
+                    if (row >= A.T) continue; // rows of a matrix are a multiple of 32
+                    float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+                    if (A.geglu) {
+                        *reinterpret_cast<uint2 *>(A.geglu + (size_t)row * sg.rows + sn0 + c0 + 4 * p) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+                        continue;
+                    }
+                    if (A.resid) {
+                        const float4 r4 = load4(A.resid + (size_t)row * sg.ldc + sn0 + c0 + 4 * p, A.vec);
+                        o.x += r4.x, o.y += r4.y, o.z += r4.z, o.w += r4.w;
+                    }
+                    store4(cbase + ((size_t)plane * A.T + row) * cld + c0 + 4 * p, o, A.ws || A.vec);
                 }
-                if (A.resid) {
-                    const float4 r4 = load4(A.resid + (size_t)row * sg.ldc + sn0 + c0 + 4 * p, A.vec);
-                    o.x += r4.x, o.y += r4.y, o.z += r4.z, o.w += r4.w;
-                }
-                store4(cbase + (size_t)row * cld + c0 + 4 * p, o, A.ws || A.vec);
             }
         }
         tc_fence_before();
@@ -372,8 +374,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
     }
 }
 
-// partial tiles of a K-split GEMM summed in split order (+ residual)
-__global__ void splitk_reduce_kernel(const GemmArgs A, int splits) {
+// the pieces of a product that several CTAs summed along K, in order (+ residual)
+__global__ void splitk_reduce_kernel(const GemmArgs A, int pieces) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4, T = A.T, N = A.N; // N and the segments: multiples of 32
     if (i >= T * N) return;
     const int64_t t = i / N;
@@ -388,7 +390,7 @@ __global__ void splitk_reduce_kernel(const GemmArgs A, int splits) {
         const float4 v = load4(p, vec);
         acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
     };
-    for (int s = 1; s < splits; s++) add(A.ws + (int64_t)s * T * N + i, 1);
+    for (int s = 1; s < pieces; s++) add(A.ws + (int64_t)s * T * N + i, 1);
     if (A.resid) add(A.resid + t * sg.ldc + col, A.vec);
     store4(sg.c + t * sg.ldc + col, acc, A.vec);
 }
@@ -804,8 +806,9 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
                 const int64_t tiles = (N + bn - 1) / bn * ((T + rows - 1) / rows) * sp, slots = pair ? sms / 2 : sms;
                 const double mma = MT * std::max(bn, 96) * 2.0, smem = (MT * 16384.0 + br * (4.0 * pb + 128.0) + MT * 4 * (4096.0 + br * 32.0)) / 128.0;
                 const double stage = std::max(std::max(mma, smem), std::max(br * 2.7, 1000.0));
-                double cost = (double)((tiles + slots - 1) / slots) * (chunks * chunk_kb * stage + MT * 128.0 * bn / (geglu ? 24.0 : 12.0) + 3000.0);
-                if (sp > 1) cost += 6000.0 + (double)sp * T * N * 8.0 / (32.0 * sms);
+                const double store = MT * 128.0 * bn / (geglu ? 24.0 : 12.0) * (sp > 1 ? chunks : 1);
+                double cost = (double)((tiles + slots - 1) / slots) * (chunks * chunk_kb * stage + store + 3000.0);
+                if (sp > 1) cost += 6000.0 + (double)pieces * T * N * 8.0 / (32.0 * sms);
                 if (best < 0.0 || cost < best) {
                     best = cost;
                     splits = sp;
@@ -847,7 +850,7 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     if (splits > 1) {
         A.resid = resid;
         const int64_t cnt = T * N;
-        splitk_reduce_kernel<<<(unsigned)((cnt / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, splits);
+        splitk_reduce_kernel<<<(unsigned)((cnt / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, (kblocks + A.chunk_kb - 1) / A.chunk_kb);
         GGB_LAUNCH_CHECK();
     }
     return GGB_OK;

@@ -49,6 +49,26 @@ def test_products(gpu, wtype, T, N, K, resid):
         assert rel(c.download(np.float32).reshape(T, N), want) < (K / 16 + 8) * 2.0 ** -23 + 1e-7
 
 
+@pytest.mark.parametrize("wtype", [O.TYPE_Q4_0, O.TYPE_Q8_0])
+@pytest.mark.parametrize("T,N,K", [(257, 512, 2048), (300, 2048, 4096), (276, 1184, 3200), (129, 512, 2048), (70, 1056, 2112), (270, 800, 2048)])
+def test_pieces_of_k_are_added_in_order(gpu, wtype, T, N, K):
+    """With a workspace, a product is the sum of its pieces along K, the first to the last, whether one CTA or several summed them."""
+    r, lib = np.random.default_rng(K), gpu.cuda_lib()
+    q, ar = O.quantize(wtype, f32(r.standard_normal((N, K)) * 0.02)), bf16_round(r.standard_normal((T, K)))[1]
+    n_ws, x, c = lib.ggb_gemm_workspace_bytes(T, N, K), f32(r.standard_normal((T, N))), zeros(gpu, T * N * 4)
+    w, pieces = gpu.Weight.upload(wtype, q, K), lib.ggb_gemm_pieces(T, N, K)
+    assert pieces > 1
+    gpu.check(lib.ggb_op_gemm_bf16(w.h, dev(gpu, ar).ptr, T, c.ptr, N, dev(gpu, x).ptr, zeros(gpu, n_ws).ptr, n_ws))
+    step, want, y = -(-(K // 64) // pieces) * 64, None, zeros(gpu, T * N * 4)
+    for k in range(0, K, step):
+        n, row = min(step, K - k), q.shape[1] // (K // 32)
+        part = gpu.Weight.upload(wtype, np.ascontiguousarray(q[:, k // 32 * row:(k + n) // 32 * row]), n)
+        gpu.check(lib.ggb_op_gemm_bf16(part.h, dev(gpu, np.ascontiguousarray(ar[:, k:k + n])).ptr, T, y.ptr, N, None, None, 0))
+        piece = y.download(np.float32).reshape(T, N)
+        want = piece.copy() if want is None else want + piece
+    assert (c.download(np.float32).reshape(T, N) == want + x).all()
+
+
 @pytest.mark.parametrize("T,N,K", [(128, 96, 576), (300, 2048, 4096), (257, 64, 1024), (512, 256, 2048), (129, 32, 64)])
 def test_outputs_that_start_anywhere(gpu, T, N, K):
     """Results and residuals on any 4-byte boundary, whether the product is cut along K in tensor memory, over CTAs or not at all."""
