@@ -695,7 +695,7 @@ int ggb_op_latent_attn_window(int dt, const float *qa, const void *cache, const 
                       n_split <= 65535 && block_size > 0,
                   "latent_attn: bad arguments (latent size up to 1024)");
     const int64_t ldk = ggb_latent_cache_ld(R, Dr);
-    if (dt == GGB_TYPE_BF16 && latent_tile::fits(R, Dr, H, T, qa, cache)) {
+    if (dt == GGB_TYPE_BF16 && latent_tile::fits(R, Dr, H, T, n_split, qa, cache)) {
         const int vp = R <= 256 ? R : R / 2, tq = latent_tile::kRows / H;
         const latent_tile::args a{qa, (const __nv_bfloat16 *)cache, ldk, block_table, block_size, pos0, (int)T, H, R, R + Dr, vp, window, part, ggb_wait_error_flag()};
         const int rc = ggb_allow_smem(latent_tile::latent_tile_kernel, latent_tile::kSmem);

@@ -48,9 +48,11 @@ struct args {
     int *wait_error;
 };
 
-// 128 rows x QK, R a multiple of 32 so that half a latent is whole MMA steps and 16-byte pieces
-inline bool fits(int R, int Dr, int H, int64_t T, const void *qa, const void *cache) {
-    return T >= 9 && T < (1 << 24) && H <= kRows && R % 32 == 0 && R <= 512 && Dr % 16 == 0 && (uintptr_t)qa % 16 == 0 && (uintptr_t)cache % 16 == 0;
+// 128 rows x QK, R a multiple of 32 so that half a latent is whole MMA steps and 16-byte pieces.  From 9 tokens on; two CTAs' rows or fewer
+// whose positions are not split (there are few of them then: a caller splits a hundred and more) are quicker on the CUDA cores: 16 tokens x
+// 8 heads of 256 at position 0 14 us (25), 24 tokens x 4 heads of 128 at 50 20 us (22), 9 x 16 of 512 at 0 and 50 22 and 36 us (34, 34).
+inline bool fits(int R, int Dr, int H, int64_t T, int n_split, const void *qa, const void *cache) {
+    return T >= 9 && T < (1 << 24) && (n_split > 1 || T * H > 2 * kRows) && H <= kRows && R % 32 == 0 && R <= 512 && Dr % 16 == 0 && (uintptr_t)qa % 16 == 0 && (uintptr_t)cache % 16 == 0;
 }
 
 // 2048 groups of four numbers of a left operand's block: thread tid takes groups tid + 256 u, row = group / 16

@@ -23,7 +23,9 @@ def rel(a, b):
 # H, R, Dr, Dv, T, pos, window, splits, page, gate, scale
 CASES = [(16, 512, 64, 128, 33, 250, 0, 1, 64, 0, 1.0), (16, 512, 64, 128, 32, 224, 100, 2, 64, 1, 3.0), (8, 256, 32, 64, 40, 0, 0, 1, 7, 0, 1.0), (4, 128, 64, 16, 65, 700, 300, 3, 64, 1, 0.5),
          (1, 32, 16, 16, 129, 127, 0, 1, 64, 0, 1.0), (3, 96, 0, 48, 50, 1, 1, 2, 16, 0, 2.0), (128, 64, 16, 32, 9, 255, 0, 2, 64, 0, 1.0), (5, 320, 48, 256, 100, 513, 0, 7, 64, 0, 8.0),
-         (16, 480, 32, 80, 200, 56, 256, 1, 64, 1, 1.0), (7, 288, 16, 96, 31, 0, 0, 4, 64, 0, 1.0)]
+         (16, 480, 32, 80, 200, 56, 256, 1, 64, 1, 1.0), (7, 288, 16, 96, 31, 0, 0, 4, 64, 0, 1.0),
+         # unsplit positions: up to two CTAs' rows on the CUDA cores, more here
+         (1, 32, 16, 16, 256, 2, 0, 1, 64, 0, 1.0), (1, 32, 16, 16, 257, 2, 0, 1, 64, 0, 1.0), (16, 512, 64, 128, 16, 40, 0, 1, 64, 0, 1.0), (16, 512, 64, 128, 17, 40, 0, 1, 64, 0, 1.0)]
 
 
 @pytest.mark.parametrize("H,R,Dr,Dv,T,pos,window,ns,page,gate,scale", CASES)
@@ -57,7 +59,7 @@ def test_parts_and_output(gpu, H, R, Dr, Dv, T, pos, window, ns, page, gate, sca
 
 
 @pytest.mark.parametrize("where", ["rotated", "latent", "w_uv", "query", "nan"])
-@pytest.mark.parametrize("H,R,Dr,Dv,T,pos,window,ns", [(5, 320, 48, 32, 40, 20, 0, 2), (4, 128, 16, 48, 33, 500, 300, 1)])
+@pytest.mark.parametrize("H,R,Dr,Dv,T,pos,window,ns", [(5, 320, 48, 32, 40, 20, 0, 2), (4, 128, 16, 48, 33, 500, 300, 1), (4, 128, 16, 48, 70, 500, 300, 1)])
 def test_infinities_as_plain_arithmetic_has_them(gpu, where, H, R, Dr, Dv, T, pos, window, ns):
     r = np.random.default_rng(R)
     lib, QK, n, page = gpu.cuda_lib(), R + Dr, pos + T, 64
