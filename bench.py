@@ -94,7 +94,7 @@ def workload_name(args):
 
 
 def matvec_bytes_per_step(dims, wtype):
-    """algorithmic bytes of the mat-vec launches of one token (SURVEY.md §8d): weights at 18|34 B per 32
+    """algorithmic bytes of the mat-vec launches of one token: weights at 18|34 B per 32
     + Q8_0 activations read + fp32 outputs written."""
     bpb = 18 if wtype == 2 else 34
     E, L, H, Hkv, d, F, V = (dims[k] for k in ("n_embd", "n_layer", "n_head", "n_head_kv", "head_dim", "n_ff", "n_vocab"))
@@ -142,7 +142,7 @@ def bench_config(args, world, lowering, kernels_per_step):
 
 def run_reference(args):
     """--impl reference: the reference's own CPU implementation of the path.  The reference cannot be compiled
-    (un-vendored ggml, DESIGN.md section 3), so this is the oracle's restatement of its thread_pool mul_mat path
+    (un-vendored ggml), so this is the oracle's restatement of its thread_pool mul_mat path
     with all host threads (kind "port": scalar vec_dot, not ggml's hand-written SIMD).  One step = one full decode
     token of the same workload; the timed region is capped at ~150 s."""
     rank = int(os.environ.get("RANK", "0"))
@@ -194,7 +194,7 @@ def time_decode(G, L, m, steps, warmup, pos, barrier, dist):
 
 def rank_bytes(m, dims, ctx, world):
     """algorithmic bytes THIS GPU streams per token: its weight pass streams (row shards + replicated phases; 18 | 34 B
-    per 32 weights, the same figure as SURVEY 8d for one GPU) + the KV rows of the heads whose cache it holds"""
+    per 32 weights, the same figure as for one GPU) + the KV rows of the heads whose cache it holds"""
     kv = dims["n_layer"] * 2 * m.rank_kv_heads * dims["head_dim"] * 2 * ctx
     return m.rank_stream_bytes + kv
 
@@ -286,7 +286,7 @@ def mul_mat_dropin_us(G):
 
 
 def kquant_matvec_record(G, peak_gbs):
-    """SURVEY.md 8f-2 on the record: the resident (packed) K-quant mat-vecs on the tied-embedding shape of Gemma-2B
+    """The resident (packed) K-quant mat-vecs on the tied-embedding shape of Gemma-2B
     (256000 x 2048, one Q8_K activation row), device-timed; algorithmic bytes = ggml's block bytes (144 / 210 per 256)."""
     L = G.cuda_lib()
     rng = np.random.default_rng(11)
@@ -417,7 +417,7 @@ def run_ours(args):
     per_class = {}
     wname = "Q4_0" if wtype == 2 else "Q8_0"
     if fused:
-        # one persistent kernel per token: algorithmic bytes per launch = weights + KV this GPU reads (SURVEY.md 8d),
+        # one persistent kernel per token: algorithmic bytes per launch = weights + KV this GPU reads,
         # duration = the CUDA-event time of the timed region / launches
         step_bytes = (m.weight_bytes + kv_bytes) if world == 1 else rank_bytes(m, dims, args.ctx, world)
         achieved = step_bytes / step_s / 1e9

@@ -1,6 +1,6 @@
-// comm.cu — multi-GPU plumbing for row-sharded tensor parallelism (SURVEY.md §8e): one process per
+// comm.cu — multi-GPU plumbing for row-sharded tensor parallelism: one process per
 // GPU, NCCL over NVLink 5 / NVSwitch, allgather at the layer boundaries where the row shards meet.
-// The reference has no communication backend (SURVEY.md §2a); nothing is ported.
+// The reference has no communication backend; nothing is ported.
 // NCCL is resolved with dlopen so the library loads (and single-GPU paths run) without it.
 #include <dlfcn.h>
 

@@ -2,7 +2,7 @@
 // +KV-cache store), K8 get_rows+scale, K9 argmax, and the small element-wise graph nodes
 // (add / mul / scale / gelu / soft_max_ext / cpy) the builder emits
 // (ref: src/gemma_model.cpp:438-452, 499-518, 675-679, 698-716; [UPSTREAM] ggml op semantics,
-// SURVEY.md Appendix A).  All HBM-bound or latency-bound; no tensor cores.
+// ggml as the reference uses it).  All HBM-bound or latency-bound; no tensor cores.
 #include "common.cuh"
 
 namespace {

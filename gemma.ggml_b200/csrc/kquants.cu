@@ -1,4 +1,4 @@
-// kquants.cu — SURVEY.md 8f-2: the formats the reference's own offload kernels target.
+// kquants.cu — the formats the reference's own offload kernels target.
 //   Q4_K x Q8_K   ref: src/kernals.cl:48-111  (matrix_multiply_q4_K :166-214)
 //   Q6_K x Q8_K   ref: src/kernals.cl:114-156 ([UPSTREAM] ggml's QK_K = 256 layout; the reference's copy indexes
 //                 the block as QK_K = 64 and reads an uninitialised aux8 tail - its host never launches it,

@@ -10,7 +10,8 @@
 //
 // qkv_store: one CTA per token.  The query is multiplied by its temperature 1 + coef ln(floor((p + 1) / every) + 1) and
 // by the score scale; each value head is divided by its root mean square before it is cached.
-// sigmoid_attn, portions: bf16 caches of whole 16-wide heads on the tensor cores (tile_attention.cuh); else sigmoid_attn_tile_kernel: a CTA owns 32 consecutive tokens of one head, 4 per warp; tiles of
+// sigmoid_attn, portions: bf16 caches of whole 16-wide heads on the tensor cores (tile_attention.cuh); else sigmoid_attn_tile_kernel: a CTA
+// owns 32 consecutive tokens of one head, 4 per warp; tiles of
 // 32 cache rows are staged once in shared memory as fp32 and serve all 32 queries.  The penalty depends on i - j only:
 // the 63 distances a tile can meet are computed once per tile (63 logarithms instead of 1024).
 // sigmoid_attn, steps of few tokens (sigmoid_attn_step_kernel): 8 warps x up to 16 CTAs split one (token, head)'s keys a

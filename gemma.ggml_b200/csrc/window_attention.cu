@@ -8,7 +8,8 @@
 // qkv_store: one CTA per token: root mean square over the whole q and the whole k projection, weights, rotation, store.
 // window_attn, both forms: lane = key for the scores, lane = pair of value coordinates for the weighted sum, running
 // maximum and sum in registers.
-//   portions: bf16 caches of whole 16-wide heads on the tensor cores (tile_attention.cuh); else window_attn_tile_kernel: a CTA owns 32 consecutive tokens of one head, 4 per warp.  Their windows
+//   portions: bf16 caches of whole 16-wide heads on the tensor cores (tile_attention.cuh); else window_attn_tile_kernel: a CTA owns 32
+//   consecutive tokens of one head, 4 per warp.  Their windows
 //   overlap almost wholly, so every tile of 32 cache rows is staged once in shared memory as fp32 (row pitch odd in words:
 //   lane = row reads are conflict-free) and serves all 32 queries; a K word read feeds 4 multiply-adds.
 //   steps of few tokens (window_attn_kernel): 8 warps split one (token, head)'s keys, rows straight from the cache

@@ -65,7 +65,7 @@ int gm_generate(void *m, const int32_t *prompt, int n_prompt, int n_decode, int3
     memcpy(out, o.data(), o.size() * sizeof(int32_t));
     return 0;
 }
-// ---- GGUF loader + tokenizer (SURVEY.md 8f-1, 8f-4).  gm_gguf_probe parses a file on the host only (no GPU needed).
+// ---- GGUF loader + tokenizer.  gm_gguf_probe parses a file on the host only (no GPU needed).
 static thread_local std::string g_capi_err;
 const char *gm_last_error() { return g_capi_err.c_str(); }
 int gm_gguf_probe(const char *path, gemma_config *cfg, int32_t *n_tensors, int32_t *n_kv, int32_t *n_tokens, int32_t *bos, int32_t *eos) {

@@ -21,7 +21,7 @@ static void kq_free(void *&p) {
     p = nullptr;
 }
 
-static constexpr float kNormSigma = 0.02f; // norm weights: 1 + N(0, 0.02^2) (SURVEY.md §8d)
+static constexpr float kNormSigma = 0.02f; // norm weights: 1 + N(0, 0.02^2)
 
 gemma_model::gemma_model(const gemma_config &cfg) : cfg_(cfg) {
     layers_.resize((size_t)cfg.n_layer);
@@ -406,7 +406,7 @@ int gemma_model::alloc_buffers() {
     return ggb_sync();
 }
 
-// The op sequence of ONE token — the reference's per-layer node list (SURVEY.md §3.3,
+// The op sequence of ONE token — the reference's per-layer node list (
 // ref: src/gemma_model.cpp:688-740) with adjacent nodes fused:
 //   norm+mul+quantize | Q,K,V mat-vecs | rope+scale+KV store | kq/softmax/kqv split-K (+quantize)
 //   | o-proj + residual | norm+mul+quantize | gate,up mat-vecs + gelu*up + quantize | down + residual
@@ -503,7 +503,7 @@ int gemma_model::emit_decode_step_kq() {
     return 0;
 }
 
-// The same token step, row-sharded over plan_.size ranks (SURVEY.md 8e).  Every rank keeps the replicated
+// The same token step, row-sharded over plan_.size ranks.  Every rank keeps the replicated
 // fp32 residual stream; each weight mat-vec computes this rank's rows only and the shards meet in four
 // allgathers per layer: attention output, o-proj (+residual), GeGLU activations (already Q8_0: int8 codes and
 // block scales are gathered, 4.25x fewer bytes than fp32), down-proj (+residual); plus 8 bytes per rank for the

@@ -16,7 +16,7 @@ typedef int32_t token_id; // ref: src/type.h
 enum class inference_stage { PREFILL, DECODE }; // ref: src/gemma_model.h:25-28
 
 // ref: gemma_hyper_param (src/gemma_model.h:30-40), read from GGUF keys at :403-415.  head_dim is
-// explicit (the reference derives n_embd/n_head, wrong for Gemma-7B; SURVEY.md §8).
+// explicit (the reference derives n_embd/n_head, wrong for Gemma-7B).
 struct gemma_config {
     int32_t n_embd, n_layer, n_head, n_head_kv, head_dim, n_ff, n_vocab, n_ctx;
     float eps, rope_base;
@@ -40,7 +40,7 @@ struct gemma_layer { // ref: gemma_layer (src/gemma_model.h:42-50 region)
     ggb_weight *sh_gate = nullptr, *sh_up = nullptr, *sh_down = nullptr;
 };
 
-// Row-sharded tensor parallelism (SURVEY.md 8e): every weight mat-vec is split by OUTPUT ROWS — the axis the
+// Row-sharded tensor parallelism: every weight mat-vec is split by OUTPUT ROWS — the axis the
 // reference already splits between its CPU threads and the GPU (ref: src/hpc.cpp:245-269) — so each output
 // element is computed by exactly one rank in the same K-order and sharded results are bit-identical to
 // 1-GPU results.  Pure host logic, testable without a GPU.
@@ -87,7 +87,7 @@ class gemma_model {
     int set_tensor_typed(int tensor_id, int type, const void *host_data, int64_t nbytes);
     bool kquant_mode() const { return kq_mode_; }
     int init_kv_cache();                       // ref: :361-401
-    int fill_kv_cache_synthetic(uint64_t seed); // bandwidth sweeps (SURVEY.md §8d)
+    int fill_kv_cache_synthetic(uint64_t seed); // bandwidth sweeps
     // ref: :665-747.  fused = true lowers the token step to the persistent decode kernel
     // (ggb_decoder_*); fused = false emits one ggb_op_* per (fused group of) graph node(s).
     int build_compute_graph(bool capture_acts, bool fused = true);

@@ -1,4 +1,4 @@
-// gguf_loader.h — GGUF file reader + Gemma tokenizer (SURVEY.md 8f-1, 8f-4).  Mirrors what the reference does through
+// gguf_loader.h — GGUF file reader + Gemma tokenizer.  Mirrors what the reference does through
 // ggml's gguf_* API (ref: src/gemma_model.cpp:19-51 load_model_from_file, :583-648 header KV / tensor table,
 // :403-415 hyper-parameters, :159-194 tensor binding by name, load_tokenizer) with a self-contained parser: the file
 // is read once, the 2 + 9 L tensors are handed to gemma_model::set_tensor (ggml AoS blocks, uploaded and repacked on
@@ -64,7 +64,7 @@ struct gemma_tokenizer {
 };
 
 // ref: init_hyper_param (:403-415).  head_dim comes from gemma.attention.key_length when present (the reference's
-// n_embd / n_head is wrong for Gemma-7B, SURVEY.md 8); n_ctx: 0 = the file's gemma.context_length
+// n_embd / n_head is wrong for Gemma-7B); n_ctx: 0 = the file's gemma.context_length
 int gguf_gemma_config(const gguf_file &f, int32_t n_ctx, gemma_config *cfg, std::string *err);
 // ref: load_tokenizer
 int gguf_gemma_tokenizer(const gguf_file &f, gemma_tokenizer *tok);

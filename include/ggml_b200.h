@@ -37,7 +37,7 @@ enum { GGB_TYPE_F32 = 0, GGB_TYPE_F16 = 1, GGB_TYPE_Q4_0 = 2, GGB_TYPE_Q8_0 = 8,
 
 /* Arithmetic: every result of the Q4_0 / Q8_0 decode path and of the K-quant operators is BIT-IDENTICAL to the scalar
  * ggml code the reference's CPU path runs (one fp32 accumulator per row, blocks in order; double accumulators where
- * ggml has them) - there is no kernel-specific summation order (DESIGN.md section 3).  The constants below are tiling
+ * ggml has them) - there is no kernel-specific summation order.  The constants below are tiling
  * parameters only: blocks per K segment of the decode kernel's pass stream, threads of the rms_norm partial sums
  * (double: insensitive to their grouping at fp32 precision), positions per attention item. */
 #define GGB_DEV_SEG_BLOCKS 64
@@ -95,7 +95,7 @@ int ggb_graph_kernel_count(const ggb_graph *g);
 typedef struct ggb_weight ggb_weight;
 int ggb_weight_upload(int type, int64_t rows, int64_t cols, const void *host_blocks, int64_t nb01,
                       ggb_weight **out);
-/* synthetic matrix generated and quantised on the device (SURVEY.md §8d generator):
+/* synthetic matrix generated and quantised on the device:
  * value(row, col) = synth(seed, tensor_id, row*cols + col) * sigma; bit-identical to the oracle's. */
 int ggb_weight_synth(int type, int64_t rows, int64_t cols, uint64_t seed, uint64_t tensor_id, float sigma,
                      ggb_weight **out);
@@ -136,7 +136,7 @@ int ggb_op_quantize_q8_0(const float *x, int64_t cols, int64_t T, void *q8);
 int ggb_op_q8_to_blocks(const void *q8, int64_t cols, int64_t T, void *blocks);   /* planar -> ggml AoS (34 B) */
 int ggb_op_q8_from_blocks(const void *blocks, int64_t cols, int64_t T, int64_t row_size, void *q8);
 
-/* K-quants (SURVEY.md 8f-2).  Blocks stay in ggml's AoS layout on the device.
+/* K-quants.  Blocks stay in ggml's AoS layout on the device.
  * ggb_type_row_bytes: bytes of one row of `cols` elements in `type` (0 for an unknown type).
  * ggb_op_quantize_q8_K: [UPSTREAM] quantize_row_q8_K (block: src/kernals.cl:29-34), rows x cols floats ->
  *   rows x cols/256 block_q8_K (292 B), bit-exact.

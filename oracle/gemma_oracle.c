@@ -266,7 +266,7 @@ void orc_model_reset(orc_model *m) {
     }
 }
 
-/* KV cache pre-filled with seeded ~N(0,1) values rounded to fp16 (SURVEY.md §8d, bandwidth sweeps);
+/* KV cache pre-filled with seeded ~N(0,1) values rounded to fp16 (bandwidth sweeps);
  * same generator and tensor ids (2*layer, 2*layer+1) as the device-side fill. */
 void orc_model_fill_kv_synth(orc_model *m, uint64_t seed) {
     const int64_t n = (int64_t)m->cfg.n_ctx * m->cfg.n_head_kv * m->cfg.head_dim;

@@ -21,7 +21,7 @@ typedef struct {
     int32_t wtype; /* ORC_TYPE_Q4_0 | ORC_TYPE_Q8_0, used for every 2-D matrix */
     int32_t pad_;
     uint64_t seed;
-    /* synthetic-weight std: token_embd / every other matrix.  SURVEY.md §8d uses 0.02 for both;
+    /* synthetic-weight std: token_embd / every other matrix.  0.02 for both is the default;
      * tests also use a small sigma_embd so the (tied) output projection does not simply echo
      * the input token and greedy parity is a sensitive check. */
     float sigma_embd, sigma_mat;

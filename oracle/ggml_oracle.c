@@ -3,10 +3,10 @@
  *
  * Each function cites what it follows.  "[UPSTREAM]" = semantics of the un-vendored ggml
  * (ggml.c / ggml-quants.c, llama.cpp circa Feb-Mar 2024) restated from its published
- * algorithm (SURVEY.md Appendix A); "ref:" = a file:line under /root/reference.
+ * algorithm; "ref:" = a file:line under /root/reference.
  * Build: gcc -O3 -ffp-contract=off (no FMA contraction, no fast-math).
  *
- * PINNING (DESIGN.md section 3).  Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference
+ * PINNING.  Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference
  * legs may load this library.
  *   - Q4_K x Q8_K and F16 x F16 dots: bit-identical to the REFERENCE'S OWN CODE (src/kernals.cl compiled where it lies
  *     into oracle/_ref, tests/test_kquants_cpu.py);
@@ -458,7 +458,7 @@ void orc_synth_row(uint64_t seed, uint64_t tensor_id, int64_t row, int64_t k, fl
         out[i] = bias + orc_synth_value(seed, tensor_id, (uint64_t)(row * k + i), sigma);
 }
 
-/* ------------------------------------------------------- K-quants (SURVEY.md 8f-2) */
+/* ------------------------------------------------------- K-quants */
 
 static inline int orc_nearest_int(float fval) { /* [UPSTREAM] ggml-quants.c nearest_int: round half to even */
     float val = fval + 12582912.f;

@@ -9,7 +9,7 @@
  * links or calls it.
  *
  * PARITY STATUS: "parity unpinned" by the reference's own fixtures — the
- * reference commits no golden tensors (SURVEY.md §8c).  What pins it instead:
+ * reference commits no golden tensors.  What pins it instead:
  *   - Q4_0 / Q8_0 codecs: known-answer vectors from gguf-py 0.19.0
  *     (tests/golden/, generator tests/golden/make_golden.py), whose Q8_0 is
  *     documented bit-exact to ggml-quants.c;
@@ -100,13 +100,13 @@ int32_t orc_argmax(int64_t n, const float *x);
 void orc_attn_decode_ref(int H, int Hkv, int d, int64_t n_pos, int64_t n_ctx, const float *q,
                          const uint16_t *kcache, const uint16_t *vcache, int64_t kv_stride, float *out);
 
-/* ---- synthetic weights (SURVEY.md §8d): counter-based, integer-exact ---- */
+/* ---- synthetic weights: counter-based, integer-exact ---- */
 uint64_t orc_splitmix64(uint64_t x);
 float orc_synth_value(uint64_t seed, uint64_t tensor_id, uint64_t index, float sigma);
 void orc_synth_row(uint64_t seed, uint64_t tensor_id, int64_t row, int64_t k, float sigma, float bias, float *out);
 
 
-/* ---- K-quants (SURVEY.md 8f-2): the formats the reference's own device kernels target ----
+/* ---- K-quants: the formats the reference's own device kernels target ----
  * block layouts: src/kernals.cl:13-34 (= ggml block_q4_K 144 B, block_q6_K 210 B, block_q8_K 292 B; QK_K = 256) */
 #define ORC_QK_K 256
 #define ORC_TYPE_Q4_K 12

@@ -1,6 +1,6 @@
 """Generate tests/golden/codecs_gguf.npz — known-answer vectors for the Q4_0 / Q8_0 codecs from
 gguf-py 0.19.0 (gguf/quants.py:220-251, 378-402; its Q8_0 is documented bit-exact to ggml-quants.c).
-The reference repo commits no golden tensors (SURVEY.md §8c), so these pin the oracle's codecs.
+The reference repo commits no golden tensors, so these pin the oracle's codecs.
 Run in the build container:  python tests/golden/make_golden.py
 """
 import os

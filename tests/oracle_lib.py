@@ -299,7 +299,7 @@ def tensor_id(layer, which):
     return 2 + 9 * layer + which
 
 
-# ---- K-quants (SURVEY.md 8f-2) -------------------------------------------------------------
+# ---- K-quants -------------------------------------------------------------
 TYPE_F16, TYPE_Q4_K, TYPE_Q6_K, TYPE_Q8_K = 1, 12, 14, 15
 KQ_BLOCK = {TYPE_Q4_K: 144, TYPE_Q6_K: 210, TYPE_Q8_K: 292}
 

@@ -1,4 +1,4 @@
-"""K-quant kernels (SURVEY.md 8f-2) against the oracle, bit for bit: quantize_row_q8_K, Q4_K / Q6_K x Q8_K and
+"""K-quant kernels against the oracle, bit for bit: quantize_row_q8_K, Q4_K / Q6_K x Q8_K and
 F16 x F16 through the device operator and through the drop-in entry ggb_mul_mat with host pointers
 (ref: src/kernals.cl:48-164, src/hpc.cpp:132-143, 216-277)."""
 import numpy as np

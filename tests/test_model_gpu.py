@@ -267,7 +267,7 @@ def _full_size_checks(gpu, dims, wtype, pos, token=4242):
 def test_full_size_gemma_2b_q4_0(gpu):
     """BASELINE config 2 at full size (Gemma-2B, Q4_0, n_kv = 2048)."""
     wb = _full_size_checks(gpu, dict(gpu.GEMMA_2B, n_ctx=2048), O.TYPE_Q4_0, 2047)
-    assert wb == 1409679360  # SURVEY.md 8d algorithmic bytes for 2B Q4_0
+    assert wb == 1409679360  # algorithmic bytes for 2B Q4_0
 
 
 def test_full_size_gemma_7b_q4_0(gpu):

@@ -76,7 +76,7 @@ def _matvec(gpu, W, act_f32, T, n, resid=None):
     return dst.download(np.float32).reshape(T, n)
 
 
-# the Gemma-2B / 7B (K, N) shapes of SURVEY.md §8a (N cut to keep the oracle in seconds) + ragged ones
+# the Gemma-2B / 7B (K, N) shapes (N cut to keep the oracle in seconds) + ragged ones
 SHAPES = [(2048, 2048), (2048, 256), (2048, 512), (16384, 256), (3072, 512), (4096, 384), (24576, 128),
           (2048, 1001), (64, 5), (4128, 33)]
 

@@ -1,7 +1,7 @@
 """GPU parity tests for the prefill path (mul_mat with col_num = T > 1): the dequant -> bf16 tcgen05 GEMM
 (csrc/prefill.cu) against a numpy model of the same contraction, and the prefill forward pass against the
 CPU oracle's REF-order forward pass within a stated tolerance (prefill rounds activations to bf16 instead
-of re-quantising them to Q8_0, so it is tolerance-exact, not bit-exact: DESIGN.md section 3)."""
+of re-quantising them to Q8_0, so it is tolerance-exact, not bit-exact)."""
 import numpy as np
 import pytest
 

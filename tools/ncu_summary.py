@@ -1,5 +1,5 @@
 """Summarise one kernel of an .ncu-rep into JSON: python tools/ncu_summary.py <report.ncu-rep> <kernel regex> <out.json>
-(reads `ncu -i <report> --page raw --csv`; keeps the metrics DESIGN.md / bench.py cite)."""
+(reads `ncu -i <report> --page raw --csv`; keeps the metrics that bench.py cites)."""
 import csv
 import io
 import json
