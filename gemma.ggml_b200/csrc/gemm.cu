@@ -10,10 +10,10 @@
 // without work, over several CTAs that meet in a workspace.  The number of pieces is what a split over the SMs in 256 x 256 tiles needs;
 // the tile is then the one with the least estimated time.
 //
-// What bounds it: 1024 x 8192 x 2048 runs in one round of 128 tiles, 32 stages of 1024 cycles of the tensor cores each (61 % of the kernel's
-// cycles); the stores behind the last stage, which nothing hides in a single round, take 6 us.  38.8 us, 885 TFLOP/s (47.6 us with both
-// operands copied by cp.async and rows stored by their own lanes; 40.9 us in 128 x 256 tiles).  32 experts x 128 rows, 1408 x 2048: 47 us a
-// product, 4.2 TB/s of matrices (256-row tiles, half of them empty: 68 us).
+// What bounds it: 1024 x 8192 x 2048 is 128 tiles of 256 x 256 on 74 pairs of CTAs, two rounds of 32 stages of 512 cycles of the tensor cores,
+// the second for 54 pairs; the tensor cores are busy for 61 to 64 % of the cycles.  37.3 us, 921 TFLOP/s (47.6 us with both operands
+// copied by cp.async and rows stored by their own lanes; 38.8 us in one round of 256 x 256 tiles a CTA, whose stores nothing hides).  32
+// experts x 128 rows, 1408 x 2048: 47 us a product, 4.2 TB/s of matrices (256-row tiles, half of them empty: 68 us).
 #include <cuda.h>
 #include <cuda_bf16.h>
 

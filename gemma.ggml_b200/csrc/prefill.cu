@@ -22,8 +22,8 @@
 //
 // What bounds it: shared memory (128 bytes a cycle).  A K block of a pair's CTA (256 rows, 128 weight rows) moves 40 KB in by TMA, 8 KB of codes
 // out, 16 KB of weights in and 64 to 96 KB out for the MMAs: 1550 cycles where the MMAs alone take 1024; the weights of a block stand half a
-// block before its MMAs.  512 tokens, Q8_0: gate | up with gelu 81 us, 848 TFLOP/s (115 us in two launches before), 2048 x 16384 60 us (85 us
-// with its reduction), 2048 x 2048 27 us.
+// block before its MMAs.  512 tokens, Q8_0: gate | up with gelu 82 us, 838 TFLOP/s, tensor cores 49 % of the cycles (115 us in two launches
+// before), 2048 x 16384 43 us with its reduction (68 us by one CTA a 256 x 256 tile), 2048 x 2048 20 us (36).
 //
 // Numerics: weights q*d are exact in fp32 (8 x 11 bits) and rounded once to bf16; activations are rounded
 // to bf16 instead of being re-quantised to Q8_0 per 32 (the reference's INIT stage), so prefill agrees with
@@ -798,7 +798,7 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     // 170 instructions of one lane), and no less than 1000, the way of a K block through its hands, however narrow the tile
     double best = -1.0;
     int splits = 1;
-    for (int MT = T > (pair ? 256 : 128) ? 2 : 1; MT >= 1; MT--)
+    for (int MT = 1; MT <= (T > (pair ? 256 : 128) ? 2 : 1); MT++) // the smaller of two that cost the same: 64 columns at 512 rows take longer
         for (int bn = pair ? 256 : 128; bn >= (geglu ? 256 : 64); bn /= 2)
             for (int sp = 1; sp <= pieces; sp *= 2) {
                 const int chunks = pieces / sp, chunk_kb = (kblocks + pieces - 1) / pieces, br = pair ? bn / 2 : bn, rows = MT * (pair ? 256 : 128);

@@ -4,7 +4,8 @@
 // A CTA owns 128 rows of queries: tokens x the query heads of one key head (for two maps: 64 of those, then the same 64 with the
 // second map), so a key tile is read once for the whole group and its causal edge is short.  Queries and weights are fp32 numbers and
 // stay so: each is the sum of three bf16 numbers (split3), so a product with a bf16 key or value is three products of the tensor cores,
-// exact before they are added up in fp32 tensor memory.
+// exact before they are added up in fp32 tensor memory (which truncates the running sum once per 16 of them: a score is off by up to 3 D / 16
+// steps of 2^-23, a weighted sum by half a step of 2^-24 per 16 keys and part; below the bf16 of the result).
 //
 //   scores   S [128][64 keys] = (q_l + q_m + q_h) K^T: queries in shared memory, K tile K-major as the cache rows lie
 //   weights  one thread a row (no shuffles): tcgen05.ld, soft cap, mask, exp or sigmoid, split, back to tensor memory over the scores
@@ -22,8 +23,8 @@
 //
 // What bounds it: the instructions around the weights, about 40 a number with a soft cap (2.2 us a tile on the 128 rows of an SM, of which
 // 1.0 us would be the MMAs alone).  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft
-// cap, gate: 55 us, 156 TFLOP/s of the products asked for (785 us by the fp32 CUDA cores, tiles of 32 queries x 32 keys); 777 tokens
-// of sigmoid heads at position 1024, no window: 63 us (686 us).  Unrolling the 64 scores of a row whole: 150 us.
+// cap, gate: 57 us, 151 TFLOP/s of the products asked for, tensor cores 26 % of the cycles (785 us by the fp32 CUDA cores, tiles of 32 queries x 32 keys); 777 tokens
+// of sigmoid heads at position 1024, no window: 64 us (686 us).  Unrolling the 64 scores of a row whole: 150 us.
 #pragma once
 
 #include "dense.cuh"
