@@ -23,8 +23,8 @@
 //
 // What bounds it: the instructions around the weights, about 40 a number with a soft cap (2.2 us a tile on the 128 rows of an SM, of which
 // 1.0 us would be the MMAs alone).  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft
-// cap, gate: 57 us, 151 TFLOP/s of the products asked for, tensor cores 26 % of the cycles (785 us by the fp32 CUDA cores, tiles of 32 queries x 32 keys); 777 tokens
-// of sigmoid heads at position 1024, no window: 64 us (686 us).  Unrolling the 64 scores of a row whole: 150 us.
+// cap, gate: 56 us, 154 TFLOP/s of the products asked for, tensor cores 26 % of the cycles (785 us by the fp32 CUDA cores, tiles of 32
+// queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 64 us (686 us).  Unrolling the 64 scores of a row whole: 150 us.
 #pragma once
 
 #include "dense.cuh"
@@ -201,7 +201,7 @@ struct row_job {
     float cap, r1, r2, pb;
 };
 // one row by one warp, a key a lane: weighted sums to out[Dv], maximum and denominator to *m_out and *l_out
-template <int MODE> __device__ __noinline__ void plain_row(const row_job &j, float *out, float *m_out, float *l_out) {
+template <int MODE> __device__ __forceinline__ void plain_row(const row_job &j, float *out, float *m_out, float *l_out) {
     const int lane = threadIdx.x & 31;
     const int64_t n_keep = MODE == SOFTMAX ? min(j.keep, j.lo) : 0, total = n_keep + (j.i - j.lo + 1);
     float acc[4] = {0.f, 0.f, 0.f, 0.f}, m = -INFINITY, l = 0.f; // Dv <= 128
@@ -234,10 +234,27 @@ template <int MODE> __device__ __noinline__ void plain_row(const row_job &j, flo
     __syncwarp();
 }
 
+// the rows of a warp's set bits (row warp + 8 b) once more; out of line, so that the code that every call runs through stays short
+template <int MODE, int MAPS>
+__device__ __noinline__ void plain_rows(const shape &a, uint32_t again, int64_t t0, int64_t i0, int g, int hpg, int n_pairs, float *of, float *st) {
+    constexpr int PR = kRows / MAPS;
+    const int warp = threadIdx.x >> 5;
+    while (again) {
+        const int rr = warp + 8 * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
+        again &= again - 1;
+        if (rp >= n_pairs) continue;
+        row_job j{a.q + (((t0 + rq) * a.H + h) * MAPS + rm) * a.D, a.cache + ((int64_t)g * MAPS + rm) * a.D, a.cache + (int64_t)a.G * MAPS * a.D + (int64_t)g * a.Dv,
+                  a.cache_ld, a.table, a.B, first_visible(i0 + rq, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i0 + rq, a.D, a.Dv, a.cap, 0.f, 0.f, 0.f};
+        if (MODE == SIGMOID && a.r1) j.r1 = a.r1[h], j.r2 = a.r2[h];
+        if (MODE == SIGMOID && a.pb) j.pb = a.pb[h];
+        plain_row<MODE>(j, of + rr * (a.Dv + 1), st + rr, st + kRows + rr);
+    }
+}
+
 // FIN: what becomes of a row, a warp's work when the sums stand in shared memory: load() requests what a row needs from memory, row()
 // gets it with the sums of the row (of both maps) and their maximum and denominators
 template <int MODE, int MAPS, typename FIN>
-__global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const FIN fin) {
+__global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant__ shape a, const FIN fin) {
     extern __shared__ uint8_t ta_raw[];
     const uint32_t raw0 = smem_u32(ta_raw), base = (raw0 + 1023u) & ~1023u;
     uint8_t *gbase = ta_raw + (base - raw0);
@@ -511,17 +528,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const shape a, const 
         // a warp's 16 rows: warp, warp + 8, ...; those whose sums are not finite once more, without the split
         {
             const int er = warp + 8 * (lane & 15);
-            uint32_t again = __ballot_sync(0xffffffffu, st[2 * kRows + er] + st[3 * kRows + er] != 0.f) & 0xffffu;
-            while (again) {
-                const int rr = warp + 8 * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
-                again &= again - 1;
-                if (rp >= n_pairs) continue;
-                row_job j{a.q + (((t0 + rq) * a.H + h) * MAPS + rm) * a.D, a.cache + ((int64_t)g * MAPS + rm) * a.D, a.cache + (int64_t)a.G * MAPS * a.D + (int64_t)g * a.Dv,
-                          a.cache_ld, a.table, a.B, first_visible(i0 + rq, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i0 + rq, a.D, a.Dv, a.cap, 0.f, 0.f, 0.f};
-                if (MODE == SIGMOID && a.r1) j.r1 = a.r1[h], j.r2 = a.r2[h];
-                if (MODE == SIGMOID && a.pb) j.pb = a.pb[h];
-                plain_row<MODE>(j, of + rr * op, st + rr, st + kRows + rr);
-            }
+            const uint32_t again = __ballot_sync(0xffffffffu, st[2 * kRows + er] + st[3 * kRows + er] != 0.f) & 0xffffu;
+            if (again) plain_rows<MODE, MAPS>(a, again, t0, i0, g, hpg, n_pairs, of, st);
         }
         // a warp a row, four rows' reads from memory in flight
         for (int p0 = warp; p0 < n_pairs; p0 += 32) {
