@@ -7,8 +7,8 @@
 //
 // A product along a long K is summed in `chunks` pieces of K, each with an accumulator of its own in tensor memory, added up in order by
 // the epilogue (the tensor cores truncate a running sum at every step: shorter sums are more exact), and, where that still leaves SMs
-// without work, over several CTAs that meet in a workspace.  The number of pieces is what a split over the SMs in 256 x 256 tiles needs;
-// the tile is then the one with the least estimated time.
+// without work, over several CTAs whose sums (each of its own pieces) meet in a workspace and are added in order.  The number of pieces is
+// what a split over the SMs in 256 x 256 tiles needs; the tile is then the one with the least estimated time.
 //
 // What bounds it: 1024 x 8192 x 2048 is 128 tiles of 256 x 256 on 74 pairs of CTAs, two rounds of 32 stages of 512 cycles of the tensor cores,
 // the second for 54 pairs; the tensor cores are busy for 61 to 64 % of the cycles.  37.3 us, 921 TFLOP/s (47.6 us with both operands
