@@ -16,6 +16,8 @@
 //
 // Weights and activations stay in ggml's AoS blocks (144 / 210 / 292 B): at 4.5 / 6.56 bits per weight a row of a
 // super-block is one 128 B + one 16 B line, so the warp's loads are already contiguous and a repack buys nothing.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace {
@@ -65,13 +67,6 @@ __device__ __forceinline__ int warp_sum_i32(int v) {
 __device__ __forceinline__ float finish_lanes(float sumf, float sums) {
 #pragma unroll
     for (int l = 0; l < 8; l++) sumf = __fadd_rn(sumf, __shfl_sync(0xffffffffu, sums, 4 * l));
-    return sumf;
-}
-
-// the same with the eight chains in lanes 0..7
-__device__ __forceinline__ float finish_lanes8(float sumf, float sums) {
-#pragma unroll
-    for (int l = 0; l < 8; l++) sumf = __fadd_rn(sumf, __shfl_sync(0xffffffffu, sums, l));
     return sumf;
 }
 
@@ -244,293 +239,332 @@ quantize_q8_K_kernel(const float *__restrict__ x, int64_t n_blocks, uint8_t *__r
 }
 
 
-// ---------------------------------------------------------------- Q4_K, packed form (resident weights)
-// The AoS kernel above spends 14 shuffles and ~60 instructions on a 144-byte super-block; it reaches 0.8-0.9 TB/s.  For
-// weights that stay on the device (ggb_mul_mat's cache) the super-block is re-laid out ONCE so that the four nibbles a
-// lane-sum index l meets inside a 32-element sub-block - elements l, 8 + l, 16 + l, 24 + l - are adjacent:
-//   block (144 B, same size) = d | dmin | scales[12] | X[8 sub-blocks][4 words], word p of sub-block j:
-//   bits 4g .. 4g+3 = nibble of element 32 j + 8 g + 2 p, bits 16 + 4g .. = nibble of element 32 j + 8 g + 2 p + 1.
-// The activation row is transposed the same way when a CTA stages it in shared memory (once per CTA, for all of its
-// rows): qT[j][l] = bytes q8[32 j + 8 g + l], g = 0..3.  Then lane (s, j) - super-block s of four, sub-block j - turns
-// its 16 bytes into eight dp4a (one per l), multiplies by its 6-bit scale, and a three-step folded butterfly inside
-// the 8-lane group leaves aux32[l = j] of super-block s in lane (s, j).  The fp32 part is the scalar code's, in its
-// order: the products d * aux32[l] of the four super-blocks are made in parallel, then lanes 0..7 add them to
-// sums[l] one by one; lane 0 does the same for sumf -= dmin * sumi.  4 shuffles per super-block instead of 14.
-constexpr int kActSB = 304; // staged activation super-block: qT 256 B | pair sums int[8] | d float | pad
+// ---------------------------------------------------------------- packed form (resident weights)
+// The AoS kernel above spends 14 shuffles and ~60 instructions on a super-block.  Weights that stay on the device are
+// re-laid out ONCE as fragments of integer tensor-core tiles: 16 rows x one sub-block are the A operand, and the B
+// operand's column l holds the activations of lane-sum index l (zero elsewhere), so one mma.sync gives the integer part
+// sum(code * a) of 16 rows x 8 lane sums; four multiply-adds a lane apply the sub-block's scales.  The integers are
+// exact in any order.  The fp32 part keeps the scalar order: a warp leaves d * aux32[l] of its super-block in shared
+// memory and 128 threads (row, l) add them to sums[l] super-block by super-block, then sumf += sums[0..7].
+//
+// A tile is 16 rows; a warp takes one super-block of it (an item), the warps of a CTA take consecutive super-blocks,
+// and the next item's 2.3 (Q4_K) or 3.3 KB (Q6_K) are on their way while one is computed.  Layout of an item with R rows
+// (R = 16; Q4_K's last tile has what is left, Q6_K pads it), lane (g, c) of the warp owning rows g and g + 8:
+//   Q4_K: header[R][16 B] as in ggml | X[2][R][4 c][16 B], word i of plane p: sub-block 4p + i, byte b: low nibble =
+//         element 4c + b, high nibble = element 16 + 4c + b                                     (144 B a row, as before)
+//   Q6_K: L[2][R][4 c][16 B], word i of plane p: low nibbles = elements 4c + b of sub-block 8p + 2i, high nibbles =
+//         those of 8p + 2i + 1 | H[R][4 c][16 B], word i: bits 2m of byte b = upper two bits (the top one inverted) of
+//         element 4c + b of sub-block 4i + m | scales[R][16] | d[R]                              (210 B a row)
+// A Q6_K byte (lo << 2 | hi << 6) with its top bit inverted is 4 * (q - 32) as int8; the 4 leaves by an exact shift.
+//
+// Bound by HBM and by the unpacking in turn (a tensor-core instruction's codes cost a warp about 15 others: instructions issue in 70 % of the
+// cycles, 5.1 TB/s).  256000 x 2048: Q6_K 122 -> 75 us, Q4_K 91 -> 72 us in graph replays (a row a
+// warp, a dot of four codes per instruction and lane sum).  A matrix of 256 rows, one tile a CTA, pays for the codes' longer way: 2.7 -> 3.0 us.
+constexpr int kActSB = 304;  // staged activation super-block, Q4_K: 256 B of codes | pair sums int[8] | d float | pad
+constexpr int kActSB6 = 272; // Q6_K: 256 B of codes | d float | pad
+constexpr int kTileRows = 16;
 
-__device__ __forceinline__ uint32_t ldg_u32(const uint8_t *p) { return __ldg(reinterpret_cast<const uint32_t *>(p)); }
+__host__ __device__ inline int64_t q6k_packed_bytes(int64_t rows, int nb) { return (rows + kTileRows - 1) / kTileRows * kTileRows * nb * kQ6K; }
 
+// thread = (row, super-block, c)
 __global__ void __launch_bounds__(256) q4k_repack_kernel(const uint8_t *__restrict__ raw, int64_t rows, int64_t nb01, int nb,
                                                         uint8_t *__restrict__ out) {
-    const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x; // (row, super-block, sub-block j)
-    if (idx >= rows * nb * 8) return;
-    const int j = (int)(idx & 7);
-    const int64_t rb = idx >> 3, row = rb / nb;
-    const int sb = (int)(rb - row * nb);
+    const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (idx >= rows * nb * 4) return;
+    const int c = (int)(idx & 3);
+    const int64_t rb = idx >> 2, row = rb / nb;
+    const int sb = (int)(rb - row * nb), r = (int)(row % kTileRows);
+    const int64_t row0 = row - r;
+    const int R = (int)min((int64_t)kTileRows, rows - row0);
     const uint8_t *x = raw + row * nb01 + (int64_t)sb * kQ4K;
-    uint8_t *o = out + (row * nb + sb) * kQ4K;
-    if (j < 4) *reinterpret_cast<uint32_t *>(o + 4 * j) = *reinterpret_cast<const uint32_t *>(x + 4 * j); // d, dmin, scales
-    const uint8_t *q = x + 16 + 32 * (j >> 1);
-    const int sh = (j & 1) * 4;
-    uint32_t w[4] = {0, 0, 0, 0};
-    for (int g = 0; g < 4; g++)
-        for (int l = 0; l < 8; l++) {
-            const uint32_t nib = (q[8 * g + l] >> sh) & 0xFu;
-            w[l >> 1] |= nib << (16 * (l & 1) + 4 * g);
+    uint8_t *o = out + (row0 * nb + (int64_t)sb * R) * kQ4K;
+    *reinterpret_cast<uint32_t *>(o + 16 * r + 4 * c) = ld_u32(x + 4 * c); // d, dmin, scales
+    for (int p = 0; p < 2; p++) {
+        uint32_t w[4];
+        for (int i = 0; i < 4; i++) { // sub-block j = 4p + i: nibble (j & 1) of the bytes of chunk j / 2
+            const int j = 4 * p + i, sh = (j & 1) * 4;
+            const uint8_t *q = x + 16 + 32 * (j >> 1) + 4 * c;
+            w[i] = ((ld_u32(q) >> sh) & 0x0f0f0f0fu) | (((ld_u32(q + 16) >> sh) & 0x0f0f0f0fu) << 4);
         }
-    *reinterpret_cast<uint4 *>(o + 16 + 16 * j) = make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-// grid (x: row groups, strided; y: activation row); 8 warps; dynamic shared memory nb * kActSB
-// F32ACT: `act` is the fp32 activation row (pitch row_size bytes); the CTA quantises it to Q8_K itself while staging
-// (ggml's INIT stage of the mul_mat node, fused: the stand-alone quantiser launch per node goes away)
-template <bool F32ACT>
-__global__ void __launch_bounds__(256)
-q4k_packed_kernel(const uint8_t *__restrict__ w, int64_t rows, int nb, const uint8_t *__restrict__ act, int64_t row_size,
-                  float *__restrict__ dst, int64_t dst_stride) {
-    extern __shared__ __align__(16) uint8_t s_act[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint8_t *y = act + (int64_t)blockIdx.y * row_size;
-    // ---- stage the activation row, transposed
-    if (F32ACT) {
-        const float *xf = reinterpret_cast<const float *>(y);
-        for (int sb = warp; sb < nb; sb += kWarps) { // a warp quantises one super-block at a time: lane = elements 8L..8L+7
-            const float4 f0 = *reinterpret_cast<const float4 *>(xf + sb * kQK + 8 * lane);
-            const float4 f1 = *reinterpret_cast<const float4 *>(xf + sb * kQK + 8 * lane + 4);
-            const float v[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-            int q[8];
-            const float d = q8k_quantize_lane(v, lane, q);
-            // element 8L + l = sub-block j = L / 4, group g = L % 4, lane-sum index l: byte g of qT[j][l]
-            const int j = lane >> 2, g = lane & 3;
-            uint8_t *base = s_act + sb * kActSB + j * 16 + g;
-            int ssum = 0;
-#pragma unroll
-            for (int l = 0; l < 8; l++) {
-                base[(l >> 2) * 128 + (l & 3) * 4] = (uint8_t)q[l];
-                ssum += q[l];
-            }
-            ssum += __shfl_xor_sync(0xffffffffu, ssum, 1);
-            ssum += __shfl_xor_sync(0xffffffffu, ssum, 2);
-            if (g == 0) *reinterpret_cast<int *>(s_act + sb * kActSB + 256 + 4 * j) = ssum; // bsums[2j] + bsums[2j + 1]
-            if (lane == 0) *reinterpret_cast<float *>(s_act + sb * kActSB + 288) = d;
-        }
-    } else {
-    for (int i = tid; i < nb * 64; i += 256) { // word (sb, j, l)
-        const int sb = i >> 6, j = (i >> 3) & 7, l = i & 7;
-        const uint8_t *q8 = y + (int64_t)sb * kQ8K + 4 + 32 * j + l;
-        const uint32_t v = (uint32_t)q8[0] | ((uint32_t)q8[8] << 8) | ((uint32_t)q8[16] << 16) | ((uint32_t)q8[24] << 24);
-        *reinterpret_cast<uint32_t *>(s_act + sb * kActSB + (l >> 2) * 128 + j * 16 + (l & 3) * 4) = v;
-    }
-    for (int i = tid; i < nb * 9; i += 256) {
-        const int sb = i / 9, k = i - sb * 9;
-        const uint8_t *yb = y + (int64_t)sb * kQ8K;
-        if (k < 8) {
-            const int16_t *bs = reinterpret_cast<const int16_t *>(yb + 260);
-            *reinterpret_cast<int *>(s_act + sb * kActSB + 256 + 4 * k) = (int)bs[2 * k] + (int)bs[2 * k + 1];
-        } else {
-            *reinterpret_cast<uint32_t *>(s_act + sb * kActSB + 288) = ld_u32(yb);
-        }
-    }
-    }
-    __syncthreads();
-    // lane (s, c): super-block s of EIGHT, sub-blocks 2c and 2c + 1 (64 elements per lane: the fold runs over four lanes
-    // only, and the scalar bookkeeping of an iteration is paid per eight super-blocks)
-    const int s = lane >> 2, c = lane & 3;
-    const bool b1 = lane & 2, b0 = lane & 1;
-    for (int64_t row = (int64_t)blockIdx.x * kWarps + warp; row < rows; row += (int64_t)gridDim.x * kWarps) {
-        const uint8_t *xrow = w + row * (int64_t)nb * kQ4K;
-        float sumsA = 0.0f, sumsB = 0.0f, sumf = 0.0f; // lane (0, c): sums[2c], sums[2c + 1]; lane 0: sumf
-#pragma unroll 1
-        for (int sb0 = 0; sb0 < nb; sb0 += 8) {
-            const int sb = sb0 + s;
-            const bool valid = sb < nb;
-            const uint8_t *blk = xrow + (int64_t)(valid ? sb : 0) * kQ4K;
-            const uint4 X0 = __ldg(reinterpret_cast<const uint4 *>(blk + 16 + 32 * c));
-            const uint4 X1 = __ldg(reinterpret_cast<const uint4 *>(blk + 32 + 32 * c));
-            const uint32_t dd = ldg_u32(blk);
-            uint32_t u0 = ldg_u32(blk + 4), u1 = ldg_u32(blk + 8), u2 = ldg_u32(blk + 12);
-            // 6-bit scales / mins (src/kernals.cl:75-80)
-            const uint32_t u3 = ((u2 >> 4) & 0x0f0f0f0fu) | (((u1 >> 6) & 0x03030303u) << 4);
-            const uint32_t uaux = u1 & 0x3f3f3f3fu;
-            u1 = (u2 & 0x0f0f0f0fu) | (((u0 >> 6) & 0x03030303u) << 4);
-            u2 = uaux;
-            u0 &= 0x3f3f3f3fu;
-            const uint32_t sc2 = ((c < 2 ? u0 : u1) >> (16 * (c & 1))) & 0xffffu; // scales of sub-blocks 2c, 2c + 1
-            const uint32_t mn2 = ((c < 2 ? u2 : u3) >> (16 * (c & 1))) & 0xffffu;
-            const uint8_t *ya = s_act + (valid ? sb : 0) * kActSB;
-            int v[8];
-#pragma unroll
-            for (int h = 0; h < 2; h++) { // sub-block j = 2c + h
-                const uint4 X = h ? X1 : X0;
-                const int scale = (int)((sc2 >> (8 * h)) & 0xff);
-                const uint4 qa = *reinterpret_cast<const uint4 *>(ya + 32 * c + 16 * h);       // qT[j][0..3]
-                const uint4 qb = *reinterpret_cast<const uint4 *>(ya + 128 + 32 * c + 16 * h); // qT[j][4..7]
-                const uint32_t xs[4] = {X.x, X.y, X.z, X.w};
-                const uint32_t qs[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#pragma unroll
-                for (int p = 0; p < 4; p++) {
-                    const uint32_t t1 = xs[p] & 0x0f0f0f0fu, t2 = (xs[p] >> 4) & 0x0f0f0f0fu;
-                    const int pe = __dp4a((int)__byte_perm(t1, t2, 0x5140), (int)qs[2 * p], 0);
-                    const int po = __dp4a((int)__byte_perm(t1, t2, 0x7362), (int)qs[2 * p + 1], 0);
-                    v[2 * p] = h ? v[2 * p] + scale * pe : scale * pe;
-                    v[2 * p + 1] = h ? v[2 * p + 1] + scale * po : scale * po;
-                }
-            }
-            // fold inside the 4-lane group: lane (s, c) ends with aux32[2c] and aux32[2c + 1]
-            int w4[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) w4[k] = (b1 ? v[4 + k] : v[k]) + __shfl_xor_sync(0xffffffffu, b1 ? v[k] : v[4 + k], 2);
-            const int aux0 = (b0 ? w4[2] : w4[0]) + __shfl_xor_sync(0xffffffffu, b0 ? w4[0] : w4[2], 1);
-            const int aux1 = (b0 ? w4[3] : w4[1]) + __shfl_xor_sync(0xffffffffu, b0 ? w4[1] : w4[3], 1);
-            const int *sp = reinterpret_cast<const int *>(ya + 256);
-            int sumi = (int)(mn2 & 0xff) * sp[2 * c] + (int)(mn2 >> 8) * sp[2 * c + 1];
-            sumi += __shfl_xor_sync(0xffffffffu, sumi, 1);
-            sumi += __shfl_xor_sync(0xffffffffu, sumi, 2);
-            const float yd = *reinterpret_cast<const float *>(ya + 288);
-            const float d = __fmul_rn(half_bits_to_float((uint16_t)(dd & 0xffff)), yd);
-            const float dmin = __fmul_rn(half_bits_to_float((uint16_t)(dd >> 16)), yd);
-            const float tA = valid ? __fmul_rn(d, (float)aux0) : 0.0f; // x + 0.0f == x: a missing super-block adds nothing
-            const float tB = valid ? __fmul_rn(d, (float)aux1) : 0.0f;
-            const float tm = valid ? __fmul_rn(dmin, (float)sumi) : 0.0f;
-            // the scalar order: the eight super-blocks one after the other
-            sumsA = __fadd_rn(sumsA, tA);
-            sumsB = __fadd_rn(sumsB, tB);
-            sumf = __fsub_rn(sumf, tm);
-#pragma unroll
-            for (int k = 1; k < 8; k++) {
-                sumsA = __fadd_rn(sumsA, __shfl_sync(0xffffffffu, tA, c + 4 * k)); // (meaningful in lanes 0..3)
-                sumsB = __fadd_rn(sumsB, __shfl_sync(0xffffffffu, tB, c + 4 * k));
-                sumf = __fsub_rn(sumf, __shfl_sync(0xffffffffu, tm, 4 * k));       // (meaningful in lane 0)
-            }
-        }
-#pragma unroll
-        for (int l = 0; l < 8; l++) {
-            const float a = __shfl_sync(0xffffffffu, (l & 1) ? sumsB : sumsA, l >> 1);
-            sumf = __fadd_rn(sumf, a);
-        }
-        if (lane == 0) dst[(int64_t)blockIdx.y * dst_stride + row] = sumf;
+        *reinterpret_cast<uint4 *>(o + 16 * R + (p * R + r) * 64 + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
-
-// ---------------------------------------------------------------- Q6_K, packed form (resident weights)
-// Same idea for Q6_K.  The 6-bit codes are expanded to int8 (q - 32) once - a row becomes W[nb][16 sub-blocks][16 B] |
-// scales[nb][16] | d[nb] (274 instead of 210 bytes per super-block: the kernel is bound by instruction issue, not by
-// HBM) - with word p of sub-block j = [a(g0, l = 2p), a(g1, 2p), a(g0, 2p + 1), a(g1, 2p + 1)], element = 16 j + 8 g + l,
-// and the activation words are staged in the same arrangement: two masked dp4a per word give the two lane sums.
-// Lane (s, c): super-block s of four, sub-blocks 2c and 2c + 1 of sixteen; the fold runs over the 8-lane group.
-constexpr int kActSB6 = 272; // staged activation super-block: qT 256 B | d float | pad
-
-__host__ __device__ inline int64_t q6k_packed_pitch(int nb) { return ((int64_t)nb * 274 + 15) & ~(int64_t)15; }
 
 __global__ void __launch_bounds__(256) q6k_repack_kernel(const uint8_t *__restrict__ raw, int64_t rows, int64_t nb01, int nb,
                                                         uint8_t *__restrict__ out) {
-    const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x; // (row, super-block, sub-block j)
-    if (idx >= rows * nb * 16) return;
-    const int j = (int)(idx & 15);
-    const int64_t rb = idx >> 4, row = rb / nb;
-    const int sb = (int)(rb - row * nb);
+    const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (idx >= rows * nb * 4) return;
+    const int c = (int)(idx & 3);
+    const int64_t rb = idx >> 2, row = rb / nb;
+    const int sb = (int)(rb - row * nb), r = (int)(row % kTileRows);
     const uint8_t *x = raw + row * nb01 + (int64_t)sb * kQ6K;
-    uint8_t *orow = out + row * q6k_packed_pitch(nb);
-    // element e of the scalar code's aux8 (ggml QK_K = 256 layout): chunk c = e / 128, quarter = (e % 128) / 32, i = e % 32
+    uint8_t *o = out + ((row - r) * nb + (int64_t)sb * kTileRows) * kQ6K;
+    // element e of the scalar code's aux8 (ggml QK_K = 256 layout): chunk e / 128, quarter = (e % 128) / 32, i = e % 32
     auto code = [&](int e) {
-        const int c = e >> 7, quarter = (e >> 5) & 3, i = e & 31;
-        const uint8_t ql = x[64 * c + 32 * (quarter & 1) + i], qh = x[128 + 32 * c + i];
-        const int lo = (quarter & 2) ? (ql >> 4) : (ql & 0xF);
-        return (int)(int8_t)(lo | (((qh >> (2 * quarter)) & 3) << 4)) - 32;
+        const int ch = e >> 7, quarter = (e >> 5) & 3, i = e & 31;
+        const uint8_t ql = x[64 * ch + 32 * (quarter & 1) + i], qh = x[128 + 32 * ch + i];
+        return (uint32_t)((quarter & 2) ? (ql >> 4) : (ql & 0xF)) | (uint32_t)((qh >> (2 * quarter)) & 3) << 4;
     };
-    uint32_t w[4];
-    for (int p = 0; p < 4; p++) {
-        const int e0 = 16 * j + 2 * p;
-        w[p] = (uint32_t)(uint8_t)code(e0) | ((uint32_t)(uint8_t)code(e0 + 8) << 8) | ((uint32_t)(uint8_t)code(e0 + 1) << 16) |
-               ((uint32_t)(uint8_t)code(e0 + 9) << 24);
-    }
-    *reinterpret_cast<uint4 *>(orow + ((int64_t)sb * 16 + j) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-    orow[(int64_t)nb * 256 + sb * 16 + j] = x[192 + j];
-    if (j == 0) *reinterpret_cast<uint16_t *>(orow + (int64_t)nb * 272 + 2 * sb) = *reinterpret_cast<const uint16_t *>(x + 208);
+    uint32_t lo[8] = {}, hi[4] = {};
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const uint32_t q = code(16 * j + 4 * c + b) ^ 0x20u;
+            lo[j >> 1] |= (q & 0xFu) << (8 * b + 4 * (j & 1));
+            hi[j >> 2] |= (q >> 4) << (8 * b + 2 * (j & 3));
+        }
+    for (int p = 0; p < 2; p++)
+        *reinterpret_cast<uint4 *>(o + (p * kTileRows + r) * 64 + 16 * c) = make_uint4(lo[4 * p], lo[4 * p + 1], lo[4 * p + 2], lo[4 * p + 3]);
+    *reinterpret_cast<uint4 *>(o + 128 * kTileRows + r * 64 + 16 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    for (int b = 0; b < 4; b++) o[192 * kTileRows + 16 * r + 4 * c + b] = x[192 + 4 * c + b];
+    if (c == 0) *reinterpret_cast<uint16_t *>(o + 208 * kTileRows + 2 * r) = *reinterpret_cast<const uint16_t *>(x + 208);
 }
 
-template <bool F32ACT>
-__global__ void __launch_bounds__(256)
-q6k_packed_kernel(const uint8_t *__restrict__ w, int64_t rows, int nb, const uint8_t *__restrict__ act, int64_t row_size,
-                  float *__restrict__ dst, int64_t dst_stride) {
+__device__ __forceinline__ uint4 ld_stream(const uint8_t *p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// byte i of w as a signed number
+template <int I>
+__device__ __forceinline__ int byte_s8(uint32_t w) {
+    int v;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(v) : "r"(w), "n"(0x8880 + 0x1111 * I));
+    return v;
+}
+
+__device__ __forceinline__ uint32_t comp(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// one item of a lane: rows g (index 0) and g + 8 (index 1)
+template <bool Q6>
+struct kq_item {
+    uint4 x[2][2];        // [row][plane]
+    uint4 h[Q6 ? 2 : 1];  // Q6_K: upper bits
+    uint4 hd[2];          // Q4_K: header, Q6_K: scales
+    uint16_t d[2];        // Q6_K
+
+    __device__ __forceinline__ void load(const uint8_t *w, int64_t rows, int nb, int64_t tile, int sb, int lane) {
+        const int g = lane >> 2;
+        const int64_t row0 = tile * kTileRows;
+        const int R = Q6 ? kTileRows : (int)min((int64_t)kTileRows, rows - row0);
+        const uint8_t *o = w + (row0 * nb + (int64_t)sb * R) * (Q6 ? kQ6K : kQ4K);
+        const uint8_t *codes = Q6 ? o : o + 16 * R;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int r = Q6 ? g + 8 * u : min(g + 8 * u, R - 1); // a row past the end is read as the last one and not stored
+#pragma unroll
+            for (int p = 0; p < 2; p++) x[u][p] = ld_stream(codes + (p * R + r) * 64 + 16 * (lane & 3));
+            if (Q6) {
+                h[Q6 ? u : 0] = ld_stream(o + 128 * kTileRows + r * 64 + 16 * (lane & 3));
+                hd[u] = __ldg(reinterpret_cast<const uint4 *>(o + 192 * kTileRows + 16 * r));
+                d[u] = __ldg(reinterpret_cast<const uint16_t *>(o + 208 * kTileRows + 2 * r));
+            } else {
+                hd[u] = __ldg(reinterpret_cast<const uint4 *>(o + 16 * r));
+            }
+        }
+    }
+};
+
+// aux32 of rows g and g + 8, lane sums 2c and 2c + 1, of a super-block whose activations start at ya: half a super-block at a time, the second half's
+// registers moved down
+__device__ __forceinline__ void kq_dot(const kq_item<true> &it, const uint8_t *ya, int c, uint32_t mask, int (&aux)[4]) {
+    uint4 x[2] = {it.x[0][0], it.x[1][0]};
+    uint2 h[2], sc[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) h[u] = make_uint2(it.h[u].x, it.h[u].y), sc[u] = make_uint2(it.hd[u].x, it.hd[u].y);
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+#pragma unroll
+        for (int jq = 0; jq < 2; jq++) {
+            const uint4 act = *reinterpret_cast<const uint4 *>(ya + 128 * p + 64 * jq + 16 * c);
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                const int j = 4 * jq + m; // of the half
+                uint32_t a[2];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const uint32_t lo = comp(x[u], j >> 1), hi = jq ? h[u].y : h[u].x;
+                    a[u] = ((j & 1 ? lo >> 2 : lo << 2) & 0x3c3c3c3cu) | ((hi << (6 - 2 * m)) & 0xc0c0c0c0u);
+                }
+                int v[4];
+                asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a[0]), "r"(a[1]), "r"(comp(act, m) & mask), "r"(0));
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const uint32_t w = jq ? sc[u].y : sc[u].x;
+                    const int s = m == 0 ? byte_s8<0>(w) : m == 1 ? byte_s8<1>(w) : m == 2 ? byte_s8<2>(w) : byte_s8<3>(w);
+                    aux[2 * u] += s * v[2 * u];
+                    aux[2 * u + 1] += s * v[2 * u + 1];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) x[u] = it.x[u][1], h[u] = make_uint2(it.h[u].z, it.h[u].w), sc[u] = make_uint2(it.hd[u].z, it.hd[u].w);
+    }
+}
+
+__device__ __forceinline__ void kq_dot(const kq_item<false> &it, const uint8_t *ya, int c, uint32_t mask, int (&aux)[4]) {
+    uint4 x[2] = {it.x[0][0], it.x[1][0]};
+    uint32_t sc[2] = {it.hd[0].y & 0x3f3f3f3fu, it.hd[1].y & 0x3f3f3f3fu}; // 6-bit scales of sub-blocks 0..3 (src/kernals.cl:75-80)
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+#pragma unroll
+        for (int jp = 0; jp < 2; jp++) {
+            const uint4 act = *reinterpret_cast<const uint4 *>(ya + 128 * p + 64 * jp + 16 * c);
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                const int j = 2 * jp + m; // of the half
+                const uint32_t x0 = comp(x[0], j), x1 = comp(x[1], j);
+                int v[4];
+                asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                    : "r"(x0 & 0x0f0f0f0fu), "r"(x1 & 0x0f0f0f0fu), "r"((x0 >> 4) & 0x0f0f0f0fu), "r"((x1 >> 4) & 0x0f0f0f0fu),
+                      "r"((m ? act.z : act.x) & mask), "r"((m ? act.w : act.y) & mask), "r"(0));
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int s = (int)((sc[u] >> (8 * j)) & 0xff);
+                    aux[2 * u] += s * v[2 * u];
+                    aux[2 * u + 1] += s * v[2 * u + 1];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) { // sub-blocks 4..7
+            x[u] = it.x[u][1];
+            sc[u] = (it.hd[u].w & 0x0f0f0f0fu) | (((it.hd[u].y >> 6) & 0x03030303u) << 4);
+        }
+    }
+}
+
+// where word wi (elements 4 wi .. 4 wi + 3) of a super-block's activations is staged: a lane's words of four (Q6_K) or
+// two (Q4_K) sub-blocks are adjacent
+template <bool Q6>
+__device__ __forceinline__ int act_word(int wi) {
+    return Q6 ? (wi >> 4) * 64 + (wi & 3) * 16 + ((wi >> 2) & 3) * 4 : (wi >> 4) * 64 + (wi & 3) * 16 + ((wi >> 3) & 1) * 8 + ((wi >> 2) & 1) * 4;
+}
+
+// grid (x: groups of P tiles, strided; y: activation row); `chunk` super-blocks of a tile are computed at once, by a warp each:
+// P > 1 only where chunk = nb.  Dynamic shared memory: nb staged super-blocks.
+// F32ACT: `act` is the fp32 activation row (pitch row_size bytes); the CTA quantises it to Q8_K itself while staging
+template <bool Q6, bool F32ACT>
+__global__ void __launch_bounds__(kWarps * 32, 2)
+kq_packed_kernel(const uint8_t *__restrict__ w, int64_t rows, int nb, const uint8_t *__restrict__ act, int64_t row_size,
+                 float *__restrict__ dst, int64_t dst_stride, int P, int chunk) {
+    constexpr int SB = Q6 ? kActSB6 : kActSB, kD = Q6 ? 256 : 288;
     extern __shared__ __align__(16) uint8_t s_act[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ __align__(16) float s_t[2][kWarps][kTileRows * 8];
+    __shared__ float s_m[Q6 ? 1 : 2][Q6 ? 1 : kWarps][kTileRows];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    const int g = lane >> 2, c = lane & 3;
+    const int64_t n_tiles = (rows + kTileRows - 1) / kTileRows, n_groups = (n_tiles + P - 1) / P;
+    const int ip = warp / chunk, ik = warp - ip * chunk; // this warp's item of a round: tile ip of the group, super-block ik of the chunk
+    kq_item<Q6> cur, nxt;
+    int64_t grp = blockIdx.x;
+    int sb0 = 0;
+    auto valid = [&](int64_t gr, int s0) { return gr < n_groups && gr * P + ip < n_tiles && ip < P && s0 + ik < nb; };
+    if (valid(grp, 0)) cur.load(w, rows, nb, grp * P + ip, ik, lane); // weights first: they take longest
+    // ---- stage the activation row
     const uint8_t *y = act + (int64_t)blockIdx.y * row_size;
     if (F32ACT) {
         const float *xf = reinterpret_cast<const float *>(y);
-        for (int sb = warp; sb < nb; sb += kWarps) {
+        for (int sb = warp; sb < nb; sb += n_warps) { // a warp quantises one super-block at a time: lane = elements 8L..8L+7
             const float4 f0 = *reinterpret_cast<const float4 *>(xf + sb * kQK + 8 * lane);
             const float4 f1 = *reinterpret_cast<const float4 *>(xf + sb * kQK + 8 * lane + 4);
             const float v[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
             int q[8];
             const float d = q8k_quantize_lane(v, lane, q);
-            // element 8L + l = sub-block j = L / 2 (of sixteen), group g = L % 2: word l / 2, byte 2 (l % 2) + g
-            uint8_t *base = s_act + sb * kActSB6 + (lane >> 1) * 16 + (lane & 1);
+            uint8_t *base = s_act + sb * SB;
 #pragma unroll
-            for (int l = 0; l < 8; l++) base[(l >> 1) * 4 + (l & 1) * 2] = (uint8_t)q[l];
-            if (lane == 0) *reinterpret_cast<float *>(s_act + sb * kActSB6 + 256) = d;
+            for (int u = 0; u < 2; u++)
+                *reinterpret_cast<uint32_t *>(base + act_word<Q6>(2 * lane + u)) =
+                    (q[4 * u] & 0xff) | ((q[4 * u + 1] & 0xff) << 8) | ((q[4 * u + 2] & 0xff) << 16) | ((uint32_t)(q[4 * u + 3] & 0xff) << 24);
+            if (!Q6) {
+                int ssum = 0;
+#pragma unroll
+                for (int l = 0; l < 8; l++) ssum += q[l];
+                ssum += __shfl_xor_sync(0xffffffffu, ssum, 1);
+                ssum += __shfl_xor_sync(0xffffffffu, ssum, 2);
+                if (c == 0) *reinterpret_cast<int *>(base + 256 + 4 * g) = ssum; // bsums[2j] + bsums[2j + 1]
+            }
+            if (lane == 0) *reinterpret_cast<float *>(base + kD) = d;
         }
     } else {
-    for (int i = tid; i < nb * 64; i += 256) { // word (sb, j, p)
-        const int sb = i >> 6, j = (i >> 2) & 15, p = i & 3;
-        const uint8_t *q8 = y + (int64_t)sb * kQ8K + 4 + 16 * j + 2 * p;
-        const uint32_t v = (uint32_t)q8[0] | ((uint32_t)q8[8] << 8) | ((uint32_t)q8[1] << 16) | ((uint32_t)q8[9] << 24);
-        *reinterpret_cast<uint32_t *>(s_act + sb * kActSB6 + j * 16 + p * 4) = v;
-    }
-    for (int sb = tid; sb < nb; sb += 256) *reinterpret_cast<uint32_t *>(s_act + sb * kActSB6 + 256) = ld_u32(y + (int64_t)sb * kQ8K);
+        for (int i = tid; i < nb * 64; i += blockDim.x)
+            *reinterpret_cast<uint32_t *>(s_act + (i >> 6) * SB + act_word<Q6>(i & 63)) = ld_u32(y + (int64_t)(i >> 6) * kQ8K + 4 + 4 * (i & 63));
+        for (int i = tid; i < nb * 9; i += blockDim.x) {
+            const int sb = i / 9, k = i - sb * 9;
+            const uint8_t *yb = y + (int64_t)sb * kQ8K;
+            if (k == 8) *reinterpret_cast<uint32_t *>(s_act + sb * SB + kD) = ld_u32(yb);
+            else if (!Q6) {
+                const int16_t *bs = reinterpret_cast<const int16_t *>(yb + 260);
+                *reinterpret_cast<int *>(s_act + sb * SB + 256 + 4 * k) = (int)bs[2 * k] + (int)bs[2 * k + 1];
+            }
+        }
     }
     __syncthreads();
-    // lane (s, c): super-block s of four, sub-blocks 2c and 2c + 1 (32 elements per lane); the fold runs over the 8-lane group
-    const int s = lane >> 3, c = lane & 7;
-    const bool b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
-    const int64_t pitch = q6k_packed_pitch(nb);
-    for (int64_t row = (int64_t)blockIdx.x * kWarps + warp; row < rows; row += (int64_t)gridDim.x * kWarps) {
-        const uint8_t *xrow = w + row * pitch;
-        float sums = 0.0f; // lane (0, l): sums[l]
-#pragma unroll 1
-        for (int sb0 = 0; sb0 < nb; sb0 += 4) {
-            const int sb = sb0 + s;
-            const bool valid = sb < nb;
-            const int sbc = valid ? sb : 0;
-            const uint8_t *xw = xrow + ((int64_t)sbc * 16 + 2 * c) * 16;
-            const uint4 X0 = __ldg(reinterpret_cast<const uint4 *>(xw)), X1 = __ldg(reinterpret_cast<const uint4 *>(xw + 16));
-            const uint32_t sc2 = __ldg(reinterpret_cast<const uint16_t *>(xrow + (int64_t)nb * 256 + sbc * 16 + 2 * c));
-            const uint16_t dh = __ldg(reinterpret_cast<const uint16_t *>(xrow + (int64_t)nb * 272 + 2 * sbc));
-            const uint8_t *ya = s_act + sbc * kActSB6;
-            const uint4 q0 = *reinterpret_cast<const uint4 *>(ya + 32 * c), q1 = *reinterpret_cast<const uint4 *>(ya + 32 * c + 16);
-            int v[8];
+    const uint32_t mask = (g >> 2) == (c & 1) ? 0xffu << (8 * (g & 3)) : 0u; // of the elements 4c .. 4c + 3, those = g mod 8
+    float sums = 0.f, sumf = 0.f; // P == 1: thread (row, l)'s chains, carried from chunk to chunk
+    int buf = 0;
+    while (grp < n_groups) {
+        int64_t grp_n = grp;
+        int sb_n = sb0 + chunk;
+        if (sb_n >= nb) { sb_n = 0; grp_n += gridDim.x; }
+        if (valid(grp_n, sb_n)) nxt.load(w, rows, nb, grp_n * P + ip, sb_n + ik, lane);
+        if (valid(grp, sb0)) {
+            const uint8_t *ya = s_act + (sb0 + ik) * SB;
+            int aux[4] = {0, 0, 0, 0};
+            kq_dot(cur, ya, c, mask, aux);
+            const float yd = *reinterpret_cast<const float *>(ya + kD);
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const uint4 X = h ? X1 : X0, q = h ? q1 : q0;
-                const int scale = (int)(int8_t)(sc2 >> (8 * h));
-                const uint32_t xs[4] = {X.x, X.y, X.z, X.w}, qs[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                for (int p = 0; p < 4; p++) {
-                    const int pe = __dp4a((int)(xs[p] & 0x0000ffffu), (int)qs[p], 0);
-                    const int po = __dp4a((int)(xs[p] & 0xffff0000u), (int)qs[p], 0);
-                    v[2 * p] = h ? v[2 * p] + scale * pe : scale * pe;
-                    v[2 * p + 1] = h ? v[2 * p + 1] + scale * po : scale * po;
+            for (int u = 0; u < 2; u++) {
+                const float d = __fmul_rn(half_bits_to_float(Q6 ? cur.d[u] : (uint16_t)(cur.hd[u].x & 0xffff)), yd);
+                const float t0 = __fmul_rn(d, (float)(Q6 ? aux[2 * u] >> 2 : aux[2 * u]));
+                const float t1 = __fmul_rn(d, (float)(Q6 ? aux[2 * u + 1] >> 2 : aux[2 * u + 1]));
+                *reinterpret_cast<float2 *>(&s_t[buf][warp][(g + 8 * u) * 8 + 2 * c]) = make_float2(t0, t1);
+                if (!Q6) {
+                    const uint32_t u2 = cur.hd[u].z & 0x3f3f3f3fu, u3 = ((cur.hd[u].w >> 4) & 0x0f0f0f0fu) | (((cur.hd[u].z >> 6) & 0x03030303u) << 4);
+                    const uint32_t mn2 = ((c < 2 ? u2 : u3) >> (16 * (c & 1))) & 0xffffu; // mins of sub-blocks 2c, 2c + 1
+                    const int *sp = reinterpret_cast<const int *>(ya + 256);
+                    int sumi = (int)(mn2 & 0xff) * sp[2 * c] + (int)(mn2 >> 8) * sp[2 * c + 1];
+                    sumi += __shfl_xor_sync(0xffffffffu, sumi, 1);
+                    sumi += __shfl_xor_sync(0xffffffffu, sumi, 2);
+                    const float dmin = __fmul_rn(half_bits_to_float((uint16_t)(cur.hd[u].x >> 16)), yd);
+                    if (c == 0) s_m[Q6 ? 0 : buf][Q6 ? 0 : warp][g + 8 * u] = __fmul_rn(dmin, (float)sumi);
                 }
             }
-            int w4[4], w2[2];
-#pragma unroll
-            for (int k = 0; k < 4; k++) w4[k] = (b2 ? v[4 + k] : v[k]) + __shfl_xor_sync(0xffffffffu, b2 ? v[k] : v[4 + k], 4);
-#pragma unroll
-            for (int k = 0; k < 2; k++) w2[k] = (b1 ? w4[2 + k] : w4[k]) + __shfl_xor_sync(0xffffffffu, b1 ? w4[k] : w4[2 + k], 2);
-            const int aux = (b0 ? w2[1] : w2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? w2[0] : w2[1], 1); // aux32[l = c]
-            const float d = __fmul_rn(half_bits_to_float(dh), *reinterpret_cast<const float *>(ya + 256));
-            const float t = valid ? __fmul_rn(d, (float)aux) : 0.0f;
-            sums = __fadd_rn(sums, t); // the scalar order: the four super-blocks one after the other (lanes 0..7)
-#pragma unroll
-            for (int k = 1; k < 4; k++) sums = __fadd_rn(sums, __shfl_sync(0xffffffffu, t, c + 8 * k));
         }
-        float sumf = 0.0f;
+        __syncthreads();
+        // the scalar order: the super-blocks one after the other.  Two tables: the next round writes the other one.
+        for (int ch = tid; ch < P * kTileRows * 8; ch += blockDim.x) {
+            const int p = ch >> 7, r = (ch >> 3) & 15, l = ch & 7, n = min(chunk, nb - sb0);
+            float tv[kWarps], mv[kWarps];
 #pragma unroll
-        for (int l = 0; l < 8; l++) sumf = __fadd_rn(sumf, __shfl_sync(0xffffffffu, sums, l));
-        if (lane == 0) dst[(int64_t)blockIdx.y * dst_stride + row] = sumf;
+            for (int k = 0; k < kWarps; k++) { // past the end: x + 0 and x - 0 are x (no chain ever holds -0)
+                const int i = min(p * chunk + k, kWarps - 1);
+                tv[k] = k < n ? s_t[buf][i][r * 8 + l] : 0.f;
+                mv[k] = !Q6 && k < n ? s_m[Q6 ? 0 : buf][Q6 ? 0 : i][r] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < kWarps; k++) {
+                sums = __fadd_rn(sums, tv[k]);
+                if (!Q6) sumf = __fsub_rn(sumf, mv[k]);
+            }
+            if (sb0 + chunk >= nb) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) sumf = __fadd_rn(sumf, __shfl_sync(0xffffffffu, sums, (lane & 24) + i));
+                const int64_t row = (grp * P + p) * kTileRows + r;
+                if (l == 0 && row < rows) dst[(int64_t)blockIdx.y * dst_stride + row] = sumf;
+                sums = sumf = 0.f;
+            }
+        }
+        buf ^= 1;
+        grp = grp_n;
+        sb0 = sb_n;
+        cur = nxt;
     }
 }
-
 
 // ---------------------------------------------------------------- get_rows on K-quant blocks (embedding lookup)
 // [UPSTREAM] dequantize_row_q4_K / dequantize_row_q6_K for the rows ids[t], times `scale` (ggml_scale): one thread per
@@ -607,7 +641,7 @@ int ggb_op_q4k_repack(const void *raw, int64_t rows, int64_t nb01, int64_t K, vo
     GGB_CHECK_ARG(raw && packed && rows > 0 && K > 0 && K % kQK == 0 && nb01 >= K / kQK * kQ4K && nb01 % 4 == 0,
                   "q4k_repack: bad arguments");
     const int nb = (int)(K / kQK);
-    const int64_t n = rows * nb * 8;
+    const int64_t n = rows * nb * 4;
     q4k_repack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ggb_cuda_stream()>>>((const uint8_t *)raw, rows, nb01, nb,
                                                                                  (uint8_t *)packed);
     GGB_LAUNCH_CHECK();
@@ -624,15 +658,19 @@ static int launch_packed(int type, bool f32act, const void *packed, int64_t rows
     const bool q4 = type == GGB_TYPE_Q4_K;
     const size_t smem = (size_t)nb * (q4 ? kActSB : kActSB6);
     GGB_CHECK_ARG(smem <= 200 * 1024, "mul_mat_packed: K %lld too long for the staged activation row", (long long)K);
-    auto kern = q4 ? (f32act ? q4k_packed_kernel<true> : q4k_packed_kernel<false>)
-                   : (f32act ? q6k_packed_kernel<true> : q6k_packed_kernel<false>);
-    if (smem > 48 * 1024) GGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t groups = (rows + kWarps - 1) / kWarps;
-    const unsigned gx = (unsigned)(groups < 148 * 8 ? groups : 148 * 8);
+    auto kern = q4 ? (f32act ? kq_packed_kernel<false, true> : kq_packed_kernel<false, false>)
+                   : (f32act ? kq_packed_kernel<true, true> : kq_packed_kernel<true, false>);
+    if (smem > 32 * 1024) GGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The super-blocks of a tile in as few rounds of at most 8 warps as they need, evenly.  Several tiles a CTA where a row is short and tiles are
+    // left for every SM all the same; 16 warps an SM (128 registers a thread).
+    const int64_t tiles = (rows + kTileRows - 1) / kTileRows;
+    const int rounds = (nb + kWarps - 1) / kWarps, chunk = (nb + rounds - 1) / rounds;
+    const int P = rounds > 1 ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(kWarps / nb, tiles / ggb_sm_count())), warps = chunk * P;
+    const unsigned gx = (unsigned)std::min<int64_t>((tiles + P - 1) / P, (int64_t)ggb_sm_count() * (2 * kWarps / warps));
     for (int64_t t0 = 0; t0 < T; t0 += 65535) {
         const dim3 grid(gx, (unsigned)(T - t0 < 65535 ? T - t0 : 65535));
-        kern<<<grid, 256, smem, ggb_cuda_stream()>>>((const uint8_t *)packed, rows, nb, (const uint8_t *)act + t0 * row_size,
-                                                     row_size, dst + t0 * dst_stride, dst_stride);
+        kern<<<grid, warps * 32, smem, ggb_cuda_stream()>>>((const uint8_t *)packed, rows, nb, (const uint8_t *)act + t0 * row_size,
+                                                            row_size, dst + t0 * dst_stride, dst_stride, P, chunk);
         GGB_LAUNCH_CHECK();
     }
     return GGB_OK;
@@ -654,14 +692,14 @@ int ggb_op_mul_mat_kq_packed_f32(int type, const void *packed, int64_t rows, int
     return launch_packed(type, true, packed, rows, K, x, K * 4, T, dst, dst_stride);
 }
 
-size_t ggb_q6k_packed_bytes(int64_t rows, int64_t K) { return (size_t)rows * (size_t)q6k_packed_pitch((int)(K / kQK)); }
+size_t ggb_q6k_packed_bytes(int64_t rows, int64_t K) { return (size_t)q6k_packed_bytes(rows, (int)(K / kQK)); }
 
 int ggb_op_q6k_repack(const void *raw, int64_t rows, int64_t nb01, int64_t K, void *packed) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(raw && packed && rows > 0 && K > 0 && K % kQK == 0 && nb01 >= K / kQK * kQ6K && nb01 % 2 == 0,
                   "q6k_repack: bad arguments");
     const int nb = (int)(K / kQK);
-    const int64_t n = rows * nb * 16;
+    const int64_t n = rows * nb * 4;
     q6k_repack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ggb_cuda_stream()>>>((const uint8_t *)raw, rows, nb01, nb,
                                                                                  (uint8_t *)packed);
     GGB_LAUNCH_CHECK();

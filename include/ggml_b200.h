@@ -147,14 +147,14 @@ size_t ggb_type_row_bytes(int type, int64_t cols);
 int ggb_op_quantize_q8_K(const float *x, int64_t cols, int64_t rows, void *out);
 int ggb_op_mul_mat_blocks(int type, const void *w, int64_t rows, int64_t nb01, int64_t K, const void *act,
                           int64_t row_size, int64_t T, float *dst, int64_t dst_stride);
-/* Q4_K weights that stay on the device: ggb_op_q4k_repack re-lays a matrix out once (same 144 B per super-block, the
- * nibbles that share a lane-sum index adjacent), ggb_op_mul_mat_q4k_packed is the mat-vec on that layout (same bits as
- * ggb_op_mul_mat_blocks / src/kernals.cl:48-111, ~4x its throughput).  ggb_mul_mat uses it for its cached src0. */
+/* Q4_K weights that stay on the device: ggb_op_q4k_repack re-lays a matrix out once (same 144 B per super-block, in
+ * tiles of 16 rows), ggb_op_mul_mat_q4k_packed is the mat-vec on that layout (same bits as
+ * ggb_op_mul_mat_blocks / src/kernals.cl:48-111, several times its throughput).  ggb_mul_mat uses it for its cached src0. */
 int ggb_op_q4k_repack(const void *raw, int64_t rows, int64_t nb01, int64_t K, void *packed);
 int ggb_op_mul_mat_q4k_packed(const void *packed, int64_t rows, int64_t K, const void *act, int64_t row_size, int64_t T,
                               float *dst, int64_t dst_stride);
-/* the same for Q6_K: codes expanded to int8 (q - 32) in the transposed arrangement; ggb_q6k_packed_bytes = size of the
- * packed matrix (274 B per super-block, rows padded to 16 B) */
+/* the same for Q6_K (210 B per super-block); ggb_q6k_packed_bytes = size of the packed matrix, whose last tile is 16 rows
+ * whatever it holds */
 /* the packed mat-vecs on an fp32 activation row x[t][K]: the kernel quantises the row to Q8_K itself while it stages it
  * (ggml's INIT stage of the mul_mat node fused into the COMPUTE stage; same bits as quantize + packed mat-vec) */
 int ggb_op_mul_mat_kq_packed_f32(int type, const void *packed, int64_t rows, int64_t K, const float *x, int64_t T, float *dst,
