@@ -12,7 +12,7 @@
 // the left and four for the right operand, two steps ahead, one warp issuing the MMAs.
 //
 // What bounds it: the MMAs (58 % of the tensor cores' cycles, a half of the scores repeated at R > 256), then the rounds in which the weights
-// of a tile wait for its last scores.  1024 tokens x 16 heads at position 1024, R = 512, Dr = 64: 245 us, 228 TFLOP/s of the products asked
+// of a tile wait for its last scores.  1024 tokens x 16 heads at position 1024, R = 512, Dr = 64: 234 us, 239 TFLOP/s of the products asked
 // for (3420 us on the fp32 CUDA cores, two tokens a CTA); from 9 tokens on: fewer are steps, which spread their positions over warps.
 //
 // Infinite numbers are not the sums of their parts: a row (of a CTA) or an output whose sums are not finite is computed once more by fp32
@@ -61,8 +61,8 @@ __device__ __forceinline__ void store_left(uint32_t dst, int tid, const float4 (
     for (int u = 0; u < 8; u++) {
         const int g = tid + 256 * u, r = g >> 4, d = 4 * (g & 15);
         uint32_t h[2], m[2], l[2];
-        split3(x[u].x, x[u].y, h[0], m[0], l[0]);
-        split3(x[u].z, x[u].w, h[1], m[1], l[1]);
+        split3(pack2(x[u].x, x[u].y), h[0], m[0], l[0]);
+        split3(pack2(x[u].z, x[u].w), h[1], m[1], l[1]);
         const uint32_t at = dst + r * 128 + (((d >> 3) ^ (r & 7)) << 4) + (d & 4) * 2;
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(h[0]), "r"(h[1]) : "memory");
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + kPart), "r"(m[0]), "r"(m[1]) : "memory");
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
             for (int s = 0; s < subs; s++) {
                 // weights of 64 positions, 32 a group: four 16-byte pieces of each part of the thread's row
                 uint32_t ph[16], pm[16], pl[16];
-                float sum[4] = {0.f, 0.f, 0.f, 0.f};
+                f32x2 sum[2] = {0, 0};
 #pragma unroll
                 for (int hf = 0; hf < 2; hf++) {
                     const int c0 = kSub * s + 32 * grp + 16 * hf;
@@ -320,14 +320,15 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
                         for (int c = 0; c < 16; c++) p[c] = (c0 + c < c_hi && c0 + c >= c_lo) ? p[c] : -INFINITY;
                     }
 #pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        p[c] = expf(p[c] - mm);
-                        sum[c & 3] += p[c];
+                    for (int c = 0; c < 8; c++) { // exp(s - m) = 2^((s - m) log2 e), as in tile_attention.cuh
+                        const float2 t = unpack2(mul2(add2(pack2(p[2 * c], p[2 * c + 1]), pack2(-mm, -mm)), pack2(1.4426950408889634f, 1.4426950408889634f)));
+                        const f32x2 w = pack2(ex2_approx(t.x), ex2_approx(t.y));
+                        sum[c & 1] = add2(sum[c & 1], w);
+                        split3(w, ph[8 * hf + c], pm[8 * hf + c], pl[8 * hf + c]);
                     }
-#pragma unroll
-                    for (int c = 0; c < 8; c++) split3(p[2 * c], p[2 * c + 1], ph[8 * hf + c], pm[8 * hf + c], pl[8 * hf + c]);
                 }
-                l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+                const float2 s2 = unpack2(add2(sum[0], sum[1]));
+                l += s2.x + s2.y;
                 tc_fence_before(); // the last of these scores are read before the next tile's are written
                 wait_free();
                 load_ahead(nc + s);

@@ -40,6 +40,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     *dead = 1;
     return false;
 }
+// The same for a warp that reads a buffer of shared memory behind the wait and hands it back by one lane's arrival: one lane polls.  Where every
+// lane polls they leave the loop one after the other, and the barrier of the warp ahead of the arrival did not hold them together (the loop
+// passes for uniform): the buffer was refilled while the last lanes read it, in 9 of 10 launches of a kernel whose copies came late.
+__device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *dead) {
+    if ((threadIdx.x & 31) == 0) mbar_wait_bounded(bar, parity, dead);
+    __syncwarp();
+}
 // Behind a wait that ran out: copies and MMAs may still be under way, and what they write stays this CTA's for another half second.  By one
 // warp, when all of them are done.
 __device__ __forceinline__ void settle(volatile int *dead) {
@@ -100,6 +107,11 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
     return r;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -180,19 +192,54 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
+// two fp32 numbers in one register pair: one instruction for both where the issue of instructions is what bounds a loop
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Two fp32 numbers as three pairs of bf16 numbers whose sums they are: 3 x 8 significant bits hold the 24 of an fp32 number, each
-// remainder is exact.  An fp32 x bf16 product is then three bf16 x bf16 products of the tensor cores, each exact before it is added.
+// remainder is exact (and taken two at a time).  An fp32 x bf16 product is then three bf16 x bf16 products of the tensor cores, each exact before it is added.
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&p);
 }
-__device__ __forceinline__ void split3(float a, float b, uint32_t &h, uint32_t &m, uint32_t &l) {
-    h = pack_bf16x2(a, b);
-    a -= __uint_as_float(h << 16);
-    b -= __uint_as_float(h & 0xffff0000u);
-    m = pack_bf16x2(a, b);
-    a -= __uint_as_float(m << 16);
-    b -= __uint_as_float(m & 0xffff0000u);
-    l = pack_bf16x2(a, b);
+__device__ __forceinline__ void split3(f32x2 v, uint32_t &h, uint32_t &m, uint32_t &l) {
+    const f32x2 minus = pack2(-1.f, -1.f);
+    float2 x = unpack2(v);
+    h = pack_bf16x2(x.x, x.y);
+    v = fma2(pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, v);
+    x = unpack2(v);
+    m = pack_bf16x2(x.x, x.y);
+    v = fma2(pack2(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)), minus, v);
+    x = unpack2(v);
+    l = pack_bf16x2(x.x, x.y);
 }
 #endif

@@ -8,10 +8,10 @@
 // steps of 2^-23, a weighted sum by half a step of 2^-24 per 16 keys and part; below the bf16 of the result).
 //
 //   scores   S [128][64 keys] = (q_l + q_m + q_h) K^T: queries in shared memory, K tile K-major as the cache rows lie
-//   weights  one thread a row (no shuffles): tcgen05.ld, soft cap, mask, exp or sigmoid, split, back to tensor memory over the scores
+//   weights  two threads a row (32 keys each, no shuffles): tcgen05.ld, soft cap, mask, exp or sigmoid, split, back to tensor memory over the scores
 //   output   O [128][Dv] += (p_l + p_m + p_h) V: weights from tensor memory, the V tile as the cache rows lie (MN-major B operand)
 //
-// Two groups of four warps take the key tiles alternately, each with its own scores, maximum, sum and output, so the tensor cores work
+// Two groups of eight warps take the key tiles alternately, each with its own scores, maximum, sum and output, so the tensor cores work
 // for one group while the other one computes weights; the two are added up at the end.  A warp stages the K tiles, one the V tiles
 // (cp.async, page table per row), one warp issues every MMA.  A maximum is kept until a score exceeds it by 8 (the weights then reach
 // e^8, and sum and output are relative to the kept one all the same), so the output is hardly ever rescaled.
@@ -21,10 +21,10 @@
 // computed once more over its visible keys by fp32 multiply-adds (plain_row): an infinite key, value or query gives what the plain
 // arithmetic gives for it.
 //
-// What bounds it: the instructions around the weights, about 40 a number with a soft cap (2.2 us a tile on the 128 rows of an SM, of which
-// 1.0 us would be the MMAs alone).  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft
-// cap, gate: 56 us, 154 TFLOP/s of the products asked for, tensor cores 26 % of the cycles (785 us by the fp32 CUDA cores, tiles of 32
-// queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 64 us (686 us).  Unrolling the 64 scores of a row whole: 150 us.
+// What bounds it: the instructions around the weights (two numbers an instruction where the unit has a packed form: fma.rn.f32x2), then the
+// MMAs.  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft cap, gate: 43 us, 200 TFLOP/s of
+// the products asked for (57 us with four warps a group and one thread a row, number by number; 785 us by the fp32 CUDA cores, tiles of 32
+// queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 55 us (64 us; 686 us).
 #pragma once
 
 #include "dense.cuh"
@@ -33,8 +33,8 @@
 namespace tile_attn {
 
 constexpr int kRows = 128, kKeys = 64; // rows of a CTA, keys of a tile
-constexpr int kThreads = 32 * 12;      // three warps a scheduler
-constexpr int kMmaWarp = 10;
+constexpr int kWarps = 16;              // that turn scores into weights
+constexpr int kThreads = 32 * (kWarps + 4), kMmaWarp = kWarps + 2;
 constexpr int kMaxBlocks = 3; // 64-wide blocks of a key or value: D, Dv <= 192
 constexpr int kBarWords = 64; // barriers, tensor-memory slot, `dead`, in 4-byte words
 
@@ -57,6 +57,7 @@ struct shape {
     int *wait_error;
 };
 
+constexpr int kStats = 12; // rows of 128 numbers: maximum and sum at the end; per group and half a row's maxima, two tables (softmax), later sums
 inline int pad64(int n) { return (n + 63) / 64 * 64; }
 // sigmoid heads: penalties of one tile, a row of them per head of the group, rows of a warp in different banks
 __host__ __device__ inline int pen_pitch(int TQ, int hpg) { return (TQ + kKeys + 31) / 32 * 32 + (hpg <= 32 ? 32 / hpg : 1); }
@@ -64,7 +65,7 @@ inline size_t smem_bytes(int mode, int maps, int D, int Dv, int hpg) {
     const size_t tiles = (size_t)3 * kRows * pad64(D) * 2 + 2 * (size_t)kKeys * (maps * pad64(D) + pad64(Dv)) * 2;
     const size_t finish = (size_t)kRows * (Dv + 1) * 4; // the output rows, over the tiles
     const size_t pen = mode == SIGMOID ? (size_t)2 * hpg * pen_pitch(kRows / maps / hpg, hpg) * 4 : 0;
-    return 1024 + (tiles > finish ? tiles : finish) + kBarWords * 4 + (size_t)4 * kRows * 4 + pen;
+    return 1024 + (tiles > finish ? tiles : finish) + kBarWords * 4 + (size_t)kStats * kRows * 4 + pen;
 }
 // Sizes the kernel takes (bf16 cache).  D, Dv and the offsets of a head's keys and values in a cache row are whole 16-byte pieces and
 // whole MMA steps; tensor memory holds 2 x (scores of the maps, then weights) + 2 x Dv columns.
@@ -82,31 +83,44 @@ __device__ __forceinline__ int64_t first_visible(int64_t i, int64_t size, int ch
 // squares at Chebyshev nodes (largest relative error 1.3 x 2^-24 with these roundings); beyond: 1 - 2 e / (1 + e), e = exp(-2 |y|), computed
 // only when a score of the warp is that large.
 __device__ __forceinline__ void soft_cap16(float *z, float cap, float inv_cap) {
-    float y[16], t[16], big = 0.f;
+    const f32x2 ic = pack2(inv_cap, inv_cap), cc = pack2(cap, cap);
+    auto both = [](float v) { return pack2(v, v); };
+    f32x2 y[8], t[8];
+    float big = 0.f;
 #pragma unroll
-    for (int c = 0; c < 16; c++) {
-        y[c] = z[c] * inv_cap;
-        big = fmaxf(big, fabsf(y[c]));
+    for (int c = 0; c < 8; c++) {
+        y[c] = mul2(pack2(z[2 * c], z[2 * c + 1]), ic);
+        const float2 v = unpack2(y[c]);
+        big = fmaxf(big, fmaxf(fabsf(v.x), fabsf(v.y)));
     }
 #pragma unroll
-    for (int c = 0; c < 16; c++) {
-        const float u = y[c] * y[c];
-        float p = fmaf(u, -0.005893945228308439f, 0.020794617012143135f);
-        p = fmaf(u, p, -0.053783293813467026f);
-        p = fmaf(u, p, 0.13331915438175201f);
-        p = fmaf(u, p, -0.33333298563957214f);
-        t[c] = fmaf(y[c] * u, p, y[c]);
+    for (int c = 0; c < 8; c++) {
+        const f32x2 u = mul2(y[c], y[c]);
+        f32x2 p = fma2(u, both(-0.005893945228308439f), both(0.020794617012143135f));
+        p = fma2(u, p, both(-0.053783293813467026f));
+        p = fma2(u, p, both(0.13331915438175201f));
+        p = fma2(u, p, both(-0.33333298563957214f));
+        t[c] = fma2(mul2(y[c], u), p, y[c]);
     }
     if (__any_sync(0xffffffffu, !(big <= 0.6f))) {
 #pragma unroll
-        for (int c = 0; c < 16; c++) {
-            const float ay = fabsf(y[c]), e = expf(-2.0f * ay);
-            const float b = fmaf(-2.0f * e, __frcp_rn(1.0f + e), 1.0f);
-            t[c] = ay <= 0.6f ? t[c] : copysignf(b, y[c]); // (a NaN stays one: e is)
+        for (int c = 0; c < 8; c++) {
+            const float2 yv = unpack2(y[c]), tv = unpack2(t[c]);
+            float w[2] = {tv.x, tv.y};
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float v = e ? yv.y : yv.x, ay = fabsf(v), x = expf(-2.0f * ay);
+                const float b = fmaf(-2.0f * x, __frcp_rn(1.0f + x), 1.0f);
+                w[e] = ay <= 0.6f ? w[e] : copysignf(b, v); // (a NaN stays one: x is)
+            }
+            t[c] = pack2(w[0], w[1]);
         }
     }
 #pragma unroll
-    for (int c = 0; c < 16; c++) z[c] = cap * t[c];
+    for (int c = 0; c < 8; c++) {
+        const float2 v = unpack2(mul2(cc, t[c]));
+        z[2 * c] = v.x, z[2 * c + 1] = v.y;
+    }
 }
 // 1 / (1 + exp(-z)): the reciprocal by one Newton step from the approximate one (no division's slow path); exp(-z) stays finite, a NaN
 // stays one
@@ -116,6 +130,27 @@ __device__ __forceinline__ float sigmoid_fast(float z) {
     const float d = 1.0f + expf(e);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+// the same for two numbers.  exp(x) = 2^t (1 + ln 2 r), t = x log2 e rounded, r what the rounding left: as exact as expf.  -z is kept within
+// +-88 (beyond, the result is 0 or 1 to 32 bits).
+__device__ __forceinline__ f32x2 sigmoid_fast2(f32x2 z) {
+    auto both = [](float v) { return pack2(v, v); };
+    const float2 v = unpack2(z);
+    float x, y, rx, ry;
+    asm("min.NaN.f32 %0, %1, %2;\nmax.NaN.f32 %0, %0, %3;" : "=f"(x) : "f"(-v.x), "f"(88.0f), "f"(-88.0f));
+    asm("min.NaN.f32 %0, %1, %2;\nmax.NaN.f32 %0, %0, %3;" : "=f"(y) : "f"(-v.y), "f"(88.0f), "f"(-88.0f));
+    const f32x2 a = pack2(x, y), l2e = both(1.4426950408889634f), t = mul2(a, l2e), rest = fma2(a, l2e, mul2(t, both(-1.f)));
+    // log2 e is not the fp32 number: what is missing, 1.9259629911e-8, goes with the rest
+    const f32x2 r = fma2(a, both(1.925963033500312e-8f), rest);
+    const float2 tv = unpack2(t);
+    f32x2 e = pack2(ex2_approx(tv.x), ex2_approx(tv.y));
+    e = fma2(mul2(e, r), both(0.6931471805599453f), e);
+    const f32x2 d = add2(e, both(1.f));
+    const float2 dv = unpack2(d);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(dv.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(dv.y));
+    const f32x2 q = pack2(rx, ry), err = fma2(mul2(d, both(-1.f)), q, both(1.f));
+    return fma2(q, err, q);
 }
 __device__ __forceinline__ float penalty(float r1, float r2, int64_t dist) { return dist > 0 ? r1 * log1pf(r2 * (float)dist) : 0.f; }
 
@@ -234,13 +269,13 @@ template <int MODE> __device__ __forceinline__ void plain_row(const row_job &j, 
     __syncwarp();
 }
 
-// the rows of a warp's set bits (row warp + 8 b) once more; out of line, so that the code that every call runs through stays short
+// the rows of a warp's set bits (row warp + kWarps b) once more; out of line, so that the code that every call runs through stays short
 template <int MODE, int MAPS>
 __device__ __noinline__ void plain_rows(const shape &a, uint32_t again, int64_t t0, int64_t i0, int g, int hpg, int n_pairs, float *of, float *st) {
     constexpr int PR = kRows / MAPS;
     const int warp = threadIdx.x >> 5;
     while (again) {
-        const int rr = warp + 8 * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
+        const int rr = warp + kWarps * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
         again &= again - 1;
         if (rp >= n_pairs) continue;
         row_job j{a.q + (((t0 + rq) * a.H + h) * MAPS + rm) * a.D, a.cache + ((int64_t)g * MAPS + rm) * a.D, a.cache + (int64_t)a.G * MAPS * a.D + (int64_t)g * a.Dv,
@@ -269,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     uint32_t *ctlw = reinterpret_cast<uint32_t *>(gbase + ctl);
     volatile int *dead = reinterpret_cast<volatile int *>(ctlw + 40);
     float *st = reinterpret_cast<float *>(ctlw + kBarWords); // [group][m, l][128]
-    float *pen = st + 4 * kRows;                             // sigmoid: [group][heads][pitch]
+    float *pen = st + kStats * kRows;                        // sigmoid: [group][heads][pitch]
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     constexpr int PR = kRows / MAPS; // (token, head) pairs of a CTA
@@ -288,10 +323,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
             mbar_init(bars + V_FULL + 8 * s, 1);
             mbar_init(bars + V_FREE + 8 * s, 1);
             mbar_init(bars + S_FULL + 8 * s, 1);
-            mbar_init(bars + P_FULL + 8 * s, 4);
+            mbar_init(bars + P_FULL + 8 * s, 8);
         }
         mbar_init(bars + DONE, 1);
-        mbar_init(bars + Q_FULL, 8);
+        mbar_init(bars + Q_FULL, kWarps);
         *dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -303,9 +338,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     const uint32_t reg_cols = MAPS == 1 ? 96 : 128; // scores [MAPS][64], then weights over them
     const uint32_t o_col = 2 * reg_cols;
 
-    if (warp == 8 || warp == 9) {
+    if (warp == kWarps || warp == kWarps + 1) {
         // ---- a warp stages K, one V: eight lanes a 128-byte piece of a row
-        const bool is_k = warp == 8;
+        const bool is_k = warp == kWarps;
         const int sub = lane >> 3, pc = lane & 7;
         const int pcs = (is_k ? a.D : a.Dv) / 8; // 16-byte pieces of a row (and map)
         const uint32_t stage_bytes = is_k ? k_stage : v_stage, s0 = is_k ? sk : sv;
@@ -346,15 +381,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         if (a.D == 128) mma_role<MAPS, 8>(ma);
         else if (a.D == 64) mma_role<MAPS, 4>(ma);
         else mma_role<MAPS, 0>(ma);
-    } else if (warp < 8) {
+    } else if (warp < kWarps) {
         // the rows of q as three bf16 numbers each, rows and coordinates past the end as zeros: four numbers a thread, eight loads in flight
         {
             const int gpr = 16 * D64, n_items = kRows * gpr;
-            for (int it0 = tid; it0 < n_items; it0 += 8 * 256) {
+            for (int it0 = tid; it0 < n_items; it0 += 8 * 32 * kWarps) {
                 float4 x[8];
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
-                    const int it = it0 + 256 * u, r = it / gpr, d = 4 * (it - r * gpr);
+                    const int it = it0 + 32 * kWarps * u, r = it / gpr, d = 4 * (it - r * gpr);
                     const int mp = MAPS == 1 ? 0 : r / PR, pr = MAPS == 1 ? r : r - mp * PR, qi = pr / hpg;
                     x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (it < n_items && pr < n_pairs && d < a.D)
@@ -362,11 +397,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 }
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
-                    const int it = it0 + 256 * u, r = it / gpr, d = 4 * (it - r * gpr);
+                    const int it = it0 + 32 * kWarps * u, r = it / gpr, d = 4 * (it - r * gpr);
                     if (it >= n_items) break;
                     uint32_t h[2], m[2], l[2];
-                    split3(x[u].x, x[u].y, h[0], m[0], l[0]);
-                    split3(x[u].z, x[u].w, h[1], m[1], l[1]);
+                    split3(pack2(x[u].x, x[u].y), h[0], m[0], l[0]);
+                    split3(pack2(x[u].z, x[u].w), h[1], m[1], l[1]);
                     const uint32_t at = base + (uint32_t)(d >> 6) * (kRows * 128) + r * 128 + ((((d >> 3) & 7) ^ (r & 7)) << 4) + (d & 4) * 2;
                     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(h[0]), "r"(h[1]) : "memory");
                     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + q_split), "r"(m[0]), "r"(m[1]) : "memory");
@@ -377,8 +412,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         fence_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(bars + Q_FULL);
-        // ---- weights: group grp takes the tiles n = grp, grp + 2, ...; a thread owns one row
-        const int grp = warp >> 2, lq = warp & 3, r = 32 * lq + lane;
+        // ---- weights: group grp takes the tiles n = grp, grp + 2, ...; a thread owns 32 keys of one row, two threads the row
+        const int grp = warp >> 3, half = (warp >> 2) & 1, lq = warp & 3, r = 32 * lq + lane;
         const int mp = MAPS == 1 ? 0 : r / PR, pr = MAPS == 1 ? r : r - mp * PR, qi = pr / hpg, hh = pr - qi * hpg;
         const int64_t i = i0 + qi, lo = first_visible(i, a.window, a.chunked);
         const bool live = pr < n_pairs;
@@ -393,12 +428,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
             const int64_t j0 = tl.first(n), jl = min(tl.last(n), j0 + kKeys - 1);
             const bool whole = jl - j0 == kKeys - 1 && jl <= i0 && (n < tl.n_kt || j0 >= first_visible(i_last, a.window, a.chunked));
             if (MODE == SIGMOID && a.r1) { // the penalties a tile can meet: distances (i0 - j0) + qi - jj, qi < TQ, jj < 64
-                if (n > grp) bar_sync(1 + grp, 128);
-                for (int e = (tid & 127); e < hpg * (TQ + kKeys - 1); e += 128) {
+                if (n > grp) bar_sync(1 + grp, 256);
+                for (int e = (tid & 255); e < hpg * (TQ + kKeys - 1); e += 256) {
                     const int eh = e / (TQ + kKeys - 1), ed = e - eh * (TQ + kKeys - 1);
                     mypen[eh * pitch + ed] = penalty(a.r1[g * hpg + eh], a.r2[g * hpg + eh], i0 - j0 + ed - (kKeys - 1));
                 }
-                bar_sync(1 + grp, 128);
             }
             mbar_wait_bounded(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
             tc_fence_after();
@@ -410,27 +444,30 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 c_lo = (int)max((int64_t)0, min((int64_t)kKeys, lo_c));
                 c_keep = MODE == SOFTMAX ? (int)max((int64_t)0, min((int64_t)kKeys, kp)) : 0;
             }
-            // 16 scores at a time and no further unrolling: longer straight-line code leaves the instruction cache, which also starves
-            // the warp that issues the MMAs
-            float mm = 0.f, sum[4] = {0.f, 0.f, 0.f, 0.f};
-            auto masked = [&](float *x, int c0, float none) {
+            // both halves' scores are in registers before either one's weights go over them (the barrier)
+            float x[2][16], mm = 0.f;
+            f32x2 sum[2] = {0, 0};
+            auto masked = [&](float *y, int c0, float none) {
 #pragma unroll
-                for (int c = 0; c < 16; c++) x[c] = (c0 + c < c_hi && (c0 + c >= c_lo || c0 + c < c_keep)) ? x[c] : none;
+                for (int c = 0; c < 16; c++) y[c] = (c0 + c < c_hi && (c0 + c >= c_lo || c0 + c < c_keep)) ? y[c] : none;
             };
-            if (MODE == SOFTMAX) {
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-                for (int c0 = 0; c0 < 64; c0 += 16) {
-                    float x[16];
-                    tmem_load16(ts + mp * 64 + c0, reinterpret_cast<uint32_t *>(x));
-                    if (a.cap > 0.f) soft_cap16(x, a.cap, inv_cap);
-                    if (!whole) masked(x, c0, -INFINITY);
-                    if (a.cap > 0.f || !whole) tmem_store16(ts + mp * 64 + c0, reinterpret_cast<uint32_t *>(x));
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                    for (int c = 0; c < 16; c++) mx4[c & 3] = fmaxf(mx4[c & 3], x[c]);
-                }
-                if (a.cap > 0.f || !whole) tmem_wait_st();
-                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            for (int k = 0; k < 2; k++) {
+                const int c0 = 32 * half + 16 * k;
+                tmem_load16(ts + mp * 64 + c0, reinterpret_cast<uint32_t *>(x[k]));
+                if (MODE != SOFTMAX) continue;
+                if (a.cap > 0.f) soft_cap16(x[k], a.cap, inv_cap);
+                if (!whole) masked(x[k], c0, -INFINITY);
+#pragma unroll
+                for (int c = 0; c < 16; c++) mx4[c & 3] = fmaxf(mx4[c & 3], x[k][c]);
+            }
+            if (MODE == SOFTMAX) {
+                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                float *swap = st + (4 + 4 * ((n >> 1) & 1) + 2 * grp) * kRows + r; // two tables: the next tile writes the other one
+                swap[half * kRows] = mx;
+                bar_sync(1 + grp, 256);
+                mx = fmaxf(mx, swap[(half ^ 1) * kRows]);
                 float corr = 1.f;
                 const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY);
                 if (grow) {
@@ -440,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 }
                 if (n >= 2 && __any_sync(0xffffffffu, grow)) { // the tile before has been added: its MMAs precede this tile's scores
 #pragma unroll 1
-                    for (int c = 0; c < a.Dv; c += 16) {
+                    for (int c = 16 * half; c < a.Dv; c += 32) {
                         uint32_t o[16];
                         tmem_load16(to + c, o);
 #pragma unroll
@@ -449,69 +486,79 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                     }
                 }
                 mm = m == -INFINITY ? 0.f : m; // nothing visible yet: every weight is exp(-inf) = 0
+            } else {
+                bar_sync(1 + grp, 256);
             }
             const float *prow = MODE == SIGMOID ? mypen + hh * pitch + qi + kKeys - 1 : nullptr;
-            // the weights of 16 keys go to 24 columns [p_h | p_m | p_l] from 24 k on: from the last 16 keys to the first (a second map,
-            // whose scores lie 64 columns further: from the first to the last) they only cover scores that have been read
-#pragma unroll 1
-            for (int k = 0; k < 4; k++) {
-                const int c0 = 16 * (mp == 0 ? 3 - k : k);
-                float x[16];
-                tmem_load16(ts + mp * 64 + c0, reinterpret_cast<uint32_t *>(x));
-                if (MODE == SOFTMAX) {
+            // the weights of 16 keys go to 24 columns [p_h | p_m | p_l] from 24 k on
 #pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        x[c] = expf(x[c] - mm);
-                        sum[c & 3] += x[c];
+            for (int k = 0; k < 2; k++) {
+                const int c0 = 32 * half + 16 * k;
+                float *y = x[k];
+                f32x2 w[8];
+                if (MODE == SOFTMAX) { // exp(s - m) = 2^((s - m) log2 e): the product's rounding moves a weight by less than 2^-24 of the largest one
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        const float2 t = unpack2(mul2(add2(pack2(y[2 * c], y[2 * c + 1]), pack2(-mm, -mm)), pack2(1.4426950408889634f, 1.4426950408889634f)));
+                        w[c] = pack2(ex2_approx(t.x), ex2_approx(t.y));
+                        sum[c & 1] = add2(sum[c & 1], w[c]);
                     }
                 } else {
                     if (a.r1) {
 #pragma unroll
-                        for (int c = 0; c < 16; c++) x[c] -= prow[-(c0 + c)];
+                        for (int c = 0; c < 16; c++) y[c] -= prow[-(c0 + c)];
                     }
 #pragma unroll
-                    for (int c = 0; c < 16; c++) x[c] = sigmoid_fast(x[c] + hpb);
-                    if (!whole) masked(x, c0, 0.f);
+                    for (int c = 0; c < 8; c++) {
+                        const float2 v = unpack2(sigmoid_fast2(add2(pack2(y[2 * c], y[2 * c + 1]), pack2(hpb, hpb))));
+                        y[2 * c] = v.x, y[2 * c + 1] = v.y;
+                    }
+                    if (!whole) masked(y, c0, 0.f);
+#pragma unroll
+                    for (int c = 0; c < 8; c++) w[c] = pack2(y[2 * c], y[2 * c + 1]);
                 }
                 uint32_t ph[8], pm[8], pl[8];
 #pragma unroll
-                for (int c = 0; c < 8; c++) split3(x[2 * c], x[2 * c + 1], ph[c], pm[c], pl[c]);
+                for (int c = 0; c < 8; c++) split3(w[c], ph[c], pm[c], pl[c]);
                 const uint32_t tp = ts + (c0 >> 4) * 24;
                 tmem_store8(tp, ph);
                 tmem_store8(tp + 8, pm);
                 tmem_store8(tp + 16, pl);
             }
-            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            const float2 s2 = unpack2(add2(sum[0], sum[1]));
+            l += s2.x + s2.y;
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + P_FULL + 8 * grp);
         }
         // ---- both groups' sums meet: O = O_0 f_0 + O_1 f_1 relative to the larger maximum, as rows in shared memory
-        if (MODE == SOFTMAX) {
-            st[(2 * grp) * kRows + r] = m;
-            st[(2 * grp + 1) * kRows + r] = l;
-        }
+        const int quarter = 2 * grp + half;
         mbar_wait_bounded(bars + DONE, 0, dead); // all MMAs are done: the tiles are no longer read
         tc_fence_after();
-        bar_sync(3, 256);
+        bar_sync(3, 32 * kWarps);
+        if (MODE == SOFTMAX) {
+            st[(4 + quarter) * kRows + r] = l;
+            if (half == 0) st[(2 + grp) * kRows + r] = m;
+            bar_sync(3, 32 * kWarps);
+        }
         float f0 = 1.f, f1 = NT > 1 ? 1.f : 0.f, M = 0.f, L = 1.f;
         if (MODE == SOFTMAX) {
-            const float m0 = st[r], l0 = st[kRows + r], m1 = st[2 * kRows + r], l1 = st[3 * kRows + r];
+            const float m0 = st[2 * kRows + r], l0 = st[4 * kRows + r] + st[5 * kRows + r], m1 = st[3 * kRows + r], l1 = st[6 * kRows + r] + st[7 * kRows + r];
             M = fmaxf(m0, m1);
             f0 = m0 == -INFINITY ? 0.f : expf(m0 - M);
             f1 = m1 == -INFINITY ? 0.f : expf(m1 - M);
             L = l0 * f0 + l1 * f1;
-        }
-        bar_sync(3, 256);
-        if (MODE == SOFTMAX && grp == 0) {
-            st[r] = M;
-            st[kRows + r] = L;
+            bar_sync(3, 32 * kWarps);
+            if (quarter == 0) {
+                st[r] = M;
+                st[kRows + r] = L;
+            }
         }
         float *of = reinterpret_cast<float *>(gbase);
         const int op = a.Dv + 1, n16 = a.Dv / 16;
         float odd = MODE == SOFTMAX ? 0.f * L : 0.f; // 0, or NaN when a sum of the row is not finite
-        for (int cb = grp; cb < n16; cb += 2) {
+        for (int cb = quarter; cb < n16; cb += 4) {
             uint32_t o0[16], o1[16];
             tmem_load16(tmem + lanes + o_col + 16 * cb, o0);
             if (NT > 1) tmem_load16(tmem + lanes + o_col + a.Dv + 16 * cb, o1);
@@ -523,25 +570,25 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 odd = fmaf(0.f, v, odd);
             }
         }
-        st[(2 + grp) * kRows + r] = odd;
-        bar_sync(3, 256);
-        // a warp's 16 rows: warp, warp + 8, ...; those whose sums are not finite once more, without the split
+        st[(2 + quarter) * kRows + r] = odd;
+        bar_sync(3, 32 * kWarps);
+        // a warp's 8 rows: warp, warp + 16, ...; those whose sums are not finite once more, without the split
         {
-            const int er = warp + 8 * (lane & 15);
-            const uint32_t again = __ballot_sync(0xffffffffu, st[2 * kRows + er] + st[3 * kRows + er] != 0.f) & 0xffffu;
+            const float *er = st + warp + kWarps * (lane & 7);
+            const uint32_t again = __ballot_sync(0xffffffffu, (er[2 * kRows] + er[3 * kRows]) + (er[4 * kRows] + er[5 * kRows]) != 0.f) & 0xffu;
             if (again) plain_rows<MODE, MAPS>(a, again, t0, i0, g, hpg, n_pairs, of, st);
         }
         // a warp a row, four rows' reads from memory in flight
-        for (int p0 = warp; p0 < n_pairs; p0 += 32) {
+        for (int p0 = warp; p0 < n_pairs; p0 += 4 * kWarps) {
             typename FIN::reads rd[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int p = min(p0 + 8 * u, n_pairs - 1), pq = p / hpg;
+                const int p = min(p0 + kWarps * u, n_pairs - 1), pq = p / hpg;
                 fin.load(rd[u], i0 + pq, t0 + pq, g * hpg + (p - pq * hpg), lane);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int p = p0 + 8 * u, pq = p / hpg;
+                const int p = p0 + kWarps * u, pq = p / hpg;
                 if (p >= n_pairs) break;
                 fin.row(rd[u], of + p * op, of + (p + PR) * op, st[p], st[kRows + p], MAPS == 2 ? st[kRows + p + PR] : 0.f, t0 + pq, g * hpg + (p - pq * hpg), lane);
             }
