@@ -1,0 +1,312 @@
+// gemm_any.cu — C[T][N] = A[T][K] W[N][K]^T on the tensor cores (tcgen05) for fp32 matrices, and for the bf16 matrices that gemm.cu's TMA form does
+// not take (fewer than 64 rows of A, odd sizes, strides and addresses).  Results and accuracy are those of fp32 multiply-adds.
+//
+// A tile is 128 rows of W (the M of an MMA: one lane of tensor memory each) x BT rows of A, so that few tokens cost few columns and a store of
+// one token's 32 features is one line.  Sixteen warps bring both operands from memory, K in stages of 64, and write them as swizzled bf16
+// tiles; nothing is asked of sizes or alignment (VEC: 16-byte loads, else numbers one by one).  One warp issues the MMAs, eight drain.
+//
+// fp32: a number is the sum of three bf16 numbers, x = xh + xm + xl (split3, exact), and a product is xh yh + (xh ym + xm yh) + (xh yl + xm ym + xl yh),
+// what is left out is below 2^-24 of it.  The three parts of A lie behind one another as one operand of 3 BT columns, so that a part
+// of W is read from shared memory once for all of its products: Wh [Ah Am Al], Wm [Ah Am], Wl [Ah], into columns for xh yh, first-order and
+// second-order terms.  The tensor cores truncate their running sum, so every stage has an accumulator of its own (two, in turn), which the
+// draining warps add to registers, rounding to nearest: the error against 64 bits is smaller than that of one chain of multiply-adds
+// (K = 1000: 1.0e-7 against 5.7e-7).  A result that is not finite is computed once more by plain multiply-adds (an infinity is not the
+// sum of its parts).  (Numbers below 2^-110 lose their last parts to the smallest bf16 number.)
+//
+// A product of few tiles is cut along K over the CTAs of a cluster (up to 8), whose sums meet in shared memory and are added in order.
+//
+// What bounds it: fp32, shared memory (written and read: BT = 64: 170 KB a stage, 1330 cycles of 128 bytes); bf16, the loads in flight.
+// 333 x 2816 x 1000 fp32: 98.4 -> 33.0 us (64 x 64 tiles of FMAs).
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "dense.cuh"
+#include "gemm_any.cuh"
+#include "tc.cuh"
+
+namespace {
+
+constexpr int kM = 128, kBK = 64;
+constexpr int kDrain = 8, kLoad = 16, kMmaWarp = kDrain, kThreads = 32 * (kDrain + 1 + kLoad);
+constexpr int kMaxBT = 64, kMaxSplits = 8;
+enum { FULL = 0, EMPTY = 32, ACC_FULL = 64, ACC_FREE = 80, SLOT = 96, DEAD = 100, kCtl = 128 };
+
+template <typename E> struct parts_of { static constexpr int n = sizeof(E) == 4 ? 3 : 1, stages_per_acc = 1, stages = sizeof(E) == 4 ? 2 : 4; };
+template <typename E> __host__ __device__ inline uint32_t stage_bytes(int BT) { return (uint32_t)parts_of<E>::n * (kM + BT) * 128; }
+
+struct any_args {
+    const void *w, *a;
+    int64_t N, K, T, lda, ldc;
+    float *c;
+    void *c_act; // when set: act(c) in the matrices' type instead of c
+    int act, BT, splits, kblocks;
+    int *wait_error;
+};
+
+__device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\ntcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_load8x3(uint32_t ta, uint32_t tb, uint32_t tc, uint32_t (&u)[8], uint32_t (&v)[8], uint32_t (&w)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%24];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%25];\n"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%26];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]),
+                   "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "r"(ta), "r"(tb), "r"(tc)
+                 : "memory");
+}
+
+// one result in plain arithmetic
+template <typename E> __device__ __noinline__ float plain_dot(const E *w, const E *a, int64_t K) {
+    float s = 0.f;
+    for (int64_t k = 0; k < K; k++) s = fmaf(to_f32(w[k]), to_f32(a[k]), s);
+    return s;
+}
+
+// 16 bytes of a row from column k on: whole, or what lies inside K number by number
+template <typename E, bool VEC> __device__ __forceinline__ uint4 load_piece(const E *row, int64_t k, int64_t K) {
+    constexpr int V = 16 / (int)sizeof(E);
+    if (VEC) return k < K ? ldg_stream_u4(row + k) : make_uint4(0, 0, 0, 0); // K is a multiple of V
+    union {
+        E e[V];
+        uint4 u;
+    } p;
+    p.u = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < V; i++)
+        if (k + i < K) p.e[i] = row[k + i];
+    return p.u;
+}
+
+template <typename E, bool VEC>
+__global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_constant__ any_args g) {
+    constexpr int P = parts_of<E>::n, SPA = parts_of<E>::stages_per_acc, STAGES = parts_of<E>::stages;
+    extern __shared__ uint8_t ga_raw[];
+    const uint32_t raw0 = smem_u32(ga_raw), base = (raw0 + 1023u) & ~1023u;
+    uint8_t *gbase = ga_raw + (base - raw0);
+    const int BT = g.BT;
+    const uint32_t st_bytes = stage_bytes<E>(BT), part_a = P * kM * 128, bars = base + STAGES * st_bytes;
+    uint8_t *ctl = gbase + STAGES * st_bytes;
+    volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int rank = g.splits > 1 ? (int)cluster_rank() : 0;
+    const int64_t tile = blockIdx.x / g.splits, n_tiles = (g.N + kM - 1) / kM, m_tiles = (g.T + BT - 1) / BT;
+    const int64_t t0 = tile % m_tiles * BT, n0 = tile / m_tiles * kM; // those that share rows of W run together
+    (void)n_tiles;
+    const int per = (g.kblocks + g.splits - 1) / g.splits, kb0 = min(rank * per, g.kblocks), kb1 = min(kb0 + per, g.kblocks), nkb = kb1 - kb0;
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; s++) {
+            mbar_init(bars + FULL + 8 * s, kLoad);
+            mbar_init(bars + EMPTY + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(bars + ACC_FULL + 8 * s, 1);
+            mbar_init(bars + ACC_FREE + 8 * s, kDrain);
+        }
+        *dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
+    const uint32_t acc_cols = P * BT; // of one accumulator; two of them: at most 384
+
+    if (warp > kMmaWarp) {
+        // ---- a thread owns one 16-byte piece of every RS-th row of the stage: rows of W, then rows of A
+        constexpr int V = 16 / (int)sizeof(E), PCS = kBK / V, RS = 32 * kLoad / PCS, NI = (kM + kMaxBT + RS - 1) / RS, NW = kM / RS;
+        const int lt = tid - 32 * (kMmaWarp + 1), pc = lt % PCS, r0 = lt / PCS;
+        const E *wp = static_cast<const E *>(g.w) + (n0 + r0) * g.K, *ap = static_cast<const E *>(g.a) + (t0 + r0) * g.lda;
+        uint32_t live = 0; // bit i: row r0 + RS i of the stage exists
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+            const int r = r0 + RS * i;
+            if (i < NW ? n0 + r < g.N : (r - kM < BT && t0 + r - kM < g.T)) live |= 1u << i;
+        }
+        uint4 v[NI];
+        auto fetch = [&](int i, int kb) {
+            const E *row = i < NW ? wp + (int64_t)(RS * i) * g.K : ap + (int64_t)(RS * i - kM) * g.lda;
+            v[i] = live >> i & 1 ? load_piece<E, VEC>(row, (int64_t)kb * kBK + pc * V, g.K) : make_uint4(0, 0, 0, 0);
+        };
+        if (nkb > 0)
+#pragma unroll
+            for (int i = 0; i < NI; i++) fetch(i, kb0);
+        int s = 0;
+        uint32_t ph = 1;
+        for (int kb = kb0; kb < kb1; kb++) {
+            if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph, dead)) break;
+            uint8_t *st = gbase + s * st_bytes;
+#pragma unroll
+            for (int i0 = 0; i0 < NI; i0 += 4) { // four pieces at a time: their chains of instructions side by side
+                uint2 h[4], m[4], l[4];
+                if (P == 3)
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (i0 + u < NI) {
+                            const uint4 x = v[i0 + u];
+                            split3(pack2(__uint_as_float(x.x), __uint_as_float(x.y)), h[u].x, m[u].x, l[u].x);
+                            split3(pack2(__uint_as_float(x.z), __uint_as_float(x.w)), h[u].y, m[u].y, l[u].y);
+                        }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int i = i0 + u;
+                    if (i >= NI) continue;
+                    const int r = r0 + RS * i, ra = r - kM; // row of W's or A's tile
+                    const bool is_w = i < NW;
+                    uint8_t *dst = is_w ? st + r * 128 : st + part_a + ra * 128;
+                    const int pitch = (is_w ? kM : BT) * 128; // between the parts
+                    if (is_w || ra < BT) {
+                        if (P == 1) *reinterpret_cast<uint4 *>(dst + ((pc ^ (r & 7)) << 4)) = v[i];
+                        else {
+                            uint8_t *d = dst + (((pc >> 1) ^ (r & 7)) << 4) + 8 * (pc & 1);
+                            *reinterpret_cast<uint2 *>(d) = h[u];
+                            *reinterpret_cast<uint2 *>(d + pitch) = m[u];
+                            *reinterpret_cast<uint2 *>(d + 2 * pitch) = l[u];
+                        }
+                    }
+                    if (kb + 1 < kb1) fetch(i, kb + 1); // its way from memory is the rest of this stage and the wait for the next
+                }
+            }
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + FULL + 8 * s);
+            if (++s == STAGES) s = 0, ph ^= 1u;
+        }
+    } else if (warp == kMmaWarp) {
+        int s = 0;
+        uint32_t ph = 0;
+        for (int kb = kb0; kb < kb1; kb++) {
+            const int q = kb - kb0, acc = q / SPA, buf = acc & 1;
+            if (q % SPA == 0) mbar_wait_bounded(bars + ACC_FREE + 8 * buf, ((acc >> 1) & 1) ^ 1, dead);
+            mbar_wait_bounded(bars + FULL + 8 * s, ph, dead);
+            tc_fence_after();
+            const uint32_t d = tmem + buf * acc_cols, w_lo = umma_desc_lo(base + s * st_bytes, 16), a_lo = umma_desc_lo(base + s * st_bytes + part_a, 16);
+#pragma unroll
+            for (int k = 0; k < kBK / 16; k++) { // 16 numbers are 2 descriptor units
+                umma_ss(d, w_lo + 2 * k, a_lo + 2 * k, umma_idesc(kM, P * BT), k > 0 || q % SPA != 0);
+                if (P == 3) {
+                    umma_ss(d + BT, w_lo + kM * 8 + 2 * k, a_lo + 2 * k, umma_idesc(kM, 2 * BT), 1);
+                    umma_ss(d + 2 * BT, w_lo + 2 * kM * 8 + 2 * k, a_lo + 2 * k, umma_idesc(kM, BT), 1);
+                }
+            }
+            umma_arrive(bars + EMPTY + 8 * s);
+            if (q % SPA == SPA - 1 || kb == kb1 - 1) umma_arrive(bars + ACC_FULL + 8 * buf);
+            if (++s == STAGES) s = 0, ph ^= 1u;
+        }
+    }
+    constexpr int kCols = kMaxBT / 2; // of a draining warp: one half of the tile's tokens, 32 rows of W
+    float sum[kCols];
+    const int lq = warp & 3, half = warp >> 2, hc = BT / 2, row = lq * 32 + lane;
+    if (warp < kDrain) {
+#pragma unroll
+        for (int c = 0; c < kCols; c++) sum[c] = 0.f;
+        const int accs = (nkb + SPA - 1) / SPA;
+        for (int q = 0; q < accs; q++) {
+            const int buf = q & 1;
+            mbar_wait_bounded(bars + ACC_FULL + 8 * buf, (q >> 1) & 1, dead);
+            tc_fence_after();
+            const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + buf * acc_cols + half * hc;
+#pragma unroll
+            for (int c0 = 0; c0 < kCols; c0 += 8)
+                if (c0 < hc) {
+                    uint32_t x[8], y[8], z[8];
+                    if (P == 3) tmem_load8x3(col + c0, col + BT + c0, col + 2 * BT + c0, x, y, z);
+                    else tmem_load8(col + c0, x);
+#pragma unroll
+                    for (int c = 0; c < 8; c++) sum[c0 + c] += P == 3 ? __uint_as_float(x[c]) + (__uint_as_float(y[c]) + __uint_as_float(z[c])) : __uint_as_float(x[c]);
+                }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + ACC_FREE + 8 * buf);
+        }
+    }
+    __syncthreads(); // every MMA and every write of a stage is done
+    auto store = [&](int c, float v) { // token column c of the tile
+        const int64_t t = t0 + c, n = n0 + row;
+        if (t >= g.T || n >= g.N) return;
+        if (!isfinite(v) && !*dead) v = plain_dot(static_cast<const E *>(g.w) + n * g.K, static_cast<const E *>(g.a) + t * g.lda, g.K);
+        if (g.c_act) static_cast<E *>(g.c_act)[t * g.ldc + n] = from_f32<E>(act_f32(v, g.act));
+        else g.c[t * g.ldc + n] = v;
+    };
+    if (g.splits > 1) { // the ranks' sums, [token][row], in order
+        float *mine = reinterpret_cast<float *>(gbase);
+        if (warp < kDrain) {
+#pragma unroll
+            for (int c = 0; c < kCols; c++)
+                if (c < hc) mine[(half * hc + c) * kM + row] = sum[c];
+        }
+        cluster_sync();
+        if (warp < kDrain)
+            for (int c = half + 2 * rank; c < BT; c += 2 * g.splits) {
+                float v = 0.f;
+                for (int q = 0; q < g.splits; q++) v += ld_cluster_f32(cluster_addr(base + (uint32_t)(c * kM + row) * 4, q));
+                store(c, v);
+            }
+        cluster_sync(); // a rank's sums are read until here
+    } else if (warp < kDrain) {
+#pragma unroll
+        for (int c = 0; c < kCols; c++)
+            if (c < hc) store(half * hc + c, sum[c]);
+    }
+    if (warp == kMmaWarp) {
+        settle(dead);
+        tc_fence_after();
+        tmem_free512(tmem);
+        if (lane == 0 && *dead) *g.wait_error = 1;
+    }
+}
+
+template <typename E>
+int launch_any(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
+    constexpr int P = parts_of<E>::n, V = 16 / (int)sizeof(E);
+    any_args g{w, a, N, K, T, lda, ldc, c, c_act, act, 0, 1, (int)((K + kBK - 1) / kBK), ggb_wait_error_flag()};
+    // the tile and the split of the least estimate.  Cycles of a stage: the bytes that pass through shared memory at 128 a cycle (written once;
+    // read for the MMAs: every part of W once, the parts of A as often as they are multiplied), the loading warps' instructions (about 35 a 16-byte
+    // piece and thread), or the bytes from memory at 20 a cycle and SM; a tile: its prologue and its stores
+    const int64_t n_tiles = (N + kM - 1) / kM;
+    const int sms = ggb_sm_count();
+    double best = 0.0;
+    for (int bt = 16; bt <= kMaxBT; bt += 16) {
+        const int64_t tiles = n_tiles * ((T + bt - 1) / bt);
+        for (int splits = 1; splits <= kMaxSplits && splits <= g.kblocks; splits *= 2) {
+            const double smem = (P * (kM + bt) * 128.0 + P * kM * 128.0 + (P == 3 ? 6 : 1) * bt * 128.0) / 128.0;
+            const double issue = (P == 3 ? 36.0 : 8.0) * (kM + bt) * (kBK / V) / 32.0 / 4.0, bytes = (kM + bt) * kBK * sizeof(E) / 24.0;
+            const double stage = std::max(smem, std::max(issue, bytes));
+            const double rounds = (double)((tiles * splits + sms - 1) / sms);
+            const double cost = rounds * (((g.kblocks + splits - 1) / splits) * stage + 3000.0 + 20.0 * bt) + (splits > 1 ? 3000.0 : 0.0);
+            if (!g.BT || cost < best) best = cost, g.BT = bt, g.splits = splits;
+        }
+    }
+    const bool vec = K % V == 0 && lda % V == 0 && ((uintptr_t)w | (uintptr_t)a) % 16 == 0;
+    auto kern = vec ? gemm_any_kernel<E, true> : gemm_any_kernel<E, false>;
+    const size_t smem = 1024 + (size_t)parts_of<E>::stages * std::max<size_t>(stage_bytes<E>(g.BT), (size_t)g.BT * kM * 4 / parts_of<E>::stages) + kCtl;
+    const int rc = ggb_allow_smem(kern, smem);
+    if (rc) return rc;
+    const int64_t ctas = n_tiles * ((T + g.BT - 1) / g.BT) * g.splits;
+    GGB_CHECK_ARG(ctas < (1ll << 31), "linear: %lld tiles", (long long)ctas);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ggb_cuda_stream();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)g.splits, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+    cfg.attrs = at, cfg.numAttrs = g.splits > 1 ? 1 : 0;
+    GGB_CUDA(cudaLaunchKernelEx(&cfg, kern, g));
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
+}
+
+} // namespace
+
+int ggb_gemm_any(int dt, const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
+    return dt == GGB_TYPE_BF16 ? launch_any<__nv_bfloat16>(w, N, K, a, lda, T, c, ldc, c_act, act) : launch_any<float>(w, N, K, a, lda, T, c, ldc, c_act, act);
+}
