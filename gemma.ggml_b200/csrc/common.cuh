@@ -20,8 +20,9 @@ cudaStream_t ggb_cuda_stream();
 void ggb_count_launch(int n = 1);
 // What is kept from call to call belongs to the context (ggb_shutdown gives it back; a later ggb_init, of another device perhaps, starts
 // without it): device memory that only grows, its content not kept, and how much dynamic shared memory a kernel may take
-enum ggb_workspace_id { GGB_WS_GEMM_SPLITS, GGB_WS_MOE_GATHER, GGB_WS_ARGMAX, GGB_WS_COUNT };
+enum ggb_workspace_id { GGB_WS_GEMM_SPLITS, GGB_WS_MOE_GATHER, GGB_WS_ARGMAX, GGB_WS_RECURRENCE, GGB_WS_COUNT };
 int ggb_workspace(ggb_workspace_id id, size_t bytes, void **p);
+bool ggb_workspace_fits(ggb_workspace_id id, size_t bytes); // it is that large, or may grow: no graph is being captured
 int ggb_allow_smem_of(const void *kernel, size_t bytes);
 template <typename... P> int ggb_allow_smem(void (*kernel)(P...), size_t bytes) { return ggb_allow_smem_of(reinterpret_cast<const void *>(kernel), bytes); }
 

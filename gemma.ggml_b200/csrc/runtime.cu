@@ -83,6 +83,7 @@ int ggb_workspace(ggb_workspace_id id, size_t bytes, void **p) {
     *p = g_ctx.ws[id];
     return GGB_OK;
 }
+bool ggb_workspace_fits(ggb_workspace_id id, size_t bytes) { return bytes <= g_ctx.ws_bytes[id] || !g_ctx.capturing; }
 int ggb_allow_smem_of(const void *kernel, size_t bytes) {
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
