@@ -154,14 +154,20 @@ static inline float ggb_synth_unit(float sigma) {
 // A layer of 10 such kernels (2048 wide, 16 heads, 8192 in the feed-forward, one token, replayed as a graph): 60.1 us plainly launched,
 // 56.8 like this.  Letting the next one start at once (griddepcontrol.launch_dependents) gives no more: 57.3 behind the wait, 63.5 ahead of
 // it.  Nor does bringing a mat-vec's matrix into L2 before the wait: 63 to 70, the lines are asked for twice.
-template <typename... P, typename... A> cudaError_t ggb_launch_step(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+// cluster_z: CTAs along z that are one cluster
+template <typename... P, typename... A> cudaError_t ggb_launch_step_cluster(void (*k)(P...), int cluster_z, dim3 grid, dim3 block, size_t smem, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at, cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = (unsigned)cluster_z;
+    cfg.attrs = at, cfg.numAttrs = cluster_z > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+template <typename... P, typename... A> cudaError_t ggb_launch_step(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    return ggb_launch_step_cluster(k, 1, grid, block, smem, args...);
 }
 #endif
 

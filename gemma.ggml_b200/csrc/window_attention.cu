@@ -12,8 +12,8 @@
 //   consecutive tokens of one head, 4 per warp.  Their windows
 //   overlap almost wholly, so every tile of 32 cache rows is staged once in shared memory as fp32 (row pitch odd in words:
 //   lane = row reads are conflict-free) and serves all 32 queries; a K word read feeds 4 multiply-adds.
-//   steps of few tokens (window_attn_kernel): 8 warps split one (token, head)'s keys, rows straight from the cache
-//   (several loads in flight), parts merged through shared memory.
+//   steps of few tokens (window_step_kernel): the keys of one (token, head) cut over the CTAs of a cluster, rows straight from the cache in
+//   16-byte pieces, parts merged through shared memory; other types, sizes and alignments in window_attn_kernel, a lane a row.
 //
 // The same kernels serve other masks and layouts, all arguments: the visible range of a query is a sliding window or the
 // chunk of consecutive positions it lies in (chunks counted from position 0), a score may pass a soft cap
@@ -440,6 +440,182 @@ __global__ void __launch_bounds__(32 * kWarps) window_attn_kernel(const float *q
     else diff_finish(acc[0], l[0], acc[MAPS - 1], l[MAPS - 1], t, h, lane, Dv, da, orow);
 }
 
+// A step of few tokens over heads of whole 16-byte pieces: CTA (token, head, split), the splits of a head a cluster.
+// LG lanes share a cache row, a 16-byte piece of it each: a warp's load covers 32 / LG rows without a gap, all of a tile's keys
+// and values are in flight together (the values of two maps follow the scores: registers), and the queries stay in registers.  The lanes'
+// partial scores of a tile meet in one folded butterfly, which leaves a row's score in a lane; the splits' sums meet in
+// shared memory of the cluster's first CTA.
+// Bound by latency: position, page table, rows, one after the other, then the merge.  One token, 16 heads of 128 over 4, 1024 + 4 keys, bf16: 18.8 + 6.6
+// us cold in two launches (a lane a row, values in 2-byte loads), 12.9 us; a dense layer's step 57.1 -> 51.8 us.
+// More than kStepHeads (token, head) pairs keep window_attn_kernel: it holds several CTAs an SM, and many clusters are slow to place (64 pairs over 500
+// positions 17 against 26 us, 256 over 16 positions 15 against 73).
+constexpr int kMaxCluster = 8, kStepHeads = 32;
+template <int LG> struct step_tile { // rows of a tile and the loads they take
+    static constexpr int rows_per_load = 32 / LG, loads = LG <= 16 ? LG : 16, rows = loads * rows_per_load;
+};
+
+template <typename E, int MAPS, int LG>
+__global__ void __launch_bounds__(32 * kWarps) window_step_kernel(const float *q, const E *cache, int64_t cache_ld, const int32_t *table, int B, const int32_t *pos0,
+                                                                  int H, int G, int D, int Dv, int64_t window, int chunked, int64_t keep, float cap,
+                                                                  const float *cs_v, finish_args da, E *out) {
+    constexpr int VN = RowVec<E>::n, RPL = step_tile<LG>::rows_per_load, NL = step_tile<LG>::loads, RT = step_tile<LG>::rows, W = LG * VN;
+    __shared__ float s_acc[kWarps][MAPS][W], s_ml[kWarps][MAPS][2], s_out[MAPS][W + 2]; // s_out: this CTA's sums, maximum, denominator
+    step_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LG, pc = lane % LG;
+    const int h = blockIdx.y, g = h / (H / G);
+    const int64_t t = blockIdx.x, i = (int64_t)*pos0 + t;
+    float qv[MAPS][VN];
+#pragma unroll
+    for (int a = 0; a < MAPS; a++)
+#pragma unroll
+        for (int u = 0; u < VN; u++) qv[a][u] = pc * VN < D ? q[((t * H + h) * MAPS + a) * D + pc * VN + u] : 0.f;
+    // tiles: those of the kept positions [0, n_keep) first, then those of [jlo, i]
+    const int64_t jlo = first_visible(i, window, chunked), n_keep = min(keep, jlo);
+    const int n_kt = (int)((n_keep + RT - 1) / RT);
+    const E *krow0 = cache + (int64_t)g * MAPS * D + pc * VN, *vrow0 = cache + (int64_t)G * MAPS * D + (int64_t)g * Dv + pc * VN;
+    float acc[MAPS][VN], m[MAPS], l[MAPS];
+#pragma unroll
+    for (int a = 0; a < MAPS; a++) {
+        m[a] = -INFINITY, l[a] = 0.f;
+#pragma unroll
+        for (int u = 0; u < VN; u++) acc[a][u] = 0.f;
+    }
+    for (int64_t n = (int64_t)blockIdx.z * kWarps + warp;; n += kWarps * (int64_t)gridDim.z) {
+        const int64_t j0 = n < n_kt ? RT * n : jlo + RT * (n - n_kt), j_last = n < n_kt ? n_keep - 1 : i;
+        if (j0 > j_last) break; // only behind the last tile of the window: the kept tiles hold a position each
+        const int64_t jr = min(j0 + (lane < RT ? lane : RT - 1), j_last); // a row past the last visible one repeats it with weight 0
+        const int64_t my_row = ((int64_t)table[jr / B] * B + jr % B) * cache_ld;
+        RowVec<E> kx[MAPS][NL], vx[NL];
+        auto load_v = [&]() {
+#pragma unroll
+            for (int b = 0; b < NL; b++) {
+                const int64_t row = __shfl_sync(0xffffffffu, my_row, b * RPL + sub);
+                vx[b].raw = pc * VN < Dv ? *reinterpret_cast<const uint4 *>(vrow0 + row) : make_uint4(0, 0, 0, 0);
+            }
+        };
+#pragma unroll
+        for (int b = 0; b < NL; b++) {
+            const int64_t row = __shfl_sync(0xffffffffu, my_row, b * RPL + sub);
+#pragma unroll
+            for (int a = 0; a < MAPS; a++) kx[a][b].raw = pc * VN < D ? *reinterpret_cast<const uint4 *>(krow0 + row + a * D) : make_uint4(0, 0, 0, 0);
+        }
+        if (MAPS == 1) load_v();
+        float p[MAPS];
+        // the load whose row's score this lane gets, and whether it is the one lane that counts it
+        const int mine = LG == 32 ? lane >> 1 : pc;
+        const bool seen = j0 + mine * RPL + sub <= j_last, counts = seen && (LG < 32 || !(lane & 1));
+#pragma unroll
+        for (int a = 0; a < MAPS; a++) {
+            float v[NL];
+#pragma unroll
+            for (int b = 0; b < NL; b++) {
+                float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+                for (int u = 0; u < VN; u += 2) {
+                    a0 = fmaf(kx[a][b].at(u), qv[a][u], a0);
+                    a1 = fmaf(kx[a][b].at(u + 1), qv[a][u + 1], a1);
+                }
+                v[b] = a0 + a1;
+            }
+#pragma unroll
+            for (int k = NL / 2, off = LG / 2; k >= 1; k >>= 1, off >>= 1) {
+                const bool up = lane & off;
+#pragma unroll
+                for (int b = 0; b < k; b++) v[b] = (up ? v[k + b] : v[b]) + __shfl_xor_sync(0xffffffffu, up ? v[b] : v[k + b], off);
+            }
+            if (LG == 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            const float s = seen ? soft_cap(v[0], cap) : -INFINITY;
+            const float m_new = fmaxf(m[a], warp_max_f32(s)); // finite: key j0 of the tile is always visible
+            p[a] = seen ? expf(s - m_new) : 0.f;
+            const float corr = expf(m[a] - m_new); // m = -inf at the first tile: 0
+            l[a] = l[a] * corr + warp_sum_f32(counts ? p[a] : 0.f);
+#pragma unroll
+            for (int u = 0; u < VN; u++) acc[a][u] *= corr;
+            m[a] = m_new;
+        }
+        if (MAPS != 1) load_v();
+#pragma unroll
+        for (int b = 0; b < NL; b++)
+#pragma unroll
+            for (int a = 0; a < MAPS; a++) {
+                const float pb = __shfl_sync(0xffffffffu, p[a], LG == 32 ? 2 * b : sub * LG + b);
+#pragma unroll
+                for (int u = 0; u < VN; u++) acc[a][u] = fmaf(pb, vx[b].at(u), acc[a][u]);
+            }
+    }
+    // the warps' sums, then the splits', each in order
+#pragma unroll
+    for (int a = 0; a < MAPS; a++) {
+#pragma unroll
+        for (int off = LG; off < 32; off <<= 1)
+#pragma unroll
+            for (int u = 0; u < VN; u++) acc[a][u] += __shfl_xor_sync(0xffffffffu, acc[a][u], off);
+        if (sub == 0)
+#pragma unroll
+            for (int u = 0; u < VN; u++) s_acc[warp][a][pc * VN + u] = acc[a][u];
+        if (lane == 0) s_ml[warp][a][0] = m[a], s_ml[warp][a][1] = l[a];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < MAPS * W; e += 32 * kWarps) {
+        const int a = e / W, c = e - a * W;
+        float M = -INFINITY, x = 0.f, y = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) M = fmaxf(M, s_ml[w][a][0]);
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) {
+            const float f = s_ml[w][a][0] == -INFINITY ? 0.f : expf(s_ml[w][a][0] - M); // a warp without keys
+            x = fmaf(s_acc[w][a][c], f, x);
+            y = fmaf(s_ml[w][a][1], f, y);
+        }
+        s_out[a][c] = x;
+        if (c == 0) s_out[a][W] = M, s_out[a][W + 1] = y;
+    }
+    if (gridDim.z > 1) {
+        cluster_sync();
+        if (blockIdx.z == 0) {
+            __syncthreads();
+            for (int e = threadIdx.x; e < MAPS * W; e += 32 * kWarps) {
+                const int a = e / W, c = e - a * W, n = (int)gridDim.z;
+                const uint32_t at = smem_u32(&s_out[a][0]);
+                float mz[kMaxCluster], xz[kMaxCluster], lz[kMaxCluster], M = -INFINITY, x = 0.f, y = 0.f;
+#pragma unroll
+                for (int z = 0; z < kMaxCluster; z++) {
+                    const uint32_t from = cluster_addr(at, min(z, n - 1));
+                    xz[z] = ld_cluster_f32(from + 4 * c), mz[z] = ld_cluster_f32(from + 4 * W), lz[z] = ld_cluster_f32(from + 4 * W + 4);
+                }
+#pragma unroll
+                for (int z = 0; z < kMaxCluster; z++) M = fmaxf(M, mz[z]);
+#pragma unroll
+                for (int z = 0; z < kMaxCluster; z++) {
+                    const float f = z >= n || mz[z] == -INFINITY ? 0.f : expf(mz[z] - M); // a split without keys
+                    if (z < n) x = fmaf(xz[z], f, x), y = fmaf(lz[z], f, y);
+                }
+                s_acc[0][a][c] = x; // (the first CTA's own sums are read by all of its threads until the barrier below)
+                if (c == 0) s_ml[0][a][0] = M, s_ml[0][a][1] = y;
+            }
+        }
+        cluster_sync(); // the others' shared memory is read until here
+        if (blockIdx.z != 0) return;
+    } else {
+        __syncthreads();
+        for (int e = threadIdx.x; e < MAPS * W; e += 32 * kWarps) s_acc[0][e / W][e % W] = s_out[e / W][e % W];
+        if (threadIdx.x < MAPS) s_ml[0][threadIdx.x][0] = s_out[threadIdx.x][W], s_ml[0][threadIdx.x][1] = s_out[threadIdx.x][W + 1];
+        __syncthreads();
+    }
+    if (warp != 0) return;
+    float o[MAPS][kMaxDvRegs];
+#pragma unroll
+    for (int a = 0; a < MAPS; a++)
+#pragma unroll
+        for (int r = 0; r < kMaxDvRegs; r++) {
+            const int c = 2 * lane + 64 * (r >> 1) + (r & 1);
+            o[a][r] = c < W ? s_acc[0][a][c] : 0.f;
+        }
+    E *orow = out + (t * H + h) * Dv;
+    if (MAPS == 1) window_finish(o[0], s_ml[0][0][0], s_ml[0][0][1], i, t, h, lane, Dv, cs_v, da, orow);
+    else diff_finish(o[0], s_ml[0][0][1], o[MAPS - 1], s_ml[0][MAPS - 1][1], t, h, lane, Dv, da, orow);
+}
+
 // one warp per (token, head): the splits' parts merged, then as above
 template <typename E, int MAPS>
 __global__ void __launch_bounds__(32) window_merge_kernel(const float *part, int n_split, const int32_t *pos0, int H, int Dv,
@@ -826,6 +1002,22 @@ static int masked_attn_launch(int dt, const float *q, const void *cache, const i
         }
 #undef WT_NP
 #undef WT_LAUNCH
+    } else if (vec && Dv % vn == 0 && std::max(D, Dv) <= 32 * vn && T * H <= kStepHeads) { // a step: whole pieces, a row by at most a warp
+        const int pieces = std::max(D, Dv) / vn, lg = pieces <= 8 ? 8 : pieces <= 16 ? 16 : 32, rows = lg <= 16 ? 32 : 16;
+        // a warp a tile: as many splits as the longest visible range has groups of 8 tiles (bounded by the window), up to a cluster that the chip
+        // has room for beside the others (an SM holds one such CTA)
+        int n_split = T * H <= 8 ? kMaxCluster : kMaxCluster / 2;
+        if (window > 0) n_split = (int)std::min<int64_t>(n_split, ((window + 2 * rows - 2) / rows + (keep + rows - 1) / rows + kWarps - 1) / kWarps);
+        const dim3 grid((unsigned)T, (unsigned)H, (unsigned)n_split);
+#define ST_LAUNCH(ET, LG)                                                                                                                            \
+    GGB_CUDA(ggb_launch_step_cluster(window_step_kernel<ET, MAPS, LG>, n_split, grid, dim3(32 * kWarps), 0, q, (const ET *)cache, cld, block_table, block_size, \
+                                     pos0, H, G, D, Dv, window, chunked, keep, softcap, cos_sin_v, da, (ET *)out));
+        if (dt == GGB_TYPE_BF16) {
+            if (lg == 8) { ST_LAUNCH(__nv_bfloat16, 8) } else if (lg == 16) { ST_LAUNCH(__nv_bfloat16, 16) } else { ST_LAUNCH(__nv_bfloat16, 32) }
+        } else {
+            if (lg == 8) { ST_LAUNCH(float, 8) } else if (lg == 16) { ST_LAUNCH(float, 16) } else { ST_LAUNCH(float, 32) }
+        }
+#undef ST_LAUNCH
     } else {
         const size_t smem = (size_t)kWarps * MAPS * ((size_t)Dp + kPartW) * 4;
         GGB_CHECK_ARG(smem <= 48 * 1024, "window_attn: key size %d does not fit shared memory", D);
