@@ -117,6 +117,8 @@ _CUDA_SIG = {
     "ggb_gemm_workspace_bytes": (sz, [i64, i64, i64]),
     "ggb_op_gemm_bf16": (i32, [vp, vp, i64, vp, i64, vp, vp, sz]),
     "ggb_op_gemm_bf16_multi": (i32, [i32, vp, vp, i64, vp, vp, vp, sz]),
+    "ggb_op_gemm_norm_bf16": (i32, [vp, vp, i64, vp, vp, vp, sz, vp, f32, vp]),
+    "ggb_op_gemm_rope_store_bf16": (i32, [vp, vp, i64, vp, vp, sz, vp, i32, i32, i32, f32, vp, vp]),
     "ggb_op_cvt_f32_bf16": (i32, [vp, i64, vp]), "ggb_op_gemm_geglu_bf16": (i32, [vp, vp, vp, i64, vp]),
     "ggb_gemm_pieces": (i32, [i64, i64, i64]),
     "ggb_op_rms_norm_bf16": (i32, [vp, vp, f32, i64, i64, vp]), "ggb_op_geglu_bf16": (i32, [vp, vp, i64, vp]),

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 if (kbase + 2 * u >= kb1) break;
-                mbar_wait_bounded(bars + C_FULL + 8 * s, ph, dead);
+                mbar_wait_warp(bars + C_FULL + 8 * s, ph, dead);
                 uint4 o[4];
                 if (mine) { // rows past the matrix: zero codes (TMA) and zero scales
                     const float d0 = __half2float(cur[u]);
@@ -418,6 +418,84 @@ rms_norm_bf16_kernel(const float *__restrict__ x, const float *__restrict__ w, f
     for (int64_t i = tid; i < E; i += GGB_DEV_NORM_THREADS)
         y[(int64_t)blockIdx.x * E + i] = __float2bfloat16_rn(__fmul_rn(__fmul_rn(xr[i], scale), w[i]));
 }
+
+// What follows a product that several CTAs summed along K, with the adding of its pieces: the sums as splitk_reduce_kernel takes them, then the
+// arithmetic of the kernel that would read them, to the bit, without a launch and a pass over memory between.  512 x 2048 in 8 pieces: 10.2 + 4.9 us
+// for sums and norm, 12.8 us; 512 x 2560 in 4 pieces: 8 + 6.5 us for sums and rotation, 11.8 us (all cold).  Bound by reading the pieces.
+__device__ __forceinline__ float pieces_sum(const float *ws, int64_t plane, int pieces) {
+    float v[8], s;
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = i < pieces ? ws[i * plane] : 0.f;
+    s = v[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++)
+        if (i < pieces) s += v[i];
+    return s;
+}
+
+// c = pieces (+ residual); y = rms_norm(c) * w in bf16 (rms_norm_bf16_kernel)
+__global__ void __launch_bounds__(GGB_DEV_NORM_THREADS) splitk_norm_kernel(const GemmArgs A, int pieces, const float *w, float eps, __nv_bfloat16 *y) {
+    __shared__ double s_w[GGB_DEV_NORM_THREADS / 32];
+    extern __shared__ float s_row[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, E = A.N;
+    const int64_t t = blockIdx.x, plane = (int64_t)A.T * E;
+    const GemmSeg &sg = A.seg[0];
+    double acc = 0.0;
+#pragma unroll 2
+    for (int i = tid; i < E; i += GGB_DEV_NORM_THREADS) {
+        float v = pieces_sum(A.ws + t * E + i, plane, pieces);
+        if (A.resid) v += A.resid[t * sg.ldc + i];
+        sg.c[t * sg.ldc + i] = v;
+        s_row[i] = v;
+        acc = __dadd_rn(acc, (double)__fmul_rn(v, v));
+    }
+    acc = warp_sum_f64(acc);
+    if (lane == 0) s_w[warp] = acc;
+    __syncthreads();
+    double sum = s_w[0];
+#pragma unroll
+    for (int i = 1; i < GGB_DEV_NORM_THREADS / 32; i++) sum = __dadd_rn(sum, s_w[i]);
+    const float mean = __double2float_rn(__ddiv_rn(sum, (double)E));
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+    for (int i = tid; i < E; i += GGB_DEV_NORM_THREADS) y[t * E + i] = __float2bfloat16_rn(__fmul_rn(__fmul_rn(s_row[i], scale), w[i]));
+}
+
+// q | k | v: the rotation of q (times q_scale, to seg[0].c) and k, k and v to the cache (rope_kv_store_batch_kernel)
+struct rope_args {
+    const int32_t *pos;
+    int H, Hkv, d, table_ctx;
+    float q_scale;
+    const float *cosT, *sinT;
+    __half *kcache, *vcache;
+};
+__global__ void splitk_rope_kernel(const GemmArgs A, int pieces, const rope_args r) {
+    const int half = r.d / 2, nq = r.H * half, nk = r.Hkv * half, nv = r.Hkv * r.d, idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t t = blockIdx.y, plane = (int64_t)A.T * A.N;
+    int pos = r.pos[t];
+    pos = pos < 0 ? 0 : (pos >= r.table_ctx ? r.table_ctx - 1 : pos);
+    const float *row = A.ws + t * A.N;
+    if (idx < nq + nk) {
+        const bool is_q = idx < nq;
+        const int j = is_q ? idx : idx - nq, h = j / half, i = j % half;
+        const float c = r.cosT[(int64_t)pos * half + i], s = r.sinT[(int64_t)pos * half + i];
+        const float *src = row + A.seg[is_q ? 0 : 1].n_begin + h * r.d + i;
+        const float x0 = pieces_sum(src, plane, pieces), x1 = pieces_sum(src + half, plane, pieces);
+        const float r0 = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)), r1 = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
+        if (is_q) {
+            float *qt = A.seg[0].c + t * A.seg[0].ldc + h * r.d + i;
+            qt[0] = __fmul_rn(r0, r.q_scale);
+            qt[half] = __fmul_rn(r1, r.q_scale);
+        } else {
+            __half *kr = r.kcache + (int64_t)pos * r.Hkv * r.d + h * r.d + i;
+            kr[0] = __float2half_rn(r0);
+            kr[half] = __float2half_rn(r1);
+        }
+    } else if (idx < nq + nk + nv) {
+        const int j = idx - nq - nk;
+        r.vcache[(int64_t)pos * r.Hkv * r.d + j] = __float2half_rn(pieces_sum(row + A.seg[2].n_begin + j, plane, pieces));
+    }
+}
+
 // gelu(gate) * up -> bf16 (fp16 gelu table like the reference's ggml_gelu; ref: src/gemma_model.cpp:448-449)
 __global__ void geglu_bf16_kernel(const float *gate, const float *up, int64_t n, const uint16_t *__restrict__ table,
                                   __nv_bfloat16 *y) {
@@ -762,8 +840,17 @@ int ggb_op_geglu_bf16(const float *gate, const float *up, int64_t n, void *y_bf1
     return GGB_OK;
 }
 
+// what the sums of a split product go through; `done` says that they did (a product that is not split leaves it to its caller)
+struct gemm_tail {
+    const float *norm_w = nullptr;
+    float eps = 0.f;
+    __nv_bfloat16 *y = nullptr;
+    const rope_args *rope = nullptr;
+    bool done = false;
+};
+
 static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, const int64_t *ldc,
-                       const float *resid, void *workspace, size_t workspace_bytes, void *geglu = nullptr) {
+                       const float *resid, void *workspace, size_t workspace_bytes, void *geglu = nullptr, gemm_tail *tail = nullptr) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(n >= 1 && n <= kMaxSegs && w && a_bf16 && c && ldc && T > 0, "bad gemm args");
     GGB_CHECK_ARG(n == 1 || !resid, "gemm: a residual needs a single matrix");
@@ -851,7 +938,19 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     if (splits > 1) {
         A.resid = resid;
         const int64_t cnt = T * N;
-        splitk_reduce_kernel<<<(unsigned)((cnt / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, (kblocks + A.chunk_kb - 1) / A.chunk_kb);
+        const int planes = (kblocks + A.chunk_kb - 1) / A.chunk_kb;
+        if (tail && tail->rope) {
+            const rope_args &r = *tail->rope;
+            const int total = (r.H + r.Hkv) * (r.d / 2) + r.Hkv * r.d;
+            splitk_rope_kernel<<<dim3((unsigned)((total + 255) / 256), (unsigned)T), 256, 0, ggb_cuda_stream()>>>(A, planes, r);
+        } else if (tail) {
+            const size_t row = (size_t)N * 4;
+            if ((rc = ggb_allow_smem(splitk_norm_kernel, row))) return rc;
+            splitk_norm_kernel<<<(unsigned)T, GGB_DEV_NORM_THREADS, row, ggb_cuda_stream()>>>(A, planes, tail->norm_w, tail->eps, tail->y);
+        } else {
+            splitk_reduce_kernel<<<(unsigned)((cnt / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, planes);
+        }
+        if (tail) tail->done = true;
         GGB_LAUNCH_CHECK();
     }
     return GGB_OK;
@@ -869,6 +968,32 @@ int ggb_op_gemm_bf16(const ggb_weight *w, const void *a_bf16, int64_t T, float *
 int ggb_op_gemm_bf16_multi(int n, const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, const int64_t *ldc,
                            void *workspace, size_t workspace_bytes) {
     return gemm_launch(n, w, a_bf16, T, c, ldc, nullptr, workspace, workspace_bytes);
+}
+
+int ggb_op_gemm_norm_bf16(const ggb_weight *w, const void *a_bf16, int64_t T, float *c, const float *resid, void *workspace, size_t workspace_bytes,
+                          const float *norm_w, float eps, void *y_bf16) {
+    GGB_CHECK_ARG(w && norm_w && y_bf16, "bad gemm_norm args");
+    const ggb_weight *ws[1] = {w};
+    float *cs[1] = {c};
+    const int64_t ls[1] = {w->rows};
+    gemm_tail tail{norm_w, eps, (__nv_bfloat16 *)y_bf16};
+    const bool fits = (size_t)w->rows * 4 <= 200 * 1024; // a row in shared memory
+    const int rc = gemm_launch(1, ws, a_bf16, T, cs, ls, resid, workspace, workspace_bytes, nullptr, fits ? &tail : nullptr);
+    return rc || tail.done ? rc : ggb_op_rms_norm_bf16(c, norm_w, eps, w->rows, T, y_bf16);
+}
+
+int ggb_op_gemm_rope_store_bf16(const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, void *workspace, size_t workspace_bytes,
+                                const int32_t *pos, int H, int Hkv, int d, float q_scale, void *kcache, void *vcache) {
+    GGB_REQUIRE_INIT();
+    GGB_CHECK_ARG(w && w[0] && w[1] && w[2] && c && c[0] && c[1] && c[2] && pos && kcache && vcache && T > 0 && T <= 65535, "bad gemm_rope_store args");
+    GGB_CHECK_ARG(w[0]->rows == (int64_t)H * d && w[1]->rows == (int64_t)Hkv * d && w[2]->rows == (int64_t)Hkv * d, "gemm_rope_store: rows of q, k, v");
+    GGB_CHECK_ARG(ggb_rope_cos_dev() && ggb_rope_n_dims() == d, "rope table not initialised for head_dim %d", d);
+    const rope_args r{pos, H, Hkv, d, ggb_rope_n_ctx(), q_scale, ggb_rope_cos_dev(), ggb_rope_sin_dev(), (__half *)kcache, (__half *)vcache};
+    const int64_t ls[3] = {w[0]->rows, w[1]->rows, w[2]->rows};
+    gemm_tail tail;
+    tail.rope = &r;
+    const int rc = gemm_launch(3, w, a_bf16, T, c, ls, nullptr, workspace, workspace_bytes, nullptr, &tail);
+    return rc || tail.done ? rc : ggb_op_rope_kv_store_batch(c[0], c[1], c[2], pos, T, H, Hkv, d, q_scale, kcache, vcache);
 }
 
 int ggb_op_gemm_geglu_bf16(const ggb_weight *gate, const ggb_weight *up, const void *a_bf16, int64_t T, void *y_bf16) {

@@ -767,13 +767,12 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
     for (int i = 0; i < T; i++) pos[(size_t)i] = pos0 + i;
     GM_TRY(ggb_upload(pf_ids_, tokens, (size_t)T * 4));
     GM_TRY(ggb_upload(pf_pos_, pos.data(), (size_t)T * 4));
-    auto gemm_of = [&](const ggb_weight *w, int64_t K, const void *a, float *out, const float *resid) -> int {
+    // a product whose rows are normed next (the A operand of the product after it): pf_a_
+    auto gemm_norm = [&](const ggb_weight *w, int64_t K, const void *a, float *out, const float *resid, const float *norm_w) -> int {
         pf_flops_ += 2.0 * (double)t * (double)K * (double)ggb_weight_rows(w);
-        const int64_t N = ggb_weight_rows(w);
-        const bool small = N <= pf_ws_n_;
-        return ggb_op_gemm_bf16(w, a, t, out, N, resid, small ? pf_ws_ : nullptr, small ? pf_ws_bytes_ : 0);
+        const bool small = ggb_weight_rows(w) <= pf_ws_n_;
+        return ggb_op_gemm_norm_bf16(w, a, t, out, resid, small ? pf_ws_ : nullptr, small ? pf_ws_bytes_ : 0, norm_w, c.eps, pf_a_);
     };
-    auto gemm = [&](const ggb_weight *w, int64_t K, float *out, const float *resid) -> int { return gemm_of(w, K, pf_a_, out, resid); };
     // matrices that share the A operand go out as ONE launch (more tiles per launch, one pass over A)
     auto gemm_multi = [&](int n, const ggb_weight *const *w, int64_t K, float *const *outs) -> int {
         int64_t ld[3], total = 0;
@@ -790,24 +789,29 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
     const bool fuse_gate_up = t > 128 && F % 256 == 0 && (2 * F > pf_ws_n_ || ggb_gemm_pieces(t, 2 * F, E) == 1);
     pf_flops_ = 0.0;
     PROFILE("op_get_rows", ggb_op_get_rows(token_embd_, pf_ids_, t, sqrtf((float)c.n_embd), pf_x_));   // :675-679
+    PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_x_, c.n_layer ? layers_[0].attn_norm : output_norm_, c.eps, E, t, pf_a_)); // :690
     for (int il = 0; il < c.n_layer; il++) {
         const gemma_layer &l = layers_[(size_t)il];
         void *kc = k_cache_[(size_t)il], *vc = v_cache_[(size_t)il];
-        PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_x_, l.attn_norm, c.eps, E, t, pf_a_));           // :690
         {
+            // q | k | v (:692-696), rope(q) * q_scale, rope(k) and v straight into the position-major fp16 cache rows pos0 .. pos0+T-1
+            // (ref :698-716 rope + scale, :499-518 KV store)
             const ggb_weight *w3[3] = {l.attn_q, l.attn_k, l.attn_v};
             float *o3[3] = {pf_q_, pf_k_, pf_v_};
-            PROFILE("op_mul_mat", gemm_multi(3, w3, E, o3));                                             // :692-696
+            int64_t total = 0;
+            for (int i = 0; i < 3; i++) {
+                const int64_t rows = ggb_weight_rows(w3[i]);
+                pf_flops_ += 2.0 * (double)t * (double)E * (double)rows;
+                total += i < 2 ? (rows + 255) / 256 * 256 : rows;
+            }
+            const bool small = total <= pf_ws_n_;
+            PROFILE("op_mul_mat", ggb_op_gemm_rope_store_bf16(w3, pf_a_, t, o3, small ? pf_ws_ : nullptr, small ? pf_ws_bytes_ : 0, pf_pos_, c.n_head, c.n_head_kv,
+                                                              c.head_dim, q_scale, kc, vc));
         }
-        // rope(q) * q_scale in place, rope(k) and v straight into the position-major fp16 cache rows pos0 .. pos0+T-1
-        // (ref :698-716 rope + scale, :499-518 KV store): one launch
-        PROFILE("op_rope", ggb_op_rope_kv_store_batch(pf_q_, pf_k_, pf_v_, pf_pos_, t, c.n_head, c.n_head_kv, c.head_dim,
-                                                       q_scale, kc, vc));
         // kqv goes straight out as the bf16 A operand of the o-projection (the fp32 copy only for captures)
         PROFILE("op_attn", ggb_op_attn_prefill(pf_q_, kc, vc, t, pos0, c.n_head, c.n_head_kv, c.head_dim,
                                                capture_acts_ ? pf_attn_ : nullptr, pf_a_)); // :454-489
-        PROFILE("op_mul_mat", gemm(l.attn_output, QD, pf_sa_, pf_x_));                                   // :493 + :723
-        PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_sa_, l.ffn_norm, c.eps, E, t, pf_a_));            // :727
+        PROFILE("op_mul_mat", gemm_norm(l.attn_output, QD, pf_a_, pf_sa_, pf_x_, l.ffn_norm));           // :493 + :723, :727
         if (fuse_gate_up) { // both products and gelu(gate) * up in one launch                                // :446-449
             pf_flops_ += 4.0 * (double)t * (double)E * (double)F;
             PROFILE("op_mul_mat", ggb_op_gemm_geglu_bf16(l.ffn_gate, l.ffn_up, pf_a_, t, pf_act_));
@@ -817,10 +821,10 @@ int gemma_model::prefill(const token_id *tokens, int T, int32_t pos0, token_id *
             PROFILE("op_mul_mat", gemm_multi(2, w2, E, o2));                                             // :446-447
             PROFILE("op_gelu", ggb_op_geglu_bf16(pf_g_, pf_u_, t * F, pf_act_));                         // :448-449
         }
-        PROFILE("op_mul_mat", gemm_of(l.ffn_down, F, pf_act_, pf_x_, pf_sa_));                           // :450 + :731
+        PROFILE("op_mul_mat", gemm_norm(l.ffn_down, F, pf_act_, pf_x_, pf_sa_, il + 1 < c.n_layer ? layers_[(size_t)il + 1].attn_norm : output_norm_)); // :450 + :731, :690 / :735
     }
-    PROFILE("op_rms_norm", ggb_op_rms_norm_bf16(pf_x_, output_norm_, c.eps, E, t, pf_a_));               // :735
-    PROFILE("op_mul_mat", gemm(token_embd_, E, pf_logits_, nullptr));                                    // :740 (all T rows)
+    pf_flops_ += 2.0 * (double)t * (double)E * (double)V;
+    PROFILE("op_mul_mat", ggb_op_gemm_bf16(token_embd_, pf_a_, t, pf_logits_, V, nullptr, V <= pf_ws_n_ ? pf_ws_ : nullptr, V <= pf_ws_n_ ? pf_ws_bytes_ : 0)); // :740 (all T rows)
     // greedy token of the last position; decode continues at pos0 + T
     h_state_[0] = 0; h_state_[1] = pos0 + T - 1; h_state_[2] = 1; h_state_[3] = c.n_ctx;
     pos_hint_ = pos0 + T; pos_step_hint_ = 1;

@@ -243,6 +243,13 @@ int ggb_op_gemm_bf16_multi(int n, const ggb_weight *const *w, const void *a_bf16
                            const int64_t *ldc, void *workspace, size_t workspace_bytes);
 /* the pieces along K in which such a product is summed where its workspace is given (one where it is not) */
 int ggb_gemm_pieces(int64_t T, int64_t N, int64_t K);
+/* ggb_op_gemm_bf16 of one matrix (c dense) and y (bf16, [T][rows]) = rms_norm(c) * norm_w, the same bits as ggb_op_rms_norm_bf16 behind it; and
+ * ggb_op_gemm_bf16_multi of q, k and v (dense), then ggb_op_rope_kv_store_batch, again to the bit.  Where the product is cut along K, the kernel that
+ * adds the pieces does the rest (c of k and v is then not written). */
+int ggb_op_gemm_norm_bf16(const ggb_weight *w, const void *a_bf16, int64_t T, float *c, const float *resid, void *workspace,
+                          size_t workspace_bytes, const float *norm_w, float eps, void *y_bf16);
+int ggb_op_gemm_rope_store_bf16(const ggb_weight *const *w, const void *a_bf16, int64_t T, float *const *c, void *workspace, size_t workspace_bytes,
+                                const int32_t *pos, int H, int Hkv, int d, float q_scale, void *kcache, void *vcache);
 /* gate and up of a feed-forward and gelu(gate x) * (up x) in one launch: y (bf16, [T][rows]), the same bits as ggb_op_gemm_bf16_multi
  * without a workspace and ggb_op_geglu_bf16; T > 128, rows %% 256 == 0 */
 int ggb_op_gemm_geglu_bf16(const ggb_weight *gate, const ggb_weight *up, const void *a_bf16, int64_t T, void *y_bf16);
