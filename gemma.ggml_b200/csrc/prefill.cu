@@ -5,11 +5,11 @@
 //
 //   C[T][N] (fp32) = A[T][K] (bf16 activations) x dequant(W[N][K] Q4_0 | Q8_0)^T       (+ residual)
 //
-// More than 256 rows: two CTAs of a cluster compute a tile (cta_group::2) of 512 or 256 rows x up to 256 columns; each holds half of the
-// rows of A and dequantises half of the tile's weight rows, so a prompt of 512 tokens dequantises every weight once.  Fewer rows: one
+// Large products of more than 256 rows: two CTAs of a cluster compute a tile (cta_group::2) of 512 or 256 rows x up to 256 columns; each holds half of the
+// rows of A and dequantises half of the tile's weight rows, so a prompt of 512 tokens dequantises every weight once.  Others: one
 // CTA, 256 or 128 rows x up to 128 columns.  Per 64-wide K block
 //   * one thread requests the CTA's A rows by TMA, another one the raw codes (a ring of their own: they are needed a dequantisation earlier);
-//   * two groups of eight warps take the K blocks alternately and DEQUANTISE the W rows (int8 / int4 codes x fp16 block scale -> bf16, exact
+//   * two groups of eight warps (four of four, eight of two where the tile has fewer weight rows) take the K blocks in turn and DEQUANTISE the W rows (int8 / int4 codes x fp16 block scale -> bf16, exact
 //     product rounded once) from shared memory into shared memory, canonical K-major 128-byte-swizzled UMMA layout;
 //   * one warp (of the pair's first CTA) issues the tcgen05.mma (K = 16, kind::f16, bf16 x bf16 -> fp32) whose accumulators live in TENSOR
 //     MEMORY, up to all 512 columns; tcgen05.commit releases the buffers of both CTAs;
@@ -20,10 +20,12 @@
 // CTA in tensor memory, added in order by the epilogue, and, where SMs are left, several CTAs, whose pieces all meet in a workspace and are
 // added in order by a second kernel: the same bits whichever tile is chosen.
 //
-// What bounds it: shared memory (128 bytes a cycle).  A K block of a pair's CTA (256 rows, 128 weight rows) moves 40 KB in by TMA, 8 KB of codes
-// out, 16 KB of weights in and 64 to 96 KB out for the MMAs: 1550 cycles where the MMAs alone take 1024; the weights of a block stand half a
-// block before its MMAs.  512 tokens, Q8_0: gate | up with gelu 82 us, 838 TFLOP/s, tensor cores 49 % of the cycles (115 us in two launches
-// before), 2048 x 16384 43 us with its reduction (68 us by one CTA a 256 x 256 tile), 2048 x 2048 20 us (36).
+// What bounds it.  Large products: the MMAs (140 cycles each of the 128 that a pair's 256 x 256 x 16 takes at least) and what no other tile
+// hides, 3 us up to the first MMA and 7 us from the last one to the end, at clocks that fall under the power limit.  A K block has one barrier
+// that its A rows and all its dequantising warps arrive on, of both CTAs, and one commit: a wait or commit costs the issuing warp 100 to 200
+// cycles whether it has to wait or not (three waits and two commits a block: 900 cycles a block of any tile).  Small products: that start
+// and end.  512 tokens, Q8_0: gate | up with gelu 72 -> 68 us (1010 TFLOP/s; 115 us in two launches before), 2048 x 16384 in 8 pieces 45 -> 43 us
+// with its sums, 2048 x 2048 20 -> 17 us, q | k | v 22.5 -> 18 us.
 //
 // Numerics: weights q*d are exact in fp32 (8 x 11 bits) and rounded once to bf16; activations are rounded
 // to bf16 instead of being re-quantised to Q8_0 per 32 (the reference's INIT stage), so prefill agrees with
@@ -42,12 +44,13 @@
 namespace {
 
 constexpr int BK = 64;
-constexpr int kWorkWarps = 16, kGroupWarps = 8, kTmaWarp = 16, kMmaWarp = 17, kCodesWarp = 18, kGemmThreads = 32 * 19;
+constexpr int kWorkWarps = 16, kTmaWarp = 16, kMmaWarp = 17, kCodesWarp = 18, kGemmThreads = 32 * 19;
 constexpr uint32_t kRing = 224 * 1024;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 8;
 constexpr size_t kGemmSmem = 1024 + kRing + 512;
-constexpr int kTiles = 2, kMaxCodeStages = 12; // buffers of dequantised weights, of codes
-enum { A_FULL = 0, A_FREE = 48, B_FULL = 96, B_FREE = 128, PEER_FULL = 160, C_FULL = 192, C_FREE = 288, DONE = 384, SLOT = 392, DEAD = 400, TABLE_FULL = 408 };
+constexpr uint32_t kTiles = 256 * 128; // bytes of the buffers of dequantised weights, one a group
+constexpr int kMaxCodeStages = 16;
+enum { FULL = 0, FREE = 64, C_FULL = 128, C_FREE = 256, DONE = 384, SLOT = 392, DEAD = 400, TABLE_FULL = 408 }; // FULL, FREE: of a K block, by its stage of A
 constexpr uint32_t kGeluBytes = 65536 * 2, kGeluAt = 64 * 1024; // the gelu table, behind the epilogue's 16 x 4 KB, in the ring, which the last MMA has left
 
 // up to 3 weight matrices that share the A operand run as ONE launch (Q | K | V, gate | up): a segment = one matrix, its first row is a
@@ -64,7 +67,8 @@ struct GemmArgs {
     int n_seg;
     int N, nb, kblocks;  // N = concatenated rows (padded between segments), nb = K / 32, kblocks = K / 64
     int T, MT, BN;       // a CTA's rows: MT x 128; a tile's columns
-    int chunks, chunk_kb, stages, code_stages; // stages of A rows, of codes (an even number: two groups take them in turn)
+    int groups;                                // of warps, that take the K blocks in turn
+    int chunks, chunk_kb, stages, code_stages; // stages of A rows, of codes (a multiple of the groups)
     uint32_t a_tx;       // bytes of a stage of A that are loaded: a single row tile leaves out what lies 8 rows and more past the last
     int vec;             // rows of every C and of resid start on 16 bytes
     float *ws;           // workspace [pieces of K][T][N] or null (one CTA along K: tiles go straight to seg.c)
@@ -150,21 +154,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
     const int kb0 = split * A.chunks * A.chunk_kb, kb1 = min(kb0 + A.chunks * A.chunk_kb, A.kblocks);
     if (sn0 >= sg.rows) return; // padding between matrices: all CTAs of the tile, before any barrier or tensor memory exists
     const uint32_t b_bytes = (uint32_t)BR * 128, a_bytes = (uint32_t)A.MT * 16384, c_bytes = (uint32_t)BR * 2 * PB;
-    const uint32_t codes = smem0 + kTiles * b_bytes, ring = codes + A.code_stages * c_bytes; // dequantised tiles | codes | A rows
+    const uint32_t codes = smem0 + kTiles, ring = codes + A.code_stages * c_bytes; // dequantised tiles | codes | A rows
 
+    const int group_warps = kWorkWarps / A.groups;
     if (tid == 0) {
         for (int s = 0; s < A.stages; s++) {
-            mbar_init(bars + A_FULL + 8 * s, 1);
-            mbar_init(bars + A_FREE + 8 * s, 1);
+            mbar_init(bars + FULL + 8 * s, 1 + CTAS * group_warps); // the bytes of A and the warps that dequantise, of both CTAs
+            mbar_init(bars + FREE + 8 * s, 1);
         }
         for (int s = 0; s < A.code_stages; s++) {
             mbar_init(bars + C_FULL + 8 * s, 1);
-            mbar_init(bars + C_FREE + 8 * s, kGroupWarps);
-        }
-        for (int s = 0; s < kTiles; s++) {
-            mbar_init(bars + B_FULL + 8 * s, kGroupWarps);
-            mbar_init(bars + B_FREE + 8 * s, 1);
-            mbar_init(bars + PEER_FULL + 8 * s, 1);
+            mbar_init(bars + C_FREE + 8 * s, group_warps);
         }
         mbar_init(bars + DONE, 1);
         mbar_init(bars + TABLE_FULL, 1);
@@ -181,57 +181,58 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(gbase + kRing + SLOT), 0);
 
+    const uint32_t full = PAIR ? cluster_addr(bars + FULL, 0) : bars + FULL; // the issuing CTA's
+
     if (warp < kWorkWarps) {
-        // ================= a group takes every other K block; thread t of it owns ONE quant block (32 weights): row w_row0 + (t >> 1), block 2 kb + (t & 1)
-        const int grp = warp / kGroupWarps, gt = tid & (32 * kGroupWarps - 1), wr = gt >> 1, whalf = gt & 1, wrow = w_row0 + wr;
-        const bool mine = wr < BR, live = mine && wrow < sg.rows;
+        // ================= the groups take the K blocks in turn; thread t of one owns ONE quant block (32 weights): row w_row0 + (t >> 1), block 2 kb + (t & 1)
+        const int G = A.groups, grp = warp / group_warps, gt = tid & (32 * group_warps - 1), wr = gt >> 1, whalf = gt & 1, wrow = w_row0 + wr;
+        const bool live = wrow < sg.rows;
         const __half *dp = sg.d + (size_t)wrow * A.nb + whalf;
+        const uint32_t dst = smem0 + grp * b_bytes + wr * 128;
         __half cur[4], nxt[4]; // scales of the group's next four K blocks, requested while the four before are used
         auto scales = [&](int kb, __half (&d)[4]) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) d[u] = live && kb + 2 * u < kb1 ? __ldg(dp + 2 * (kb + 2 * u)) : __float2half(0.f);
+            for (int u = 0; u < 4; u++) d[u] = live && kb + G * u < kb1 ? __ldg(dp + 2 * (kb + G * u)) : __float2half(0.f);
         };
         scales(kb0 + grp, nxt);
-        uint32_t use = 0; // the group's K blocks so far
-        int s = grp;
-        uint32_t ph = 0;
-        for (int kbase = kb0 + grp; kbase < kb1; kbase += 8) {
+        int s = grp, as = grp, before = -1; // stages of codes and of A; that of A of the group's block before
+        uint32_t ph = 0, aph = 0, bph = 0;
+        for (int kbase = kb0 + grp; kbase < kb1; kbase += 4 * G) {
 #pragma unroll
             for (int u = 0; u < 4; u++) cur[u] = nxt[u];
-            scales(kbase + 8, nxt);
+            scales(kbase + 4 * G, nxt);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                if (kbase + 2 * u >= kb1) break;
+                if (kbase + G * u >= kb1) break;
                 mbar_wait_warp(bars + C_FULL + 8 * s, ph, dead);
                 uint4 o[4];
-                if (mine) { // rows past the matrix: zero codes (TMA) and zero scales
-                    const float d0 = __half2float(cur[u]);
-                    const uint32_t src = codes + s * c_bytes + gt * PB;
-                    if (TYPE == GGB_TYPE_Q8_0) {
-                        // the two 16-byte pieces in an order in which eight lanes meet eight groups of banks
-                        const uint32_t first = (lane >> 2) & 1;
-                        const uint4 x = lds_u4(src + 16 * first), y = lds_u4(src + 16 * (first ^ 1));
-                        dequant16_q8(first ? y : x, d0, o[0], o[1]);
-                        dequant16_q8(first ? x : y, d0, o[2], o[3]);
-                    } else {
-                        dequant32_q4(lds_u4(src), d0, o);
-                    }
+                // rows past the matrix: zero codes (TMA) and zero scales
+                const float d0 = __half2float(cur[u]);
+                const uint32_t src = codes + s * c_bytes + gt * PB;
+                if (TYPE == GGB_TYPE_Q8_0) {
+                    // the two 16-byte pieces in an order in which eight lanes meet eight groups of banks
+                    const uint32_t first = (lane >> 2) & 1;
+                    const uint4 x = lds_u4(src + 16 * first), y = lds_u4(src + 16 * (first ^ 1));
+                    dequant16_q8(first ? y : x, d0, o[0], o[1]);
+                    dequant16_q8(first ? x : y, d0, o[2], o[3]);
+                } else {
+                    dequant32_q4(lds_u4(src), d0, o);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bars + C_FREE + 8 * s); // the codes are in registers
-                constexpr uint32_t kOwn = kTiles / 2;
-                const uint32_t b = grp + 2 * (use % kOwn);
-                if (use >= kOwn) mbar_wait_bounded(bars + B_FREE + 8 * b, (use / kOwn - 1) & 1, dead);
-                if (mine) {
-                    const uint32_t dst = smem0 + b * b_bytes + wr * 128;
+                if (before >= 0) mbar_wait_bounded(bars + FREE + 8 * before, bph, dead); // the group's buffer
 #pragma unroll
-                    for (int q = 0; q < 4; q++) sts_u4(dst + (((4 * whalf + q) ^ (wr & 7)) << 4), o[q]);
-                }
+                for (int q = 0; q < 4; q++) sts_u4(dst + (((4 * whalf + q) ^ (wr & 7)) << 4), o[q]);
                 fence_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bars + B_FULL + 8 * b);
-                use++;
-                s += 2;
+                if (lane == 0) {
+                    if (PAIR) mbar_arrive_cluster(full + 8 * as);
+                    else mbar_arrive(full + 8 * as);
+                }
+                before = as, bph = aph;
+                as += G;
+                if (as >= A.stages) as -= A.stages, aph ^= 1u;
+                s += G;
                 if (s >= A.code_stages) s -= A.code_stages, ph ^= 1u;
             }
         }
@@ -304,15 +305,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         // ================= A rows wait for the MMAs of their stage, codes, requested further ahead, for the warps that read them
         if (lane == 0) {
             const bool is_a = warp == kTmaWarp;
-            const int n = is_a ? A.stages : A.code_stages, full = is_a ? A_FULL : C_FULL, fre = is_a ? A_FREE : C_FREE;
+            const int n = is_a ? A.stages : A.code_stages, fre = is_a ? FREE : C_FREE;
             int s = 0;
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
                 if (!mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead)) break;
-                const uint32_t bar = bars + full + 8 * s;
-                mbar_expect_tx(bar, is_a ? A.a_tx : c_bytes);
-                if (is_a) tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, bar);
-                else tma_load_2d(codes + s * c_bytes, &maps.w[si], kb * 2 * PB, w_row0, bar);
+                if (is_a) {
+                    if (rank == 0) mbar_expect_tx(bars + FULL + 8 * s, CTAS * A.a_tx);
+                    if (PAIR) tma_load_2d_pair(ring + s * a_bytes, &maps.a, kb * BK, m0, full + 8 * s);
+                    else tma_load_2d(ring + s * a_bytes, &maps.a, kb * BK, m0, full + 8 * s);
+                } else {
+                    const uint32_t bar = bars + C_FULL + 8 * s;
+                    mbar_expect_tx(bar, c_bytes);
+                    tma_load_2d(codes + s * c_bytes, &maps.w[si], kb * 2 * PB, w_row0, bar);
+                }
                 if (++s == n) s = 0, ph ^= 1u;
             }
             if (A.geglu && is_a) { // the MMAs have read the ring: the gelu table takes its place
@@ -325,44 +331,32 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         }
         __syncwarp();
     } else if (rank == 0) {
-        // ================= MMA issuer
+        // ================= MMA issuer: one wait, asked for a K block ahead, and one commit a K block
         const uint32_t idesc = umma_idesc(128 * CTAS, A.BN);
-        int s = 0, chunk = 0, left = A.chunk_kb;
-        uint32_t ph = 0, it = 0;
-        for (int kb = kb0; kb < kb1; kb++, it++) {
-            const uint32_t b = it & (kTiles - 1), first = left == A.chunk_kb ? 0u : 1u;
-            mbar_wait_bounded(bars + A_FULL + 8 * s, ph, dead);
-            mbar_wait_bounded(bars + B_FULL + 8 * b, (it / kTiles) & 1, dead);
-            if (PAIR) mbar_wait_bounded(bars + PEER_FULL + 8 * b, (it / kTiles) & 1, dead);
+        int s = 0, chunk = 0, left = A.chunk_kb, grp = 0;
+        uint32_t ph = 0;
+        bool ready = false;
+        for (int kb = kb0; kb < kb1; kb++) {
+            const uint32_t first = left == A.chunk_kb ? 0u : 1u;
+            if (!ready) mbar_wait_bounded(bars + FULL + 8 * s, ph, dead);
             tc_fence_after();
-            const uint32_t a_lo = umma_desc_lo(ring + s * a_bytes, 16), b_lo = umma_desc_lo(smem0 + b * b_bytes, 16);
+            const bool wrap = s + 1 == A.stages;
+            ready = mbar_peek(bars + FULL + 8 * (wrap ? 0 : s + 1), wrap ? ph ^ 1u : ph); // of a block past the last: not done
+            const uint32_t a_lo = umma_desc_lo(ring + s * a_bytes, 16), b_lo = umma_desc_lo(smem0 + grp * b_bytes, 16);
             for (int mt = 0; mt < A.MT; mt++) {
                 const uint32_t d = tmem + (mt * A.chunks + chunk) * A.BN;
-#pragma unroll
-                for (int k = 0; k < BK / 16; k++) {
-                    if (PAIR) umma_ss_pair(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, b_lo + 2 * k, idesc, k > 0 ? 1u : first);
-                    else umma_ss(d, a_lo + mt * (128 * 128 >> 4) + 2 * k, b_lo + 2 * k, idesc, k > 0 ? 1u : first);
-                }
+                if (PAIR) umma_ss_pair_k4(d, a_lo + mt * (128 * 128 >> 4), b_lo, idesc, first);
+                else umma_ss_k4(d, a_lo + mt * (128 * 128 >> 4), b_lo, idesc, first);
             }
-            if (PAIR) umma_arrive_pair(bars + A_FREE + 8 * s), umma_arrive_pair(bars + B_FREE + 8 * b);
-            else umma_arrive(bars + A_FREE + 8 * s), umma_arrive(bars + B_FREE + 8 * b);
+            if (PAIR) umma_arrive_pair(bars + FREE + 8 * s);
+            else umma_arrive(bars + FREE + 8 * s);
             if (--left == 0) chunk++, left = A.chunk_kb;
-            if (++s == A.stages) s = 0, ph ^= 1u;
+            if (++grp == A.groups) grp = 0;
+            s = wrap ? 0 : s + 1;
+            ph ^= wrap ? 1u : 0u;
         }
         if (PAIR) umma_arrive_pair(bars + DONE);
         else umma_arrive(bars + DONE);
-    } else {
-        // ================= the second CTA's word that its A rows and weights of a K block stand
-        const uint32_t peer = cluster_addr(bars + PEER_FULL, 0);
-        int s = 0;
-        uint32_t ph = 0, it = 0;
-        for (int kb = kb0; kb < kb1; kb++, it++) {
-            mbar_wait_bounded(bars + A_FULL + 8 * s, ph, dead);
-            mbar_wait_bounded(bars + B_FULL + 8 * (it & (kTiles - 1)), (it / kTiles) & 1, dead);
-            if (lane == 0) mbar_arrive_cluster(peer + 8 * (it & (kTiles - 1)));
-            if (++s == A.stages) s = 0, ph ^= 1u;
-        }
-        __syncwarp();
     }
     __syncthreads();
     if (warp == kMmaWarp) settle(dead);
@@ -876,39 +870,48 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     const int kblocks = (int)(K / BK), sms = ggb_sm_count(), pb = ggb_payload_bytes(type);
     int pieces = ggb_gemm_pieces(T, N, K);
     if (pieces > 1 && (!workspace || workspace_bytes < (size_t)pieces * T * N * 4)) pieces = 1;
-    // a prompt of up to 256 rows fits one CTA's tile: 256000 x 2048, Q4_0, 129 rows: @S129@ us (pairs of CTAs: 408)
-    const bool pair = geglu || T > 256;
     GGB_CHECK_ARG(!geglu || (T > 128 && n == 2 && w[0]->rows == w[1]->rows && w[0]->rows % 256 == 0), "gemm_geglu: two matrices of as many rows and more than 128 tokens");
     if (geglu) pieces = 1, N = 2 * w[0]->rows;
     A.gelu = ggb_gelu_table_dev();
-    // the tile and the CTAs along K with the least estimated time (cycles): a stage takes what its MMAs, the bytes through shared memory (128 a
-    // cycle: written by TMA, read and written by the dequantisation, read for the MMAs) or the dequantisation take (2.7 a row: 32 weights are
-    // 170 instructions of one lane), and no less than 1000, the way of a K block through its hands, however narrow the tile
+    // The tile (of one CTA or of a pair), and the CTAs along K, with the least estimated time (cycles).  A K block takes what its MMAs (130 each by a
+    // pair of 256 columns, 100 of fewer, 80 by one CTA of 128, 40 of 64, and 100 for the wait and the commit), the bytes through shared memory
+    // (written by TMA, read and written by the dequantisation, read for the MMAs), the bytes from L2 or the dequantisation take (2.7 a row: 32
+    // weights are 170 instructions of one lane), and no less than a group's way with it, 2000, over the groups.  The constants choose the
+    // fastest of all tiles for 28 shapes from 16 x 2048 x 2048 to 512 x 65536 x 2048 and 2048 x 16384, all of which were timed.
+    auto stages_of = [&](bool pr, int MT, int br, int *codes) { // of A rows (a K block's also tell of the group's buffer: no fewer than groups), of codes
+        const int cs = br == 32 ? kMaxCodeStages : MT == 1 ? 12 : pr ? 4 : 8;
+        if (codes) *codes = cs;
+        return std::min<int>(kMaxStages, (int)((kRing - kTiles - cs * br * 2 * pb) / (MT * 16384)));
+    };
     double best = -1.0;
     int splits = 1;
-    for (int MT = 1; MT <= (T > (pair ? 256 : 128) ? 2 : 1); MT++) // the smaller of two that cost the same: 64 columns at 512 rows take longer
-        for (int bn = pair ? 256 : 128; bn >= (geglu ? 256 : 64); bn /= 2)
-            for (int sp = 1; sp <= pieces; sp *= 2) {
-                const int chunks = pieces / sp, chunk_kb = (kblocks + pieces - 1) / pieces, br = pair ? bn / 2 : bn, rows = MT * (pair ? 256 : 128);
-                if (MT * chunks * bn > 512) continue;
-                const int64_t tiles = (N + bn - 1) / bn * ((T + rows - 1) / rows) * sp, slots = pair ? sms / 2 : sms;
-                const double mma = MT * std::max(bn, 96) * 2.0, smem = (MT * 16384.0 + br * (4.0 * pb + 128.0) + MT * 4 * (4096.0 + br * 32.0)) / 128.0;
-                const double stage = std::max(std::max(mma, smem), std::max(br * 2.7, 1000.0));
-                const double store = MT * 128.0 * bn / (geglu ? 24.0 : 12.0) * (sp > 1 ? chunks : 1);
-                double cost = (double)((tiles + slots - 1) / slots) * (chunks * chunk_kb * stage + store + 3000.0);
-                if (sp > 1) cost += 6000.0 + (double)pieces * T * N * 8.0 / (32.0 * sms);
-                if (best < 0.0 || cost < best) {
-                    best = cost;
-                    splits = sp;
-                    A.MT = MT, A.BN = bn, A.chunks = chunks, A.chunk_kb = chunk_kb;
+    bool pair = false;
+    for (int pr = geglu ? 1 : 0; pr <= (geglu || T > 256 ? 1 : 0); pr++)
+        for (int MT = 1; MT <= (T > (pr ? 256 : 128) ? 2 : 1); MT++)
+            for (int bn = pr ? 256 : 128; bn >= (geglu ? 256 : 64); bn /= 2)
+                for (int sp = 1; sp <= pieces; sp *= 2) {
+                    const int chunks = pieces / sp, chunk_kb = (kblocks + pieces - 1) / pieces, br = pr ? bn / 2 : bn, rows = MT * (pr ? 256 : 128);
+                    if (MT * chunks * bn > 512 || stages_of(pr, MT, br, nullptr) < 256 / br) continue;
+                    const int64_t tiles = (N + bn - 1) / bn * ((T + rows - 1) / rows) * sp, slots = pr ? sms / 2 : sms, busy = std::min(tiles, slots) * (pr ? 2 : 1);
+                    const double mma = MT * 4.0 * (pr ? (bn == 256 ? 130.0 : 100.0) : (bn == 128 ? 80.0 : 41.0)) + 100.0;
+                    const double smem = (MT * 16384.0 + br * (4.0 * pb + 128.0) + MT * 4 * (4096.0 + br * 32.0)) / 190.0;
+                    const double l2 = (MT * 16384.0 + br * 2.0 * pb) / std::min(90.0, 7450.0 / busy);
+                    const double stage = std::max(std::max(std::max(mma, smem), l2), std::max(br * 2.7, 2030.0 * br / 256.0));
+                    const double store = MT * 128.0 * bn / (geglu ? 20.0 : 10.0) * (sp > 1 ? chunks : 1);
+                    double cost = (double)((tiles + slots - 1) / slots) * (chunks * chunk_kb * stage + store + (pr ? 12000.0 : 6150.0));
+                    if (sp > 1) cost += 3240.0 + (double)pieces * T * N * 8.0 / (60.0 * sms);
+                    if (best < 0.0 || cost < best) {
+                        best = cost;
+                        splits = sp, pair = pr;
+                        A.MT = MT, A.BN = bn, A.chunks = chunks, A.chunk_kb = chunk_kb;
+                    }
                 }
-            }
     const int br = pair ? A.BN / 2 : A.BN;
+    A.groups = 256 / br;
     A.N = (int)N, A.nb = (int)w[0]->nb, A.kblocks = kblocks, A.T = (int)T;
     // Codes come from memory, A rows from L2: what is in flight of the codes bounds a product of few rows (256000 x 2048, Q4_0, 33 to 128 rows:
     // 4 stages 276 to 289 us, 12 stages 263 to 275), the MMAs and shared memory one of 512 rows a tile.
-    A.code_stages = A.MT == 1 ? kMaxCodeStages : pair ? 4 : 8;
-    A.stages = std::min<int>(kMaxStages, (int)((kRing - kTiles * br * 128 - A.code_stages * br * 2 * pb) / (A.MT * 16384)));
+    A.stages = stages_of(pair, A.MT, br, &A.code_stages);
     const int a_rows = !pair && T <= A.MT * 128 ? (int)(T + 7) / 8 * 8 : A.MT * 128;
     A.a_tx = (uint32_t)a_rows * 128;
     A.ws = splits > 1 ? (float *)workspace : nullptr;

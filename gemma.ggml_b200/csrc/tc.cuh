@@ -27,6 +27,12 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// The same without waiting: asked ahead, so that a warp does not stand for the hundred cycles and more that an answer takes
+__device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Waits for a phase.  Every wait ends: after kWaitTries tries (seconds) the CTA's `dead` word is set, which ends all of its other
 // waits at once; the kernel then requests no more copies, runs through with whatever is in its buffers, gives what it has requested time to
 // arrive (settle), gives its tensor memory back and reports the failure.
@@ -73,6 +79,15 @@ __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t
                  "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi)
                  : "memory");
 }
+// The four steps of a block of 64 along K (K-major operands: 32 bytes further each) under one election
+#define GGB_K4(G) "{\n.reg .pred p, q, e;\n.reg .b64 a, b;\n" GGB_ELECT "setp.ne.b32 p, %4, 0;\nsetp.eq.b32 q, %4, %4;\nmov.b64 a, {%1, %5};\nmov.b64 b, {%2, %5};\n" \
+    "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a, b, %3, p;\nadd.s64 a, a, 2;\nadd.s64 b, b, 2;\n" \
+    "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a, b, %3, q;\nadd.s64 a, a, 2;\nadd.s64 b, b, 2;\n" \
+    "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a, b, %3, q;\nadd.s64 a, a, 2;\nadd.s64 b, b, 2;\n" \
+    "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], a, b, %3, q;\n}\n"
+__device__ __forceinline__ void umma_ss_k4(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(GGB_K4("1") ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi) : "memory");
+}
 // A from tensor memory: row = lane, a 32-bit column holds two neighbours of K
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n.reg .pred p, e;\n.reg .b64 b;\n" GGB_ELECT "setp.ne.b32 p, %4, 0;\nmov.b64 b, {%2, %5};\n"
@@ -92,6 +107,10 @@ __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint32_t a_lo, uin
                  "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi)
                  : "memory");
 }
+__device__ __forceinline__ void umma_ss_pair_k4(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(GGB_K4("2") ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHi) : "memory");
+}
+#undef GGB_K4
 __device__ __forceinline__ void umma_arrive_pair(uint32_t bar) {
     asm volatile("{\n.reg .pred e;\n" GGB_ELECT "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n" ::"r"(bar),
                  "h"((uint16_t)3)
