@@ -108,6 +108,9 @@ __device__ __forceinline__ uint4 ldg_stream_u4(const void *p) {
 // not written while the kernel runs, none is reached by another way) does not hold until here, and a compiler that believes it may read
 // through the read-only cache or ahead of this statement.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Behind step_wait: once every block has said so, blocks of the next kernel may take what room there is and run up to their own step_wait.  What
+// they read ahead of it was written before the kernels that came before this one ended.
+__device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float half_bits_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 __device__ __forceinline__ uint16_t float_to_half_bits(float f) { return __half_as_ushort(__float2half_rn(f)); }

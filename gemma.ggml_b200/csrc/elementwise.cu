@@ -208,10 +208,10 @@ __global__ void rope_kv_store_kernel(float *__restrict__ q, const float *__restr
 }
 
 // the same for T tokens (prefill): token t = blockIdx.y, its position pos[t]; q / k / v are [T][H*d] / [T][Hkv*d]
-__global__ void rope_kv_store_batch_kernel(float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
-                                           const int32_t *__restrict__ pos_p, int H, int Hkv, int d, float q_scale,
-                                           const float *__restrict__ cosT, const float *__restrict__ sinT, int table_ctx,
-                                           __half *__restrict__ kcache, __half *__restrict__ vcache) {
+__global__ void rope_kv_store_batch_kernel(float *q, const float *k, const float *v, const int32_t *pos_p, int H, int Hkv, int d, float q_scale,
+                                           const float *cosT, const float *sinT, int table_ctx, __half *kcache, __half *vcache) {
+    step_wait();
+    step_next();
     const int half = d / 2;
     const int64_t t = blockIdx.y;
     int pos = pos_p[t];
@@ -457,9 +457,8 @@ int ggb_op_rope_kv_store_batch(float *q, const float *k, const float *v, const i
     GGB_CHECK_ARG(ggb_rope_cos_dev() && ggb_rope_n_dims() == d, "rope table not initialised for head_dim %d", d);
     const int total = (H + Hkv) * (d / 2) + Hkv * d;
     const dim3 grid((unsigned)((total + 255) / 256), (unsigned)T);
-    rope_kv_store_batch_kernel<<<grid, 256, 0, ggb_cuda_stream()>>>(q, k, v, pos, H, Hkv, d, q_scale, ggb_rope_cos_dev(),
-                                                                     ggb_rope_sin_dev(), ggb_rope_n_ctx(), (__half *)kcache,
-                                                                     (__half *)vcache);
+    GGB_CUDA(ggb_launch_step(rope_kv_store_batch_kernel, grid, dim3(256), 0, q, k, v, pos, H, Hkv, d, q_scale, ggb_rope_cos_dev(), ggb_rope_sin_dev(),
+                             ggb_rope_n_ctx(), (__half *)kcache, (__half *)vcache));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

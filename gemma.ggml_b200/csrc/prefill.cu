@@ -306,6 +306,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         if (lane == 0) {
             const bool is_a = warp == kTmaWarp;
             const int n = is_a ? A.stages : A.code_stages, fre = is_a ? FREE : C_FREE;
+            // A is what the kernel before wrote, and everything stored here waits for A; weights stand since a launch before that one at least
+            if (is_a) step_wait(), step_next();
             int s = 0;
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
@@ -371,6 +373,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
 
 // the pieces of a product that several CTAs summed along K, in order (+ residual)
 __global__ void splitk_reduce_kernel(const GemmArgs A, int pieces) {
+    step_wait();
+    step_next();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4, T = A.T, N = A.N; // N and the segments: multiples of 32
     if (i >= T * N) return;
     const int64_t t = i / N;
@@ -392,8 +396,10 @@ __global__ void splitk_reduce_kernel(const GemmArgs A, int pieces) {
 
 // rms_norm * w -> bf16 (the A operand of the next GEMM): same double-sum order as rms_norm_kernel (elementwise.cu)
 __global__ void __launch_bounds__(GGB_DEV_NORM_THREADS)
-rms_norm_bf16_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int64_t E, __nv_bfloat16 *__restrict__ y) {
+rms_norm_bf16_kernel(const float *x, const float *w, float eps, int64_t E, __nv_bfloat16 *y) {
     __shared__ double s_w[GGB_DEV_NORM_THREADS / 32];
+    step_wait();
+    step_next();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float *xr = x + (int64_t)blockIdx.x * E;
     double acc = 0.0;
@@ -431,6 +437,8 @@ __device__ __forceinline__ float pieces_sum(const float *ws, int64_t plane, int 
 __global__ void __launch_bounds__(GGB_DEV_NORM_THREADS) splitk_norm_kernel(const GemmArgs A, int pieces, const float *w, float eps, __nv_bfloat16 *y) {
     __shared__ double s_w[GGB_DEV_NORM_THREADS / 32];
     extern __shared__ float s_row[];
+    step_wait();
+    step_next();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, E = A.N;
     const int64_t t = blockIdx.x, plane = (int64_t)A.T * E;
     const GemmSeg &sg = A.seg[0];
@@ -463,6 +471,8 @@ struct rope_args {
     __half *kcache, *vcache;
 };
 __global__ void splitk_rope_kernel(const GemmArgs A, int pieces, const rope_args r) {
+    step_wait();
+    step_next();
     const int half = r.d / 2, nq = r.H * half, nk = r.Hkv * half, nv = r.Hkv * r.d, idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t t = blockIdx.y, plane = (int64_t)A.T * A.N;
     int pos = r.pos[t];
@@ -821,7 +831,7 @@ int ggb_op_cvt_f32_bf16(const float *x, int64_t n, void *y_bf16) {
 int ggb_op_rms_norm_bf16(const float *x, const float *w, float eps, int64_t E, int64_t T, void *y_bf16) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(x && w && y_bf16 && E > 0 && T > 0, "bad rms_norm_bf16 args");
-    rms_norm_bf16_kernel<<<(unsigned)T, GGB_DEV_NORM_THREADS, 0, ggb_cuda_stream()>>>(x, w, eps, E, (__nv_bfloat16 *)y_bf16);
+    GGB_CUDA(ggb_launch_step(rms_norm_bf16_kernel, dim3((unsigned)T), dim3(GGB_DEV_NORM_THREADS), 0, x, w, eps, E, (__nv_bfloat16 *)y_bf16));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -932,10 +942,12 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = kGemmSmem;
     cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-    cfg.attrs = at, cfg.numAttrs = pair ? 1 : 0;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+    cfg.attrs = at, cfg.numAttrs = pair ? 2 : 1;
     GGB_CUDA(cudaLaunchKernelEx(&cfg, kfn, maps, A));
     GGB_LAUNCH_CHECK();
     if (splits > 1) {
@@ -945,13 +957,13 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
         if (tail && tail->rope) {
             const rope_args &r = *tail->rope;
             const int total = (r.H + r.Hkv) * (r.d / 2) + r.Hkv * r.d;
-            splitk_rope_kernel<<<dim3((unsigned)((total + 255) / 256), (unsigned)T), 256, 0, ggb_cuda_stream()>>>(A, planes, r);
+            GGB_CUDA(ggb_launch_step(splitk_rope_kernel, dim3((unsigned)((total + 255) / 256), (unsigned)T), dim3(256), 0, A, planes, r));
         } else if (tail) {
             const size_t row = (size_t)N * 4;
             if ((rc = ggb_allow_smem(splitk_norm_kernel, row))) return rc;
-            splitk_norm_kernel<<<(unsigned)T, GGB_DEV_NORM_THREADS, row, ggb_cuda_stream()>>>(A, planes, tail->norm_w, tail->eps, tail->y);
+            GGB_CUDA(ggb_launch_step(splitk_norm_kernel, dim3((unsigned)T), dim3(GGB_DEV_NORM_THREADS), row, A, planes, tail->norm_w, tail->eps, tail->y));
         } else {
-            splitk_reduce_kernel<<<(unsigned)((cnt / 4 + 255) / 256), 256, 0, ggb_cuda_stream()>>>(A, planes);
+            GGB_CUDA(ggb_launch_step(splitk_reduce_kernel, dim3((unsigned)((cnt / 4 + 255) / 256)), dim3(256), 0, A, planes));
         }
         if (tail) tail->done = true;
         GGB_LAUNCH_CHECK();

@@ -119,6 +119,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
+    step_wait();
+    step_next();
     if (warp < 8) { // queries, rounded to fp16: 8 numbers a step, neighbouring lanes along a row, eight steps in flight
         const int pieces = D / 8, n = kRows * pieces;
         for (int i0 = tid; i0 < n; i0 += 8 * 256) {
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
                 x[u][0] = x[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (i < n && r < n_rows) {
                     const float4 *src = reinterpret_cast<const float4 *>(a.q + ((int64_t)(t0 + tq) * a.H + g * hpg + (r - tq * hpg)) * D + 8 * pc);
-                    x[u][0] = __ldg(src), x[u][1] = __ldg(src + 1);
+                    x[u][0] = src[0], x[u][1] = src[1];
                 }
             }
 #pragma unroll
@@ -329,7 +331,7 @@ int ggb_attn_prefill_tiles(const float *q, const void *kcache, const void *vcach
     rc = ggb_allow_smem(attn_prefill_tile_kernel, smem);
     if (rc) return rc;
     const int TQ = kRows / (H / Hkv);
-    attn_prefill_tile_kernel<<<dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv), kThreads, smem, ggb_cuda_stream()>>>(maps, a);
+    GGB_CUDA(ggb_launch_step(attn_prefill_tile_kernel, dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv), dim3(kThreads), smem, maps, a));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
