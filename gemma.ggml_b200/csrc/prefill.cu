@@ -24,8 +24,8 @@
 // hides, 3 us up to the first MMA and 7 us from the last one to the end, at clocks that fall under the power limit.  A K block has one barrier
 // that its A rows and all its dequantising warps arrive on, of both CTAs, and one commit: a wait or commit costs the issuing warp 100 to 200
 // cycles whether it has to wait or not (three waits and two commits a block: 900 cycles a block of any tile).  Small products: that start
-// and end.  512 tokens, Q8_0: gate | up with gelu 72 -> 68 us (1010 TFLOP/s; 115 us in two launches before), 2048 x 16384 in 8 pieces 45 -> 43 us
-// with its sums, 2048 x 2048 20 -> 17 us, q | k | v 22.5 -> 18 us.
+// and end.  512 tokens, Q8_0: gate | up with gelu 65 us (1060 TFLOP/s; 72 with three waits and two commits a K block; 115 in two launches before),
+// 2048 x 16384 in 8 pieces 45 -> 40 to 42 us with its sums, 2048 x 2048 20 -> 16 us, q | k | v 22.5 -> 17 us.
 //
 // Numerics: weights q*d are exact in fp32 (8 x 11 bits) and rounded once to bf16; activations are rounded
 // to bf16 instead of being re-quantised to Q8_0 per 32 (the reference's INIT stage), so prefill agrees with
@@ -81,39 +81,49 @@ struct GemmMaps {
     CUtensorMap a, w[kMaxSegs];
 };
 
-// int8 / int4 code -> fp32 without the conversion pipe: the (biased) code is dropped into the mantissa of
-// 2^23 with one PRMT, the bias is removed with one exact FADD, and one FMUL applies the block scale
-// (code * d is exact in fp32: 8 x 11 significant bits); the product is then rounded once to bf16.
-template <int SEL> __device__ __forceinline__ float code_to_f32(uint32_t biased_word, float bias, float d) {
-    return __fmul_rn(__fadd_rn(__uint_as_float(__byte_perm(biased_word, 0x4B000000u, SEL)), bias), d);
+// int8 / int4 codes -> bf16 weights without the conversion pipe.  A byte permute puts the biased code into the mantissa of 2^15, and one
+// multiply-add of two numbers takes the bias out and applies the block scale: (2^15 + bias + code) d - (2^15 + bias) d, exact, since d has 11
+// significant bits and 2^15 + 128 has 9 of them, 2^15 + 8 has 13; the product, exact in fp32 (8 x 11 bits), is rounded once to bf16.  A scale
+// that is infinite is applied behind the bias.  Bound by the permutes and roundings, which issue every other cycle: 32 weights of a lane are 110
+// instructions (170 with an addition and a multiplication each).
+struct block_scale {
+    f32x2 d, c;
+    float last; // an infinite scale
+    __device__ __forceinline__ block_scale(float scale, float bias) {
+        const bool odd = fabsf(scale) > 65504.f;
+        last = odd ? scale : 1.f;
+        const float f = odd ? 1.f : scale;
+        d = pack2(f, f), c = pack2(__fmul_rn(-bias, f), __fmul_rn(-bias, f));
+    }
+};
+__device__ __forceinline__ void codes_to_bf16x16(const uint32_t (&w)[4], const block_scale &b, uint32_t (&o)[8]) {
+    float2 v[8];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        v[2 * i] = unpack2(fma2(pack2(__uint_as_float(__byte_perm(w[i], 0x47000000u, 0x7404)), __uint_as_float(__byte_perm(w[i], 0x47000000u, 0x7414))), b.d, b.c));
+        v[2 * i + 1] = unpack2(fma2(pack2(__uint_as_float(__byte_perm(w[i], 0x47000000u, 0x7424)), __uint_as_float(__byte_perm(w[i], 0x47000000u, 0x7434))), b.d, b.c));
+    }
+    if (b.last != 1.f)
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i].x *= b.last, v[i].y *= b.last;
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i] = pack_bf16x2(v[i].x, v[i].y);
 }
-__device__ __forceinline__ void word_to_bf16x4(uint32_t biased_word, float bias, float d, uint32_t &o0, uint32_t &o1) {
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(code_to_f32<0x7540>(biased_word, bias, d), code_to_f32<0x7541>(biased_word, bias, d));
-    __nv_bfloat162 p1 = __floats2bfloat162_rn(code_to_f32<0x7542>(biased_word, bias, d), code_to_f32<0x7543>(biased_word, bias, d));
-    o0 = *reinterpret_cast<uint32_t *>(&p0);
-    o1 = *reinterpret_cast<uint32_t *>(&p1);
-}
-// 16 bf16 of dequantised weights (two 16-byte chunks of the swizzled row) from 16 int8 codes
-__device__ __forceinline__ void dequant16_q8(const uint4 w, float d, uint4 &lo, uint4 &hi) {
-    const float bias = -8388736.0f; // -(2^23 + 128): code ^ 0x80 = code + 128
+// 16 bf16 of dequantised weights (two 16-byte chunks of the swizzled row) from 16 int8 codes; b of 32896
+__device__ __forceinline__ void dequant16_q8(const uint4 w, const block_scale &b, uint4 &lo, uint4 &hi) {
+    const uint32_t u[4] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u, w.z ^ 0x80808080u, w.w ^ 0x80808080u}; // code + 128
     uint32_t out[8];
-    word_to_bf16x4(w.x ^ 0x80808080u, bias, d, out[0], out[1]);
-    word_to_bf16x4(w.y ^ 0x80808080u, bias, d, out[2], out[3]);
-    word_to_bf16x4(w.z ^ 0x80808080u, bias, d, out[4], out[5]);
-    word_to_bf16x4(w.w ^ 0x80808080u, bias, d, out[6], out[7]);
+    codes_to_bf16x16(u, b, out);
     lo = make_uint4(out[0], out[1], out[2], out[3]);
     hi = make_uint4(out[4], out[5], out[6], out[7]);
 }
-// one Q4_0 block (16 payload bytes -> 32 weights): elements 0..15 are the low nibbles, 16..31 the high ones
-__device__ __forceinline__ void dequant32_q4(const uint4 w, float d, uint4 (&o)[4]) {
-    const float bias = -8388616.0f; // -(2^23 + 8): value = nibble - 8
-    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+// one Q4_0 block (16 payload bytes -> 32 weights, nibble - 8): elements 0..15 are the low nibbles, 16..31 the high ones; b of 32776
+__device__ __forceinline__ void dequant32_q4(const uint4 w, const block_scale &b, uint4 (&o)[4]) {
+    const uint32_t l[4] = {w.x & 0x0F0F0F0Fu, w.y & 0x0F0F0F0Fu, w.z & 0x0F0F0F0Fu, w.w & 0x0F0F0F0Fu};
+    const uint32_t h[4] = {(w.x >> 4) & 0x0F0F0F0Fu, (w.y >> 4) & 0x0F0F0F0Fu, (w.z >> 4) & 0x0F0F0F0Fu, (w.w >> 4) & 0x0F0F0F0Fu};
     uint32_t lo[8], hi[8];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        word_to_bf16x4(ws[i] & 0x0F0F0F0Fu, bias, d, lo[2 * i], lo[2 * i + 1]);
-        word_to_bf16x4((ws[i] >> 4) & 0x0F0F0F0Fu, bias, d, hi[2 * i], hi[2 * i + 1]);
-    }
+    codes_to_bf16x16(l, b, lo);
+    codes_to_bf16x16(h, b, hi);
     o[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     o[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
     o[2] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -207,7 +217,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                 mbar_wait_warp(bars + C_FULL + 8 * s, ph, dead);
                 uint4 o[4];
                 // rows past the matrix: zero codes (TMA) and zero scales
-                const float d0 = __half2float(cur[u]);
+                const block_scale d0(__half2float(cur[u]), TYPE == GGB_TYPE_Q8_0 ? 32896.f : 32776.f);
                 const uint32_t src = codes + s * c_bytes + gt * PB;
                 if (TYPE == GGB_TYPE_Q8_0) {
                     // the two 16-byte pieces in an order in which eight lanes meet eight groups of banks
@@ -367,6 +377,254 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
         tc_fence_after();
         if (PAIR) tmem_free512_pair(tmem);
         else tmem_free512(tmem);
+        if (lane == 0 && *dead) *A.wait_error = 1;
+    }
+}
+
+// Products that are not cut along K (the logits; gate | up of up to 256 tokens): two CTAs a tile of 256 x 256, persistent.  A tile takes half of
+// tensor memory, so that four warps store one tile (or take gelu(gate) * up) while the tensor cores are on the next; sixteen others dequantise, each
+// CTA its 128 of the tile's weight rows, into the stage of the ring whose other half TMA fills with A rows.
+//
+// What bounds it: the way of a K block through the ring (A rows from L2, codes, dequantisation, MMAs: 800 cycles a block where the MMAs take 560)
+// at clocks that fall under the power limit.  Q8_0: 512 x 65536 x 2048 144 -> 123 us (1117 TFLOP/s; tiles of 512 x 256 that end before the next
+// begins), gate | up of 256 tokens, 2 x 16384 x 2048, 52 -> 40 us.
+constexpr int kStreamThreads = 32 * 24, kStreamStages = 5, kStreamCodes = 6, kStreamEpi = 4, kStreamDeq = 8, kStreamGroups = 4; // warps 4..7 store, 8..23 dequantise
+enum { Q_FULL = 0, Q_EMPTY = 40, Q_C_FULL = 80, Q_C_FREE = 128, Q_ACC_FULL = 176, Q_ACC_FREE = 192, Q_SLOT = 208, Q_DEAD = 212 };
+
+// gelu of an fp16 number, rounded to fp16: the numbers of the table that ggb_op_geglu_bf16 reads, computed as the table was (equal for every fp16
+// number, test_gelu_of_every_fp16_number: a lookup would take shared memory's bandwidth)
+__device__ __forceinline__ float gelu_f16(float g) {
+    const float x = __half2float(__float2half_rn(g));
+    const float inner = __fmul_rn(__fmul_rn(0.79788456080286535587989211986876f, x), __fadd_rn(1.0f, __fmul_rn(__fmul_rn(0.044715f, x), x)));
+    return __half2float(__float2half_rn(__fmul_rn(__fmul_rn(0.5f, x), __fadd_rn(1.0f, tanhf(inner)))));
+}
+
+template <int TYPE, bool GEGLU>
+__global__ void __launch_bounds__(kStreamThreads, 1) gemm_quant_stream_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs A) {
+    extern __shared__ uint8_t gemm_smem_raw[];
+    constexpr int PB = TYPE == GGB_TYPE_Q8_0 ? 32 : 16; // payload bytes of a block of 32 weights
+    constexpr uint32_t kHalf = 128 * 128, kStage = 2 * kHalf, kCodes = 128 * 2 * PB;
+    const uint32_t raw0 = smem_u32(gemm_smem_raw), smem0 = (raw0 + 1023u) & ~1023u, bars = smem0 + kRing;
+    const uint32_t codes = smem0 + kStreamStages * kStage, turn = codes + kStreamCodes * 8192;
+    uint8_t *ctl = gemm_smem_raw + (bars - raw0);
+    volatile int *dead = reinterpret_cast<volatile int *>(ctl + Q_DEAD);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int rank = (int)cluster_rank();
+    const uint32_t bars0 = cluster_addr(bars, 0);
+    if (tid == 0) {
+        for (int s = 0; s < kStreamStages; s++) {
+            mbar_init(bars + Q_FULL + 8 * s, 1 + 2 * 4); // the bytes of A and the warps that dequantise, of both CTAs
+            mbar_init(bars + Q_EMPTY + 8 * s, 1);
+        }
+        for (int s = 0; s < kStreamCodes; s++) {
+            mbar_init(bars + Q_C_FULL + 8 * s, 1);
+            mbar_init(bars + Q_C_FREE + 8 * s, 4);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(bars + Q_ACC_FULL + 8 * s, 1);
+            mbar_init(bars + Q_ACC_FREE + 8 * s, 8);
+        }
+        *dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 3) tmem_alloc512_pair(bars + Q_SLOT);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + Q_SLOT), 0);
+
+    const int pairs = gridDim.x / 2, me = blockIdx.x / 2, m_tiles = (A.T + 255) / 256, total = m_tiles * ((A.N + 255) / 256), kblocks = A.kblocks;
+    struct place {
+        int m0, si, sn0, w_row0; // first row of A of the pair, matrix, first output column and first weight row of this CTA inside it
+    };
+    auto locate = [&](int t) { // row tiles first: those that share a piece of W run together
+        place r;
+        r.m0 = t % m_tiles * 256;
+        const int n0 = t / m_tiles * 256;
+        r.si = 0;
+        if (GEGLU) r.si = rank;
+        else if (A.n_seg > 1 && n0 >= A.seg[1].n_begin) r.si = (A.n_seg > 2 && n0 >= A.seg[2].n_begin) ? 2 : 1;
+        r.sn0 = GEGLU ? n0 / 2 : n0 - A.seg[r.si].n_begin;
+        r.w_row0 = GEGLU ? r.sn0 : r.sn0 + rank * 128;
+        return r;
+    };
+
+    if (warp == 0 || warp == 2) {
+        if (lane == 0) { // warp 0: A rows, counted on the first CTA's barrier; warp 2: codes
+            const bool is_a = warp == 0;
+            const int n = is_a ? kStreamStages : kStreamCodes, fre = is_a ? Q_EMPTY : Q_C_FREE;
+            int s = 0;
+            uint32_t ph = 0;
+            if (is_a) step_wait(), step_next(); // as gemm_quant_kernel
+            for (int t = me; t < total; t += pairs) {
+                const place at = locate(t);
+                for (int kb = 0; kb < kblocks; kb++) {
+                    if (!mbar_wait_bounded(bars + fre + 8 * s, ph ^ 1u, dead)) break;
+                    if (is_a) {
+                        if (rank == 0) mbar_expect_tx(bars + Q_FULL + 8 * s, 2 * kHalf);
+                        tma_load_2d_pair(smem0 + s * kStage, &maps.a, kb * BK, at.m0 + rank * 128, bars0 + Q_FULL + 8 * s);
+                    } else {
+                        mbar_expect_tx(bars + Q_C_FULL + 8 * s, kCodes);
+                        tma_load_2d(codes + s * kCodes, &maps.w[at.si], kb * 2 * PB, at.w_row0, bars + Q_C_FULL + 8 * s);
+                    }
+                    if (++s == n) s = 0, ph ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1 && rank == 0) {
+        const uint32_t idesc = umma_idesc(256, 256);
+        int s = 0, it = 0;
+        uint32_t ph = 0;
+        bool ready = false; // asked for a K block ahead
+        for (int t = me; t < total; t += pairs, it++) {
+            const int buf = it & 1;
+            mbar_wait_bounded(bars + Q_ACC_FREE + 8 * buf, ((it >> 1) & 1) ^ 1, dead);
+            for (int kb = 0; kb < kblocks; kb++) {
+                if (!ready) mbar_wait_bounded(bars + Q_FULL + 8 * s, ph, dead);
+                tc_fence_after();
+                const uint32_t at = smem0 + s * kStage;
+                if (++s == kStreamStages) s = 0, ph ^= 1u;
+                ready = mbar_peek(bars + Q_FULL + 8 * s, ph);
+                umma_ss_pair_k4(tmem + buf * 256, umma_desc_lo(at, 16), umma_desc_lo(at + kHalf, 16), idesc, kb > 0);
+                umma_arrive_pair(bars + Q_EMPTY + (at - smem0) / kStage * 8);
+            }
+            umma_arrive_pair(bars + Q_ACC_FULL + 8 * buf);
+        }
+    } else if (warp >= kStreamDeq) {
+        // Four groups of four warps take the K blocks of all tiles in turn: a block is 1400 to 2000 cycles in the hands of one, mostly latency, and
+        // the MMAs want one every 560.  A thread owns a row of the CTA's 128: 64 weights, two scales.  It takes the four pieces of 16 codes in
+        // the order q ^ turn, in which eight neighbouring rows meet eight groups of banks, where the codes lie (64 bytes a row) and where the
+        // weights go (the 128-byte swizzle): turn = w * (r >> 1) in the field of four elements, whose w and 1 + w both have inverses.
+        const int grp = (warp - kStreamDeq) >> 2, wr = tid & 127, r2 = (wr >> 2) & 1, r1 = (wr >> 1) & 1, turn_of = ((r2 ^ r1) << 1) | r2;
+        const float bias = TYPE == GGB_TYPE_Q8_0 ? 32896.f : 32776.f;
+        int ft = me, fkb = grp; // whose scales are asked for next: four of the group's blocks ahead
+        const __half *dp = nullptr;
+        auto row_of = [&]() { // rows past the matrix: zero codes (TMA), any scale
+            const place at = locate(ft);
+            dp = A.seg[at.si].d + (size_t)min(at.w_row0 + wr, A.seg[at.si].rows - 1) * A.nb;
+        };
+        auto ask = [&]() {
+            if (fkb >= kblocks || !dp) {
+                while (fkb >= kblocks) fkb -= kblocks, ft += pairs;
+                if (ft < total) row_of();
+            }
+            const __half2 d = ft < total ? __ldg(reinterpret_cast<const __half2 *>(dp + 2 * fkb)) : __float2half2_rn(0.f);
+            fkb += kStreamGroups;
+            return d;
+        };
+        __half2 sc[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) sc[u] = ask();
+        const int n_blocks = (total - me + pairs - 1) / pairs * kblocks;
+        int s = grp, cs = grp;
+        uint32_t ph = 0, cph = 0;
+        for (int b0 = grp; b0 < n_blocks; b0 += 4 * kStreamGroups) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (b0 + kStreamGroups * u >= n_blocks) break;
+                const float2 d = __half22float2(sc[u]);
+                sc[u] = ask();
+                const block_scale d0(d.x, bias), d1(d.y, bias);
+                mbar_wait_warp(bars + Q_C_FULL + 8 * cs, cph, dead);
+                const uint32_t src = codes + cs * kCodes + wr * 2 * PB, dst = smem0 + s * kStage + kHalf + wr * 128;
+                uint4 x[4];
+                if (TYPE == GGB_TYPE_Q8_0) {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) x[q] = lds_u4(src + 16 * (q ^ turn_of));
+                } else { // 32 bytes a row: the two pieces in an order in which eight rows meet eight groups of banks; low nibbles, then high ones
+                    x[0] = lds_u4(src + 16 * r2), x[1] = lds_u4(src + 16 * (r2 ^ 1));
+                }
+                mbar_wait_warp(bars + Q_EMPTY + 8 * s, ph ^ 1u, dead);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int p = q ^ turn_of;
+                    uint32_t c[4], o[8];
+                    block_scale b = d0;
+                    if (p >> 1) b = d1;
+                    if (TYPE == GGB_TYPE_Q8_0) {
+                        const uint4 w = x[q];
+                        c[0] = w.x ^ 0x80808080u, c[1] = w.y ^ 0x80808080u, c[2] = w.z ^ 0x80808080u, c[3] = w.w ^ 0x80808080u;
+                    } else {
+                        const uint4 w = (p >> 1) == r2 ? x[0] : x[1];
+                        const int sh = (p & 1) * 4;
+                        c[0] = (w.x >> sh) & 0x0F0F0F0Fu, c[1] = (w.y >> sh) & 0x0F0F0F0Fu, c[2] = (w.z >> sh) & 0x0F0F0F0Fu, c[3] = (w.w >> sh) & 0x0F0F0F0Fu;
+                    }
+                    codes_to_bf16x16(c, b, o);
+                    sts_u4(dst + (((2 * p) ^ (wr & 7)) << 4), make_uint4(o[0], o[1], o[2], o[3]));
+                    sts_u4(dst + (((2 * p + 1) ^ (wr & 7)) << 4), make_uint4(o[4], o[5], o[6], o[7]));
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(bars + Q_C_FREE + 8 * cs);
+                    mbar_arrive_cluster(bars0 + Q_FULL + 8 * s);
+                }
+                s += kStreamGroups;
+                if (s >= kStreamStages) s -= kStreamStages, ph ^= 1u;
+                cs += kStreamGroups;
+                if (cs >= kStreamCodes) cs -= kStreamCodes, cph ^= 1u;
+            }
+        }
+    } else if (warp >= kStreamEpi) {
+        const int lq = warp & 3, p = lane & 7;
+        const uint32_t my = turn + lq * 4096;
+        int it = 0;
+        for (int t = me; t < total; t += pairs, it++) {
+            const place at = locate(t);
+            const GemmSeg &sg = A.seg[at.si];
+            const int buf = it & 1, row0 = at.m0 + rank * 128 + lq * 32;
+            mbar_wait_bounded(bars + Q_ACC_FULL + 8 * buf, (it >> 1) & 1, dead);
+            tc_fence_after();
+            if (row0 < A.T)
+                for (int c0 = 0; c0 < (GEGLU ? 128 : 256) && at.sn0 + c0 < sg.rows; c0 += 32) {
+                    const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0;
+                    uint32_t v[32];
+                    tmem_load32(col, v);
+                    if (GEGLU) { // the other half of the tile's columns is up
+#pragma unroll
+                        for (int hf = 0; hf < 2; hf++) {
+                            uint32_t u[16];
+                            tmem_load16(col + 128 + 16 * hf, u);
+#pragma unroll
+                            for (int q = 0; q < 16; q++) v[16 * hf + q] = __float_as_uint(__fmul_rn(gelu_f16(__uint_as_float(v[16 * hf + q])), __uint_as_float(u[q])));
+                        }
+                    }
+                    // row = lane -> eight lanes a row: 16-byte piece p of row r at place p ^ (r & 7)
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 8; q++) sts_u4(my + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const int r = 4 * q + (lane >> 3), row = row0 + r;
+                        const uint4 w = lds_u4(my + r * 128 + ((p ^ (r & 7)) << 4));
+                        if (row >= A.T) continue; // rows of a matrix are a multiple of 32
+                        float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+                        const int n = at.sn0 + c0 + 4 * p;
+                        if (GEGLU) {
+                            *reinterpret_cast<uint2 *>(A.geglu + (size_t)row * sg.rows + n) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
+                            continue;
+                        }
+                        if (A.resid) {
+                            const float4 r4 = load4(A.resid + (size_t)row * sg.ldc + n, A.vec);
+                            o.x += r4.x, o.y += r4.y, o.z += r4.z, o.w += r4.w;
+                        }
+                        store4(sg.c + (size_t)row * sg.ldc + n, o, A.vec);
+                    }
+                }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(bars0 + Q_ACC_FREE + 8 * buf);
+        }
+    }
+    __syncthreads();
+    if (warp == 3) settle(dead);
+    cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
+    if (warp == 3) {
+        tc_fence_after();
+        tmem_free512_pair(tmem);
         if (lane == 0 && *dead) *A.wait_error = 1;
     }
 }
@@ -916,6 +1174,11 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
                         A.MT = MT, A.BN = bn, A.chunks = chunks, A.chunk_kb = chunk_kb;
                     }
                 }
+    // Persistent pairs with tiles of 256 x 256, which dequantise every weight once per 256 tokens and store a tile behind the next one's MMAs: 800 cycles a K
+    // block.  gate | up, 2 x 16384 x 2048 Q8_0: 256 tokens 40 us (52), but 512 tokens 72 us (68 in tiles of 512 rows); 65536 x 2048, 512 tokens 123 us (144)
+    const int64_t big = (N + 255) / 256 * ((T + 255) / 256);
+    const bool stream = geglu ? T <= 256 : pieces == 1 && T > 256 && (double)((big + sms / 2 - 1) / (sms / 2)) * kblocks * 800.0 + 14000.0 < best;
+    if (stream) pair = true, splits = 1, A.MT = 1, A.BN = 256;
     const int br = pair ? A.BN / 2 : A.BN;
     A.groups = 256 / br;
     A.N = (int)N, A.nb = (int)w[0]->nb, A.kblocks = kblocks, A.T = (int)T;
@@ -934,12 +1197,16 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     const bool q4 = type == GGB_TYPE_Q4_0;
     auto kfn = pair ? (q4 ? gemm_quant_kernel<GGB_TYPE_Q4_0, true> : gemm_quant_kernel<GGB_TYPE_Q8_0, true>)
                     : (q4 ? gemm_quant_kernel<GGB_TYPE_Q4_0, false> : gemm_quant_kernel<GGB_TYPE_Q8_0, false>);
+    if (stream)
+        kfn = geglu ? (q4 ? gemm_quant_stream_kernel<GGB_TYPE_Q4_0, true> : gemm_quant_stream_kernel<GGB_TYPE_Q8_0, true>)
+                    : (q4 ? gemm_quant_stream_kernel<GGB_TYPE_Q4_0, false> : gemm_quant_stream_kernel<GGB_TYPE_Q8_0, false>);
     if ((rc = ggb_allow_smem(kfn, kGemmSmem))) return rc;
     // row tiles first: those that share a piece of W run together
     const int rows = A.MT * (pair ? 256 : 128);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)((T + rows - 1) / rows * (pair ? 2 : 1)), (unsigned)((N + A.BN - 1) / A.BN), (unsigned)splits);
-    cfg.blockDim = dim3(kGemmThreads);
+    if (stream) cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(big, sms / 2)));
+    cfg.blockDim = dim3(stream ? kStreamThreads : kGemmThreads);
     cfg.dynamicSmemBytes = kGemmSmem;
     cfg.stream = ggb_cuda_stream();
     cudaLaunchAttribute at[2];
