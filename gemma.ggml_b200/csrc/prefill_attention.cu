@@ -10,8 +10,10 @@
 // A CTA owns 128 rows: 128 / G tokens x the G query heads of one key head, so that a key tile is read once for all of them.  Two groups of
 // four warps take the key tiles in turn, a thread a row; one warp requests K and V tiles (TMA, two stages each), one issues every MMA; weights
 // go back to tensor memory over the scores and are the A operand of the second product.
-// Bound by the chain scores -> weights -> output of the CTA with the most keys (few CTAs: 32 for 512 tokens x 8 heads of one key head).
-// 512 tokens x 8 heads x 256 over one key head: 81 -> 30 us a layer.
+// Where those are few CTAs (32 for 512 tokens x 8 heads of one key head), the key tiles of 128 rows are dealt to the CTAs of a cluster: the maxima meet
+// between the two passes, and each CTA adds up its share of the rows from the others' shared memory, in order.
+// Bound by the chain scores -> weights -> output of the CTAs with the most keys.  512 tokens x 8 heads x 256 over one key head: 81 us a layer by
+// plain dot products, 25 by one CTA, 18 by four.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -39,7 +41,7 @@ struct attn_maps {
 };
 
 __host__ __device__ inline size_t tile_bytes(int D) { return (size_t)(kRows + 4 * kKeys) * D * 2; }
-inline size_t smem_bytes(int D) { return 1024 + tile_bytes(D) + kBarBytes + kRows * (2 * 4 + 2 * 8 + 4); }
+inline size_t smem_bytes(int D) { return 1024 + tile_bytes(D) + kBarBytes + kRows * (2 * 4 + 2 * 8 + 4 + 4); }
 
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, bool b_mn) { // fp32 accumulators, A and B fp16
     return (1u << 4) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -84,6 +86,8 @@ __device__ __noinline__ void plain_row(const attn_args &a, int t, int h, float *
     bar_sync(1, 256);
 }
 
+// C: CTAs of a cluster, that share the key tiles
+template <int C>
 __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __grid_constant__ attn_maps maps, const __grid_constant__ attn_args a) {
     extern __shared__ uint8_t raw[];
     const uint32_t raw0 = smem_u32(raw), base = (raw0 + 1023u) & ~1023u;
@@ -95,13 +99,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
     volatile int *dead = reinterpret_cast<volatile int *>(ctl + SLOT + 4);
     double *s_sum = reinterpret_cast<double *>(ctl + kBarBytes); // [group][row]
     float *s_max = reinterpret_cast<float *>(s_sum + 2 * kRows); // [group][row]
-    int *s_bad = reinterpret_cast<int *>(s_max + 2 * kRows);     // [row]
+    float *s_inv = s_max + 2 * kRows;                            // [row]
+    int *s_bad = reinterpret_cast<int *>(s_inv + kRows);         // [row]
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = blockIdx.y, hpg = a.H / a.Hkv, TQ = kRows / hpg;
     const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * TQ; // the CTAs with the most keys first
     const int nq = min(TQ, a.T - t0), n_rows = nq * hpg;
-    const int NT = (a.pos0 + t0 + nq - 1) / kKeys + 1;
+    const int rank = C > 1 ? (int)blockIdx.z : 0, all = (a.pos0 + t0 + nq - 1) / kKeys + 1;
+    const int NT = (all - rank + C - 1) / C; // key tiles rank, rank + C, ... (all >= 1, C <= 8: at least 0)
 
     if (tid == 0) {
         for (int s = 0; s < 2; s++) {
@@ -151,22 +157,34 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<const uint32_t *>(ctl + SLOT), 0);
 
+    // three meetings of a cluster: maxima, sums, sums read.  These warps have part in none, but count.
+    if (C > 1 && warp >= kTmaWarp) cluster_arrive();
+    auto count_on = [&]() {
+        if (C > 1) cluster_wait(), cluster_sync();
+    };
+    auto meet = [&]() {
+        __syncwarp();
+        if (C > 1) cluster_sync();
+        else bar_sync(1, 256);
+    };
+    auto at_rank = [&](uint32_t addr, int c) { return C > 1 ? cluster_addr(addr, c) : addr; };
     if (warp == kTmaWarp) {
         if (lane == 0) {
             for (int n = 0; n < 2 * NT; n++) {
                 const int s = n & 1, j = n < NT ? n : n - NT;
                 if (n >= 2 && !mbar_wait_bounded(bars + K_FREE + 8 * s, ((n >> 1) - 1) & 1, dead)) break;
                 mbar_expect_tx(bars + K_FULL + 8 * s, stage);
-                for (int b = 0; b < blocks; b++) tma_load_2d(sk + s * stage + b * (kKeys * 128), &maps.k, g * D + 64 * b, kKeys * j, bars + K_FULL + 8 * s);
+                for (int b = 0; b < blocks; b++) tma_load_2d(sk + s * stage + b * (kKeys * 128), &maps.k, g * D + 64 * b, kKeys * (rank + C * j), bars + K_FULL + 8 * s);
                 if (n >= NT) {
                     const int v = j & 1;
                     if (j >= 2 && !mbar_wait_bounded(bars + V_FREE + 8 * v, ((j >> 1) - 1) & 1, dead)) break;
                     mbar_expect_tx(bars + V_FULL + 8 * v, stage);
-                    for (int b = 0; b < blocks; b++) tma_load_2d(sv + v * stage + b * (kKeys * 128), &maps.v, g * D + 64 * b, kKeys * j, bars + V_FULL + 8 * v);
+                    for (int b = 0; b < blocks; b++) tma_load_2d(sv + v * stage + b * (kKeys * 128), &maps.v, g * D + 64 * b, kKeys * (rank + C * j), bars + V_FULL + 8 * v);
                 }
             }
         }
         __syncwarp();
+        count_on();
     } else if (warp == kMmaWarp) {
         const uint32_t id_s = idesc_f16(kRows, kKeys, false), id_o = idesc_f16(kRows, D, true);
         const uint32_t q_lo = umma_desc_lo(base, 16), k_lo = umma_desc_lo(sk, 16), v_lo = umma_desc_lo(sv, kKeys * 128);
@@ -186,7 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
             umma_arrive(bars + K_FREE + 8 * s);
         };
         for (int n = 0; n < NT; n++) scores(n);
-        scores(NT);
+        if (NT) scores(NT);
         for (int m = 0; m < NT; m++) {
             if (m + 1 < NT) scores(NT + m + 1);
             const uint32_t s = (NT + m) & 1, v = m & 1;
@@ -200,6 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
             umma_arrive(bars + PV_DONE + 8 * s);
         }
         umma_arrive(bars + DONE);
+        count_on();
     } else {
         const int grp = warp >> 2, row = (warp & 3) * 32 + lane;
         const uint32_t lanes = (uint32_t)(warp & 3) << 21; // 32 lanes of tensor memory a warp
@@ -209,7 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         for (int n = grp; n < NT; n += 2) {
             mbar_wait_bounded(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
             tc_fence_after();
-            const int last = i_row - kKeys * n; // the row's last key of this tile
+            const int last = i_row - kKeys * (rank + C * n); // the row's last key of this tile
 #pragma unroll
             for (int c0 = 0; c0 < kKeys; c0 += 32) {
                 uint32_t v[32];
@@ -222,14 +241,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
             if (lane == 0) mbar_arrive(bars + S_FREE + 8 * grp);
         }
         s_max[grp * kRows + row] = m;
-        bar_sync(1, 256);
-        m = fmaxf(s_max[row], s_max[kRows + row]);
+        meet();
+        float parts[2 * C];
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const uint32_t there = at_rank(smem_u32(s_max + row), c);
+            parts[2 * c] = ld_cluster_f32(there), parts[2 * c + 1] = ld_cluster_f32(there + 4 * kRows);
+        }
+#pragma unroll
+        for (int c = 0; c < 2 * C; c++) m = fmaxf(m, parts[c]);
         const float l2e = 1.4426950408889634f, m2 = m * l2e;
         double sum = 0.0;
         for (int n = NT + ((NT ^ grp) & 1); n < 2 * NT; n += 2) {
             mbar_wait_bounded(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
             tc_fence_after();
-            const int last = i_row - kKeys * (n - NT);
+            const int last = i_row - kKeys * (rank + C * (n - NT));
 #pragma unroll
             for (int c0 = 0; c0 < kKeys; c0 += 32) {
                 uint32_t v[32], w[16];
@@ -261,44 +287,98 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         mbar_wait_bounded(bars + DONE, 0, dead);
         tc_fence_after();
         bar_sync(1, 256);
-        sum = s_sum[row] + s_sum[kRows + row];
-        const float inv = (float)(1.0 / sum);
-        const int tq = row / hpg, half = D / 2;
-        const int64_t at = ((int64_t)(t0 + tq) * a.H + g * hpg + (row - tq * hpg)) * D + grp * half;
-        // rows of bf16 in shared memory (the tiles are no longer read), from there whole lines: the o-projection's A operand, rounded exactly as
-        // ggb_op_cvt_f32_bf16 would
-        bool finite = isfinite((float)sum);
-        const uint32_t pitch = 2 * D + 16;
-        for (int c0 = 0; c0 < half; c0 += 32) {
-            uint32_t v[32];
-            tmem_load32(tmem + lanes + kOCol + grp * half + c0, v);
-            float o[32];
+        if constexpr (C == 1) {
+            sum = s_sum[row] + s_sum[kRows + row];
+            const float inv = (float)(1.0 / sum);
+            const int tq = row / hpg, half = D / 2;
+            const int64_t at = ((int64_t)(t0 + tq) * a.H + g * hpg + (row - tq * hpg)) * D + grp * half;
+            // rows of bf16 in shared memory (the tiles are no longer read), from there whole lines: the o-projection's A operand, rounded exactly as
+            // ggb_op_cvt_f32_bf16 would
+            bool finite = isfinite((float)sum);
+            const uint32_t pitch = 2 * D + 16;
+            for (int c0 = 0; c0 < half; c0 += 32) {
+                uint32_t v[32];
+                tmem_load32(tmem + lanes + kOCol + grp * half + c0, v);
+                float o[32];
 #pragma unroll
-            for (int c = 0; c < 32; c++) {
-                o[c] = __uint_as_float(v[c]) * inv;
-                finite = finite && isfinite(o[c]);
+                for (int c = 0; c < 32; c++) {
+                    o[c] = __uint_as_float(v[c]) * inv;
+                    finite = finite && isfinite(o[c]);
+                }
+                if (row < n_rows && a.out) {
+#pragma unroll
+                    for (int c = 0; c < 32; c++) a.out[at + c0 + c] = o[c];
+                }
+#pragma unroll
+                for (int c = 0; c < 32; c += 8)
+                    *reinterpret_cast<uint4 *>(gbase + row * pitch + 2 * (grp * half + c0 + c)) =
+                        make_uint4(pack_bf16x2(o[c], o[c + 1]), pack_bf16x2(o[c + 2], o[c + 3]), pack_bf16x2(o[c + 4], o[c + 5]), pack_bf16x2(o[c + 6], o[c + 7]));
             }
-            if (row < n_rows && a.out) {
+            if (!finite) s_bad[row] = 1;
+            bar_sync(1, 256);
+            if (a.out_bf16)
+                for (int i = tid, pieces = D / 8; i < n_rows * pieces; i += 256) {
+                    const int r = i / pieces, pc = i - r * pieces, q = r / hpg;
+                    *reinterpret_cast<uint4 *>(a.out_bf16 + ((int64_t)(t0 + q) * a.H + g * hpg + (r - q * hpg)) * D + 8 * pc) = *reinterpret_cast<const uint4 *>(gbase + r * pitch + 16 * pc);
+                }
+        } else {
+            // this CTA's sums, fp32, where the tiles were (they are no longer read): 16-byte piece p of row r at place p ^ (r & 7)
+            const int half = D / 2, pieces = D / 4;
+            for (int c0 = 0; c0 < half; c0 += 32) {
+                uint32_t v[32];
+                if (NT) tmem_load32(tmem + lanes + kOCol + grp * half + c0, v);
 #pragma unroll
-                for (int c = 0; c < 32; c++) a.out[at + c0 + c] = o[c];
+                for (int c = 0; c < 32; c += 4)
+                    *reinterpret_cast<uint4 *>(gbase + (row * pieces + (((grp * half + c0 + c) >> 2) ^ (row & 7))) * 16) = NT ? make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]) : make_uint4(0, 0, 0, 0);
             }
+            meet();
+            // a share of the rows, from all CTAs of the cluster
+            constexpr int R = kRows / C, U = 8 / C; // rows, pieces of them a thread has in flight (D is a multiple of 64: R * pieces of 256 U)
+            const int r0 = rank * R;
+            if (tid < R) {
+                double part[2 * C], sum = 0.0;
 #pragma unroll
-            for (int c = 0; c < 32; c += 8)
-                *reinterpret_cast<uint4 *>(gbase + row * pitch + 2 * (grp * half + c0 + c)) =
-                    make_uint4(pack_bf16x2(o[c], o[c + 1]), pack_bf16x2(o[c + 2], o[c + 3]), pack_bf16x2(o[c + 4], o[c + 5]), pack_bf16x2(o[c + 6], o[c + 7]));
+                for (int c = 0; c < C; c++) {
+                    const uint32_t there = at_rank(smem_u32(s_sum + r0 + tid), c);
+                    part[2 * c] = ld_cluster_f64(there), part[2 * c + 1] = ld_cluster_f64(there + 8 * kRows);
+                }
+#pragma unroll
+                for (int c = 0; c < C; c++) sum += part[2 * c] + part[2 * c + 1];
+                s_inv[r0 + tid] = (float)(1.0 / sum);
+                if (!isfinite((float)sum)) s_bad[r0 + tid] = 1;
+            }
+            bar_sync(1, 256);
+            for (int i0 = tid; i0 < R * pieces; i0 += 256 * U) {
+                float4 x[U][C];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int i = i0 + 256 * u, r = r0 + i / pieces, p = i % pieces;
+#pragma unroll
+                    for (int c = 0; c < C; c++) x[u][c] = ld_cluster_f32x4(at_rank(base + (r * pieces + (p ^ (r & 7))) * 16, c));
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int i = i0 + 256 * u, r = r0 + i / pieces, p = i % pieces, tq = r / hpg;
+                    float4 o = x[u][0];
+#pragma unroll
+                    for (int c = 1; c < C; c++) o.x += x[u][c].x, o.y += x[u][c].y, o.z += x[u][c].z, o.w += x[u][c].w;
+                    const float inv = s_inv[r];
+                    o.x *= inv, o.y *= inv, o.z *= inv, o.w *= inv;
+                    if (r >= n_rows) continue;
+                    if (!(isfinite(o.x) && isfinite(o.y) && isfinite(o.z) && isfinite(o.w))) s_bad[r] = 1;
+                    const int64_t at = ((int64_t)(t0 + tq) * a.H + g * hpg + (r - tq * hpg)) * D + 4 * p;
+                    if (a.out) a.out[at] = o.x, a.out[at + 1] = o.y, a.out[at + 2] = o.z, a.out[at + 3] = o.w;
+                    if (a.out_bf16) *reinterpret_cast<uint2 *>(a.out_bf16 + at) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w)); // as ggb_op_cvt_f32_bf16 would
+                }
+            }
         }
-        if (!finite) s_bad[row] = 1;
-        bar_sync(1, 256);
-        if (a.out_bf16)
-            for (int i = tid, pieces = D / 8; i < n_rows * pieces; i += 256) {
-                const int r = i / pieces, pc = i - r * pieces, q = r / hpg;
-                *reinterpret_cast<uint4 *>(a.out_bf16 + ((int64_t)(t0 + q) * a.H + g * hpg + (r - q * hpg)) * D + 8 * pc) = *reinterpret_cast<const uint4 *>(gbase + r * pitch + 16 * pc);
-            }
-        bar_sync(1, 256);
-        if (!*dead)
-            for (int r = 0; r < n_rows; r++)
-                if (s_bad[r]) plain_row(a, t0 + r / hpg, g * hpg + r % hpg, reinterpret_cast<float *>(gbase), s_sum);
     }
+    __syncwarp();
+    if (C > 1) cluster_sync(); // the others have read this CTA's sums
+    else if (warp < 8) bar_sync(1, 256);
+    if (warp < 8 && !*dead)
+        for (int r = rank * (kRows / C); r < min((rank + 1) * (kRows / C), n_rows); r++)
+            if (s_bad[r]) plain_row(a, t0 + r / hpg, g * hpg + r % hpg, reinterpret_cast<float *>(gbase), s_sum);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -328,10 +408,16 @@ int ggb_attn_prefill_tiles(const float *q, const void *kcache, const void *vcach
     if (rc) return rc;
     const attn_args a{q, (const __half *)kcache, (const __half *)vcache, (int)T, pos0, H, Hkv, d, ggb_exp_table_dev(), out, (__nv_bfloat16 *)out_bf16, ggb_wait_error_flag()};
     const size_t smem = smem_bytes(d);
-    rc = ggb_allow_smem(attn_prefill_tile_kernel, smem);
-    if (rc) return rc;
-    const int TQ = kRows / (H / Hkv);
-    GGB_CUDA(ggb_launch_step(attn_prefill_tile_kernel, dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv), dim3(kThreads), smem, maps, a));
+    const int TQ = kRows / (H / Hkv), tiles = (int)((T + TQ - 1) / TQ) * Hkv, n_tiles = (int)((n_kv + kKeys - 1) / kKeys);
+    // CTAs that share the key tiles of 128 rows, and the adding up: up to 4 while there are SMs for them (8 heads of 256 over one: 512 tokens 25 us by
+    // one, 22, 18; 128 tokens 17, 16, 16); 8 for many keys and so few rows that clusters of 8 find room at once (64 tokens behind 1000 positions: 43, 29,
+    // 22, 19; 512 tokens, 256 CTAs: 48).  Heads of up to 128 over two tiles of keys: 7.5 us by one, 8.4, 8.7
+    int C = 1;
+    while (C < 4 && 2 * C * tiles <= ggb_sm_count() && n_tiles >= (d > 128 ? 2 : 3)) C *= 2;
+    if (C == 4 && 8 * tiles <= 112 && n_tiles >= 8) C = 8;
+    auto kern = C == 8 ? attn_prefill_tile_kernel<8> : C == 4 ? attn_prefill_tile_kernel<4> : C == 2 ? attn_prefill_tile_kernel<2> : attn_prefill_tile_kernel<1>;
+    if ((rc = ggb_allow_smem(kern, smem))) return rc;
+    GGB_CUDA(ggb_launch_step_cluster(kern, C, dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv, (unsigned)C), dim3(kThreads), smem, maps, a));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

@@ -41,7 +41,9 @@ def plain(q, k, v, pos0):
 
 
 @pytest.mark.parametrize("T,pos0,H,Hkv,D", [(16, 112, 8, 1, 256), (17, 111, 8, 1, 256), (130, 0, 8, 8, 64), (64, 0, 4, 4, 128), (65, 63, 4, 1, 64), (33, 191, 6, 2, 192), (40, 1, 5, 1, 128),
-                                            (16, 700, 4, 2, 256), (129, 300, 2, 2, 256)])
+                                            (16, 700, 4, 2, 256), (129, 300, 2, 2, 256),
+                                            # key tiles dealt to 4, 8 and 2 CTAs, of which some have none
+                                            (512, 0, 8, 1, 256), (200, 1000, 8, 1, 128), (300, 0, 8, 4, 64)])
 def test_prompts(gpu, T, pos0, H, Hkv, D):
     r = np.random.default_rng(T + pos0 + H)
     q = r.standard_normal((T, H, D)) * 2.0 * D ** -0.5
