@@ -109,7 +109,8 @@ __device__ __forceinline__ uint4 ldg_stream_u4(const void *p) {
 // through the read-only cache or ahead of this statement.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Behind step_wait: once every block has said so, blocks of the next kernel may take what room there is and run up to their own step_wait.  What
-// they read ahead of it was written before the kernels that came before this one ended.
+// they read ahead of it was written before the kernels that came before this one ended.  A kernel with tensor memory says so when it has it:
+// a block of the next kernel that took it first would hold it until this kernel ends.
 __device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float half_bits_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }

@@ -126,7 +126,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
     step_wait();
-    step_next();
     if (warp < 8) { // queries, rounded to fp16: 8 numbers a step, neighbouring lanes along a row, eight steps in flight
         const int pieces = D / 8, n = kRows * pieces;
         for (int i0 = tid; i0 < n; i0 += 8 * 256) {
@@ -155,6 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<const uint32_t *>(ctl + SLOT), 0);
 
     // three meetings of a cluster: maxima, sums, sums read.  These warps have part in none, but count.
