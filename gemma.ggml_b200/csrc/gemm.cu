@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) tmem_alloc512(bars + SLOT);
+    step_wait();
     const bool listed = a.m_ranges && a.n_groups <= kMaxGroups;
     if (listed && warp == 3) { // prefix sums of the groups' row tiles
         int sum = 0;
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
     int row_tiles = a.m_tiles;
     if (listed) row_tiles = first_tile[a.n_groups];
@@ -282,10 +284,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) tmem_alloc512_pair(bars + SLOT);
+    step_wait();
     tc_fence_before();
     __syncthreads();
     cluster_sync();
     tc_fence_after();
+    step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
     const int total = a.m_tiles * a.n_tiles * a.splits, pairs = gridDim.x / 2, me = blockIdx.x / 2;
     // row tiles first: those that share a piece of W run together
@@ -403,10 +407,12 @@ int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmem;
     cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-    cfg.attrs = at, cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at, cfg.numAttrs = 2;
     GGB_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -418,7 +424,7 @@ int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_ro
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
-    gemm_tma_kernel<<<std::min(ctas, ggb_sm_count()), kThreads, kSmem, ggb_cuda_stream()>>>(ma, mw, g);
+    GGB_CUDA(ggb_launch_step(gemm_tma_kernel, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

@@ -16,7 +16,7 @@
 // A product of few tiles is cut along K over the CTAs of a cluster (up to 8), whose sums meet in shared memory and are added in order.
 //
 // What bounds it: fp32, shared memory (written and read: BT = 64: 170 KB a stage, 1330 cycles of 128 bytes); bf16, the loads in flight.
-// 333 x 2816 x 1000 fp32: 98.4 -> 33.0 us (64 x 64 tiles of FMAs).
+// 333 x 2816 x 1000 fp32: 98.4 -> 30.5 us (64 x 64 tiles of FMAs).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -113,9 +113,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
+    step_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
     const uint32_t acc_cols = P * BT; // of one accumulator; two of them: at most 384
 
@@ -296,10 +298,12 @@ int launch_any(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, 
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)g.splits, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-    cfg.attrs = at, cfg.numAttrs = g.splits > 1 ? 1 : 0;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)g.splits, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+    cfg.attrs = at, cfg.numAttrs = g.splits > 1 ? 2 : 1;
     GGB_CUDA(cudaLaunchKernelEx(&cfg, kern, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;

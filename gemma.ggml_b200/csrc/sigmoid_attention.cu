@@ -352,7 +352,7 @@ int ggb_op_sigmoid_attn(int dt, const float *q, const void *cache, const int32_t
     cudaStream_t st = ggb_cuda_stream();
     if (dt == GGB_TYPE_BF16 && tile_attn::fits(tile_attn::SIGMOID, 1, D, Dv, H, G, q, cache, T)) {
         const tile_attn::shape sh{q, (const __nv_bfloat16 *)cache, cld, block_table, block_size, pos0, T, H, G, D, Dv, window, 0, 0, 0.f, r1, r2, pb, ggb_wait_error_flag()};
-        return tile_attn::launch<tile_attn::SIGMOID, 1>(sh, tile_store{(__nv_bfloat16 *)out, H, Dv}, st);
+        return tile_attn::launch<tile_attn::SIGMOID, 1>(sh, tile_store{(__nv_bfloat16 *)out, H, Dv});
     }
     if (T >= kQT) {
         const bool tv = vec && Dv % vn == 0;

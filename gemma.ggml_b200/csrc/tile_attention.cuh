@@ -22,9 +22,9 @@
 // arithmetic gives for it.
 //
 // What bounds it: the instructions around the weights (two numbers an instruction where the unit has a packed form: fma.rn.f32x2), then the
-// MMAs.  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft cap, gate: 43 us, 200 TFLOP/s of
+// MMAs.  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft cap, gate: 42 us, 207 TFLOP/s of
 // the products asked for (57 us with four warps a group and one thread a row, number by number; 785 us by the fp32 CUDA cores, tiles of 32
-// queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 55 us (64 us; 686 us).
+// queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 53 us (64 us; 686 us).
 #pragma once
 
 #include "dense.cuh"
@@ -312,10 +312,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     // the CTAs with the most keys first
     const int64_t t0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * TQ;
     const int nq = (int)min((int64_t)TQ, a.T - t0), n_pairs = nq * hpg;
-    const int64_t i0 = (int64_t)*a.pos0 + t0, i_last = i0 + nq - 1;
-    const tiles tl(first_visible(i0, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i_last);
-    const int NT = tl.n;
-
     if (tid == 0) {
         for (int s = 0; s < 2; s++) {
             mbar_init(bars + K_FULL + 8 * s, 1);
@@ -331,9 +327,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
+    step_wait();
+    const int64_t i0 = (int64_t)*a.pos0 + t0, i_last = i0 + nq - 1;
+    const tiles tl(first_visible(i0, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i_last);
+    const int NT = tl.n;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, ctlw[SLOT / 4], 0);
     const uint32_t reg_cols = MAPS == 1 ? 96 : 128; // scores [MAPS][64], then weights over them
     const uint32_t o_col = 2 * reg_cols;
@@ -604,13 +605,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     }
 }
 
-template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin, cudaStream_t st) {
+template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin) {
     const size_t smem = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G);
     auto kfn = attn_kernel<MODE, MAPS, FIN>;
     const int rc = ggb_allow_smem(kfn, smem);
     if (rc) return rc;
     const int TQ = kRows / MAPS / (a.H / a.G);
-    kfn<<<dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), kThreads, smem, st>>>(a, fin);
+    GGB_CUDA(ggb_launch_step(kfn, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), dim3(kThreads), smem, a, fin));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

@@ -968,7 +968,7 @@ static int masked_attn_launch(int dt, const float *q, const void *cache, const i
     if (dt == GGB_TYPE_BF16 && (uintptr_t)out % 4 == 0 && tile_attn::fits(tile_attn::SOFTMAX, MAPS, D, Dv, H, G, q, cache, T)) {
         const tile_attn::shape sh{q, (const __nv_bfloat16 *)cache, cld, block_table, block_size, pos0, T, H, G, D, Dv, window, chunked, keep, softcap,
                                   nullptr, nullptr, nullptr, ggb_wait_error_flag()};
-        return tile_attn::launch<tile_attn::SOFTMAX, MAPS>(sh, tile_finish<MAPS>{da, cos_sin_v, (__nv_bfloat16 *)out, H, Dv}, st);
+        return tile_attn::launch<tile_attn::SOFTMAX, MAPS>(sh, tile_finish<MAPS>{da, cos_sin_v, (__nv_bfloat16 *)out, H, Dv});
     }
     if (T >= kQT) { // a portion: tiles of cache rows staged once for 32 queries
         // 16-byte pieces need every head's keys and values to start on one: D, Dv and G * D whole pieces
