@@ -108,7 +108,9 @@ __device__ __forceinline__ uint4 ldg_stream_u4(const void *p) {
 // not written while the kernel runs, none is reached by another way) does not hold until here, and a compiler that believes it may read
 // through the read-only cache or ahead of this statement.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Behind step_wait: once every block has said so, blocks of the next kernel may take what room there is and run up to their own step_wait.  What
+// The same in a kernel that sets itself up ahead of it: barriers, tensor memory, numbers of its arguments, and at most weights, which stand longer
+__device__ __forceinline__ void early_wait() { step_wait(); }
+// Behind the wait: once every block has said so, blocks of the next kernel may take what room there is and run up to their own wait.  What
 // they read ahead of it was written before the kernels that came before this one ended.  A kernel with tensor memory says so when it has it:
 // a block of the next kernel that took it first would hold it until this kernel ends.
 __device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) tmem_alloc512(bars + SLOT);
-    step_wait();
+    early_wait();
     const bool listed = a.m_ranges && a.n_groups <= kMaxGroups;
     if (listed && warp == 3) { // prefix sums of the groups' row tiles
         int sum = 0;
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) tmem_alloc512_pair(bars + SLOT);
-    step_wait();
+    early_wait();
     tc_fence_before();
     __syncthreads();
     cluster_sync();
@@ -424,7 +424,7 @@ int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_ro
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
-    GGB_CUDA(ggb_launch_step(gemm_tma_kernel, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
+    GGB_CUDA(ggb_launch_step_cluster(gemm_tma_kernel, 1, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

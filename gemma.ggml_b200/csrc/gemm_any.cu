@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
-    step_wait();
+    early_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

@@ -815,7 +815,8 @@ int ggb_op_moe_combine(const float *y, const int32_t *ws, const float *wt, int64
     GGB_CHECK_ARG(y && ws && wt && out && T > 0 && top > 0 && W > 0, "moe_combine: bad arguments");
     const int32_t *inv = ws + n_exp + 1 + T * top;
     const bool vec = W % 4 == 0 && ((uintptr_t)y | (uintptr_t)out) % 16 == 0;
-    ggb_launch_step(vec ? moe_combine_kernel<true> : moe_combine_kernel<false>, dim3((unsigned)T), dim3(256), 0, y, inv, wt, top, W, out);
+    if (vec) ggb_launch_step(moe_combine_kernel<true>, dim3((unsigned)T), dim3(256), 0, y, inv, wt, top, W, out);
+    else ggb_launch_step(moe_combine_kernel<false>, dim3((unsigned)T), dim3(256), 0, y, inv, wt, top, W, out);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

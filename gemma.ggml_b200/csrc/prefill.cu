@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
             const bool is_a = warp == kTmaWarp;
             const int n = is_a ? A.stages : A.code_stages, fre = is_a ? FREE : C_FREE;
             // A is what the kernel before wrote, and everything stored here waits for A; weights stand since a launch before that one at least
-            if (is_a) step_wait(), step_next();
+            if (is_a) early_wait(), step_next();
             int s = 0;
             uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_quant_stream_kernel(co
             const int n = is_a ? kStreamStages : kStreamCodes, fre = is_a ? Q_EMPTY : Q_C_FREE;
             int s = 0;
             uint32_t ph = 0;
-            if (is_a) step_wait(), step_next(); // as gemm_quant_kernel
+            if (is_a) early_wait(), step_next(); // as gemm_quant_kernel
             for (int t = me; t < total; t += pairs) {
                 const place at = locate(t);
                 for (int kb = 0; kb < kblocks; kb++) {

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
-    step_wait();
+    early_wait();
     if (warp < 8) { // queries, rounded to fp16: 8 numbers a step, neighbouring lanes along a row, eight steps in flight
         const int pieces = D / 8, n = kRows * pieces;
         for (int i0 = tid; i0 < n; i0 += 8 * 256) {
@@ -172,12 +172,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         if (lane == 0) {
             for (int n = 0; n < 2 * NT; n++) {
                 const int s = n & 1, j = n < NT ? n : n - NT;
-                if (n >= 2 && !mbar_wait_bounded(bars + K_FREE + 8 * s, ((n >> 1) - 1) & 1, dead)) break;
+                if (!mbar_wait_bounded(bars + K_FREE + 8 * s, ((n >> 1) & 1) ^ 1, dead)) break;
                 mbar_expect_tx(bars + K_FULL + 8 * s, stage);
                 for (int b = 0; b < blocks; b++) tma_load_2d(sk + s * stage + b * (kKeys * 128), &maps.k, g * D + 64 * b, kKeys * (rank + C * j), bars + K_FULL + 8 * s);
                 if (n >= NT) {
                     const int v = j & 1;
-                    if (j >= 2 && !mbar_wait_bounded(bars + V_FREE + 8 * v, ((j >> 1) - 1) & 1, dead)) break;
+                    if (!mbar_wait_bounded(bars + V_FREE + 8 * v, ((j >> 1) & 1) ^ 1, dead)) break;
                     mbar_expect_tx(bars + V_FULL + 8 * v, stage);
                     for (int b = 0; b < blocks; b++) tma_load_2d(sv + v * stage + b * (kKeys * 128), &maps.v, g * D + 64 * b, kKeys * (rank + C * j), bars + V_FULL + 8 * v);
                 }

@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kRecThreads, 1) recurrence_chunk_kernel(rec_ar
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    step_wait();
+    early_wait();
     if (warp == kRecWarps) { // the blocks of the chunks
         if (lane == 0) {
             const int hk = CH || MODE == 0 ? h : h / (p.H / p.G);
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kRecThreads, 1) recurrence_chunk_kernel(rec_ar
             const unsigned char *v = ws.v + ((size_t)h * gridDim.y + blockIdx.y) * chunks * sizeof(block_t::v);
             for (int c = 0; c < chunks; c++) {
                 const int s = c % kRing;
-                if (c >= kRing && !mbar_wait_bounded(fre + 8 * s, (c / kRing - 1) & 1, dead)) break;
+                if (!mbar_wait_lane(fre + 8 * s, (c / kRing & 1) ^ 1, dead)) break;
                 mbar_expect_tx(full + 8 * s, sizeof(block_t));
                 bulk_load(smem_u32(&ring[s].rows), rows + (size_t)c * sizeof(block_t::rows), sizeof(block_t::rows), full + 8 * s);
                 bulk_load(smem_u32(&ring[s].coef), coef + (size_t)c * sizeof(chunk_coef), sizeof(chunk_coef), full + 8 * s);
@@ -805,7 +805,7 @@ int recurrence_launch_chunks(rec_args p, bool *done) {
         if (q.a) q.a += t0 * p.ld_a;
         GGB_CUDA(ggb_launch_step(recurrence_prepare_kernel<DP, MODE>, dim3((unsigned)chunks, (unsigned)rows_of), dim3(32 * kTok), 0, q, ws));
         GGB_LAUNCH_CHECK();
-        GGB_CUDA(ggb_launch_step(k, dim3((unsigned)p.H, (unsigned)slices), dim3(kRecThreads), smem, q, ws, ggb_wait_error_flag()));
+        GGB_CUDA(ggb_launch_step_cluster(k, 1, dim3((unsigned)p.H, (unsigned)slices), dim3(kRecThreads), smem, q, ws, ggb_wait_error_flag()));
         GGB_LAUNCH_CHECK();
     }
     return rc;

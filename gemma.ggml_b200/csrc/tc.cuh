@@ -46,6 +46,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     *dead = 1;
     return false;
 }
+// The same by one lane of a kernel without tensor memory
+__device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, volatile int *dead) { return mbar_wait_bounded(bar, parity, dead); }
 // The same for a warp that reads a buffer of shared memory behind the wait and hands it back by one lane's arrival: one lane polls.  Where every
 // lane polls they leave the loop one after the other, and the barrier of the warp ahead of the arrival did not hold them together (the loop
 // passes for uniform): the buffer was refilled while the last lanes read it, in 9 of 10 launches of a kernel whose copies came late.

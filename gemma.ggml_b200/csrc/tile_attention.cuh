@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) tmem_alloc512(bars + SLOT);
-    step_wait();
+    early_wait();
     const int64_t i0 = (int64_t)*a.pos0 + t0, i_last = i0 + nq - 1;
     const tiles tl(first_visible(i0, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i_last);
     const int NT = tl.n;
@@ -611,7 +611,7 @@ template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN
     const int rc = ggb_allow_smem(kfn, smem);
     if (rc) return rc;
     const int TQ = kRows / MAPS / (a.H / a.G);
-    GGB_CUDA(ggb_launch_step(kfn, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), dim3(kThreads), smem, a, fin));
+    GGB_CUDA(ggb_launch_step_cluster(kfn, 1, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), dim3(kThreads), smem, a, fin));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

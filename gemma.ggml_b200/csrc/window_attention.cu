@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(32 * kWarps) window_step_kernel(const float *q
                                                                   const float *cs_v, finish_args da, E *out) {
     constexpr int VN = RowVec<E>::n, RPL = step_tile<LG>::rows_per_load, NL = step_tile<LG>::loads, RT = step_tile<LG>::rows, W = LG * VN;
     __shared__ float s_acc[kWarps][MAPS][W], s_ml[kWarps][MAPS][2], s_out[MAPS][W + 2]; // s_out: this CTA's sums, maximum, denominator
-    step_wait();
+    early_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LG, pc = lane % LG;
     const int h = blockIdx.y, g = h / (H / G);
     const int64_t t = blockIdx.x, i = (int64_t)*pos0 + t;
