@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
             k_range(at.split, kb0, kb1);
             const int chunks = (kb1 - kb0 + a.chunk_kb - 1) / a.chunk_kb; // the last CTA along K may have fewer
             const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
-            mbar_wait_bounded(bars + ACC_FULL + 8 * buf, use & 1, dead);
+            mbar_wait_warp(bars + ACC_FULL + 8 * buf, use & 1, dead);
             tc_fence_after();
             // a warp's 32 rows, every other 32 columns (the two warps of a quarter share them)
             const int row0 = at.m0 + lq * 32;
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
             k_range(split, kb0, kb1);
             const int chunks = kb1 > kb0 ? (kb1 - kb0 + a.chunk_kb - 1) / a.chunk_kb : 0;
             const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
-            mbar_wait_bounded(bars + ACC_FULL + 8 * buf, use & 1, dead);
+            mbar_wait_warp(bars + ACC_FULL + 8 * buf, use & 1, dead);
             tc_fence_after();
             const int row0 = m0 + (int)rank * BM + lq * 32;
             if (row0 < a.T)

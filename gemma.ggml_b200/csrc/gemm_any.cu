@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
         int s = 0;
         uint32_t ph = 1;
         for (int kb = kb0; kb < kb1; kb++) {
-            if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph, dead)) break;
+            if (!mbar_wait_warp(bars + EMPTY + 8 * s, ph, dead)) break;
             uint8_t *st = gbase + s * st_bytes;
 #pragma unroll
             for (int i0 = 0; i0 < NI; i0 += 4) { // four pieces at a time: their chains of instructions side by side
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
         const int accs = (nkb + SPA - 1) / SPA;
         for (int q = 0; q < accs; q++) {
             const int buf = q & 1;
-            mbar_wait_bounded(bars + ACC_FULL + 8 * buf, (q >> 1) & 1, dead);
+            mbar_wait_warp(bars + ACC_FULL + 8 * buf, (q >> 1) & 1, dead);
             tc_fence_after();
             const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + buf * acc_cols + half * hc;
 #pragma unroll

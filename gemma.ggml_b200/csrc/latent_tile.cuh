@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
             b++;
         };
         auto wait_free = [&]() { // the step that used this left buffer (and the right one two steps ahead) is done
-            if (b >= 2) mbar_wait_bounded(bars + FREE + 8 * (b & 1), ((b >> 1) - 1) & 1, dead);
+            if (b >= 2) mbar_wait_warp(bars + FREE + 8 * (b & 1), ((b >> 1) - 1) & 1, dead);
         };
         look_up(0, cur);
         if (n_mine > 0) {
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
             const int n_keys = (int)min(i_last - j0 + 1, (int64_t)kKeys);
             const bool whole = n_keys == kKeys && j0 + kKeys - 1 <= i0 && (a.window <= 0 || j0 >= i_last - a.window + 1);
             const int c_hi = live ? (int)max((int64_t)0, min((int64_t)n_keys, i - j0 + 1)) : 0, c_lo = (int)max((int64_t)0, min((int64_t)kKeys, lo - j0));
-            mbar_wait_bounded(bars + S_FULL, k & 1, dead);
+            mbar_wait_warp(bars + S_FULL, k & 1, dead);
             tc_fence_after();
             { // maximum of the tile: a group takes every other 64 positions
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
         cp_async_wait<0>();
         // ---- the part: relative to the true maximum, rows through shared memory
         if (b > 0) {
-            mbar_wait_bounded(bars + FREE + 8 * ((b - 1) & 1), ((b - 1) >> 1) & 1, dead);
+            mbar_wait_warp(bars + FREE + 8 * ((b - 1) & 1), ((b - 1) >> 1) & 1, dead);
             tc_fence_after();
         }
         mxs[grp * kRows + r] = l;
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_out_kernel(const out_args 
                     }
                 }
             }
-            if (c >= 2) mbar_wait_bounded(bars + FREE + 8 * s, ((c >> 1) - 1) & 1, dead);
+            if (c >= 2) mbar_wait_warp(bars + FREE + 8 * s, ((c >> 1) - 1) & 1, dead);
             if (64 * c + 8 * pc < a.R)
                 for (int v = pr; v < a.Dv; v += 32)
                     cp_async16(base + s * kStage + kLeft + v * 128 + ((pc ^ (v & 7)) << 4), a.w_uv + ((int64_t)h * a.Dv + v) * a.R + 64 * c + 8 * pc);
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_out_kernel(const out_args 
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + FULL + 8 * s);
         }
-        mbar_wait_bounded(bars + FREE + 8 * ((nc - 1) & 1), ((nc - 1) >> 1) & 1, dead);
+        mbar_wait_warp(bars + FREE + 8 * ((nc - 1) & 1), ((nc - 1) >> 1) & 1, dead);
         tc_fence_after();
         const int r = 32 * (warp & 3) + lane, t = t0 + r;
         const float gsc = a.gate && r < nq ? 1.0f / (1.0f + expf(-a.gate[(int64_t)t * a.ldg + h])) : 1.0f;

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bars + C_FREE + 8 * s); // the codes are in registers
-                if (before >= 0) mbar_wait_bounded(bars + FREE + 8 * before, bph, dead); // the group's buffer
+                if (before >= 0) mbar_wait_warp(bars + FREE + 8 * before, bph, dead); // the group's buffer
 #pragma unroll
                 for (int q = 0; q < 4; q++) sts_u4(dst + (((4 * whalf + q) ^ (wr & 7)) << 4), o[q]);
                 fence_async_smem();
@@ -247,14 +247,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
             }
         }
         // ================= epilogue: pieces of 32 rows x 32 columns, dealt to the four warps of a lane quarter
-        mbar_wait_bounded(bars + DONE, 0, dead);
+        mbar_wait_warp(bars + DONE, 0, dead);
         tc_fence_after();
         const int chunks = kb1 > kb0 ? (kb1 - kb0 + A.chunk_kb - 1) / A.chunk_kb : 0, lq = warp & 3, cols = (A.geglu ? A.BN / 2 : A.BN) / 32;
         const int planes = A.ws ? chunks : 1; // in a workspace every piece along K stands alone: they are added in order, whichever CTA summed them
         float *cbase = A.ws ? A.ws + (size_t)split * A.chunks * A.T * A.N + n0 : sg.c + sn0;
         const int cld = A.ws ? A.N : sg.ldc;
         const uint32_t my = smem0 + warp * 4096; // the ring is no longer used
-        if (A.geglu) mbar_wait_bounded(bars + TABLE_FULL, 0, dead);
+        if (A.geglu) mbar_wait_warp(bars + TABLE_FULL, 0, dead);
         auto gelu = [&](uint32_t g) { // of an fp16 number, rounded to fp16: the table, as ggb_op_geglu_bf16 reads it
             uint16_t h;
             asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(smem0 + kGeluAt + 2u * float_to_half_bits(__uint_as_float(g))) : "memory");
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_quant_kernel(const __gri
             if (!ready) mbar_wait_bounded(bars + FULL + 8 * s, ph, dead);
             tc_fence_after();
             const bool wrap = s + 1 == A.stages;
-            ready = mbar_peek(bars + FULL + 8 * (wrap ? 0 : s + 1), wrap ? ph ^ 1u : ph); // of a block past the last: not done
+            ready = mbar_test(bars + FULL + 8 * (wrap ? 0 : s + 1), wrap ? ph ^ 1u : ph); // of a block past the last: not done
             const uint32_t a_lo = umma_desc_lo(ring + s * a_bytes, 16), b_lo = umma_desc_lo(smem0 + grp * b_bytes, 16);
             for (int mt = 0; mt < A.MT; mt++) {
                 const uint32_t d = tmem + (mt * A.chunks + chunk) * A.BN;
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_quant_stream_kernel(co
                 tc_fence_after();
                 const uint32_t at = smem0 + s * kStage;
                 if (++s == kStreamStages) s = 0, ph ^= 1u;
-                ready = mbar_peek(bars + Q_FULL + 8 * s, ph);
+                ready = mbar_test(bars + Q_FULL + 8 * s, ph);
                 umma_ss_pair_k4(tmem + buf * 256, umma_desc_lo(at, 16), umma_desc_lo(at + kHalf, 16), idesc, kb > 0);
                 umma_arrive_pair(bars + Q_EMPTY + (at - smem0) / kStage * 8);
             }
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_quant_stream_kernel(co
             const place at = locate(t);
             const GemmSeg &sg = A.seg[at.si];
             const int buf = it & 1, row0 = at.m0 + rank * 128 + lq * 32;
-            mbar_wait_bounded(bars + Q_ACC_FULL + 8 * buf, (it >> 1) & 1, dead);
+            mbar_wait_warp(bars + Q_ACC_FULL + 8 * buf, (it >> 1) & 1, dead);
             tc_fence_after();
             if (row0 < A.T)
                 for (int c0 = 0; c0 < (GEGLU ? 128 : 256) && at.sn0 + c0 < sg.rows; c0 += 32) {

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         const int i_row = a.pos0 + t0 + min(row, n_rows - 1) / hpg;
         float m = -INFINITY;
         for (int n = grp; n < NT; n += 2) {
-            mbar_wait_bounded(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
+            mbar_wait_warp(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
             tc_fence_after();
             const int last = i_row - kKeys * (rank + C * n); // the row's last key of this tile
 #pragma unroll
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
         const float l2e = 1.4426950408889634f, m2 = m * l2e;
         double sum = 0.0;
         for (int n = NT + ((NT ^ grp) & 1); n < 2 * NT; n += 2) {
-            mbar_wait_bounded(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
+            mbar_wait_warp(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
             tc_fence_after();
             const int last = i_row - kKeys * (rank + C * (n - NT));
 #pragma unroll
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tile_kernel(const __
             if (lane == 0) mbar_arrive(bars + P_FULL + 8 * grp);
         }
         s_sum[grp * kRows + row] = sum;
-        mbar_wait_bounded(bars + DONE, 0, dead);
+        mbar_wait_warp(bars + DONE, 0, dead);
         tc_fence_after();
         bar_sync(1, 256);
         if constexpr (C == 1) {

@@ -545,13 +545,13 @@ __global__ void __launch_bounds__(kRecThreads, 1) recurrence_chunk_kernel(rec_ar
     __syncthreads();
     early_wait();
     if (warp == kRecWarps) { // the blocks of the chunks
-        if (lane == 0) {
-            const int hk = CH || MODE == 0 ? h : h / (p.H / p.G);
-            const unsigned char *rows = ws.rows + (size_t)hk * chunks * sizeof(block_t::rows), *coef = ws.coef + (size_t)h * chunks * sizeof(chunk_coef);
-            const unsigned char *v = ws.v + ((size_t)h * gridDim.y + blockIdx.y) * chunks * sizeof(block_t::v);
-            for (int c = 0; c < chunks; c++) {
-                const int s = c % kRing;
-                if (!mbar_wait_lane(fre + 8 * s, (c / kRing & 1) ^ 1, dead)) break;
+        const int hk = CH || MODE == 0 ? h : h / (p.H / p.G);
+        const unsigned char *rows = ws.rows + (size_t)hk * chunks * sizeof(block_t::rows), *coef = ws.coef + (size_t)h * chunks * sizeof(chunk_coef);
+        const unsigned char *v = ws.v + ((size_t)h * gridDim.y + blockIdx.y) * chunks * sizeof(block_t::v);
+        for (int c = 0; c < chunks; c++) {
+            const int s = c % kRing;
+            if (!mbar_wait_warp(fre + 8 * s, (c / kRing & 1) ^ 1, dead)) break;
+            if (lane == 0) {
                 mbar_expect_tx(full + 8 * s, sizeof(block_t));
                 bulk_load(smem_u32(&ring[s].rows), rows + (size_t)c * sizeof(block_t::rows), sizeof(block_t::rows), full + 8 * s);
                 bulk_load(smem_u32(&ring[s].coef), coef + (size_t)c * sizeof(chunk_coef), sizeof(chunk_coef), full + 8 * s);

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 const uint32_t j = (uint32_t)min(tl.first(n) + 32 * u + lane, tl.last(n)), pg = j / (uint32_t)a.B;
                 my_row[u] = (uint32_t)a.table[pg] * (uint32_t)a.B + (j - pg * a.B);
             }
-            if (n >= 2) mbar_wait_bounded(bars + fre + 8 * s, ((n >> 1) - 1) & 1, dead);
+            if (n >= 2) mbar_wait_warp(bars + fre + 8 * s, ((n >> 1) - 1) & 1, dead);
 #pragma unroll
             for (int k = 0; k < 16; k++) {
                 const __nv_bfloat16 *row = part0 + __shfl_sync(0xffffffffu, my_row[k >> 3], (4 * k + sub) & 31) * (uint64_t)a.cache_ld + 8 * pc;
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                     mypen[eh * pitch + ed] = penalty(a.r1[g * hpg + eh], a.r2[g * hpg + eh], i0 - j0 + ed - (kKeys - 1));
                 }
             }
-            mbar_wait_bounded(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
+            mbar_wait_warp(bars + S_FULL + 8 * grp, (n >> 1) & 1, dead);
             tc_fence_after();
             // the first and one past the last visible key of the row, from j0; a kept prefix inside a window tile as a third bound
             int c_lo = 0, c_hi = kKeys, c_keep = 0;
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         }
         // ---- both groups' sums meet: O = O_0 f_0 + O_1 f_1 relative to the larger maximum, as rows in shared memory
         const int quarter = 2 * grp + half;
-        mbar_wait_bounded(bars + DONE, 0, dead); // all MMAs are done: the tiles are no longer read
+        mbar_wait_warp(bars + DONE, 0, dead); // all MMAs are done: the tiles are no longer read
         tc_fence_after();
         bar_sync(3, 32 * kWarps);
         if (MODE == SOFTMAX) {

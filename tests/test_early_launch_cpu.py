@@ -2,6 +2,7 @@
 memory lets the next one in behind its allocation, and one whose copies may be under way outlives them."""
 import glob
 import os
+import re
 
 import test_step_launch_cpu as steps
 
@@ -19,12 +20,49 @@ def test_pointers_and_order():
             assert body.index("tmem_alloc512") < body.index("__syncthreads()") < body.index("step_next()"), n
 
 
+def enclosing(src, at):
+    """(what stands ahead of it, its text) of every block around a place, the innermost first"""
+    blocks, depth = [], 0
+    for k in range(at - 1, -1, -1):
+        depth += {"}": 1, "{": -1}.get(src[k], 0)
+        if depth < 0:
+            depth = 0
+            end, open_ = k, 0
+            while True:
+                open_ += {"{": 1, "}": -1}.get(src[end], 0)
+                if open_ == 0:
+                    break
+                end += 1
+            blocks.append((src[max(src.rfind(c, 0, k) for c in ";{}") + 1:k], src[k:end]))
+    return blocks
+
+
+def test_who_waits():
+    """A warp whose lanes leave a wait one by one may hand a buffer on that its last lanes still read or write.  So lanes wait for themselves only where one
+    goes on: in a block of lane 0, or where a warp does nothing but issue MMAs, whose lanes meet in every election; any other warp waits by mbar_wait_warp."""
+    alone = warps = 0
+    one = re.compile(r"if \(lane == 0\)\s*$")
+    for p in glob.glob(os.path.join(steps.CSRC, "*.cu*")):
+        if os.path.basename(p) == "tc.cuh":
+            continue
+        s = re.sub(r"//[^\n]*", "", open(p).read())
+        for m in re.finditer(r"mbar_(wait_bounded|try|test)\(", s):
+            alone += 1
+            blocks = enclosing(s, m.start())
+            role = next((text for _, text in blocks if "umma_" in text or "mma_block(" in text), "mbar_arrive(")
+            assert any(one.search(h) for h, _ in blocks) or not re.search(r"mbar_arrive(_cluster)?\(|sts_u|st\.shared|lds_u|tmem_(load|store)", role), (p, s[m.start():m.start() + 80])
+        for m in re.finditer(r"mbar_wait_warp\(", s):
+            warps += 1
+            assert not any(one.search(h) for h, _ in enclosing(s, m.start())), (p, s[m.start():m.start() + 80])
+    assert alone > 20 and warps > 15
+
+
 def test_copies_of_a_kernel_without_tensor_memory():
-    waiting = {n: body for n, (_, body) in steps.kernels().items() if "mbar_wait_lane(" in body}
+    waiting = {n: body for n, (_, body) in steps.kernels().items() if "mbar_wait_warp(" in body and "mbar_expect_tx(" in body and "tmem_alloc512" not in body}
     assert waiting
     for n, body in waiting.items():
         for part in body.split("mbar_expect_tx(")[:-1]:
-            assert "break;" in part[part.rindex("if (!mbar_wait_lane("):], n
+            assert "break;" in part[part.rindex("if (!mbar_wait_warp("):], n
         assert "settle(dead);" in body[body.rindex("bulk_load("):], n
 
 
