@@ -94,7 +94,8 @@ __device__ __forceinline__ float warp_max_f32(float v) {
     return v;
 }
 
-// 128-bit streaming load (weights are read once per token: do not allocate in L1)
+// 128-bit streaming loads (read once per token: do not allocate in L1): of weights, through the path that takes it for granted that nobody writes
+// them while the kernel runs; and of anything
 __device__ __forceinline__ uint4 ldg_stream_u4(const void *p) {
     uint4 r;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -102,11 +103,16 @@ __device__ __forceinline__ uint4 ldg_stream_u4(const void *p) {
                  : "l"(p));
     return r;
 }
+__device__ __forceinline__ uint4 ld_stream_u4(const void *p) {
+    uint4 r;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
 
 // Holds until the kernels before this one are done and their writes are seen: ahead of every access to memory in a kernel that
 // ggb_launch_step launches, run by every thread.  No pointer parameter of such a kernel is __restrict__: what that promises (a const one is
 // not written while the kernel runs, none is reached by another way) does not hold until here, and a compiler that believes it may read
-// through the read-only cache or ahead of this statement.
+// through the read-only cache or ahead of this statement.  For the same reason only weights are read by __ldg and ldg_stream_u4 there.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The same in a kernel that sets itself up ahead of it: barriers, tensor memory, numbers of its arguments, and at most weights, which stand longer
 __device__ __forceinline__ void early_wait() { step_wait(); }

@@ -72,7 +72,7 @@ template <typename E> __device__ __noinline__ float plain_dot(const E *w, const 
 // 16 bytes of a row from column k on: whole, or what lies inside K number by number
 template <typename E, bool VEC> __device__ __forceinline__ uint4 load_piece(const E *row, int64_t k, int64_t K) {
     constexpr int V = 16 / (int)sizeof(E);
-    if (VEC) return k < K ? ldg_stream_u4(row + k) : make_uint4(0, 0, 0, 0); // K is a multiple of V
+    if (VEC) return k < K ? ld_stream_u4(row + k) : make_uint4(0, 0, 0, 0); // K is a multiple of V
     union {
         E e[V];
         uint4 u;

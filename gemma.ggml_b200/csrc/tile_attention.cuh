@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                     const int mp = MAPS == 1 ? 0 : r / PR, pr = MAPS == 1 ? r : r - mp * PR, qi = pr / hpg;
                     x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (it < n_items && pr < n_pairs && d < a.D)
-                        x[u] = __ldg(reinterpret_cast<const float4 *>(a.q + (((t0 + qi) * a.H + (int64_t)g * hpg + (pr - qi * hpg)) * MAPS + mp) * a.D + d));
+                        x[u] = *reinterpret_cast<const float4 *>(a.q + (((t0 + qi) * a.H + (int64_t)g * hpg + (pr - qi * hpg)) * MAPS + mp) * a.D + d);
                 }
 #pragma unroll
                 for (int u = 0; u < 8; u++) {

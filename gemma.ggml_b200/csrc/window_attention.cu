@@ -824,12 +824,12 @@ template <int MAPS> struct tile_finish {
     };
     __device__ __forceinline__ static int coord(int lane, int r) { return 2 * lane + 64 * (r >> 1) + (r & 1); }
     __device__ __forceinline__ void load(reads &rd, int64_t i, int64_t t, int h, int lane) const {
-        rd.sink = fa.sink ? __ldg(fa.sink + h) : 0.f;
+        rd.sink = fa.sink ? fa.sink[h] : 0.f;
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int c = coord(lane, r);
-            rd.gate[r] = fa.gate && c < Dv ? __ldg(fa.gate + t * fa.ldg + (int64_t)h * Dv + c) : 0.f;
-            rd.cs[r] = cs_v && c < Dv ? __ldg(cs_v + i * Dv + c) : 0.f; // pair c / 2: [cos, sin]
+            rd.gate[r] = fa.gate && c < Dv ? fa.gate[t * fa.ldg + (int64_t)h * Dv + c] : 0.f;
+            rd.cs[r] = cs_v && c < Dv ? cs_v[i * Dv + c] : 0.f; // pair c / 2: [cos, sin]
         }
     }
     __device__ __forceinline__ void row(const reads &rd, const float *o1, const float *o2, float m, float l, float l2, int64_t t, int h, int lane) const {

@@ -20,6 +20,29 @@ def test_pointers_and_order():
             assert body.index("tmem_alloc512") < body.index("__syncthreads()") < body.index("step_next()"), n
 
 
+# what they read by loads that take it for granted that nobody writes there while the kernel runs: rows of weight matrices and their scales
+WEIGHTS = {"dense.cu": {"wr + k"}, "moe.cu": {"wr + k", "wu + k"},
+           "prefill.cu": {"dp + 2 * (kb + G * u)", "reinterpret_cast<const __half2 *>(dp + 2 * fkb)"}}
+
+
+def test_only_weights_by_read_only_loads():
+    """What the kernel before writes is read by ordinary loads: a read-only one may be moved ahead of the wait, and may find what was there before."""
+    seen = 0
+    for p in glob.glob(os.path.join(steps.CSRC, "*.cu*")):
+        s, name = re.sub(r"//[^\n]*", "", open(p).read()), os.path.basename(p)
+        if name == "common.cuh" or not re.search(r"\b(early|step)_wait\(\)", s):
+            continue
+        assert "global.nc" not in s, name
+        for m in re.finditer(r"\b(__ldg|ldg_stream_u4)\(", s):
+            depth, k = 1, m.end()
+            while depth:
+                depth += {"(": 1, ")": -1}.get(s[k], 0)
+                k += 1
+            assert s[m.end():k - 1] in WEIGHTS.get(name, ()), (name, s[m.end():k - 1])
+            seen += 1
+    assert seen >= 6
+
+
 def enclosing(src, at):
     """(what stands ahead of it, its text) of every block around a place, the innermost first"""
     blocks, depth = [], 0
