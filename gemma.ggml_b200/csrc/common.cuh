@@ -114,8 +114,9 @@ __device__ __forceinline__ uint4 ld_stream_u4(const void *p) {
 // not written while the kernel runs, none is reached by another way) does not hold until here, and a compiler that believes it may read
 // through the read-only cache or ahead of this statement.  For the same reason only weights are read by __ldg and ldg_stream_u4 there.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The same in a kernel that sets itself up ahead of it: barriers, tensor memory, numbers of its arguments, and at most weights, which stand longer
-__device__ __forceinline__ void early_wait() { step_wait(); }
+// The same in a kernel that ggb_launch_early launches.  Ahead of it such a kernel sets itself up - barriers, tensor memory, numbers of its arguments - and
+// reads weights at most, which stand longer; threads that do not come by here touch memory only behind one that does.
+__device__ __forceinline__ void early_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Behind the wait: once every block has said so, blocks of the next kernel may take what room there is and run up to their own wait.  What
 // they read ahead of it was written before the kernels that came before this one ended.  A kernel with tensor memory says so when it has it:
 // a block of the next kernel that took it first would hold it until this kernel ends.
@@ -166,20 +167,30 @@ static inline float ggb_synth_unit(float sigma) {
 // A layer of 10 such kernels (2048 wide, 16 heads, 8192 in the feed-forward, one token, replayed as a graph): 60.1 us plainly launched,
 // 56.8 like this.  Letting the next one start at once (griddepcontrol.launch_dependents) gives no more: 57.3 behind the wait, 63.5 ahead of
 // it.  Nor does bringing a mat-vec's matrix into L2 before the wait: 63 to 70, the lines are asked for twice.
-// cluster_z: CTAs along z that are one cluster
-template <typename... P, typename... A> cudaError_t ggb_launch_step_cluster(void (*k)(P...), int cluster_z, dim3 grid, dim3 block, size_t smem, A... args) {
+template <typename... P, typename... A>
+cudaError_t ggb_launch_ahead(void (*k)(P...), dim3 cluster, dim3 grid, dim3 block, size_t smem, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = ggb_cuda_stream();
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = (unsigned)cluster_z;
-    cfg.attrs = at, cfg.numAttrs = cluster_z > 1 ? 2 : 1;
+    at[1].val.clusterDim.x = cluster.x, at[1].val.clusterDim.y = cluster.y, at[1].val.clusterDim.z = cluster.z;
+    cfg.attrs = at, cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
+struct ggb_cluster { // CTAs that share their shared memory
+    unsigned x, y, z;
+};
 template <typename... P, typename... A> cudaError_t ggb_launch_step(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
-    return ggb_launch_step_cluster(k, 1, grid, block, smem, args...);
+    return ggb_launch_ahead(k, dim3(1), grid, block, smem, args...);
+}
+template <typename... P, typename... A> cudaError_t ggb_launch_step(void (*k)(P...), ggb_cluster c, dim3 grid, dim3 block, size_t smem, A... args) {
+    return ggb_launch_ahead(k, dim3(c.x, c.y, c.z), grid, block, smem, args...);
+}
+// The same for kernels that set themselves up ahead of their wait (early_wait)
+template <typename... P, typename... A> cudaError_t ggb_launch_early(void (*k)(P...), ggb_cluster c, dim3 grid, dim3 block, size_t smem, A... args) {
+    return ggb_launch_ahead(k, dim3(c.x, c.y, c.z), grid, block, smem, args...);
 }
 #endif
 

@@ -402,18 +402,7 @@ int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, 128);
     if (rc) return rc;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(2 * std::min(pairs, ggb_sm_count() / 2)));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmem;
-    cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at, cfg.numAttrs = 2;
-    GGB_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel, ma, mw, g));
+    GGB_CUDA(ggb_launch_early(gemm_pair_kernel, ggb_cluster{2, 1, 1}, dim3((unsigned)(2 * std::min(pairs, ggb_sm_count() / 2))), dim3(kThreads), kSmem, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -424,7 +413,7 @@ int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_ro
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
-    GGB_CUDA(ggb_launch_step_cluster(gemm_tma_kernel, 1, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
+    GGB_CUDA(ggb_launch_early(gemm_tma_kernel, ggb_cluster{1, 1, 1}, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

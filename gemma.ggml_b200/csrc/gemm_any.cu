@@ -293,18 +293,7 @@ int launch_any(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, 
     if (rc) return rc;
     const int64_t ctas = n_tiles * ((T + g.BT - 1) / g.BT) * g.splits;
     GGB_CHECK_ARG(ctas < (1ll << 31), "linear: %lld tiles", (long long)ctas);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = (unsigned)g.splits, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
-    cfg.attrs = at, cfg.numAttrs = g.splits > 1 ? 2 : 1;
-    GGB_CUDA(cudaLaunchKernelEx(&cfg, kern, g));
+    GGB_CUDA(ggb_launch_early(kern, ggb_cluster{(unsigned)g.splits, 1, 1}, dim3((unsigned)ctas), dim3(kThreads), smem, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

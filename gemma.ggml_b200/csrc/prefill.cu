@@ -1203,19 +1203,9 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     if ((rc = ggb_allow_smem(kfn, kGemmSmem))) return rc;
     // row tiles first: those that share a piece of W run together
     const int rows = A.MT * (pair ? 256 : 128);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)((T + rows - 1) / rows * (pair ? 2 : 1)), (unsigned)((N + A.BN - 1) / A.BN), (unsigned)splits);
-    if (stream) cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(big, sms / 2)));
-    cfg.blockDim = dim3(stream ? kStreamThreads : kGemmThreads);
-    cfg.dynamicSmemBytes = kGemmSmem;
-    cfg.stream = ggb_cuda_stream();
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = 2, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
-    cfg.attrs = at, cfg.numAttrs = pair ? 2 : 1;
-    GGB_CUDA(cudaLaunchKernelEx(&cfg, kfn, maps, A));
+    dim3 grid((unsigned)((T + rows - 1) / rows * (pair ? 2 : 1)), (unsigned)((N + A.BN - 1) / A.BN), (unsigned)splits);
+    if (stream) grid = dim3((unsigned)(2 * std::min<int64_t>(big, sms / 2)));
+    GGB_CUDA(ggb_launch_early(kfn, ggb_cluster{pair ? 2u : 1u, 1, 1}, grid, dim3(stream ? kStreamThreads : kGemmThreads), kGemmSmem, maps, A));
     GGB_LAUNCH_CHECK();
     if (splits > 1) {
         A.resid = resid;

@@ -417,7 +417,7 @@ int ggb_attn_prefill_tiles(const float *q, const void *kcache, const void *vcach
     if (C == 4 && 8 * tiles <= 112 && n_tiles >= 8) C = 8;
     auto kern = C == 8 ? attn_prefill_tile_kernel<8> : C == 4 ? attn_prefill_tile_kernel<4> : C == 2 ? attn_prefill_tile_kernel<2> : attn_prefill_tile_kernel<1>;
     if ((rc = ggb_allow_smem(kern, smem))) return rc;
-    GGB_CUDA(ggb_launch_step_cluster(kern, C, dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv, (unsigned)C), dim3(kThreads), smem, maps, a));
+    GGB_CUDA(ggb_launch_early(kern, ggb_cluster{1, 1, (unsigned)C}, dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv, (unsigned)C), dim3(kThreads), smem, maps, a));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

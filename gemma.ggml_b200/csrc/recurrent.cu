@@ -805,7 +805,7 @@ int recurrence_launch_chunks(rec_args p, bool *done) {
         if (q.a) q.a += t0 * p.ld_a;
         GGB_CUDA(ggb_launch_step(recurrence_prepare_kernel<DP, MODE>, dim3((unsigned)chunks, (unsigned)rows_of), dim3(32 * kTok), 0, q, ws));
         GGB_LAUNCH_CHECK();
-        GGB_CUDA(ggb_launch_step_cluster(k, 1, dim3((unsigned)p.H, (unsigned)slices), dim3(kRecThreads), smem, q, ws, ggb_wait_error_flag()));
+        GGB_CUDA(ggb_launch_early(k, ggb_cluster{1, 1, 1}, dim3((unsigned)p.H, (unsigned)slices), dim3(kRecThreads), smem, q, ws, ggb_wait_error_flag()));
         GGB_LAUNCH_CHECK();
     }
     return rc;

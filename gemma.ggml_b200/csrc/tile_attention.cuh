@@ -611,7 +611,7 @@ template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN
     const int rc = ggb_allow_smem(kfn, smem);
     if (rc) return rc;
     const int TQ = kRows / MAPS / (a.H / a.G);
-    GGB_CUDA(ggb_launch_step_cluster(kfn, 1, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), dim3(kThreads), smem, a, fin));
+    GGB_CUDA(ggb_launch_early(kfn, ggb_cluster{1, 1, 1}, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), dim3(kThreads), smem, a, fin));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }

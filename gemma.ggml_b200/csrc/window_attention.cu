@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(32 * kWarps) window_step_kernel(const float *q
                                                                   const float *cs_v, finish_args da, E *out) {
     constexpr int VN = RowVec<E>::n, RPL = step_tile<LG>::rows_per_load, NL = step_tile<LG>::loads, RT = step_tile<LG>::rows, W = LG * VN;
     __shared__ float s_acc[kWarps][MAPS][W], s_ml[kWarps][MAPS][2], s_out[MAPS][W + 2]; // s_out: this CTA's sums, maximum, denominator
-    early_wait();
+    step_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LG, pc = lane % LG;
     const int h = blockIdx.y, g = h / (H / G);
     const int64_t t = blockIdx.x, i = (int64_t)*pos0 + t;
@@ -1010,7 +1010,7 @@ static int masked_attn_launch(int dt, const float *q, const void *cache, const i
         if (window > 0) n_split = (int)std::min<int64_t>(n_split, ((window + 2 * rows - 2) / rows + (keep + rows - 1) / rows + kWarps - 1) / kWarps);
         const dim3 grid((unsigned)T, (unsigned)H, (unsigned)n_split);
 #define ST_LAUNCH(ET, LG)                                                                                                                            \
-    GGB_CUDA(ggb_launch_step_cluster(window_step_kernel<ET, MAPS, LG>, n_split, grid, dim3(32 * kWarps), 0, q, (const ET *)cache, cld, block_table, block_size, \
+    GGB_CUDA(ggb_launch_step(window_step_kernel<ET, MAPS, LG>, ggb_cluster{1, 1, (unsigned)n_split}, grid, dim3(32 * kWarps), 0, q, (const ET *)cache, cld, block_table, block_size, \
                                      pos0, H, G, D, Dv, window, chunked, keep, softcap, cos_sin_v, da, (ET *)out));
         if (dt == GGB_TYPE_BF16) {
             if (lg == 8) { ST_LAUNCH(__nv_bfloat16, 8) } else if (lg == 16) { ST_LAUNCH(__nv_bfloat16, 16) } else { ST_LAUNCH(__nv_bfloat16, 32) }

@@ -1,5 +1,6 @@
-"""Kernels that set themselves up ahead of their wait for the kernel before them (early_wait): nothing of theirs is __restrict__, a kernel with tensor
-memory lets the next one in behind its allocation, and one whose copies may be under way outlives them."""
+"""Kernels that set themselves up ahead of their wait for the kernel before them (early_wait): what they do ahead of it touches no memory but weights,
+nothing of theirs is __restrict__, a kernel with tensor memory lets the next one in behind its allocation, and one whose copies may be under way
+outlives them.  A kernel that does nothing ahead of its wait is a step kernel (test_step_launch_cpu)."""
 import glob
 import os
 import re
@@ -18,6 +19,60 @@ def test_pointers_and_order():
         assert "__restrict__" not in sig and "step_wait()" not in body, n
         if "tmem_alloc512" in body and "step_next()" in body:
             assert body.index("tmem_alloc512") < body.index("__syncthreads()") < body.index("step_next()"), n
+
+
+def launched():
+    """the kernels that ggb_launch_early launches; a variable stands for every kernel that its declaration and assignments name"""
+    names = set()
+    for p in glob.glob(os.path.join(steps.CSRC, "*.cu*")):
+        s = re.sub(r"//[^\n]*", "", open(p).read())
+        for m in re.finditer(r"ggb_launch_early\(\s*(\w+)", s):
+            if m.group(1) == "void":
+                continue
+            found = [m.group(1)]
+            if not found[0].endswith("_kernel"):
+                ahead = s[s.rindex("auto %s = " % found[0], 0, m.start()):m.start()]
+                found = re.findall(r"\b(\w+_kernel)\b", "".join(re.findall(r"\b%s = ([^;]*);" % found[0], ahead)))
+            assert found, (p, m.group())
+            names |= {(p, n) for n in found}
+    return names
+
+
+def test_which_kernels_and_how():
+    """Every kernel with an early_wait is launched by ggb_launch_early and every one that it launches has one; no other launch asks for the attribute."""
+    ks = early()
+    assert len(ks) >= 8 and launched() == set(ks)
+    for p in glob.glob(os.path.join(steps.CSRC, "*.cu*")):
+        s = open(p).read()
+        assert os.path.basename(p) in ("common.cuh", "decoder.cu") or "cudaLaunchKernelEx" not in s, p
+        for _, name in ks:
+            assert not re.search(name + r"(<[^;{}()]*>)?<<<", s), name
+
+
+TOUCHES = r"->|\)\*\w|\w\s*\[|\*\s*reinterpret_cast|[=(,]\s*\*\s*\w|\b(__ldg|ldg?_stream_u4|load4|store4|tma_load\w*|bulk_load\w*|cp_async\w*|atomic\w*|memcpy)\("
+
+
+def test_what_is_done_ahead_of_the_wait():
+    ks, by_role = early(), set()
+    for (p, name), (_, body) in ks.items():
+        body = re.sub(r"(extern )?__shared__[^;]*;", "", body)
+        at = body.index("early_wait()")
+        if "if (is_a) early_wait()" not in body:  # every thread comes by
+            assert len(enclosing(body, at)) == 0 and not re.search(TOUCHES, body[:at]), (name, re.search(TOUCHES, body[:at]))
+            assert re.search(r"\*dead = 0;|s_dead = 0;", body[:at]), name
+            continue
+        # One lane comes by, ahead of the first copy of what the kernel before wrote.  The others: weights (their codes and scales) and, behind the wait
+        # for the last MMA of a tile, which that copy feeds, results, residual and the operand of the next product
+        by_role.add(name)
+        assert at < min(m.start() for m in re.finditer(r"&maps\.a\b", body))
+        assert all(m.group(1) in ("a", "w") for m in re.finditer(r"&maps\.(\w+)", body))
+        done = [m.start() for m in re.finditer(r"mbar_wait_(?:warp|bounded)\(bars \+ (?:DONE|Q_ACC_FULL)\b", body)]
+        for m in re.finditer(r"\b(load4|store4)\(|A\.geglu \+|A\.gelu\)", body):
+            around = [text for _, text in enclosing(body, m.start())]
+            assert any(d < m.start() and (enclosing(body, d) or [("", body)])[0][1] in around for d in done), (name, m.group())
+        reads = re.findall(r"(?<!reinterpret_cast<)\*\s*reinterpret_cast<([^>]*)>\(([^;]*);", body)
+        assert all("ctl + " in r or "gbase + " in r or "A.geglu + " in r for _, r in reads), (name, reads)
+    assert by_role == {"gemm_quant_kernel", "gemm_quant_stream_kernel"}
 
 
 # what they read by loads that take it for granted that nobody writes there while the kernel runs: rows of weight matrices and their scales
@@ -87,9 +142,3 @@ def test_copies_of_a_kernel_without_tensor_memory():
         for part in body.split("mbar_expect_tx(")[:-1]:
             assert "break;" in part[part.rindex("if (!mbar_wait_warp("):], n
         assert "settle(dead);" in body[body.rindex("bulk_load("):], n
-
-
-def test_every_launch_of_theirs_has_the_attribute():
-    src = "".join(open(p).read() for p in glob.glob(os.path.join(steps.CSRC, "*.cu*")))
-    for _, name in early():
-        assert name + "<<<" not in src, name
