@@ -325,10 +325,6 @@ __global__ void cvt_to_f32_kernel(const E *__restrict__ x, int64_t n, float *__r
     if (i < n) y[i] = to_f32(x[i]);
 }
 
-// Up to here a product stays on the tile kernel: its few steps take no longer than bringing up a tensor-core tile (65 x 65: 8.4 against 10.5 us,
-// fp32 128 x 128: 10.5 against 11.5), and a chain this short is as exact as sums that the tensor cores truncate (K = 65: 5e-8 against 7e-8).
-constexpr int64_t kShortK = 128;
-
 template <typename E>
 int linear_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, int64_t T, float *c, int64_t ldc) {
     if (T <= kVecT) {

@@ -17,6 +17,7 @@
 //
 // What bounds it: fp32, shared memory (written and read: BT = 64: 170 KB a stage, 1330 cycles of 128 bytes); bf16, the loads in flight.
 // 333 x 2816 x 1000 fp32: 98.4 -> 30.5 us (64 x 64 tiles of FMAs).
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -96,9 +97,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
     volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int rank = g.splits > 1 ? (int)cluster_rank() : 0;
-    const int64_t tile = blockIdx.x / g.splits, n_tiles = (g.N + kM - 1) / kM, m_tiles = (g.T + BT - 1) / BT;
+    const int64_t tile = blockIdx.x / g.splits, m_tiles = (g.T + BT - 1) / BT;
     const int64_t t0 = tile % m_tiles * BT, n0 = tile / m_tiles * kM; // those that share rows of W run together
-    (void)n_tiles;
     const int per = (g.kblocks + g.splits - 1) / g.splits, kb0 = min(rank * per, g.kblocks), kb1 = min(kb0 + per, g.kblocks), nkb = kb1 - kb0;
     if (tid == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -265,13 +265,185 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
     }
 }
 
+// ------------------------------------------------------------------------------------------------ the slots of a mixture of experts, bf16
+// C[slot][N] = A[row of the slot][K] W[expert of the slot][N][K]^T for a portion of few slots.  A tile is 128 rows of an expert's matrix, by TMA, x up to 64
+// of its slots, whose rows of A four warps copy through the slot list (rows past the last stay as they are: they give columns that nobody stores).
+// Persistent CTAs; the tile list lies in shared memory.  Every block of 64 along K has an accumulator of its own (four, in turn), which eight warps add up
+// in fp32: K = 8192: error against 64 bits 3e-7, one chain of multiply-adds 9.5e-7, one accumulator of the tensor cores 9.2e-6.
+//
+// Bound by memory.  32 experts, 1408 x 2048: 64 slots 34 us, 256 slots 37 us, 5.0 TB/s of matrices (440 us on the tile kernel; 46 us by gathered rows in
+// gemm.cu's tiles of 128).
+constexpr int kMaxSlots = 511, kMaxTiles = kMaxSlots + kMaxSlots / kMaxBT;
+constexpr int kFewStages = 8, kFewAccs = 4, kCopy = 4, kTmaWarp = kDrain + 1, kFewThreads = 32 * (kTmaWarp + 1 + kCopy);
+constexpr int kLag = 3; // stages whose rows of A are under way
+constexpr uint32_t kFewStage = (kM + kMaxBT) * 128;
+enum { F_FULL = 0, F_EMPTY = 64, F_ACC_FULL = 128, F_ACC_FREE = 160, F_SLOT = 192, F_DEAD = 196, kFewCtl = 256 };
+
+struct few_args {
+    const __nv_bfloat16 *a;
+    int64_t N, lda, ldc;
+    float *c;
+    __nv_bfloat16 *c_act;
+    int act, kblocks, n, max_tiles; // slots; tiles there may be
+    int *wait_error;
+    ggb_moe_groups grp;
+};
+struct few_tile {
+    int row0, expert, rows, BT; // first slot, slots, as a multiple of 16
+};
+
+__global__ void __launch_bounds__(kFewThreads, 1) gemm_few_slots_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ few_args g) {
+    typedef __nv_bfloat16 E;
+    extern __shared__ uint8_t ga_raw[];
+    __shared__ few_tile tiles[kMaxTiles];
+    __shared__ int row_src[kMaxSlots];
+    const uint32_t raw0 = smem_u32(ga_raw), base = (raw0 + 1023u) & ~1023u, bars = base + kFewStages * kFewStage;
+    uint8_t *ctl = ga_raw + (bars - raw0);
+    volatile int *dead = reinterpret_cast<volatile int *>(ctl + F_DEAD);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < kFewStages; s++) {
+            mbar_init(bars + F_FULL + 8 * s, 1 + kCopy);
+            mbar_init(bars + F_EMPTY + 8 * s, 1);
+        }
+        for (int s = 0; s < kFewAccs; s++) {
+            mbar_init(bars + F_ACC_FULL + 8 * s, 1);
+            mbar_init(bars + F_ACC_FREE + 8 * s, kDrain);
+        }
+        *dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) tmem_alloc512(bars + F_SLOT);
+    early_wait();
+    const int n_tiles = min(*g.grp.n_tiles, g.max_tiles);
+    for (int i = tid; i < n_tiles; i += kFewThreads) {
+        const int e = g.grp.tile_expert[i], r0 = g.grp.tile_row0[i], rows = min(kMaxBT, g.grp.offsets[e + 1] - r0);
+        tiles[i] = few_tile{r0, e, rows, (rows + 15) / 16 * 16};
+    }
+    for (int i = tid; i < g.n; i += kFewThreads) row_src[i] = g.grp.row_src ? g.grp.row_src[i] : i;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    step_next();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + F_SLOT), 0);
+    const int cols = (int)((g.N + kM - 1) / kM), total = n_tiles * cols; // item: tile item / cols, rows item % cols * 128 of its matrix
+
+    if (warp == kTmaWarp) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 1;
+            for (int item = blockIdx.x; item < total; item += gridDim.x) {
+                const int row = (int)(tiles[item / cols].expert * g.N) + item % cols * kM;
+                for (int kb = 0; kb < g.kblocks; kb++) {
+                    if (!mbar_wait_bounded(bars + F_EMPTY + 8 * s, ph, dead)) break;
+                    mbar_expect_tx(bars + F_FULL + 8 * s, kM * 128);
+                    tma_load_2d(base + s * kFewStage, &map_w, kb * kBK, row, bars + F_FULL + 8 * s);
+                    if (++s == kFewStages) s = 0, ph ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp > kTmaWarp) {
+        // ---- a thread copies one 16-byte piece of every 16th row; a stage is handed over kLag stages behind its request
+        const int lt = tid - 32 * (kTmaWarp + 1), pc = lt & 7, r0 = lt >> 3;
+        int s = 0, asked = 0, given = 0;
+        uint32_t ph = 1;
+        auto give = [&]() {
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + F_FULL + 8 * (given % kFewStages));
+            given++;
+        };
+        for (int item = blockIdx.x; item < total; item += gridDim.x) {
+            const few_tile t = tiles[item / cols];
+            const E *ap[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) ap[i] = g.a + (int64_t)row_src[t.row0 + min(r0 + 16 * i, t.rows - 1)] * g.lda + 8 * pc;
+            for (int kb = 0; kb < g.kblocks; kb++) {
+                if (!mbar_wait_warp(bars + F_EMPTY + 8 * s, ph, dead)) break;
+#pragma unroll
+                for (int i = 0; i < 4; i++) // rows 16 apart lie at the same place of the swizzle
+                    if (r0 + 16 * i < t.rows) cp_async16(base + s * kFewStage + (kM + r0 + 16 * i) * 128 + ((pc ^ (r0 & 7)) << 4), ap[i] + kb * kBK);
+                cp_async_commit();
+                if (++s == kFewStages) s = 0, ph ^= 1u;
+                if (++asked > kLag) {
+                    cp_async_wait<kLag>();
+                    give();
+                }
+            }
+        }
+        cp_async_wait<0>();
+        while (given < asked) give();
+    } else if (warp == kMmaWarp) {
+        int s = 0;
+        uint32_t ph = 0, q = 0;
+        for (int item = blockIdx.x; item < total; item += gridDim.x) {
+            const uint32_t idesc = umma_idesc(kM, tiles[item / cols].BT);
+            for (int kb = 0; kb < g.kblocks; kb++, q++) {
+                const uint32_t buf = q % kFewAccs, at = base + s * kFewStage;
+                mbar_wait_bounded(bars + F_ACC_FREE + 8 * buf, ((q / kFewAccs) & 1) ^ 1, dead);
+                mbar_wait_bounded(bars + F_FULL + 8 * s, ph, dead);
+                tc_fence_after();
+                umma_ss_k4(tmem + buf * kMaxBT, umma_desc_lo(at, 16), umma_desc_lo(at + kM * 128, 16), idesc, 0);
+                umma_arrive(bars + F_EMPTY + 8 * s);
+                umma_arrive(bars + F_ACC_FULL + 8 * buf);
+                if (++s == kFewStages) s = 0, ph ^= 1u;
+            }
+        }
+    } else {
+        constexpr int kCols = kMaxBT / 2; // of a draining warp: one half of the tile's slots, 32 rows of W
+        const int lq = warp & 3, half = warp >> 2;
+        uint32_t q = 0;
+        for (int item = blockIdx.x; item < total; item += gridDim.x) {
+            const few_tile t = tiles[item / cols];
+            const int hc = t.BT / 2;
+            float sum[kCols];
+#pragma unroll
+            for (int c = 0; c < kCols; c++) sum[c] = 0.f;
+            for (int kb = 0; kb < g.kblocks; kb++, q++) {
+                const uint32_t buf = q % kFewAccs;
+                mbar_wait_warp(bars + F_ACC_FULL + 8 * buf, (q / kFewAccs) & 1, dead);
+                tc_fence_after();
+                const uint32_t col = tmem + ((uint32_t)(lq * 32) << 16) + buf * kMaxBT + half * hc;
+#pragma unroll
+                for (int c0 = 0; c0 < kCols; c0 += 8)
+                    if (c0 < hc) {
+                        uint32_t x[8];
+                        tmem_load8(col + c0, x);
+#pragma unroll
+                        for (int c = 0; c < 8; c++) sum[c0 + c] += __uint_as_float(x[c]);
+                    }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bars + F_ACC_FREE + 8 * buf);
+            }
+            const int64_t n = (int64_t)(item % cols) * kM + lq * 32 + lane;
+#pragma unroll
+            for (int c = 0; c < kCols; c++) {
+                const int r = half * hc + c;
+                if (c >= hc || r >= t.rows || n >= g.N) continue;
+                const int64_t out = (int64_t)(t.row0 + r) * g.ldc + n;
+                if (g.c_act) g.c_act[out] = from_f32<E>(act_f32(sum[c], g.act));
+                else g.c[out] = sum[c];
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        settle(dead);
+        tc_fence_after();
+        tmem_free512(tmem);
+        if (lane == 0 && *dead) *g.wait_error = 1;
+    }
+}
+
 template <typename E>
 int launch_any(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
     constexpr int P = parts_of<E>::n, V = 16 / (int)sizeof(E);
     any_args g{w, a, N, K, T, lda, ldc, c, c_act, act, 0, 1, (int)((K + kBK - 1) / kBK), ggb_wait_error_flag()};
     // the tile and the split of the least estimate.  Cycles of a stage: the bytes that pass through shared memory at 128 a cycle (written once;
     // read for the MMAs: every part of W once, the parts of A as often as they are multiplied), the loading warps' instructions (about 35 a 16-byte
-    // piece and thread), or the bytes from memory at 20 a cycle and SM; a tile: its prologue and its stores
+    // piece and thread), or the bytes from memory at 24 a cycle and SM; a tile: its prologue and its stores
     const int64_t n_tiles = (N + kM - 1) / kM;
     const int sms = ggb_sm_count();
     double best = 0.0;
@@ -302,4 +474,23 @@ int launch_any(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, 
 
 int ggb_gemm_any(int dt, const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
     return dt == GGB_TYPE_BF16 ? launch_any<__nv_bfloat16>(w, N, K, a, lda, T, c, ldc, c_act, act) : launch_any<float>(w, N, K, a, lda, T, c, ldc, c_act, act);
+}
+
+int ggb_gemm_any_grouped(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t n, int n_exp, float *c, int64_t ldc, void *c_act, int act,
+                         const ggb_moe_groups &grp) {
+    typedef __nv_bfloat16 E;
+    GGB_CHECK_ARG(n <= kMaxSlots && K % kBK == 0 && lda % 8 == 0 && ((uintptr_t)w | (uintptr_t)a) % 16 == 0, "moe_linear: %lld slots, K %lld", (long long)n, (long long)K);
+    // the list's tiles, at most: an expert with slots leaves one of its tiles half empty
+    const int max_tiles = (int)(n / kMaxBT + std::min<int64_t>(n, n_exp));
+    const few_args g{(const E *)a, N, lda, ldc, c, (E *)c_act, act, (int)(K / kBK), (int)n, max_tiles, ggb_wait_error_flag(), grp};
+    const int64_t items = (N + kM - 1) / kM * max_tiles;
+    GGB_CHECK_ARG(items < (1ll << 31) && n_exp * N < (1ll << 31), "moe_linear: %lld tiles of %lld rows", (long long)items, (long long)(n_exp * N));
+    CUtensorMap map_w;
+    const size_t smem = 1024 + (size_t)kFewStages * kFewStage + kFewCtl;
+    int rc = ggb_allow_smem(gemm_few_slots_kernel, smem);
+    if (!rc) rc = ggb_tensor_map_bf16(&map_w, w, n_exp * N, K, K, kM);
+    if (rc) return rc;
+    GGB_CUDA(ggb_launch_early(gemm_few_slots_kernel, ggb_cluster{1, 1, 1}, dim3((unsigned)std::min<int64_t>(items, ggb_sm_count())), dim3(kFewThreads), smem, map_w, g));
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
 }
