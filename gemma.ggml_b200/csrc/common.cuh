@@ -19,7 +19,8 @@ bool ggb_is_init();
 cudaStream_t ggb_cuda_stream();
 void ggb_count_launch(int n = 1);
 // What is kept from call to call belongs to the context (ggb_shutdown gives it back; a later ggb_init, of another device perhaps, starts
-// without it): device memory that only grows, its content not kept, and how much dynamic shared memory a kernel may take
+// without it): device memory that only grows, its content not kept, its address good for as long as a graph may hold it, and how much dynamic
+// shared memory a kernel may take
 enum ggb_workspace_id { GGB_WS_GEMM_SPLITS, GGB_WS_MOE_GATHER, GGB_WS_ARGMAX, GGB_WS_RECURRENCE, GGB_WS_COUNT };
 int ggb_workspace(ggb_workspace_id id, size_t bytes, void **p);
 bool ggb_workspace_fits(ggb_workspace_id id, size_t bytes); // it is that large, or may grow: no graph is being captured

@@ -452,7 +452,7 @@ bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc) {
     return T >= 64 && K % 64 == 0 && N % 32 == 0 && ldc % 4 == 0 && N < (1ll << 31) && K < (1ll << 31) && T < (1ll << 31);
 }
 
-// The K-split workspace only grows (one stream, no capture: products of 64 rows and more).
+// The K-split workspace only grows (one stream).
 int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t T, float *c, int64_t ldc, void *c_act, int act) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(w && a && (c || c_act) && ((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");

@@ -2,6 +2,7 @@
 // profiling and CUDA-graph capture.  Replaces the reference's OpenCL wrapper
 // (ref: src/opencl.cpp:19-34 global state, :161-245 setup, :300-348 enqueue/buffers) and its
 // wall-clock profiler (ref: src/profiling.cpp:15-134).
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -41,6 +42,8 @@ struct Context {
     std::map<std::string, ProfEntry> prof;
     void *ws[GGB_WS_COUNT] = {};
     size_t ws_bytes[GGB_WS_COUNT] = {};
+    bool ws_in_graph[GGB_WS_COUNT] = {}; // a capture has been given the present one
+    std::vector<void *> ws_kept;         // those that graphs may hold and larger ones have taken the place of
     std::map<const void *, size_t> smem_allowed;
 };
 
@@ -71,15 +74,27 @@ void ggb_count_launch(int n) {
 const uint16_t *ggb_exp_table_dev() { return g_ctx.exp_table; }
 const uint16_t *ggb_gelu_table_dev() { return g_ctx.gelu_table; }
 int *ggb_wait_error_flag() { return g_ctx.wait_error; }
+// A graph holds the address of the workspace that it was captured with.  Such a one is kept when a larger one takes its place, until ggb_shutdown; the larger
+// one is then at least twice its size, so that all that are kept are together no larger than the one in use.
 int ggb_workspace(ggb_workspace_id id, size_t bytes, void **p) {
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
     if (bytes > g_ctx.ws_bytes[id]) {
-        cudaFree(g_ctx.ws[id]);
-        g_ctx.ws[id] = nullptr, g_ctx.ws_bytes[id] = 0;
+        if (g_ctx.capturing) {
+            ggb_set_error("a workspace of %zu bytes cannot be allocated inside a capture: run the call once ahead of it", bytes);
+            return GGB_ERR_CUDA;
+        }
+        if (g_ctx.ws_in_graph[id]) {
+            g_ctx.ws_kept.push_back(g_ctx.ws[id]);
+            bytes = std::max(bytes, 2 * g_ctx.ws_bytes[id]);
+        } else {
+            cudaFree(g_ctx.ws[id]);
+        }
+        g_ctx.ws[id] = nullptr, g_ctx.ws_bytes[id] = 0, g_ctx.ws_in_graph[id] = false;
         GGB_CUDA(cudaMalloc(&g_ctx.ws[id], bytes));
         g_ctx.ws_bytes[id] = bytes;
     }
+    g_ctx.ws_in_graph[id] |= g_ctx.capturing;
     *p = g_ctx.ws[id];
     return GGB_OK;
 }
@@ -180,6 +195,7 @@ int ggb_shutdown(void) {
     cudaFree(g_ctx.rope_sin);
     cudaFreeHost(g_ctx.wait_error);
     for (void *w : g_ctx.ws) cudaFree(w);
+    for (void *w : g_ctx.ws_kept) cudaFree(w);
     for (auto &kv : g_ctx.prof) {
         for (auto &p : kv.second.pending) {
             cudaEventDestroy(p.first);

@@ -1,5 +1,6 @@
 """What the library keeps between calls belongs to its context: ggb_shutdown gives the memory back, and after another ggb_init every form of the
-products runs as before.  A captured product finds the workspace of an earlier one of its T and N.  Each in a process of its own.  And a wait
+products runs as before.  A captured product finds the workspace of an earlier one of its T and N, and keeps it when a larger one takes its place.
+Each in a process of its own.  And a wait
 that ran out in a kernel is reported once, by the call that next waits for the GPU."""
 import ctypes as C
 import os
@@ -76,8 +77,51 @@ assert (got == again).all() and np.linalg.norm(got - want) < 1e-4 * np.linalg.no
 print("ok")
 """
 
+# graphs of a product cut along K and of a gathered product of experts, behind larger ones that take their workspaces' place
+GROWN = """
+import sys
+sys.path[:0] = sys.argv[1:3]
+import ctypes as C
+import numpy as np
+import gemma_ggml_b200 as G
+from device_util import BF16, as_dt, dev, zeros
+from test_moe_few_slots_gpu import Portion
 
-@pytest.mark.parametrize("program", [SHUTDOWN, CAPTURE], ids=["shutdown", "capture"])
+G.init(0)
+lib, N, K = G.cuda_lib(), 256, 4096
+r = np.random.default_rng(1)
+dw, da, c, c2 = dev(G, as_dt(BF16, r.standard_normal((N, K)))[1]), dev(G, as_dt(BF16, r.standard_normal((1024, K)))[1]), zeros(G, 64 * N * 4), zeros(G, 1024 * N * 4)
+p, big = Portion(G, 150, 4, 8, 64, 256), Portion(G, 2048, 4, 8, 64, 1024, seed=2)
+def small():
+    return lib.ggb_op_linear(BF16, dw.ptr, N, K, da.ptr, K, 64, c.ptr, N) or p.launch()
+G.check(small())
+first = c.download(np.float32), p.c.download(np.float32)
+G.check(lib.ggb_capture_begin())
+rc = big.launch()
+g = C.c_void_p()
+lib.ggb_capture_end(C.byref(g))
+assert rc != 0  # no room, and none can be had there
+graphs = []
+for _ in range(2):
+    G.check(lib.ggb_capture_begin())
+    rc = small()
+    g = C.c_void_p()
+    G.check(lib.ggb_capture_end(C.byref(g)))
+    G.check(rc)
+    graphs.append(g)
+    G.check(lib.ggb_op_linear(BF16, dw.ptr, N, K, da.ptr, K, 1024, c2.ptr, N))
+    G.check(big.launch())
+    G.sync()
+    for g in graphs:
+        c.zero(); p.c.zero()
+        G.check(lib.ggb_graph_launch(g))
+        assert (c.download(np.float32) == first[0]).all() and (p.c.download(np.float32) == first[1]).all()
+G.check(lib.ggb_shutdown())
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("program", [SHUTDOWN, CAPTURE, GROWN], ids=["shutdown", "capture", "grown"])
 def test_in_a_process_of_its_own(program):
     tests = os.path.dirname(os.path.abspath(__file__))
     r = subprocess.run([sys.executable, "-c", program, os.path.dirname(tests), tests], capture_output=True, text=True, timeout=300)
