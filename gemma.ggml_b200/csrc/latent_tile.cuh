@@ -56,13 +56,16 @@ inline bool fits(int R, int Dr, int H, int64_t T, int n_split, const void *qa, c
 }
 
 // 2048 groups of four numbers of a left operand's block: thread tid takes groups tid + 256 u, row = group / 16
+template <bool LOG2E = false> // times log2 e
 __device__ __forceinline__ void store_left(uint32_t dst, int tid, const float4 (&x)[8]) {
 #pragma unroll
     for (int u = 0; u < 8; u++) {
         const int g = tid + 256 * u, r = g >> 4, d = 4 * (g & 15);
         uint32_t h[2], m[2], l[2];
-        split3(pack2(x[u].x, x[u].y), h[0], m[0], l[0]);
-        split3(pack2(x[u].z, x[u].w), h[1], m[1], l[1]);
+        f32x2 v = pack2(x[u].x, x[u].y), w = pack2(x[u].z, x[u].w);
+        if (LOG2E) v = mul2(v, pack2(kLog2e, kLog2e)), w = mul2(w, pack2(kLog2e, kLog2e));
+        split3(v, h[0], m[0], l[0]);
+        split3(w, h[1], m[1], l[1]);
         const uint32_t at = dst + r * 128 + (((d >> 3) ^ (r & 7)) << 4) + (d & 4) * 2;
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(h[0]), "r"(h[1]) : "memory");
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + kPart), "r"(m[0]), "r"(m[1]) : "memory");
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
             for (int c = 0; c < nc; c++) {
                 wait_free();
                 load_ahead(c);
-                store_left(left + (b & 1) * kLeft, tid, x);
+                store_left<true>(left + (b & 1) * kLeft, tid, x); // scores in powers of two
                 load_q(c + 1 < nc ? c + 1 : 0);
                 hand_over();
             }
@@ -287,9 +290,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
                 bar_sync(1, 32 * kWarps);
                 m_true = fmaxf(m_true, mx);
                 float corr = 1.f;
-                const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY); // a maximum is kept until a score exceeds it by 8
+                const bool grow = mx > m + 8.f * kLog2e || (m == -INFINITY && mx > -INFINITY); // a maximum is kept until a score exceeds it by 8 log2 e
                 if (grow) {
-                    corr = expf(m - mx);
+                    corr = exp2f(m - mx);
                     m = mx;
                     l *= corr;
                 }
@@ -320,8 +323,8 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
                         for (int c = 0; c < 16; c++) p[c] = (c0 + c < c_hi && c0 + c >= c_lo) ? p[c] : -INFINITY;
                     }
 #pragma unroll
-                    for (int c = 0; c < 8; c++) { // exp(s - m) = 2^((s - m) log2 e), as in tile_attention.cuh
-                        const float2 t = unpack2(mul2(add2(pack2(p[2 * c], p[2 * c + 1]), pack2(-mm, -mm)), pack2(1.4426950408889634f, 1.4426950408889634f)));
+                    for (int c = 0; c < 8; c++) {
+                        const float2 t = unpack2(add2(pack2(p[2 * c], p[2 * c + 1]), pack2(-mm, -mm)));
                         const f32x2 w = pack2(ex2_approx(t.x), ex2_approx(t.y));
                         sum[c & 1] = add2(sum[c & 1], w);
                         split3(w, ph[8 * hf + c], pm[8 * hf + c], pl[8 * hf + c]);
@@ -352,7 +355,8 @@ __global__ void __launch_bounds__(kThreads, 1) latent_tile_kernel(const args a) 
         }
         mxs[grp * kRows + r] = l;
         bar_sync(1, 32 * kWarps);
-        const float f = m == -INFINITY ? 0.f : expf(m - m_true), l_row = (mxs[r] + mxs[kRows + r]) * f;
+        m_true *= kLn2; // what other parts are compared with
+        const float f = over_e(m, m_true), l_row = (mxs[r] + mxs[kRows + r]) * f;
         float odd = 0.f * l_row; // 0, or NaN when a sum of the row is not finite
         if (grp == 0) mxs[2 * kRows + r] = l_row - l_row == 0.f ? m_true : NAN; // what this row's sums are relative to, where that is known
         bar_sync(1, 32 * kWarps);

@@ -265,6 +265,15 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return r;
 }
 
+// Attention with soft-max counts its scores in powers of two: the queries are multiplied by log2 e, so that a weight is 2^(s - m) by the unit that
+// computes it, as exact as expf of the difference and without its product (which, rounded and left at that, moves a weight by up to
+// |s - m| 2^-24 of itself).
+constexpr double kLog2E = 1.4426950408889634074; // 1 / ln 2
+constexpr float kLog2e = (float)kLog2E, kLog2eRest = (float)(kLog2E - (double)kLog2e), kLn2 = 0.69314718055994530942f;
+// 2^m over e^nat: for sums that are relative to m, counted in powers of two, where others are relative to nat.  What nat's rounding left of m is kept
+// (a multiply-add is exact where its terms nearly cancel).
+__device__ __forceinline__ float over_e(float m, float nat) { return m == -INFINITY ? 0.f : exp2f(fmaf(-nat, kLog2eRest, fmaf(-nat, kLog2e, m))); }
+
 // Two fp32 numbers as three pairs of bf16 numbers whose sums they are: 3 x 8 significant bits hold the 24 of an fp32 number, each
 // remainder is exact (and taken two at a time).  An fp32 x bf16 product is then three bf16 x bf16 products of the tensor cores, each exact before it is added.
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

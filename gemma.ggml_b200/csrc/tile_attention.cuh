@@ -13,8 +13,8 @@
 //
 // Two groups of eight warps take the key tiles alternately, each with its own scores, maximum, sum and output, so the tensor cores work
 // for one group while the other one computes weights; the two are added up at the end.  A warp stages the K tiles, one the V tiles
-// (cp.async, page table per row), one warp issues every MMA.  A maximum is kept until a score exceeds it by 8 (the weights then reach
-// e^8, and sum and output are relative to the kept one all the same), so the output is hardly ever rescaled.
+// (cp.async, page table per row), one warp issues every MMA.  Soft-max scores are counted in powers of two.  A maximum is kept until a score exceeds it by 8 log2 e (the weights
+// then reach e^8, and sum and output are relative to the kept one all the same), so the output is hardly ever rescaled.
 //
 // An infinite number is not the sum of its three parts (inf, NaN, NaN), and a part of a finite query or weight that is zero makes NaN of an
 // infinite key or value; so does a weight of zero of a value that the row does not see.  A row whose sums are not all finite is therefore
@@ -22,7 +22,7 @@
 // arithmetic gives for it.
 //
 // What bounds it: the instructions around the weights (two numbers an instruction where the unit has a packed form: fma.rn.f32x2), then the
-// MMAs.  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft cap, gate: 42 us, 207 TFLOP/s of
+// MMAs.  1024 tokens x 16 heads of 128 (4 key heads) at position 1024, window 1024 + 4 kept positions, soft cap, gate: 41 us, 210 TFLOP/s of
 // the products asked for (57 us with four warps a group and one thread a row, number by number; 785 us by the fp32 CUDA cores, tiles of 32
 // queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 53 us (64 us; 686 us).
 #pragma once
@@ -139,12 +139,11 @@ __device__ __forceinline__ f32x2 sigmoid_fast2(f32x2 z) {
     float x, y, rx, ry;
     asm("min.NaN.f32 %0, %1, %2;\nmax.NaN.f32 %0, %0, %3;" : "=f"(x) : "f"(-v.x), "f"(88.0f), "f"(-88.0f));
     asm("min.NaN.f32 %0, %1, %2;\nmax.NaN.f32 %0, %0, %3;" : "=f"(y) : "f"(-v.y), "f"(88.0f), "f"(-88.0f));
-    const f32x2 a = pack2(x, y), l2e = both(1.4426950408889634f), t = mul2(a, l2e), rest = fma2(a, l2e, mul2(t, both(-1.f)));
-    // log2 e is not the fp32 number: what is missing, 1.9259629911e-8, goes with the rest
-    const f32x2 r = fma2(a, both(1.925963033500312e-8f), rest);
+    const f32x2 a = pack2(x, y), t = mul2(a, both(kLog2e)), rest = fma2(a, both(kLog2e), mul2(t, both(-1.f)));
+    const f32x2 r = fma2(a, both(kLog2eRest), rest); // log2 e is not an fp32 number: what is missing goes with the rest
     const float2 tv = unpack2(t);
     f32x2 e = pack2(ex2_approx(tv.x), ex2_approx(tv.y));
-    e = fma2(mul2(e, r), both(0.6931471805599453f), e);
+    e = fma2(mul2(e, r), both(kLn2), e);
     const f32x2 d = add2(e, both(1.f));
     const float2 dv = unpack2(d);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(dv.x));
@@ -401,8 +400,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                     const int it = it0 + 32 * kWarps * u, r = it / gpr, d = 4 * (it - r * gpr);
                     if (it >= n_items) break;
                     uint32_t h[2], m[2], l[2];
-                    split3(pack2(x[u].x, x[u].y), h[0], m[0], l[0]);
-                    split3(pack2(x[u].z, x[u].w), h[1], m[1], l[1]);
+                    f32x2 q01 = pack2(x[u].x, x[u].y), q23 = pack2(x[u].z, x[u].w);
+                    if (MODE == SOFTMAX) q01 = mul2(q01, pack2(kLog2e, kLog2e)), q23 = mul2(q23, pack2(kLog2e, kLog2e)); // scores in powers of two
+                    split3(q01, h[0], m[0], l[0]);
+                    split3(q23, h[1], m[1], l[1]);
                     const uint32_t at = base + (uint32_t)(d >> 6) * (kRows * 128) + r * 128 + ((((d >> 3) & 7) ^ (r & 7)) << 4) + (d & 4) * 2;
                     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(h[0]), "r"(h[1]) : "memory");
                     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + q_split), "r"(m[0]), "r"(m[1]) : "memory");
@@ -420,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         const bool live = pr < n_pairs;
         const uint32_t lanes = (uint32_t)(32 * lq) << 16;
         const uint32_t ts = tmem + lanes + grp * reg_cols, to = tmem + lanes + o_col + grp * a.Dv;
-        const float inv_cap = a.cap > 0.f ? 1.0f / a.cap : 0.f;
+        const float cap = a.cap * kLog2e, inv_cap = a.cap > 0.f ? kLn2 / a.cap : 0.f;
         float m = -INFINITY, l = 0.f, hpb = 0.f;
         const int pitch = pen_pitch(TQ, hpg);
         float *mypen = pen + grp * hpg * pitch;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 const int c0 = 32 * half + 16 * k;
                 tmem_load16(ts + mp * 64 + c0, reinterpret_cast<uint32_t *>(x[k]));
                 if (MODE != SOFTMAX) continue;
-                if (a.cap > 0.f) soft_cap16(x[k], a.cap, inv_cap);
+                if (a.cap > 0.f) soft_cap16(x[k], cap, inv_cap);
                 if (!whole) masked(x[k], c0, -INFINITY);
 #pragma unroll
                 for (int c = 0; c < 16; c++) mx4[c & 3] = fmaxf(mx4[c & 3], x[k][c]);
@@ -470,9 +471,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 bar_sync(1 + grp, 256);
                 mx = fmaxf(mx, swap[(half ^ 1) * kRows]);
                 float corr = 1.f;
-                const bool grow = mx > m + 8.f || (m == -INFINITY && mx > -INFINITY);
+                const bool grow = mx > m + 8.f * kLog2e || (m == -INFINITY && mx > -INFINITY);
                 if (grow) {
-                    corr = expf(m - mx); // m = -inf: 0
+                    corr = exp2f(m - mx); // m = -inf: 0
                     m = mx;
                     l *= corr;
                 }
@@ -497,10 +498,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
                 const int c0 = 32 * half + 16 * k;
                 float *y = x[k];
                 f32x2 w[8];
-                if (MODE == SOFTMAX) { // exp(s - m) = 2^((s - m) log2 e): the product's rounding moves a weight by less than 2^-24 of the largest one
+                if (MODE == SOFTMAX) {
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
-                        const float2 t = unpack2(mul2(add2(pack2(y[2 * c], y[2 * c + 1]), pack2(-mm, -mm)), pack2(1.4426950408889634f, 1.4426950408889634f)));
+                        const float2 t = unpack2(add2(pack2(y[2 * c], y[2 * c + 1]), pack2(-mm, -mm)));
                         w[c] = pack2(ex2_approx(t.x), ex2_approx(t.y));
                         sum[c & 1] = add2(sum[c & 1], w[c]);
                     }
@@ -546,9 +547,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         float f0 = 1.f, f1 = NT > 1 ? 1.f : 0.f, M = 0.f, L = 1.f;
         if (MODE == SOFTMAX) {
             const float m0 = st[2 * kRows + r], l0 = st[4 * kRows + r] + st[5 * kRows + r], m1 = st[3 * kRows + r], l1 = st[6 * kRows + r] + st[7 * kRows + r];
-            M = fmaxf(m0, m1);
-            f0 = m0 == -INFINITY ? 0.f : expf(m0 - M);
-            f1 = m1 == -INFINITY ? 0.f : expf(m1 - M);
+            M = fmaxf(m0, m1) * kLn2;
+            f0 = over_e(m0, M);
+            f1 = over_e(m1, M);
             L = l0 * f0 + l1 * f1;
             bar_sync(3, 32 * kWarps);
             if (quarter == 0) {
