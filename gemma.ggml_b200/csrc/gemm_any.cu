@@ -5,13 +5,15 @@
 // one token's 32 features is one line.  Sixteen warps bring both operands from memory, K in stages of 64, and write them as swizzled bf16
 // tiles; nothing is asked of sizes or alignment (VEC: 16-byte loads, else numbers one by one).  One warp issues the MMAs, eight drain.
 //
-// fp32: a number is the sum of three bf16 numbers, x = xh + xm + xl (split3, exact), and a product is xh yh + (xh ym + xm yh) + (xh yl + xm ym + xl yh),
-// what is left out is below 2^-24 of it.  The three parts of A lie behind one another as one operand of 3 BT columns, so that a part
+// fp32: a number is the sum of three bf16 numbers, x = xh + xm + xl (exact), and a product is xh yh + (xh ym + xm yh) + (xh yl + xm ym + xl yh),
+// what is left out is below 2^-24 of it.  xm and xl are kept as 2^8 xm and 2^16 xl, and the sums of the two brackets come 2^8 and 2^16 times as
+// large: so a number keeps its bits down to 2^-128, not only to 2^-110 (the smallest bf16 number is 2^-133, and below that the first
+// part is no longer the largest: numbers of 2^-140, which have ten bits, come out to 12 bits).  The three parts of A lie behind one another as one operand of 3 BT columns, so that a part
 // of W is read from shared memory once for all of its products: Wh [Ah Am Al], Wm [Ah Am], Wl [Ah], into columns for xh yh, first-order and
 // second-order terms.  The tensor cores truncate their running sum, so every stage has an accumulator of its own (two, in turn), which the
 // draining warps add to registers, rounding to nearest: the error against 64 bits is smaller than that of one chain of multiply-adds
 // (K = 1000: 1.0e-7 against 5.7e-7).  A result that is not finite is computed once more by plain multiply-adds (an infinity is not the
-// sum of its parts).  (Numbers below 2^-110 lose their last parts to the smallest bf16 number.)
+// sum of its parts).
 //
 // A product of few tiles is cut along K over the CTAs of a cluster (up to 8), whose sums meet in shared memory and are added in order.
 //
@@ -61,6 +63,19 @@ __device__ __forceinline__ void tmem_load8x3(uint32_t ta, uint32_t tb, uint32_t 
                    "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                  : "r"(ta), "r"(tb), "r"(tc)
                  : "memory");
+}
+
+// Two fp32 numbers as three pairs of bf16 numbers: h + 2^-8 m + 2^-16 l, each remainder exact
+__device__ __forceinline__ void split3_scaled(f32x2 v, uint32_t &h, uint32_t &m, uint32_t &l) {
+    const f32x2 minus = pack2(-1.f, -1.f), up = pack2(256.f, 256.f);
+    float2 x = unpack2(v);
+    h = pack_bf16x2(x.x, x.y);
+    v = mul2(fma2(pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, v), up);
+    x = unpack2(v);
+    m = pack_bf16x2(x.x, x.y);
+    v = mul2(fma2(pack2(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u)), minus, v), up);
+    x = unpack2(v);
+    l = pack_bf16x2(x.x, x.y);
 }
 
 // one result in plain arithmetic
@@ -153,8 +168,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
                     for (int u = 0; u < 4; u++)
                         if (i0 + u < NI) {
                             const uint4 x = v[i0 + u];
-                            split3(pack2(__uint_as_float(x.x), __uint_as_float(x.y)), h[u].x, m[u].x, l[u].x);
-                            split3(pack2(__uint_as_float(x.z), __uint_as_float(x.w)), h[u].y, m[u].y, l[u].y);
+                            split3_scaled(pack2(__uint_as_float(x.x), __uint_as_float(x.y)), h[u].x, m[u].x, l[u].x);
+                            split3_scaled(pack2(__uint_as_float(x.z), __uint_as_float(x.w)), h[u].y, m[u].y, l[u].y);
                         }
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
@@ -222,7 +237,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
                     if (P == 3) tmem_load8x3(col + c0, col + BT + c0, col + 2 * BT + c0, x, y, z);
                     else tmem_load8(col + c0, x);
 #pragma unroll
-                    for (int c = 0; c < 8; c++) sum[c0 + c] += P == 3 ? __uint_as_float(x[c]) + (__uint_as_float(y[c]) + __uint_as_float(z[c])) : __uint_as_float(x[c]);
+                    for (int c = 0; c < 8; c++) sum[c0 + c] += P == 3 ? fmaf(fmaf(__uint_as_float(z[c]), 0x1p-8f, __uint_as_float(y[c])), 0x1p-8f, __uint_as_float(x[c])) : __uint_as_float(x[c]);
                 }
             tc_fence_before();
             __syncwarp();

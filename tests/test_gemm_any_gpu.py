@@ -55,6 +55,20 @@ def test_activations(gpu, dt, act):
     assert rel(from_dt(dt, y, (T, N)), want) < (2.0 ** -8 if dt == BF16 else 2e-6)
 
 
+def test_small_numbers_keep_their_bits(gpu):
+    """fp32 numbers around 2^-110, 2^-120 and 2^-128, whose bf16 parts the smallest bf16 number would cut off, times large ones."""
+    T, N, K = 40, 130, 300
+    r = np.random.default_rng(8)
+    w, a = f32(r.standard_normal((N, K))), f32(r.standard_normal((T, K)))
+    c, out = zeros(gpu, T * N * 4), {}
+    for e in (0, -110, -120, -128):
+        ae, we = np.ldexp(a, e), np.ldexp(w, -e // 2)
+        gpu.check(gpu.cuda_lib().ggb_op_linear(F32, dev(gpu, we).ptr, N, K, dev(gpu, ae).ptr, K, T, c.ptr, N))
+        out[e] = c.download(np.float32).reshape(T, N)
+        assert rel(out[e].astype(np.float64), ae.astype(np.float64) @ we.astype(np.float64).T) < TOL, e
+    assert np.array_equal(np.ldexp(out[-110], 55), out[0])
+
+
 @pytest.mark.parametrize("dt", [BF16, F32])
 def test_numbers_that_are_not_finite(gpu, dt):
     """Infinities and NaN, and the largest numbers (which round up to an infinity in bf16), give what plain multiply-adds give."""
