@@ -12,8 +12,8 @@
 // of W is read from shared memory once for all of its products: Wh [Ah Am Al], Wm [Ah Am], Wl [Ah], into columns for xh yh, first-order and
 // second-order terms.  The tensor cores truncate their running sum, so every stage has an accumulator of its own (two, in turn), which the
 // draining warps add to registers, rounding to nearest: the error against 64 bits is smaller than that of one chain of multiply-adds
-// (K = 1000: 1.0e-7 against 5.7e-7).  A result that is not finite is computed once more by plain multiply-adds (an infinity is not the
-// sum of its parts).
+// (K = 1000: 1.0e-7 against 5.7e-7).  A result that is not finite is computed once more by plain multiply-adds (plain_tile: an infinity is
+// not the sum of its parts).
 //
 // A product of few tiles is cut along K over the CTAs of a cluster (up to 8), whose sums meet in shared memory and are added in order.
 //
@@ -78,11 +78,58 @@ __device__ __forceinline__ void split3_scaled(f32x2 v, uint32_t &h, uint32_t &m,
     l = pack_bf16x2(x.x, x.y);
 }
 
-// one result in plain arithmetic
-template <typename E> __device__ __noinline__ float plain_dot(const E *w, const E *a, int64_t K) {
-    float s = 0.f;
-    for (int64_t k = 0; k < K; k++) s = fmaf(to_f32(w[k]), to_f32(a[k]), s);
-    return s;
+// The results of a tile that are not finite (odd: of a row of W, a bit a token) once more by plain multiply-adds, by all threads: 4 x 4 results a thread
+// of the first 16 warps, K in steps of 32 through shared memory.  smem: where the stages were.  A portion of NaN takes 150 us where
+// finite numbers take 22 (333 x 1408 x 1000; each result by a walk of its own along K: 1040).
+template <typename E, typename PUT> __device__ __noinline__ void plain_tile(const any_args &g, int64_t n0, int64_t t0, int BT, const uint64_t *odd, float *smem, PUT put) {
+    constexpr int KB = 32, PITCH = KB + 1, NL = ((kM + kMaxBT) * KB + kThreads - 1) / kThreads;
+    const int tid = threadIdx.x, rg = tid & 31, cg = tid >> 5;
+    float *sw = smem, *sa = smem + kM * PITCH, acc[4][4], next[NL];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    auto fetch = [&](int64_t k0) {
+#pragma unroll
+        for (int u = 0; u < NL; u++) {
+            const int i = tid + kThreads * u, r = i / KB;
+            const int64_t k = k0 + i % KB, row = r < kM ? n0 + r : t0 + r - kM;
+            next[u] = 0.f;
+            if (r < kM + BT && k < g.K && row < (r < kM ? g.N : g.T))
+                next[u] = to_f32(r < kM ? static_cast<const E *>(g.w)[row * g.K + k] : static_cast<const E *>(g.a)[row * g.lda + k]);
+        }
+    };
+    fetch(0);
+    for (int64_t k0 = 0; k0 < g.K; k0 += KB) {
+        const int ks = (int)min((int64_t)KB, g.K - k0);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < NL; u++) {
+            const int i = tid + kThreads * u;
+            if (i < (kM + BT) * KB) smem[i / KB * PITCH + i % KB] = next[u];
+        }
+        __syncthreads();
+        fetch(k0 + KB);
+        if (cg < 16)
+            for (int k = 0; k < ks; k++) {
+                float w[4], x[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) w[i] = sw[(rg + 32 * i) * PITCH + k], x[i] = cg + 16 * i < BT ? sa[(cg + 16 * i) * PITCH + k] : 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] = fmaf(w[i], x[j], acc[i][j]);
+            }
+    }
+    if (cg < 16)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int row = rg + 32 * i;
+            const uint64_t again = odd[row] | odd[kM + row];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (again >> (cg + 16 * j) & 1) put(cg + 16 * j, row, acc[i][j]);
+        }
 }
 
 // 16 bytes of a row from column k on: whole, or what lies inside K number by number
@@ -104,6 +151,7 @@ template <typename E, bool VEC>
 __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_constant__ any_args g) {
     constexpr int P = parts_of<E>::n, SPA = parts_of<E>::stages_per_acc, STAGES = parts_of<E>::stages;
     extern __shared__ uint8_t ga_raw[];
+    __shared__ uint64_t s_odd[P == 3 ? 2 * kM : 1]; // of a draining thread: tokens of its row whose results are not finite
     const uint32_t raw0 = smem_u32(ga_raw), base = (raw0 + 1023u) & ~1023u;
     uint8_t *gbase = ga_raw + (base - raw0);
     const int BT = g.BT;
@@ -245,12 +293,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
         }
     }
     __syncthreads(); // every MMA and every write of a stage is done
+    auto put = [&](int c, int row, float v) {
+        const int64_t at = (t0 + c) * g.ldc + n0 + row;
+        if (g.c_act) static_cast<E *>(g.c_act)[at] = from_f32<E>(act_f32(v, g.act));
+        else g.c[at] = v;
+    };
+    uint64_t odd = 0;
     auto store = [&](int c, float v) { // token column c of the tile
-        const int64_t t = t0 + c, n = n0 + row;
-        if (t >= g.T || n >= g.N) return;
-        if (!isfinite(v) && !*dead) v = plain_dot(static_cast<const E *>(g.w) + n * g.K, static_cast<const E *>(g.a) + t * g.lda, g.K);
-        if (g.c_act) static_cast<E *>(g.c_act)[t * g.ldc + n] = from_f32<E>(act_f32(v, g.act));
-        else g.c[t * g.ldc + n] = v;
+        if (t0 + c >= g.T || n0 + row >= g.N) return;
+        if (P == 3 && !isfinite(v)) odd |= 1ull << c;
+        put(c, row, v);
     };
     if (g.splits > 1) { // the ranks' sums, [token][row], in order
         float *mine = reinterpret_cast<float *>(gbase);
@@ -277,6 +329,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_any_kernel(const __grid_cons
         tc_fence_after();
         tmem_free512(tmem);
         if (lane == 0 && *dead) *g.wait_error = 1;
+    }
+    if constexpr (P == 3) { // in bf16 the tensor cores' sums are plain arithmetic's
+        if (__syncthreads_or(odd != 0 && !*dead)) {
+            if (warp < kDrain) s_odd[half * kM + row] = odd;
+            plain_tile<E>(g, n0, t0, BT, s_odd, reinterpret_cast<float *>(gbase), put);
+        }
     }
 }
 

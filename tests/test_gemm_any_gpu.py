@@ -89,3 +89,24 @@ def test_numbers_that_are_not_finite(gpu, dt):
     assert np.array_equal(np.sign(got[np.isinf(want)]), np.sign(want[np.isinf(want)]))
     ok = np.isfinite(want)
     assert (np.abs(got[ok] - want[ok]) <= 1e-5 * np.abs(av[:, None, :] * wv[None]).sum(2)[ok] + 1e-6).all()
+
+
+def test_a_portion_of_nan_takes_about_as_long(gpu):
+    """Results that are not finite are computed once more together: a few times the time of finite ones (a thread a result was several hundred times)."""
+    import time
+    T, N, K = 333, 1408, 1000
+    r = np.random.default_rng(4)
+    w, a, lib = dev(gpu, f32(r.standard_normal((N, K)))), f32(r.standard_normal((T, K))), gpu.cuda_lib()
+    c, took = zeros(gpu, T * N * 4), []
+    for x in (a, np.full_like(a, np.nan)):
+        d = dev(gpu, x)
+        for n in (2, 20):
+            gpu.sync()
+            t = time.perf_counter()
+            for _ in range(n):
+                gpu.check(lib.ggb_op_linear(F32, w.ptr, N, K, d.ptr, K, T, c.ptr, N))
+            gpu.sync()
+        took.append(time.perf_counter() - t)
+        assert np.isnan(c.download(np.float32)).all() == np.isnan(x).all()
+    assert took[1] < 20 * took[0], took
+    print("us: finite %.1f, NaN %.1f" % (took[0] / 20 * 1e6, took[1] / 20 * 1e6))
