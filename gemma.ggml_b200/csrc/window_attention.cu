@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(32 * kWarps) window_step_kernel(const float *q
     for (int64_t n = (int64_t)blockIdx.z * kWarps + warp;; n += kWarps * (int64_t)gridDim.z) {
         const int64_t j0 = n < n_kt ? RT * n : jlo + RT * (n - n_kt), j_last = n < n_kt ? n_keep - 1 : i;
         if (j0 > j_last) break; // only behind the last tile of the window: the kept tiles hold a position each
-        const int64_t jr = min(j0 + (lane < RT ? lane : RT - 1), j_last); // a row past the last visible one repeats it with weight 0
+        const int64_t jr = min(j0 + (lane < RT ? lane : RT - 1), j_last); // a row past the last visible one repeats it, its score not counted, its values set to zero
         const int64_t my_row = ((int64_t)table[jr / B] * B + jr % B) * cache_ld;
         RowVec<E> kx[MAPS][NL], vx[NL];
         auto load_v = [&]() {
@@ -534,6 +534,10 @@ __global__ void __launch_bounds__(32 * kWarps) window_step_kernel(const float *q
             m[a] = m_new;
         }
         if (MAPS != 1) load_v();
+        if (j0 + RT - 1 > j_last) // 0 times an infinity would be a NaN
+#pragma unroll
+            for (int b = 0; b < NL; b++)
+                if (j0 + b * RPL + sub > j_last) vx[b].raw = make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int b = 0; b < NL; b++)
 #pragma unroll

@@ -60,3 +60,29 @@ def test_steps(gpu, dt, maps, D, Dv, H, kv, T, pos, window, keep):
     # sums of up to 2200 fp32 terms; a difference of two maps divided by its root mean square magnifies their error a little
     tol = 2.0 ** -8 if dt == BF16 else 5e-6
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < tol
+
+
+@pytest.mark.parametrize("dt", [BF16, F32])
+@pytest.mark.parametrize("D,pos", [(64, 0), (64, 12), (128, 31), (128, 700), (256, 21)])
+def test_infinite_values(gpu, dt, D, pos):
+    """An infinite value at the newest position (which ends a tile that is not whole) and one at the first: infinities where they are, the rest as ever."""
+    if dt == F32 and D == 256:
+        D = 128
+    r = np.random.default_rng(pos)
+    n, H = pos + 1, 2
+    c = r.standard_normal((-(-n // PAGE) * PAGE, 2 * D))
+    c[n - 1, D + 3] = c[0, D + 6] = np.inf
+    c[n - 1, D + 5] = -np.inf
+    cv, cr = as_dt(dt, c)
+    q = f32(r.standard_normal((1, H, D)) * D ** -0.5)
+    lib = gpu.cuda_lib()
+    out, scratch = zeros(gpu, H * D * size_of(dt)), zeros(gpu, lib.ggb_window_attn_scratch_bytes(H))
+    gpu.check(lib.ggb_op_masked_attn_gated(dt, dev(gpu, q).ptr, dev(gpu, cr).ptr, dev(gpu, i32(np.arange(len(c) // PAGE))).ptr, PAGE, dev(gpu, i32([pos, 0, 0, 0])).ptr, 1, H, 1,
+                                           D, D, 0, 0, 0.0, None, None, 0, out.ptr, scratch.ptr))
+    got = from_dt(dt, out, (H, D))
+    assert (got[:, [3, 6]] == np.inf).all() and (got[:, 5] == -np.inf).all()
+    V = np.where(np.isinf(cv[:n, D:]), 0, cv[:n, D:])
+    s = np.einsum("jd,hd->hj", cv[:n, :D], q[0].astype(np.float64))
+    want = np.einsum("hj,jd->hd", np.exp(s - s.max(1, keepdims=True)) / np.exp(s - s.max(1, keepdims=True)).sum(1, keepdims=True), V)
+    rest = [d for d in range(D) if d not in (3, 5, 6)]
+    assert np.linalg.norm(got[:, rest] - want[:, rest]) / np.linalg.norm(want[:, rest]) < (2.0 ** -8 if dt == BF16 else 5e-6)
