@@ -1280,10 +1280,12 @@ int ggb_op_attn_prefill(const float *q, const void *kcache, const void *vcache, 
                         float *out, void *out_bf16) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(q && kcache && vcache && (out || out_bf16) && T > 0 && d % 8 == 0 && d <= 256 && H % Hkv == 0, "bad attn_prefill args");
-    if (ggb_attn_prefill_fits(q, kcache, vcache, T, pos0, H, Hkv, d, out, out_bf16))
+    // GGB_PREFILL_ATTN_SIMPLE: a warp a (token, head), with GGB_PREFILL_ATTN_GH4 a warp a token and four heads, whatever the sizes
+    const bool simple = getenv("GGB_PREFILL_ATTN_SIMPLE") != nullptr;
+    if (!simple && ggb_attn_prefill_fits(q, kcache, vcache, T, pos0, H, Hkv, d, out, out_bf16))
         return ggb_attn_prefill_tiles(q, kcache, vcache, T, pos0, H, Hkv, d, out, out_bf16);
     const int n_kv_max = pos0 + (int)T;
-    if ((H / Hkv) % 4 == 0 && !getenv("GGB_PREFILL_ATTN_SIMPLE")) { // MQA / GQA: one CTA per (token, 4 heads of one KV head)
+    if ((H / Hkv) % 4 == 0 && !simple) { // MQA / GQA: one CTA per (token, 4 heads of one KV head)
         const size_t smem4 = ((size_t)4 * n_kv_max + 4 * 4 * 256 + 16) * 4 + 16 * 8;
         GGB_CHECK_ARG(smem4 <= 200 * 1024, "attn_prefill: context %d too long for the score buffer", n_kv_max);
         if (smem4 > 48 * 1024) GGB_CUDA(cudaFuncSetAttribute(attn_prefill_gqa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4));

@@ -69,3 +69,18 @@ def test_numbers_that_are_not_finite(gpu):
     rest[7, 0] = False
     rest[40:, 2:, 3] = False
     assert (np.abs(got[rest] - clean[rest]) <= 2e-3).all()  # rows computed once more round every weight to fp16 behind its division
+
+
+def test_the_switch_to_plain_kernels(gpu, monkeypatch):
+    """GGB_PREFILL_ATTN_SIMPLE (and with it GGB_PREFILL_ATTN_GH4) picks the kernels without tensor cores for sizes that the tiles take, too."""
+    r = np.random.default_rng(3)
+    q = f32(r.standard_normal((130, 8, 128)) * 128 ** -0.5)
+    k, v = (r.standard_normal((130, 1, 128)).astype(np.float16) for _ in range(2))
+    want, size = plain(q, k, v, 0)
+    tiles, _ = run(gpu, q, k, v, 0)
+    monkeypatch.setenv("GGB_PREFILL_ATTN_SIMPLE", "1")
+    simple, _ = run(gpu, q, k, v, 0)
+    monkeypatch.setenv("GGB_PREFILL_ATTN_GH4", "1")
+    four, _ = run(gpu, q, k, v, 0)
+    for got in (simple, four):  # a weight's exponent and the weight are fp16 numbers
+        assert (np.abs(got - want) <= 2.0 ** -7 * size).all() and not np.array_equal(got, tiles)
