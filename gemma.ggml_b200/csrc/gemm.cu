@@ -30,6 +30,7 @@ constexpr int kThreads = 384; // warp 0: TMA, 1: MMA, 2: tensor memory, 4..11: e
 constexpr uint32_t kRing = 192 * 1024, kTurn = 8 * 4096;
 constexpr int kMaxStages = 8, kMaxGroups = 256; // groups whose first tiles are kept in shared memory
 constexpr size_t kSmem = 1024 + kRing + kTurn + 256;
+static_assert(kSmem >= kOneCtaSmem, "pairs of CTAs");
 enum { FULL = 0, EMPTY = 64, ACC_FULL = 128, ACC_FREE = 144, SLOT = 160, DEAD = 168 };
 
 struct gemm_args {

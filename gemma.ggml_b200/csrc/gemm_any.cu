@@ -533,7 +533,8 @@ int launch_any(const void *w, int64_t N, int64_t K, const void *a, int64_t lda, 
     }
     const bool vec = K % V == 0 && lda % V == 0 && ((uintptr_t)w | (uintptr_t)a) % 16 == 0;
     auto kern = vec ? gemm_any_kernel<E, true> : gemm_any_kernel<E, false>;
-    const size_t smem = 1024 + (size_t)parts_of<E>::stages * std::max<size_t>(stage_bytes<E>(g.BT), (size_t)g.BT * kM * 4 / parts_of<E>::stages) + kCtl;
+    size_t smem = 1024 + (size_t)parts_of<E>::stages * stage_bytes<E>(g.BT) + kCtl;
+    if (g.splits > 1) smem = std::max(smem, kOneCtaSmem);
     const int rc = ggb_allow_smem(kern, smem);
     if (rc) return rc;
     const int64_t ctas = n_tiles * ((T + g.BT - 1) / g.BT) * g.splits;

@@ -48,6 +48,7 @@ constexpr int kWorkWarps = 16, kTmaWarp = 16, kMmaWarp = 17, kCodesWarp = 18, kG
 constexpr uint32_t kRing = 224 * 1024;
 constexpr int kMaxStages = 8;
 constexpr size_t kGemmSmem = 1024 + kRing + 512;
+static_assert(kGemmSmem >= kOneCtaSmem, "pairs of CTAs");
 constexpr uint32_t kTiles = 256 * 128; // bytes of the buffers of dequantised weights, one a group
 constexpr int kMaxCodeStages = 16;
 enum { FULL = 0, FREE = 64, C_FULL = 128, C_FREE = 256, DONE = 384, SLOT = 392, DEAD = 400, TABLE_FULL = 408 }; // FULL, FREE: of a K block, by its stage of A

@@ -17,6 +17,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "prefill_attention.cuh"
 #include "tc.cuh"
@@ -407,7 +409,6 @@ int ggb_attn_prefill_tiles(const float *q, const void *kcache, const void *vcach
     if (!rc) rc = ggb_tensor_map_bf16(&maps.v, vcache, n_kv, ld, ld, kKeys);
     if (rc) return rc;
     const attn_args a{q, (const __half *)kcache, (const __half *)vcache, (int)T, pos0, H, Hkv, d, ggb_exp_table_dev(), out, (__nv_bfloat16 *)out_bf16, ggb_wait_error_flag()};
-    const size_t smem = smem_bytes(d);
     const int TQ = kRows / (H / Hkv), tiles = (int)((T + TQ - 1) / TQ) * Hkv, n_tiles = (int)((n_kv + kKeys - 1) / kKeys);
     // CTAs that share the key tiles of 128 rows, and the adding up: up to 4 while there are SMs for them (8 heads of 256 over one: 512 tokens 25 us by
     // one, 22, 18; 128 tokens 17, 16, 16); 8 for many keys and so few rows that clusters of 8 find room at once (64 tokens behind 1000 positions: 43, 29,
@@ -415,6 +416,7 @@ int ggb_attn_prefill_tiles(const float *q, const void *kcache, const void *vcach
     int C = 1;
     while (C < 4 && 2 * C * tiles <= ggb_sm_count() && n_tiles >= (d > 128 ? 2 : 3)) C *= 2;
     if (C == 4 && 8 * tiles <= 112 && n_tiles >= 8) C = 8;
+    const size_t smem = C > 1 ? std::max(smem_bytes(d), kOneCtaSmem) : smem_bytes(d);
     auto kern = C == 8 ? attn_prefill_tile_kernel<8> : C == 4 ? attn_prefill_tile_kernel<4> : C == 2 ? attn_prefill_tile_kernel<2> : attn_prefill_tile_kernel<1>;
     if ((rc = ggb_allow_smem(kern, smem))) return rc;
     GGB_CUDA(ggb_launch_early(kern, ggb_cluster{1, 1, (unsigned)C}, dim3((unsigned)((T + TQ - 1) / TQ), (unsigned)Hkv, (unsigned)C), dim3(kThreads), smem, maps, a));

@@ -69,6 +69,10 @@ __device__ __forceinline__ void settle(volatile int *dead) {
         for (int i = 0; i < 500; i++) __nanosleep(1000000);
 }
 
+// Shared memory of which an SM has room for one CTA.  The CTAs of a cluster that allocate tensor memory ask for at least this much: with two on an SM, a
+// cluster could wait on one SM for the tensor memory that another one holds, which on a second SM waits for what this one holds.
+constexpr size_t kOneCtaSmem = 116 * 1024;
+
 // Shared-memory matrix operands, 128-byte swizzle: rows of 128 bytes, 16-byte piece c of row r at place c ^ (r & 7), 1024-byte atoms
 // of 8 rows that follow one another.  K-major: rows are M / N.  MN-major: rows are K, a row holds 64 numbers of M / N, and lbo is the
 // distance between blocks of 64 numbers of M / N.  A descriptor's upper half (distance of the atoms, version, swizzle) is the same for

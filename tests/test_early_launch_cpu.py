@@ -142,3 +142,24 @@ def test_copies_of_a_kernel_without_tensor_memory():
         for part in body.split("mbar_expect_tx(")[:-1]:
             assert "break;" in part[part.rindex("if (!mbar_wait_warp("):], n
         assert "settle(dead);" in body[body.rindex("bulk_load("):], n
+
+
+def test_clusters_with_tensor_memory():
+    """Their CTAs ask for so much shared memory that an SM has room for one: two clusters never hold what the other one waits for."""
+    seen = 0
+    for p in glob.glob(os.path.join(steps.CSRC, "*.cu*")):
+        s = re.sub(r"//[^\n]*", "", open(p).read())
+        for m in re.finditer(r"ggb_launch_early\(\s*\w+, ggb_cluster\{([^}]*)\},", s):
+            if "tmem_alloc512" not in s or m.group(1) == "1, 1, 1":
+                continue
+            args, depth, last, k = [], 0, m.end(), m.end()
+            while depth >= 0:  # grid, block, shared memory, the kernel's own
+                depth += {"(": 1, ")": -1, "{": 1, "}": -1}.get(s[k], 0)
+                if s[k] == "," and not depth:
+                    args.append(s[last:k].strip())
+                    last = k + 1
+                k += 1
+            smem = args[2]
+            assert re.search(r"%s >= kOneCtaSmem|\b%s = [^;]*kOneCtaSmem" % (smem, smem), s), (p, smem)
+            seen += 1
+    assert seen == 4
