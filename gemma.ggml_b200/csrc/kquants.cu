@@ -14,8 +14,8 @@
 // chains sums[l] += d * aux32[l] advanced super-block by super-block, sumf -= dmin * sumi, then sumf += sums[0..7].
 // Results are bit-identical to the scalar code (tests compare bits with oracle/_ref, the reference's own source).
 //
-// Weights and activations stay in ggml's AoS blocks (144 / 210 / 292 B): at 4.5 / 6.56 bits per weight a row of a
-// super-block is one 128 B + one 16 B line, so the warp's loads are already contiguous and a repack buys nothing.
+// That form takes weights and activations as they come, in ggml's AoS blocks (144 / 210 / 292 B).  Weights that stay on the device are
+// re-laid out once and multiplied by integer tensor cores (below: packed form).
 #include <algorithm>
 
 #include "common.cuh"

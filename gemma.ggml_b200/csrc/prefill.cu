@@ -1144,8 +1144,8 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
     A.gelu = ggb_gelu_table_dev();
     // The tile (of one CTA or of a pair), and the CTAs along K, with the least estimated time (cycles).  A K block takes what its MMAs (130 each by a
     // pair of 256 columns, 100 of fewer, 80 by one CTA of 128, 40 of 64, and 100 for the wait and the commit), the bytes through shared memory
-    // (written by TMA, read and written by the dequantisation, read for the MMAs), the bytes from L2 or the dequantisation take (2.7 a row: 32
-    // weights are 170 instructions of one lane), and no less than a group's way with it, 2000, over the groups.  The constants choose the
+    // (written by TMA, read and written by the dequantisation, read for the MMAs), the bytes from L2 or the dequantisation take (2.7 a row: a fit, as
+    // all of these), and no less than a group's way with it, 2000, over the groups.  The constants choose the
     // fastest of all tiles for 28 shapes from 16 x 2048 x 2048 to 512 x 65536 x 2048 and 2048 x 16384, all of which were timed.
     auto stages_of = [&](bool pr, int MT, int br, int *codes) { // of A rows (a K block's also tell of the group's buffer: no fewer than groups), of codes
         const int cs = br == 32 ? kMaxCodeStages : MT == 1 ? 12 : pr ? 4 : 8;
@@ -1176,7 +1176,7 @@ static int gemm_launch(int n, const ggb_weight *const *w, const void *a_bf16, in
                     }
                 }
     // Persistent pairs with tiles of 256 x 256, which dequantise every weight once per 256 tokens and store a tile behind the next one's MMAs: 800 cycles a K
-    // block.  gate | up, 2 x 16384 x 2048 Q8_0: 256 tokens 40 us (52), but 512 tokens 72 us (68 in tiles of 512 rows); 65536 x 2048, 512 tokens 123 us (144)
+    // block.  gate | up, 2 x 16384 x 2048 Q8_0: 256 tokens 40 us (52), but 512 tokens 72 us (65 in tiles of 512 rows); 65536 x 2048, 512 tokens 123 us (144)
     const int64_t big = (N + 255) / 256 * ((T + 255) / 256);
     const bool stream = geglu ? T <= 256 : pieces == 1 && T > 256 && (double)((big + sms / 2 - 1) / (sms / 2)) * kblocks * 800.0 + 14000.0 < best;
     if (stream) pair = true, splits = 1, A.MT = 1, A.BN = 256;

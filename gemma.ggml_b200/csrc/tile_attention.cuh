@@ -131,7 +131,8 @@ __device__ __forceinline__ float sigmoid_fast(float z) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
-// the same for two numbers.  exp(x) = 2^t (1 + ln 2 r), t = x log2 e rounded, r what the rounding left: as exact as expf.  -z is kept within
+// the same for two numbers.  exp(x) = 2^t (1 + ln 2 r), t = x log2 e rounded, r what the rounding left (rms error 6e-8; expf 4e-8,
+// t alone 1.2e-6 at 87).  -z is kept within
 // +-88 (beyond, the result is 0 or 1 to 32 bits).
 __device__ __forceinline__ f32x2 sigmoid_fast2(f32x2 z) {
     auto both = [](float v) { return pack2(v, v); };

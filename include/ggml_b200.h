@@ -267,11 +267,13 @@ int ggb_op_attn_prefill(const float *q, const void *kcache, const void *vcache, 
 /* ------------------------------------------------------------------ plain bf16 / fp32 matrices (csrc/dense.cu)
  * Operators of models whose matrices are stored unquantised, row-major [out][in] and applied as W x.  `dt` is
  * GGB_TYPE_BF16 (matrices and the activations that feed them are bf16, products accumulate in fp32) or GGB_TYPE_F32
- * (true fp32 everywhere, no reduced-precision matrix mode).  The residual stream, norms, soft-max and every other
+ * (fp32 everywhere, no reduced-precision matrix mode: where a linear layer of more than 8 rows runs on the tensor cores, a number is the
+ * sum of three bf16 parts and results are as exact as fp32 multiply-adds; numbers below 2^-130 lose bits).  The residual stream, norms, soft-max and every other
  * reduction are fp32 in both.  Pointers typed void* are in `dt`. */
 size_t ggb_dtype_size(int dt);
 /* c[t][n] (fp32) = sum_k a[t][k] w[n][k]: a streaming mat-vec for T <= 8, the tcgen05 GEMM for aligned bf16 shapes
- * (K %% 64 == 0, N %% 32 == 0, lda == K, T >= 64), a shared-memory tile kernel for every other shape */
+ * (K %% 64 == 0, N %% 32 == 0, lda == K, T >= 64), tensor cores behind ordinary loads for other shapes and fp32 from K > 128 on, a shared-memory
+ * tile kernel for shorter sums */
 int ggb_op_linear(int dt, const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t T, float *c, int64_t ldc);
 /* y = x / sqrt(mean(x^2) + eps) * w for up to two weights of the same rows (the root mean square is computed once);
  * w_stride 0: the weight is one number, 1: a vector of E; y1 / y2 ([T][E] in dt) may be NULL */
