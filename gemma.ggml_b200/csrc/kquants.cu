@@ -259,7 +259,8 @@ quantize_q8_K_kernel(const float *__restrict__ x, int64_t n_blocks, uint8_t *__r
 //
 // Bound by HBM and by the unpacking in turn (a tensor-core instruction's codes cost a warp about 15 others: instructions issue in 70 % of the
 // cycles, 5.1 TB/s).  256000 x 2048: Q6_K 122 -> 75 us, Q4_K 91 -> 72 us in graph replays (a row a
-// warp, a dot of four codes per instruction and lane sum).  A matrix of 256 rows, one tile a CTA, pays for the codes' longer way: 2.7 -> 3.0 us.
+// warp, a dot of four codes per instruction and lane sum).  Launched ahead like a step's kernels, which makes up for the codes' longer way where a
+// matrix has few tiles: 256 x 2048 Q6_K 2.8 -> 2.55, Q4_K 2.35 -> 2.55 us (3.0 and 2.75 in plain launches).
 constexpr int kActSB = 304;  // staged activation super-block, Q4_K: 256 B of codes | pair sums int[8] | d float | pad
 constexpr int kActSB6 = 272; // Q6_K: 256 B of codes | d float | pad
 constexpr int kTileRows = 16;
@@ -321,12 +322,6 @@ __global__ void __launch_bounds__(256) q6k_repack_kernel(const uint8_t *__restri
     if (c == 0) *reinterpret_cast<uint16_t *>(o + 208 * kTileRows + 2 * r) = *reinterpret_cast<const uint16_t *>(x + 208);
 }
 
-__device__ __forceinline__ uint4 ld_stream(const uint8_t *p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
 // byte i of w as a signed number
 template <int I>
 __device__ __forceinline__ int byte_s8(uint32_t w) {
@@ -355,9 +350,9 @@ struct kq_item {
         for (int u = 0; u < 2; u++) {
             const int r = Q6 ? g + 8 * u : min(g + 8 * u, R - 1); // a row past the end is read as the last one and not stored
 #pragma unroll
-            for (int p = 0; p < 2; p++) x[u][p] = ld_stream(codes + (p * R + r) * 64 + 16 * (lane & 3));
+            for (int p = 0; p < 2; p++) x[u][p] = ldg_stream_u4(codes + (p * R + r) * 64 + 16 * (lane & 3));
             if (Q6) {
-                h[Q6 ? u : 0] = ld_stream(o + 128 * kTileRows + r * 64 + 16 * (lane & 3));
+                h[Q6 ? u : 0] = ldg_stream_u4(o + 128 * kTileRows + r * 64 + 16 * (lane & 3));
                 hd[u] = __ldg(reinterpret_cast<const uint4 *>(o + 192 * kTileRows + 16 * r));
                 d[u] = __ldg(reinterpret_cast<const uint16_t *>(o + 208 * kTileRows + 2 * r));
             } else {
@@ -450,12 +445,12 @@ __device__ __forceinline__ int act_word(int wi) {
 // F32ACT: `act` is the fp32 activation row (pitch row_size bytes); the CTA quantises it to Q8_K itself while staging
 template <bool Q6, bool F32ACT>
 __global__ void __launch_bounds__(kWarps * 32, 2)
-kq_packed_kernel(const uint8_t *__restrict__ w, int64_t rows, int nb, const uint8_t *__restrict__ act, int64_t row_size,
-                 float *__restrict__ dst, int64_t dst_stride, int P, int chunk) {
+kq_packed_kernel(const uint8_t *w, int64_t rows, int nb, const uint8_t *act, int64_t row_size, float *dst, int64_t dst_stride, int P, int chunk) {
     constexpr int SB = Q6 ? kActSB6 : kActSB, kD = Q6 ? 256 : 288;
     extern __shared__ __align__(16) uint8_t s_act[];
     __shared__ __align__(16) float s_t[2][kWarps][kTileRows * 8];
     __shared__ float s_m[Q6 ? 1 : 2][Q6 ? 1 : kWarps][kTileRows];
+    step_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
     const int g = lane >> 2, c = lane & 3;
     const int64_t n_tiles = (rows + kTileRows - 1) / kTileRows, n_groups = (n_tiles + P - 1) / P;
@@ -669,8 +664,15 @@ static int launch_packed(int type, bool f32act, const void *packed, int64_t rows
     const unsigned gx = (unsigned)std::min<int64_t>((tiles + P - 1) / P, (int64_t)ggb_sm_count() * (2 * kWarps / warps));
     for (int64_t t0 = 0; t0 < T; t0 += 65535) {
         const dim3 grid(gx, (unsigned)(T - t0 < 65535 ? T - t0 : 65535));
-        kern<<<grid, warps * 32, smem, ggb_cuda_stream()>>>((const uint8_t *)packed, rows, nb, (const uint8_t *)act + t0 * row_size,
-                                                            row_size, dst + t0 * dst_stride, dst_stride, P, chunk);
+#define KQ(Q6, F32ACT)                                                                                                                                \
+    GGB_CUDA(ggb_launch_step(kq_packed_kernel<Q6, F32ACT>, grid, dim3((unsigned)(warps * 32)), smem, (const uint8_t *)packed, rows, nb, (const uint8_t *)act + t0 * row_size, \
+                             row_size, dst + t0 * dst_stride, dst_stride, P, chunk));
+        if (q4) {
+            if (f32act) { KQ(false, true) } else { KQ(false, false) }
+        } else {
+            if (f32act) { KQ(true, true) } else { KQ(true, false) }
+        }
+#undef KQ
         GGB_LAUNCH_CHECK();
     }
     return GGB_OK;

@@ -77,6 +77,8 @@ def test_what_is_done_ahead_of_the_wait():
 
 # what they read by loads that take it for granted that nobody writes there while the kernel runs: rows of weight matrices and their scales
 WEIGHTS = {"dense.cu": {"wr + k"}, "moe.cu": {"wr + k", "wu + k"},
+           "kquants.cu": {"codes + (p * R + r) * 64 + 16 * (lane & 3)", "o + 128 * kTileRows + r * 64 + 16 * (lane & 3)", "reinterpret_cast<const uint4 *>(o + 16 * r)",
+                          "reinterpret_cast<const uint4 *>(o + 192 * kTileRows + 16 * r)", "reinterpret_cast<const uint16_t *>(o + 208 * kTileRows + 2 * r)"},
            "prefill.cu": {"dp + 2 * (kb + G * u)", "reinterpret_cast<const __half2 *>(dp + 2 * fkb)"}}
 
 
