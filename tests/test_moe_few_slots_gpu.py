@@ -68,9 +68,9 @@ def test_through_the_slot_list(gpu, T, top, E, N, K, identity):
     assert np.abs(act[real][:, :N] - gelu).max() <= 2.0 ** -8 * np.abs(gelu).max() and not act[:, N:].any()
 
 
-@pytest.mark.parametrize("K", [256, 2048, 8192])
+@pytest.mark.parametrize("K", [64, 128, 256, 2048, 8192])
 def test_error_is_no_larger_than_that_of_multiply_adds(gpu, K):
-    p = Portion(gpu, 10, 2, 2, 64, K)
+    p = Portion(gpu, 20, 2, 2, 256, K)
     gpu.check(p.launch())
     real, want = p.want()
     e, t = p.rows()
@@ -78,7 +78,7 @@ def test_error_is_no_larger_than_that_of_multiply_adds(gpu, K):
     for k in range(K):  # fmaf in k order: the products of bf16 numbers are exact, one rounding a step
         chain = (chain + p.wf[e, :, k] * p.af[t, k][:, None]).astype(np.float32).astype(np.float64)
     err = lambda x: np.linalg.norm(x - want) / np.linalg.norm(want)  # noqa: E731
-    assert err(p.c.download(np.float32).reshape(want.shape)) <= err(chain)
+    assert err(p.c.download(np.float32).reshape(want.shape)) <= err(chain) * 1.001  # (equal sums where the tile kernel takes them)
 
 
 def test_a_matrix_and_results_off_their_boundaries(gpu):
