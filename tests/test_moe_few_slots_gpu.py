@@ -1,4 +1,5 @@
 """The grouped product of a portion of few slots (17 to 511), bf16: through the slot list, without a workspace, as exact as multiply-adds."""
+import math
 import os
 import subprocess
 import sys
@@ -62,7 +63,6 @@ def test_through_the_slot_list(gpu, T, top, E, N, K, identity):
     y = zeros(gpu, T * top * (N + 8) * 2)
     gpu.check(p.launch(act=4, a=dev(gpu, rows).ptr, c=y.ptr, ldc=N + 8, gather=0))
     act = from_dt(BF16, y, (T * top, N + 8))
-    import math
     z = got[real].astype(np.float64)
     gelu = 0.5 * z * (1 + np.vectorize(math.erf)(z / math.sqrt(2)))
     assert np.abs(act[real][:, :N] - gelu).max() <= 2.0 ** -8 * np.abs(gelu).max() and not act[:, N:].any()
@@ -88,7 +88,6 @@ def test_a_matrix_and_results_off_their_boundaries(gpu):
     want = p.c.download(np.float32).reshape(24, 64)
     w = zeros(gpu, 4 * 64 * 192 * 2 + 2)
     _, raw = as_dt(BF16, p.wf)
-    from gemma_ggml_b200 import DeviceBuffer  # noqa: F401
     w.upload(np.concatenate([np.zeros(1, np.uint16), raw.reshape(-1).view(np.uint16)]))
     gpu.check(p.launch(w=w.ptr.value + 2))
     assert np.abs(p.c.download(np.float32).reshape(24, 64) - want).max() < 2e-4
