@@ -1,6 +1,6 @@
 // gemm.cu — products of plain bf16 matrices on the tensor cores: C[T][N] = A[T][K] W[N][K]^T, and the grouped form for a mixture of experts.
 //
-// A tile of C is 256 x 256, by two CTAs of a cluster, or 128 x (256, 128, 64), by one.  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
+// A dense tile of C is 256 x 256, by two CTAs of a cluster, or 128 x (256, 128, 64), by one; a tile of an expert's slots is gemm_slots_kernel's.  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
 // in a ring that takes all of shared memory but the epilogue's corner; one warp issues the MMAs, eight drain tensor memory.  CTAs are
 // persistent: where a tile needs half of tensor memory, the next one's products run while the last one's are stored.  The epilogue
 // turns 32 x 32 pieces in shared memory, so that a store instruction writes whole 128-byte lines.
@@ -12,8 +12,7 @@
 //
 // What bounds it: 1024 x 8192 x 2048 is 128 tiles of 256 x 256 on 74 pairs of CTAs, two rounds of 32 stages of 512 cycles of the tensor cores,
 // the second for 54 pairs; the tensor cores are busy for 61 to 64 % of the cycles.  37.3 us, 921 TFLOP/s (47.6 us with both operands
-// copied by cp.async and rows stored by their own lanes; 38.8 us in one round of 256 x 256 tiles a CTA, whose stores nothing hides).  32
-// experts x 128 rows, 1408 x 2048: 47 us a product, 4.2 TB/s of matrices (256-row tiles, half of them empty: 68 us).
+// copied by cp.async and rows stored by their own lanes; 38.8 us in one round of 256 x 256 tiles a CTA, whose stores nothing hides).
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -28,7 +27,7 @@ namespace {
 constexpr int BK = 64, BM = 128; // a stage of K, the rows of a CTA
 constexpr int kThreads = 384; // warp 0: TMA, 1: MMA, 2: tensor memory, 4..11: epilogue
 constexpr uint32_t kRing = 192 * 1024, kTurn = 8 * 4096;
-constexpr int kMaxStages = 8, kMaxGroups = 256; // groups whose first tiles are kept in shared memory
+constexpr int kMaxStages = 8;
 constexpr size_t kSmem = 1024 + kRing + kTurn + 256;
 static_assert(kSmem >= kOneCtaSmem, "pairs of CTAs");
 enum { FULL = 0, EMPTY = 64, ACC_FULL = 128, ACC_FREE = 144, SLOT = 160, DEAD = 168 };
@@ -38,8 +37,10 @@ struct gemm_args {
     int BN, n_tiles, m_tiles;
     int chunks, chunk_kb, splits; // K pieces a CTA sums, their blocks of 64, CTAs along K
     int stages;
-    const int32_t *m_ranges; // grouped: group g has the rows [m_ranges[g], m_ranges[g + 1]) of A and C and the rows g * N .. of W
+    // grouped: group g has the rows [m_ranges[g], m_ranges[g + 1]) of C, whose rows of a are row_src[.] (or the same, by TMA), and the rows g * N .. of W
+    const int32_t *m_ranges, *row_src;
     int n_groups;
+    const __nv_bfloat16 *a;
     float *c;
     __nv_bfloat16 *act_out; // when set: bf16 act(c) instead of c
     int act;
@@ -49,8 +50,11 @@ struct gemm_args {
     int *wait_error;
 };
 
+struct pair_maps {
+    CUtensorMap w, a[4]; // a: boxes of 128 rows; of a grouped product 32, 64, 96 and 128
+};
 struct tile_at {
-    int m0, m_end, n0, split, group;
+    int m0, n0, split;
 };
 
 // a warp's 32 rows x 32 columns of accumulators, K pieces added in order, stored as whole lines
@@ -95,7 +99,6 @@ __device__ __forceinline__ void store_piece(const gemm_args &a, uint32_t col, in
 
 __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
     extern __shared__ uint8_t gm_raw[];
-    __shared__ int first_tile[kMaxGroups + 1]; // grouped: the first row tile of a group
     const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, turn = base + kRing, bars = turn + kTurn;
     uint8_t *ctl = gm_raw + (bars - raw0);
     volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
@@ -116,67 +119,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
     }
     if (warp == 2) tmem_alloc512(bars + SLOT);
     early_wait();
-    const bool listed = a.m_ranges && a.n_groups <= kMaxGroups;
-    if (listed && warp == 3) { // prefix sums of the groups' row tiles
-        int sum = 0;
-        for (int g0 = 0; g0 < a.n_groups; g0 += 32) {
-            const int g = g0 + lane;
-            int v = g < a.n_groups ? (a.m_ranges[g + 1] - a.m_ranges[g] + BM - 1) / BM : 0;
-            for (int off = 1; off < 32; off *= 2) {
-                const int o = __shfl_up_sync(0xffffffffu, v, off);
-                if (lane >= off) v += o;
-            }
-            if (g < a.n_groups) first_tile[g + 1] = sum + v;
-            sum += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) first_tile[0] = 0;
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
-    int row_tiles = a.m_tiles;
-    if (listed) row_tiles = first_tile[a.n_groups];
-    else if (a.m_ranges) {
-        row_tiles = 0;
-        for (int g = 0; g < a.n_groups; g++) row_tiles += (a.m_ranges[g + 1] - a.m_ranges[g] + BM - 1) / BM;
-    }
-    const int total = row_tiles * a.n_tiles * a.splits;
-    auto locate = [&](int t) {
+    const int total = a.m_tiles * a.n_tiles * a.splits;
+    auto locate = [&](int t) { // row tiles first: those that share a piece of W run together
         tile_at r;
-        r.group = 0;
-        if (!a.m_ranges) { // row tiles first: those that share a piece of W run together
-            r.m0 = t % a.m_tiles * BM;
-            r.m_end = a.T;
-            t /= a.m_tiles;
-            r.n0 = t % a.n_tiles * a.BN;
-            r.split = t / a.n_tiles;
-            return r;
-        }
-        const int rt = t / a.n_tiles;
-        r.n0 = (t - rt * a.n_tiles) * a.BN;
-        r.split = 0;
-        int f;
-        if (listed) {
-            int lo = 0, hi = a.n_groups - 1; // the last group whose first tile is not behind rt
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (first_tile[mid] <= rt) lo = mid;
-                else hi = mid - 1;
-            }
-            r.group = lo;
-            f = first_tile[lo];
-        } else {
-            f = 0;
-            for (;; r.group++) {
-                const int n = (a.m_ranges[r.group + 1] - a.m_ranges[r.group] + BM - 1) / BM;
-                if (f + n > rt) break;
-                f += n;
-            }
-        }
-        r.m0 = a.m_ranges[r.group] + (rt - f) * BM;
-        r.m_end = a.m_ranges[r.group + 1];
+        r.m0 = t % a.m_tiles * BM;
+        t /= a.m_tiles;
+        r.n0 = t % a.n_tiles * a.BN;
+        r.split = t / a.n_tiles;
         return r;
     };
     auto k_range = [&](int split, int &kb0, int &kb1) {
@@ -197,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
                     const uint32_t sa = base + s * stage_bytes, bar = bars + FULL + 8 * s;
                     mbar_expect_tx(bar, stage_bytes);
                     tma_load_2d(sa, &map_a, kb * BK, at.m0, bar);
-                    tma_load_2d(sa + a_bytes, &map_w, kb * BK, at.group * a.N + at.n0, bar);
+                    tma_load_2d(sa + a_bytes, &map_w, kb * BK, at.n0, bar);
                     if (++s == a.stages) s = 0, ph ^= 1u;
                 }
             }
@@ -241,9 +195,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
             tc_fence_after();
             // a warp's 32 rows, every other 32 columns (the two warps of a quarter share them)
             const int row0 = at.m0 + lq * 32;
-            if (row0 < at.m_end)
+            if (row0 < a.T)
                 for (int c0 = 32 * half; c0 < a.BN && at.n0 + c0 < a.N; c0 += 64)
-                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, chunks, my, lane, row0, at.m_end, at.n0 + c0, at.split);
+                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, chunks, my, lane, row0, a.T, at.n0 + c0, at.split);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + ACC_FREE + 8 * buf);
@@ -262,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
 // reads A and W tiles of 12 KB from shared memory for an MMA of 128 cycles while TMA writes 64 bytes a cycle: 160 of the 128 bytes a cycle that
 // shared memory has; a pair needs 112.  2048 x 8192 x 4096: 104 us, 1320 TFLOP/s (107 us single, 131 us before either); 1024 x 32000 x 2048: 109 us
 // (125, 190 us).
-__global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
+__global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_constant__ pair_maps maps, const gemm_args a) {
     extern __shared__ uint8_t gm_raw[];
     const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, turn = base + kRing, bars = turn + kTurn;
     uint8_t *ctl = gm_raw + (bars - raw0);
@@ -316,8 +270,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
                     if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead)) break;
                     const uint32_t sa = base + s * stage_bytes;
                     if (rank == 0) mbar_expect_tx(bars + FULL + 8 * s, 2 * stage_bytes);
-                    tma_load_2d_pair(sa, &map_a, kb * BK, m0 + (int)rank * BM, bars0 + FULL + 8 * s);
-                    tma_load_2d_pair(sa + a_bytes, &map_w, kb * BK, n0 + (int)rank * 128, bars0 + FULL + 8 * s);
+                    tma_load_2d_pair(sa, &maps.a[0], kb * BK, m0 + (int)rank * BM, bars0 + FULL + 8 * s);
+                    tma_load_2d_pair(sa + a_bytes, &maps.w, kb * BK, n0 + (int)rank * 128, bars0 + FULL + 8 * s);
                     if (++s == kStages) s = 0, ph ^= 1u;
                 }
             }
@@ -378,6 +332,227 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
     }
 }
 
+// The slots of a mixture of experts, sorted by group: C[slot][N] = A[slot][K] W[group of the slot][N][K]^T.  A pair of CTAs owns 256 features (the M of an MMA, half
+// a CTA) x up to 256 slots of a group in equal tiles of a multiple of 32: so a group's matrix is read once whatever its slots, and no row is computed for nothing but
+// the last 31.  A lane of tensor memory is a feature, so that 32 lanes store a line of a slot's row as they are.
+//
+// Rows of A come by TMA where they lie sorted.  Where they do not (row_src) and a tile has few of them, three groups of four warps copy them through the slot
+// list, which takes the stages in turn: a group hands one over when it has asked for its next (asking takes 500 cycles of a stage's 700, arriving 2500).
+//
+// Bound by memory, the matrices, and by the third round of tiles.  32 experts x 128 +- 11 slots, 1408 x 2048: 44.2 us a product from sorted rows (row tiles of 128
+// slots x 256 features, in which half of the groups read their matrix twice: 47.0), 42.9 through the slot list (50.9 gathered ahead of it, 52 gathered ahead of this
+// kernel); with GELU 44.6 (64.2).  8 experts x 768 slots, 2048 x 2048, bound by the MMAs: 52 (52.9).  TMA's gather of four rows
+// takes 80 cycles a row: 80 us.
+constexpr uint32_t kSlotStage = BM * 128 + 128 * 128;
+constexpr int kSlotStages = 6, kMaxGroups = 8192;
+constexpr int kCopyGroups = 3, kCopyWarps = 4, kSlotThreads = kThreads + 32 * kCopyWarps * kCopyGroups; // warps 12..: rows of A through the slot list
+static_assert(kSlotStages == 2 * kCopyGroups, "a copying group has two places of the ring");
+constexpr size_t kSlotSmem = 1024 + kSlotStages * kSlotStage + 256; // and the list of first tiles
+static_assert(kSlotSmem >= kOneCtaSmem && kSlotSmem + 4 * (kMaxGroups + 1) <= 232448, "pairs of CTAs");
+
+__global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __grid_constant__ pair_maps maps, const gemm_args a) {
+    extern __shared__ uint8_t gm_raw[];
+    __shared__ int warp_sum[kSlotThreads / 32];
+    const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, bars = base + kSlotStages * kSlotStage;
+    uint8_t *ctl = gm_raw + (bars - raw0);
+    volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
+    int *first_tile = reinterpret_cast<int *>(ctl + 256); // [n_groups + 1]: the first slot tile of a group
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t rank = cluster_rank(), bars0 = cluster_addr(bars, 0);
+    if (tid == 0) {
+        for (int s = 0; s < kSlotStages; s++) {
+            mbar_init(bars + FULL + 8 * s, a.row_src ? 1 + 2 * kCopyWarps : 1); // TMA, the copying warps of both CTAs
+            mbar_init(bars + EMPTY + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(bars + ACC_FULL + 8 * s, 1);
+            mbar_init(bars + ACC_FREE + 8 * s, 16);
+        }
+        *dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) tmem_alloc512_pair(bars + SLOT);
+    early_wait();
+    { // prefix sums of the groups' slot tiles: a thread takes `each` neighbouring groups
+        const int nt = blockDim.x, each = (a.n_groups + nt - 1) / nt, g0 = min(tid * each, a.n_groups), g1 = min(g0 + each, a.n_groups);
+        int own = 0;
+        for (int g = g0; g < g1; g++) own += (a.m_ranges[g + 1] - a.m_ranges[g] + 255) / 256;
+        int sum = own;
+        for (int off = 1; off < 32; off *= 2) {
+            const int o = __shfl_up_sync(0xffffffffu, sum, off);
+            if (lane >= off) sum += o;
+        }
+        if (lane == 31) warp_sum[warp] = sum;
+        __syncthreads();
+        sum -= own;
+        for (int w = 0; w < warp; w++) sum += warp_sum[w];
+        for (int g = g0; g < g1; g++) {
+            first_tile[g] = sum;
+            sum += (a.m_ranges[g + 1] - a.m_ranges[g] + 255) / 256;
+        }
+        if (tid == nt - 1) first_tile[a.n_groups] = sum;
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    step_next();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
+    const int total = first_tile[a.n_groups] * a.n_tiles, pairs = gridDim.x / 2, me = blockIdx.x / 2;
+    struct slot_tile {
+        int group, row0, rows, width, n0; // width: rows as a multiple of 32
+    };
+    auto locate = [&](int t) { // a group's features follow one another: its rows of A stay in L2
+        slot_tile r;
+        const int st = t / a.n_tiles;
+        r.n0 = (t - st * a.n_tiles) * 256;
+        int lo = 0, hi = a.n_groups - 1; // the last group whose first tile is not behind st
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first_tile[mid] <= st) lo = mid;
+            else hi = mid - 1;
+        }
+        const int f = first_tile[lo], n = first_tile[lo + 1] - f, g0 = a.m_ranges[lo], g1 = a.m_ranges[lo + 1];
+        r.group = lo;
+        r.width = ((g1 - g0 + n - 1) / n + 31) / 32 * 32;
+        r.row0 = g0 + (st - f) * r.width;
+        r.rows = min(r.width, g1 - r.row0);
+        return r;
+    };
+    // one copy a stage and CTA for either operand (a thread takes 150 cycles for each): the box of A that covers half a tile, whose last rows may be the next
+    // group's or behind the matrix: columns that nobody stores
+    auto box_of = [](const slot_tile &at) { return (at.width / 2 + 31) / 32; };
+    if (warp == 3) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 1;
+            for (int t = me; t < total && !a.row_src; t += pairs) {
+                const slot_tile at = locate(t);
+                const CUtensorMap *map = &maps.a[box_of(at) - 1];
+                const int r0 = at.row0 + (int)rank * (at.width / 2);
+                for (int kb = 0; kb < a.kblocks; kb++) {
+                    if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph, dead)) break;
+                    tma_load_2d_pair(base + s * kSlotStage + BM * 128, map, kb * BK, r0, bars0 + FULL + 8 * s);
+                    if (++s == kSlotStages) s = 0, ph ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 0) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 1;
+            for (int t = me; t < total; t += pairs) {
+                const slot_tile at = locate(t);
+                const bool both = at.n0 + BM < a.N, mine = rank == 0 || both; // features behind the last one: not read, not stored
+                for (int kb = 0; kb < a.kblocks; kb++) {
+                    if (!mbar_wait_bounded(bars + EMPTY + 8 * s, ph, dead)) break;
+                    if (rank == 0) mbar_expect_tx(bars + FULL + 8 * s, (both ? 2 * BM * 128 : BM * 128) + (a.row_src ? 0 : 2 * box_of(at) * 32 * 128));
+                    if (mine) tma_load_2d_pair(base + s * kSlotStage, &maps.w, kb * BK, at.group * a.N + at.n0 + (int)rank * BM, bars0 + FULL + 8 * s);
+                    if (++s == kSlotStages) s = 0, ph ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1 && rank == 0) {
+        int s = 0, it = 0;
+        uint32_t ph = 0;
+        for (int t = me; t < total; t += pairs, it++) {
+            const uint32_t idesc = umma_idesc(256, locate(t).width), buf = it & 1;
+            mbar_wait_bounded(bars + ACC_FREE + 8 * buf, ((it >> 1) & 1) ^ 1, dead);
+            tc_fence_after();
+            for (int kb = 0; kb < a.kblocks; kb++) {
+                mbar_wait_bounded(bars + FULL + 8 * s, ph, dead);
+                tc_fence_after();
+                const uint32_t at = base + s * kSlotStage;
+                umma_ss_pair_k4(tmem + buf * 256, umma_desc_lo(at, 16), umma_desc_lo(at + BM * 128, 16), idesc, kb > 0);
+                umma_arrive_pair(bars + EMPTY + 8 * s);
+                if (++s == kSlotStages) s = 0, ph ^= 1u;
+            }
+            umma_arrive_pair(bars + ACC_FULL + 8 * buf);
+        }
+    } else if (warp >= 12) {
+        // stages grp, grp + 3, ... of all of this CTA's, into two places of the ring: a thread copies one 16-byte piece of every 16th row
+        const int grp = (warp - 12) / kCopyWarps, lt = (tid - kThreads) % (32 * kCopyWarps), pc = lt & 7, r0 = lt >> 3;
+        int next = grp, n = 0; // its next stage, counted from the tile's first; stages asked for
+        auto give = [&](int k) {
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(bars0 + FULL + 8 * (grp + kCopyGroups * (k & 1)));
+        };
+        for (int t = me; t < total; t += pairs, next -= a.kblocks) {
+            if (next >= a.kblocks) continue;
+            const slot_tile at = locate(t);
+            const int h0 = (int)rank * (at.width / 2), mine = min(at.width / 2, at.rows - h0); // this CTA's half of the tile (none: not above 0)
+            const __nv_bfloat16 *from[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) from[i] = a.a + (int64_t)a.row_src[at.row0 + min(h0 + r0 + 16 * i, at.rows - 1)] * (a.kblocks * BK) + 8 * pc;
+            for (; next < a.kblocks; next += kCopyGroups, n++) {
+                const int s = grp + kCopyGroups * (n & 1);
+                if (!mbar_wait_warp(bars + EMPTY + 8 * s, ((n >> 1) & 1) ^ 1, dead)) break;
+#pragma unroll
+                for (int i = 0; i < 8; i++) // rows 16 apart lie at the same place of the swizzle; those behind the last stay as they are: columns that nobody stores
+                    if (r0 + 16 * i < mine) cp_async16(base + s * kSlotStage + (BM + r0 + 16 * i) * 128 + ((pc ^ (r0 & 7)) << 4), from[i] + next * BK);
+                cp_async_commit();
+                if (n > 0) {
+                    cp_async_wait<1>();
+                    give(n - 1);
+                }
+            }
+        }
+        cp_async_wait<0>();
+        if (n > 0) give(n - 1);
+    } else if (warp >= 4) {
+        const int lq = warp & 3, half = (warp - 4) >> 2;
+        int it = 0;
+        for (int t = me; t < total; t += pairs, it++) {
+            const slot_tile at = locate(t);
+            const uint32_t buf = it & 1;
+            mbar_wait_warp(bars + ACC_FULL + 8 * buf, (it >> 1) & 1, dead);
+            tc_fence_after();
+            const int n = at.n0 + (int)rank * BM + lq * 32 + lane; // N is a multiple of 32: a warp's features are all there or none
+            if (n < a.N)
+                for (int c0 = 32 * half; c0 < at.rows; c0 += 64) {
+                    uint32_t v[32];
+                    tmem_load32(tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, v);
+                    const int64_t row = at.row0 + c0;
+                    if (a.act_out) { // two slots at a time: an even lane stores its and its neighbour's feature of the first one, an odd lane of the second
+                        __nv_bfloat16 *dst = a.act_out + (row + (lane & 1)) * a.ldc + (n & ~1);
+                        const int left = at.rows - c0 - (lane & 1);
+                        if (a.act == GGB_ACT_GELU_ERF) {
+#pragma unroll
+                            for (int c = 0; c < 32; c++) v[c] = __float_as_uint(act_f32(__uint_as_float(v[c]), GGB_ACT_GELU_ERF));
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 32; c++) v[c] = __float_as_uint(act_f32(__uint_as_float(v[c]), a.act));
+                        }
+#pragma unroll
+                        for (int c = 0; c < 32; c += 2) {
+                            const float x = __uint_as_float(v[c]), y = __uint_as_float(v[c + 1]), o = __shfl_xor_sync(0xffffffffu, lane & 1 ? x : y, 1);
+                            if (c < left) *reinterpret_cast<uint32_t *>(dst + c * a.ldc) = lane & 1 ? pack_bf16x2(o, y) : pack_bf16x2(x, o);
+                        }
+                    } else {
+                        float *dst = a.c + row * a.ldc + n;
+#pragma unroll
+                        for (int c = 0; c < 32; c++)
+                            if (c0 + c < at.rows) dst[c * a.ldc] = __uint_as_float(v[c]);
+                    }
+                }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(bars0 + ACC_FREE + 8 * buf);
+        }
+    }
+    __syncthreads();
+    if (warp == 2) settle(dead);
+    cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
+    if (warp == 2) {
+        tc_fence_after();
+        tmem_free512_pair(tmem);
+        if (lane == 0 && *dead) *a.wait_error = 1;
+    }
+}
+
 // the CTAs' sums along K in order
 __global__ void splits_add_kernel(const float *__restrict__ ws, int splits, int64_t T, int64_t N, float *__restrict__ c, __nv_bfloat16 *__restrict__ act_out, int act,
                                   int64_t ldc) {
@@ -398,12 +573,14 @@ __global__ void splits_add_kernel(const float *__restrict__ ws, int splits, int6
 }
 
 int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, const gemm_args &g, int pairs) {
-    CUtensorMap ma, mw;
-    int rc = ggb_allow_smem(gemm_pair_kernel, kSmem);
-    if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
-    if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, 128);
+    pair_maps maps;
+    auto kern = g.m_ranges ? gemm_slots_kernel : gemm_pair_kernel;
+    const size_t pair_smem = std::max(kOneCtaSmem, g.m_ranges ? kSlotSmem + 4 * ((size_t)g.n_groups + 1) : kSmem);
+    int rc = ggb_allow_smem(kern, g.m_ranges ? kSlotSmem + 4 * (kMaxGroups + 1) : kSmem);
+    if (!rc) rc = ggb_tensor_map_bf16(&maps.w, w, w_rows, K, K, 128);
+    for (int i = 0; i < (g.row_src ? 0 : g.m_ranges ? 4 : 1) && !rc; i++) rc = ggb_tensor_map_bf16(&maps.a[i], a, a_rows, K, K, g.m_ranges ? 32 * (i + 1) : BM);
     if (rc) return rc;
-    GGB_CUDA(ggb_launch_early(gemm_pair_kernel, ggb_cluster{2, 1, 1}, dim3((unsigned)(2 * std::min(pairs, ggb_sm_count() / 2))), dim3(kThreads), kSmem, ma, mw, g));
+    GGB_CUDA(ggb_launch_early(kern, ggb_cluster{2, 1, 1}, dim3((unsigned)(2 * std::min(pairs, ggb_sm_count() / 2))), dim3(g.row_src ? kSlotThreads : kThreads), pair_smem, maps, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -504,19 +681,19 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
     return GGB_OK;
 }
 
-// The grouped form: w = [n_exp][N][K], a / c rows in sorted-slot order, offsets[e] .. offsets[e + 1] the rows of expert e (device).  Row
-// tiles of 128: an expert of a portion has about that many rows (256 would be computed for nothing to a half).
+// The grouped form: w = [n_exp][N][K], rows of c in sorted-slot order, offsets[e] .. offsets[e + 1] those of expert e (device), row_src their rows of a (or
+// null: the same)
 bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc) { return K % 64 == 0 && N % 32 == 0 && ldc % 8 == 0; }
-int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, float *c, void *c_act, int act, int64_t ldc) {
+int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, const int32_t *row_src, float *c, void *c_act,
+                          int act, int64_t ldc) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
+    GGB_CHECK_ARG(n_exp <= kMaxGroups && n_exp * N < (1ll << 31), "gemm: %d experts of %lld rows", n_exp, (long long)N);
     gemm_args g{};
-    g.BN = N <= 64 ? 64 : N <= 128 ? 128 : 256;
-    g.T = (int)n_rows, g.N = (int)N, g.kblocks = (int)(K / BK), g.n_tiles = (int)((N + g.BN - 1) / g.BN);
-    g.chunks = 1, g.chunk_kb = g.kblocks, g.splits = 1, g.stages = stages_of(g.BN);
-    g.m_ranges = offsets, g.n_groups = n_exp;
-    g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc, g.vec = (uintptr_t)c % 16 == 0;
+    g.T = (int)n_rows, g.N = (int)N, g.kblocks = (int)(K / BK), g.n_tiles = (int)((N + 255) / 256);
+    g.m_ranges = offsets, g.row_src = row_src, g.n_groups = n_exp, g.a = (const __nv_bfloat16 *)a;
+    g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc;
     g.wait_error = ggb_wait_error_flag();
-    const int64_t most = ((n_rows + BM - 1) / BM + n_exp) * g.n_tiles;
-    return launch(w, (int64_t)n_exp * N, K, a, n_rows, g, (int)std::min<int64_t>(most, 1 << 20));
+    const int64_t most = (n_rows / 256 + std::min<int64_t>(n_rows, n_exp)) * g.n_tiles;
+    return launch_pair(w, (int64_t)n_exp * N, K, a, n_rows, g, (int)std::min<int64_t>(most, 1 << 20));
 }

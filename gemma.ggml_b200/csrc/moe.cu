@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "dense.cuh"
 #include "gemm_any.cuh"
+#include "tc.cuh"
 
 namespace {
 
@@ -50,86 +51,8 @@ __global__ void __launch_bounds__(256) moe_logits_kernel(const E *h, int64_t W, 
     if (lane == 0) z[i] = s + (b ? b[e] : 0.f);
 }
 
-// A portion of tokens: a warp computes 4 tokens x 4 experts, so that a row of the router is read once for four tokens and a token's row once
-// for four experts (a warp per logit reads 268 MB through L2 for 1024 tokens x 32 experts of width 2048).  Every logit is the same
-// sum in the same order as router_dot's, to the bit: a choice between experts does not depend on how many tokens share the call.
-// Bound by instruction issue.  1024 x 32 x 2048: 20.4 -> 15.2 us.
-constexpr int kLogitTile = 4;
-template <typename E>
-__global__ void __launch_bounds__(256) moe_logits_tile_kernel(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, float *z) {
-    step_wait();
-    struct alignas(4 * sizeof(E)) quad {
-        E v[4];
-    };
-    const int lane = threadIdx.x & 31, groups = (n_exp + kLogitTile - 1) / kLogitTile;
-    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), t0 = item / groups * kLogitTile;
-    const int e0 = (int)(item % groups) * kLogitTile;
-    if (t0 >= T) return;
-    const E *hr[kLogitTile];
-    const float *wr[kLogitTile];
-#pragma unroll
-    for (int i = 0; i < kLogitTile; i++) { // past the end: the last one again, not stored
-        hr[i] = h + min(t0 + i, T - 1) * W;
-        wr[i] = w + (int64_t)min(e0 + i, n_exp - 1) * W;
-    }
-    float s[kLogitTile * kLogitTile]; // [token][expert]
-#pragma unroll
-    for (int i = 0; i < kLogitTile * kLogitTile; i++) s[i] = 0.f;
-#pragma unroll 2
-    for (int64_t k = (int64_t)lane * 4; k < W; k += 128) {
-        float hv[kLogitTile][4];
-        float4 wv[kLogitTile];
-#pragma unroll
-        for (int i = 0; i < kLogitTile; i++) {
-            const quad q = *reinterpret_cast<const quad *>(hr[i] + k);
-            wv[i] = *reinterpret_cast<const float4 *>(wr[i] + k);
-#pragma unroll
-            for (int c = 0; c < 4; c++) hv[i][c] = to_f32(q.v[c]);
-        }
-#pragma unroll
-        for (int i = 0; i < kLogitTile; i++)
-#pragma unroll
-            for (int j = 0; j < kLogitTile; j++) {
-                float &a = s[i * kLogitTile + j];
-                a = fmaf(wv[j].x, hv[i][0], a);
-                a = fmaf(wv[j].y, hv[i][1], a);
-                a = fmaf(wv[j].z, hv[i][2], a);
-                a = fmaf(wv[j].w, hv[i][3], a);
-            }
-    }
-    // sixteen sums at once, each by the additions of warp_sum_f32: a lane ends with sum lane / 2
-#pragma unroll
-    for (int n = 8, off = 16; n >= 1; n >>= 1, off >>= 1) {
-        const bool up = lane & off;
-#pragma unroll
-        for (int i = 0; i < n; i++) s[i] = __fadd_rn(up ? s[n + i] : s[i], __shfl_xor_sync(0xffffffffu, up ? s[i] : s[n + i], off));
-    }
-    s[0] = __fadd_rn(s[0], __shfl_xor_sync(0xffffffffu, s[0], 1));
-    const int i = lane >> 3, j = (lane >> 1) & 3;
-    if (!(lane & 1) && t0 + i < T && e0 + j < n_exp) z[(t0 + i) * n_exp + e0 + j] = s[0] + (b ? b[e0 + j] : 0.f);
-}
-
-// the form by the number of logits: below a warp for every scheduler of the chip, tiles would leave SMs idle
-template <typename E>
-int logits_launch(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, float *z) {
-    const int64_t tiles = (T + kLogitTile - 1) / kLogitTile * ((n_exp + kLogitTile - 1) / kLogitTile);
-    if (W % 4 == 0 && tiles >= 4 * ggb_sm_count())
-        ggb_launch_step(moe_logits_tile_kernel<E>, dim3((unsigned)((tiles + 7) / 8)), dim3(256), 0, h, W, T, w, b, n_exp, z);
-    else ggb_launch_step(moe_logits_kernel<E>, dim3((unsigned)((T * n_exp + 7) / 8)), dim3(256), 0, h, W, T, w, b, n_exp, z);
-    GGB_LAUNCH_CHECK();
-    return GGB_OK;
-}
-
-// one warp per token: `top` rounds of arg-max over its logits (ties: the lower index), soft-max over the chosen
-__global__ void __launch_bounds__(32) moe_select_kernel(const float *zg, int n_exp, int top, int32_t *idx,
-                                                        float *wt) {
-    step_wait();
-    extern __shared__ float z[]; // [n_exp] logits, then [top] chosen values
-    float *sel = z + n_exp;
-    const int64_t t = blockIdx.x;
-    const int lane = threadIdx.x;
-    for (int e = lane; e < n_exp; e += 32) z[e] = zg[t * n_exp + e];
-    __syncwarp();
+// one warp: `top` rounds of arg-max over a token's logits z (ties: the lower index; z is used up), soft-max over the chosen; sel: [top] scratch
+__device__ __forceinline__ void select_top_warp(float *z, float *sel, int n_exp, int top, int64_t t, int lane, int32_t *idx, float *wt) {
     for (int k = 0; k < top; k++) {
         float bv = -INFINITY;
         int bi = 0x7fffffff;
@@ -144,6 +67,7 @@ __global__ void __launch_bounds__(32) moe_select_kernel(const float *zg, int n_e
             if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
         }
         if (lane == 0) {
+            if (bi >= n_exp) bi = 0; // logits that are no numbers: any expert, but one that exists
             idx[t * top + k] = bi;
             sel[k] = bv;
             z[bi] = -INFINITY;
@@ -158,6 +82,152 @@ __global__ void __launch_bounds__(32) moe_select_kernel(const float *zg, int n_e
         }
         for (int k = 0; k < top; k++) wt[t * top + k] = sel[k] / sum;
     }
+}
+
+// one warp per token
+__global__ void __launch_bounds__(32) moe_select_kernel(const float *zg, int n_exp, int top, int32_t *idx,
+                                                        float *wt) {
+    step_wait();
+    extern __shared__ float z[]; // [n_exp] logits, then [top] chosen values
+    const int64_t t = blockIdx.x;
+    const int lane = threadIdx.x;
+    for (int e = lane; e < n_exp; e += 32) z[e] = zg[t * n_exp + e];
+    __syncwarp();
+    select_top_warp(z, z + n_exp, n_exp, top, t, lane, idx, wt);
+}
+
+// A portion of tokens: a warp computes TT (4 or 8) tokens x 4 experts, so that a row of the router is read once for TT tokens and a token's row once
+// for four experts (a warp per logit reads 268 MB through L2 for 1024 tokens x 32 experts of width 2048); `wide` of a CTA's eight warps stand beside each other
+// with the same tokens, whose rows come from L1 to all but one of them.  Every logit is the same sum in the same order as router_dot's, to the bit: a choice
+// between experts does not depend on how many tokens share the call.  TOP: the experts are 32 at most, and a warp then chooses for each token of the CTA
+// (idx and wt), which spares a launch.
+// Bound by the issue of instructions (two multiply-adds in one) and by L2's latency, against which each lane brings its own numbers of the next kLogitAhead
+// steps of 128 into shared memory.  1024 x 32 x 2048: 10.6 us with the choice (11.7 with two steps in registers; 11.0 with 4 x 4 tiles, single multiply-adds and
+// another launch for the choice); 1024 x 16 x 1024: 5.5 (6.5).
+constexpr int kLogitExperts = 4, kLogitWarps = 8, kLogitAhead = 4;
+template <typename E, int TT> constexpr size_t logit_smem() { return (size_t)kLogitAhead * 32 * kLogitWarps * (kLogitExperts * 16 + TT * 4 * sizeof(E)); }
+template <typename E, int TT, bool TOP>
+__global__ void __launch_bounds__(32 * kLogitWarps) moe_logits_tile_kernel(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, int wide, float *z, int top,
+                                                                           int32_t *idx, float *wt) {
+    constexpr int NE = kLogitExperts, NS = TT * NE, AT = kLogitAhead; // sums of a warp; steps under way
+    extern __shared__ uint8_t lg_raw[];
+    __shared__ float zs[TOP ? NS * kLogitWarps : 1], sel[TOP ? NS * kLogitWarps : 1]; // [token][expert]
+    step_wait();
+    struct alignas(4 * sizeof(E)) quad {
+        E v[4];
+    };
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tokens = TT * (kLogitWarps / wide), tw = warp / wide * TT;
+    const int64_t tc = (int64_t)blockIdx.x * tokens, t0 = tc + tw;
+    const int e0 = ((int)blockIdx.y * wide + warp % wide) * NE;
+    if (!TOP && (e0 >= n_exp || t0 >= T)) return;
+    const E *hr = h + min(t0, T - 1) * W;
+    const float *wr = w + (int64_t)min(e0, n_exp - 1) * W;
+    uint32_t ho[TT], wo[NE]; // rows past the end: the last one again, not stored
+#pragma unroll
+    for (int i = 0; i < TT; i++) ho[i] = (uint32_t)((min(t0 + i, T - 1) - min(t0, T - 1)) * W);
+#pragma unroll
+    for (int j = 0; j < NE; j++) wo[j] = (uint32_t)((min(e0 + j, n_exp - 1) - min(e0, n_exp - 1)) * W);
+    f32x2 s2[TT / 2 * NE]; // [two tokens][expert]
+#pragma unroll
+    for (int i = 0; i < TT / 2 * NE; i++) s2[i] = 0;
+    // a lane's own numbers: [step][row][thread], w in pieces of 16 bytes, then h
+    const uint32_t wb = smem_u32(lg_raw) + threadIdx.x * 16, hb = smem_u32(lg_raw) + AT * NE * blockDim.x * 16 + threadIdx.x * sizeof(quad);
+    const uint32_t wp = blockDim.x * 16, hp = blockDim.x * sizeof(quad); // from one row to the next
+    auto load = [&](int64_t k, int u) {
+        if (k < W) {
+#pragma unroll
+            for (int i = 0; i < TT; i++)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(hb + (u * TT + i) * hp), "l"(hr + k + ho[i]), "n"(sizeof(quad)) : "memory");
+#pragma unroll
+            for (int j = 0; j < NE; j++) cp_async16(wb + (u * NE + j) * wp, wr + k + wo[j]);
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int u = 0; u < AT - 1; u++) load(4 * lane + 128 * u, u);
+    for (int64_t k0 = 4 * lane; k0 < W; k0 += 128 * AT)
+#pragma unroll
+        for (int u = 0; u < AT; u++) {
+            const int64_t k = k0 + 128 * u;
+            load(k + 128 * (AT - 1), (u + AT - 1) % AT);
+            if (k >= W) continue;
+            cp_async_wait<AT - 1>();
+            quad hq[TT];
+            float4 wq[NE];
+#pragma unroll
+            for (int i = 0; i < TT; i++) hq[i] = *reinterpret_cast<const quad *>(lg_raw + (hb - smem_u32(lg_raw)) + (u * TT + i) * hp);
+#pragma unroll
+            for (int j = 0; j < NE; j++) wq[j] = *reinterpret_cast<const float4 *>(lg_raw + (wb - smem_u32(lg_raw)) + (u * NE + j) * wp);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                f32x2 w2[NE];
+#pragma unroll
+                for (int j = 0; j < NE; j++) {
+                    const float x = c == 0 ? wq[j].x : c == 1 ? wq[j].y : c == 2 ? wq[j].z : wq[j].w;
+                    w2[j] = pack2(x, x);
+                }
+#pragma unroll
+                for (int i = 0; i < TT / 2; i++) {
+                    const f32x2 h2 = pack2(to_f32(hq[2 * i].v[c]), to_f32(hq[2 * i + 1].v[c]));
+#pragma unroll
+                    for (int j = 0; j < NE; j++) s2[i * NE + j] = fma2(w2[j], h2, s2[i * NE + j]);
+                }
+            }
+        }
+    cp_async_wait<0>();
+    __syncwarp();
+    // all sums at once, each by the additions of warp_sum_f32: a lane ends with sum lane (of 32) or lane / 2 (of 16)
+    float s[NS]; // [token][expert]
+#pragma unroll
+    for (int i = 0; i < TT / 2; i++)
+#pragma unroll
+        for (int j = 0; j < NE; j++) {
+            const float2 v = unpack2(s2[i * NE + j]);
+            s[2 * i * NE + j] = v.x, s[(2 * i + 1) * NE + j] = v.y;
+        }
+#pragma unroll
+    for (int n = NS / 2, off = 16; n >= 1; n >>= 1, off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < n; i++) s[i] = __fadd_rn(up ? s[n + i] : s[i], __shfl_xor_sync(0xffffffffu, up ? s[i] : s[n + i], off));
+    }
+    if (NS == 16) s[0] = __fadd_rn(s[0], __shfl_xor_sync(0xffffffffu, s[0], 1));
+    const int own = NS == 16 ? lane >> 1 : lane, i = own / NE, j = own % NE;
+    if ((NS == 32 || !(lane & 1)) && e0 + j < n_exp) {
+        const float v = s[0] + (b ? b[e0 + j] : 0.f);
+        if (t0 + i < T) z[(t0 + i) * n_exp + e0 + j] = v;
+        if (TOP) zs[(tw + i) * wide * NE + e0 + j] = v;
+    }
+    if (TOP) {
+        __syncthreads();
+        for (int t = warp; t < tokens && tc + t < T; t += kLogitWarps) select_top_warp(zs + t * wide * NE, sel + t * wide * NE, n_exp, top, tc + t, lane, idx, wt);
+    }
+}
+
+// The form by the number of logits: below a warp for every scheduler of the chip, tiles would leave SMs idle; eight tokens a warp where that still is
+// a CTA for two SMs of three, since a CTA of four reads the router as often for half the tokens.  chosen: idx and wt have been computed too
+template <typename E>
+int logits_launch(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, float *z, int top = 0, int32_t *idx = nullptr, float *wt = nullptr,
+                  bool *chosen = nullptr) {
+    const int64_t groups = (n_exp + kLogitExperts - 1) / kLogitExperts, tiles = (T + 3) / 4 * groups;
+    if (W % 4 == 0 && W < (1 << 28) && tiles >= 4 * ggb_sm_count()) {
+        int wide = 1; // warps beside each other
+        while (wide < kLogitWarps && wide < groups) wide *= 2;
+        const int rows = kLogitWarps / wide;
+        const unsigned ey = (unsigned)((groups + wide - 1) / wide);
+        const bool eight = (T + 8 * rows - 1) / (8 * rows) * ey * 3 >= 2 * ggb_sm_count(), fused = chosen && ey == 1;
+        const int tokens = rows * (eight ? 8 : 4);
+        const dim3 grid((unsigned)((T + tokens - 1) / tokens), ey), block(32 * kLogitWarps);
+        if (chosen) *chosen = fused;
+        int rc = GGB_OK;
+#define TILE(TT, TOP)                                                                                                                              \
+    if ((rc = ggb_allow_smem(moe_logits_tile_kernel<E, TT, TOP>, logit_smem<E, TT>()))) return rc;                                               \
+    ggb_launch_step(moe_logits_tile_kernel<E, TT, TOP>, grid, block, logit_smem<E, TT>(), h, W, T, w, b, n_exp, wide, z, top, idx, wt)
+        if (eight && fused) { TILE(8, true); } else if (eight) { TILE(8, false); } else if (fused) { TILE(4, true); } else { TILE(4, false); }
+#undef TILE
+    } else ggb_launch_step(moe_logits_kernel<E>, dim3((unsigned)((T * n_exp + 7) / 8)), dim3(256), 0, h, W, T, w, b, n_exp, z);
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
 }
 
 // one warp: the choice scores of every group but the `keep` best ones (larger score, then lower index) become -inf
@@ -528,11 +598,23 @@ __global__ void __launch_bounds__(256) moe_vec_shared_kernel(const E *w, int64_t
     else (t < 0 ? c : sh.c)[at] = acc;
 }
 
-// rows of A in sorted-slot order (the tensor-core product reads its operand contiguously): y[i] = a[row_src[i]], 16 bytes a thread
-__global__ void moe_gather_kernel(const uint4 *a, int64_t row_u4, const int32_t *row_src, uint4 *y) {
+// rows of A in sorted-slot order (the tensor-core product reads its operand contiguously): y[i] = a[row_src[i]], a warp a row, 16 bytes a lane, eight of
+// them under way
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4 *a, int64_t row_u4, const int32_t *row_src, int64_t n, uint4 *y) {
     step_wait();
-    const uint4 *src = a + (int64_t)row_src[blockIdx.x] * row_u4;
-    for (int64_t i = threadIdx.x; i < row_u4; i += blockDim.x) y[(int64_t)blockIdx.x * row_u4 + i] = src[i];
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= n) return;
+    const uint4 *src = a + (int64_t)row_src[row] * row_u4;
+    uint4 *dst = y + row * row_u4;
+    for (int64_t i = threadIdx.x & 31; i < row_u4; i += 256) {
+        uint4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (i + 32 * u < row_u4) v[u] = src[i + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (i + 32 * u < row_u4) dst[i + 32 * u] = v[u];
+    }
 }
 
 // VEC: four numbers a thread, the slots' rows in flight together (W a multiple of four, rows on 16 bytes).  Bound by memory: 1024 x 4 rows
@@ -596,9 +678,10 @@ int ggb_op_moe_route(int dt, const void *h, int64_t W, int64_t T, const float *w
                   "moe_route: bad arguments");
     GGB_CHECK_ARG(logits != nullptr, "moe_route: needs T * n_exp floats for the logits");
     const size_t smem = (size_t)(n_exp + top) * 4;
-    const int rc = dt == GGB_TYPE_BF16 ? logits_launch((const __nv_bfloat16 *)h, W, T, w_router, bias, n_exp, logits)
-                                       : logits_launch((const float *)h, W, T, w_router, bias, n_exp, logits);
-    if (rc) return rc;
+    bool chosen = false;
+    const int rc = dt == GGB_TYPE_BF16 ? logits_launch((const __nv_bfloat16 *)h, W, T, w_router, bias, n_exp, logits, top, idx, wt, &chosen)
+                                       : logits_launch((const float *)h, W, T, w_router, bias, n_exp, logits, top, idx, wt, &chosen);
+    if (rc || chosen) return rc;
     ggb_launch_step(moe_select_kernel, dim3((unsigned)T), dim3(32), smem, logits, n_exp, top, idx, wt);
     GGB_LAUNCH_CHECK();
     return GGB_OK;
@@ -738,23 +821,26 @@ int ggb_op_moe_linear_identity(int dt, const void *w, int64_t N, int64_t K, cons
         GGB_LAUNCH_CHECK();
         return GGB_OK;
     }
-    // Portions, bf16, aligned shapes, on the tensor cores: many slots by TMA from gathered rows, in tiles of 128 rows.  Fewer through the slot list, without a
+    // Portions, bf16, aligned shapes, on the tensor cores: many slots in tiles of an expert's slots.  Fewer in the same way without a
     // workspace (such a portion may be captured, and a workspace that grows would move under the graph), every 64 numbers of K summed by
     // themselves: no further off than the multiply-adds of the tile kernel, which takes what is left.  32 experts, 1408 x 2048: 480 slots 39 us
     // (47 gathered), 20 slots 24 (33).
     if (dt == GGB_TYPE_BF16 && ggb_gemm_grouped_bf16_fits(N, K, ldc) && lda == K && ((uintptr_t)a & 15) == 0) {
         const int64_t n = T * top;
         if (n >= 512) {
+            // many slots an expert: rows gathered ahead (the product's tiles are wide, and copying them through the slot list would bound it: 768 slots an
+            // expert 56 us, 68); fewer: through the slot list (256: 28.8; 128: 42.9, 52.4; 32: 37.6, 41.5)
             const void *a_sorted = a;
-            if (gather) {
+            const bool ahead = gather && n > 256 * (int64_t)n_real;
+            if (ahead) {
                 void *gbuf;
                 const int rc = ggb_workspace(GGB_WS_MOE_GATHER, (size_t)n * (size_t)K * 2, &gbuf);
                 if (rc) return rc;
-                ggb_launch_step(moe_gather_kernel, dim3((unsigned)n), dim3(128), 0, (const uint4 *)a, K / 8, g.row_src, (uint4 *)gbuf);
+                ggb_launch_step(moe_gather_kernel, dim3((unsigned)((n + 7) / 8)), dim3(256), 0, (const uint4 *)a, K / 8, g.row_src, n, (uint4 *)gbuf);
                 GGB_LAUNCH_CHECK();
                 a_sorted = gbuf;
             }
-            return ggb_gemm_grouped_bf16(w, N, K, a_sorted, n, n_real, g.offsets, act ? nullptr : (float *)c, act ? c : nullptr, act, ldc);
+            return ggb_gemm_grouped_bf16(w, N, K, a_sorted, n, n_real, g.offsets, ahead ? nullptr : g.row_src, act ? nullptr : (float *)c, act ? c : nullptr, act, ldc);
         }
         if (K >= 128 && ((uintptr_t)w & 15) == 0) // (sums of 64: 7e-8, multiply-adds 5e-8; K = 128: 7.0e-8, 7.2e-8)
             return ggb_gemm_any_grouped(w, N, K, a, lda, n, n_real, act ? nullptr : (float *)c, ldc, act ? c : nullptr, act, g);

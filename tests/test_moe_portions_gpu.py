@@ -3,7 +3,7 @@ than its threads hold and more experts than it has threads, the weighted sum in 
 import numpy as np
 import pytest
 
-from device_util import BF16, F32, as_dt, dev, f32, i32, release, zeros
+from device_util import BF16, F32, as_dt, dev, f32, from_dt, i32, release, zeros
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +62,50 @@ def test_weighted_sum(gpu, W, top):
     gpu.check(lib.ggb_op_moe_combine(dev(gpu, y).ptr, dev(gpu, ws).ptr, dev(gpu, wt).ptr, T, top, E, W, out.ptr))
     want = (wt[:, :, None].astype(np.float64) * y[inv].reshape(T, top, W)).sum(1)
     assert np.abs(out.download(np.float32).reshape(T, W) - want).max() < top * 2.0 ** -23 * 8
+
+
+@pytest.mark.parametrize("E", [5, 8, 32])
+@pytest.mark.parametrize("T", [1203, 2400])
+def test_choice_does_not_depend_on_the_tokens_of_a_call(gpu, E, T):
+    """up to 32 experts of a portion are chosen where their logits are computed: the bits of a token by itself, ties to the lower index"""
+    W, top, r, lib = 132, 4, np.random.default_rng(E), gpu.cuda_lib()
+    h = dev(gpu, as_dt(BF16, r.standard_normal((T, W)))[1])
+    router = f32(r.standard_normal((E, W)))
+    router[E - 1] = router[1]  # equal logits
+    w, idx, wt = dev(gpu, router), zeros(gpu, T * top * 4), zeros(gpu, T * top * 4)
+    z = zeros(gpu, T * E * 4)
+    gpu.check(lib.ggb_op_moe_route(BF16, h.ptr, W, T, w.ptr, None, E, top, z.ptr, idx.ptr, wt.ptr))
+    many = idx.download(np.int32).reshape(T, top).copy(), wt.download(np.uint32).reshape(T, top).copy()
+    order = np.argsort(-z.download(np.float32).reshape(T, E), axis=1, kind="stable")[:, :top]
+    assert np.array_equal(many[0], order)
+    for t in (0, T // 2, T - 1):
+        gpu.check(lib.ggb_op_moe_route(BF16, h.ptr.value + t * W * 2, W, 1, w.ptr, None, E, top, z.ptr, idx.ptr, wt.ptr))
+        assert np.array_equal(idx.download(np.int32, top), many[0][t]) and np.array_equal(wt.download(np.uint32, top), many[1][t])
+
+
+@pytest.mark.parametrize("gather", [0, 1])
+@pytest.mark.parametrize("counts,N,K", [([0, 1, 16, 17, 31, 33, 0, 160, 255, 0], 160, 448), ([256, 257, 0], 416, 64), ([513, 1, 2], 96, 192), ([700, 900], 1408, 128),
+                                        ([3] * 300, 32, 64), ([17, 600, 0, 0], 288, 1024)])
+def test_tiles_of_slots(gpu, counts, N, K, gather):
+    """The grouped product at the edges of its tiles: halves of a tile without slots, groups without any, features that leave a CTA of a pair without work, fewer
+    blocks of K than the ring has places.  Products are exact; a running sum is truncated once per 16 of K, at most 2^-23 of it."""
+    r, lib = np.random.default_rng(len(counts) + N), gpu.cuda_lib()
+    E, n = len(counts), sum(counts)
+    assert n >= 512
+    (w, wr), (a, ar) = as_dt(BF16, r.standard_normal((E, N, K))), as_dt(BF16, r.standard_normal((n, K)))
+    idx = r.permutation(np.repeat(np.arange(E), counts))
+    ws, c, y = zeros(gpu, 4 * lib.ggb_moe_group_ints(n, E)), zeros(gpu, n * N * 4), zeros(gpu, n * N * 2)
+    gpu.check(lib.ggb_op_moe_group(dev(gpu, i32(idx)).ptr, n, 1, E, ws.ptr))
+    lists = ws.download(np.int32)
+    row_src, expert = lists[E + 1:E + 1 + n], np.repeat(np.arange(E), counts)
+    dw, da = dev(gpu, wr), dev(gpu, ar)
+    gpu.check(lib.ggb_op_moe_linear(BF16, dw.ptr, N, K, da.ptr, K, gather, n, 1, E, ws.ptr, 0, c.ptr, N))
+    gpu.check(lib.ggb_op_moe_linear(BF16, dw.ptr, N, K, da.ptr, K, gather, n, 1, E, ws.ptr, 1, y.ptr, N))  # the square of what is positive
+    rows = a[row_src] if gather else a
+    want = np.empty((n, N))
+    for e in range(E):
+        want[expert == e] = rows[expert == e] @ w[e].T
+    got = c.download(np.float32).reshape(n, N)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < (K / 16 + 8) * 2.0 ** -23 + 1e-7
+    square = from_dt(BF16, y, (n, N))
+    assert np.array_equal(square, as_dt(BF16, np.maximum(got, np.float32(0)) ** 2)[0])
