@@ -16,19 +16,19 @@
 namespace {
 
 // ------------------------------------------------------------------------------------------------ mat-vec
-// T <= kVecT activation rows: a warp owns output row n for all of them, streams the weight row once with
+// T <= kVecT activation rows: a warp, or KS of them, owns output row n for all of them, streams the weight row once with
 // 16-byte loads and keeps T accumulators.  HBM-bound (decode).
 constexpr int kVecT = 8;
 
-// acc[t] = the lane's share of row wr (K numbers) against TT rows of a
-template <typename E, int TT>
+// acc[t] = the lane's share of row wr (K numbers) against TT rows of a: pieces lane, lane + 32 KS, ...
+template <typename E, int TT, int KS = 1>
 __device__ __forceinline__ void vec_row_dot(const E *__restrict__ wr, const E *__restrict__ a, int64_t lda, int64_t K, bool vec, int lane, float (&acc)[TT]) {
     constexpr int VE = 16 / (int)sizeof(E); // elements per 16-byte load
 #pragma unroll
     for (int t = 0; t < TT; t++) acc[t] = 0.f;
     if (vec) {
 #pragma unroll 4
-        for (int64_t k = (int64_t)lane * VE; k < K; k += 32 * VE) { // several 16-byte loads of the row in flight
+        for (int64_t k = (int64_t)lane * VE; k < K; k += 32 * KS * VE) { // several 16-byte loads of the row in flight
             const uint4 wv = ldg_stream_u4(wr + k);
             const E *we = reinterpret_cast<const E *>(&wv);
             float wf[VE];
@@ -43,7 +43,7 @@ __device__ __forceinline__ void vec_row_dot(const E *__restrict__ wr, const E *_
             }
         }
     } else {
-        for (int64_t k = lane; k < K; k += 32) {
+        for (int64_t k = lane; k < K; k += 32 * KS) {
             const float wf = to_f32(wr[k]);
 #pragma unroll
             for (int t = 0; t < TT; t++) acc[t] = fmaf(wf, to_f32(a[t * lda + k]), acc[t]);
@@ -51,27 +51,64 @@ __device__ __forceinline__ void vec_row_dot(const E *__restrict__ wr, const E *_
     }
 }
 
-// ACT: the output is act(.) in the matrices' type (c_act) instead of fp32 (c)
-template <typename E, int TT, int ACT = 0>
-__global__ void __launch_bounds__(256) linear_vec_kernel(const E *w, int64_t N, int64_t K, const E *a,
+// ACT: the output is act(.) in the matrices' type (c_act) instead of fp32 (c).  KS warps share a row, their sums are added in order: few long
+// rows leave too few bytes in flight with a warp each (in a graph, matrices from memory, 2048 rows of 8192 bf16 numbers: 14 warps an SM, 13.7 us;
+// four a row: 7.3, 4.6 TB/s; two: 8.8; 2048 x 2048: 4.9, 3.5 with two; 300 x 7000: 13.3, 3.9).  One token: 32 registers, so that an SM holds 64 warps
+// (4096 x 4096 with two a row in 34 registers: 9.2 us, in two waves).
+template <typename E, int TT, int ACT, int KS>
+__global__ void __launch_bounds__(256, TT == 1 ? 8 : 0) linear_vec_kernel(const E *w, int64_t N, int64_t K, const E *a,
                                                          int64_t lda, float *c, int64_t ldc, E *c_act = nullptr) {
     constexpr int VE = 16 / (int)sizeof(E);
-    const int lane = threadIdx.x & 31;
-    const int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t n = (int64_t)blockIdx.x * (8 / KS) + warp / KS;
     step_wait();
-    if (n >= N) return;
+    if (KS == 1 && n >= N) return;
     float acc[TT];
     const bool vec = (K % VE == 0) && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(a)) % 16 == 0) &&
                      (lda % VE == 0);
-    vec_row_dot<E, TT>(w + n * K, a, lda, K, vec, lane, acc);
+    vec_row_dot<E, TT, KS>(w + (KS > 1 ? min(n, N - 1) : n) * K, a, lda, K, vec, lane + 32 * (warp % KS), acc);
+    auto put = [&](int t, float s) {
+        if (ACT) c_act[t * ldc + n] = from_f32<E>(act_f32(s, ACT));
+        else c[t * ldc + n] = s;
+    };
+    if constexpr (KS == 1) {
 #pragma unroll
-    for (int t = 0; t < TT; t++) {
-        const float s = warp_sum_f32(acc[t]);
-        if (lane == 0) {
-            if (ACT) c_act[t * ldc + n] = from_f32<E>(act_f32(s, ACT));
-            else c[t * ldc + n] = s;
+        for (int t = 0; t < TT; t++) {
+            const float s = warp_sum_f32(acc[t]);
+            if (lane == 0) put(t, s);
         }
+    } else {
+        __shared__ float red[8][TT];
+#pragma unroll
+        for (int t = 0; t < TT; t++) {
+            const float s = warp_sum_f32(acc[t]);
+            if (lane == 0) red[warp][t] = s;
+        }
+        __syncthreads();
+        if (warp % KS != 0 || n >= N || lane >= TT) return;
+        float s = red[warp][lane];
+#pragma unroll
+        for (int i = 1; i < KS; i++) s += red[warp + i][lane];
+        put(lane, s);
     }
+}
+
+// Warps a row: doubled while there are 32 of them an SM at most (24 with the registers of more tokens) and each still has two rounds of 16-byte loads; beyond
+// that, up to what an SM holds, while each has four (one token; with four and more, which run in waves then, eight)
+template <typename E> int vec_splits(int64_t N, int64_t K, int T) {
+    const int64_t rounds = K * (int64_t)sizeof(E) / 512, held = (T <= 3 ? 32 : 24) * ggb_sm_count(), most = (T == 2 || T == 3 ? 40 : 64) * ggb_sm_count();
+    int ks = 1;
+    while (ks < 8 && N * ks * 2 <= most && rounds >= ks * 2 * (N * ks * 2 <= held ? 2 : T <= 3 ? 4 : 8)) ks *= 2;
+    return ks;
+}
+template <typename E, int TT, int ACT>
+void vec_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, float *c, int64_t ldc, E *c_act) {
+    const int ks = vec_splits<E>(N, K, TT);
+    const dim3 grid((unsigned)((N + 8 / ks - 1) / (8 / ks))), block(256);
+    if (ks == 8) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 8>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
+    else if (ks == 4) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 4>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
+    else if (ks == 2) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 2>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
+    else ggb_launch_step(linear_vec_kernel<E, TT, ACT, 1>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
 }
 
 // ------------------------------------------------------------------------------------------------ tile kernel
@@ -328,9 +365,8 @@ __global__ void cvt_to_f32_kernel(const E *__restrict__ x, int64_t n, float *__r
 template <typename E>
 int linear_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, int64_t T, float *c, int64_t ldc) {
     if (T <= kVecT) {
-        const dim3 grid((unsigned)((N + 7) / 8));
         switch ((int)T) {
-#define VEC_CASE(TT) case TT: ggb_launch_step(linear_vec_kernel<E, TT>, grid, dim3(256), 0, w, N, K, a, lda, c, ldc, nullptr); break;
+#define VEC_CASE(TT) case TT: vec_launch<E, TT, 0>(w, N, K, a, lda, c, ldc, nullptr); break;
             VEC_CASE(1) VEC_CASE(2) VEC_CASE(3) VEC_CASE(4) VEC_CASE(5) VEC_CASE(6) VEC_CASE(7) VEC_CASE(8)
 #undef VEC_CASE
         }
@@ -348,9 +384,8 @@ int linear_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, int
 template <typename E, int ACT>
 int linear_act_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, int64_t T, E *y) {
     if (T <= kVecT) {
-        const dim3 grid((unsigned)((N + 7) / 8));
         switch ((int)T) {
-#define VEC_CASE(TT) case TT: ggb_launch_step(linear_vec_kernel<E, TT, ACT>, grid, dim3(256), 0, w, N, K, a, lda, nullptr, N, y); break;
+#define VEC_CASE(TT) case TT: vec_launch<E, TT, ACT>(w, N, K, a, lda, nullptr, N, y); break;
             VEC_CASE(1) VEC_CASE(2) VEC_CASE(3) VEC_CASE(4) VEC_CASE(5) VEC_CASE(6) VEC_CASE(7) VEC_CASE(8)
 #undef VEC_CASE
         }

@@ -57,6 +57,22 @@ def test_linear_any_shape(gpu, dt, T, N, K):
 
 
 @pytest.mark.parametrize("dt", [F32, BF16])
+@pytest.mark.parametrize("T,N,K", [(1, 2048, 8192), (3, 33, 8200), (8, 2047, 4096), (2, 4736, 2048), (1, 4737, 2048), (1, 1, 8191), (5, 700, 1024), (4, 9473, 1024)])
+def test_linear_of_few_tokens_and_long_rows(gpu, dt, T, N, K):
+    """one to eight warps a row: sums of K products in fp32"""
+    r = np.random.default_rng(N)
+    (wv, wu), (av, au) = as_dt(dt, r.standard_normal((N, K))), as_dt(dt, r.standard_normal((T, K)))
+    c, es = gpu.DeviceBuffer(T * N * 4), 2 if dt == BF16 else 4
+    y = gpu.DeviceBuffer(T * N * es)
+    w, a = dev(gpu, wu), dev(gpu, au)
+    gpu.check(gpu.cuda_lib().ggb_op_linear(dt, w.ptr, N, K, a.ptr, K, T, c.ptr, N), "linear")
+    gpu.check(gpu.cuda_lib().ggb_op_linear_act(dt, w.ptr, N, K, a.ptr, K, T, 1, y.ptr), "linear_act")
+    want = av @ wv.T
+    assert F.rel_err(c.download(np.float32).reshape(T, N), want) < 2e-6
+    assert F.rel_err(from_dt(dt, y, (T, N)), np.maximum(want, 0) ** 2) < (2.5e-3 if dt == BF16 else 4e-6)
+
+
+@pytest.mark.parametrize("dt", [F32, BF16])
 def test_rms_norm_one_number_and_vector(gpu, dt):
     r = np.random.default_rng(0)
     T, E, eps = 5, 77, 1e-3
