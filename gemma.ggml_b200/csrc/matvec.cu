@@ -10,6 +10,8 @@
 //     round through a shuffle chain), so every output is bit-identical to ggml's scalar vec_dot.
 //     This per-operator form is the fallback / T > 1 lowering; the persistent decode kernel
 //     (decoder.cu) produces the same bits with a dedicated chain warp.
+#include <string.h>
+
 #include "dot.cuh"
 
 namespace {
@@ -56,6 +58,58 @@ __global__ void __launch_bounds__(kMvWarps * 32) matvec_kernel(const MatvecArgs 
         if (a.m[mi].resid) v = __fadd_rn(v, a.m[mi].resid[(int64_t)blockIdx.y * a.dst_stride + r]);
         dst[r] = v;
     }
+}
+
+// The rows of a host program's call (ggb_mul_mat): its Q8_0 blocks come with the launch, as a parameter, and each result goes to page-locked host memory beside
+// the number of the call, for which the host looks: no copy, no second launch, no synchronisation, and no fence (a word of eight bytes arrives whole; with a
+// flag behind the results, 256 CTAs' fences to the host take 6 us).  Every CTA orders one row's blocks in shared memory.  Bound by latency: 2048 x 2048, Q4_0:
+// a call takes 15.4 us (30.3 with copies from and to the program's memory, another launch that orders the blocks, and a synchronisation).
+template <int BYTES> struct host_rows_args {
+    const uint8_t *qs;
+    const __half *d;
+    int64_t rows, nb;
+    uint2 *out; // [T][rows] {result, call}, host memory
+    uint32_t call;
+    uint32_t raw[BYTES / 4]; // [T][nb] blocks of a scale and 32 numbers
+};
+
+template <int TYPE, int BYTES>
+__global__ void __launch_bounds__(kMvWarps * 32) matvec_host_rows_kernel(const __grid_constant__ host_rows_args<BYTES> a) {
+    extern __shared__ __align__(16) uint8_t mv_row[];
+    __shared__ float sums[kMvWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t cols = a.nb * GGB_QK, r0 = (int64_t)blockIdx.x * kMvWarps, r = r0 + warp;
+    constexpr int PB = TYPE == GGB_TYPE_Q4_0 ? 16 : 32;
+    if (r < a.rows) // the weights are on their way while the blocks are ordered
+        for (int64_t o = lane * 128; o < a.nb * PB; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.qs + r * a.nb * PB + o));
+    uint64_t at = reinterpret_cast<uint64_t>(&a.raw[0]); // by ordinary loads: a constant one takes a turn for each of a warp's addresses
+    asm volatile("" : "+l"(at));
+    const uint16_t *raw = reinterpret_cast<const uint16_t *>(at) + (int64_t)blockIdx.y * a.nb * 17;
+    for (int i = threadIdx.x; i < (int)a.nb * 17; i += kMvWarps * 32) {
+        const int b = i / 17, j = i - 17 * b;
+        *reinterpret_cast<uint16_t *>(mv_row + (j ? 32 * b + 2 * (j - 1) : cols + 2 * b)) = raw[i];
+    }
+    __syncthreads();
+    if (r < a.rows) {
+        const float v = row_dot_ref<TYPE>(a.qs, a.d, r, a.nb, mv_row, cols, lane);
+        if (lane == 0) sums[warp] = v;
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    if (lane < kMvWarps && r0 + lane < a.rows) // eight words of eight bytes: a line of the host
+        asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(a.out + (int64_t)blockIdx.y * a.rows + r0 + lane), "r"(__float_as_uint(sums[lane])), "r"(a.call) : "memory");
+}
+
+template <int TYPE, int BYTES>
+int launch_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call) {
+    host_rows_args<BYTES> a;
+    a.qs = w->qs, a.d = w->d, a.rows = w->rows, a.nb = w->nb;
+    a.out = out, a.call = call;
+    for (int64_t t = 0; t < T; t++) memcpy(reinterpret_cast<char *>(a.raw) + t * w->nb * 34, blocks + t * row_size, (size_t)w->nb * 34);
+    const dim3 grid((unsigned)((w->rows + kMvWarps - 1) / kMvWarps), (unsigned)T);
+    matvec_host_rows_kernel<TYPE, BYTES><<<grid, kMvWarps * 32, (size_t)((w->nb * 34 + 15) & ~15ll), ggb_cuda_stream()>>>(a);
+    GGB_LAUNCH_CHECK();
+    return GGB_OK;
 }
 
 // FFN front half: one CTA per 32 output rows: gate and up dots, GeGLU through the fp16 gelu
@@ -135,7 +189,23 @@ int launch_matvec(int n, const ggb_weight *const *w, const void *q8, int64_t T, 
     return GGB_OK;
 }
 
+// Sizes of the parameter: a launch takes all of it along.  2048 columns are 2176 bytes, 8192 are 8704; a kernel's parameters are 32764 bytes at most.
+constexpr int kHostRows[3] = {3840, 8832, 32000};
+
+template <int TYPE> int host_rows_of(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call) {
+    const int64_t bytes = T * w->nb * 34;
+    if (bytes <= kHostRows[0]) return launch_host_rows<TYPE, kHostRows[0]>(w, blocks, T, row_size, out, call);
+    if (bytes <= kHostRows[1]) return launch_host_rows<TYPE, kHostRows[1]>(w, blocks, T, row_size, out, call);
+    return launch_host_rows<TYPE, kHostRows[2]>(w, blocks, T, row_size, out, call);
+}
+
 } // namespace
+
+bool ggb_matvec_host_rows_fits(const ggb_weight *w, int64_t T) { return T * w->nb * 34 <= kHostRows[2] && T < 65536; }
+int ggb_matvec_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call) {
+    return w->type == GGB_TYPE_Q4_0 ? host_rows_of<GGB_TYPE_Q4_0>(w, blocks, T, row_size, out, call)
+                                    : host_rows_of<GGB_TYPE_Q8_0>(w, blocks, T, row_size, out, call);
+}
 
 extern "C" {
 

@@ -3,8 +3,10 @@
 // Same fields, HOST pointers, synchronous.  Where the reference split rows 90/10 between a CPU
 // thread pool and a verify-only OpenCL kernel (src/hpc.cpp:245-277, src/kernals.cl:203-211), every
 // row is computed on the B200; src0 is uploaded (+ repacked for Q4_0 / Q8_0) once and cached, only the
-// activations (wdata) and the result cross PCIe per call.  Types: Q4_0 / Q8_0 (the benchmark's), and the three
+// activations (wdata) and the result cross PCIe per call (few of them without copies: matvec.cu).  Types: Q4_0 / Q8_0 (the benchmark's), and the three
 // the reference's kernels cover, Q4_K / Q6_K / F16 (kquants.cu).
+#include <string.h>
+
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -51,6 +53,38 @@ int copy_back(void *dst_data, int64_t col_num, int64_t ne01, int64_t ne12, int64
         }
     }
     GGB_CUDA(cudaStreamSynchronize(st));
+    return GGB_OK;
+}
+
+// Few results: page-locked memory that the kernel writes, a word of a result and the number of the call each.  Beyond kPinnedResults a copy engine's lines
+// are fuller.
+constexpr int64_t kPinnedResults = 16 * 1024;
+uint64_t *g_pinned = nullptr;
+uint32_t g_call = 0;
+
+int ensure_pinned() {
+    if (g_pinned) return GGB_OK;
+    void *p = nullptr;
+    GGB_CUDA(cudaHostAlloc(&p, kPinnedResults * 8, cudaHostAllocMapped | cudaHostAllocPortable));
+    memset(p, 0, kPinnedResults * 8);
+    g_pinned = (uint64_t *)p;
+    return GGB_OK;
+}
+
+// n results of this call from word `first` on, each as soon as it is there, or an error when the stream says that it never will be
+int take_results(float *dst, int64_t first, int64_t n, cudaStream_t st) {
+    for (int64_t i = 0; i < n; i++) {
+        uint64_t w;
+        for (int spins = 1; (w = __atomic_load_n(g_pinned + first + i, __ATOMIC_ACQUIRE)) >> 32 != g_call; spins++) {
+            if (spins % 2000) continue;
+            const cudaError_t e = cudaStreamQuery(st);
+            if (e == cudaErrorNotReady || (e == cudaSuccess && __atomic_load_n(g_pinned + first + i, __ATOMIC_ACQUIRE) >> 32 == g_call)) continue;
+            ggb_set_error("mul_mat: %s", e == cudaSuccess ? "the kernel left no result" : cudaGetErrorString(e));
+            return GGB_ERR_CUDA;
+        }
+        const uint32_t v = (uint32_t)w;
+        memcpy(dst + i, &v, 4);
+    }
     return GGB_OK;
 }
 
@@ -147,8 +181,21 @@ int ggb_mul_mat(int64_t ne01, int64_t ne11, int64_t ne12, int64_t nb01, int64_t 
         w = it->second;
     }
 
-    // 2. activations: AoS Q8_0 rows -> device -> planar
+    // 2. few rows and results: both travel with one kernel (a capture takes neither a wait nor host memory that changes: it is refused below, by the copies)
     const int64_t col_num = ne11 * ne12; // ref: src/hpc.cpp:232
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (col_num * ne01 <= kPinnedResults && ggb_matvec_host_rows_fits(w, col_num) && cudaStreamIsCapturing(ggb_cuda_stream(), &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone) {
+        int rc = ensure_pinned();
+        if (rc) return rc;
+        if (++g_call == 0) g_call = 1; // what no call has written is zero
+        rc = ggb_matvec_host_rows(w, wdata, col_num, (int64_t)row_size, (uint2 *)g_pinned, g_call);
+        for (int64_t col = 0; col < col_num && !rc; col++) // the reference's addressing, as in copy_back
+            rc = take_results((float *)((char *)dst_data + (col % ne1) * nb1 + (col / ne1) * nb2), col * ne01, ne01, ggb_cuda_stream());
+        return rc;
+    }
+
+    //    others: AoS Q8_0 rows -> device -> planar
     const size_t q8_stride = ggb_q8_row_bytes(K);
     int rc;
     if ((rc = ensure(&g_act_raw, &g_act_raw_cap, (size_t)col_num * row_size))) return rc;

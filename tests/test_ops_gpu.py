@@ -160,6 +160,32 @@ def test_mul_mat_dropin_host_pointers(gpu, wtype, k, n, T):
     assert np.abs(got - O.mul_mat(wtype, O.REF, w, a, k)).max() < 1e-4
 
 
+@pytest.mark.parametrize("wtype", [O.TYPE_Q4_0, O.TYPE_Q8_0])
+@pytest.mark.parametrize("k,n,T", [(32, 1, 1), (3584, 9, 1), (3616, 7, 1), (1184, 65, 3), (8288, 33, 1), (8320, 8, 1), (15040, 5, 2), (15072, 5, 2), (64, 16384, 1), (64, 16385, 1),
+                                   (96, 2048, 8), (96, 2049, 8)])
+def test_mul_mat_dropin_by_parameter_and_by_copies(gpu, wtype, k, n, T):
+    """at the sizes where the rows of a call no longer fit the launch's parameter (three sizes of it) or its results the page-locked buffer; calls that follow
+    one another with other rows, a result with gaps, several threads"""
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(k + n + T)
+    L = gpu.cuda_lib()
+    w = O.quantize(wtype, rng.standard_normal((n, k)).astype(np.float32) * 0.02)
+    rows = [O.quantize(O.TYPE_Q8_0, rng.standard_normal((T, k)).astype(np.float32)) for _ in range(4)]
+    want = [bits(O.mul_mat(wtype, O.REF, w, a, k)) for a in rows]
+    pitch = n + 3
+
+    def call(a):
+        dst = np.full((T, pitch), np.float32(-3))
+        gpu.check(L.ggb_mul_mat(n, T, 1, w.shape[1], T, pitch * 4, pitch * 4 * T, a.shape[1], k, w.ctypes.data, dst.ctypes.data, wtype, a.ctypes.data))
+        return dst
+
+    with ThreadPoolExecutor(4) as pool:
+        for got in ([call(a) for a in rows], list(pool.map(call, rows))):
+            for g, x in zip(got, want):
+                assert np.array_equal(bits(np.ascontiguousarray(g[:, :n])), x) and (g[:, n:] == -3).all()
+    L.ggb_mul_mat_forget(w.ctypes.data)
+
+
 def test_mul_mat_dropin_strided_dst_and_errors(gpu):
     rng = np.random.default_rng(3)
     k, n, T = 64, 10, 3
