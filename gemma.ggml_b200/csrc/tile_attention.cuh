@@ -27,6 +27,8 @@
 // queries x 32 keys); 777 tokens of sigmoid heads at position 1024, no window: 53 us (64 us; 686 us).
 #pragma once
 
+#include <algorithm>
+
 #include "dense.cuh"
 #include "tc.cuh"
 
@@ -175,7 +177,7 @@ struct mma_args {
     volatile int *dead;
 };
 // the warp that issues every MMA.  KS: D / 16, or 0 for a number known at run time only
-template <int MAPS, int KS> __device__ __forceinline__ void mma_role(const mma_args &m) {
+template <int MAPS, bool SPLIT, int KS> __device__ __forceinline__ void mma_role(const mma_args &m) {
     const uint32_t id_s = umma_idesc(128, kKeys), id_o = umma_idesc(128, m.Dv, true);
     const uint32_t q_lo = umma_desc_lo(m.sq, 16), k_lo = umma_desc_lo(m.sk, 16), v_lo = umma_desc_lo(m.sv, kKeys * 128);
     auto scores = [&](int n) {
@@ -205,6 +207,7 @@ template <int MAPS, int KS> __device__ __forceinline__ void mma_role(const mma_a
         umma_arrive(m.bars + S_FULL + 8 * s);
         umma_arrive(m.bars + K_FREE + 8 * s);
     };
+    if (SPLIT && m.NT == 0) return;
     mbar_wait_bounded(m.bars + Q_FULL, 0, m.dead);
     scores(0);
     if (m.NT > 1) scores(1);
@@ -269,13 +272,12 @@ template <int MODE> __device__ __forceinline__ void plain_row(const row_job &j, 
     __syncwarp();
 }
 
-// the rows of a warp's set bits (row warp + kWarps b) once more; out of line, so that the code that every call runs through stays short
+// the rows first + step b of a CTA, b the set bits, once more; out of line, so that the code that every call runs through stays short
 template <int MODE, int MAPS>
-__device__ __noinline__ void plain_rows(const shape &a, uint32_t again, int64_t t0, int64_t i0, int g, int hpg, int n_pairs, float *of, float *st) {
+__device__ __noinline__ void plain_rows(const shape &a, uint32_t again, int first, int step, int64_t t0, int64_t i0, int g, int hpg, int n_pairs, float *of, float *st) {
     constexpr int PR = kRows / MAPS;
-    const int warp = threadIdx.x >> 5;
     while (again) {
-        const int rr = warp + kWarps * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
+        const int rr = first + step * (__ffs((int)again) - 1), rm = MAPS == 1 ? 0 : rr / PR, rp = rr - rm * PR, rq = rp / hpg, h = g * hpg + (rp - rq * hpg);
         again &= again - 1;
         if (rp >= n_pairs) continue;
         row_job j{a.q + (((t0 + rq) * a.H + h) * MAPS + rm) * a.D, a.cache + ((int64_t)g * MAPS + rm) * a.D, a.cache + (int64_t)a.G * MAPS * a.D + (int64_t)g * a.Dv,
@@ -286,9 +288,40 @@ __device__ __noinline__ void plain_rows(const shape &a, uint32_t again, int64_t 
     }
 }
 
+// Few CTAs take a cluster each, whose `parts` CTAs have the key tiles in turn.  One row of it by one warp: the parts' sums from their shared memory, added in order
+// relative to the largest maximum, over this CTA's.  false: one of them is not finite
+template <int MODE> __device__ __forceinline__ bool gather_row(int parts, int rr, int Dv, float *of, float *st) {
+    const int lane = threadIdx.x & 31;
+    const float odd = lane < 4 * parts ? ld_cluster_f32(cluster_addr(smem_u32(st + (2 + (lane & 3)) * kRows + rr), lane >> 2)) : 0.f; // a part's four quarters
+    if (__any_sync(0xffffffffu, odd != 0.f)) return false;
+    const uint32_t row = smem_u32(of + rr * (Dv + 1));
+    float f = lane < parts ? 1.f : 0.f;
+    if (MODE == SOFTMAX) {
+        const uint32_t at = cluster_addr(smem_u32(st + rr), min(lane, parts - 1));
+        const float m = ld_cluster_f32(at), l = ld_cluster_f32(at + 4 * kRows), M = warp_max_f32(lane < parts ? m : -INFINITY);
+        f = lane < parts && m != -INFINITY ? expf(m - M) : 0.f;
+        float L = 0.f;
+        for (int z = 0; z < parts; z++) L = fmaf(__shfl_sync(0xffffffffu, l, z), __shfl_sync(0xffffffffu, f, z), L);
+        if (lane == 0) st[rr] = M, st[kRows + rr] = L;
+    }
+    float x[4] = {0.f, 0.f, 0.f, 0.f}; // Dv <= 128
+    for (int z = 0; z < parts; z++) {
+        const uint32_t from = cluster_addr(row, z) + 4 * lane;
+        const float fz = __shfl_sync(0xffffffffu, f, z);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (lane + 32 * u < Dv) x[u] = fmaf(ld_cluster_f32(from + 128 * u), fz, x[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (lane + 32 * u < Dv) of[rr * (Dv + 1) + lane + 32 * u] = x[u];
+    return true;
+}
+
 // FIN: what becomes of a row, a warp's work when the sums stand in shared memory: load() requests what a row needs from memory, row()
 // gets it with the sums of the row (of both maps) and their maximum and denominators
-template <int MODE, int MAPS, typename FIN>
+// SPLIT: a cluster of CTAs shares the key tiles
+template <int MODE, int MAPS, bool SPLIT, typename FIN>
 __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant__ shape a, const FIN fin) {
     extern __shared__ uint8_t ta_raw[];
     const uint32_t raw0 = smem_u32(ta_raw), base = (raw0 + 1023u) & ~1023u;
@@ -330,7 +363,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     early_wait();
     const int64_t i0 = (int64_t)*a.pos0 + t0, i_last = i0 + nq - 1;
     const tiles tl(first_visible(i0, a.window, a.chunked), MODE == SOFTMAX ? a.keep : 0, i_last);
-    const int NT = tl.n;
+    // tiles z, z + parts, ...; three a part at least, and a CTA too many has none
+    const int z = SPLIT ? blockIdx.z : 0, parts = SPLIT ? max(1, min((int)gridDim.z, tl.n / 3)) : 1, NT = !SPLIT ? tl.n : z < parts ? (tl.n - 1 - z) / parts + 1 : 0;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -355,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
             uint32_t my_row[2];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
-                const uint32_t j = (uint32_t)min(tl.first(n) + 32 * u + lane, tl.last(n)), pg = j / (uint32_t)a.B;
+                const uint32_t j = (uint32_t)min(tl.first(z + n * parts) + 32 * u + lane, tl.last(z + n * parts)), pg = j / (uint32_t)a.B;
                 my_row[u] = (uint32_t)a.table[pg] * (uint32_t)a.B + (j - pg * a.B);
             }
             if (n >= 2) mbar_wait_warp(bars + fre + 8 * s, ((n >> 1) - 1) & 1, dead);
@@ -379,10 +413,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     } else if (warp == kMmaWarp) {
         // the whole warp, converged; a number of K steps known to the compiler makes an MMA a few instructions
         const mma_args ma{bars, base, q_split, sk, k_stage, k_part, sv, v_stage, tmem, reg_cols, o_col, a.D / 16, a.Dv, NT, dead};
-        if (a.D == 128) mma_role<MAPS, 8>(ma);
-        else if (a.D == 64) mma_role<MAPS, 4>(ma);
-        else mma_role<MAPS, 0>(ma);
-    } else if (warp < kWarps) {
+        if (a.D == 128) mma_role<MAPS, SPLIT, 8>(ma);
+        else if (a.D == 64) mma_role<MAPS, SPLIT, 4>(ma);
+        else mma_role<MAPS, SPLIT, 0>(ma);
+    } else if (warp < kWarps && (!SPLIT || NT > 0)) {
         // the rows of q as three bf16 numbers each, rows and coordinates past the end as zeros: four numbers a thread, eight loads in flight
         {
             const int gpr = 16 * D64, n_items = kRows * gpr;
@@ -428,8 +462,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         float *mypen = pen + grp * hpg * pitch;
         if (MODE == SIGMOID && a.pb && live) hpb = a.pb[g * hpg + hh];
         for (int n = grp; n < NT; n += 2) {
-            const int64_t j0 = tl.first(n), jl = min(tl.last(n), j0 + kKeys - 1);
-            const bool whole = jl - j0 == kKeys - 1 && jl <= i0 && (n < tl.n_kt || j0 >= first_visible(i_last, a.window, a.chunked));
+            const int tile = z + n * parts;
+            const int64_t j0 = tl.first(tile), jl = min(tl.last(tile), j0 + kKeys - 1);
+            const bool whole = jl - j0 == kKeys - 1 && jl <= i0 && (tile < tl.n_kt || j0 >= first_visible(i_last, a.window, a.chunked));
             if (MODE == SIGMOID && a.r1) { // the penalties a tile can meet: distances (i0 - j0) + qi - jj, qi < TQ, jj < 64
                 if (n > grp) bar_sync(1 + grp, 256);
                 for (int e = (tid & 255); e < hpg * (TQ + kKeys - 1); e += 256) {
@@ -575,28 +610,40 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
         }
         st[(2 + quarter) * kRows + r] = odd;
         bar_sync(3, 32 * kWarps);
-        // a warp's 8 rows: warp, warp + 16, ...; those whose sums are not finite once more, without the split
-        {
+        if (SPLIT && parts > 1) { // this CTA's pairs: z, z + parts, ...
+            __syncwarp();
+            cluster_sync(); // the sums of all parts stand
+            for (int p = z + parts * warp; p < n_pairs; p += parts * kWarps)
+                for (int rr = p; rr < kRows; rr += PR)
+                    if (!gather_row<MODE>(parts, rr, a.Dv, of, st)) plain_rows<MODE, MAPS>(a, 1u, rr, 0, t0, i0, g, hpg, n_pairs, of, st);
+            __syncwarp();
+            cluster_sync(); // and are read
+        } else { // a warp's 8 rows: warp, warp + 16, ...; those whose sums are not finite once more, without the split
             const float *er = st + warp + kWarps * (lane & 7);
             const uint32_t again = __ballot_sync(0xffffffffu, (er[2 * kRows] + er[3 * kRows]) + (er[4 * kRows] + er[5 * kRows]) != 0.f) & 0xffu;
-            if (again) plain_rows<MODE, MAPS>(a, again, t0, i0, g, hpg, n_pairs, of, st);
+            if (again) plain_rows<MODE, MAPS>(a, again, warp, kWarps, t0, i0, g, hpg, n_pairs, of, st);
         }
         // a warp a row, four rows' reads from memory in flight
-        for (int p0 = warp; p0 < n_pairs; p0 += 4 * kWarps) {
+        for (int p0 = z + parts * warp; p0 < n_pairs; p0 += 4 * parts * kWarps) {
             typename FIN::reads rd[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int p = min(p0 + kWarps * u, n_pairs - 1), pq = p / hpg;
+                const int p = min(p0 + parts * kWarps * u, n_pairs - 1), pq = p / hpg;
                 fin.load(rd[u], i0 + pq, t0 + pq, g * hpg + (p - pq * hpg), lane);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int p = p0 + kWarps * u, pq = p / hpg;
+                const int p = p0 + parts * kWarps * u, pq = p / hpg;
                 if (p >= n_pairs) break;
                 fin.row(rd[u], of + p * op, of + (p + PR) * op, st[p], st[kRows + p], MAPS == 2 ? st[kRows + p + PR] : 0.f, t0 + pq, g * hpg + (p - pq * hpg), lane);
             }
         }
         tc_fence_before();
+    }
+    if (SPLIT && !(warp < kWarps && parts > 1 && NT > 0)) { // the other threads of a cluster come by both of its barriers, too
+        __syncwarp();
+        cluster_sync();
+        cluster_sync();
     }
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -607,13 +654,23 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     }
 }
 
+// Few CTAs (few key heads, portions that are not long) leave SMs without work: up to eight CTAs then share a CTA's key tiles, as many as there are SMs for.  How many
+// positions come before the portion is known on the device only, and a cluster costs 2 us, so that the portion itself (or its window) has to hold three tiles a part.
+// Heads of 128, graph replays: 1000 tokens x 4 heads (1 key head) at position 900, four parts 26.4 us (48.5 alone); 500 tokens of 4 sigmoid heads (1) at 1000, two
+// parts 31.7 (45.5); 480 tokens x 8 heads (8) of 64 at position 0 17.9 (17.8).  128 tokens at position 700 would take 18.4 in eight parts (28.0), but at position 0
+// 17.5 (14.3).
 template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin) {
-    const size_t smem = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G);
-    auto kfn = attn_kernel<MODE, MAPS, FIN>;
+    const int TQ = kRows / MAPS / (a.H / a.G);
+    const int64_t ctas = (a.T + TQ - 1) / TQ * a.G, most = (a.window > 0 ? std::min(a.T, a.window) : a.T) / (3 * kKeys);
+    unsigned parts = 1;
+    while (parts < 8 && parts * 2 <= most && ctas * parts * 2 <= ggb_sm_count()) parts *= 2;
+    size_t smem = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G);
+    if (parts > 1) smem = std::max(smem, kOneCtaSmem); // clusters with tensor memory
+    auto kfn = parts > 1 ? attn_kernel<MODE, MAPS, true, FIN> : attn_kernel<MODE, MAPS, false, FIN>;
     const int rc = ggb_allow_smem(kfn, smem);
     if (rc) return rc;
-    const int TQ = kRows / MAPS / (a.H / a.G);
-    GGB_CUDA(ggb_launch_early(kfn, ggb_cluster{1, 1, 1}, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G), dim3(kThreads), smem, a, fin));
+    const ggb_cluster cluster{1, 1, parts};
+    GGB_CUDA(ggb_launch_early(kfn, cluster, dim3((unsigned)((a.T + TQ - 1) / TQ), (unsigned)a.G, parts), dim3(kThreads), smem, a, fin));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
