@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * kLogitWarps) moe_logits_tile_kernel(const
 }
 
 // The form by the number of logits: below a warp for every scheduler of the chip, tiles would leave SMs idle; eight tokens a warp where that still is
-// a CTA for two SMs of three, since a CTA of four reads the router as often for half the tokens.  chosen: idx and wt have been computed too
+// a CTA for two SMs of three: a CTA of four reads the router as often for half the tokens (1024 tokens x 32 experts of 2048: 10.6 us, with four 12.6).  chosen: idx and wt have been computed too
 template <typename E>
 int logits_launch(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, float *z, int top = 0, int32_t *idx = nullptr, float *wt = nullptr,
                   bool *chosen = nullptr) {

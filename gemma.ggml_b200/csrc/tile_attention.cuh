@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
 // positions come before the portion is known on the device only, and a cluster costs 2 us, so that the portion itself (or its window) has to hold three tiles a part.
 // Heads of 128, graph replays: 1000 tokens x 4 heads (1 key head) at position 900, four parts 26.4 us (48.5 alone); 500 tokens of 4 sigmoid heads (1) at 1000, two
 // parts 31.7 (45.5); 480 tokens x 8 heads (8) of 64 at position 0 17.9 (17.8).  128 tokens at position 700 would take 18.4 in eight parts (28.0), but at position 0
-// 17.5 (14.3).
+// 17.5 (14.3).  With more CTAs than SMs two parts cost: 777 tokens of 16 sigmoid heads (4) at 1024, 100 CTAs: 63.8 (53.6).
 template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin) {
     const int TQ = kRows / MAPS / (a.H / a.G);
     const int64_t ctas = (a.T + TQ - 1) / TQ * a.G, most = (a.window > 0 ? std::min(a.T, a.window) : a.T) / (3 * kKeys);
