@@ -77,9 +77,9 @@ static inline int ggb_payload_bytes(int type) { return type == GGB_TYPE_Q4_0 ? 1
 static inline int ggb_block_bytes(int type) { return type == GGB_TYPE_Q4_0 ? 18 : 34; }
 
 // The mat-vecs of a host program's call (matvec.cu): T rows of nb Q8_0 blocks in host memory; each result goes to `out` [T][rows] in page-locked host memory as
-// {result, call}
+// one word, the call in its upper half
 bool ggb_matvec_host_rows_fits(const ggb_weight *w, int64_t T);
-int ggb_matvec_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call);
+int ggb_matvec_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint64_t *out, uint32_t call);
 
 // ---- device helpers -------------------------------------------------------
 #ifdef __CUDACC__

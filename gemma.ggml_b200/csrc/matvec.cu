@@ -61,14 +61,14 @@ __global__ void __launch_bounds__(kMvWarps * 32) matvec_kernel(const MatvecArgs 
 }
 
 // The rows of a host program's call (ggb_mul_mat): its Q8_0 blocks come with the launch, as a parameter, and each result goes to page-locked host memory beside
-// the number of the call, for which the host looks: no copy, no second launch, no synchronisation, and no fence (a word of eight bytes arrives whole; with a
-// flag behind the results, 256 CTAs' fences to the host take 6 us).  Every CTA orders one row's blocks in shared memory.  Bound by latency: 2048 x 2048, Q4_0:
+// the number of the call, for which the host looks: no copy, no second launch, no synchronisation, and no fence (both are one scalar store of eight bytes, which
+// arrives whole; a vector store's numbers are stores of their own, in no stated order.  With a flag behind the results, 256 CTAs' fences to the host take 6 us).  Every CTA orders one row's blocks in shared memory.  Bound by latency: 2048 x 2048, Q4_0:
 // a call takes 15.4 us (30.3 with copies from and to the program's memory, another launch that orders the blocks, and a synchronisation).
 template <int BYTES> struct host_rows_args {
     const uint8_t *qs;
     const __half *d;
     int64_t rows, nb;
-    uint2 *out; // [T][rows] {result, call}, host memory
+    uint64_t *out; // [T][rows] the result, above it the number of the call; host memory
     uint32_t call;
     uint32_t raw[BYTES / 4]; // [T][nb] blocks of a scale and 32 numbers
 };
@@ -97,11 +97,11 @@ __global__ void __launch_bounds__(kMvWarps * 32) matvec_host_rows_kernel(const _
     __syncthreads();
     if (warp != 0) return;
     if (lane < kMvWarps && r0 + lane < a.rows) // eight words of eight bytes: a line of the host
-        asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(a.out + (int64_t)blockIdx.y * a.rows + r0 + lane), "r"(__float_as_uint(sums[lane])), "r"(a.call) : "memory");
+        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(a.out + (int64_t)blockIdx.y * a.rows + r0 + lane), "l"((uint64_t)a.call << 32 | __float_as_uint(sums[lane])) : "memory");
 }
 
 template <int TYPE, int BYTES>
-int launch_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call) {
+int launch_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint64_t *out, uint32_t call) {
     host_rows_args<BYTES> a;
     a.qs = w->qs, a.d = w->d, a.rows = w->rows, a.nb = w->nb;
     a.out = out, a.call = call;
@@ -192,7 +192,7 @@ int launch_matvec(int n, const ggb_weight *const *w, const void *q8, int64_t T, 
 // Sizes of the parameter: a launch takes all of it along.  2048 columns are 2176 bytes, 8192 are 8704; a kernel's parameters are 32764 bytes at most.
 constexpr int kHostRows[3] = {3840, 8832, 32000};
 
-template <int TYPE> int host_rows_of(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call) {
+template <int TYPE> int host_rows_of(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint64_t *out, uint32_t call) {
     const int64_t bytes = T * w->nb * 34;
     if (bytes <= kHostRows[0]) return launch_host_rows<TYPE, kHostRows[0]>(w, blocks, T, row_size, out, call);
     if (bytes <= kHostRows[1]) return launch_host_rows<TYPE, kHostRows[1]>(w, blocks, T, row_size, out, call);
@@ -202,7 +202,7 @@ template <int TYPE> int host_rows_of(const ggb_weight *w, const char *blocks, in
 } // namespace
 
 bool ggb_matvec_host_rows_fits(const ggb_weight *w, int64_t T) { return T * w->nb * 34 <= kHostRows[2] && T < 65536; }
-int ggb_matvec_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint2 *out, uint32_t call) {
+int ggb_matvec_host_rows(const ggb_weight *w, const char *blocks, int64_t T, int64_t row_size, uint64_t *out, uint32_t call) {
     return w->type == GGB_TYPE_Q4_0 ? host_rows_of<GGB_TYPE_Q4_0>(w, blocks, T, row_size, out, call)
                                     : host_rows_of<GGB_TYPE_Q8_0>(w, blocks, T, row_size, out, call);
 }

@@ -189,7 +189,7 @@ int ggb_mul_mat(int64_t ne01, int64_t ne11, int64_t ne12, int64_t nb01, int64_t 
         int rc = ensure_pinned();
         if (rc) return rc;
         if (++g_call == 0) g_call = 1; // what no call has written is zero
-        rc = ggb_matvec_host_rows(w, wdata, col_num, (int64_t)row_size, (uint2 *)g_pinned, g_call);
+        rc = ggb_matvec_host_rows(w, wdata, col_num, (int64_t)row_size, g_pinned, g_call);
         for (int64_t col = 0; col < col_num && !rc; col++) // the reference's addressing, as in copy_back
             rc = take_results((float *)((char *)dst_data + (col % ne1) * nb1 + (col / ne1) * nb2), col * ne01, ne01, ggb_cuda_stream());
         return rc;
