@@ -54,13 +54,14 @@ __device__ __forceinline__ void vec_row_dot(const E *__restrict__ wr, const E *_
 // ACT: the output is act(.) in the matrices' type (c_act) instead of fp32 (c).  KS warps share a row, their sums are added in order: few long
 // rows leave too few bytes in flight with a warp each (in a graph, matrices from memory, 2048 rows of 8192 bf16 numbers: 14 warps an SM, 13.7 us;
 // four a row: 7.3, 4.6 TB/s; two: 8.8; 2048 x 2048: 4.9, 3.5 with two; 300 x 7000: 13.3, 3.9).  One token: 32 registers, so that an SM holds 64 warps
-// (4096 x 4096 with two a row in 34 registers: 9.2 us, in two waves).
-template <typename E, int TT, int ACT, int KS>
+// (4096 x 4096 with two a row in 34 registers: 9.2 us, in two waves).  FEW, of one warp a row: the warps of a CTA counted at run time, by which the compiler
+// holds fewer loads ahead (bf16, 6, 7, 8 tokens: 60, 72, 72 registers, 4, 3, 3 CTAs an SM; counted ahead 68, 84, 94: 3, 2, 2).
+template <typename E, int TT, int ACT, int KS, bool FEW = false>
 __global__ void __launch_bounds__(256, TT == 1 ? 8 : 0) linear_vec_kernel(const E *w, int64_t N, int64_t K, const E *a,
                                                          int64_t lda, float *c, int64_t ldc, E *c_act = nullptr) {
     constexpr int VE = 16 / (int)sizeof(E);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t n = (int64_t)blockIdx.x * (8 / KS) + warp / KS;
+    const int64_t n = (int64_t)blockIdx.x * (FEW ? (int)(blockDim.x >> 5) : 8 / KS) + warp / KS;
     step_wait();
     if (KS == 1 && n >= N) return;
     float acc[TT];
@@ -94,21 +95,30 @@ __global__ void __launch_bounds__(256, TT == 1 ? 8 : 0) linear_vec_kernel(const 
 }
 
 // Warps a row: doubled while there are 32 of them an SM at most (24 with the registers of more tokens) and each still has two rounds of 16-byte loads; beyond
-// that, up to what an SM holds, while each has four (one token; with four and more, which run in waves then, eight)
+// that, up to what an SM holds, while each has four (one token; with four and more, which run in waves then, eight, and only where the rows alone leave half
+// of an SM's warps out, or run in waves themselves: three CTAs an SM of seven or eight bf16 tokens.  Otherwise a second wave is all that comes of it: fp32, 5 x 3072 x
+// 2048 10.4 us with two warps a row, 8.9 with one; bf16, 4 x 4096 x 4096 13.1, 12.2)
 template <typename E> int vec_splits(int64_t N, int64_t K, int T) {
     const int64_t rounds = K * (int64_t)sizeof(E) / 512, held = (T <= 3 ? 32 : 24) * ggb_sm_count(), most = (T == 2 || T == 3 ? 40 : 64) * ggb_sm_count();
+    const bool waves = T <= 3 || N <= 16 * ggb_sm_count() || (sizeof(E) == 2 && T >= 7 && N > held);
     int ks = 1;
-    while (ks < 8 && N * ks * 2 <= most && rounds >= ks * 2 * (N * ks * 2 <= held ? 2 : T <= 3 ? 4 : 8)) ks *= 2;
+    while (ks < 8 && N * ks * 2 <= (waves ? most : held) && rounds >= ks * 2 * (N * ks * 2 <= held ? 2 : T <= 3 ? 4 : 8)) ks *= 2;
     return ks;
 }
+// One warp a row: one bf16 token (5120 x 2048 5.8 us; 5.95) and five tokens and more by the form of fewer registers (fp32, 5 x 8192 x 2048 17.8 us, the other one 19.9; 7 x 4096 x 1024 7.5, 12.0; bf16, 7 x 3072 x
+// 2048 8.5, 11.5; 6 x 8192 x 2048 15.5, 19.9), but seven and eight where the other one's CTAs, one fewer an SM, take no more waves (bf16, 8 x 2048 x 2048 8.3, 7.4; 8
+// x 4096 x 1024 9.1, 8.1; fp32, 8 x 5120 x 2048 23, 21)
 template <typename E, int TT, int ACT>
 void vec_launch(const E *w, int64_t N, int64_t K, const E *a, int64_t lda, float *c, int64_t ldc, E *c_act) {
     const int ks = vec_splits<E>(N, K, TT);
     const dim3 grid((unsigned)((N + 8 / ks - 1) / (8 / ks))), block(256);
+    constexpr bool kFew = TT >= 5 || (TT == 1 && sizeof(E) == 2), kBoth = TT >= 7;
+    const int64_t more = (sizeof(E) == 2 ? 16 : 24) * ggb_sm_count(), fewer = more + 8 * ggb_sm_count(); // rows that are under way at once
     if (ks == 8) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 8>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
     else if (ks == 4) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 4>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
     else if (ks == 2) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 2>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
-    else ggb_launch_step(linear_vec_kernel<E, TT, ACT, 1>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
+    else if (kBoth && (N + more - 1) / more <= (N + fewer - 1) / fewer) ggb_launch_step(linear_vec_kernel<E, TT, ACT, 1, kFew && !kBoth>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
+    else ggb_launch_step(linear_vec_kernel<E, TT, ACT, 1, kFew>, grid, block, 0, w, N, K, a, lda, c, ldc, c_act);
 }
 
 // ------------------------------------------------------------------------------------------------ tile kernel

@@ -57,7 +57,8 @@ def test_linear_any_shape(gpu, dt, T, N, K):
 
 
 @pytest.mark.parametrize("dt", [F32, BF16])
-@pytest.mark.parametrize("T,N,K", [(1, 2048, 8192), (3, 33, 8200), (8, 2047, 4096), (2, 4736, 2048), (1, 4737, 2048), (1, 1, 8191), (5, 700, 1024), (4, 9473, 1024)])
+@pytest.mark.parametrize("T,N,K", [(1, 2048, 8192), (3, 33, 8200), (8, 2047, 4096), (2, 4736, 2048), (1, 4737, 2048), (1, 1, 8191), (5, 700, 1024), (4, 9473, 1024),
+                                   (7, 2368, 264), (8, 2369, 264), (6, 3553, 2048), (7, 3553, 2048), (8, 4736, 4096), (4, 2369, 4096)])
 def test_linear_of_few_tokens_and_long_rows(gpu, dt, T, N, K):
     """one to eight warps a row: sums of K products in fp32"""
     r = np.random.default_rng(N)
