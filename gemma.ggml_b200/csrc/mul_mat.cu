@@ -12,6 +12,7 @@
 #include <tuple>
 
 #include "common.cuh"
+#include "host_words.cuh"
 
 namespace {
 
@@ -56,36 +57,32 @@ int copy_back(void *dst_data, int64_t col_num, int64_t ne01, int64_t ne12, int64
     return GGB_OK;
 }
 
-// Few results: page-locked memory that the kernel writes, a word of a result and the number of the call each.  Beyond kPinnedResults a copy engine's lines
-// are fuller.
+// Few results: page-locked memory that the kernel writes.  Beyond kPinnedResults a copy engine's lines are fuller.
 constexpr int64_t kPinnedResults = 16 * 1024;
-uint64_t *g_pinned = nullptr;
-uint32_t g_call = 0;
+host_words g_words;
 
-int ensure_pinned() {
-    if (g_pinned) return GGB_OK;
-    void *p = nullptr;
-    GGB_CUDA(cudaHostAlloc(&p, kPinnedResults * 8, cudaHostAllocMapped | cudaHostAllocPortable));
-    memset(p, 0, kPinnedResults * 8);
-    g_pinned = (uint64_t *)p;
+int next_call(cudaStream_t st) {
+    if (!g_words.words) {
+        void *p = nullptr;
+        GGB_CUDA(cudaHostAlloc(&p, kPinnedResults * 8, cudaHostAllocMapped | cudaHostAllocPortable));
+        memset(p, 0, kPinnedResults * 8);
+        g_words.words = (uint64_t *)p, g_words.n = kPinnedResults;
+    }
+    cudaError_t e = cudaSuccess;
+    if (!g_words.next([&] { return (e = cudaStreamSynchronize(st)) == cudaSuccess; })) GGB_CUDA(e);
     return GGB_OK;
 }
 
 // n results of this call from word `first` on, each as soon as it is there, or an error when the stream says that it never will be
 int take_results(float *dst, int64_t first, int64_t n, cudaStream_t st) {
-    for (int64_t i = 0; i < n; i++) {
-        uint64_t w;
-        for (int spins = 1; (w = __atomic_load_n(g_pinned + first + i, __ATOMIC_ACQUIRE)) >> 32 != g_call; spins++) {
-            if (spins % 2000) continue;
-            const cudaError_t e = cudaStreamQuery(st);
-            if (e == cudaErrorNotReady || (e == cudaSuccess && __atomic_load_n(g_pinned + first + i, __ATOMIC_ACQUIRE) >> 32 == g_call)) continue;
-            ggb_set_error("mul_mat: %s", e == cudaSuccess ? "the kernel left no result" : cudaGetErrorString(e));
-            return GGB_ERR_CUDA;
-        }
-        const uint32_t v = (uint32_t)w;
-        memcpy(dst + i, &v, 4);
-    }
-    return GGB_OK;
+    cudaError_t e = cudaSuccess;
+    const bool there = g_words.take(dst, first, n, [&] {
+        e = cudaStreamQuery(st);
+        return e == cudaErrorNotReady ? 1 : e == cudaSuccess ? 0 : -1;
+    });
+    if (there) return GGB_OK;
+    ggb_set_error("mul_mat: %s", e == cudaSuccess ? "the kernel left no result" : cudaGetErrorString(e));
+    return GGB_ERR_CUDA;
 }
 
 // Q4_K / Q6_K / F16: the types the reference's own kernels cover (ref: src/hpc.cpp:132-143)
@@ -186,10 +183,9 @@ int ggb_mul_mat(int64_t ne01, int64_t ne11, int64_t ne12, int64_t nb01, int64_t 
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (col_num * ne01 <= kPinnedResults && ggb_matvec_host_rows_fits(w, col_num) && cudaStreamIsCapturing(ggb_cuda_stream(), &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone) {
-        int rc = ensure_pinned();
+        int rc = next_call(ggb_cuda_stream());
         if (rc) return rc;
-        if (++g_call == 0) g_call = 1; // what no call has written is zero
-        rc = ggb_matvec_host_rows(w, wdata, col_num, (int64_t)row_size, g_pinned, g_call);
+        rc = ggb_matvec_host_rows(w, wdata, col_num, (int64_t)row_size, g_words.words, g_words.call);
         for (int64_t col = 0; col < col_num && !rc; col++) // the reference's addressing, as in copy_back
             rc = take_results((float *)((char *)dst_data + (col % ne1) * nb1 + (col / ne1) * nb2), col * ne01, ne01, ggb_cuda_stream());
         return rc;
