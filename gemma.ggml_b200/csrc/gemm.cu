@@ -480,7 +480,8 @@ __global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(bars0 + FULL + 8 * (grp + kCopyGroups * (k & 1)));
         };
-        for (int t = me; t < total; t += pairs, next -= a.kblocks) {
+        bool going = true; // a wait that gave up ends all of its tiles: `next` is then no stage of the following one
+        for (int t = me; going && t < total; t += pairs, next -= a.kblocks) {
             if (next >= a.kblocks) continue;
             const slot_tile at = locate(t);
             const int h0 = (int)rank * (at.width / 2), mine = min(at.width / 2, at.rows - h0); // this CTA's half of the tile (none: not above 0)
@@ -489,7 +490,7 @@ __global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __gri
             for (int i = 0; i < 8; i++) from[i] = a.a + (int64_t)a.row_src[at.row0 + min(h0 + r0 + 16 * i, at.rows - 1)] * (a.kblocks * BK) + 8 * pc;
             for (; next < a.kblocks; next += kCopyGroups, n++) {
                 const int s = grp + kCopyGroups * (n & 1);
-                if (!mbar_wait_warp(bars + EMPTY + 8 * s, ((n >> 1) & 1) ^ 1, dead)) break;
+                if (!(going = mbar_wait_warp(bars + EMPTY + 8 * s, ((n >> 1) & 1) ^ 1, dead))) break;
 #pragma unroll
                 for (int i = 0; i < 8; i++) // rows 16 apart lie at the same place of the swizzle; those behind the last stay as they are: columns that nobody stores
                     if (r0 + 16 * i < mine) cp_async16(base + s * kSlotStage + (BM + r0 + 16 * i) * 128 + ((pc ^ (r0 & 7)) << 4), from[i] + next * BK);
@@ -501,7 +502,7 @@ __global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __gri
             }
         }
         cp_async_wait<0>();
-        if (n > 0) give(n - 1);
+        if (going && n > 0) give(n - 1);
     } else if (warp >= 4) {
         const int lq = warp & 3, half = (warp - 4) >> 2;
         int it = 0;

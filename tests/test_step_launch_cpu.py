@@ -65,3 +65,22 @@ def test_a_kernel_whose_wait_ran_out_lets_its_copies_arrive():
             ahead = body[:m.start()]
             since = ahead[ahead.rindex("mbar_wait_bounded("):]
             assert re.search(r"if \(!$", ahead[:ahead.rindex("mbar_wait_bounded(")]) and "break;" in since or re.search(r"if \($", ahead[:ahead.rindex("mbar_wait_bounded(")]), n
+
+
+def test_a_copying_warp_whose_wait_ran_out_leaves_every_loop():
+    """Copies by the threads (cp.async) behind a wait by whole warps: where the place that they copy from is carried from one tile to the next, a wait that gave up
+    ends the loop over tiles, too: the place is no place of the following tile."""
+    found = 0
+    for n, (_, body) in kernels().items():
+        for m in re.finditer(r"for \(([^;]*);([^;]*); [^()]*\b(\w+) -= [^()]*\) \{", body):  # a loop that carries a position
+            depth, k = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(body[k], 0)
+                k += 1
+            loop = body[m.end():k]
+            if "mbar_wait_warp(" not in loop or "cp_async16(" not in loop:
+                continue
+            found += 1
+            flags = re.findall(r"if \(!\((\w+) = mbar_wait_warp\(", loop)
+            assert loop.count("mbar_wait_warp(") == len(flags) and all(re.search(r"\b%s\b" % f, m.group(2)) for f in flags), n
+    assert found >= 1
