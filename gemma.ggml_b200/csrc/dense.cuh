@@ -26,11 +26,14 @@ int ggb_linear_grouped_launch(int dt, const void *w, int64_t N, int64_t K, const
 bool ggb_gemm_dense_bf16_fits(int64_t N, int64_t K, int64_t T, int64_t ldc);
 int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t T, float *c, int64_t ldc, void *c_act = nullptr, int act = 0);
 
-// the grouped tcgen05 form: w [n_exp][N][K] bf16, c: n_rows rows in all, in sorted-slot order, offsets [n_exp + 1] on the device, row_src the rows
-// of a of pitch K that they belong to, or null: a is sorted too; c fp32 or (c_act) bf16 act(c)
+// the grouped tcgen05 forms: w [n_exp][N][K] bf16, c: n_rows rows in all, in sorted-slot order, offsets [n_exp + 1] on the device, row_src the rows
+// of a of pitch K that they belong to, or null: a is sorted too; c fp32 or (c_act) bf16 act(c).  slots: tiles of an expert's slots by two CTAs, otherwise tiles of 128
+// sorted rows by one
 bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc);
-int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, const int32_t *row_src, float *c,
-                          void *c_act, int act, int64_t ldc);
+// which of them is the faster one.  equal: groups of the same number of rows; gather: the rows of a are not sorted, tiles of rows ask for them copied
+bool ggb_gemm_grouped_bf16_slots(int64_t N, int64_t K, int64_t n_rows, int n_exp, bool equal, bool gather, bool act);
+int ggb_gemm_grouped_bf16(bool slots, const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, const int32_t *row_src,
+                          float *c, void *c_act, int act, int64_t ldc);
 
 // norms on both sides of a sublayer (ggb_op_norm_add_norm); with inv / wt the sublayer's output is the weighted sum of
 // the token's `top` expert slots, gathered on the way in (moe.cu)

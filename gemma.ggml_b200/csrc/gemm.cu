@@ -1,6 +1,6 @@
 // gemm.cu — products of plain bf16 matrices on the tensor cores: C[T][N] = A[T][K] W[N][K]^T, and the grouped form for a mixture of experts.
 //
-// A dense tile of C is 256 x 256, by two CTAs of a cluster, or 128 x (256, 128, 64), by one; a tile of an expert's slots is gemm_slots_kernel's.  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
+// A tile of C is 256 x 256, by two CTAs of a cluster, or 128 x (256, 128, 64), by one; a tile of an expert's slots is gemm_slots_kernel's.  Both operands arrive by TMA (tensor maps, 128-byte swizzle, 64 numbers of K a stage)
 // in a ring that takes all of shared memory but the epilogue's corner; one warp issues the MMAs, eight drain tensor memory.  CTAs are
 // persistent: where a tile needs half of tensor memory, the next one's products run while the last one's are stored.  The epilogue
 // turns 32 x 32 pieces in shared memory, so that a store instruction writes whole 128-byte lines.
@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "dense.cuh"
@@ -27,7 +28,7 @@ namespace {
 constexpr int BK = 64, BM = 128; // a stage of K, the rows of a CTA
 constexpr int kThreads = 384; // warp 0: TMA, 1: MMA, 2: tensor memory, 4..11: epilogue
 constexpr uint32_t kRing = 192 * 1024, kTurn = 8 * 4096;
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = 8, kListed = 256; // groups whose first row tiles are kept in shared memory
 constexpr size_t kSmem = 1024 + kRing + kTurn + 256;
 static_assert(kSmem >= kOneCtaSmem, "pairs of CTAs");
 enum { FULL = 0, EMPTY = 64, ACC_FULL = 128, ACC_FREE = 144, SLOT = 160, DEAD = 168 };
@@ -54,7 +55,7 @@ struct pair_maps {
     CUtensorMap w, a[4]; // a: boxes of 128 rows; of a grouped product 32, 64, 96 and 128
 };
 struct tile_at {
-    int m0, n0, split;
+    int m0, m_end, n0, split, group;
 };
 
 // a warp's 32 rows x 32 columns of accumulators, K pieces added in order, stored as whole lines
@@ -97,8 +98,11 @@ __device__ __forceinline__ void store_piece(const gemm_args &a, uint32_t col, in
     }
 }
 
+// GROUPED: row tiles of a group's own rows
+template <bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const gemm_args a) {
     extern __shared__ uint8_t gm_raw[];
+    __shared__ int first_tile[GROUPED ? kListed + 1 : 1]; // the first row tile of a group
     const uint32_t raw0 = smem_u32(gm_raw), base = (raw0 + 1023u) & ~1023u, turn = base + kRing, bars = turn + kTurn;
     uint8_t *ctl = gm_raw + (bars - raw0);
     volatile int *dead = reinterpret_cast<volatile int *>(ctl + DEAD);
@@ -119,18 +123,67 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
     }
     if (warp == 2) tmem_alloc512(bars + SLOT);
     early_wait();
+    const bool listed = GROUPED && a.n_groups <= kListed;
+    if (listed && warp == 3) { // prefix sums of the groups' row tiles
+        int sum = 0;
+        for (int g0 = 0; g0 < a.n_groups; g0 += 32) {
+            const int g = g0 + lane;
+            int v = g < a.n_groups ? (a.m_ranges[g + 1] - a.m_ranges[g] + BM - 1) / BM : 0;
+            for (int off = 1; off < 32; off *= 2) {
+                const int o = __shfl_up_sync(0xffffffffu, v, off);
+                if (lane >= off) v += o;
+            }
+            if (g < a.n_groups) first_tile[g + 1] = sum + v;
+            sum += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) first_tile[0] = 0;
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     step_next();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<uint32_t *>(ctl + SLOT), 0);
-    const int total = a.m_tiles * a.n_tiles * a.splits;
-    auto locate = [&](int t) { // row tiles first: those that share a piece of W run together
+    int row_tiles = a.m_tiles;
+    if (listed) row_tiles = first_tile[a.n_groups];
+    else if (GROUPED) {
+        row_tiles = 0;
+        for (int g = 0; g < a.n_groups; g++) row_tiles += (a.m_ranges[g + 1] - a.m_ranges[g] + BM - 1) / BM;
+    }
+    const int total = row_tiles * a.n_tiles * a.splits;
+    auto locate = [&](int t) {
         tile_at r;
-        r.m0 = t % a.m_tiles * BM;
-        t /= a.m_tiles;
-        r.n0 = t % a.n_tiles * a.BN;
-        r.split = t / a.n_tiles;
+        r.group = 0;
+        if (!GROUPED) { // row tiles first: those that share a piece of W run together
+            r.m0 = t % a.m_tiles * BM;
+            r.m_end = a.T;
+            t /= a.m_tiles;
+            r.n0 = t % a.n_tiles * a.BN;
+            r.split = t / a.n_tiles;
+            return r;
+        }
+        const int rt = t / a.n_tiles;
+        r.n0 = (t - rt * a.n_tiles) * a.BN;
+        r.split = 0;
+        int f;
+        if (listed) {
+            int lo = 0, hi = a.n_groups - 1; // the last group whose first tile is not behind rt
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (first_tile[mid] <= rt) lo = mid;
+                else hi = mid - 1;
+            }
+            r.group = lo;
+            f = first_tile[lo];
+        } else {
+            f = 0;
+            for (;; r.group++) {
+                const int n = (a.m_ranges[r.group + 1] - a.m_ranges[r.group] + BM - 1) / BM;
+                if (f + n > rt) break;
+                f += n;
+            }
+        }
+        r.m0 = a.m_ranges[r.group] + (rt - f) * BM;
+        r.m_end = a.m_ranges[r.group + 1];
         return r;
     };
     auto k_range = [&](int split, int &kb0, int &kb1) {
@@ -151,7 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
                     const uint32_t sa = base + s * stage_bytes, bar = bars + FULL + 8 * s;
                     mbar_expect_tx(bar, stage_bytes);
                     tma_load_2d(sa, &map_a, kb * BK, at.m0, bar);
-                    tma_load_2d(sa + a_bytes, &map_w, kb * BK, at.n0, bar);
+                    tma_load_2d(sa + a_bytes, &map_w, kb * BK, at.group * a.N + at.n0, bar);
                     if (++s == a.stages) s = 0, ph ^= 1u;
                 }
             }
@@ -195,9 +248,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tma_kernel(const __grid_cons
             tc_fence_after();
             // a warp's 32 rows, every other 32 columns (the two warps of a quarter share them)
             const int row0 = at.m0 + lq * 32;
-            if (row0 < a.T)
+            if (row0 < at.m_end)
                 for (int c0 = 32 * half; c0 < a.BN && at.n0 + c0 < a.N; c0 += 64)
-                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, chunks, my, lane, row0, a.T, at.n0 + c0, at.split);
+                    store_piece(a, tmem + ((uint32_t)(lq * 32) << 16) + buf * 256 + c0, chunks, my, lane, row0, at.m_end, at.n0 + c0, at.split);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bars + ACC_FREE + 8 * buf);
@@ -336,13 +389,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
 // a CTA) x up to 256 slots of a group in equal tiles of a multiple of 32: so a group's matrix is read once whatever its slots, and no row is computed for nothing but
 // the last 31.  A lane of tensor memory is a feature, so that 32 lanes store a line of a slot's row as they are.
 //
-// Rows of A come by TMA where they lie sorted.  Where they do not (row_src) and a tile has few of them, three groups of four warps copy them through the slot
+// Rows of A come by TMA where they lie sorted.  Where they do not (row_src), three groups of four warps copy them through the slot
 // list, which takes the stages in turn: a group hands one over when it has asked for its next (asking takes 500 cycles of a stage's 700, arriving 2500).
 //
-// Bound by memory, the matrices, and by the third round of tiles.  32 experts x 128 +- 11 slots, 1408 x 2048: 44.2 us a product from sorted rows (row tiles of 128
+// Bound by memory, the matrices, and by the last round of tiles.  32 experts x 128 +- 11 slots, 1408 x 2048: 44.2 us a product from sorted rows (row tiles of 128
 // slots x 256 features, in which half of the groups read their matrix twice: 47.0), 42.9 through the slot list (50.9 gathered ahead of it, 52 gathered ahead of this
-// kernel); with GELU 44.6 (64.2).  8 experts x 768 slots, 2048 x 2048, bound by the MMAs: 52 (52.9).  TMA's gather of four rows
-// takes 80 cycles a row: 80 us.
+// kernel, which is the slower way up to 4096 slots an expert); with GELU 44.6 (64.2).  TMA's gather of four rows takes 80 cycles: 80 us.  Where it is not the
+// faster form: ggb_gemm_grouped_bf16_slots.
 constexpr uint32_t kSlotStage = BM * 128 + 128 * 128;
 constexpr int kSlotStages = 6, kMaxGroups = 8192;
 constexpr int kCopyGroups = 3, kCopyWarps = 4, kSlotThreads = kThreads + 32 * kCopyWarps * kCopyGroups; // warps 12..: rows of A through the slot list
@@ -588,11 +641,12 @@ int launch_pair(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t
 
 int launch(const void *w, int64_t w_rows, int64_t K, const void *a, int64_t a_rows, const gemm_args &g, int ctas) {
     CUtensorMap ma, mw;
-    int rc = ggb_allow_smem(gemm_tma_kernel, kSmem);
+    auto kern = g.m_ranges ? gemm_tma_kernel<true> : gemm_tma_kernel<false>;
+    int rc = ggb_allow_smem(kern, kSmem);
     if (!rc) rc = ggb_tensor_map_bf16(&ma, a, a_rows, K, K, BM);
     if (!rc) rc = ggb_tensor_map_bf16(&mw, w, w_rows, K, K, g.BN);
     if (rc) return rc;
-    GGB_CUDA(ggb_launch_early(gemm_tma_kernel, ggb_cluster{1, 1, 1}, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
+    GGB_CUDA(ggb_launch_early(kern, ggb_cluster{1, 1, 1}, dim3((unsigned)std::min(ctas, ggb_sm_count())), dim3(kThreads), kSmem, ma, mw, g));
     GGB_LAUNCH_CHECK();
     return GGB_OK;
 }
@@ -682,19 +736,29 @@ int ggb_gemm_dense_bf16(const void *w, int64_t N, int64_t K, const void *a, int6
     return GGB_OK;
 }
 
-// The grouped form: w = [n_exp][N][K], rows of c in sorted-slot order, offsets[e] .. offsets[e + 1] those of expert e (device), row_src their rows of a (or
+static int rows_tile_n(int64_t N) { return N <= 64 ? 64 : N <= 128 ? 128 : 256; }
+// The grouped forms: w = [n_exp][N][K], rows of c in sorted-slot order, offsets[e] .. offsets[e + 1] those of expert e (device), row_src their rows of a (or
 // null: the same)
 bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc) { return K % 64 == 0 && N % 32 == 0 && ldc % 8 == 0; }
-int ggb_gemm_grouped_bf16(const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, const int32_t *row_src, float *c, void *c_act,
-                          int act, int64_t ldc) {
+
+// Tiles of an expert's slots, as many groups as their kernel has room to list, and as many rows of W as its coordinates reach
+bool ggb_gemm_grouped_bf16_slots(int64_t N, int64_t, int64_t, int n_exp, bool, bool, bool) { return n_exp <= kMaxGroups && n_exp * N < (1ll << 31); }
+int ggb_gemm_grouped_bf16(bool slots, const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, const int32_t *row_src,
+                          float *c, void *c_act, int act, int64_t ldc) {
     GGB_REQUIRE_INIT();
     GGB_CHECK_ARG(((uintptr_t)w | (uintptr_t)a) % 16 == 0, "gemm: operands start on 16 bytes");
-    GGB_CHECK_ARG(n_exp <= kMaxGroups && n_exp * N < (1ll << 31), "gemm: %d experts of %lld rows", n_exp, (long long)N);
     gemm_args g{};
-    g.T = (int)n_rows, g.N = (int)N, g.kblocks = (int)(K / BK), g.n_tiles = (int)((N + 255) / 256);
-    g.m_ranges = offsets, g.row_src = row_src, g.n_groups = n_exp, g.a = (const __nv_bfloat16 *)a;
+    g.T = (int)n_rows, g.N = (int)N, g.kblocks = (int)(K / BK);
+    g.m_ranges = offsets, g.n_groups = n_exp;
     g.c = c, g.act_out = (__nv_bfloat16 *)c_act, g.act = act, g.ldc = ldc;
     g.wait_error = ggb_wait_error_flag();
+    if (!slots) {
+        g.BN = rows_tile_n(N), g.n_tiles = (int)((N + g.BN - 1) / g.BN);
+        g.chunks = 1, g.chunk_kb = g.kblocks, g.splits = 1, g.stages = stages_of(g.BN), g.vec = (uintptr_t)c % 16 == 0;
+        const int64_t most = ((n_rows + BM - 1) / BM + n_exp) * g.n_tiles;
+        return launch(w, (int64_t)n_exp * N, K, a, n_rows, g, (int)std::min<int64_t>(most, 1 << 20));
+    }
+    g.n_tiles = (int)((N + 255) / 256), g.row_src = row_src, g.a = (const __nv_bfloat16 *)a;
     const int64_t most = (n_rows / 256 + std::min<int64_t>(n_rows, n_exp)) * g.n_tiles;
     return launch_pair(w, (int64_t)n_exp * N, K, a, n_rows, g, (int)std::min<int64_t>(most, 1 << 20));
 }

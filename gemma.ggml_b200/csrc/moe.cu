@@ -821,17 +821,16 @@ int ggb_op_moe_linear_identity(int dt, const void *w, int64_t N, int64_t K, cons
         GGB_LAUNCH_CHECK();
         return GGB_OK;
     }
-    // Portions, bf16, aligned shapes, on the tensor cores: many slots in tiles of an expert's slots.  Fewer in the same way without a
+    // Portions, bf16, aligned shapes, on the tensor cores: many slots in tiles of rows or of an expert's slots.  Fewer through the slot list without a
     // workspace (such a portion may be captured, and a workspace that grows would move under the graph), every 64 numbers of K summed by
     // themselves: no further off than the multiply-adds of the tile kernel, which takes what is left.  32 experts, 1408 x 2048: 480 slots 39 us
     // (47 gathered), 20 slots 24 (33).
     if (dt == GGB_TYPE_BF16 && ggb_gemm_grouped_bf16_fits(N, K, ldc) && lda == K && ((uintptr_t)a & 15) == 0) {
         const int64_t n = T * top;
         if (n >= 512) {
-            // many slots an expert: rows gathered ahead (the product's tiles are wide, and copying them through the slot list would bound it: 768 slots an
-            // expert 56 us, 68); fewer: through the slot list (256: 28.8; 128: 42.9, 52.4; 32: 37.6, 41.5)
+            const bool slots = ggb_gemm_grouped_bf16_slots(N, K, n, n_real, false, gather, act != 0);
             const void *a_sorted = a;
-            const bool ahead = gather && n > 256 * (int64_t)n_real;
+            const bool ahead = gather && !slots;
             if (ahead) {
                 void *gbuf;
                 const int rc = ggb_workspace(GGB_WS_MOE_GATHER, (size_t)n * (size_t)K * 2, &gbuf);
@@ -840,7 +839,7 @@ int ggb_op_moe_linear_identity(int dt, const void *w, int64_t N, int64_t K, cons
                 GGB_LAUNCH_CHECK();
                 a_sorted = gbuf;
             }
-            return ggb_gemm_grouped_bf16(w, N, K, a_sorted, n, n_real, g.offsets, ahead ? nullptr : g.row_src, act ? nullptr : (float *)c, act ? c : nullptr, act, ldc);
+            return ggb_gemm_grouped_bf16(slots, w, N, K, a_sorted, n, n_real, g.offsets, ahead ? nullptr : g.row_src, act ? nullptr : (float *)c, act ? c : nullptr, act, ldc);
         }
         if (K >= 128 && ((uintptr_t)w & 15) == 0) // (sums of 64: 7e-8, multiply-adds 5e-8; K = 128: 7.0e-8, 7.2e-8)
             return ggb_gemm_any_grouped(w, N, K, a, lda, n, n_real, act ? nullptr : (float *)c, ldc, act ? c : nullptr, act, g);

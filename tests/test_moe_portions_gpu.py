@@ -109,3 +109,22 @@ def test_tiles_of_slots(gpu, counts, N, K, gather):
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < (K / 16 + 8) * 2.0 ** -23 + 1e-7
     square = from_dt(BF16, y, (n, N))
     assert np.array_equal(square, as_dt(BF16, np.maximum(got, np.float32(0)) ** 2)[0])
+
+
+@pytest.mark.parametrize("E", [8192, 8193, 9001])
+def test_more_groups_than_are_listed(gpu, E):
+    """lists that a program has made itself, of more experts than the slots' kernel has room for"""
+    r, lib, N, K, n = np.random.default_rng(E), gpu.cuda_lib(), 32, 64, 700
+    idx = r.permutation(np.concatenate([r.integers(0, E, n - 70), np.full(67, 4000), [0, E - 1, E - 1]]))
+    order = np.argsort(idx, kind="stable")
+    lists = np.zeros(int(lib.ggb_moe_group_ints(n, E)), dtype=np.int32)
+    lists[:E + 1] = np.concatenate([[0], np.cumsum(np.bincount(idx, minlength=E))])
+    lists[E + 1:E + 1 + n] = order
+    (w, wr), (a, ar) = as_dt(BF16, r.standard_normal((E, N, K))), as_dt(BF16, r.standard_normal((n, K)))
+    ws, dw, da, c = dev(gpu, lists), dev(gpu, wr), dev(gpu, ar), zeros(gpu, n * N * 4)
+    want = np.einsum("nk,nfk->nf", a[order], w[idx[order]])
+    for gather in (1, 0):
+        rows = da if gather else dev(gpu, ar[order])
+        gpu.check(lib.ggb_op_moe_linear(BF16, dw.ptr, N, K, rows.ptr, K, gather, n, 1, E, ws.ptr, 0, c.ptr, N), "moe_linear")
+        got = c.download(np.float32).reshape(n, N)
+        assert np.linalg.norm(got - want) / np.linalg.norm(want) < (K / 16 + 8) * 2.0 ** -23 + 1e-7

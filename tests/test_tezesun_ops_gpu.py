@@ -416,6 +416,20 @@ def test_gates_on_the_tensor_cores_keep_32_bits(gpu):
     assert e_split < 5e-6 and e_tile < 5e-6 and F.rel_err(rounded, last) > 50 * e_split
 
 
+def test_gates_of_more_blocks_than_a_list_of_groups_holds(gpu):
+    """8200 blocks, of two kinds by turns"""
+    r, lib = np.random.default_rng(8), gpu.cuda_lib()
+    nb, d, T = 8200, 64, 64
+    (w, wr), (s, sr) = as_dt(BF16, r.standard_normal((2, 2 * d, 3 * d))), as_dt(BF16, r.standard_normal((2, T, 3 * d)))
+    u, z, off = zeros(gpu, T * nb * d * 4), zeros(gpu, nb * T * 2 * d * 4), dev(gpu, i32(np.arange(nb + 1) * T))
+    split, w3 = dev(gpu, np.tile(sr, (nb // 2, 1, 1))), dev(gpu, np.tile(wr, (nb // 2, 1, 1)))
+    assert lib.ggb_rglru_split_fits(BF16, T, d)
+    gpu.check(lib.ggb_op_rglru_gates(BF16, u.ptr, split.ptr, off.ptr, T, nb, d, w3.ptr, w3.ptr, z.ptr), "gates")
+    got = z.download(np.float32).reshape(nb // 2, 2, T, 2 * d)
+    want = np.einsum("btk,bfk->btf", s, w)
+    assert F.rel_err(got[0], want) < 2e-6 and (got == got[0]).all()
+
+
 def test_hardly_decaying_and_forgetting_channels(gpu):
     """1 - a^2 is taken without cancellation (a channel that keeps everything), and a channel with a = 0 holds its own input only"""
     r = np.random.default_rng(6)
