@@ -741,8 +741,24 @@ static int rows_tile_n(int64_t N) { return N <= 64 ? 64 : N <= 128 ? 128 : 256; 
 // null: the same)
 bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc) { return K % 64 == 0 && N % 32 == 0 && ldc % 8 == 0; }
 
-// Tiles of an expert's slots, as many groups as their kernel has room to list, and as many rows of W as its coordinates reach
-bool ggb_gemm_grouped_bf16_slots(int64_t N, int64_t, int64_t, int n_exp, bool, bool, bool) { return n_exp <= kMaxGroups && n_exp * N < (1ll << 31); }
+// Which of the two forms, by the least estimated time in microseconds: the rounds of tiles, each K / 64 stages and its stores, or the bytes.  The counts of a router's
+// groups are taken to spread by about their square root.  The figures are fitted to 6752 calls (4 to 128 groups of 32 to 2048 rows, N 64 to 2048, K 256 to 2048, sums and GELU, rows sorted or
+// not, gates of 2 to 32 equal blocks): the chosen form is 0.5 % above the better one on the average, 11 % at the 99th percentile (always tiles of slots: 17 %, of rows: 9 %).  They
+// differ by up to a factor of two either way: a pair of CTAs takes 256 features whatever N is (8 x 2048 rows, 64 x 1024, sorted: tiles of rows 7.4 us, of slots 14.9; 8 x 64 rows,
+// 256 x 2048: 15.6, 11.7), half as many tiles leave half of the chip out (8 x 512 rows, 1024 x 2048: 19.8, 29.3) or read a matrix once where two read it (64 x 256
+// rows, 1408 x 2048: 159, 116).
+bool ggb_gemm_grouped_bf16_slots(int64_t N, int64_t K, int64_t n_rows, int n_exp, bool equal, bool gather, bool act) {
+    if (n_exp > kMaxGroups || n_exp * N >= (1ll << 31)) return false;
+    if (gather && !ggb_workspace_fits(GGB_WS_MOE_GATHER, (size_t)n_rows * (size_t)K * 2)) return true; // a capture that it would have to grow in
+    const double per = (double)n_rows / n_exp, spread = equal ? 0 : 0.75 * std::sqrt(per), kb = (double)(K / BK), sms = ggb_sm_count();
+    auto tiles = [&](double size) { return (std::max(1.0, std::ceil((per - spread) / size)) + std::max(1.0, std::ceil((per + spread) / size))) / 2; };
+    const double BN = rows_tile_n(N), mb = 1e-6 * ((double)n_exp * N * K * 2 + (double)n_rows * N * (act ? 2 : 4));
+    const double width = std::min(256.0, 32 * std::ceil(per / tiles(256) / 32));
+    const double rounds_r = std::ceil(n_exp * tiles(BM) * std::ceil(N / BN) / sms - 0.02), rounds_s = std::ceil(n_exp * tiles(256) * std::ceil(N / 256.0) / (sms / 2) - 0.02);
+    const double rows = std::max(2.6 + rounds_r * (kb * (0.095 + 0.0007 * BN) + (act ? 0.034 : 0.022) * BN), 2.6 + 0.24 * mb) + (gather ? 1.1 + 0.55e-6 * n_rows * K : 0);
+    const double slots = (gather ? 5.7 : 5) + std::max(rounds_s * (0.158 * kb + (act ? 0.052 * width : 0.3 + 0.033 * width)), 0.163 * mb);
+    return slots < rows;
+}
 int ggb_gemm_grouped_bf16(bool slots, const void *w, int64_t N, int64_t K, const void *a, int64_t n_rows, int n_exp, const int32_t *offsets, const int32_t *row_src,
                           float *c, void *c_act, int act, int64_t ldc) {
     GGB_REQUIRE_INIT();

@@ -85,7 +85,10 @@ def test_choice_does_not_depend_on_the_tokens_of_a_call(gpu, E, T):
 
 @pytest.mark.parametrize("gather", [0, 1])
 @pytest.mark.parametrize("counts,N,K", [([0, 1, 16, 17, 31, 33, 0, 160, 255, 0], 160, 448), ([256, 257, 0], 416, 64), ([513, 1, 2], 96, 192), ([700, 900], 1408, 128),
-                                        ([3] * 300, 32, 64), ([17, 600, 0, 0], 288, 1024)])
+                                        ([3] * 300, 32, 64), ([17, 600, 0, 0], 288, 1024),
+                                        # the same edges at sizes where the tiles are an expert's slots rather than rows
+                                        ([0, 1, 16, 17, 31, 33, 0, 160, 255, 0], 416, 1024), ([0, 256, 257, 0, 1, 0, 0, 0], 288, 2048), ([0, 513, 1, 2] + [0] * 8, 160, 2048),
+                                        ([700, 900] + [0] * 14, 288, 2048), ([3] * 300, 160, 256), ([3] * 300, 288, 64), ([3] * 200, 416, 192), ([17, 600, 0, 0, 5, 9, 30, 64], 288, 1024)])
 def test_tiles_of_slots(gpu, counts, N, K, gather):
     """The grouped product at the edges of its tiles: halves of a tile without slots, groups without any, features that leave a CTA of a pair without work, fewer
     blocks of K than the ring has places.  Products are exact; a running sum is truncated once per 16 of K, at most 2^-23 of it."""
