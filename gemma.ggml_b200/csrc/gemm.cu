@@ -749,7 +749,8 @@ bool ggb_gemm_grouped_bf16_fits(int64_t N, int64_t K, int64_t ldc) { return K % 
 // rows, 1408 x 2048: 159, 116).
 bool ggb_gemm_grouped_bf16_slots(int64_t N, int64_t K, int64_t n_rows, int n_exp, bool equal, bool gather, bool act) {
     if (n_exp > kMaxGroups || n_exp * N >= (1ll << 31)) return false;
-    if (gather && !ggb_workspace_fits(GGB_WS_MOE_GATHER, (size_t)n_rows * (size_t)K * 2)) return true; // a capture that it would have to grow in
+    // in a capture that the workspace of the copied rows would have to grow in: up to 256 rows a group in the form that needs none, beyond that refused if that is not the faster one
+    if (gather && n_rows <= 256 * (int64_t)n_exp && !ggb_workspace_fits(GGB_WS_MOE_GATHER, (size_t)n_rows * (size_t)K * 2)) return true;
     const double per = (double)n_rows / n_exp, spread = equal ? 0 : 0.75 * std::sqrt(per), kb = (double)(K / BK), sms = ggb_sm_count();
     auto tiles = [&](double size) { return (std::max(1.0, std::ceil((per - spread) / size)) + std::max(1.0, std::ceil((per + spread) / size))) / 2; };
     const double BN = rows_tile_n(N), mb = 1e-6 * ((double)n_exp * N * K * 2 + (double)n_rows * N * (act ? 2 : 4));
