@@ -654,19 +654,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
     }
 }
 
-// Few CTAs (few key heads, portions that are not long) leave SMs without work: up to eight CTAs then share a CTA's key tiles, as many as there are SMs for.  How many
-// positions come before the portion is known on the device only, and a cluster costs 2 us, so that the portion itself (or its window) has to hold three tiles a part.
-// Heads of 128, graph replays: 1000 tokens x 4 heads (1 key head) at position 900, four parts 26.4 us (48.5 alone); 500 tokens of 4 sigmoid heads (1) at 1000, two
-// parts 31.7 (45.5); 480 tokens x 8 heads (8) of 64 at position 0 17.9 (17.8).  128 tokens at position 700 would take 18.4 in eight parts (28.0), but at position 0
-// 17.5 (14.3).  With more CTAs than SMs two parts cost: 777 tokens of 16 sigmoid heads (4) at 1024, 100 CTAs: 63.8 (53.6).
+// Few CTAs (few key heads, portions that are not long) leave SMs without work: up to eight CTAs then share a CTA's key tiles.  How many positions come before
+// the portion is known on the device only, and a cluster costs 2 us (its two meetings; and more numbers than the loop over tiles has registers for), so that the portion
+// itself (or its window) has to hold what saves that at position 0: three tiles a part, and ten of them where there is a maximum to find.  Soft-max heads, two parts, graph
+// replays: 385 tokens x 4 heads (1 key head) of 64 17.5 us (15.3 alone), 512 18.3 (17.4), 512 x 2 (2) of 128 21.5 (20.9), 640 19.3 (19.1) and 22.7 (23.9), a window of 400 18.8 (17.2); sigmoid
+// heads, 385 x 4 (1) of 64 17.0 (17.1), 640 19.2 (23.1).  Four parts, heads of 128: 1000 tokens x 4 heads (1) at position 900 26.4 us (48.5 alone).
+// With more CTAs than SMs two parts cost: 777 tokens of 16 sigmoid heads (4) at 1024, 100 CTAs: 63.8 (53.6).
 template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin) {
     const int TQ = kRows / MAPS / (a.H / a.G);
-    const int64_t ctas = (a.T + TQ - 1) / TQ * a.G, most = (a.window > 0 ? std::min(a.T, a.window) : a.T) / (3 * kKeys);
+    const int64_t ctas = (a.T + TQ - 1) / TQ * a.G, own = (a.window > 0 ? std::min(a.T, a.window) : a.T) / kKeys; // tiles of the portion
+    const size_t alone = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G), shared = std::max(alone, kOneCtaSmem); // clusters with tensor memory
+    auto split = attn_kernel<MODE, MAPS, true, FIN>;
     unsigned parts = 1;
-    while (parts < 8 && parts * 2 <= most && ctas * parts * 2 <= ggb_sm_count()) parts *= 2;
-    size_t smem = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G);
-    if (parts > 1) smem = std::max(smem, kOneCtaSmem); // clusters with tensor memory
-    auto kfn = parts > 1 ? attn_kernel<MODE, MAPS, true, FIN> : attn_kernel<MODE, MAPS, false, FIN>;
+    while (parts < 8 && own >= (MODE == SOFTMAX ? 10 : 6) && parts * 2 <= own / 3 && ctas * parts * 2 <= ggb_sm_count()) parts *= 2;
+    const size_t smem = parts > 1 ? shared : alone;
+    auto kfn = parts > 1 ? split : attn_kernel<MODE, MAPS, false, FIN>;
     const int rc = ggb_allow_smem(kfn, smem);
     if (rc) return rc;
     const ggb_cluster cluster{1, 1, parts};

@@ -59,9 +59,11 @@ SOFT = [(1, 1, 16, 16, 32, 0, 64, 0, 0, 0, 0.0, 0.3, 1, 0), (4, 1, 64, 64, 33, 3
         (6, 2, 192, 64, 127, 129, 16, 100, 0, 1, 0.0, 0.1, 0, 0), (4, 1, 176, 48, 70, 30, 64, 0, 0, 0, 30.0, 0.5, 1, 1)]
 
 
-# clusters of two and four CTAs that share key tiles: CTAs of few tiles, of a part or none for some of them, rows that see nothing of a part, a window of a part
+# clusters of two, four and eight CTAs that share key tiles: CTAs of few tiles, of a part or none for some of them, rows that see nothing of a part, a window of a part
 SOFT += [(4, 1, 64, 64, 385, 0, 64, 0, 0, 0, 30.0, 0.5, 1, 1), (2, 1, 128, 128, 800, 90, 64, 0, 0, 0, 0.0, 1.0, 0, 0), (3, 1, 32, 48, 900, 5, 16, 400, 70, 0, 0.0, 0.3, 0, 1),
-         (6, 3, 16, 80, 1000, 130, 64, 768, 0, 0, 2.0, 0.4, 1, 0), (1, 1, 64, 128, 777, 500, 64, 390, 0, 1, 0.0, 0.3, 0, 0)]
+         (6, 3, 16, 80, 1000, 130, 64, 768, 0, 0, 2.0, 0.4, 1, 0), (1, 1, 64, 128, 777, 500, 64, 390, 0, 1, 0.0, 0.3, 0, 0),
+         (4, 1, 64, 64, 640, 0, 64, 0, 0, 0, 30.0, 0.5, 1, 1), (2, 2, 48, 32, 639, 200, 64, 0, 0, 0, 0.0, 0.5, 0, 0), (1, 1, 64, 128, 777, 500, 64, 650, 0, 1, 0.0, 0.3, 0, 0),
+         (1, 1, 64, 64, 1536, 0, 64, 0, 0, 0, 30.0, 0.5, 1, 1), (1, 1, 32, 48, 1750, 333, 16, 0, 0, 0, 0.0, 1.0, 0, 0), (1, 1, 16, 80, 1700, 900, 64, 1600, 70, 0, 0.0, 0.3, 0, 1)]
 
 
 @pytest.mark.parametrize("dt", [BF16, F32])
@@ -84,7 +86,7 @@ def test_soft_max_heads(gpu, dt, H, Gk, D, Dv, T, pos, page, window, keep, chunk
 
 
 @pytest.mark.parametrize("H,Gk,D,Dv,T,pos,window,keep,cap", [(2, 1, 16, 16, 32, 0, 0, 0, 0.0), (4, 2, 64, 128, 65, 63, 64, 3, 30.0), (3, 3, 128, 128, 64, 200, 0, 0, 2.0), (64, 1, 32, 48, 33, 90, 70, 65, 0.0),
-                                                                   (2, 1, 64, 64, 800, 300, 0, 0, 30.0), (1, 1, 32, 128, 450, 0, 400, 9, 0.0)])
+                                                                   (2, 1, 64, 64, 800, 300, 0, 0, 30.0), (1, 1, 32, 128, 450, 0, 400, 9, 0.0), (2, 1, 64, 64, 640, 0, 0, 0, 0.0), (1, 1, 32, 128, 1600, 70, 700, 9, 0.0)])
 def test_differential_heads(gpu, H, Gk, D, Dv, T, pos, window, keep, cap):
     G = Gk
     r, q, K, V, cache, table, pos0 = inputs(gpu, BF16, H, G, D, Dv, 2, pos, T, 64, D + T, 0.3)
@@ -97,7 +99,7 @@ def test_differential_heads(gpu, H, Gk, D, Dv, T, pos, window, keep, cap):
     assert rel(from_dt(BF16, out, (T, H, Dv)), o) < LIMIT
 
 
-@pytest.mark.parametrize("H,Gk,D,Dv,T,pos,window,page,bare", [(1, 1, 16, 16, 32, 0, 0, 64, 0), (4, 1, 64, 64, 33, 31, 0, 5, 0), (16, 1, 128, 128, 129, 64, 65, 64, 0), (6, 2, 80, 96, 200, 700, 128, 64, 0), (4, 1, 64, 80, 800, 200, 0, 64, 0), (2, 2, 32, 32, 390, 0, 0, 16, 1),
+@pytest.mark.parametrize("H,Gk,D,Dv,T,pos,window,page,bare", [(1, 1, 16, 16, 32, 0, 0, 64, 0), (4, 1, 64, 64, 33, 31, 0, 5, 0), (16, 1, 128, 128, 129, 64, 65, 64, 0), (6, 2, 80, 96, 200, 700, 128, 64, 0), (4, 1, 64, 80, 800, 200, 0, 64, 0), (2, 2, 32, 32, 390, 0, 0, 16, 1), (1, 1, 64, 64, 1600, 0, 0, 64, 0), (1, 1, 48, 80, 1750, 500, 0, 16, 0),
                                                             (64, 1, 48, 32, 40, 100, 0, 64, 0), (3, 3, 128, 128, 128, 0, 1, 64, 1)])
 def test_sigmoid_heads(gpu, H, Gk, D, Dv, T, pos, window, page, bare):
     G = Gk
@@ -219,27 +221,29 @@ def test_infinities_as_plain_arithmetic_has_them(gpu, kind, cap, window, keep, w
     assert np.isfinite(got[ok]).all() and rel(got[ok], want[ok]) < LIMIT
 
 
-@pytest.mark.parametrize("kind,cap,window,keep", [("soft", 30.0, 0, 0), ("soft", 0.0, 390, 9), ("diff", 0.0, 0, 0), ("sigmoid", 0.0, 0, 0)])
+@pytest.mark.parametrize("kind,cap,window,keep,H,Gk,T", [("soft", 30.0, 0, 0, 6, 2, 450), ("soft", 0.0, 390, 9, 6, 2, 450), ("diff", 0.0, 0, 0, 6, 2, 450), ("sigmoid", 0.0, 0, 0, 6, 2, 450),
+                                                        ("soft", 30.0, 0, 0, 6, 2, 700), ("soft", 0.0, 650, 9, 6, 2, 900), ("diff", 0.0, 0, 0, 6, 2, 700), ("soft", 0.0, 0, 0, 1, 1, 1600),
+                                                        ("sigmoid", 0.0, 0, 0, 1, 1, 1600)])
 @pytest.mark.parametrize("where", ["query", "key", "value"])
-def test_infinities_in_the_tiles_of_a_cluster(gpu, kind, cap, window, keep, where):
+def test_infinities_in_the_tiles_of_a_cluster(gpu, kind, cap, window, keep, H, Gk, T, where):
     """the same where several CTAs have the key tiles: a row that is not finite in one of them is computed once more over all of its keys"""
-    H, G, D, Dv, T, pos, maps = 6, 2, 48, 80, 450, 260, 2 if kind == "diff" else 1
+    G, D, Dv, pos, maps = Gk, 48, 80, 260, 2 if kind == "diff" else 1
     r, q, K, V, cache, table, pos0 = inputs(gpu, BF16, H, G, D, Dv, maps, pos, T, 64, 7, 0.3)
     K, V = K.copy(), V.copy()
     offsets = np.float32([r.uniform(0.2, 1.0, H), r.uniform(0.1, 1.5, H), r.uniform(-2.5, 0.0, H)])
     ld = int(gpu.cuda_lib().ggb_window_cache_ld(G, D * maps, Dv))
     raw, tab = cache.download(np.uint16).reshape(-1, ld), table.download(np.int32)
-    q[5, 1, 0, 3] = np.float32(1.5)  # a query number whose second and third parts are zero
+    q[5, min(1, H - 1), 0, 3] = np.float32(1.5)  # a query number whose second and third parts are zero
     for at, c, v in [(1, 3, np.inf), (pos + 7, 9, -np.inf), (pos + 33, 3, np.inf)]:  # first page, inside the portion
         slot = tab[at // 64] * 64 + at % 64
         if where == "key":
-            K[at, 1, 0, c] = v
-            raw[slot, maps * D + c] = 0x7f80 if v > 0 else 0xff80
+            K[at, G - 1, 0, c] = v
+            raw[slot, (G - 1) * maps * D + c] = 0x7f80 if v > 0 else 0xff80
         elif where == "value":
             V[at, 0, c] = v
             raw[slot, G * maps * D + c] = 0x7f80 if v > 0 else 0xff80
         elif at >= pos:
-            q[at - pos, 4, 0, c] = v
+            q[at - pos, min(4, H - 1), 0, c] = v
     cache.upload(raw)
     vis = seen(pos, T, window, keep, 0)
     dist = np.maximum(np.arange(pos, pos + T)[:, None] - np.arange(pos + T)[None], 0)
