@@ -25,6 +25,8 @@ enum ggb_workspace_id { GGB_WS_GEMM_SPLITS, GGB_WS_MOE_GATHER, GGB_WS_ARGMAX, GG
 int ggb_workspace(ggb_workspace_id id, size_t bytes, void **p);
 bool ggb_workspace_fits(ggb_workspace_id id, size_t bytes); // it is that large, or may grow: no graph is being captured
 int ggb_allow_smem_of(const void *kernel, size_t bytes);
+// how many clusters of `ctas` CTAs (along z) the device runs at once: a cluster lies in one GPC, whose SMs are no multiple of it
+int ggb_clusters_at_once_of(const void *kernel, int ctas, int threads, size_t smem, int *n);
 template <typename... P> int ggb_allow_smem(void (*kernel)(P...), size_t bytes) { return ggb_allow_smem_of(reinterpret_cast<const void *>(kernel), bytes); }
 
 #define GGB_CUDA(...)                                                                           \

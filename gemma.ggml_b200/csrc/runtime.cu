@@ -9,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include <math.h>
@@ -45,6 +46,7 @@ struct Context {
     bool ws_in_graph[GGB_WS_COUNT] = {}; // a capture has been given the present one
     std::vector<void *> ws_kept;         // those that graphs may hold and larger ones have taken the place of
     std::map<const void *, size_t> smem_allowed;
+    std::map<std::tuple<const void *, int, int, size_t>, int> clusters; // kernel, CTAs of a cluster, threads, shared memory
 };
 
 Context g_ctx;
@@ -107,6 +109,24 @@ int ggb_allow_smem_of(const void *kernel, size_t bytes) {
         GGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         allowed = bytes;
     }
+    return GGB_OK;
+}
+int ggb_clusters_at_once_of(const void *kernel, int ctas, int threads, size_t smem, int *n) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    const auto at = g_ctx.clusters.find({kernel, ctas, threads, smem});
+    if (at != g_ctx.clusters.end()) {
+        *n = at->second;
+        return GGB_OK;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1, 1, (unsigned)ctas), cfg.blockDim = dim3((unsigned)threads), cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = 1, cluster.val.clusterDim.y = 1, cluster.val.clusterDim.z = (unsigned)ctas;
+    cfg.attrs = &cluster, cfg.numAttrs = 1;
+    GGB_CUDA(cudaOccupancyMaxActiveClusters(n, kernel, &cfg));
+    g_ctx.clusters[{kernel, ctas, threads, smem}] = *n;
     return GGB_OK;
 }
 size_t ggb_tables_bytes() { return 2 * 65536 * 2; } // exp then gelu, contiguous from ggb_exp_table_dev()

@@ -659,14 +659,20 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
 // itself (or its window) has to hold what saves that at position 0: three tiles a part, and ten of them where there is a maximum to find.  Soft-max heads, two parts, graph
 // replays: 385 tokens x 4 heads (1 key head) of 64 17.5 us (15.3 alone), 512 18.3 (17.4), 512 x 2 (2) of 128 21.5 (20.9), 640 19.3 (19.1) and 22.7 (23.9), a window of 400 18.8 (17.2); sigmoid
 // heads, 385 x 4 (1) of 64 17.0 (17.1), 640 19.2 (23.1).  Four parts, heads of 128: 1000 tokens x 4 heads (1) at position 900 26.4 us (48.5 alone).
-// With more CTAs than SMs two parts cost: 777 tokens of 16 sigmoid heads (4) at 1024, 100 CTAs: 63.8 (53.6).
+// No more parts than clusters of them run at once: the last ones would wait for the first (777 tokens x 8 heads (8) of 64, 56 clusters of four, 36; alone 25; 2048 x 1, 16 clusters of
+// eight 28.7, of four 20.3), which pays only where the first ones, without a window, have few tiles and the last ones many (4500 x 1, 36 clusters of four 34, of two 48).  With more CTAs
+// than SMs two parts cost: 777 tokens of 16 sigmoid heads (4) at 1024, 100 CTAs: 63.8 (53.6).
 template <int MODE, int MAPS, typename FIN> int launch(const shape &a, const FIN &fin) {
     const int TQ = kRows / MAPS / (a.H / a.G);
     const int64_t ctas = (a.T + TQ - 1) / TQ * a.G, own = (a.window > 0 ? std::min(a.T, a.window) : a.T) / kKeys; // tiles of the portion
     const size_t alone = smem_bytes(MODE, MAPS, a.D, a.Dv, a.H / a.G), shared = std::max(alone, kOneCtaSmem); // clusters with tensor memory
     auto split = attn_kernel<MODE, MAPS, true, FIN>;
     unsigned parts = 1;
-    while (parts < 8 && own >= (MODE == SOFTMAX ? 10 : 6) && parts * 2 <= own / 3 && ctas * parts * 2 <= ggb_sm_count()) parts *= 2;
+    for (int rc, n; parts < 8 && own >= (MODE == SOFTMAX ? 10 : 6) && parts * 2 <= own / 3 && ctas * parts * 2 <= ggb_sm_count(); parts *= 2) {
+        if ((rc = ggb_allow_smem(split, shared))) return rc;
+        if ((rc = ggb_clusters_at_once_of(reinterpret_cast<const void *>(split), (int)parts * 2, kThreads, shared, &n))) return rc;
+        if (ctas > n && (a.window > 0 || own < 20 * parts)) break;
+    }
     const size_t smem = parts > 1 ? shared : alone;
     auto kfn = parts > 1 ? split : attn_kernel<MODE, MAPS, false, FIN>;
     const int rc = ggb_allow_smem(kfn, smem);
