@@ -83,6 +83,22 @@ def test_choice_does_not_depend_on_the_tokens_of_a_call(gpu, E, T):
         assert np.array_equal(idx.download(np.int32, top), many[0][t]) and np.array_equal(wt.download(np.uint32, top), many[1][t])
 
 
+@pytest.mark.parametrize("T,E", [(3, 8), (1203, 8), (2400, 32), (3, 40), (1203, 40)])
+def test_logits_that_are_no_numbers_choose_experts_that_exist(gpu, T, E):
+    """tokens of NaN beside others, in the launch that computes the logits and in one of its own; the others' choice stays theirs"""
+    W, top, r, lib = 132, 4, np.random.default_rng(E + T), gpu.cuda_lib()
+    hv, hr = as_dt(BF16, r.standard_normal((T, W)))
+    bad = [0, T // 2, T - 1]
+    hr = hr.reshape(T, W).copy()
+    hr[bad, 5] = 0x7fc0
+    w, idx, wt, z = dev(gpu, f32(r.standard_normal((E, W)))), zeros(gpu, T * top * 4), zeros(gpu, T * top * 4), zeros(gpu, T * E * 4)
+    gpu.check(lib.ggb_op_moe_route(BF16, dev(gpu, hr).ptr, W, T, w.ptr, None, E, top, z.ptr, idx.ptr, wt.ptr))
+    got, logits = idx.download(np.int32).reshape(T, top), z.download(np.float32).reshape(T, E)
+    assert ((got >= 0) & (got < E)).all() and np.isnan(logits[bad]).all()
+    good = np.setdiff1d(np.arange(T), bad)
+    assert np.array_equal(got[good], np.argsort(-logits[good], axis=1, kind="stable")[:, :top]) and np.isfinite(wt.download(np.float32).reshape(T, top)[good]).all()
+
+
 @pytest.mark.parametrize("gather", [0, 1])
 @pytest.mark.parametrize("counts,N,K", [([0, 1, 16, 17, 31, 33, 0, 160, 255, 0], 160, 448), ([256, 257, 0], 416, 64), ([513, 1, 2], 96, 192), ([700, 900], 1408, 128),
                                         ([3] * 300, 32, 64), ([17, 600, 0, 0], 288, 1024),
