@@ -5,7 +5,7 @@ with the mat-vec kernels' HBM roofline fraction and the reference's CPU path tim
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
 A "step" is one decode token through the whole path (embedding row -> L layers -> logits -> greedy
-token) at a pinned context length n_kv = ctx (BASELINE.json config 2: Gemma-2B, Q4_0, batch 1,
+token) at a pinned context length n_kv = ctx (Gemma-2B, Q4_0, batch 1,
 ctx 2048).  Weights (1.41 GB) are larger than the 126 MB L2, so every step re-streams them from HBM;
 no L2 flush is needed.  One JSON line is printed by rank 0.
 """
@@ -513,7 +513,7 @@ def run_ours(args):
 
 
 def run_prefill(args):
-    """Secondary workload: batched prefill of T tokens through the dequant -> bf16
+    """Secondary workload (a prompt of Gemma-2B, Q8_0): batched prefill of T tokens through the dequant -> bf16
     tcgen05 GEMMs.  value = prompt tokens/s; roofline = tensor pipe (GEMM flops / cudaEvent time of the GEMM
     launches vs the measured dense bf16 peak)."""
     import gemma_ggml_b200 as G

@@ -3,7 +3,7 @@
 //   * the directory is a run-time setting (the reference hard-codes /home/geraltigas/..., src/tensor_dump.h:12),
 //   * tensors are handed over as (pointer, byte size) - dump_ptr_data's signature - because the B200 path has no
 //     ggml_tensor (device intermediates are fetched with gemma_model::get_capture first),
-//   * besides the reference's byte compare (compare_tensors -> bool) there is the report BASELINE.json asks for:
+//   * besides the reference's byte compare (compare_tensors -> bool) there is a report:
 //     max-abs / max-rel error and the number of differing elements of an fp32 tensor pair.
 #ifndef GGB_TENSOR_DUMP_H
 #define GGB_TENSOR_DUMP_H

@@ -3,7 +3,7 @@
  *
  * A plain-C restatement of the ggml numerics that gemma.ggml's hot path runs
  * through (the reference links an un-vendored, patched ggml under lib/, absent
- * from /root/reference: CMakeLists.txt:13, .gitignore:4).  Only tests/,
+ * from the reference: CMakeLists.txt:13, .gitignore:4).  Only tests/,
  * __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs
  * may load this library; the product (libggb_cuda.so / libggb_host.so) never
  * links or calls it.

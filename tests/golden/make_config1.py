@@ -1,4 +1,4 @@
-"""Generates tests/golden/config1_<model>_<wtype>.npz — BASELINE.json config 1 at FULL size on the CPU oracle.
+"""Generates tests/golden/config1_<model>_<wtype>.npz — a greedy stream at FULL size on the CPU oracle.
 
 Gemma-2B architecture, seeded random-init weights, prompt id_i = (1 + 7919 i) mod V (128 tokens), 64 greedy
 tokens, through the oracle's REF order (the scalar ggml order of the reference's CPU path; loop of

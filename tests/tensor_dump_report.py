@@ -1,7 +1,7 @@
 """Per-layer parity report at FULL model size through the tensor_dump harness (script, not a test: it uses the CPU
 oracle, so it lives under tests/).  Gemma-2B, a short prompt decoded token by token on the GPU (persistent kernel) and by
 the oracle (scalar ggml order); every named intermediate of the LAST step is dumped as <name>-<layer>_source /
-_target and compared.  Writes gpurun_out/tensor_dump_report_<model>_<wtype>.json; copy it to profiles/.
+_target and compared.  Writes build/reports/tensor_dump_report_<model>_<wtype>.json.
 
 usage: python tests/tensor_dump_report.py [2b|7b] [q4_0|q8_0] [n_prompt] [n_decode]"""
 import ctypes as C
@@ -43,7 +43,7 @@ def main():
     om = O.Model(wtype=wtype, **dims)
     rep = (C.c_double * 5)()
     rows, summary = [], {}
-    for order, oname in ((O.REF, "REF"),):  # one order since round 2: the scalar ggml order
+    for order, oname in ((O.REF, "REF"),):  # the scalar ggml order
         otoks, _, _ = om.generate(prompt, n_decode, order)
         names = [(f"{cap}-{il}", om.capture(cap, il)) for il in range(dims["n_layer"]) for cap in sizes]
         names.append(("result_output", om.capture("result_output")))
@@ -63,7 +63,7 @@ def main():
                               worst_max_abs=worst_abs, worst_max_abs_over_tensor_max=worst_rel_scale)
     out = dict(model=model, wtype=wname, n_prompt=n_prompt, n_decode=n_decode, tokens=[int(x) for x in toks],
                exp_computed=bool(m.exp_computed), summary=summary, tensors=rows)
-    path = os.path.join(ROOT, "gpurun_out", f"tensor_dump_report_{model}_{wname}.json")
+    path = os.path.join(ROOT, "build", "reports", f"tensor_dump_report_{model}_{wname}.json")
     os.makedirs(os.path.dirname(path), exist_ok=True)
     json.dump(out, open(path, "w"), indent=0)
     print(json.dumps(summary))

@@ -1,5 +1,5 @@
 """K-quant dots: the oracle's restatements pinned (a) to the REFERENCE's own scalar code compiled from
-/root/reference/src/kernals.cl into oracle/_ref (bit-exact: Q4_K x Q8_K and F16 x F16), (b) to gguf-py's block layouts
+the reference's src/kernals.cl into oracle/_ref (bit-exact: Q4_K x Q8_K and F16 x F16), (b) to gguf-py's block layouts
 (dequantize_blocks) and a float64 model (Q4_K and Q6_K; the reference's Q6_K copy is broken, see oracle/ggml_oracle.h)."""
 import ctypes as C
 import os

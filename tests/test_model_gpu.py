@@ -80,7 +80,7 @@ def test_generate_matches_oracle(gpu, name, wtype, fused):
 
 @pytest.mark.parametrize("wname", ["q8_0", "q4_0"])
 def test_config1_full_size_greedy_stream(gpu, wname):
-    """BASELINE.json config 1 at FULL size: Gemma-2B, 128-token prompt id_i = (1 + 7919 i) mod V, 64 greedy tokens,
+    """A greedy stream at FULL size: Gemma-2B, 128-token prompt id_i = (1 + 7919 i) mod V, 64 greedy tokens,
     against the oracle's run of the reference CPU path (tests/golden/config1_2b_*.npz, made by
     tests/golden/make_config1.py; loop of ref: src/gemma_model.cpp:548-575).  The stream is NOT degenerate
     (sigma_embd = 0.004: 64 distinct ids, top-2 margins down to 4e-5 of |logit| ~ 0.85), so it is reproduced only by
@@ -107,7 +107,7 @@ def test_config1_full_size_greedy_stream(gpu, wname):
         assert tok == int(z["tokens"][s]), f"step {s}: token {tok} != {int(z['tokens'][s])} (top-2 margin {margins[s]:.2e})"
         assert np.array_equal(bits(lg[z["top_idx"][s]]), bits(z["top_val"][s])), f"step {s}: top-16 logits differ"
         assert np.array_equal(bits(lg[z["sample_idx"]]), bits(z["sample_val"][s])), f"step {s}: sampled logits differ"
-    out_dir = os.path.join(os.path.dirname(GOLDEN), "..", "gpurun_out")
+    out_dir = os.path.join(os.path.dirname(GOLDEN), "..", "build", "reports")
     if os.path.isdir(out_dir):
         import json
         json.dump(dict(config="gemma-2b %s, 128-token prompt + 64 greedy tokens" % wname, tokens_identical=64,

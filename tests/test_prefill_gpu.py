@@ -153,7 +153,7 @@ def test_prefill_agrees_with_token_by_token_decode_path(gpu):
     m.close()
 
 
-# Full size (BASELINE.json config 3: Gemma-2B Q8_0, 512-token prompt).  The reference for the comparison is our own decode
+# Full size (Gemma-2B Q8_0, 512-token prompt).  The reference for the comparison is our own decode
 # path run token by token, which is bit-identical to the oracle's scalar ggml order (tests/test_model_gpu.py) - the oracle
 # itself would need ~15 minutes for 512 positions.  The two paths round differently BY DESIGN (bf16 activations and
 # weights vs Q8_0 re-quantised activations), and 18 layers of random-init weights amplify that: the full-size tolerance
@@ -187,8 +187,8 @@ def test_config3_full_size_prefill_against_the_bit_exact_path(gpu):
         gk, gv = (a[:T].view(np.float16).astype(np.float32) for a in m.kv(il))
         report["kv"][str(il)] = {"k_dev_rel": float(np.abs(gk - dk).max() / max(1.0, np.abs(dk).max())),
                                  "v_dev_rel": float(np.abs(gv - dv).max() / max(1.0, np.abs(dv).max()))}
-    os.makedirs(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out"), exist_ok=True)
-    json.dump(report, open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out",
+    os.makedirs(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "build", "reports"), exist_ok=True)
+    json.dump(report, open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "build", "reports",
                                         "config3_prefill_parity.json"), "w"), indent=1)
     print(json.dumps(report))
     assert dev < FULL_PREFILL_TOL * max(1.0, rng_), report

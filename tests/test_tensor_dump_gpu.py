@@ -48,7 +48,7 @@ def test_per_layer_parity_via_tensor_dump(gpu, tmp_path, wtype):
                     assert H.td_compare_tensors(key) == 1, key   # the reference's byte compare
                 else:
                     assert rep[2] <= REF_TOL * max(1.0, rep[4]), (key, list(rep))
-    out_dir = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out")
+    out_dir = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "build", "reports")
     if os.path.isdir(out_dir):
         json.dump(report, open(os.path.join(out_dir, f"tensor_dump_report_small_{'q4_0' if wtype == O.TYPE_Q4_0 else 'q8_0'}.json"), "w"), indent=0)
     m.close(); om.close()
