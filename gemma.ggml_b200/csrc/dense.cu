@@ -53,7 +53,7 @@ __device__ __forceinline__ void vec_row_dot(const E *__restrict__ wr, const E *_
 
 // ACT: the output is act(.) in the matrices' type (c_act) instead of fp32 (c).  KS warps share a row, their sums are added in order: few long
 // rows leave too few bytes in flight with a warp each (in a graph, matrices from memory, 2048 rows of 8192 bf16 numbers: 14 warps an SM, 13.7 us;
-// four a row: 7.3, 4.6 TB/s; two: 8.8; 2048 x 2048: 4.9, 3.5 with two; 300 x 7000: 13.3, 3.9).  One token: 32 registers, so that an SM holds 64 warps
+// four a row: 7.3, 4.6 TB/s; two: 8.8; 2048 x 2048: 5.0, 3.5 with two; 300 x 7000: 13.6, 4.3 with eight).  One token: 32 registers, so that an SM holds 64 warps
 // (4096 x 4096 with two a row in 34 registers: 9.2 us, in two waves).  FEW, of one warp a row: the warps of a CTA counted at run time, by which the compiler
 // holds fewer loads ahead (bf16, 6, 7, 8 tokens: 60, 72, 72 registers, 4, 3, 3 CTAs an SM; counted ahead 68, 84, 94: 3, 2, 2).
 template <typename E, int TT, int ACT, int KS, bool FEW = false>

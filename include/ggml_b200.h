@@ -273,7 +273,8 @@ int ggb_op_attn_prefill(const float *q, const void *kcache, const void *vcache, 
 size_t ggb_dtype_size(int dt);
 /* c[t][n] (fp32) = sum_k a[t][k] w[n][k]: a streaming mat-vec for T <= 8, the tcgen05 GEMM for aligned bf16 shapes
  * (K %% 64 == 0, N %% 32 == 0, lda == K, T >= 64), tensor cores behind ordinary loads for other shapes and fp32 from K > 128 on, a shared-memory
- * tile kernel for shorter sums */
+ * tile kernel for shorter sums.  The order of the sums goes by N, K and T: a token's numbers are the same to rounding, not to the bit, in
+ * calls of other numbers of tokens */
 int ggb_op_linear(int dt, const void *w, int64_t N, int64_t K, const void *a, int64_t lda, int64_t T, float *c, int64_t ldc);
 /* y = x / sqrt(mean(x^2) + eps) * w for up to two weights of the same rows (the root mean square is computed once);
  * w_stride 0: the weight is one number, 1: a vector of E; y1 / y2 ([T][E] in dt) may be NULL */
