@@ -96,18 +96,75 @@ __global__ void __launch_bounds__(32) moe_select_kernel(const float *zg, int n_e
     select_top_warp(z, z + n_exp, n_exp, top, t, lane, idx, wt);
 }
 
-// A portion of tokens: a warp computes TT (4 or 8) tokens x 4 experts, so that a row of the router is read once for TT tokens and a token's row once
-// for four experts (a warp per logit reads 268 MB through L2 for 1024 tokens x 32 experts of width 2048); `wide` of a CTA's eight warps stand beside each other
-// with the same tokens, whose rows come from L1 to all but one of them.  Every logit is the same sum in the same order as router_dot's, to the bit: a choice
-// between experts does not depend on how many tokens share the call.  TOP: the experts are 32 at most, and a warp then chooses for each token of the CTA
+// A portion of tokens: a warp computes 4 tokens x 4 experts, so that a row of the router is read once for four tokens and a token's row once
+// for four experts (a warp per logit reads 268 MB through L2 for 1024 tokens x 32 experts of width 2048).  Every logit is the same
+// sum in the same order as router_dot's, to the bit: a choice between experts does not depend on how many tokens share the call.
+// Bound by instruction issue.
+constexpr int kLogitExperts = 4;
+template <typename E>
+__global__ void __launch_bounds__(256) moe_logits_tile_kernel(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, float *z) {
+    step_wait();
+    struct alignas(4 * sizeof(E)) quad {
+        E v[4];
+    };
+    const int lane = threadIdx.x & 31, groups = (n_exp + kLogitExperts - 1) / kLogitExperts;
+    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), t0 = item / groups * kLogitExperts;
+    const int e0 = (int)(item % groups) * kLogitExperts;
+    if (t0 >= T) return;
+    const E *hr[kLogitExperts];
+    const float *wr[kLogitExperts];
+#pragma unroll
+    for (int i = 0; i < kLogitExperts; i++) { // past the end: the last one again, not stored
+        hr[i] = h + min(t0 + i, T - 1) * W;
+        wr[i] = w + (int64_t)min(e0 + i, n_exp - 1) * W;
+    }
+    float s[kLogitExperts * kLogitExperts]; // [token][expert]
+#pragma unroll
+    for (int i = 0; i < kLogitExperts * kLogitExperts; i++) s[i] = 0.f;
+#pragma unroll 2
+    for (int64_t k = (int64_t)lane * 4; k < W; k += 128) {
+        float hv[kLogitExperts][4];
+        float4 wv[kLogitExperts];
+#pragma unroll
+        for (int i = 0; i < kLogitExperts; i++) {
+            const quad q = *reinterpret_cast<const quad *>(hr[i] + k);
+            wv[i] = *reinterpret_cast<const float4 *>(wr[i] + k);
+#pragma unroll
+            for (int c = 0; c < 4; c++) hv[i][c] = to_f32(q.v[c]);
+        }
+#pragma unroll
+        for (int i = 0; i < kLogitExperts; i++)
+#pragma unroll
+            for (int j = 0; j < kLogitExperts; j++) {
+                float &a = s[i * kLogitExperts + j];
+                a = fmaf(wv[j].x, hv[i][0], a);
+                a = fmaf(wv[j].y, hv[i][1], a);
+                a = fmaf(wv[j].z, hv[i][2], a);
+                a = fmaf(wv[j].w, hv[i][3], a);
+            }
+    }
+    // sixteen sums at once, each by the additions of warp_sum_f32: a lane ends with sum lane / 2
+#pragma unroll
+    for (int n = 8, off = 16; n >= 1; n >>= 1, off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < n; i++) s[i] = __fadd_rn(up ? s[n + i] : s[i], __shfl_xor_sync(0xffffffffu, up ? s[i] : s[n + i], off));
+    }
+    s[0] = __fadd_rn(s[0], __shfl_xor_sync(0xffffffffu, s[0], 1));
+    const int i = lane >> 3, j = (lane >> 1) & 3;
+    if (!(lane & 1) && t0 + i < T && e0 + j < n_exp) z[(t0 + i) * n_exp + e0 + j] = s[0] + (b ? b[e0 + j] : 0.f);
+}
+
+// The same of TT (4 or 8) tokens x 4 experts a warp, where there are no more CTAs than SMs; `wide` of a CTA's eight warps stand beside each other
+// with the same tokens, whose rows come from L1 to all but one of them.  TOP: the experts are 32 at most, and a warp then chooses for each token of the CTA
 // (idx and wt), which spares a launch.
 // Bound by the issue of instructions (two multiply-adds in one) and by L2's latency, against which each lane brings its own numbers of the next kLogitAhead
-// steps of 128 into shared memory.  1024 x 32 x 2048: 10.6 us with the choice (11.7 with two steps in registers; 11.0 with 4 x 4 tiles, single multiply-adds and
+// steps of 128 into shared memory: all that an SM has for one CTA.  1024 x 32 x 2048: 10.6 us with the choice (11.7 with two steps in registers; 11.0 with 4 x 4 tiles, single multiply-adds and
 // another launch for the choice); 1024 x 16 x 1024: 5.5 (6.5).
-constexpr int kLogitExperts = 4, kLogitWarps = 8, kLogitAhead = 4;
+constexpr int kLogitWarps = 8, kLogitAhead = 4;
 template <typename E, int TT> constexpr size_t logit_smem() { return (size_t)kLogitAhead * 32 * kLogitWarps * (kLogitExperts * 16 + TT * 4 * sizeof(E)); }
 template <typename E, int TT, bool TOP>
-__global__ void __launch_bounds__(32 * kLogitWarps) moe_logits_tile_kernel(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, int wide, float *z, int top,
+__global__ void __launch_bounds__(32 * kLogitWarps) moe_logits_cta_kernel(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, int wide, float *z, int top,
                                                                            int32_t *idx, float *wt) {
     constexpr int NE = kLogitExperts, NS = TT * NE, AT = kLogitAhead; // sums of a warp; steps under way
     extern __shared__ uint8_t lg_raw[];
@@ -204,26 +261,30 @@ __global__ void __launch_bounds__(32 * kLogitWarps) moe_logits_tile_kernel(const
     }
 }
 
-// The form by the number of logits: below a warp for every scheduler of the chip, tiles would leave SMs idle; eight tokens a warp where that still is
-// a CTA for two SMs of three: a CTA of four reads the router as often for half the tokens (1024 tokens x 32 experts of 2048: 10.6 us, with four 12.6).  chosen: idx and wt have been computed too
+// The form by the number of logits: below a warp for every scheduler of the chip, tiles would leave SMs idle.  Tiles by CTAs that share rows only while there are no
+// more of them than SMs (more: 4096 x 32 x 2048 27.0 us by warps, 38.6; 1536 x 20 10.9, 20.3; 1024 x 128 25.7, 39.0), without idle warps (20, 33 or 40 experts; 1024 x 33 x 2048
+// 11.1, 19.1) and with four warps beside each other at least (4096 x 4 11.4, 15.8), of long rows if the choice takes another launch (128 x 128 x 256 4.9, 5.2; x 2048 9.7, 9.5; 256 x 64 10.3, 9.6).
+// Eight tokens a warp only of bf16 rows (1024 x 32 x 2048 10.9, 10.5; fp32 11.8, 12.4), with the choice (256 x 128 10.7, 12.9).  chosen: idx and wt have been computed too
 template <typename E>
 int logits_launch(const E *h, int64_t W, int64_t T, const float *w, const float *b, int n_exp, float *z, int top = 0, int32_t *idx = nullptr, float *wt = nullptr,
                   bool *chosen = nullptr) {
     const int64_t groups = (n_exp + kLogitExperts - 1) / kLogitExperts, tiles = (T + 3) / 4 * groups;
-    if (W % 4 == 0 && W < (1 << 28) && tiles >= 4 * ggb_sm_count()) {
-        int wide = 1; // warps beside each other
-        while (wide < kLogitWarps && wide < groups) wide *= 2;
-        const int rows = kLogitWarps / wide;
+    if (W % 4 == 0 && tiles >= 4 * ggb_sm_count()) {
+        const int wide = (int)std::min<int64_t>(groups, kLogitWarps), rows = kLogitWarps / wide; // warps beside each other; where they are four or eight
         const unsigned ey = (unsigned)((groups + wide - 1) / wide);
-        const bool eight = (T + 8 * rows - 1) / (8 * rows) * ey * 3 >= 2 * ggb_sm_count(), fused = chosen && ey == 1;
-        const int tokens = rows * (eight ? 8 : 4);
-        const dim3 grid((unsigned)((T + tokens - 1) / tokens), ey), block(32 * kLogitWarps);
-        if (chosen) *chosen = fused;
+        const bool fits = (groups == 4 || groups % 8 == 0) && W < (1 << 28), fused = chosen && ey == 1;
+        auto ctas = [&](int tokens) { return (T + tokens * rows - 1) / (tokens * rows); };
         int rc = GGB_OK;
 #define TILE(TT, TOP)                                                                                                                              \
-    if ((rc = ggb_allow_smem(moe_logits_tile_kernel<E, TT, TOP>, logit_smem<E, TT>()))) return rc;                                               \
-    ggb_launch_step(moe_logits_tile_kernel<E, TT, TOP>, grid, block, logit_smem<E, TT>(), h, W, T, w, b, n_exp, wide, z, top, idx, wt)
-        if (eight && fused) { TILE(8, true); } else if (eight) { TILE(8, false); } else if (fused) { TILE(4, true); } else { TILE(4, false); }
+    if ((rc = ggb_allow_smem(moe_logits_cta_kernel<E, TT, TOP>, logit_smem<E, TT>()))) return rc;                                                \
+    ggb_launch_step(moe_logits_cta_kernel<E, TT, TOP>, dim3((unsigned)ctas(TT), ey), dim3(32 * kLogitWarps), logit_smem<E, TT>(), h, W, T, w, b, n_exp, wide, z, top, idx, wt)
+        if (fits && ctas(4) * ey <= ggb_sm_count() && (fused || W >= 512)) {
+            if (chosen) *chosen = fused;
+            if (fused) { TILE(4, true); } else { TILE(4, false); }
+        } else if (sizeof(E) == 2 && fits && fused && groups == 8 && ctas(8) <= ggb_sm_count()) {
+            *chosen = true;
+            if constexpr (sizeof(E) == 2) { TILE(8, true); }
+        } else ggb_launch_step(moe_logits_tile_kernel<E>, dim3((unsigned)((tiles + 7) / 8)), dim3(256), 0, h, W, T, w, b, n_exp, z);
 #undef TILE
     } else ggb_launch_step(moe_logits_kernel<E>, dim3((unsigned)((T * n_exp + 7) / 8)), dim3(256), 0, h, W, T, w, b, n_exp, z);
     GGB_LAUNCH_CHECK();

@@ -64,9 +64,8 @@ def test_weighted_sum(gpu, W, top):
     assert np.abs(out.download(np.float32).reshape(T, W) - want).max() < top * 2.0 ** -23 * 8
 
 
-@pytest.mark.parametrize("E", [5, 8, 32])
-@pytest.mark.parametrize("T", [1203, 2400])
-def test_choice_does_not_depend_on_the_tokens_of_a_call(gpu, E, T):
+@pytest.mark.parametrize("T,E", [(1203, 5), (2400, 5), (1203, 8), (2400, 8), (1203, 32), (2400, 32), (1184, 16), (1185, 16), (592, 32), (593, 32), (1183, 31), (1184, 30), (1185, 32), (1203, 20)])
+def test_choice_does_not_depend_on_the_tokens_of_a_call(gpu, T, E):
     """up to 32 experts of a portion are chosen where their logits are computed: the bits of a token by itself, ties to the lower index"""
     W, top, r, lib = 132, 4, np.random.default_rng(E), gpu.cuda_lib()
     h = dev(gpu, as_dt(BF16, r.standard_normal((T, W)))[1])
@@ -83,7 +82,22 @@ def test_choice_does_not_depend_on_the_tokens_of_a_call(gpu, E, T):
         assert np.array_equal(idx.download(np.int32, top), many[0][t]) and np.array_equal(wt.download(np.uint32, top), many[1][t])
 
 
-@pytest.mark.parametrize("T,E", [(3, 8), (1203, 8), (2400, 32), (3, 40), (1203, 40)])
+@pytest.mark.parametrize("T,W,E", [(150, 516, 64), (296, 512, 64), (297, 516, 64), (148, 512, 128), (150, 516, 128), (73, 1028, 256), (150, 508, 64), (300, 516, 40), (300, 514, 64)])
+def test_logits_of_many_experts_are_the_bits_of_a_token_by_itself(gpu, T, W, E):
+    top, r, lib = 3, np.random.default_rng(E + T), gpu.cuda_lib()
+    for dt in (BF16, F32):
+        h = dev(gpu, as_dt(dt, r.standard_normal((T, W)))[1])
+        w, idx, wt = dev(gpu, f32(r.standard_normal((E, W)))), zeros(gpu, T * top * 4), zeros(gpu, T * top * 4)
+        z, one = zeros(gpu, T * E * 4), zeros(gpu, E * 4)
+        gpu.check(lib.ggb_op_moe_route(dt, h.ptr, W, T, w.ptr, None, E, top, z.ptr, idx.ptr, wt.ptr))
+        many, got = z.download(np.float32).reshape(T, E), idx.download(np.int32).reshape(T, top).copy()
+        assert np.array_equal(got, np.argsort(-many, axis=1, kind="stable")[:, :top])
+        for t in (0, T // 2, T - 1):
+            gpu.check(lib.ggb_op_moe_route(dt, h.ptr.value + t * W * (2 if dt == BF16 else 4), W, 1, w.ptr, None, E, top, one.ptr, idx.ptr, wt.ptr))
+            assert np.array_equal(one.download(np.float32), many[t])
+
+
+@pytest.mark.parametrize("T,E", [(3, 8), (1203, 8), (2400, 32), (3, 40), (1203, 40), (500, 32), (1100, 32), (1100, 16)])
 def test_logits_that_are_no_numbers_choose_experts_that_exist(gpu, T, E):
     """tokens of NaN beside others, in the launch that computes the logits and in one of its own; the others' choice stays theirs"""
     W, top, r, lib = 132, 4, np.random.default_rng(E + T), gpu.cuda_lib()
