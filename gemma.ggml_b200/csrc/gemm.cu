@@ -328,6 +328,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
                     if (++s == kStages) s = 0, ph ^= 1u;
                 }
             }
+            for (int k = 0; k < kStages && mbar_wait_bounded(bars + EMPTY + 8 * s, ph ^ 1u, dead); k++) // every arrival of the MMAs is here
+                if (++s == kStages) s = 0, ph ^= 1u;
         }
         __syncwarp();
     } else if (warp == 1 && rank == 0) {
@@ -355,6 +357,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
             }
             umma_arrive_pair(bars + ACC_FULL + 8 * buf);
         }
+        for (int k = 0; k < n_acc; k++, it++) { // and of the epilogues of both
+            const int buf = n_acc == 2 ? it & 1 : 0, use = n_acc == 2 ? it >> 1 : it;
+            mbar_wait_bounded(bars + ACC_FREE + 8 * buf, (use & 1) ^ 1, dead);
+        }
     } else if (warp >= 4) {
         const int w8 = warp - 4, lq = warp & 3, half = w8 >> 2;
         int it = 0;
@@ -375,14 +381,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pair_kernel(const __grid_con
             if (lane == 0) mbar_arrive_cluster(bars0 + ACC_FREE + 8 * buf);
         }
     }
+    warp_meet();
     __syncthreads();
     if (warp == 2) settle(dead);
-    cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
+    cluster_sync(); // neither gives its tensor memory back while the other one's MMAs or arrivals may still reach it
     if (warp == 2) {
         tc_fence_after();
         tmem_free512_pair(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;
     }
+    cluster_sync(); // and neither leaves before the other one has
 }
 
 // The slots of a mixture of experts, sorted by group: C[slot][N] = A[slot][K] W[group of the slot][N][K]^T.  A pair of CTAs owns 256 features (the M of an MMA, half
@@ -505,6 +513,8 @@ __global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __gri
                     if (++s == kSlotStages) s = 0, ph ^= 1u;
                 }
             }
+            for (int k = 0; k < kSlotStages && mbar_wait_bounded(bars + EMPTY + 8 * s, ph, dead); k++) // every arrival of the MMAs is here
+                if (++s == kSlotStages) s = 0, ph ^= 1u;
         }
         __syncwarp();
     } else if (warp == 1 && rank == 0) {
@@ -524,6 +534,7 @@ __global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __gri
             }
             umma_arrive_pair(bars + ACC_FULL + 8 * buf);
         }
+        for (int k = 0; k < 2; k++, it++) mbar_wait_bounded(bars + ACC_FREE + 8 * (it & 1), ((it >> 1) & 1) ^ 1, dead); // and of the epilogues of both
     } else if (warp >= 12) {
         // stages grp, grp + 3, ... of all of this CTA's, into two places of the ring: a thread copies one 16-byte piece of every 16th row
         const int grp = (warp - 12) / kCopyWarps, lt = (tid - kThreads) % (32 * kCopyWarps), pc = lt & 7, r0 = lt >> 3;
@@ -597,14 +608,16 @@ __global__ void __launch_bounds__(kSlotThreads, 1) gemm_slots_kernel(const __gri
             if (lane == 0) mbar_arrive_cluster(bars0 + ACC_FREE + 8 * buf);
         }
     }
+    warp_meet();
     __syncthreads();
     if (warp == 2) settle(dead);
-    cluster_sync(); // neither leaves while the other one's MMAs or arrivals may still reach it
+    cluster_sync(); // neither gives its tensor memory back while the other one's MMAs or arrivals may still reach it
     if (warp == 2) {
         tc_fence_after();
         tmem_free512_pair(tmem);
         if (lane == 0 && *dead) *a.wait_error = 1;
     }
+    cluster_sync(); // and neither leaves before the other one has
 }
 
 // the CTAs' sums along K in order

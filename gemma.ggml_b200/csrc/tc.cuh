@@ -155,10 +155,18 @@ __device__ __forceinline__ double ld_cluster_f64(uint32_t addr) {
     asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The lanes of a warp together again: behind waits that each lane leaves by its own answer, and behind an `if (lane == 0)`, they may be apart for as long as nothing
+// joins them (a barrier of the warp does not, a vote does).  Ahead of every barrier of a CTA or cluster that such a warp comes to: one that is executed by parts of a warp
+// counts it twice, and then lets CTAs go on, or leave, ahead of others that still reach them.
+__device__ __forceinline__ void warp_meet() { asm volatile("{\n.reg .pred p, q;\nsetp.eq.u32 p, 0, 0;\nvote.sync.all.pred q, p, 0xffffffff;\n}" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() {
+    warp_meet();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 // An arrival on another CTA's barrier.  What it announces lies in this CTA's own shared or tensor memory and is read there by the tensor
 // cores, behind this CTA's proxy fence and barrier: no release at cluster scope, which would flush for a microsecond.

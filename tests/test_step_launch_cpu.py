@@ -84,3 +84,30 @@ def test_a_copying_warp_whose_wait_ran_out_leaves_every_loop():
             flags = re.findall(r"if \(!\((\w+) = mbar_wait_warp\(", loop)
             assert loop.count("mbar_wait_warp(") == len(flags) and all(re.search(r"\b%s\b" % f, m.group(2)) for f in flags), n
     assert found >= 1
+
+
+def test_barriers_of_a_cluster_hold_for_a_warp_whose_lanes_are_apart():
+    """Lanes that leave a wait each by its own answer may still be apart where the roles of a kernel end: a cluster's barrier that such a warp came to in parts would count
+    it twice.  Every one is behind a vote, in the form that does not take the lanes for together."""
+    found = 0
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        s = re.sub(r"//[^\n]*", "", open(path).read())
+        assert not re.search(r"barrier\.cluster\.[a-z.]*aligned", s), path
+        for m in re.finditer(r"barrier\.cluster\.arrive", s):
+            found += 1
+            assert re.search(r"warp_meet\(\);\s*asm volatile\(\"$", s[:m.start()]), path
+    assert found == 1  # cluster_arrive, which everything else calls
+
+
+def test_a_pair_of_ctas_outlives_what_is_sent_to_either():
+    """The products by pairs of CTAs: whoever fills stages, and whoever issues MMAs, waits at its end for the arrivals that nobody else waits for, and neither CTA leaves
+    before both have given their tensor memory back."""
+    ks = {n: body for n, (_, body) in kernels().items() if n[0].endswith("gemm.cu") and "umma_arrive_pair(" in body}
+    assert len(ks) == 2
+    for n, body in ks.items():
+        end = body[body.rindex("tmem_free512_pair"):]
+        assert "cluster_sync();" in end and re.search(r"warp_meet\(\);\s*__syncthreads\(\);\s*if \(warp == 2\) settle\(dead\);\s*cluster_sync\(\);", body), n
+        fills, issues = body.index("warp == 0) {"), body.index("} else if (warp == 1 && rank == 0) {")
+        assert re.search(r"for \(int k = 0; k < kS\w+ && mbar_wait_bounded\(bars \+ EMPTY", body[fills:issues]), n
+        after = body[body.index("umma_arrive_pair(bars + ACC_FULL", issues):]
+        assert "mbar_wait_bounded(bars + ACC_FREE" in after[:after.index("} else if")], n
