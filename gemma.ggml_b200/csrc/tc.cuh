@@ -177,7 +177,10 @@ __device__ __forceinline__ void tmem_alloc512_pair(uint32_t slot) { // one warp 
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_free512_pair(uint32_t base) { asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory"); }
+__device__ __forceinline__ void tmem_free512_pair(uint32_t base) {
+    warp_meet();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -216,7 +219,10 @@ __device__ __forceinline__ void tmem_alloc512(uint32_t slot) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_free512(uint32_t base) { asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory"); }
+__device__ __forceinline__ void tmem_free512(uint32_t base) { // by the warp that issued MMAs, often, whose lanes may be apart
+    warp_meet();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
+}
 
 // TMA: a box of a 2-dimensional tensor map, x (a multiple of 16 bytes) and y of its first element, to shared memory; out-of-range elements
 // arrive as zeros.  One thread.

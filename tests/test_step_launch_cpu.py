@@ -97,6 +97,9 @@ def test_barriers_of_a_cluster_hold_for_a_warp_whose_lanes_are_apart():
             found += 1
             assert re.search(r"warp_meet\(\);\s*asm volatile\(\"$", s[:m.start()]), path
     assert found == 1  # cluster_arrive, which everything else calls
+    # and tensor memory is given back by whole warps, the ones that issued MMAs among them
+    s = open(os.path.join(CSRC, "tc.cuh")).read()
+    assert len(re.findall(r"warp_meet\(\);\s*asm volatile\(\"tcgen05\.dealloc", s)) == len(re.findall(r"tcgen05\.dealloc", s)) == 2
 
 
 def test_a_pair_of_ctas_outlives_what_is_sent_to_either():
