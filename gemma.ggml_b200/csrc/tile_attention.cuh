@@ -657,8 +657,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_kernel(const __grid_constant
 // Few CTAs (few key heads, portions that are not long) leave SMs without work: up to eight CTAs then share a CTA's key tiles.  How many positions come before
 // the portion is known on the device only, and a cluster costs 2 us (its two meetings; and more numbers than the loop over tiles has registers for), so that the portion
 // itself (or its window) has to hold what saves that at position 0: three tiles a part, and ten of them where there is a maximum to find.  Soft-max heads, two parts, graph
-// replays: 385 tokens x 4 heads (1 key head) of 64 17.5 us (15.3 alone), 512 18.3 (17.4), 512 x 2 (2) of 128 21.5 (20.9), 640 19.3 (19.1) and 22.7 (23.9), a window of 400 18.8 (17.2); sigmoid
-// heads, 385 x 4 (1) of 64 17.0 (17.1), 640 19.2 (23.1).  Four parts, heads of 128: 1000 tokens x 4 heads (1) at position 900 26.4 us (48.5 alone).
+// replays: 385 tokens x 4 heads (1 key head) of 64 17.5 us (15.3 alone), 512 18.3 (17.4), 512 x 2 (2) of 128 21.5 (20.9), 640 19.4 (19.0) and 22.8 (23.8), a window of 400 18.8 (17.2); sigmoid
+// heads, 385 x 4 (1) of 64 17.0 (17.0), 640 19.4 (23.1).  Four parts, heads of 128: 1000 tokens x 4 heads (1) at position 900 26.4 us (48.5 alone).
 // No more parts than clusters of them run at once: the last ones would wait for the first (777 tokens x 8 heads (8) of 64, 56 clusters of four, 36; alone 25; 2048 x 1, 16 clusters of
 // eight 28.7, of four 20.3), which pays only where the first ones, without a window, have few tiles and the last ones many (4500 x 1, 36 clusters of four 34, of two 48).  With more CTAs
 // than SMs two parts cost: 777 tokens of 16 sigmoid heads (4) at 1024, 100 CTAs: 63.8 (53.6).
